@@ -47,6 +47,9 @@ const char *ssc_last_error(void);
 /* Number of CUDA kernels this library has launched in the calling process (memsets and copies
  * not counted).  No reference counterpart. */
 unsigned long long ssc_kernel_launches(void);
+/* out[i] = *words[i] for n int32 device words, read after everything queued on `stream` so far; waits
+ * for them.  (The reference reads counts back with .item() / .cpu().) */
+int ssc_read_words(const int32_t *const *words, int n, int32_t *out, void *stream);
 /* 1 if the tcgen05 tensor-core kernels were compiled in (always for sm_100a builds). */
 int ssc_has_tcgen05(void);
 

@@ -31,6 +31,7 @@ SIGNATURES = {
     "ssc_last_error": (ctypes.c_char_p, []),
     "ssc_has_tcgen05": (c_int, []),
     "ssc_kernel_launches": (ctypes.c_ulonglong, []),
+    "ssc_read_words": (c_int, [ctypes.POINTER(c_void_p), c_int, ctypes.POINTER(c_int), c_void_p]),
     "ssc_rulebook_scratch_bytes": (c_size_t, [c_int, c_int, _I3, _I3, c_int]),
     "ssc_rulebook_subm": (c_int, [c_void_p, c_int, c_int, _I3, _I3, _I3, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_void_p, c_size_t, c_void_p]),
@@ -241,14 +242,23 @@ def raise_on_status(value, device):
         raise RuntimeError("ssconv_b200 kernel status 0x%x (%s)" % (int(value), _STATUS_TEXT))
 
 
+def read_counts(words):
+    """Host values of device row counts (int32 words of one device).  The per-device status word rides
+    along in the same read-back, so a kernel that gave up (bounded wait, full hash, bad coordinate)
+    surfaces here, where the host waits for the device anyway, instead of handing out partial results.
+    One small kernel writes the words into mapped host memory and the host watches for them there: a
+    copy engine and a stream synchronisation per read cost several times as much."""
+    dev = words[0].device
+    n = len(words) + 1
+    ptrs = (c_void_p * n)(*[_p(w, torch.int32) for w in words], _p(status_word(dev)))
+    out = (c_int * n)()
+    _check(lib().ssc_read_words(ptrs, n, out, _stream()))
+    raise_on_status(out[n - 1], dev)
+    return out[:n - 1]
+
+
 def read_count(n_dev):
-    """Host value of a device row count.  The per-device status word rides along in the same
-    read-back, so a kernel that gave up (bounded wait, full hash, bad coordinate) surfaces here,
-    where the host waits for the device anyway, instead of handing out partial results."""
-    st = status_word(n_dev.device)
-    n, bad = torch.cat([n_dev.reshape(1), st]).tolist()
-    raise_on_status(bad, n_dev.device)
-    return int(n)
+    return read_counts([n_dev])[0]
 
 
 # =============================================================================== rulebook
@@ -447,6 +457,7 @@ class LazyPairs(object):
         self._n_out_dev = n_out_dev          # device count of a rulebook built ahead, until resolved
         self._n_out = None if n_out_dev is not None else self.capacity
         self._ratio_key = ratio_key
+        self.count = None                    # RowCount of the tensor the pending count belongs to
         self._n_in = int(n_in)
         self._tensor = None
         self.shape = torch.Size((nbr.shape[0], 2, self._n_in))
@@ -460,7 +471,9 @@ class LazyPairs(object):
         """Reads the output count of a rulebook built ahead (one host sync).  Returns it, or None
         when it exceeded the capacity (everything computed from this handle is then invalid)."""
         if self._n_out is None:
-            n = read_count(self._n_out_dev)
+            n = self.count.value if self.count is not None else None
+            if n is None:
+                n = read_count(self._n_out_dev)
             if self._ratio_key is not None:
                 _note_ratio(self._ratio_key, self._n_in, n)
             if n > self.capacity:
@@ -1121,7 +1134,7 @@ def p2v_stats(points, batch_ids, grid, unit):
     stats = torch.empty(4, dtype=torch.int32, device=points.device)
     _check(lib().ssc_p2v_stats(_p(points, torch.float32), _p(batch_ids, torch.int32), points.shape[0], _i3(grid),
                                _F3(*[float(u) for u in unit]), _p(stats), _stream()))
-    return stats.tolist()
+    return read_counts([stats[k:k + 1] for k in range(4)])
 
 
 def point2voxel(points, feats, batch_ids, batch_size, grid, unit, mode, ahead=False):

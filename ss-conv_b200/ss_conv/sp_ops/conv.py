@@ -111,6 +111,7 @@ class SparseConvolution(nn.Module):
 
                 out._rows = PendingRows(pairs._n_out_dev, pairs.capacity, input if input.pending() else None, redo,
                                         lambda n: _ext._note_ratio(key, input.features.shape[0], n))
+                pairs.count = out._rows.count
                 out._rows.indices_ready = indices_ready   # the next layer's rulebook may start here
                 return out
         if (_ext.AHEAD and input.pending() and not self.conv1x1 and not self.inverse and feats_raw.is_cuda
@@ -142,15 +143,36 @@ class SparseConvolution(nn.Module):
                 key = self.indice_key
 
                 def redo():
-                    if key is not None:
-                        input.indice_dict.pop(key, None)      # the cached table belongs to the pending rows
+                    # the table the pending rows were built on is void; one that an earlier layer of
+                    # this key has rebuilt since is the one to use (a layer that is not submanifold
+                    # itself could not build it)
+                    kept = input.find_indice_pair(key)
+                    if kept is not None and kept[2] is pairs:
+                        input.indice_dict.pop(key)
                     t = self._sparse_conv_exact(input, weight)
                     return t.features, t.indices
 
                 out._rows = PendingRows(n_in_dev, pairs.capacity, input, redo)
+                pairs.count = out._rows.count
                 out._rows.indices_ready = getattr(input._rows, "indices_ready", None)
                 return out
         return self._sparse_conv_exact(input, weight)
+
+    def _cached_rulebook(self, input):
+        """The rulebook kept under this layer's key with exact row counts (an entry made on a pending
+        row count holds capacity-sized coordinates until somebody asks), or None."""
+        cached = input.find_indice_pair(self.indice_key)
+        if cached is None or not isinstance(cached[2], _ext.LazyPairs):
+            return cached
+        outids, indices, pairs, num, shape = cached
+        n = pairs.resolve()
+        if n is None:                                  # built for rows that did not fit: void
+            input.indice_dict.pop(self.indice_key)
+            return None
+        if outids.shape[0] != n:                       # a table on pending rows has as many outputs as inputs
+            outids, indices = outids[:n], indices[:n]
+            cached = input.indice_dict[self.indice_key] = (outids, indices, pairs, num, shape)
+        return cached
 
     def _sparse_conv_exact(self, input, weight):
         features, indices = input.features, input.indices
@@ -170,7 +192,7 @@ class SparseConvolution(nn.Module):
                 input.features += self.bias
             return input
 
-        cached = input.find_indice_pair(self.indice_key)
+        cached = self._cached_rulebook(input)
         if self.inverse:
             assert cached is not None and self.indice_key is not None
             _, outids, indice_pairs, indice_pair_num, out_spatial_shape = cached

@@ -50,6 +50,7 @@ class _SparsePool(nn.Module):
 
                 out._rows = PendingRows(pairs._n_out_dev, pairs.capacity, input if input.pending() else None, redo,
                                         lambda n: _ext._note_ratio(key, input.features.shape[0], n))
+                pairs.count = out._rows.count
                 out._rows.indices_ready = indices_ready
                 return out
         return self._forward_exact(input, out_shape)
