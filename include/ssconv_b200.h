@@ -164,6 +164,13 @@ int ssc_pairs_from_nbr(const int32_t *nbr, int K, int n_out, int n_in, int32_t *
 int ssc_materialize(const float *weight, const float *basis, const int32_t *block_table,
                     int n_blocks_in, const int32_t *out_field, const int32_t *in_field, int c_out,
                     int c_in, int K, float *filters, void *stream);
+/* Adjoint of ssc_materialize: d_weight (the layout of `weight`) from d_filters [K, c_in, c_out].
+ * out_start [n_out] / in_start [n_in]: first channel of every output / input field copy;
+ * max_pair: the largest (2 l_out + 1) (2 l_in + 1) among the blocks. */
+int ssc_materialize_bwd(const float *d_filters, const float *basis, const int32_t *block_table, int n_blocks_in,
+                        const int32_t *out_field, const int32_t *in_field, const int32_t *out_start, int n_out,
+                        const int32_t *in_start, int n_in, int max_pair, int c_out, int c_in, int K,
+                        float *d_weight, void *stream);
 
 /* Pack filters [K,Cin,Cout] fp32 into the tensor-core operand image used by ssc_conv_fwd
  * with precision SSC_PREC_TF32 (round-to-nearest TF32, K-major, 128-byte swizzled, padded) or
@@ -434,6 +441,28 @@ size_t ssc_bn_scratch_bytes(int n, int c);
 int ssc_bn_stats(const float *x, int n, int c, const int32_t *field_of_channel,
                  const int32_t *scalar_of_channel, int n_field, int n_scalar, float *mean,
                  float *var, void *scratch, size_t scratch_bytes, void *stream);
+/* The training-mode pass in one call (batchnorm.py:73-99): statistics as ssc_bn_stats, running values
+ * updated as running.mul_(1 - momentum).add_(momentum * batch) where the pointers are not NULL,
+ * chan_mean [c] = batch mean of scalar channels (0 elsewhere), and, where scale is not NULL, the
+ * per-channel affine (scale, shift) of the normalisation with the affine parameters folded in. */
+int ssc_bn_train(const float *x, int n, int c, const int32_t *field_of_channel, const int32_t *scalar_of_channel,
+                 int n_field, int n_scalar, const float *weight, const float *bias, float eps, double momentum,
+                 float *running_mean, float *running_var, float *mean, float *var, float *chan_mean, float *scale,
+                 float *shift, void *scratch, size_t scratch_bytes, void *stream);
+
+/* Backward of batch norm followed by the gated activation without biases (batchnorm.py:49-136,
+ * activation.py:55-100), as one pair of passes over x [n, c] (the batch norm's input) and gout
+ * [n, c_out] (gradient of the activation's output); the normalised rows and their gradient are
+ * recomputed, never stored.  scale / shift: the affine of the forward pass; chan_mean as in
+ * ssc_bn_train; training, var, weight, gx, d_weight, d_bias as in ssc_bn_bwd; the gate arguments as
+ * in ssc_gate_bwd, or gate_of_channel NULL and c_out = c for a batch norm alone.
+ * scratch: ssc_bn_scratch_bytes(n, c). */
+int ssc_bn_gate_bwd(const float *x, const float *gout, int n, int c, int c_out, const int32_t *field_of_channel,
+                    const int32_t *scalar_of_channel, int n_field, const float *scale, const float *shift,
+                    const float *chan_mean, const float *var, const float *weight, float eps, int training,
+                    const int32_t *gate_of_channel, const int32_t *field_start, const int32_t *field_len,
+                    int scalar_act, int gate_act, float *gx, float *d_weight, float *d_bias, void *scratch,
+                    size_t scratch_bytes, void *stream);
 
 /* Backward of the batch norm (what autograd derives from SS_Conv_lib/ss_conv/batchnorm.py:49-136):
  * y = (x - mean) * w / sqrt(var + eps) (+ bias for scalars).  training != 0: mean / var are the batch

@@ -258,109 +258,161 @@ static bool launch_bn_gate_rows(const float *x, int n, uint32_t groups, int c_in
   return true;
 }
 
-// Column sums, deterministic: block (32, 8) owns 32 channels and every gridDim.y-th group of 8
-// rows and writes its partial sums to part[blockIdx.y][channel]; colsum_finish adds the partials
-// of a bucket's channels in a fixed order (ascending channel, ascending row block), so the batch
-// statistics repeat bit for bit.  MODE 0: sum of x; 1: sum of (x - mean_ch)^2; 2: TWO sums for the
-// backward pass, of gy (part) and of gy * (x - mean_ch) (part2).
-template <int MODE>
-__global__ void bn_colsum_kernel(const float *__restrict__ x, const float *__restrict__ gy, int n, int c,
-                                 const float *__restrict__ chan_mean, float *__restrict__ part,
-                                 float *__restrict__ part2) {
-  __shared__ float sm[8][33], sm2[8][33];
-  const int ch = blockIdx.x * 32 + threadIdx.x;
-  float s = 0.f, s2 = 0.f;
-  if (ch < c) {
-    const float mu = (MODE != 0 && chan_mean) ? chan_mean[ch] : 0.f;
-    for (int r = blockIdx.y * 8 + threadIdx.y; r < n; r += 8 * gridDim.y) {
-      const float v = x[(size_t)r * c + ch] - mu;
-      if (MODE == 0) s += v;
-      else if (MODE == 1) s += v * v;
-      else {
-        const float g = gy[(size_t)r * c + ch];
-        s += g;
-        s2 += g * v;
+// ---------------------------------------------------------------- batch statistics, training mode
+// Column sums over the rows, deterministic: thread = (group of VEC channels, row lane), a block strides over
+// the rows, its lanes are added in shared memory in a fixed order and one partial row per block goes
+// to part[block][channel]; a second small kernel adds the partials of a field (block per field, fixed
+// tree).  HBM-bound: 16 bytes per thread and row, two blocks per SM.  MODE 0: sum of x;
+// 1: sum of (x - mean_ch)^2.
+constexpr int kStatThreads = 256;
+template <int MODE, int VEC>
+__global__ void __launch_bounds__(kStatThreads)
+bn_colsum_kernel(const float *__restrict__ x, int n, int c, int lanes, const float *__restrict__ chan_mean, float *__restrict__ part) {
+  __shared__ float sm[kStatThreads * VEC];
+  const int groups = c / VEC;
+  for (int g0 = 0; g0 < groups; g0 += kStatThreads / lanes) {   // one pass unless the row is wider than the block
+    const int gw = min(kStatThreads / lanes, groups - g0);
+    const int g = threadIdx.x % (kStatThreads / lanes), lane = threadIdx.x / (kStatThreads / lanes);
+    const bool on = g < gw && lane < lanes;
+    float s[VEC], mu[VEC];
+#pragma unroll
+    for (int q = 0; q < VEC; ++q) {
+      s[q] = 0.f;
+      mu[q] = (MODE != 0 && on) ? chan_mean[(g0 + g) * VEC + q] : 0.f;
+    }
+    if (on) {
+#pragma unroll 4
+      for (int r = blockIdx.x * lanes + lane; r < n; r += gridDim.x * lanes) {
+        const float *p = x + (size_t)r * c + (size_t)(g0 + g) * VEC;
+        float v[VEC];
+        if (VEC == 4) {
+          const float4 f = __ldg((const float4 *)p);
+          v[0] = f.x; v[1 % VEC] = f.y; v[2 % VEC] = f.z; v[3 % VEC] = f.w;
+        } else {
+          v[0] = __ldg(p);
+        }
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) {
+          const float d = v[q] - mu[q];
+          s[q] = MODE == 0 ? s[q] + d : fmaf(d, d, s[q]);
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < VEC; ++q) sm[threadIdx.x * VEC + q] = s[q];
+    __syncthreads();
+    if (lane == 0 && g < gw) {
+#pragma unroll
+      for (int q = 0; q < VEC; ++q) {
+        float a = s[q];
+        for (int l = 1; l < lanes; ++l) a += sm[(threadIdx.x + l * (kStatThreads / lanes)) * VEC + q];
+        part[(size_t)blockIdx.x * c + (g0 + g) * VEC + q] = a;
       }
     }
   }
-  sm[threadIdx.y][threadIdx.x] = s;
-  if (MODE == 2) sm2[threadIdx.y][threadIdx.x] = s2;
-  __syncthreads();
-  if (threadIdx.y == 0 && ch < c) {
-    for (int g = 1; g < 8; ++g) s += sm[g][threadIdx.x];
-    part[(size_t)blockIdx.y * c + ch] = s;
-    if (MODE == 2) {
-      for (int g = 1; g < 8; ++g) s2 += sm2[g][threadIdx.x];
-      part2[(size_t)blockIdx.y * c + ch] = s2;
-    }
-  }
 }
 
-// acc[b] = sum over the channels ch with bucket_of_channel[ch] == b (consecutive channels) and over
-// the row blocks of part[rb][ch]; one thread per bucket, fixed order.
-__global__ void colsum_finish_kernel(const float *__restrict__ part, int row_blocks, int c,
-                                     const int32_t *__restrict__ bucket_of_channel, int n_bucket, float *__restrict__ acc) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n_bucket) return;
+// Sum of a column of partials by one block, in a fixed order; every thread gets the result.
+constexpr int kFinishThreads = 128;
+__device__ __forceinline__ float column_total(const float *__restrict__ part, int n_part, int c, int ch) {
+  __shared__ float sm[kFinishThreads / 32];
   float s = 0.f;
-  for (int ch = 0; ch < c; ++ch) {
-    if (bucket_of_channel[ch] != b) continue;
-    for (int rb = 0; rb < row_blocks; ++rb) s += part[(size_t)rb * c + ch];
+  for (int i = threadIdx.x; i < n_part; i += kFinishThreads) s += part[(size_t)i * c + ch];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  __syncthreads();
+  s = sm[0];
+#pragma unroll
+  for (int w = 1; w < kFinishThreads / 32; ++w) s += sm[w];
+  return s;
+}
+
+// Block per channel: batch mean of the scalar channels (0 for the others), running mean updated with the
+// arithmetic of running.mul_(1 - m).add_(m * mean).
+__global__ void __launch_bounds__(kFinishThreads)
+bn_finish_mean_kernel(const float *__restrict__ part, int n_part, int n, int c, const int32_t *__restrict__ scalar_of_channel,
+                      float momentum, float keep, float *running_mean, float *mean, float *chan_mean) {
+  const int ch = blockIdx.x, s = scalar_of_channel[ch];
+  if (s < 0) {
+    if (threadIdx.x == 0) chan_mean[ch] = 0.f;
+    return;
   }
-  acc[b] = s;
-}
-
-// chan_mean[ch] = batch mean of a scalar channel (0 for l>0 channels), from the channel sums.
-__global__ void bn_chan_mean_kernel(const float *sum_scalar, int n, const int32_t *scalar_of_channel, int c,
-                                    float *chan_mean) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c) return;
-  int s = scalar_of_channel[i];
-  chan_mean[i] = s >= 0 ? sum_scalar[s] / (float)n : 0.f;
-}
-
-__global__ void bn_finish_var_kernel(float *var, int n_field, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n_field) var[i] = var[i] / (float)n;
-}
-
-// ------------------------------------------------------------------ backward of the batch norm
-// y = (x - mu) * r * w (+ b), r = (v + eps)^-1/2, v = mean over rows of the squared field norm.
-// With A_f = sum over rows and components of gy * (x - mu) and G_s = sum over rows of gy:
-//   d_w[f] = r A_f,  d_b[s] = G_s,
-//   training:  gx = r w gy - (w r^3 A_f / N) (x - mu) - [scalars] (r w G_s / N)
-//   eval:      gx = r w gy
-// Per channel: ks = r w, ka = w r^3 A / N (0 in eval mode), kg = r w G / N (scalars in training mode).
-__global__ void bn_bwd_coef_kernel(const float *__restrict__ A, const float *__restrict__ G, const float *__restrict__ var,
-                                   const float *__restrict__ weight, const int32_t *__restrict__ field_of_channel,
-                                   const int32_t *__restrict__ scalar_of_channel, int c, int n_field, int n, float eps,
-                                   int training, float *__restrict__ ks, float *__restrict__ ka, float *__restrict__ kg,
-                                   float *__restrict__ d_weight, float *__restrict__ d_bias, int n_scalar) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < c) {
-    const int f = field_of_channel[i], s = scalar_of_channel[i];
-    const float r = 1.0f / sqrtf(var[f] + eps), w = weight ? weight[f] : 1.f;
-    ks[i] = r * w;
-    ka[i] = training ? w * r * r * r * A[f] / (float)n : 0.f;
-    kg[i] = (training && s >= 0) ? r * w * G[s] / (float)n : 0.f;
+  const float mu = column_total(part, n_part, c, ch) / (float)n;
+  if (threadIdx.x == 0) {
+    chan_mean[ch] = mu;
+    mean[s] = mu;
+    if (running_mean) running_mean[s] = __fadd_rn(__fmul_rn(running_mean[s], keep), __fmul_rn(momentum, mu));
   }
-  if (i < n_field && d_weight) d_weight[i] = A[i] / sqrtf(var[i] + eps);
-  if (i < n_scalar && d_bias) d_bias[i] = G[i];
 }
 
-__global__ void bn_bwd_apply_kernel(const float *__restrict__ x, const float *__restrict__ gy, long long total, int c,
-                                    const float *__restrict__ chan_mean, const float *__restrict__ ks,
-                                    const float *__restrict__ ka, const float *__restrict__ kg, float *__restrict__ gx) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= total) return;
-  const int ch = (int)(t % c);
-  gx[t] = ks[ch] * gy[t] - ka[ch] * (x[t] - chan_mean[ch]) - kg[ch];
+// First channel and number of channels of a field (the channels of a field are consecutive).
+__device__ __forceinline__ int2 field_channels(const int32_t *__restrict__ field_of_channel, int c, int f) {
+  __shared__ int first, count;
+  if (threadIdx.x == 0) { first = c; count = 0; }
+  __syncthreads();
+  for (int ch = threadIdx.x; ch < c; ch += blockDim.x)
+    if (field_of_channel[ch] == f) { atomicMin(&first, ch); atomicAdd(&count, 1); }
+  __syncthreads();
+  return make_int2(first, count);
 }
 
-// ------------------------------------------------------------- backward of the gated activation
-// x [n, c_total] = [Rs channels | gate scalars], gy [n, c_out] -> gx [n, c_total].
-//   copy channel: gx = gy; scalar channel: gx = gy * act'(x); gated channel: gx = gy * act(gate);
-//   gate scalar j: gx = act'(x_gate) * sum over the channels ch of its field of gy[ch] * x[ch].
+// Block per field: mean squared norm, running value, and (scale != NULL) the per-channel affine of the pass.
+__global__ void __launch_bounds__(kFinishThreads)
+bn_finish_var_kernel(const float *__restrict__ part, int n_part, int n, int c, const int32_t *__restrict__ field_of_channel,
+                     const int32_t *__restrict__ scalar_of_channel, const float *__restrict__ chan_mean,
+                     const float *__restrict__ weight, const float *__restrict__ bias, float eps, float momentum, float keep,
+                     float *running_var, float *var, float *scale, float *shift) {
+  const int f = blockIdx.x;
+  const int2 fc = field_channels(field_of_channel, c, f);
+  float s = 0.f;
+  for (int k = 0; k < fc.y; ++k) s += column_total(part, n_part, c, fc.x + k);
+  const float v = s / (float)n;
+  if (threadIdx.x == 0) {
+    var[f] = v;
+    if (running_var) running_var[f] = __fadd_rn(__fmul_rn(running_var[f], keep), __fmul_rn(momentum, v));
+  }
+  if (scale && threadIdx.x < fc.y) {
+    const int ch = fc.x + threadIdx.x, sc_i = scalar_of_channel[ch];
+    float sc = 1.0f / sqrtf(v + eps), sh = 0.f;
+    if (weight) sc *= weight[f];
+    if (sc_i >= 0) {
+      sh = -chan_mean[ch] * sc;
+      if (bias) sh += bias[sc_i];
+    }
+    scale[ch] = sc;
+    shift[ch] = sh;
+  }
+}
+
+// ------------------------------------------- backward of batch norm and gated activation, one pair of passes
+// Forward of a row: y = x * scale + shift (batch norm), then out[ch] = y[ch] (copy), act(y[ch]) (scalars) or
+// y[ch] * act(y[gate of ch]).  Backward, with g = gradient of y from the gradient of out:
+//   copy: g = go;  scalar: g = go * act'(y);  gated: g = go * act(y_gate);
+//   gate scalar j: g = act'(y_gate) * sum over its field of go[ch] * y[ch],
+// and through y = (x - mu) * r * w (+ b), r = (v + eps)^-1/2, v = mean of the squared field norm:
+//   A_f = sum over rows and components of g * (x - mu),  G_s = sum over rows of g:
+//   d_w[f] = r A_f,  d_b[s] = G_s,  gx = ks g - ka (x - mu) - kg  with
+//   ks = r w, ka = w r^3 A / N, kg = r w G / N (ka = kg = 0 with running statistics).
+// y and g are recomputed from x and go in both passes (PASS 0 adds up A and G, PASS 1 writes gx), so neither
+// is ever stored: 2 reads of x and go and one write of gx per backward, instead of four tensors more.
+// A block takes R whole rows at a time into shared memory (rows are contiguous: a straight copy), evaluates
+// every gate once, then walks the channels.  Without a gate table g = go (batch norm alone); without ks
+// gx = g (activation alone).  HBM-bound.
+struct BnGateBwd {
+  const float *x, *go;
+  int n, c, c_out, n_gates, rows;              // rows = R
+  const float *scale, *shift, *mu;             // per channel (may be NULL: identity / zero)
+  const int32_t *gate_of_channel, *field_start, *field_len;
+  int s_act, g_act;
+  int vec;                                     // both row lengths and pointers allow 16-byte copies
+};
+
+constexpr int kBwdThreads = 256;
+constexpr int kBwdMaxAcc = 8;                  // channels of a thread: a block covers up to 2048
+
 __device__ __forceinline__ float act_grad(float v, int kind) {
   if (kind == 1) return v > 0.f ? 1.f : 0.f;
   if (kind == 2) {
@@ -370,29 +422,133 @@ __device__ __forceinline__ float act_grad(float v, int kind) {
   return 1.f;
 }
 
-__global__ void gate_bwd_kernel(const float *__restrict__ x, const float *__restrict__ gy, long long total, int c_total,
-                                int c_out, const int32_t *__restrict__ gate_of_channel,
-                                const int32_t *__restrict__ field_start, const int32_t *__restrict__ field_len,
-                                int scalar_act, int gate_act, float *__restrict__ gx) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= total) return;
-  const long long row = t / c_total;
-  const int ch = (int)(t - row * c_total);
-  const float *xr = x + row * c_total;
-  const float *gr = gy + row * c_out;
-  float v;
-  if (ch < c_out) {
-    const int g = gate_of_channel[ch];
-    if (g == -1) v = gr[ch] * act_grad(xr[ch], scalar_act);
-    else if (g >= 0) v = gr[ch] * apply_act(xr[c_out + g], gate_act);
-    else v = gr[ch];
-  } else {
-    const int j = ch - c_out, s0 = field_start[j], len = field_len[j];
-    float acc = 0.f;
-    for (int q = 0; q < len; ++q) acc += gr[s0 + q] * xr[s0 + q];
-    v = acc * act_grad(xr[ch], gate_act);
+template <int PASS>
+__global__ void __launch_bounds__(kBwdThreads)
+bn_gate_bwd_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
+                   float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
+  extern __shared__ __align__(16) float sm[];
+  float *xs = sm, *gs = xs + (size_t)p.rows * p.c, *as = gs + (size_t)p.rows * p.c_out, *gg = as + (size_t)p.rows * p.n_gates;
+  const int tid = threadIdx.x;
+  // channels over threads; rows of the tile over the lanes that are left when the row is short
+  const int lanes = p.c >= kBwdThreads ? 1 : kBwdThreads / p.c;
+  const int ch_step = p.c >= kBwdThreads ? kBwdThreads : p.c;
+  const int ch_block = (int)blockIdx.y * kBwdThreads * kBwdMaxAcc;     // (only rows of more than 2048 channels have a second one)
+  const int ch_first = ch_block + tid % ch_step, lane = tid / ch_step;
+  float sum_a[kBwdMaxAcc], sum_g[kBwdMaxAcc];
+#pragma unroll
+  for (int i = 0; i < kBwdMaxAcc; ++i) sum_a[i] = sum_g[i] = 0.f;
+  for (int r0 = blockIdx.x * p.rows; r0 < p.n; r0 += gridDim.x * p.rows) {
+    const int rows = min(p.rows, p.n - r0);
+    const float *xg = p.x + (size_t)r0 * p.c, *gg0 = p.go + (size_t)r0 * p.c_out;
+    if (p.vec) {
+      for (int i = tid; i < rows * p.c / 4; i += kBwdThreads) ((float4 *)xs)[i] = __ldg((const float4 *)xg + i);
+      for (int i = tid; i < rows * p.c_out / 4; i += kBwdThreads) ((float4 *)gs)[i] = __ldg((const float4 *)gg0 + i);
+    } else {
+      for (int i = tid; i < rows * p.c; i += kBwdThreads) xs[i] = __ldg(xg + i);
+      for (int i = tid; i < rows * p.c_out; i += kBwdThreads) gs[i] = __ldg(gg0 + i);
+    }
+    __syncthreads();
+    if (p.n_gates > 0) {
+      for (int i = tid; i < rows * p.n_gates; i += kBwdThreads) {
+        const int r = i / p.n_gates, j = i - r * p.n_gates;
+        const float *xr = xs + r * p.c, *gr = gs + r * p.c_out;
+        const int cg = p.c_out + j;
+        float v = xr[cg];
+        if (p.scale) v = fmaf(v, p.scale[cg], p.shift[cg]);
+        const int s0 = p.field_start[j], len = p.field_len[j];
+        float acc = 0.f;
+        for (int q = 0; q < len; ++q) {
+          float y = xr[s0 + q];
+          if (p.scale) y = fmaf(y, p.scale[s0 + q], p.shift[s0 + q]);
+          acc += gr[s0 + q] * y;
+        }
+        as[i] = apply_act(v, p.g_act);
+        gg[i] = acc * act_grad(v, p.g_act);
+      }
+      __syncthreads();
+    }
+    if (lane < lanes) {
+#pragma unroll
+      for (int i = 0; i < kBwdMaxAcc; ++i) {
+        const int ch = ch_first + i * ch_step;
+        if (ch >= p.c || (i > 0 && p.c < kBwdThreads)) break;
+        const float mu = p.mu ? p.mu[ch] : 0.f;
+        const float sc = p.scale ? p.scale[ch] : 1.f, sh = p.scale ? p.shift[ch] : 0.f;
+        const int gate = p.gate_of_channel ? (ch < p.c_out ? p.gate_of_channel[ch] : -3) : -2;
+        const float k_s = (PASS == 1 && ks) ? ks[ch] : 1.f, k_a = (PASS == 1 && ks) ? ka[ch] : 0.f, k_g = (PASS == 1 && ks) ? kg[ch] : 0.f;
+        for (int r = lane; r < rows; r += lanes) {
+          const float x = xs[r * p.c + ch];
+          float g;
+          if (gate == -3) g = gg[r * p.n_gates + ch - p.c_out];
+          else {
+            g = gs[r * p.c_out + ch];
+            if (gate == -1) g *= act_grad(p.scale ? fmaf(x, sc, sh) : x, p.s_act);
+            else if (gate >= 0) g *= as[r * p.n_gates + gate];
+          }
+          if (PASS == 0) {
+            sum_g[i] += g;
+            sum_a[i] = fmaf(g, x - mu, sum_a[i]);
+          } else {
+            gx[(size_t)(r0 + r) * p.c + ch] = ks ? k_s * g - k_a * (x - mu) - k_g : g;
+          }
+        }
+      }
+    }
+    __syncthreads();
   }
-  gx[t] = v;
+  if (PASS == 0) {
+    // lanes of a channel are added in a fixed order (the tile's shared memory is free now)
+    for (int i = 0; i < kBwdMaxAcc; ++i) {
+      const int ch = ch_first + i * ch_step;
+      if (i > 0 && p.c < kBwdThreads) break;
+      if (ch_block + i * ch_step >= p.c) break;
+      sm[tid] = sum_a[i];
+      sm[kBwdThreads + tid] = sum_g[i];
+      __syncthreads();
+      if (lane == 0 && ch < p.c) {
+        float a = sum_a[i], g = sum_g[i];
+        for (int l = 1; l < lanes; ++l) { a += sm[tid + l * ch_step]; g += sm[kBwdThreads + tid + l * ch_step]; }
+        part_a[(size_t)blockIdx.x * p.c + ch] = a;
+        part_g[(size_t)blockIdx.x * p.c + ch] = g;
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// Block per field: A and G from the partials, the field's coefficients and parameter gradients.
+__global__ void __launch_bounds__(kFinishThreads)
+bn_bwd_finish_kernel(const float *__restrict__ part_a, const float *__restrict__ part_g, int n_part, int n, int c,
+                     const int32_t *__restrict__ field_of_channel, const int32_t *__restrict__ scalar_of_channel,
+                     const float *__restrict__ var, const float *__restrict__ weight, float eps, int training,
+                     float *__restrict__ ks, float *__restrict__ ka, float *__restrict__ kg, float *__restrict__ d_weight,
+                     float *__restrict__ d_bias) {
+  const int f = blockIdx.x;
+  const int2 fc = field_channels(field_of_channel, c, f);
+  float A = 0.f;
+  for (int k = 0; k < fc.y; ++k) A += column_total(part_a, n_part, c, fc.x + k);
+  const int s = fc.y == 1 ? scalar_of_channel[fc.x] : -1;
+  float G = 0.f;
+  if (s >= 0) G = column_total(part_g, n_part, c, fc.x);
+  const float r = 1.0f / sqrtf(var[f] + eps), w = weight ? weight[f] : 1.f;
+  if (threadIdx.x < fc.y) {
+    const int ch = fc.x + threadIdx.x;
+    ks[ch] = r * w;
+    ka[ch] = training ? w * r * r * r * A / (float)n : 0.f;
+    kg[ch] = (training && s >= 0) ? r * w * G / (float)n : 0.f;
+  }
+  if (threadIdx.x == 0) {
+    if (d_weight) d_weight[f] = A / sqrtf(var[f] + eps);
+    if (s >= 0 && d_bias) d_bias[s] = G;
+  }
+}
+
+// chan_mean[ch] = mean of a scalar channel (0 for l>0 channels).
+__global__ void bn_chan_mean_kernel(const float *mean, const int32_t *scalar_of_channel, int c, float *chan_mean) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= c) return;
+  const int s = scalar_of_channel[i];
+  chan_mean[i] = s >= 0 ? mean[s] : 0.f;
 }
 
 }  // namespace ssc
@@ -483,16 +639,54 @@ extern "C" int ssc_bn_gate_fwd16(const float *x, int n, int c_in_total, const fl
   return SSC_OK;
 }
 
-// Row blocks of the column-sum kernels (each contributes one partial per channel).
+// Blocks of the column-sum and backward kernels, each of which contributes one partial per channel:
+// four per SM, fewer when a block would not have a hundred rows to add.
 static int bn_row_blocks(int n) {
-  int rb = ceil_div(n, 8 * 64);
-  return rb > 64 ? 64 : (rb < 1 ? 1 : rb);
+  const int rb = ceil_div(n, 64), most = 4 * 148;
+  return rb > most ? most : (rb < 1 ? 1 : rb);
 }
 
 extern "C" size_t ssc_bn_scratch_bytes(int n, int c) {
   if (n < 0 || c < 1) return 0;
-  // two partial-sum planes [row_blocks, c], per-channel mean and three coefficient rows, two bucket rows
-  return ((size_t)2 * bn_row_blocks(n) * c + (size_t)6 * c + 64) * sizeof(float);
+  // two planes of partials [row blocks, c], per-channel mean and three coefficient rows
+  return ((size_t)2 * bn_row_blocks(n) * c + (size_t)4 * c + 64) * sizeof(float);
+}
+
+static int launch_colsum(int mode, const float *x, int n, int c, const float *chan_mean, float *part, int blocks, cudaStream_t st) {
+  const bool vec = (c & 3) == 0 && ((uintptr_t)x & 15u) == 0;
+  const int groups = vec ? c / 4 : c;
+  const int lanes = groups >= kStatThreads ? 1 : kStatThreads / groups;
+  if (vec) {
+    if (mode == 0) bn_colsum_kernel<0, 4><<<blocks, kStatThreads, 0, st>>>(x, n, c, lanes, chan_mean, part);
+    else bn_colsum_kernel<1, 4><<<blocks, kStatThreads, 0, st>>>(x, n, c, lanes, chan_mean, part);
+  } else {
+    if (mode == 0) bn_colsum_kernel<0, 1><<<blocks, kStatThreads, 0, st>>>(x, n, c, lanes, chan_mean, part);
+    else bn_colsum_kernel<1, 1><<<blocks, kStatThreads, 0, st>>>(x, n, c, lanes, chan_mean, part);
+  }
+  note_launches(1);
+  SSC_CHECK_LAUNCH("bn_colsum");
+  return SSC_OK;
+}
+
+extern "C" int ssc_bn_train(const float *x, int n, int c, const int32_t *field_of_channel, const int32_t *scalar_of_channel,
+                            int n_field, int n_scalar, const float *weight, const float *bias, float eps, double momentum,
+                            float *running_mean, float *running_var, float *mean, float *var, float *chan_mean,
+                            float *scale, float *shift, void *scratch, size_t scratch_bytes, void *stream) {
+  SSC_REQUIRE(n >= 1 && c >= 1 && n_field >= 1 && n_scalar >= 0, "bn_train: bad sizes");
+  SSC_REQUIRE(x && field_of_channel && scalar_of_channel && mean && var && chan_mean, "bn_train: null pointer");
+  SSC_REQUIRE((scale == nullptr) == (shift == nullptr), "bn_train: scale and shift go together");
+  SSC_REQUIRE(scratch && scratch_bytes >= ssc_bn_scratch_bytes(n, c), "bn_train: scratch too small (ssc_bn_scratch_bytes)");
+  cudaStream_t st = as_stream(stream);
+  float *part = (float *)scratch;
+  const int rb = bn_row_blocks(n);
+  const float m = (float)momentum, keep = (float)(1.0 - momentum);
+  if (int e = launch_colsum(0, x, n, c, nullptr, part, rb, st)) return e;
+  { bn_finish_mean_kernel<<<c, kFinishThreads, 0, st>>>(part, rb, n, c, scalar_of_channel, m, keep, running_mean, mean, chan_mean); note_launches(1); }
+  if (int e = launch_colsum(1, x, n, c, chan_mean, part, rb, st)) return e;
+  { bn_finish_var_kernel<<<n_field, kFinishThreads, 0, st>>>(part, rb, n, c, field_of_channel, scalar_of_channel, chan_mean, weight, bias,
+                                                           eps, m, keep, running_var, var, scale, shift); note_launches(1); }
+  SSC_CHECK_LAUNCH("bn_train");
+  return SSC_OK;
 }
 
 // var must have room for n_field + c floats (the tail holds the per-channel means); scratch holds the
@@ -500,23 +694,58 @@ extern "C" size_t ssc_bn_scratch_bytes(int n, int c) {
 extern "C" int ssc_bn_stats(const float *x, int n, int c, const int32_t *field_of_channel,
                             const int32_t *scalar_of_channel, int n_field, int n_scalar, float *mean, float *var,
                             void *scratch, size_t scratch_bytes, void *stream) {
-  SSC_REQUIRE(n >= 1 && c >= 1 && n_field >= 1 && n_scalar >= 0, "bn_stats: bad sizes");
-  SSC_REQUIRE(x && field_of_channel && scalar_of_channel && mean && var, "bn_stats: null pointer");
-  SSC_REQUIRE(scratch && scratch_bytes >= ssc_bn_scratch_bytes(n, c), "bn_stats: scratch too small (ssc_bn_scratch_bytes)");
-  cudaStream_t st = as_stream(stream);
-  float *chan_mean = var + n_field;  // scratch tail, c floats
-  float *part = (float *)scratch;
-  const int rb = bn_row_blocks(n);
-  dim3 block(32, 8), grid(ceil_div(c, 32), rb);
-  { bn_colsum_kernel<0><<<grid, block, 0, st>>>(x, nullptr, n, c, nullptr, part, nullptr); note_launches(1); }
-  if (n_scalar > 0) { colsum_finish_kernel<<<ceil_div(n_scalar, 64), 64, 0, st>>>(part, rb, c, scalar_of_channel, n_scalar, mean); note_launches(1); }
-  { bn_chan_mean_kernel<<<ceil_div(c, 128), 128, 0, st>>>(mean, n, scalar_of_channel, c, chan_mean); note_launches(1); }
-  if (n_scalar > 0) { bn_finish_var_kernel<<<ceil_div(n_scalar, 128), 128, 0, st>>>(mean, n_scalar, n); note_launches(1); }
-  { bn_colsum_kernel<1><<<grid, block, 0, st>>>(x, nullptr, n, c, chan_mean, part, nullptr); note_launches(1); }
-  { colsum_finish_kernel<<<ceil_div(n_field, 64), 64, 0, st>>>(part, rb, c, field_of_channel, n_field, var); note_launches(1); }
-  { bn_finish_var_kernel<<<ceil_div(n_field, 128), 128, 0, st>>>(var, n_field, n); note_launches(1); }
-  SSC_CHECK_LAUNCH("bn_stats");
+  SSC_REQUIRE(var, "bn_stats: null pointer");
+  return ssc_bn_train(x, n, c, field_of_channel, scalar_of_channel, n_field, n_scalar, nullptr, nullptr, 0.f, 0.0, nullptr, nullptr,
+                      mean, var, var + n_field, nullptr, nullptr, scratch, scratch_bytes, stream);
+}
+
+// Rows per tile of the backward kernels: as many as 32 KB of shared memory hold (up to seven blocks per SM).
+static int bwd_tile_rows(int c, int c_out, int n_gates, size_t *smem) {
+  const size_t per_row = (size_t)(c + c_out + 2 * n_gates) * sizeof(float);
+  int rows = (int)(32 * 1024 / per_row);
+  rows = rows >= 8 ? (rows & ~3) : (rows < 1 ? 1 : rows);     // multiples of four keep the copies 16-byte aligned
+  if (rows > 64) rows = 64;
+  *smem = rows * per_row;
+  if (*smem < 2 * kBwdThreads * sizeof(float)) *smem = 2 * kBwdThreads * sizeof(float);
+  return rows;
+}
+
+template <int PASS>
+static int launch_bwd(BnGateBwd p, const float *ks, const float *ka, const float *kg, float *gx, float *part_a, float *part_g, int blocks,
+                      cudaStream_t st) {
+  size_t smem;
+  p.rows = bwd_tile_rows(p.c, p.c_out, p.n_gates, &smem);
+  p.vec = (p.c & 3) == 0 && (p.c_out & 3) == 0 && (((uintptr_t)p.x | (uintptr_t)p.go) & 15u) == 0 && p.rows * (size_t)p.c % 4 == 0;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(bn_gate_bwd_kernel<PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "bn_gate_bwd: smem attribute: %s", cudaGetErrorString(e));
+  }
+  { bn_gate_bwd_kernel<PASS><<<dim3(blocks, ceil_div(p.c, kBwdThreads * kBwdMaxAcc)), kBwdThreads, smem, st>>>(p, ks, ka, kg, gx, part_a, part_g); note_launches(1); }
+  SSC_CHECK_LAUNCH("bn_gate_bwd");
   return SSC_OK;
+}
+
+extern "C" int ssc_bn_gate_bwd(const float *x, const float *gout, int n, int c, int c_out, const int32_t *field_of_channel,
+                               const int32_t *scalar_of_channel, int n_field, const float *scale, const float *shift,
+                               const float *chan_mean, const float *var, const float *weight, float eps, int training,
+                               const int32_t *gate_of_channel, const int32_t *field_start, const int32_t *field_len,
+                               int scalar_act, int gate_act, float *gx, float *d_weight, float *d_bias, void *scratch,
+                               size_t scratch_bytes, void *stream) {
+  SSC_REQUIRE(n >= 1 && c >= 1 && c_out >= 1 && c_out <= c && n_field >= 1, "bn_gate_bwd: bad sizes");
+  SSC_REQUIRE(x && gout && field_of_channel && scalar_of_channel && chan_mean && var && gx, "bn_gate_bwd: null pointer");
+  SSC_REQUIRE(gate_of_channel ? (scale && shift && (c == c_out || (field_start && field_len))) : c == c_out, "bn_gate_bwd: gate tables do not fit the channels");
+  SSC_REQUIRE(scratch && scratch_bytes >= ssc_bn_scratch_bytes(n, c), "bn_gate_bwd: scratch too small (ssc_bn_scratch_bytes)");
+  cudaStream_t st = as_stream(stream);
+  const int rb = bn_row_blocks(n);
+  float *part_a = (float *)scratch, *part_g = part_a + (size_t)rb * c;
+  float *ks = part_g + (size_t)rb * c, *ka = ks + c, *kg = ka + c;
+  BnGateBwd p = {x, gout, n, c, c_out, gate_of_channel ? c - c_out : 0, 0, scale, shift, chan_mean, gate_of_channel, field_start, field_len,
+                 scalar_act, gate_act, 0};
+  if (int e = launch_bwd<0>(p, nullptr, nullptr, nullptr, nullptr, part_a, part_g, rb, st)) return e;
+  { bn_bwd_finish_kernel<<<n_field, kFinishThreads, 0, st>>>(part_a, part_g, rb, n, c, field_of_channel, scalar_of_channel, var, weight, eps,
+                                                           training, ks, ka, kg, d_weight, d_bias); note_launches(1); }
+  SSC_CHECK_LAUNCH("bn_bwd_finish");
+  return launch_bwd<1>(p, ks, ka, kg, gx, nullptr, nullptr, rb, st);
 }
 
 extern "C" int ssc_bn_bwd(const float *x, const float *gy, int n, int c, const int32_t *field_of_channel,
@@ -524,25 +753,13 @@ extern "C" int ssc_bn_bwd(const float *x, const float *gy, int n, int c, const i
                           const float *var, const float *weight, float eps, int training, float *gx,
                           float *d_weight, float *d_bias, void *scratch, size_t scratch_bytes, void *stream) {
   SSC_REQUIRE(n >= 1 && c >= 1 && n_field >= 1 && n_scalar >= 0, "bn_bwd: bad sizes");
-  SSC_REQUIRE(x && gy && field_of_channel && scalar_of_channel && var && gx && (n_scalar == 0 || mean), "bn_bwd: null pointer");
-  SSC_REQUIRE(scratch && scratch_bytes >= ssc_bn_scratch_bytes(n, c), "bn_bwd: scratch too small (ssc_bn_scratch_bytes)");
-  cudaStream_t st = as_stream(stream);
-  const int rb = bn_row_blocks(n);
-  float *part = (float *)scratch, *part2 = part + (size_t)rb * c;
-  float *chan_mean = part2 + (size_t)rb * c, *ks = chan_mean + c, *ka = ks + c, *kg = ka + c;
-  float *A = kg + c, *G = A + c;     // per field / per scalar (at most c entries each)
-  { bn_chan_mean_kernel<<<ceil_div(c, 128), 128, 0, st>>>(mean, 1, scalar_of_channel, c, chan_mean); note_launches(1); }   // mean itself (n = 1)
-  dim3 block(32, 8), grid(ceil_div(c, 32), rb);
-  { bn_colsum_kernel<2><<<grid, block, 0, st>>>(x, gy, n, c, chan_mean, part, part2); note_launches(1); }
-  if (n_scalar > 0) { colsum_finish_kernel<<<ceil_div(n_scalar, 64), 64, 0, st>>>(part, rb, c, scalar_of_channel, n_scalar, G); note_launches(1); }
-  { colsum_finish_kernel<<<ceil_div(n_field, 64), 64, 0, st>>>(part2, rb, c, field_of_channel, n_field, A); note_launches(1); }
-  const int m = c > n_field ? c : n_field;
-  { bn_bwd_coef_kernel<<<ceil_div(m, 128), 128, 0, st>>>(A, G, var, weight, field_of_channel, scalar_of_channel, c, n_field, n, eps,
-                                                     training, ks, ka, kg, d_weight, d_bias, n_scalar); note_launches(1); }
-  const long long total = (long long)n * c;
-  { bn_bwd_apply_kernel<<<ceil_div(total, 256), 256, 0, st>>>(x, gy, total, c, chan_mean, ks, ka, kg, gx); note_launches(1); }
-  SSC_CHECK_LAUNCH("bn_bwd");
-  return SSC_OK;
+  SSC_REQUIRE(n_scalar == 0 || mean, "bn_bwd: null pointer");
+  SSC_REQUIRE(scalar_of_channel && scratch && scratch_bytes >= ssc_bn_scratch_bytes(n, c), "bn_bwd: scratch too small (ssc_bn_scratch_bytes)");
+  float *chan_mean = (float *)scratch + (size_t)2 * bn_row_blocks(n) * c + (size_t)3 * c;
+  { bn_chan_mean_kernel<<<ceil_div(c, 128), 128, 0, as_stream(stream)>>>(mean, scalar_of_channel, c, chan_mean); note_launches(1); }
+  SSC_CHECK_LAUNCH("bn_chan_mean");
+  return ssc_bn_gate_bwd(x, gy, n, c, c, field_of_channel, scalar_of_channel, n_field, nullptr, nullptr, chan_mean, var, weight, eps, training,
+                         nullptr, nullptr, nullptr, 0, 0, gx, d_weight, d_bias, scratch, scratch_bytes, stream);
 }
 
 extern "C" int ssc_gate_bwd(const float *x, const float *gy, int n, int c_total, int c_out,
@@ -551,9 +768,7 @@ extern "C" int ssc_gate_bwd(const float *x, const float *gy, int n, int c_total,
   SSC_REQUIRE(n >= 0 && c_total >= 1 && c_out >= 1 && c_out <= c_total, "gate_bwd: bad sizes");
   if (n == 0) return SSC_OK;
   SSC_REQUIRE(x && gy && gx && gate_of_channel && (c_total == c_out || (field_start && field_len)), "gate_bwd: null pointer");
-  const long long total = (long long)n * c_total;
-  { gate_bwd_kernel<<<ceil_div(total, 256), 256, 0, as_stream(stream)>>>(x, gy, total, c_total, c_out, gate_of_channel, field_start,
-                                                                      field_len, scalar_act, gate_act, gx); note_launches(1); }
-  SSC_CHECK_LAUNCH("gate_bwd");
-  return SSC_OK;
+  BnGateBwd p = {x, gy, n, c_total, c_out, c_total - c_out, 0, nullptr, nullptr, nullptr, gate_of_channel, field_start, field_len,
+                 scalar_act, gate_act, 0};
+  return launch_bwd<1>(p, nullptr, nullptr, nullptr, gx, nullptr, nullptr, bn_row_blocks(n), as_stream(stream));
 }

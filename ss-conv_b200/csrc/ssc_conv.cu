@@ -33,6 +33,51 @@ __global__ void materialize_kernel(const float *__restrict__ weight, const float
   filters[t] = acc;
 }
 
+// Adjoint: d_w[u,v,b] = sum over a, c, kappa of d_filters[kappa][cin][cout] * basis[b,a,c,kappa].  One block per
+// (output field copy, input field copy): its d_filters entries (at most 49 K for orders up to 3) go to
+// shared memory in the basis' own order, read in runs along cout, then every basis element is one
+// coalesced dot product; eight warps share the basis elements.  One launch of a few microseconds per layer:
+// as one small library contraction per pair of orders it was 20 launches and 1 ms of host time.
+constexpr int kMatBwdThreads = 256;
+__global__ void __launch_bounds__(kMatBwdThreads)
+materialize_bwd_kernel(const float *__restrict__ g, const float *__restrict__ basis, const int32_t *__restrict__ block_table,
+                       int n_blocks_in, const int32_t *__restrict__ out_field, const int32_t *__restrict__ in_field,
+                       const int32_t *__restrict__ out_start, const int32_t *__restrict__ in_start, int c_out, int c_in, int K,
+                       int staged, float *__restrict__ d_weight) {
+  extern __shared__ float gs[];
+  const int co0 = out_start[blockIdx.y], ci0 = in_start[blockIdx.x];
+  const int i = out_field[co0 * 3], u = out_field[co0 * 3 + 1], j = in_field[ci0 * 3], v = in_field[ci0 * 3 + 1];
+  const int32_t *blk = block_table + (size_t)(i * n_blocks_in + j) * 6;
+  const int boff = blk[0];
+  if (boff < 0) return;
+  const int nb = blk[2], m_in = blk[3], d_out = blk[4], d_in = blk[5], total = d_out * d_in * K;
+  if (staged) {
+#pragma unroll 4
+    for (int t = threadIdx.x; t < total; t += kMatBwdThreads) {      // a fastest: runs of d_out floats
+      const int a = t % d_out, r = t / d_out, kappa = r % K, c = r / K;
+      gs[(a * d_in + c) * K + kappa] = __ldg(g + ((size_t)kappa * c_in + ci0 + c) * c_out + co0 + a);
+    }
+    __syncthreads();
+  }
+  float *dw = d_weight + blk[1] + (size_t)(u * m_in + v) * nb;
+  for (int b = threadIdx.x >> 5; b < nb; b += kMatBwdThreads / 32) {
+    const float *bp = basis + boff + (size_t)b * total;
+    float s = 0.f;
+    if (staged) {
+#pragma unroll 8
+      for (int t = threadIdx.x & 31; t < total; t += 32) s = fmaf(gs[t], __ldg(bp + t), s);
+    } else {
+      for (int t = threadIdx.x & 31; t < total; t += 32) {
+        const int kappa = t % K, r = t / K, c = r % d_in, a = r / d_in;
+        s = fmaf(__ldg(g + ((size_t)kappa * c_in + ci0 + c) * c_out + co0 + a), __ldg(bp + t), s);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) dw[b] = s;
+  }
+}
+
 // ---------------------------------------------------------------------------------------
 // Exact fp32 path: tile of 64 output rows x 64 output channels per block, 256 threads with a
 // 4x4 register tile each, reduction over (kernel offset, input channel) in chunks of 16.
@@ -131,6 +176,25 @@ extern "C" int ssc_materialize(const float *weight, const float *basis, const in
   { materialize_kernel<<<ceil_div(total, 256), 256, 0, as_stream(stream)>>>(weight, basis, block_table, n_blocks_in,
                                                                          out_field, in_field, c_out, c_in, K, filters); note_launches(1); }
   SSC_CHECK_LAUNCH("materialize");
+  return SSC_OK;
+}
+
+extern "C" int ssc_materialize_bwd(const float *d_filters, const float *basis, const int32_t *block_table, int n_blocks_in,
+                                   const int32_t *out_field, const int32_t *in_field, const int32_t *out_start, int n_out,
+                                   const int32_t *in_start, int n_in, int max_pair, int c_out, int c_in, int K,
+                                   float *d_weight, void *stream) {
+  SSC_REQUIRE(c_out > 0 && c_in > 0 && K > 0 && n_blocks_in > 0 && n_out > 0 && n_in > 0 && n_out <= 65535 && max_pair > 0, "materialize_bwd: bad sizes");
+  SSC_REQUIRE(d_filters && basis && block_table && out_field && in_field && out_start && in_start && d_weight, "materialize_bwd: null pointer");
+  // a field pair that does not fit shared memory (very high orders with large kernels) is read in place
+  const size_t need = (size_t)K * max_pair * sizeof(float);
+  const int staged = need <= 200 * 1024 ? 1 : 0;
+  if (staged && need > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(materialize_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+    if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "materialize_bwd: smem attribute: %s", cudaGetErrorString(e));
+  }
+  { materialize_bwd_kernel<<<dim3(n_in, n_out), kMatBwdThreads, staged ? need : 0, as_stream(stream)>>>(
+        d_filters, basis, block_table, n_blocks_in, out_field, in_field, out_start, in_start, c_out, c_in, K, staged, d_weight); note_launches(1); }
+  SSC_CHECK_LAUNCH("materialize_bwd");
   return SSC_OK;
 }
 

@@ -48,6 +48,8 @@ SIGNATURES = {
     "ssc_pairs_from_nbr": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "ssc_materialize": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                                 c_void_p, c_void_p]),
+    "ssc_materialize_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
+                                    c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "ssc_conv_packed_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "ssc_conv_pack_filters": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "ssc_conv_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
@@ -103,6 +105,12 @@ SIGNATURES = {
     "ssc_bn_scratch_bytes": (c_size_t, [c_int, c_int]),
     "ssc_bn_stats": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
                              c_size_t, c_void_p]),
+    "ssc_bn_train": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_float,
+                             ctypes.c_double, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                             c_size_t, c_void_p]),
+    "ssc_bn_gate_bwd": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                c_void_p, c_void_p, c_float, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p,
+                                c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "ssc_bn_bwd": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
                            c_void_p, c_float, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "ssc_gate_bwd": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
@@ -563,6 +571,16 @@ def materialize(weight, basis, block_table, n_blocks_in, out_field, in_field, c_
     return flt
 
 
+def materialize_backward(d_filters, basis, block_table, n_blocks_in, out_field, in_field, out_start, in_start, max_pair, c_out,
+                         c_in, K, n_weight):
+    d_w = torch.empty(n_weight, dtype=torch.float32, device=d_filters.device)
+    _check(lib().ssc_materialize_bwd(_p(d_filters, torch.float32), _p(basis, torch.float32), _p(block_table, torch.int32),
+                                     int(n_blocks_in), _p(out_field, torch.int32), _p(in_field, torch.int32),
+                                     _p(out_start, torch.int32), out_start.numel(), _p(in_start, torch.int32),
+                                     in_start.numel(), int(max_pair), int(c_out), int(c_in), int(K), _p(d_w), _stream()))
+    return d_w
+
+
 def pack_filters(filters_kio, prec=PREC_TF32):
     """Tensor-core operand image (TF32 or fp16) of contiguous filters [K, Cin, Cout]."""
     K, c_in, c_out = filters_kio.shape
@@ -907,14 +925,17 @@ def conv_wgrad(features, out_grad, nbr, precision=None):
     return d_flt
 
 
-def conv_backward(features, flt, out_bp, nbr, nbr_in=None, order=None, precision=None):
+def conv_backward(features, flt, out_bp, nbr, nbr_in=None, order=None, precision=None, need=(True, True)):
     """(input gradient [n_in, Cin], filter gradient [K, Cin, Cout]) of out = conv(features, flt [K, Cin, Cout])
     over the table nbr [K, n_out].  nbr_in / order: the input-major table and its row order when the
-    caller kept them with the rulebook (built here otherwise)."""
+    caller kept them with the rulebook (built here otherwise).  need: which of the two are asked for (a
+    first layer's input needs none); None is returned for the other."""
     n_in = features.shape[0]
+    if not need[0]:
+        return None, conv_wgrad(features, out_bp, nbr, precision) if need[1] else None
     # the two gradients do not depend on each other: while a graph is recorded the filter gradient
     # goes to a side stream, so the graph runs it next to the input gradient
-    forked = torch.cuda.is_current_stream_capturing()
+    forked = need[1] and torch.cuda.is_current_stream_capturing()
     if forked:
         cur, side = torch.cuda.current_stream(features.device), side_stream(features.device)
         side.wait_stream(cur)
@@ -929,7 +950,7 @@ def conv_backward(features, flt, out_bp, nbr, nbr_in=None, order=None, precision
             # rows of the input-major table use few of the offsets each (their parity class under a
             # stride): grouped tiles skip the rest
             order = nbr_row_order(nbr_in) if (n_in >= ROW_ORDER_MIN_ROWS and nbr_in.shape[0] > 1) else None
-            if not forked:                             # tensors made while a graph is recorded belong to the graph
+            if not torch.cuda.is_current_stream_capturing():   # tensors made while a graph is recorded belong to the graph
                 try:
                     nbr._ssc_in_major = (n_in, nbr_in, order)
                 except Exception:
@@ -938,11 +959,11 @@ def conv_backward(features, flt, out_bp, nbr, nbr_in=None, order=None, precision
     if forked:
         cur.wait_stream(side)
     else:
-        d_flt = conv_wgrad(features, out_bp, nbr, precision)
+        d_flt = conv_wgrad(features, out_bp, nbr, precision) if need[1] else None
     return d_in, d_flt
 
 
-def indice_conv_backward_fp32(features, filters, out_bp, indice_pairs, indice_num, inverse, subm):
+def indice_conv_backward_fp32(features, filters, out_bp, indice_pairs, indice_num, inverse, subm, need=(True, True)):
     """Reference signature (SS_Conv_lib/src/ss_conv_ops.h:46-48): [input_grad, filters_grad].
     The input gradient is the forward gather-GEMM over the input-major table with the filters
     transposed; both gradients use the operand precision set for the forward pass.  The
@@ -954,8 +975,8 @@ def indice_conv_backward_fp32(features, filters, out_bp, indice_pairs, indice_nu
     flt = filters.reshape(-1, c_in, c_out)
     n_in, n_out = features.shape[0], out_bp.shape[0]
     nbr = neighbour_table(indice_pairs, indice_num, n_out, bool(inverse))
-    d_in, d_flt = conv_backward(features, flt, out_bp, nbr)
-    return [d_in, d_flt.reshape(filters.shape)]
+    d_in, d_flt = conv_backward(features, flt, out_bp, nbr, need=need)
+    return [d_in, None if d_flt is None else d_flt.reshape(filters.shape)]
 
 
 def indice_conv_half(features, filters, indice_pairs, indice_num, num_act_out, inverse, subm):
@@ -972,7 +993,7 @@ def indice_conv_half(features, filters, indice_pairs, indice_num, num_act_out, i
     return out.half()
 
 
-def indice_conv_backward_half(features, filters, out_bp, indice_pairs, indice_num, inverse, subm):
+def indice_conv_backward_half(features, filters, out_bp, indice_pairs, indice_num, inverse, subm, need=(True, True)):
     """Reference signature (SS_Conv_lib/src/ss_conv_ops.h:52-54): [input_grad, filters_grad] in half.
     The input gradient runs on fp16 operands, the filter gradient on TF32 operands (the same
     significand, fp32 range), both with fp32 accumulation."""
@@ -1214,16 +1235,45 @@ def bn_gate_forward(x, scale, shift, gate_of_channel, c_out, c_gate_base, scalar
     return out
 
 
-def bn_stats(x, field_of_channel, scalar_of_channel, n_field, n_scalar):
+def bn_train(x, field_of_channel, scalar_of_channel, n_field, n_scalar, weight, bias, eps, momentum, running_mean=None,
+             running_var=None):
+    """(mean [n_scalar], var [n_field], chan_mean [c], scale [c], shift [c]) of a training-mode batch norm;
+    the running values (updated in place where given) take the arithmetic of
+    running.mul_(1 - momentum).add_(momentum * batch)."""
     x = x.contiguous()
-    mean = torch.empty(max(n_scalar, 1), dtype=torch.float32, device=x.device)
-    var = torch.empty(n_field + x.shape[1], dtype=torch.float32, device=x.device)
-    nbytes = int(lib().ssc_bn_scratch_bytes(x.shape[0], x.shape[1]))
+    n, c = x.shape
+    flat = torch.empty(n_scalar + n_field + 3 * c, dtype=torch.float32, device=x.device)
+    scale, shift, chan_mean, mean, var = flat.split([c, c, c, n_scalar, n_field])   # (the first ones 16-byte aligned)
+    nbytes = int(lib().ssc_bn_scratch_bytes(n, c))
     scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
-    _check(lib().ssc_bn_stats(_p(x, torch.float32), x.shape[0], x.shape[1], _p(field_of_channel, torch.int32),
-                              _p(scalar_of_channel, torch.int32), int(n_field), int(n_scalar), _p(mean), _p(var),
-                              _p(scratch), nbytes, _stream()))
-    return mean[:n_scalar], var[:n_field]
+    _check(lib().ssc_bn_train(_p(x, torch.float32), n, c, _p(field_of_channel, torch.int32),
+                              _p(scalar_of_channel, torch.int32), int(n_field), int(n_scalar), _p(weight), _p(bias),
+                              float(eps), float(momentum), _p(running_mean), _p(running_var), mean.data_ptr() or flat.data_ptr(), _p(var),
+                              _p(chan_mean), _p(scale), _p(shift), _p(scratch), nbytes, _stream()))
+    for t in (running_mean, running_var):
+        if t is not None:
+            torch.autograd.graph.increment_version(t)     # written behind torch's back
+    return mean, var, chan_mean, scale, shift
+
+
+def bn_gate_backward(x, gout, field_of_channel, scalar_of_channel, n_field, n_scalar, scale, shift, chan_mean, var, weight,
+                     eps, training, gate=None):
+    """(gx, d_weight [n_field], d_bias [n_scalar]) of a batch norm followed by the gated activation `gate` =
+    (gate_of_channel, field_start, field_len, scalar_act, gate_act), or of the batch norm alone."""
+    x, gout = x.contiguous(), gout.contiguous()
+    n, c = x.shape
+    gx = torch.empty_like(x)
+    d_w = torch.empty(n_field, dtype=torch.float32, device=x.device)
+    d_b = torch.empty(max(n_scalar, 1), dtype=torch.float32, device=x.device)
+    nbytes = int(lib().ssc_bn_scratch_bytes(n, c))
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    table, start, length, s_act, g_act = gate if gate is not None else (None, None, None, 0, 0)
+    _check(lib().ssc_bn_gate_bwd(_p(x, torch.float32), _p(gout, torch.float32), n, c, gout.shape[1],
+                                 _p(field_of_channel, torch.int32), _p(scalar_of_channel, torch.int32), int(n_field),
+                                 _p(scale), _p(shift), _p(chan_mean), _p(var), _p(weight), float(eps),
+                                 int(bool(training)), _p(table), _p(start), _p(length), int(s_act), int(g_act), _p(gx),
+                                 _p(d_w), _p(d_b), _p(scratch), nbytes, _stream()))
+    return gx, d_w, d_b[:n_scalar]
 
 
 def bn_backward(x, gy, field_of_channel, scalar_of_channel, n_field, n_scalar, mean, var, weight, eps, training):

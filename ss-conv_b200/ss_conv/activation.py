@@ -135,6 +135,24 @@ class Activation(nn.Module):
         return _act_code(self._scalar_fn if self.scalar_act is not None else None) is not None and \
             _act_code(self._gate_fn if self.gate_act is not None else None) is not None
 
+    def c_out(self):
+        return Rs2dim(self.Rs)
+
+    def c_in(self):
+        return self.c_out() + (sum(self.multiplicities[1:]) if self.gate_act is not None else 0)
+
+    def fusable_gate(self):
+        """relu / sigmoid / identity without biases, at least one of them an activation: what the
+        library's gate kernels cover in both directions."""
+        acts = [a for a in (self.scalar_act, self.gate_act) if a is not None]
+        return bool(acts) and all(a.bias is None for a in acts) and self.fusable()
+
+    def gate_tables(self, device):
+        """(gate_of_channel, field_start, field_len, scalar act code, gate act code)."""
+        return (self._gate_table(device), *self._field_ranges(device),
+                _act_code(self._scalar_fn) if self.scalar_act is not None else 0,
+                _act_code(self._gate_fn) if self.gate_act is not None else 0)
+
     def forward(self, input):
         if self.scalar_act is None and self.gate_act is None:
             return input

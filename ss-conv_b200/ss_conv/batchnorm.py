@@ -21,39 +21,41 @@ def _channel_tables(Rs):
 
 
 class _BatchNormFn(torch.autograd.Function):
-    """y = (x - mean) * weight / sqrt(var + eps) + bias with the library's kernels in both directions.
-    Training mode: mean / var are the batch statistics (ssc_bn_stats) and the gradient flows through
-    them; eval mode: the running buffers, constants."""
+    """y = (x - mean) * weight / sqrt(var + eps) + bias, optionally followed by a gated activation (`gate`, see
+    _ext.bn_gate_backward; `c_out` its output channels), with the library's kernels in both directions.
+    Training mode: mean / var are the batch statistics (ssc_bn_train) and the gradient flows through
+    them; eval mode: the running buffers, constants.  With the activation inside, neither the normalised
+    rows nor their gradient are ever stored (ssc_bn_gate_bwd recomputes them)."""
 
     @staticmethod
-    def forward(ctx, x, weight, bias, module, training):
+    def forward(ctx, x, weight, bias, module, training, gate, c_out):
         x = x.contiguous()
         field, scalar = module._device_tables(x.device)
         n_field, n_scalar = module.running_var.numel(), module.running_mean.numel()
-        if training:
-            mean, var = _ext.bn_stats(x, field, scalar, n_field, n_scalar)
-            with torch.no_grad():
-                module.running_mean.mul_(1 - module.momentum).add_(module.momentum * mean)
-                module.running_var.mul_(1 - module.momentum).add_(module.momentum * var)
-        else:
-            mean, var = module.running_mean.clone(), module.running_var.clone()
         w = None if weight is None else weight.detach().contiguous()
         b = None if (bias is None or n_scalar == 0) else bias.detach().contiguous()
-        scale, shift = _ext.bn_fold(mean if n_scalar > 0 else None, var, w, b, field, scalar, module.eps)
-        y = _ext.bn_gate_forward(x, scale, shift, None, x.size(1), 0, 0, 0, None, None)
-        ctx.save_for_backward(x, mean, var, w if w is not None else x.new_empty(0))
+        if training:
+            mean, var, chan_mean, scale, shift = _ext.bn_train(x, field, scalar, n_field, n_scalar, w, b, module.eps,
+                                                               module.momentum, *module._running())
+        else:
+            mean, var, chan_mean = module.running_mean.clone(), module.running_var.clone(), None
+            scale, shift = _ext.bn_fold(mean if n_scalar > 0 else None, var, w, b, field, scalar, module.eps)
+            chan_mean = torch.zeros_like(scale) if n_scalar == 0 else mean[scalar.clamp(min=0).long()] * (scalar >= 0)
+        if gate is None:
+            y = _ext.bn_gate_forward(x, scale, shift, None, x.size(1), 0, 0, 0, None, None)
+        else:
+            y = _ext.bn_gate_forward(x, scale, shift, gate[0], c_out, c_out, gate[3], gate[4], None, None)
+        ctx.save_for_backward(x, var, chan_mean, scale, shift, w if w is not None else x.new_empty(0))
         ctx.tables, ctx.sizes, ctx.eps, ctx.training_mode = (field, scalar), (n_field, n_scalar), module.eps, bool(training)
-        ctx.has_w, ctx.has_b = weight is not None, bias is not None
+        ctx.has_w, ctx.has_b, ctx.gate = weight is not None, bias is not None, gate
         return y
 
     @staticmethod
     def backward(ctx, gy):
-        x, mean, var, w = ctx.saved_tensors
-        field, scalar = ctx.tables
-        n_field, n_scalar = ctx.sizes
-        gx, d_w, d_b = _ext.bn_backward(x, gy, field, scalar, n_field, n_scalar, mean, var, w if ctx.has_w else None,
-                                        ctx.eps, ctx.training_mode)
-        return gx, (d_w if ctx.has_w else None), (d_b if ctx.has_b else None), None, None
+        x, var, chan_mean, scale, shift, w = ctx.saved_tensors
+        gx, d_w, d_b = _ext.bn_gate_backward(x, gy, *ctx.tables, *ctx.sizes, scale, shift, chan_mean, var,
+                                             w if ctx.has_w else None, ctx.eps, ctx.training_mode, ctx.gate)
+        return gx, (d_w if ctx.has_w else None), (d_b if ctx.has_b else None), None, None, None, None
 
 
 class BatchNorm(nn.Module):
@@ -121,6 +123,11 @@ class BatchNorm(nn.Module):
             self._folded = (key, folded)
         return folded
 
+    def _running(self):
+        """The running buffers for an in-place update by the library."""
+        self._folded = None
+        return (self.running_mean if self.running_mean.numel() else None), self.running_var
+
     def _differentiable(self, x):
         """The layer as a composite of torch ops, used while autograd is recording so that
         gradients reach the input, the affine parameters and (training mode) the batch
@@ -161,6 +168,22 @@ class BatchNorm(nn.Module):
                 self.running_var.mul_(1 - self.momentum).add_(self.momentum * torch.cat(new_var))
         return torch.cat(parts, dim=1)
 
+    def norm_and_gate(self, input, act):
+        """act(self(input)) while autograd records, as one Function when both are the library's kernels (a
+        fused activation without biases on float32 rows); None where they have to run one by one."""
+        x = input.raw()[0]
+        if not (torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.float32 and act.fusable_gate()
+                and (x.requires_grad or (self.training and self.affine and self.weight.requires_grad))
+                and self.reduce == 'mean' and act.c_in() == x.shape[1] == len(_channel_tables(self.Rs)[0])):
+            return None
+        feats = input.features
+        if feats.shape[0] == 0:
+            return None
+        gate = act.gate_tables(feats.device)
+        input.features = _BatchNormFn.apply(feats, self.weight if self.affine else None, self.bias if self.affine else None,
+                                            self, self.training, gate, act.c_out())
+        return input
+
     def forward(self, input):
         # inference without no_grad() (nothing upstream asks for a gradient) keeps the fused kernels
         if torch.is_grad_enabled() and (input.raw()[0].requires_grad or
@@ -170,7 +193,8 @@ class BatchNorm(nn.Module):
             feats = input.features
             if feats.is_cuda and feats.dtype == torch.float32 and feats.shape[0] > 0:
                 input.features = _BatchNormFn.apply(feats, self.weight if self.affine else None,
-                                                    self.bias if self.affine else None, self, self.training)
+                                                    self.bias if self.affine else None, self, self.training, None,
+                                                    feats.shape[1])
             else:
                 input.features = self._differentiable(feats)
             return input
@@ -183,11 +207,10 @@ class BatchNorm(nn.Module):
         if self.training:
             if self.reduce != 'mean':
                 raise ValueError("Invalid reduce option {}".format(self.reduce))
-            mean, var = _ext.bn_stats(x, field, scalar, self.running_var.numel(), self.running_mean.numel())
-            scale, shift = self.folded_affine(x.device, mean, var)
-            with torch.no_grad():
-                self.running_mean.mul_(1 - self.momentum).add_(self.momentum * mean)
-                self.running_var.mul_(1 - self.momentum).add_(self.momentum * var)
+            w, b = (self.weight.detach(), self.bias.detach()) if self.affine else (None, None)
+            scale, shift = _ext.bn_train(x, field, scalar, self.running_var.numel(), self.running_mean.numel(), w,
+                                         b if self.running_mean.numel() else None, self.eps, self.momentum,
+                                         *self._running())[3:]
         else:
             scale, shift = self.folded_affine(x.device)
 

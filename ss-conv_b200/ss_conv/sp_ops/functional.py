@@ -32,7 +32,7 @@ def _conv_function(inverse, subm):
             indice_pair_num, features, filters = ctx.saved_tensors
             indice_pairs = ctx.indice_pairs
             d_in, d_flt = ops.indice_conv_backward(features, filters, grad_output.contiguous(), indice_pairs,
-                                                   indice_pair_num, inverse, subm)
+                                                   indice_pair_num, inverse, subm, ctx.needs_input_grad[:2])
             return d_in, d_flt, None, None, None
 
     return _Conv

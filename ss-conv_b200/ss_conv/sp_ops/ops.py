@@ -66,9 +66,10 @@ def indice_conv_forward(features, filters, indice_pairs, indice_pair_num, num_ac
     return fn(features, filters, indice_pairs, indice_pair_num, num_activate_out, int(inverse), int(subm))
 
 
-def indice_conv_backward(features, filters, out_bp, indice_pairs, indice_pair_num, inverse=False, subm=False):
+def indice_conv_backward(features, filters, out_bp, indice_pairs, indice_pair_num, inverse=False, subm=False,
+                         need=(True, True)):
     fn = _by_dtype(filters, _ext.indice_conv_backward_fp32, _ext.indice_conv_backward_half)
-    return fn(features, filters, out_bp, indice_pairs, indice_pair_num, int(inverse), int(subm))
+    return fn(features, filters, out_bp, indice_pairs, indice_pair_num, int(inverse), int(subm), need)
 
 
 def indice_avgpool_forward(features, indice_pairs, indice_pair_num, num_activate_out, summaryrf):

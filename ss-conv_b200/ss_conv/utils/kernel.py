@@ -108,7 +108,7 @@ def _orthogonal_(tensor, gain=1):
 
 
 class _Materialize(torch.autograd.Function):
-    """filters = M(weight) by the CUDA kernel; the backward applies M^T with torch ops."""
+    """filters = M(weight) and its adjoint M^T, one CUDA kernel each."""
 
     @staticmethod
     def forward(ctx, weight, kernel):
@@ -185,10 +185,11 @@ class SE3Kernel(torch.nn.Module):
         in_field = [(j, v, c) for j, m in enumerate(self.multiplicities_in) for v in range(m)
                     for c in range(self.dims_in[j])]
         blob = (torch.cat(blobs) if blobs else torch.zeros(1)).to(device)
-        packed = (device, blob, torch.tensor(table, dtype=torch.int32, device=device),
-                  torch.tensor(out_field, dtype=torch.int32, device=device).reshape(-1),
-                  torch.tensor(in_field, dtype=torch.int32, device=device).reshape(-1))
+        ints = lambda v: torch.tensor(v, dtype=torch.int32, device=device).reshape(-1)  # noqa: E731
+        packed = (device, blob, ints(table), ints(out_field), ints(in_field))
         self._packed = packed
+        self._starts = (ints([k for k, f in enumerate(out_field) if f[2] == 0]),
+                        ints([k for k, f in enumerate(in_field) if f[2] == 0]))
         return packed[1:]
 
     def _apply(self, fn, *args, **kwargs):
@@ -212,23 +213,11 @@ class SE3Kernel(torch.nn.Module):
 
     def _weight_grad(self, g):
         """Adjoint of the (linear) materialisation: g [k,k,k,Cin,Cout] -> gradient of the flat
-        weight vector, block by block (weights of block (i,j) are laid out [m_out, m_in, n_basis])."""
-        k = self.size
-        grads = []
-        out_off = 0
-        for i, (m_out, _) in enumerate(self.Rs_out):
-            do = self.dims_out[i]
-            in_off = 0
-            for j, (m_in, _) in enumerate(self.Rs_in):
-                di = self.dims_in[j]
-                b = getattr(self, "kernel_{}_{}".format(i, j))
-                if b is not None:
-                    blk = g[:, :, :, in_off:in_off + m_in * di, out_off:out_off + m_out * do]
-                    blk = blk.reshape(k, k, k, m_in, di, m_out, do)
-                    grads.append(torch.einsum("xyzvcua,bacxyz->uvb", blk, b.to(g.dtype)).reshape(-1))
-                in_off += m_in * di
-            out_off += m_out * do
-        return torch.cat(grads) if grads else g.new_zeros(0)
+        weight vector (weights of block (i,j) are laid out [m_out, m_in, n_basis])."""
+        blob, table, out_field, in_field = self._tables(g.device)
+        return _ext.materialize_backward(g.float(), blob, table, len(self.Rs_in), out_field, in_field, *self._starts,
+                                         max(self.dims_out) * max(self.dims_in), self.n_out, self.n_in, self.size ** 3,
+                                         self.weight.numel()).to(self.weight.dtype)
 
     def combination(self, weight):
         """[Cout, Cin, k, k, k] kernel (a permuted view of `filters`)."""

@@ -52,10 +52,14 @@ class SS_Conv(nn.Module):
 
     def forward(self, x):
         x = self.conv(x)
-        if self.bn is not None:
-            x = self.bn(x)
-        if self.activation is not None:
-            x = self.activation(x)
+        both = self.bn.norm_and_gate(x, self.activation) if self.bn is not None and self.activation is not None else None
+        if both is not None:
+            x = both
+        else:
+            if self.bn is not None:
+                x = self.bn(x)
+            if self.activation is not None:
+                x = self.activation(x)
         if self.dropout is not None:
             x = self.dropout(x)
         return x
