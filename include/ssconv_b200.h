@@ -330,6 +330,12 @@ size_t ssc_conv_wgrad_scratch_bytes(int K, int c_in, int c_out, int n_out);
 int ssc_conv_wgrad(const float *features, int c_in, const float *out_grad, int c_out, const int32_t *nbr,
                    int K, int n_out, int precision, float *d_filters, int32_t *status, void *scratch,
                    size_t scratch_bytes, void *stream);
+/* The same with the table's compacted pair lists already in hand (ssc_conv_pairs_build; layers that share a
+ * rulebook share them): nothing is built per call.  lists NULL: built in scratch, as ssc_conv_wgrad does. */
+int ssc_conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int c_out,
+                         const int32_t *nbr, int K, int n_out, void *lists, size_t list_bytes, int precision,
+                         float *d_filters, int32_t *status, void *scratch, size_t scratch_bytes,
+                         void *stream);
 int ssc_maxpool_bwd(const float *features, const float *out_features, const float *out_grad, int c,
                     const int32_t *nbr_in, int K, int n_in, float *d_in, void *stream);
 int ssc_avgpool_bwd(const float *out_grad, int c, const int32_t *nbr_in, int K, int n_in,

@@ -13,7 +13,7 @@
 //
 // Pool gradients walk the input-major table: one thread per (input row, 4 channels) adds its
 // outputs' gradients in ascending offset order (the order of the reference's loop), no atomics.
-#include "ssc_common.cuh"
+#include "ssc_conv_internal.cuh"
 
 namespace ssc {
 
@@ -239,27 +239,25 @@ static int wgrad_splits(int K, int c_in, int c_out, int n_out) {
   return splits;
 }
 
-namespace ssc {
-int conv_wgrad_tc(const float *features, int c_in, const float *out_grad, int c_out, const int32_t *nbr, int K, int n_out,
-                  int max_splits, int *splits_used, float *partial, void *lists, int32_t *status, cudaStream_t st);
-size_t conv_wgrad_tc_list_bytes(int K, int n_out);
-}
-
-// [partial tiles of the row ranges][pair lists of the tensor-core kernel]
+// [partial tiles][pair lists, where the caller has none yet]
 static size_t wgrad_partial_bytes(int K, int c_in, int c_out, int n_out) {
-  const size_t b = (size_t)wgrad_splits(K, c_in, c_out, n_out) * K * c_in * c_out * sizeof(float);
+  size_t b = (size_t)wgrad_splits(K, c_in, c_out, n_out) * K * c_in * c_out * sizeof(float);
+  for (int tf32 = 0; tf32 < 2; ++tf32) {
+    const size_t l = conv_wgrad_lists_partial_bytes(K, c_in, c_out, n_out, tf32 != 0);
+    if (l > b) b = l;
+  }
   return (b + 255) & ~(size_t)255;
 }
 
 extern "C" size_t ssc_conv_wgrad_scratch_bytes(int K, int c_in, int c_out, int n_out) {
   if (K < 1 || c_in < 1 || c_out < 1 || n_out < 0) return 0;
-  return wgrad_partial_bytes(K, c_in, c_out, n_out) + conv_wgrad_tc_list_bytes(K, n_out);
+  return wgrad_partial_bytes(K, c_in, c_out, n_out) + pair_lists_bytes(K, n_out);
 }
 
-extern "C" int ssc_conv_wgrad(const float *features, int c_in, const float *out_grad, int c_out, const int32_t *nbr, int K,
-                              int n_out, int precision, float *d_filters, int32_t *status, void *scratch,
-                              size_t scratch_bytes, void *stream) {
-  SSC_REQUIRE(K >= 1 && c_in >= 1 && c_out >= 1 && n_out >= 0 && d_filters, "conv_wgrad: bad arguments");
+extern "C" int ssc_conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int c_out, const int32_t *nbr, int K,
+                                    int n_out, void *lists, size_t list_bytes, int precision, float *d_filters,
+                                    int32_t *status, void *scratch, size_t scratch_bytes, void *stream) {
+  SSC_REQUIRE(K >= 1 && K <= 256 && c_in >= 1 && c_out >= 1 && n_out >= 0 && d_filters, "conv_wgrad: bad arguments");
   cudaStream_t st = as_stream(stream);
   const long long elems = (long long)K * c_in * c_out;
   if (n_out == 0) {
@@ -267,28 +265,39 @@ extern "C" int ssc_conv_wgrad(const float *features, int c_in, const float *out_
     return SSC_OK;
   }
   SSC_REQUIRE(features && out_grad && nbr, "conv_wgrad: null pointer");
-  const int splits = wgrad_splits(K, c_in, c_out, n_out);
-  const size_t need = ssc_conv_wgrad_scratch_bytes(K, c_in, c_out, n_out);
+  const size_t partial_bytes = wgrad_partial_bytes(K, c_in, c_out, n_out);
+  const size_t need = lists ? partial_bytes : partial_bytes + pair_lists_bytes(K, n_out);
   if (scratch == nullptr || scratch_bytes < need)
     return fail(SSC_ERR_SCRATCH, "conv_wgrad: scratch %zu < %zu bytes", scratch_bytes, need);
+  SSC_REQUIRE(lists == nullptr || list_bytes >= pair_lists_bytes(K, n_out), "conv_wgrad: list buffer too small");
+  const bool tf32 = precision == SSC_PREC_TF32;
+  if (conv_wgrad_lists_partial_bytes(K, c_in, c_out, n_out, tf32) > 0) {
+    PairLists pl;
+    if (lists) {
+      pl = pair_lists_view(lists, K, n_out);
+    } else if (int e = pair_lists_build(nbr, K, n_out, (uint8_t *)scratch + partial_bytes, &pl, st)) {
+      return e;
+    }
+    return conv_wgrad_lists(features, c_in, out_grad, c_out, pl, K, n_out, tf32, (float *)scratch, d_filters, status, st);
+  }
+  const int splits = wgrad_splits(K, c_in, c_out, n_out);
   int rows_per_split = ceil_div(n_out, splits);
   rows_per_split = ceil_div(rows_per_split, WG_ROWS) * WG_ROWS;
-  int rc = -1, used = splits;
-  if (precision == SSC_PREC_TF32)  // tensor cores where the shape allows, else the exact kernel below
-    rc = conv_wgrad_tc(features, c_in, out_grad, c_out, nbr, K, n_out, splits, &used, (float *)scratch,
-                       (uint8_t *)scratch + wgrad_partial_bytes(K, c_in, c_out, n_out), status, st);
-  if (rc > 0) return rc;
-  if (rc < 0) {
-    const int tiles_co = ceil_div(c_out, WG_T);
-    dim3 grid(splits, K, ceil_div(c_in, WG_T) * tiles_co);
-    { conv_wgrad_partial_kernel<<<grid, 256, 0, st>>>(features, c_in, out_grad, c_out, nbr, n_out, rows_per_split, tiles_co,
-                                                     (float *)scratch); note_launches(1); }
-    SSC_CHECK_LAUNCH("conv_wgrad_partial");
-    used = splits;
-  }
-  { wgrad_reduce_kernel<<<ceil_div(elems, 256), 256, 0, st>>>((const float *)scratch, used, elems, d_filters); note_launches(1); }
+  const int tiles_co = ceil_div(c_out, WG_T);
+  dim3 grid(splits, K, ceil_div(c_in, WG_T) * tiles_co);
+  { conv_wgrad_partial_kernel<<<grid, 256, 0, st>>>(features, c_in, out_grad, c_out, nbr, n_out, rows_per_split, tiles_co,
+                                                   (float *)scratch); note_launches(1); }
+  SSC_CHECK_LAUNCH("conv_wgrad_partial");
+  { wgrad_reduce_kernel<<<ceil_div(elems, 256), 256, 0, st>>>((const float *)scratch, splits, elems, d_filters); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_wgrad_reduce");
   return SSC_OK;
+}
+
+extern "C" int ssc_conv_wgrad(const float *features, int c_in, const float *out_grad, int c_out, const int32_t *nbr, int K,
+                              int n_out, int precision, float *d_filters, int32_t *status, void *scratch,
+                              size_t scratch_bytes, void *stream) {
+  return ssc_conv_wgrad_lists(features, c_in, out_grad, c_out, nbr, K, n_out, nullptr, 0, precision, d_filters, status, scratch,
+                              scratch_bytes, stream);
 }
 
 template <int MODE>

@@ -71,6 +71,8 @@ SIGNATURES = {
     "ssc_conv_wgrad_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "ssc_conv_wgrad": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
                                c_void_p, c_size_t, c_void_p]),
+    "ssc_conv_wgrad_lists": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_size_t, c_int,
+                                     c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "ssc_maxpool_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "ssc_avgpool_bwd": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "ssc_global_avgpool_bwd": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
@@ -919,9 +921,10 @@ def conv_wgrad(features, out_grad, nbr, precision=None):
     d_flt = torch.empty((K, c_in, c_out), dtype=torch.float32, device=features.device)
     nbytes = int(lib().ssc_conv_wgrad_scratch_bytes(K, c_in, c_out, n_out))
     scratch = torch.empty(max(nbytes, 4), dtype=torch.uint8, device=features.device)
-    _check(lib().ssc_conv_wgrad(_p(features, torch.float32), c_in, _p(out_grad, torch.float32), c_out,
-                                _p(nbr, torch.int32), K, n_out, mode, _p(d_flt), _p(status_word(features.device)),
-                                _p(scratch), nbytes, _stream()))
+    lists = pair_lists(nbr) if n_out > 0 and (mode == PREC_TF32 or c_in <= 16) else None
+    _check(lib().ssc_conv_wgrad_lists(_p(features, torch.float32), c_in, _p(out_grad, torch.float32), c_out,
+                                      _p(nbr, torch.int32), K, n_out, _p(lists), lists.numel() if lists is not None else 0,
+                                      mode, _p(d_flt), _p(status_word(features.device)), _p(scratch), nbytes, _stream()))
     return d_flt
 
 
