@@ -270,7 +270,10 @@ extern "C" int ssc_conv_wgrad_lists(const float *features, int c_in, const float
   if (scratch == nullptr || scratch_bytes < need)
     return fail(SSC_ERR_SCRATCH, "conv_wgrad: scratch %zu < %zu bytes", scratch_bytes, need);
   SSC_REQUIRE(lists == nullptr || list_bytes >= pair_lists_bytes(K, n_out), "conv_wgrad: list buffer too small");
-  const bool tf32 = precision == SSC_PREC_TF32;
+  const int staged = ((precision & SSC_WGRAD_X_STAGED) ? 1 : 0) | ((precision & SSC_WGRAD_DY_STAGED) ? 2 : 0);
+  const bool tf32 = (precision & ~(SSC_WGRAD_X_STAGED | SSC_WGRAD_DY_STAGED)) == SSC_PREC_TF32;
+  SSC_REQUIRE(staged == 0 || (tf32 && conv_wgrad_lists_partial_bytes(K, c_in, c_out, n_out, true) > 0),
+              "conv_wgrad: staged operands need TF32 and at most 256 input channels");
   if (conv_wgrad_lists_partial_bytes(K, c_in, c_out, n_out, tf32) > 0) {
     PairLists pl;
     if (lists) {
@@ -278,7 +281,7 @@ extern "C" int ssc_conv_wgrad_lists(const float *features, int c_in, const float
     } else if (int e = pair_lists_build(nbr, K, n_out, (uint8_t *)scratch + partial_bytes, &pl, st)) {
       return e;
     }
-    return conv_wgrad_lists(features, c_in, out_grad, c_out, pl, K, n_out, tf32, (float *)scratch, d_filters, status, st);
+    return conv_wgrad_lists(features, c_in, out_grad, c_out, pl, K, n_out, tf32, staged, (float *)scratch, d_filters, status, st);
   }
   const int splits = wgrad_splits(K, c_in, c_out, n_out);
   int rows_per_split = ceil_div(n_out, splits);

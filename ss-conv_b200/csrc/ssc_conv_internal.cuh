@@ -49,6 +49,6 @@ PairLists pair_lists_view(void *lists, int K, int n_out);
 // filter gradient over pair lists (ssc_wgrad_tc.cu): bytes of its partial tiles, 0 where the shape is not covered
 size_t conv_wgrad_lists_partial_bytes(int K, int c_in, int c_out, int n_out, bool tf32);
 int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int c_out, const PairLists &pl, int K, int n_out,
-                     bool tf32, float *partial, float *d_filters, int32_t *status, cudaStream_t st);
+                     bool tf32, int staged, float *partial, float *d_filters, int32_t *status, cudaStream_t st);
 
 }  // namespace ssc

@@ -17,15 +17,19 @@
 // which the centre offset alone kept ten CTAs busy.)
 //
 // conv_wgrad_tc_kernel (TF32 operands, tcgen05): a CTA accumulates D[co][ci] (M = 128 rows = output channels
-// of one block of 128, N = input channels) in tensor memory; K = pairs, 32 per chunk.  Both operands have
-// to be K-major, i.e. transposed with respect to how the rows lie in memory, so the producer warps
-// transpose on the way into shared memory: lane = pair of the chunk; for every channel the 32 lanes
-// store 32 consecutive K elements of that channel's operand row (one conflict-free 128-byte store, in the
-// 128-byte-swizzled layout), rounded to TF32; lanes past the end of a list store zeros.  Operand rows of
-// channels past c_out / c_in are zeroed once and never touched again.
-//   warps 0-7: producers, two per ring slot (dy rows and x rows), indices one chunk ahead
-//   warp 8: tensor-memory allocation and the MMA-issuing thread
-//   warps 9-12: write finished partials (two accumulator buffers where tensor memory allows, so that
+// of one block of 128, N = input channels) in tensor memory; K = pairs, 32 per chunk.  The rows go to
+// shared memory as they lie in global memory (channels contiguous) and the tensor core takes both
+// operands MN-major: 32 channels of a pair are one 128-byte line, pairs follow one another, the 32-byte
+// pieces of line k are exchanged by XOR with k & 3 (swizzle mode "128 bytes with 32-byte atoms", the one
+// the 32-bit formats have for this order).  Eight lanes fetch a line with 16-byte cp.async, so a gather
+// costs one L1 line per 128 bytes; transposed on the way in (lane = pair, one 16-byte piece of 32 rows
+// per instruction) it was bound by that at 32 lines per instruction.  Rows that are not rounded to
+// TF32 yet are rounded in place once they have landed.  Pairs past the end of a list are zero rows;
+// channels past c_out / c_in are whatever the buffer holds: they only reach rows and columns of D
+// that nobody reads.
+//   warps 0 .. stages-1: producers, warp w owns ring slot w, pair indices one round ahead
+//   the next warp: tensor-memory allocation and the MMA-issuing thread
+//   four more: write finished partials (two accumulator buffers where tensor memory allows, so that
 //   the next offset's sums run meanwhile)
 // conv_wgrad_small_kernel (exact fp32, up to 16 input channels): a warp is a share, lanes = output channels.
 // Every wait is bounded (status bit 16 on expiry).
@@ -36,12 +40,9 @@
 namespace ssc {
 
 constexpr int WT_M = 128;          // output channels per CTA
-constexpr int WT_K = 32;           // output rows per chunk
-constexpr int WT_STAGES = 4;
-constexpr int WT_A_BYTES = WT_M * 128;
-constexpr int WT_PRODUCERS = 2 * WT_STAGES;
-constexpr int WT_MMA_WARP = WT_PRODUCERS;
-constexpr int WT_THREADS = (WT_PRODUCERS + 1 + 4) * 32;
+constexpr int WT_K = 32;           // pairs per chunk
+constexpr int WT_MAX_STAGES = 8;
+constexpr int WT_BLOCK = WT_K * 128;   // 32 channels of a chunk's pairs
 
 // One warp per 32 output rows of one kernel offset: which of them have a neighbour.
 __global__ void pair_bitmap_kernel(const int32_t *__restrict__ nbr, int K, int n_out, int words_per_row,
@@ -69,11 +70,6 @@ __global__ void pair_scatter_kernel(const int32_t *__restrict__ nbr, int K, int 
     pair_out[pos] = r;
     pair_in[pos] = __ldg(nbr + (size_t)kappa * n_out + r);
   }
-}
-
-__device__ __forceinline__ uint32_t wt_off(int row, int k) {  // byte offset of element (row, k) of a K-major SW128 tile
-  return (uint32_t)(row >> 3) * 1024u + (uint32_t)(row & 7) * 128u + ((((uint32_t)k >> 2) ^ (uint32_t)(row & 7)) << 4) +
-         ((uint32_t)k & 3u) * 4u;
 }
 
 // ---------------------------------------------------------------- shares of the row of chunks
@@ -105,161 +101,192 @@ __device__ __forceinline__ int share_of(int q, int total, int shares) {
   return b;
 }
 
-__global__ void __launch_bounds__(WT_THREADS)
-conv_wgrad_tc_kernel(const float *__restrict__ features, int c_in, const float *__restrict__ out_grad, int c_out,
-                     const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in,
-                     const int32_t *__restrict__ starts, int K, int n_pad, uint32_t buf_cols, int n_buf,
-                     float *__restrict__ partial, int32_t *status) {
+struct WtParams {
+  const float *x, *dy;         // [n][x_words], [n][y_words]
+  int c_in, c_out;
+  int x_words, y_words;        // row strides
+  int x_round, y_round;        // 1: rows still to be rounded to TF32
+  int n_pad, a_bytes, stage_bytes, stages, n_buf;
+  uint32_t buf_cols;
+};
+
+// smem descriptor halves of an MN-major operand: 32-channel blocks WT_BLOCK bytes apart (leading offset), four
+// pairs 512 bytes (stride offset), swizzle mode 1 (128 bytes, 32-byte atoms), descriptor version 1
+constexpr uint32_t kMnDescHi = (uint32_t)(512 >> 4) | (1u << 14) | (1u << 29);
+__device__ __forceinline__ uint32_t mn_desc_lo(uint32_t saddr) { return ((saddr >> 4) & 0x3FFFu) | ((uint32_t)(WT_BLOCK >> 4) << 16); }
+__device__ __forceinline__ void mma_tf32_mn(uint32_t tmem_c, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 da, {%1, %5};\n\t"
+      "mov.b64 db, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %3, {%6, %6, %6, %6}, p;\n\t}"
+      :
+      : "r"(tmem_c), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kMnDescHi), "r"(0u)
+      : "memory");
+}
+
+__global__ void __launch_bounds__((WT_MAX_STAGES + 5) * 32)
+conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in,
+                     const int32_t *__restrict__ starts, int K, float *__restrict__ partial, int32_t *status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int first[257];
+  __shared__ uint64_t full_bars[WT_MAX_STAGES], empty_bars[WT_MAX_STAGES], accf_bars[2], acce_bars[2], done_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_word;
+  volatile int *abort_flag = &abort_word;
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int b_bytes = n_pad * 128;
-  const int stage_bytes = WT_A_BYTES + b_bytes;
-  uint8_t *ctrl = smem + (size_t)WT_STAGES * stage_bytes;
-  uint64_t *full_bars = (uint64_t *)ctrl;                  // [WT_STAGES]
-  uint64_t *empty_bars = full_bars + WT_STAGES;            // [WT_STAGES]
-  uint64_t *accf_bars = empty_bars + WT_STAGES;            // [2] a partial is complete
-  uint64_t *acce_bars = accf_bars + 2;                     // [2] and has been read out
-  uint64_t *done_bar = acce_bars + 2;
-  uint32_t *tmem_slot = (uint32_t *)(done_bar + 1);
-  volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int S = p.stages, mma_warp = S;
   const int co0 = blockIdx.y * WT_M;
   if (tid == 0) {
-    for (int s = 0; s < WT_STAGES; ++s) {
-      mbar_init(smem_u32(full_bars + s), 64);
+    for (int s = 0; s < S; ++s) {
+      mbar_init(smem_u32(full_bars + s), 32);
       mbar_init(smem_u32(empty_bars + s), 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(accf_bars + b), 1);
       mbar_init(smem_u32(acce_bars + b), 4);
     }
-    mbar_init(smem_u32(done_bar), 1);
+    mbar_init(smem_u32(&done_bar), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == WT_MMA_WARP) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(buf_cols * (uint32_t)n_buf)
+  if (warp == mma_warp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(p.buf_cols * (uint32_t)p.n_buf)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  // operand rows of channels that do not exist stay zero for the whole kernel
-  for (int i = tid; i < WT_STAGES * stage_bytes / 16; i += WT_THREADS) ((uint4 *)smem)[i] = make_uint4(0u, 0u, 0u, 0u);
-  fence_async_smem();
   chunk_prefix(starts, K, first);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = tmem_slot;
   const uint32_t smem_base = smem_u32(smem);
-  const int m_cnt = min(WT_M, c_out - co0);   // output channels of this CTA
+  const int m_cnt = min(WT_M, p.c_out - co0);   // output channels of this CTA
   const int total = first[K];
   const int q_begin = share_begin((int)blockIdx.x, total, (int)gridDim.x), q_end = share_begin((int)blockIdx.x + 1, total, (int)gridDim.x);
-  int kappa0 = 0;                             // the offset the share begins in
+  int kappa0 = 0;                               // the offset the share begins in
   while (kappa0 + 1 < K && first[kappa0 + 1] <= q_begin) ++kappa0;
 
-  if (warp < WT_PRODUCERS) {
+  if (warp < S) {
     // ====================================== producers ========================================
-    // Chunk q uses ring slot (q - q_begin) % WT_STAGES; warps 2s and 2s + 1 serve slot s: the first brings
-    // the dy rows (operand A), the second the x rows (operand B).
-    const int slot = warp >> 1, part = warp & 1;
     uint32_t par = 0;
-    uint8_t *tile = smem + (size_t)slot * stage_bytes + (part ? WT_A_BYTES : 0);
-    const bool vec = ((c_in | c_out) & 3) == 0 && (((uintptr_t)features | (uintptr_t)out_grad) & 15u) == 0;
-    const int32_t *list = part ? pair_in : pair_out;
-    const float *rows = part ? features : out_grad + co0;
-    const int width = part ? c_in : c_out, n_ch = part ? c_in : m_cnt;
     int kappa = kappa0;
-    auto row_of = [&](int q) -> int {          // this lane's row of chunk q, or -1
-      if (q >= q_end) return -1;
+    int row_y = -1, row_x = -1;                 // this lane's pair of the next chunk
+    auto load_pair = [&](int q) {
+      row_y = row_x = -1;
+      if (q >= q_end) return;
       while (first[kappa + 1] <= q) ++kappa;
       const int j = __ldg(starts + kappa) + (q - first[kappa]) * WT_K + lane;
-      return j < __ldg(starts + kappa + 1) ? __ldg(list + j) : -1;
+      if (j < __ldg(starts + kappa + 1)) {
+        row_y = __ldg(pair_out + j);
+        row_x = __ldg(pair_in + j);
+      }
     };
-    int next = row_of(q_begin + slot);
-    for (int q = q_begin + slot; q < q_end; q += WT_STAGES) {
-      const int row = next;
-      next = row_of(q + WT_STAGES);
-      const bool valid = row >= 0;
-      const float *g = rows + (size_t)(valid ? row : 0) * width;
-      bool waited = q < q_begin + WT_STAGES, ok = true;
-      if (vec) {
-        // 32 channels at a time: eight independent 16-byte loads in flight, then 32 transposed stores
-        for (int c0 = 0; c0 < n_ch && ok; c0 += 32) {
-          float4 v[8];
+    const int sub = lane & 7, grp = lane >> 3;  // 16-byte piece of a line, pair of a group of four
+    // lines 0 .. 31 of every 32-channel block; piece `sub` of line k lies at 32-byte atom (sub >> 1) ^ (k & 3)
+    const uint32_t piece = (uint32_t)grp * 128u + ((((uint32_t)sub >> 1) ^ (uint32_t)grp) << 5) + ((uint32_t)sub & 1u) * 16u;
+    // (straight-line over the eight groups of four pairs: as a rolled loop with its address arithmetic this
+    //  was 4100 warp instructions per chunk and the kernel's bound, 172 us on the layer above)
+    auto fetch = [&](const float *rows, int words, int n_ch, int my_row, uint32_t tile) {
+      const float *g[WT_K / 4];
+      uint32_t bytes[WT_K / 4];
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            v[k] = (valid && c0 + k * 4 < n_ch) ? __ldg((const float4 *)(g + c0 + k * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
-          if (!waited) {      // the slot is needed only now, with the first loads on their way
-            ok = mbar_wait_warp(smem_u32(empty_bars + slot), par ^ 1u, abort_flag);
-            tc_fence_after();
-            waited = true;
-            if (!ok) break;
-          }
+      for (int i = 0; i < WT_K / 4; ++i) {
+        const int row = __shfl_sync(0xffffffffu, my_row, i * 4 + grp);
+        g[i] = rows + (size_t)(row >= 0 ? row : 0) * words + sub * 4;
+        bytes[i] = row >= 0 ? 16u : 0u;
+      }
+      uint32_t dst = tile + piece;
+      if ((words & 3) == 0 && ((uintptr_t)rows & 15u) == 0) {
+        for (int left = n_ch - sub * 4; left > 0; left -= 32, dst += WT_BLOCK) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int c = c0 + k * 4;
-            if (c < n_ch) {
-              *(uint32_t *)(tile + wt_off(c + 0, lane)) = to_tf32(v[k].x);
-              *(uint32_t *)(tile + wt_off(c + 1, lane)) = to_tf32(v[k].y);
-              *(uint32_t *)(tile + wt_off(c + 2, lane)) = to_tf32(v[k].z);
-              *(uint32_t *)(tile + wt_off(c + 3, lane)) = to_tf32(v[k].w);
-            }
+          for (int i = 0; i < WT_K / 4; ++i) {
+            cp_async16_cg(dst + (uint32_t)i * 512u, g[i], bytes[i]);
+            g[i] += 32;
           }
         }
       } else {
-        if (!waited) {
-          ok = mbar_wait_warp(smem_u32(empty_bars + slot), par ^ 1u, abort_flag);
-          tc_fence_after();
-        }
-        for (int c0 = 0; c0 < n_ch && ok; c0 += 8) {
-          float v[8];
+        for (int left = n_ch - sub * 4; left > 0; left -= 32, dst += WT_BLOCK) {
+          for (int i = 0; i < WT_K / 4; ++i)
+            for (int e = 0; e < 4; ++e)
+              if (e < left) cp_async4(dst + (uint32_t)i * 512u + 4u * e, g[i] + e, bytes[i] >> 2);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) v[k] = (valid && c0 + k < n_ch) ? __ldg(g + c0 + k) : 0.f;
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            if (c0 + k < n_ch) *(uint32_t *)(tile + wt_off(c0 + k, lane)) = to_tf32(v[k]);
+          for (int i = 0; i < WT_K / 4; ++i) g[i] += 32;
         }
       }
-      if (!ok) break;
+    };
+    auto round_tile = [&](int n_ch, uint8_t *tile) {   // this lane's pieces, in place
+      uint8_t *at = tile + piece;
+      for (int left = n_ch - sub * 4; left > 0; left -= 32, at += WT_BLOCK) {
+        uint4 v[WT_K / 4];
+#pragma unroll
+        for (int i = 0; i < WT_K / 4; ++i) v[i] = *(const uint4 *)(at + i * 512);
+#pragma unroll
+        for (int i = 0; i < WT_K / 4; ++i) {
+          v[i].x = to_tf32(__uint_as_float(v[i].x));
+          v[i].y = to_tf32(__uint_as_float(v[i].y));
+          v[i].z = to_tf32(__uint_as_float(v[i].z));
+          v[i].w = to_tf32(__uint_as_float(v[i].w));
+          *(uint4 *)(at + i * 512) = v[i];
+        }
+      }
+    };
+    uint8_t *slot = smem + (size_t)warp * p.stage_bytes;
+    const uint32_t slot_addr = smem_base + (uint32_t)warp * (uint32_t)p.stage_bytes;
+    load_pair(q_begin + warp);
+    for (int q = q_begin + warp; q < q_end; q += S) {
+      const int ry = row_y, rx = row_x;
+      load_pair(q + S);
+      if (q >= q_begin + S) {
+        if (!mbar_wait_warp(smem_u32(empty_bars + warp), par ^ 1u, abort_flag)) break;
+        tc_fence_after();
+      }
+      fetch(p.dy + co0, p.y_words, m_cnt, ry, slot_addr);
+      fetch(p.x, p.x_words, p.c_in, rx, slot_addr + (uint32_t)p.a_bytes);
+      cp_async_commit();
+      cp_async_wait(0);
+      if (p.y_round) round_tile(m_cnt, slot);
+      if (p.x_round) round_tile(p.c_in, slot + p.a_bytes);
       fence_async_smem();
-      mbar_arrive(smem_u32(full_bars + slot));
+      mbar_arrive(smem_u32(full_bars + warp));
       par ^= 1u;
     }
-  } else if (warp == WT_MMA_WARP) {
+  } else if (warp == mma_warp) {
     // ====================================== MMA issuer =======================================
     if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n_pad >> 3) << 17) | ((uint32_t)(WT_M >> 4) << 24);
+      const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(p.n_pad >> 3) << 17) | ((uint32_t)(WT_M >> 4) << 24);
       int kappa = kappa0, seg = 0;
       bool alive = true;
       uint32_t s = 0, par = 0;
       for (int q = q_begin; q < q_end && alive;) {
         while (first[kappa + 1] <= q) ++kappa;
-        const int stop = min(q_end, first[kappa + 1]), buf = seg % n_buf, use = seg / n_buf;
+        const int stop = min(q_end, first[kappa + 1]), buf = seg % p.n_buf, use = seg / p.n_buf;
         if (use > 0) {
           if (!mbar_wait(smem_u32(acce_bars + buf), (uint32_t)(use - 1) & 1u, abort_flag)) break;
           tc_fence_after();
         }
-        const uint32_t d = tmem_base + (uint32_t)buf * buf_cols;
+        const uint32_t d = tmem_base + (uint32_t)buf * p.buf_cols;
         for (const int q0 = q; q < stop; ++q) {
           if (!mbar_wait(smem_u32(full_bars + s), par, abort_flag)) { alive = false; break; }
           tc_fence_after();
-          const uint32_t a_lo = desc_lo(smem_base + s * (uint32_t)stage_bytes);
-          const uint32_t b_lo = desc_lo(smem_base + s * (uint32_t)stage_bytes + WT_A_BYTES);
-          mma_tf32_ss(d, a_lo, b_lo, idesc, q > q0 ? 1u : 0u);
-          mma_tf32_ss(d, a_lo + 2u, b_lo + 2u, idesc, 1u);
-          mma_tf32_ss(d, a_lo + 4u, b_lo + 4u, idesc, 1u);
-          mma_tf32_ss(d, a_lo + 6u, b_lo + 6u, idesc, 1u);
+          const uint32_t a_lo = mn_desc_lo(smem_base + s * (uint32_t)p.stage_bytes);
+          const uint32_t b_lo = mn_desc_lo(smem_base + s * (uint32_t)p.stage_bytes + (uint32_t)p.a_bytes);
+          mma_tf32_mn(d, a_lo, b_lo, idesc, q > q0 ? 1u : 0u);      // eight pairs per instruction: 1024 bytes apart
+          mma_tf32_mn(d, a_lo + 64u, b_lo + 64u, idesc, 1u);
+          mma_tf32_mn(d, a_lo + 128u, b_lo + 128u, idesc, 1u);
+          mma_tf32_mn(d, a_lo + 192u, b_lo + 192u, idesc, 1u);
           mma_commit(smem_u32(empty_bars + s));
-          if (++s == WT_STAGES) { s = 0; par ^= 1u; }
+          if (++s == (uint32_t)S) { s = 0; par ^= 1u; }
         }
         if (alive) mma_commit(smem_u32(accf_bars + buf));
         ++seg;
       }
       // everything issued above (on any path) retires before the tensor memory is handed back
-      mma_commit(smem_u32(done_bar));
-      mbar_wait_drain(smem_u32(done_bar), 0u);
+      mma_commit(smem_u32(&done_bar));
+      mbar_wait_drain(smem_u32(&done_bar), 0u);
     }
   } else {
     // ====================================== epilogue ===========================================
@@ -269,13 +296,13 @@ conv_wgrad_tc_kernel(const float *__restrict__ features, int c_in, const float *
     for (int q = q_begin; q < q_end; ++seg) {
       while (first[kappa + 1] <= q) ++kappa;
       q = min(q_end, first[kappa + 1]);
-      const int buf = seg % n_buf;
-      if (!mbar_wait_warp_backoff(smem_u32(accf_bars + buf), (uint32_t)(seg / n_buf) & 1u, abort_flag, 64)) break;
+      const int buf = seg % p.n_buf;
+      if (!mbar_wait_warp_backoff(smem_u32(accf_bars + buf), (uint32_t)(seg / p.n_buf) & 1u, abort_flag, 64)) break;
       tc_fence_after();
-      float *dst = partial + ((size_t)blockIdx.x + kappa) * (size_t)c_in * c_out;
-      for (int c0 = 0; c0 < n_pad; c0 += 16) {
+      float *dst = partial + ((size_t)blockIdx.x + kappa) * (size_t)p.c_in * p.c_out;
+      for (int c0 = 0; c0 < p.n_pad; c0 += 16) {
         uint32_t v[16];
-        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * buf_cols + (uint32_t)c0;
+        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * p.buf_cols + (uint32_t)c0;
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
@@ -283,10 +310,10 @@ conv_wgrad_tc_kernel(const float *__restrict__ features, int c_in, const float *
             : "r"(taddr)
             : "memory");
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (co < c_out) {
+        if (co < p.c_out) {
 #pragma unroll
           for (int k = 0; k < 16; ++k)
-            if (c0 + k < c_in) dst[(size_t)(c0 + k) * c_out + co] = __uint_as_float(v[k]);  // lanes = consecutive co: coalesced
+            if (c0 + k < p.c_in) dst[(size_t)(c0 + k) * p.c_out + co] = __uint_as_float(v[k]);  // lanes = consecutive co: coalesced
         }
       }
       tc_fence_before();
@@ -297,8 +324,8 @@ conv_wgrad_tc_kernel(const float *__restrict__ features, int c_in, const float *
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && *abort_flag && status) atomicOr(status, 16);
-  if (warp == WT_MMA_WARP) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(buf_cols * (uint32_t)n_buf) : "memory");
+  if (warp == mma_warp) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.buf_cols * (uint32_t)p.n_buf) : "memory");
   }
 }
 
@@ -344,22 +371,33 @@ conv_wgrad_small_kernel(const float *__restrict__ features, int c_in, const floa
   }
 }
 
-// d_filters[kappa] = sum of the offset's partials in ascending order of shares.  grid (elements / 256, K).
+// d_filters[kappa] = sum of the offset's partials, in a fixed order.  grid (elements / 32, K), block 32 elements x
+// 8 slices: slice s adds every eighth share (the centre offset has most of them), the slices are added
+// one after the other.
 __global__ void __launch_bounds__(256)
 wgrad_reduce_shares_kernel(const float *__restrict__ partial, const int32_t *__restrict__ starts, int K, int shares, int elems,
                            float *__restrict__ out) {
   __shared__ int first[257];
+  __shared__ float sm[8][33];
   chunk_prefix(starts, K, first);
-  const int kappa = blockIdx.y, e = blockIdx.x * 256 + threadIdx.x, total = first[K];
-  if (e >= elems) return;
+  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+  const int kappa = blockIdx.y, e = blockIdx.x * 32 + lane, total = first[K];
   float s = 0.f;
-  if (first[kappa + 1] > first[kappa]) {
+  if (e < elems && first[kappa + 1] > first[kappa]) {
     const int lo = share_of(first[kappa], total, shares), hi = share_of(first[kappa + 1] - 1, total, shares);
-    const float *p = partial + ((size_t)lo + kappa) * elems + e;
-#pragma unroll 8
-    for (int b = lo; b <= hi; ++b, p += elems) s += share_begin(b + 1, total, shares) > share_begin(b, total, shares) ? __ldg(p) : 0.f;
+    const bool gaps = total < shares;            // shares without a chunk wrote nothing
+    const float *p = partial + ((size_t)lo + slice + kappa) * elems + e;
+#pragma unroll 4
+    for (int b = lo + slice; b <= hi; b += 8, p += (size_t)8 * elems)
+      if (!gaps || share_begin(b + 1, total, shares) > share_begin(b, total, shares)) s += __ldg(p);
   }
-  out[(size_t)kappa * elems + e] = s;
+  sm[slice][lane] = s;
+  __syncthreads();
+  if (slice == 0 && e < elems) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) s += sm[k][lane];
+    out[(size_t)kappa * elems + e] = s;
+  }
 }
 
 size_t pair_lists_bytes(int K, int n_out) {
@@ -417,7 +455,7 @@ int pair_lists_build(const int32_t *nbr, int K, int n_out, void *lists, PairList
 // Shapes and shares of the two list kernels.
 struct WgradPlan {
   bool tc, small;
-  int n_pad, n_buf, co_blocks, shares;
+  int n_pad, n_buf, co_blocks, shares, stages, a_bytes, stage_bytes;
   uint32_t buf_cols;
   size_t smem;
 };
@@ -428,15 +466,23 @@ static WgradPlan wgrad_plan(int K, int c_in, int c_out, int n_out, bool tf32) {
   const long long most = (long long)K * ceil_div(n_out > 0 ? n_out : 1, WT_K);
   if (tf32) {
     p.n_pad = (c_in + 15) & ~15;
-    p.smem = (size_t)WT_STAGES * (WT_A_BYTES + p.n_pad * 128) + 1024 + 256;
-    if (p.n_pad > 256 || p.smem > 227 * 1024) return p;
+    if (p.n_pad > 256) return p;
     p.tc = true;
     p.buf_cols = 32;
     while ((int)p.buf_cols < p.n_pad) p.buf_cols <<= 1;
-    // two CTAs per SM (tensor memory: 512 columns) where their rings fit; two accumulator buffers each where the columns allow
-    const int ctas = p.smem <= 112 * 1024 ? 2 : 1;
-    p.n_buf = (int)p.buf_cols * 2 * ctas <= 512 ? 2 : 1;
     p.co_blocks = ceil_div(c_out, WT_M);
+    // The 128 rows of an MMA are always read: channels that do not exist come from whatever lies behind the
+    // operand's real blocks (the slack behind the last slot keeps that inside the buffer).
+    p.a_bytes = ceil_div(c_out < WT_M ? c_out : WT_M, 32) * WT_BLOCK;
+    p.stage_bytes = p.a_bytes + ceil_div(p.n_pad, 32) * WT_BLOCK;
+    // two CTAs per SM (tensor memory: 512 columns) where four slots fit each; two accumulator buffers where the columns allow
+    const size_t slack = 1024 + (size_t)4 * WT_BLOCK, fixed = 2048;
+    const int ctas = 4 * (size_t)p.stage_bytes + slack + fixed <= 113 * 1024 ? 2 : 1;
+    p.stages = (int)(((ctas == 2 ? 113 : 226) * 1024 - slack - fixed) / p.stage_bytes);
+    if (p.stages > WT_MAX_STAGES) p.stages = WT_MAX_STAGES;
+    if (p.stages < 2) { p.tc = false; return p; }
+    p.smem = (size_t)p.stages * p.stage_bytes + slack;
+    p.n_buf = (int)p.buf_cols * 2 * ctas <= 512 ? 2 : 1;
     p.shares = ctas * sm_count() / p.co_blocks;
   } else {
     if (c_in > 16) return p;
@@ -455,15 +501,17 @@ size_t conv_wgrad_lists_partial_bytes(int K, int c_in, int c_out, int n_out, boo
   return (p.tc || p.small) ? (size_t)(p.shares + K) * c_in * c_out * sizeof(float) : 0;
 }
 
-// returns -1 when the shape is not covered (the caller then uses the CUDA-core kernel over the table)
+// staged: bit 0 / 1: features / out_grad are TF32 images (ssc_conv_stage: rows padded to a multiple of four floats).
+// Returns -1 when the shape is not covered (the caller then uses the CUDA-core kernel over the table).
 int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int c_out, const PairLists &pl, int K, int n_out,
-                     bool tf32, float *partial, float *d_filters, int32_t *status, cudaStream_t st) {
+                     bool tf32, int staged, float *partial, float *d_filters, int32_t *status, cudaStream_t st) {
   const WgradPlan p = wgrad_plan(K, c_in, c_out, n_out, tf32);
   if (p.tc) {
     cudaError_t e = cudaFuncSetAttribute(conv_wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_wgrad(tf32): smem attribute: %s", cudaGetErrorString(e));
-    { conv_wgrad_tc_kernel<<<dim3(p.shares, p.co_blocks), WT_THREADS, p.smem, st>>>(features, c_in, out_grad, c_out, pl.pair_out, pl.pair_in,
-                                                                                  pl.starts, K, p.n_pad, p.buf_cols, p.n_buf, partial, status); note_launches(1); }
+    const WtParams w = {features, out_grad, c_in, c_out, (staged & 1) ? (c_in + 3) & ~3 : c_in, (staged & 2) ? (c_out + 3) & ~3 : c_out,
+                        (staged & 1) ? 0 : 1, (staged & 2) ? 0 : 1, p.n_pad, p.a_bytes, p.stage_bytes, p.stages, p.n_buf, p.buf_cols};
+    { conv_wgrad_tc_kernel<<<dim3(p.shares, p.co_blocks), (p.stages + 5) * 32, p.smem, st>>>(w, pl.pair_out, pl.pair_in, pl.starts, K, partial, status); note_launches(1); }
     SSC_CHECK_LAUNCH("conv_wgrad_tc");
   } else if (p.small) {
     const dim3 grid(p.shares / 4, p.co_blocks);
@@ -475,7 +523,7 @@ int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int
     return -1;
   }
   const int elems = c_in * c_out;
-  { wgrad_reduce_shares_kernel<<<dim3(ceil_div(elems, 256), K), 256, 0, st>>>(partial, pl.starts, K, p.shares, elems, d_filters); note_launches(1); }
+  { wgrad_reduce_shares_kernel<<<dim3(ceil_div(elems, 32), K), 256, 0, st>>>(partial, pl.starts, K, p.shares, elems, d_filters); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_wgrad_reduce");
   return SSC_OK;
 }

@@ -304,6 +304,7 @@ def build_rulebook(indices, batch_size, out_shape, spatial_shape, ksize, stride,
         nbr = torch.empty((K, n_in), dtype=torch.int32, device=dev)
         _check(L.ssc_rulebook_subm(_p(indices), n_in, int(batch_size), _i3(spatial_shape), _i3(ksize), _i3(dilation),
                                    _p(nbr), _p(pairs), _p(num), _p(st), _p(scratch), scratch.numel(), _stream()))
+        nbr._ssc_symmetric = all(int(k) == 1 or (int(k) % 2 == 1 and int(d) == 1) for k, d in zip(ksize, dilation))
         return indices, nbr, pairs, num
     n_out_dev = small[K:]
     geo = (_i3(spatial_shape), _i3(out_shape), _i3(ksize), _i3(stride), _i3(padding), _i3(dilation), int(transpose))
@@ -655,6 +656,7 @@ def pair_lists(nbr):
 
 PRESTAGED = 0x100
 TABLE_IN_ORDER = 0x200
+WGRAD_X_STAGED, WGRAD_DY_STAGED = 0x400, 0x800
 # (features.data_ptr(), filters.data_ptr()) -> (prec, packed, scratch, nbytes) left by conv_prepare for the
 # conv_forward call that follows on the same tensors
 _prepared = {}
@@ -721,12 +723,13 @@ def conv_prepare(features, filters, precision=None):
 
 
 def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, row_order=None, algo=None,
-                 table_in_order=False):
+                 table_in_order=False, image=None):
     """out [n_out, Cout] = sum over offsets of gathered rows times filters (one launch).
     n_out_dev: device word with the exact row count when n_out is only a capacity.
     row_order: permutation of the output rows from nbr_row_order (same result, fewer steps).
     table_in_order: nbr is the table with its columns already in that order (nbr_row_order_planes).
-    algo: None (the module setting), 'rows' or 'pairs' (see set_algo)."""
+    algo: None (the module setting), 'rows' or 'pairs' (see set_algo).
+    image: the features' TF32 image (stage_tf32) where the caller has one already."""
     if filters.dim() != 3:
         filters = filters.reshape(-1, filters.shape[-2], filters.shape[-1])
     K, c_in, c_out = filters.shape
@@ -752,6 +755,8 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
     if _prepared:   # only the call that directly follows conv_prepare may use what it left
         ready = _prepared.pop((features.data_ptr(), filters.data_ptr()), None)
         _prepared.clear()
+    if image is not None and mode == "tf32":
+        ready = (PREC_TF32, _packed_filters(filters, PREC_TF32), image, image.numel())
     if ready is not None and ready[0] == _PREC_OF.get(mode, -1):
         prec, packed, scratch, nbytes = ready
         _check(lib().ssc_conv_fwd_ordered(_p(features, torch.float32), features.shape[0], c_in, _p(packed), K, c_out,
@@ -911,9 +916,19 @@ def nbr_row_order(nbr):
     return order
 
 
-def conv_wgrad(features, out_grad, nbr, precision=None):
+def stage_tf32(rows):
+    """The TF32 operand image of fp32 rows [n, C] (ssc_conv_stage): a flat byte buffer."""
+    n, c = rows.shape
+    nbytes = int(lib().ssc_conv_scratch_bytes(n, c, c, PREC_TF32))
+    image = torch.empty(nbytes, dtype=torch.uint8, device=rows.device)
+    _check(lib().ssc_conv_stage(_p(rows, torch.float32), n, c, PREC_TF32, _p(image), nbytes, _stream()))
+    return image
+
+
+def conv_wgrad(features, out_grad, nbr, precision=None, x_image=None, dy_image=None):
     """d_filters [K, Cin, Cout] = sum over output rows of gathered input rows (outer) out_grad rows
-    (tensor cores with TF32 operands or exact fp32, chosen like the forward pass)."""
+    (tensor cores with TF32 operands or exact fp32, chosen like the forward pass).  x_image / dy_image:
+    the operands' TF32 images (stage_tf32) where the caller has them."""
     K, n_out = nbr.shape
     c_in, c_out = features.shape[1], out_grad.shape[1]
     # the filter gradient has no 16-bit form: 'fp16' / 'bf16' take the TF32 kernel
@@ -922,9 +937,15 @@ def conv_wgrad(features, out_grad, nbr, precision=None):
     nbytes = int(lib().ssc_conv_wgrad_scratch_bytes(K, c_in, c_out, n_out))
     scratch = torch.empty(max(nbytes, 4), dtype=torch.uint8, device=features.device)
     lists = pair_lists(nbr) if n_out > 0 and (mode == PREC_TF32 or c_in <= 16) else None
-    _check(lib().ssc_conv_wgrad_lists(_p(features, torch.float32), c_in, _p(out_grad, torch.float32), c_out,
-                                      _p(nbr, torch.int32), K, n_out, _p(lists), lists.numel() if lists is not None else 0,
-                                      mode, _p(d_flt), _p(status_word(features.device)), _p(scratch), nbytes, _stream()))
+    x, dy = _p(features, torch.float32), _p(out_grad, torch.float32)
+    if mode == PREC_TF32 and c_in <= 256:
+        if x_image is not None:
+            x, mode = _p(x_image), mode | WGRAD_X_STAGED
+        if dy_image is not None:
+            dy, mode = _p(dy_image), mode | WGRAD_DY_STAGED
+    _check(lib().ssc_conv_wgrad_lists(x, c_in, dy, c_out, _p(nbr, torch.int32), K, n_out, _p(lists),
+                                      lists.numel() if lists is not None else 0, mode, _p(d_flt),
+                                      _p(status_word(features.device)), _p(scratch), nbytes, _stream()))
     return d_flt
 
 
@@ -933,36 +954,45 @@ def conv_backward(features, flt, out_bp, nbr, nbr_in=None, order=None, precision
     over the table nbr [K, n_out].  nbr_in / order: the input-major table and its row order when the
     caller kept them with the rulebook (built here otherwise).  need: which of the two are asked for (a
     first layer's input needs none); None is returned for the other."""
-    n_in = features.shape[0]
-    if not need[0]:
-        return None, conv_wgrad(features, out_bp, nbr, precision) if need[1] else None
+    n_in, (c_in, c_out) = features.shape[0], flt.shape[1:]
+    # both gradients read the output gradient as TF32 rows: rounded once
+    tf32_in = need[0] and _resolve_precision(c_out, c_in, precision) == "tf32" and not _use_pairs(
+        flt.shape[0], c_out, c_in, n_in, PREC_TF32)
+    tf32_flt = need[1] and c_in <= 256 and _resolve_precision(c_in, c_out, precision) in _PREC_OF
+    dy_image = stage_tf32(out_bp) if (tf32_in or tf32_flt) and out_bp.shape[0] >= STAGING_MIN_ROWS else None
     # the two gradients do not depend on each other: while a graph is recorded the filter gradient
     # goes to a side stream, so the graph runs it next to the input gradient
-    forked = need[1] and torch.cuda.is_current_stream_capturing()
+    forked = need[0] and need[1] and torch.cuda.is_current_stream_capturing()
+    d_in = d_flt = None
     if forked:
         cur, side = torch.cuda.current_stream(features.device), side_stream(features.device)
         side.wait_stream(cur)
         with torch.cuda.stream(side):
-            d_flt = conv_wgrad(features, out_bp, nbr, precision)
-    if nbr_in is None:
-        kept = getattr(nbr, "_ssc_in_major", None)     # layers that share a rulebook share these too
-        if kept is not None and kept[0] == n_in:
-            nbr_in, order = kept[1], kept[2]
-        else:
-            nbr_in = input_major_table(nbr, n_in)
-            # rows of the input-major table use few of the offsets each (their parity class under a
-            # stride): grouped tiles skip the rest
-            order = nbr_row_order(nbr_in) if (n_in >= ROW_ORDER_MIN_ROWS and nbr_in.shape[0] > 1) else None
-            if not torch.cuda.is_current_stream_capturing():   # tensors made while a graph is recorded belong to the graph
-                try:
-                    nbr._ssc_in_major = (n_in, nbr_in, order)
-                except Exception:
-                    pass
-    d_in = conv_forward(out_bp, flt.transpose(1, 2).contiguous(), nbr_in, n_in, precision, row_order=order)
+            d_flt = conv_wgrad(features, out_bp, nbr, precision, dy_image=dy_image)
+    if need[0]:
+        if nbr_in is None and getattr(nbr, "_ssc_symmetric", False) and n_in == nbr.shape[1]:
+            # a submanifold table with a centred kernel is its own transpose with the offsets reversed
+            nbr_in, flt = nbr, flt.flip(0)
+        elif nbr_in is None:
+            kept = getattr(nbr, "_ssc_in_major", None)     # layers that share a rulebook share these too
+            if kept is not None and kept[0] == n_in:
+                nbr_in, order = kept[1], kept[2]
+            else:
+                nbr_in = input_major_table(nbr, n_in)
+                # rows of the input-major table use few of the offsets each (their parity class under a
+                # stride): grouped tiles skip the rest
+                order = nbr_row_order(nbr_in) if (n_in >= ROW_ORDER_MIN_ROWS and nbr_in.shape[0] > 1) else None
+                if not torch.cuda.is_current_stream_capturing():   # tensors made while a graph is recorded belong to it
+                    try:
+                        nbr._ssc_in_major = (n_in, nbr_in, order)
+                    except Exception:
+                        pass
+        d_in = conv_forward(out_bp, flt.transpose(1, 2).contiguous(), nbr_in, n_in, precision, row_order=order,
+                            image=dy_image if tf32_in else None)
     if forked:
         cur.wait_stream(side)
-    else:
-        d_flt = conv_wgrad(features, out_bp, nbr, precision) if need[1] else None
+    elif need[1]:
+        d_flt = conv_wgrad(features, out_bp, nbr, precision, dy_image=dy_image)
     return d_in, d_flt
 
 
