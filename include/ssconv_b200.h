@@ -322,6 +322,9 @@ int ssc_nbr_row_order_planes(const int32_t *nbr, const int ksize[3], int n_rows,
 /* OR'ed into `precision` of ssc_conv_fwd_ordered: `nbr` is the table in the order of `row_order`
  * (nbr_in_order above), i.e. column j belongs to output row row_order[j]. */
 #define SSC_CONV_TABLE_IN_ORDER 0x200
+/* OR'ed into `precision`: the neighbours at kernel offset kappa stand in row K - 1 - kappa of `nbr`: the
+ * input-major table of a submanifold table with a centred kernel (odd extents, dilation 1), as it is. */
+#define SSC_CONV_TABLE_REVERSED 0x1000
 int ssc_conv_fwd_ordered(const float *features, int n_in, int c_in, const void *filters, int K, int c_out,
                          const int32_t *nbr, int n_out, int precision, float *out, int32_t *status,
                          void *scratch, size_t scratch_bytes, const int32_t *n_out_dev,

@@ -259,88 +259,97 @@ static bool launch_bn_gate_rows(const float *x, int n, uint32_t groups, int c_in
 }
 
 // ---------------------------------------------------------------- batch statistics, training mode
-// Column sums over the rows, deterministic: thread = (group of VEC channels, row lane), a block strides over
-// the rows, its lanes are added in shared memory in a fixed order and one partial row per block goes
-// to part[block][channel]; a second small kernel adds the partials of a field (block per field, fixed
-// tree).  HBM-bound: 16 bytes per thread and row, two blocks per SM.  MODE 0: sum of x;
-// 1: sum of (x - mean_ch)^2.
-constexpr int kStatThreads = 256;
+// Column sums over the rows in an order that depends on the row count alone: rows L, L + chains, L + 2 chains ...
+// form chain L of a channel (chains = 8 per row block, at most 512), added one after the other; the
+// eight chains of a row block are added in order, then the row blocks, then the channels of a field.
+// Batch statistics therefore repeat bit for bit, whatever grid or load width computes them.
+// A thread walks one chain of VEC channels with sixteen loads in flight; HBM- or L2-bound.
+// MODE 0: sum of x; 1: sum of (x - mean_ch)^2.  part [chains][c].
+static int bn_row_blocks(int n) {
+  const int rb = ceil_div(n, 8 * 64);
+  return rb > 64 ? 64 : (rb < 1 ? 1 : rb);
+}
 template <int MODE, int VEC>
-__global__ void __launch_bounds__(kStatThreads)
-bn_colsum_kernel(const float *__restrict__ x, int n, int c, int lanes, const float *__restrict__ chan_mean, float *__restrict__ part) {
-  __shared__ float sm[kStatThreads * VEC];
+__global__ void __launch_bounds__(256)
+bn_colsum_kernel(const float *__restrict__ x, int n, int c, int chains, int lanes, const float *__restrict__ chan_mean,
+                 float *__restrict__ part) {
   const int groups = c / VEC;
-  for (int g0 = 0; g0 < groups; g0 += kStatThreads / lanes) {   // one pass unless the row is wider than the block
-    const int gw = min(kStatThreads / lanes, groups - g0);
-    const int g = threadIdx.x % (kStatThreads / lanes), lane = threadIdx.x / (kStatThreads / lanes);
-    const bool on = g < gw && lane < lanes;
+  const int lane = threadIdx.x / (blockDim.x / lanes), chain = blockIdx.x * lanes + lane;
+  if (lane >= lanes || chain >= chains) return;
+  for (int g = threadIdx.x % (blockDim.x / lanes); g < groups; g += blockDim.x / lanes) {
+    const float *p = x + (size_t)chain * c + (size_t)g * VEC;
+    const size_t step = (size_t)chains * c;
     float s[VEC], mu[VEC];
 #pragma unroll
     for (int q = 0; q < VEC; ++q) {
       s[q] = 0.f;
-      mu[q] = (MODE != 0 && on) ? chan_mean[(g0 + g) * VEC + q] : 0.f;
+      mu[q] = MODE != 0 ? chan_mean[g * VEC + q] : 0.f;
     }
-    if (on) {
-#pragma unroll 4
-      for (int r = blockIdx.x * lanes + lane; r < n; r += gridDim.x * lanes) {
-        const float *p = x + (size_t)r * c + (size_t)(g0 + g) * VEC;
-        float v[VEC];
-        if (VEC == 4) {
-          const float4 f = __ldg((const float4 *)p);
-          v[0] = f.x; v[1 % VEC] = f.y; v[2 % VEC] = f.z; v[3 % VEC] = f.w;
-        } else {
-          v[0] = __ldg(p);
-        }
-#pragma unroll
-        for (int q = 0; q < VEC; ++q) {
-          const float d = v[q] - mu[q];
-          s[q] = MODE == 0 ? s[q] + d : fmaf(d, d, s[q]);
-        }
+#pragma unroll 16
+    for (int r = chain; r < n; r += chains, p += step) {
+      float v[VEC];
+      if (VEC == 4) {
+        const float4 f = __ldg((const float4 *)p);
+        v[0] = f.x; v[1 % VEC] = f.y; v[2 % VEC] = f.z; v[3 % VEC] = f.w;
+      } else {
+        v[0] = __ldg(p);
       }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < VEC; ++q) sm[threadIdx.x * VEC + q] = s[q];
-    __syncthreads();
-    if (lane == 0 && g < gw) {
 #pragma unroll
       for (int q = 0; q < VEC; ++q) {
-        float a = s[q];
-        for (int l = 1; l < lanes; ++l) a += sm[(threadIdx.x + l * (kStatThreads / lanes)) * VEC + q];
-        part[(size_t)blockIdx.x * c + (g0 + g) * VEC + q] = a;
+        const float d = v[q] - mu[q];
+        s[q] = MODE == 0 ? s[q] + d : fmaf(d, d, s[q]);
       }
     }
+#pragma unroll
+    for (int q = 0; q < VEC; ++q) part[(size_t)chain * c + g * VEC + q] = s[q];
   }
 }
 
-// Sum of a column of partials by one block, in a fixed order; every thread gets the result.
+// Sum of the chains of `count` consecutive channels from ch0, by one block, in the order stated above: the
+// row blocks' sums of eight chains in parallel, then one thread adds them up.  Result in every thread.
 constexpr int kFinishThreads = 128;
-__device__ __forceinline__ float column_total(const float *__restrict__ part, int n_part, int c, int ch) {
-  __shared__ float sm[kFinishThreads / 32];
+constexpr int kFinishTile = 16 * 64;       // (channel, row block) sums in shared memory at a time
+__device__ __forceinline__ float chain_total(const float *__restrict__ part, int row_blocks, int c, int ch0, int count) {
+  __shared__ float sm[kFinishTile];
+  __shared__ float result;
   float s = 0.f;
-  for (int i = threadIdx.x; i < n_part; i += kFinishThreads) s += part[(size_t)i * c + ch];
+  for (int k0 = 0; k0 < count; k0 += 16) {
+    const int m = min(16, count - k0) * row_blocks;
+    for (int i = threadIdx.x; i < m; i += kFinishThreads) {
+      const int k = i / row_blocks, rb = i - k * row_blocks;
+      const float *p = part + (size_t)rb * 8 * c + ch0 + k0 + k;
+      float v[8];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
-  __syncthreads();
-  s = sm[0];
+      for (int t = 0; t < 8; ++t) v[t] = __ldg(p + (size_t)t * c);
 #pragma unroll
-  for (int w = 1; w < kFinishThreads / 32; ++w) s += sm[w];
+      for (int t = 1; t < 8; ++t) v[0] += v[t];
+      sm[i] = v[0];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll 16
+      for (int i = 0; i < m; ++i) s += sm[i];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) result = s;
+  __syncthreads();
+  s = result;
+  __syncthreads();
   return s;
 }
 
 // Block per channel: batch mean of the scalar channels (0 for the others), running mean updated with the
 // arithmetic of running.mul_(1 - m).add_(m * mean).
 __global__ void __launch_bounds__(kFinishThreads)
-bn_finish_mean_kernel(const float *__restrict__ part, int n_part, int n, int c, const int32_t *__restrict__ scalar_of_channel,
+bn_finish_mean_kernel(const float *__restrict__ part, int row_blocks, int n, int c, const int32_t *__restrict__ scalar_of_channel,
                       float momentum, float keep, float *running_mean, float *mean, float *chan_mean) {
   const int ch = blockIdx.x, s = scalar_of_channel[ch];
   if (s < 0) {
     if (threadIdx.x == 0) chan_mean[ch] = 0.f;
     return;
   }
-  const float mu = column_total(part, n_part, c, ch) / (float)n;
+  const float mu = chain_total(part, row_blocks, c, ch, 1) / (float)n;
   if (threadIdx.x == 0) {
     chan_mean[ch] = mu;
     mean[s] = mu;
@@ -361,30 +370,30 @@ __device__ __forceinline__ int2 field_channels(const int32_t *__restrict__ field
 
 // Block per field: mean squared norm, running value, and (scale != NULL) the per-channel affine of the pass.
 __global__ void __launch_bounds__(kFinishThreads)
-bn_finish_var_kernel(const float *__restrict__ part, int n_part, int n, int c, const int32_t *__restrict__ field_of_channel,
+bn_finish_var_kernel(const float *__restrict__ part, int row_blocks, int n, int c, const int32_t *__restrict__ field_of_channel,
                      const int32_t *__restrict__ scalar_of_channel, const float *__restrict__ chan_mean,
                      const float *__restrict__ weight, const float *__restrict__ bias, float eps, float momentum, float keep,
                      float *running_var, float *var, float *scale, float *shift) {
   const int f = blockIdx.x;
   const int2 fc = field_channels(field_of_channel, c, f);
-  float s = 0.f;
-  for (int k = 0; k < fc.y; ++k) s += column_total(part, n_part, c, fc.x + k);
-  const float v = s / (float)n;
+  const float v = chain_total(part, row_blocks, c, fc.x, fc.y) / (float)n;
   if (threadIdx.x == 0) {
     var[f] = v;
     if (running_var) running_var[f] = __fadd_rn(__fmul_rn(running_var[f], keep), __fmul_rn(momentum, v));
   }
-  if (scale && threadIdx.x < fc.y) {
-    const int ch = fc.x + threadIdx.x, sc_i = scalar_of_channel[ch];
-    float sc = 1.0f / sqrtf(v + eps), sh = 0.f;
-    if (weight) sc *= weight[f];
-    if (sc_i >= 0) {
-      sh = -chan_mean[ch] * sc;
-      if (bias) sh += bias[sc_i];
+  if (scale)
+    for (int k = threadIdx.x; k < fc.y; k += kFinishThreads) {
+      const int ch = fc.x + k, sc_i = scalar_of_channel[ch];
+      float sc = 1.0f / sqrtf(v + eps), sh = 0.f;
+      if (weight) sc *= weight[f];
+      if (sc_i >= 0) {
+        // the roundings of bn_fold_kernel, so that a fold of the same statistics gives the same bits
+        sh = __fmul_rn(-chan_mean[ch], sc);
+        if (bias) sh = __fadd_rn(sh, bias[sc_i]);
+      }
+      scale[ch] = sc;
+      shift[ch] = sh;
     }
-    scale[ch] = sc;
-    shift[ch] = sh;
-  }
 }
 
 // ------------------------------------------- backward of batch norm and gated activation, one pair of passes
@@ -398,20 +407,20 @@ bn_finish_var_kernel(const float *__restrict__ part, int n_part, int n, int c, c
 //   ks = r w, ka = w r^3 A / N, kg = r w G / N (ka = kg = 0 with running statistics).
 // y and g are recomputed from x and go in both passes (PASS 0 adds up A and G, PASS 1 writes gx), so neither
 // is ever stored: 2 reads of x and go and one write of gx per backward, instead of four tensors more.
-// A block takes R whole rows at a time into shared memory (rows are contiguous: a straight copy), evaluates
-// every gate once, then walks the channels.  Without a gate table g = go (batch norm alone); without ks
-// gx = g (activation alone).  HBM-bound.
+// A block takes R whole rows at a time into shared memory, evaluates every gate once, then walks the
+// channels.  PASS 0: block = one chain of rows (the order of the sums is that of the batch statistics
+// above), thread = channels.  PASS 1: R consecutive rows (a straight copy).  Without a gate table g = go
+// (batch norm alone); without ks gx = g (activation alone).  HBM-bound.
 struct BnGateBwd {
   const float *x, *go;
-  int n, c, c_out, n_gates, rows;              // rows = R
+  int n, c, c_out, n_gates, rows, chains;      // rows = R
   const float *scale, *shift, *mu;             // per channel (may be NULL: identity / zero)
   const int32_t *gate_of_channel, *field_start, *field_len;
   int s_act, g_act;
   int vec;                                     // both row lengths and pointers allow 16-byte copies
 };
 
-constexpr int kBwdThreads = 256;
-constexpr int kBwdMaxAcc = 8;                  // channels of a thread: a block covers up to 2048
+constexpr int kBwdMaxAcc = 4;                  // channels of a thread in PASS 0
 
 __device__ __forceinline__ float act_grad(float v, int kind) {
   if (kind == 1) return v > 0.f ? 1.f : 0.f;
@@ -423,33 +432,53 @@ __device__ __forceinline__ float act_grad(float v, int kind) {
 }
 
 template <int PASS>
-__global__ void __launch_bounds__(kBwdThreads)
+__global__ void __launch_bounds__(256)
 bn_gate_bwd_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
                    float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
   extern __shared__ __align__(16) float sm[];
   float *xs = sm, *gs = xs + (size_t)p.rows * p.c, *as = gs + (size_t)p.rows * p.c_out, *gg = as + (size_t)p.rows * p.n_gates;
-  const int tid = threadIdx.x;
-  // channels over threads; rows of the tile over the lanes that are left when the row is short
-  const int lanes = p.c >= kBwdThreads ? 1 : kBwdThreads / p.c;
-  const int ch_step = p.c >= kBwdThreads ? kBwdThreads : p.c;
-  const int ch_block = (int)blockIdx.y * kBwdThreads * kBwdMaxAcc;     // (only rows of more than 2048 channels have a second one)
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int row_step = PASS == 0 ? p.chains : 1;                 // distance of a tile's rows
+  const int first = PASS == 0 ? (int)blockIdx.x : (int)blockIdx.x * p.rows;
+  const int tile_step = PASS == 0 ? p.rows * p.chains : (int)gridDim.x * p.rows;
+  // PASS 1: channels over threads, rows of the tile over the lanes that are left when the row is short
+  const int lanes = PASS == 0 || p.c >= nt ? 1 : nt / p.c;
+  const int ch_step = p.c >= nt || PASS == 0 ? nt : p.c;
+  const int ch_block = PASS == 0 ? (int)blockIdx.y * nt * kBwdMaxAcc : 0;
   const int ch_first = ch_block + tid % ch_step, lane = tid / ch_step;
   float sum_a[kBwdMaxAcc], sum_g[kBwdMaxAcc];
 #pragma unroll
   for (int i = 0; i < kBwdMaxAcc; ++i) sum_a[i] = sum_g[i] = 0.f;
-  for (int r0 = blockIdx.x * p.rows; r0 < p.n; r0 += gridDim.x * p.rows) {
-    const int rows = min(p.rows, p.n - r0);
-    const float *xg = p.x + (size_t)r0 * p.c, *gg0 = p.go + (size_t)r0 * p.c_out;
+  for (int r0 = first; r0 < p.n; r0 += tile_step) {
+    const int rows = min(p.rows, (p.n - r0 + row_step - 1) / row_step);
     if (p.vec) {
-      for (int i = tid; i < rows * p.c / 4; i += kBwdThreads) ((float4 *)xs)[i] = __ldg((const float4 *)xg + i);
-      for (int i = tid; i < rows * p.c_out / 4; i += kBwdThreads) ((float4 *)gs)[i] = __ldg((const float4 *)gg0 + i);
+      const int cx = p.c >> 2, cg = p.c_out >> 2;
+      if (PASS == 1) {
+        for (int i = tid; i < rows * cx; i += nt) ((float4 *)xs)[i] = __ldg((const float4 *)(p.x + (size_t)r0 * p.c) + i);
+        for (int i = tid; i < rows * cg; i += nt) ((float4 *)gs)[i] = __ldg((const float4 *)(p.go + (size_t)r0 * p.c_out) + i);
+      } else {
+        for (int i = tid; i < rows * cx; i += nt) {
+          const int r = i / cx;
+          ((float4 *)xs)[i] = __ldg((const float4 *)(p.x + (size_t)(r0 + r * row_step) * p.c) + (i - r * cx));
+        }
+        for (int i = tid; i < rows * cg; i += nt) {
+          const int r = i / cg;
+          ((float4 *)gs)[i] = __ldg((const float4 *)(p.go + (size_t)(r0 + r * row_step) * p.c_out) + (i - r * cg));
+        }
+      }
     } else {
-      for (int i = tid; i < rows * p.c; i += kBwdThreads) xs[i] = __ldg(xg + i);
-      for (int i = tid; i < rows * p.c_out; i += kBwdThreads) gs[i] = __ldg(gg0 + i);
+      for (int i = tid; i < rows * p.c; i += nt) {
+        const int r = i / p.c;
+        xs[i] = __ldg(p.x + (size_t)(r0 + r * row_step) * p.c + (i - r * p.c));
+      }
+      for (int i = tid; i < rows * p.c_out; i += nt) {
+        const int r = i / p.c_out;
+        gs[i] = __ldg(p.go + (size_t)(r0 + r * row_step) * p.c_out + (i - r * p.c_out));
+      }
     }
     __syncthreads();
     if (p.n_gates > 0) {
-      for (int i = tid; i < rows * p.n_gates; i += kBwdThreads) {
+      for (int i = tid; i < rows * p.n_gates; i += nt) {
         const int r = i / p.n_gates, j = i - r * p.n_gates;
         const float *xr = xs + r * p.c, *gr = gs + r * p.c_out;
         const int cg = p.c_out + j;
@@ -460,79 +489,97 @@ bn_gate_bwd_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__res
         for (int q = 0; q < len; ++q) {
           float y = xr[s0 + q];
           if (p.scale) y = fmaf(y, p.scale[s0 + q], p.shift[s0 + q]);
-          acc += gr[s0 + q] * y;
+          acc = fmaf(gr[s0 + q], y, acc);
         }
         as[i] = apply_act(v, p.g_act);
         gg[i] = acc * act_grad(v, p.g_act);
       }
       __syncthreads();
     }
-    if (lane < lanes) {
+    // g of a channel of a row; its gate's value and the gate scalars' gradients stand in shared memory
+    auto gradient = [&](int r, int ch, int gate, float x, float sc, float sh) -> float {
+      if (gate == -3) return gg[r * p.n_gates + ch - p.c_out];
+      float g = gs[r * p.c_out + ch];
+      if (gate == -1) g *= act_grad(p.scale ? fmaf(x, sc, sh) : x, p.s_act);
+      else if (gate >= 0) g *= as[r * p.n_gates + gate];
+      return g;
+    };
+    if (PASS == 0) {
+      // all threads turn go into g in place, then a thread adds up the rows of its channels in order: the
+      // chain is two shared-memory loads and two additions per row
+      if (p.gate_of_channel) {
+        const int per = p.c_out >= nt ? 1 : nt / p.c_out, step = p.c_out >= nt ? nt : p.c_out;
+        if (tid / step < per)
+          for (int ch = tid % step; ch < p.c_out; ch += step) {
+            const int gate = p.gate_of_channel[ch];
+            if (gate < -1) continue;
+            const float sc = p.scale ? p.scale[ch] : 1.f, sh = p.scale ? p.shift[ch] : 0.f;
+            for (int r = tid / step; r < rows; r += per) gs[r * p.c_out + ch] = gradient(r, ch, gate, xs[r * p.c + ch], sc, sh);
+          }
+        __syncthreads();
+      }
 #pragma unroll
       for (int i = 0; i < kBwdMaxAcc; ++i) {
         const int ch = ch_first + i * ch_step;
-        if (ch >= p.c || (i > 0 && p.c < kBwdThreads)) break;
+        if (ch < p.c) {
+          const float mu = p.mu ? p.mu[ch] : 0.f;
+          const float *gp = ch < p.c_out ? gs + ch : gg + (ch - p.c_out), *xp = xs + ch;
+          const int gstep = ch < p.c_out ? p.c_out : p.n_gates;
+          float s = sum_g[i], a = sum_a[i];
+#pragma unroll 8
+          for (int r = 0; r < rows; ++r) {
+            const float g = gp[r * gstep];
+            s += g;
+            a = fmaf(g, xp[r * p.c] - mu, a);
+          }
+          sum_g[i] = s;
+          sum_a[i] = a;
+        }
+      }
+    } else if (lane < lanes) {
+      for (int ch = ch_first; ch < p.c; ch += ch_step) {
         const float mu = p.mu ? p.mu[ch] : 0.f;
         const float sc = p.scale ? p.scale[ch] : 1.f, sh = p.scale ? p.shift[ch] : 0.f;
         const int gate = p.gate_of_channel ? (ch < p.c_out ? p.gate_of_channel[ch] : -3) : -2;
-        const float k_s = (PASS == 1 && ks) ? ks[ch] : 1.f, k_a = (PASS == 1 && ks) ? ka[ch] : 0.f, k_g = (PASS == 1 && ks) ? kg[ch] : 0.f;
+        const float k_s = ks ? ks[ch] : 1.f, k_a = ks ? ka[ch] : 0.f, k_g = ks ? kg[ch] : 0.f;
+#pragma unroll 4
         for (int r = lane; r < rows; r += lanes) {
           const float x = xs[r * p.c + ch];
-          float g;
-          if (gate == -3) g = gg[r * p.n_gates + ch - p.c_out];
-          else {
-            g = gs[r * p.c_out + ch];
-            if (gate == -1) g *= act_grad(p.scale ? fmaf(x, sc, sh) : x, p.s_act);
-            else if (gate >= 0) g *= as[r * p.n_gates + gate];
-          }
-          if (PASS == 0) {
-            sum_g[i] += g;
-            sum_a[i] = fmaf(g, x - mu, sum_a[i]);
-          } else {
-            gx[(size_t)(r0 + r) * p.c + ch] = ks ? k_s * g - k_a * (x - mu) - k_g : g;
-          }
+          const float g = gradient(r, ch, gate, x, sc, sh);
+          gx[(size_t)(r0 + r) * p.c + ch] = ks ? k_s * g - k_a * (x - mu) - k_g : g;
         }
+        if (p.c < nt) break;
       }
     }
     __syncthreads();
   }
   if (PASS == 0) {
-    // lanes of a channel are added in a fixed order (the tile's shared memory is free now)
+#pragma unroll
     for (int i = 0; i < kBwdMaxAcc; ++i) {
       const int ch = ch_first + i * ch_step;
-      if (i > 0 && p.c < kBwdThreads) break;
-      if (ch_block + i * ch_step >= p.c) break;
-      sm[tid] = sum_a[i];
-      sm[kBwdThreads + tid] = sum_g[i];
-      __syncthreads();
-      if (lane == 0 && ch < p.c) {
-        float a = sum_a[i], g = sum_g[i];
-        for (int l = 1; l < lanes; ++l) { a += sm[tid + l * ch_step]; g += sm[kBwdThreads + tid + l * ch_step]; }
-        part_a[(size_t)blockIdx.x * p.c + ch] = a;
-        part_g[(size_t)blockIdx.x * p.c + ch] = g;
+      if (ch < p.c) {
+        part_a[(size_t)blockIdx.x * p.c + ch] = sum_a[i];
+        part_g[(size_t)blockIdx.x * p.c + ch] = sum_g[i];
       }
-      __syncthreads();
     }
   }
 }
 
-// Block per field: A and G from the partials, the field's coefficients and parameter gradients.
+// Block per field: A and G from the chains, the field's coefficients and parameter gradients.
 __global__ void __launch_bounds__(kFinishThreads)
-bn_bwd_finish_kernel(const float *__restrict__ part_a, const float *__restrict__ part_g, int n_part, int n, int c,
+bn_bwd_finish_kernel(const float *__restrict__ part_a, const float *__restrict__ part_g, int row_blocks, int n, int c,
                      const int32_t *__restrict__ field_of_channel, const int32_t *__restrict__ scalar_of_channel,
                      const float *__restrict__ var, const float *__restrict__ weight, float eps, int training,
                      float *__restrict__ ks, float *__restrict__ ka, float *__restrict__ kg, float *__restrict__ d_weight,
                      float *__restrict__ d_bias) {
   const int f = blockIdx.x;
   const int2 fc = field_channels(field_of_channel, c, f);
-  float A = 0.f;
-  for (int k = 0; k < fc.y; ++k) A += column_total(part_a, n_part, c, fc.x + k);
+  const float A = chain_total(part_a, row_blocks, c, fc.x, fc.y);
   const int s = fc.y == 1 ? scalar_of_channel[fc.x] : -1;
-  float G = 0.f;
-  if (s >= 0) G = column_total(part_g, n_part, c, fc.x);
+  const float G = s >= 0 ? chain_total(part_g, row_blocks, c, fc.x, 1) : 0.f;
   const float r = 1.0f / sqrtf(var[f] + eps), w = weight ? weight[f] : 1.f;
-  if (threadIdx.x < fc.y) {
-    const int ch = fc.x + threadIdx.x;
+  for (int k = threadIdx.x; k < fc.y; k += kFinishThreads) {
+    const int ch = fc.x + k;
     ks[ch] = r * w;
     ka[ch] = training ? w * r * r * r * A / (float)n : 0.f;
     kg[ch] = (training && s >= 0) ? r * w * G / (float)n : 0.f;
@@ -639,29 +686,26 @@ extern "C" int ssc_bn_gate_fwd16(const float *x, int n, int c_in_total, const fl
   return SSC_OK;
 }
 
-// Blocks of the column-sum and backward kernels, each of which contributes one partial per channel:
-// four per SM, fewer when a block would not have a hundred rows to add.
-static int bn_row_blocks(int n) {
-  const int rb = ceil_div(n, 64), most = 4 * 148;
-  return rb > most ? most : (rb < 1 ? 1 : rb);
-}
-
 extern "C" size_t ssc_bn_scratch_bytes(int n, int c) {
   if (n < 0 || c < 1) return 0;
-  // two planes of partials [row blocks, c], per-channel mean and three coefficient rows
-  return ((size_t)2 * bn_row_blocks(n) * c + (size_t)4 * c + 64) * sizeof(float);
+  // two planes of chain sums [8 row blocks, c], per-channel mean and three coefficient rows
+  return ((size_t)2 * 8 * bn_row_blocks(n) * c + (size_t)4 * c + 64) * sizeof(float);
 }
 
-static int launch_colsum(int mode, const float *x, int n, int c, const float *chan_mean, float *part, int blocks, cudaStream_t st) {
+static int launch_colsum(int mode, const float *x, int n, int c, const float *chan_mean, float *part, cudaStream_t st) {
   const bool vec = (c & 3) == 0 && ((uintptr_t)x & 15u) == 0;
-  const int groups = vec ? c / 4 : c;
-  const int lanes = groups >= kStatThreads ? 1 : kStatThreads / groups;
+  const int groups = vec ? c / 4 : c, chains = 8 * bn_row_blocks(n);
+  // two blocks per SM where there are that many chains
+  int lanes = chains / (2 * 148);
+  if (lanes > 256 / groups) lanes = 256 / groups;
+  if (lanes < 1) lanes = 1;
+  const int threads = lanes * (groups < 256 ? groups : 256), blocks = ceil_div(chains, lanes);
   if (vec) {
-    if (mode == 0) bn_colsum_kernel<0, 4><<<blocks, kStatThreads, 0, st>>>(x, n, c, lanes, chan_mean, part);
-    else bn_colsum_kernel<1, 4><<<blocks, kStatThreads, 0, st>>>(x, n, c, lanes, chan_mean, part);
+    if (mode == 0) bn_colsum_kernel<0, 4><<<blocks, threads, 0, st>>>(x, n, c, chains, lanes, chan_mean, part);
+    else bn_colsum_kernel<1, 4><<<blocks, threads, 0, st>>>(x, n, c, chains, lanes, chan_mean, part);
   } else {
-    if (mode == 0) bn_colsum_kernel<0, 1><<<blocks, kStatThreads, 0, st>>>(x, n, c, lanes, chan_mean, part);
-    else bn_colsum_kernel<1, 1><<<blocks, kStatThreads, 0, st>>>(x, n, c, lanes, chan_mean, part);
+    if (mode == 0) bn_colsum_kernel<0, 1><<<blocks, threads, 0, st>>>(x, n, c, chains, lanes, chan_mean, part);
+    else bn_colsum_kernel<1, 1><<<blocks, threads, 0, st>>>(x, n, c, chains, lanes, chan_mean, part);
   }
   note_launches(1);
   SSC_CHECK_LAUNCH("bn_colsum");
@@ -680,9 +724,9 @@ extern "C" int ssc_bn_train(const float *x, int n, int c, const int32_t *field_o
   float *part = (float *)scratch;
   const int rb = bn_row_blocks(n);
   const float m = (float)momentum, keep = (float)(1.0 - momentum);
-  if (int e = launch_colsum(0, x, n, c, nullptr, part, rb, st)) return e;
+  if (int e = launch_colsum(0, x, n, c, nullptr, part, st)) return e;
   { bn_finish_mean_kernel<<<c, kFinishThreads, 0, st>>>(part, rb, n, c, scalar_of_channel, m, keep, running_mean, mean, chan_mean); note_launches(1); }
-  if (int e = launch_colsum(1, x, n, c, chan_mean, part, rb, st)) return e;
+  if (int e = launch_colsum(1, x, n, c, chan_mean, part, st)) return e;
   { bn_finish_var_kernel<<<n_field, kFinishThreads, 0, st>>>(part, rb, n, c, field_of_channel, scalar_of_channel, chan_mean, weight, bias,
                                                            eps, m, keep, running_var, var, scale, shift); note_launches(1); }
   SSC_CHECK_LAUNCH("bn_train");
@@ -699,28 +743,31 @@ extern "C" int ssc_bn_stats(const float *x, int n, int c, const int32_t *field_o
                       mean, var, var + n_field, nullptr, nullptr, scratch, scratch_bytes, stream);
 }
 
-// Rows per tile of the backward kernels: as many as 32 KB of shared memory hold (up to seven blocks per SM).
+// Rows per tile of the backward kernels: as many as 32 KB of shared memory hold (up to seven blocks per SM), no
+// more than a chain has.
 static int bwd_tile_rows(int c, int c_out, int n_gates, size_t *smem) {
   const size_t per_row = (size_t)(c + c_out + 2 * n_gates) * sizeof(float);
   int rows = (int)(32 * 1024 / per_row);
   rows = rows >= 8 ? (rows & ~3) : (rows < 1 ? 1 : rows);     // multiples of four keep the copies 16-byte aligned
-  if (rows > 64) rows = 64;
+  if (rows > 32) rows = 32;
   *smem = rows * per_row;
-  if (*smem < 2 * kBwdThreads * sizeof(float)) *smem = 2 * kBwdThreads * sizeof(float);
   return rows;
 }
 
 template <int PASS>
-static int launch_bwd(BnGateBwd p, const float *ks, const float *ka, const float *kg, float *gx, float *part_a, float *part_g, int blocks,
-                      cudaStream_t st) {
+static int launch_bwd(BnGateBwd p, const float *ks, const float *ka, const float *kg, float *gx, float *part_a, float *part_g, cudaStream_t st) {
   size_t smem;
   p.rows = bwd_tile_rows(p.c, p.c_out, p.n_gates, &smem);
-  p.vec = (p.c & 3) == 0 && (p.c_out & 3) == 0 && (((uintptr_t)p.x | (uintptr_t)p.go) & 15u) == 0 && p.rows * (size_t)p.c % 4 == 0;
+  p.chains = 8 * bn_row_blocks(p.n);
+  p.vec = (p.c & 3) == 0 && (p.c_out & 3) == 0 && (((uintptr_t)p.x | (uintptr_t)p.go) & 15u) == 0;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(bn_gate_bwd_kernel<PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "bn_gate_bwd: smem attribute: %s", cudaGetErrorString(e));
   }
-  { bn_gate_bwd_kernel<PASS><<<dim3(blocks, ceil_div(p.c, kBwdThreads * kBwdMaxAcc)), kBwdThreads, smem, st>>>(p, ks, ka, kg, gx, part_a, part_g); note_launches(1); }
+  const int threads = 256;
+  int blocks = PASS == 0 ? p.chains : ceil_div(p.n, p.rows);
+  if (PASS == 1 && blocks > 8 * 148) blocks = 8 * 148;
+  { bn_gate_bwd_kernel<PASS><<<dim3(blocks, PASS == 0 ? ceil_div(p.c, threads * kBwdMaxAcc) : 1), threads, smem, st>>>(p, ks, ka, kg, gx, part_a, part_g); note_launches(1); }
   SSC_CHECK_LAUNCH("bn_gate_bwd");
   return SSC_OK;
 }
@@ -737,15 +784,15 @@ extern "C" int ssc_bn_gate_bwd(const float *x, const float *gout, int n, int c, 
   SSC_REQUIRE(scratch && scratch_bytes >= ssc_bn_scratch_bytes(n, c), "bn_gate_bwd: scratch too small (ssc_bn_scratch_bytes)");
   cudaStream_t st = as_stream(stream);
   const int rb = bn_row_blocks(n);
-  float *part_a = (float *)scratch, *part_g = part_a + (size_t)rb * c;
-  float *ks = part_g + (size_t)rb * c, *ka = ks + c, *kg = ka + c;
-  BnGateBwd p = {x, gout, n, c, c_out, gate_of_channel ? c - c_out : 0, 0, scale, shift, chan_mean, gate_of_channel, field_start, field_len,
+  float *part_a = (float *)scratch, *part_g = part_a + (size_t)8 * rb * c;
+  float *ks = part_g + (size_t)8 * rb * c, *ka = ks + c, *kg = ka + c;
+  BnGateBwd p = {x, gout, n, c, c_out, gate_of_channel ? c - c_out : 0, 0, 0, scale, shift, chan_mean, gate_of_channel, field_start, field_len,
                  scalar_act, gate_act, 0};
-  if (int e = launch_bwd<0>(p, nullptr, nullptr, nullptr, nullptr, part_a, part_g, rb, st)) return e;
+  if (int e = launch_bwd<0>(p, nullptr, nullptr, nullptr, nullptr, part_a, part_g, st)) return e;
   { bn_bwd_finish_kernel<<<n_field, kFinishThreads, 0, st>>>(part_a, part_g, rb, n, c, field_of_channel, scalar_of_channel, var, weight, eps,
                                                            training, ks, ka, kg, d_weight, d_bias); note_launches(1); }
   SSC_CHECK_LAUNCH("bn_bwd_finish");
-  return launch_bwd<1>(p, ks, ka, kg, gx, nullptr, nullptr, rb, st);
+  return launch_bwd<1>(p, ks, ka, kg, gx, nullptr, nullptr, st);
 }
 
 extern "C" int ssc_bn_bwd(const float *x, const float *gy, int n, int c, const int32_t *field_of_channel,
@@ -755,7 +802,7 @@ extern "C" int ssc_bn_bwd(const float *x, const float *gy, int n, int c, const i
   SSC_REQUIRE(n >= 1 && c >= 1 && n_field >= 1 && n_scalar >= 0, "bn_bwd: bad sizes");
   SSC_REQUIRE(n_scalar == 0 || mean, "bn_bwd: null pointer");
   SSC_REQUIRE(scalar_of_channel && scratch && scratch_bytes >= ssc_bn_scratch_bytes(n, c), "bn_bwd: scratch too small (ssc_bn_scratch_bytes)");
-  float *chan_mean = (float *)scratch + (size_t)2 * bn_row_blocks(n) * c + (size_t)3 * c;
+  float *chan_mean = (float *)scratch + (size_t)2 * 8 * bn_row_blocks(n) * c + (size_t)3 * c;
   { bn_chan_mean_kernel<<<ceil_div(c, 128), 128, 0, as_stream(stream)>>>(mean, scalar_of_channel, c, chan_mean); note_launches(1); }
   SSC_CHECK_LAUNCH("bn_chan_mean");
   return ssc_bn_gate_bwd(x, gy, n, c, c, field_of_channel, scalar_of_channel, n_field, nullptr, nullptr, chan_mean, var, weight, eps, training,
@@ -768,7 +815,7 @@ extern "C" int ssc_gate_bwd(const float *x, const float *gy, int n, int c_total,
   SSC_REQUIRE(n >= 0 && c_total >= 1 && c_out >= 1 && c_out <= c_total, "gate_bwd: bad sizes");
   if (n == 0) return SSC_OK;
   SSC_REQUIRE(x && gy && gx && gate_of_channel && (c_total == c_out || (field_start && field_len)), "gate_bwd: null pointer");
-  BnGateBwd p = {x, gy, n, c_total, c_out, c_total - c_out, 0, nullptr, nullptr, nullptr, gate_of_channel, field_start, field_len,
+  BnGateBwd p = {x, gy, n, c_total, c_out, c_total - c_out, 0, 0, nullptr, nullptr, nullptr, gate_of_channel, field_start, field_len,
                  scalar_act, gate_act, 0};
-  return launch_bwd<1>(p, nullptr, nullptr, nullptr, gx, nullptr, nullptr, bn_row_blocks(n), as_stream(stream));
+  return launch_bwd<1>(p, nullptr, nullptr, nullptr, gx, nullptr, nullptr, as_stream(stream));
 }

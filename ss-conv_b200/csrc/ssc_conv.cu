@@ -86,7 +86,7 @@ constexpr int BM = 64, BN = 64, BK = 16;
 
 __global__ void __launch_bounds__(256)
 conv_fwd_fp32_kernel(const float *__restrict__ features, int c_in, const float *__restrict__ filters, int K,
-                     int c_out, const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out,
+                     int c_out, const int32_t *__restrict__ nbr, int n_out, int rev, float *__restrict__ out,
                      const int32_t *__restrict__ n_out_dev) {
   __shared__ float As[BK][BM + 4];
   __shared__ float Bs[BK][BN + 4];
@@ -104,7 +104,7 @@ conv_fwd_fp32_kernel(const float *__restrict__ features, int c_in, const float *
 
   for (int kappa = 0; kappa < K; ++kappa) {
     int r = -1;
-    if (tid < BM && m0 + tid < n_rows) r = nbr[(size_t)kappa * n_out + m0 + tid];
+    if (tid < BM && m0 + tid < n_rows) r = nbr[(size_t)(rev ? K - 1 - kappa : kappa) * n_out + m0 + tid];
     __syncthreads();  // previous iteration finished reading rows/As/Bs
     if (tid < BM) rows[tid] = r;
     if (!__syncthreads_or(r >= 0)) continue;
@@ -222,22 +222,22 @@ extern "C" int ssc_conv_fwd_ordered(const float *features, int n_in, int c_in, c
                                     const int32_t *row_order, void *stream) {
   SSC_REQUIRE(c_in > 0 && c_out > 0 && K > 0 && n_in >= 0 && n_out >= 0, "conv_fwd: bad sizes");
   const bool prestaged = (precision & SSC_CONV_PRESTAGED) != 0;
-  const bool table_in_order = (precision & SSC_CONV_TABLE_IN_ORDER) != 0;
-  precision &= ~(SSC_CONV_PRESTAGED | SSC_CONV_TABLE_IN_ORDER);
+  const int table_form = precision & (SSC_CONV_TABLE_IN_ORDER | SSC_CONV_TABLE_REVERSED);
+  precision &= ~(SSC_CONV_PRESTAGED | SSC_CONV_TABLE_IN_ORDER | SSC_CONV_TABLE_REVERSED);
   if (n_out == 0) return SSC_OK;
   SSC_REQUIRE(filters && nbr && out && (n_in == 0 || features || prestaged), "conv_fwd: null pointer");
-  SSC_REQUIRE(!table_in_order || (row_order && precision != SSC_PREC_FP32),
+  SSC_REQUIRE(!(table_form & SSC_CONV_TABLE_IN_ORDER) || (row_order && precision != SSC_PREC_FP32),
               "conv_fwd: SSC_CONV_TABLE_IN_ORDER needs a row order and a tensor-core precision");
   cudaStream_t st = as_stream(stream);
   if (precision == SSC_PREC_FP32) {
     dim3 grid(ceil_div(n_out, BM), ceil_div(c_out, BN));
-    { conv_fwd_fp32_kernel<<<grid, 256, 0, st>>>(features, c_in, (const float *)filters, K, c_out, nbr, n_out, out, n_out_dev); note_launches(1); }
+    { conv_fwd_fp32_kernel<<<grid, 256, 0, st>>>(features, c_in, (const float *)filters, K, c_out, nbr, n_out, table_form != 0, out, n_out_dev); note_launches(1); }
     SSC_CHECK_LAUNCH("conv_fwd_fp32");
     return SSC_OK;
   }
-  if (precision == SSC_PREC_TF32) return conv_fwd_tf32(features, n_in, c_in, filters, K, c_out, nbr, n_out, out, status, scratch, scratch_bytes, n_out_dev, row_order, prestaged, table_in_order, st);
+  if (precision == SSC_PREC_TF32) return conv_fwd_tf32(features, n_in, c_in, filters, K, c_out, nbr, n_out, out, status, scratch, scratch_bytes, n_out_dev, row_order, prestaged, table_form, st);
   if (precision == SSC_PREC_F16 || precision == SSC_PREC_BF16)
-    return conv_fwd_16(features, n_in, c_in, precision == SSC_PREC_BF16, filters, K, c_out, nbr, n_out, out, status, scratch, scratch_bytes, n_out_dev, row_order, prestaged, table_in_order, st);
+    return conv_fwd_16(features, n_in, c_in, precision == SSC_PREC_BF16, filters, K, c_out, nbr, n_out, out, status, scratch, scratch_bytes, n_out_dev, row_order, prestaged, table_form, st);
   return fail(SSC_ERR_INVALID, "conv_fwd: unknown precision %d", precision);
 }
 

@@ -51,6 +51,7 @@ struct TcParams {
   int fmt16;      // 16-bit operands: 0 = fp16, 1 = bf16 (operand format field of the instruction descriptor)
   int last_kk;    // MMA k-steps (32 bytes of K each) that hold real channels in the LAST slab: 1..4
   int opk;        // kernel offsets per 128-byte operand row: 1, or 32 / c_pad for TF32 layers with c_pad = 4, 8, 16
+  int rev;        // 1: the table's row of kernel offset kappa is K - 1 - kappa (the transpose of a centred submanifold table)
   int nbr_by_pos; // 1: the table's columns are already in the order of `order` (column j <-> output row order[j])
                   // channels (a first layer with 3 input channels packs 8 offsets into one step)
 };
@@ -61,6 +62,7 @@ static bool tc_params(int c_in, int c_out, TcParams &p, bool split_n = false, bo
   p.last_kk = (c_in - (p.k_slabs - 1) * TC_SLAB + 7) / 8;     // c_in counts 4-byte words of an operand row
   p.opk = opk;
   p.nbr_by_pos = 0;
+  p.rev = 0;
   if (opk > 1) {     // grouped offsets: one full slab per group of offsets
     p.k_slabs = 1;
     p.last_kk = 4;
@@ -197,6 +199,8 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
   const int m0 = blockIdx.x * TC_M;
   const int nt0 = (int)blockIdx.y * p.nt_cta;   // first N tile of this CTA
   const int S = p.stages;
+  // table row of a kernel offset
+  auto table = [&](int kap) { return nbr + (size_t)(p.rev ? K - 1 - kap : kap) * n_out; };
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
@@ -231,7 +235,7 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int r = scan_rows[q];
-          v[i][q] = (k0 + i < K && r >= 0) ? __ldg(nbr + (size_t)(k0 + i) * n_out + r) : -1;
+          v[i][q] = (k0 + i < K && r >= 0) ? __ldg(table(k0 + i) + r) : -1;
         }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -306,7 +310,7 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
       const int kap = act_list[j / p.k_groups];
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        dst[q] = (q >= q0 && q < q0 + q_per && my_rows[q] >= 0) ? __ldg(nbr + (size_t)kap * n_out + my_rows[q]) : -1;
+        dst[q] = (q >= q0 && q < q0 + q_per && my_rows[q] >= 0) ? __ldg(table(kap) + my_rows[q]) : -1;
     };
     if (GROUPED) {
       // Grouped offsets (TF32, staged rows of c_in = 4, 8 or 16 floats): the 128-byte operand row of a
@@ -338,7 +342,7 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 #pragma unroll
           for (int o = 0; o < 8; ++o) {
             const int kap = group * p.opk + o;
-            idx[o] = (o < p.opk && kap < K && my_row >= 0) ? __ldg(nbr + (size_t)kap * n_out + my_row) : -1;
+            idx[o] = (o < p.opk && kap < K && my_row >= 0) ? __ldg(table(kap) + my_row) : -1;
           }
           if (lane == 0) slot_masks[slot * 4 + q] = 0u;          // every row takes part
           const uint32_t a_row = slot_addr + (uint32_t)(q * 4 + (lane >> 3)) * 1024u + sw * 128u;
@@ -584,7 +588,7 @@ __global__ void pack_filters_16_kernel(const float *__restrict__ filters, int K,
 
 int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void *packed, int K, int c_out,
                 const int32_t *nbr, int n_out, float *out, int32_t *status, void *scratch, size_t scratch_bytes,
-                const int32_t *n_out_dev, const int32_t *order, bool prestaged, bool table_in_order, cudaStream_t st) {
+                const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, cudaStream_t st) {
   if (K > 256) return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): kernel volume %d > 256", K);
   const int words = f16_row_words(c_in);
   if (scratch == nullptr || scratch_bytes + 16 < conv_f16_scratch_bytes(n_in, c_in) || ((uintptr_t)scratch & 15u) != 0)
@@ -596,7 +600,8 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
     return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): c_out %d / kernel volume %d not supported", c_out, K);
   if (grid * (p.n_tiles / p.nt_cta) <= sms) tc_params(words, c_out, p, grid < 2 * sms, true);
   p.fmt16 = bf16 ? 1 : 0;
-  p.nbr_by_pos = (table_in_order && order) ? 1 : 0;
+  p.nbr_by_pos = ((table_form & SSC_CONV_TABLE_IN_ORDER) && order) ? 1 : 0;
+  p.rev = (table_form & SSC_CONV_TABLE_REVERSED) ? 1 : 0;
   if (!prestaged) {
     int rc = stage_features_16(features, n_in, c_in, bf16, scratch, st);
     if (rc != SSC_OK) return rc;
@@ -616,7 +621,7 @@ constexpr int kStagingMinTiles = 8;
 
 int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed, int K, int c_out,
                   const int32_t *nbr, int n_out, float *out, int32_t *status, void *scratch, size_t scratch_bytes,
-                  const int32_t *n_out_dev, const int32_t *order, bool prestaged, bool table_in_order, cudaStream_t st) {
+                  const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, cudaStream_t st) {
   TcParams p;
   if (K > 256) return fail(SSC_ERR_INVALID, "conv_fwd(tf32): kernel volume %d > 256", K);
   int grid = ceil_div(n_out, TC_M);
@@ -624,7 +629,8 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
   const int opk = tf32_offsets_per_row(c_in);
   if (!tc_params(c_in, c_out, p, split_n, false, opk)) return fail(SSC_ERR_INVALID, "conv_fwd(tf32): c_out %d / kernel volume %d not supported", c_out, K);
   if (grid * (p.n_tiles / p.nt_cta) <= sm_count()) tc_params(c_in, c_out, p, split_n, true, opk);
-  p.nbr_by_pos = (table_in_order && order) ? 1 : 0;
+  p.nbr_by_pos = ((table_form & SSC_CONV_TABLE_IN_ORDER) && order) ? 1 : 0;
+  p.rev = (table_form & SSC_CONV_TABLE_REVERSED) ? 1 : 0;
   size_t smem = tc_smem_bytes(p);
   // With a staging buffer the feature rows are rounded to TF32 once, up front, instead of after
   // every gather (a row is gathered about K/2 times).

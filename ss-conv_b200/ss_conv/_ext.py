@@ -656,6 +656,7 @@ def pair_lists(nbr):
 
 PRESTAGED = 0x100
 TABLE_IN_ORDER = 0x200
+TABLE_REVERSED = 0x1000
 WGRAD_X_STAGED, WGRAD_DY_STAGED = 0x400, 0x800
 # (features.data_ptr(), filters.data_ptr()) -> (prec, packed, scratch, nbytes) left by conv_prepare for the
 # conv_forward call that follows on the same tensors
@@ -723,13 +724,14 @@ def conv_prepare(features, filters, precision=None):
 
 
 def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, row_order=None, algo=None,
-                 table_in_order=False, image=None):
+                 table_in_order=False, image=None, reversed_table=False):
     """out [n_out, Cout] = sum over offsets of gathered rows times filters (one launch).
     n_out_dev: device word with the exact row count when n_out is only a capacity.
     row_order: permutation of the output rows from nbr_row_order (same result, fewer steps).
     table_in_order: nbr is the table with its columns already in that order (nbr_row_order_planes).
     algo: None (the module setting), 'rows' or 'pairs' (see set_algo).
-    image: the features' TF32 image (stage_tf32) where the caller has one already."""
+    image: the features' TF32 image (stage_tf32) where the caller has one already.
+    reversed_table: the neighbours at kernel offset kappa stand in row K - 1 - kappa of nbr."""
     if filters.dim() != 3:
         filters = filters.reshape(-1, filters.shape[-2], filters.shape[-1])
     K, c_in, c_out = filters.shape
@@ -737,7 +739,7 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
         raise ValueError("features have %d channels, filters expect %d" % (features.shape[1], c_in))
     features = features.contiguous()
     if features.dtype in _PREC_OF_DTYPE:
-        if c_in % 8 == 0 and c_out <= 512 and row_order is None:
+        if c_in % 8 == 0 and c_out <= 512 and row_order is None and not reversed_table:
             return _conv_forward_stored16(features, filters, nbr, n_out, n_out_dev, algo)
         features = features.float()
     out = torch.empty((n_out, c_out), dtype=torch.float32, device=features.device)
@@ -745,12 +747,14 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
     st = status_word(features.device)
     if mode in ("fp16", "bf16") and c_out > 512:
         mode = "fp32"
-    if (mode in _PREC_OF and n_out_dev is None and row_order is None and nbr.shape[1] == n_out
+    if (mode in _PREC_OF and n_out_dev is None and row_order is None and nbr.shape[1] == n_out and not reversed_table
             and _use_pairs(K, c_in, c_out, n_out, _PREC_OF[mode], algo)):
         return _conv_forward_pairs(features, filters, nbr, n_out, _PREC_OF[mode], out, st)
     flag = TABLE_IN_ORDER if (table_in_order and row_order is not None) else 0
     if flag and mode not in _PREC_OF:
         raise ValueError("ssconv_b200: a table in row order needs a tensor-core precision")
+    if reversed_table:
+        flag |= TABLE_REVERSED
     ready = None
     if _prepared:   # only the call that directly follows conv_prepare may use what it left
         ready = _prepared.pop((features.data_ptr(), filters.data_ptr()), None)
@@ -777,7 +781,7 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
     else:
         filters = filters.contiguous()
         _check(lib().ssc_conv_fwd(_p(features, torch.float32), features.shape[0], c_in, _p(filters, torch.float32), K,
-                                  c_out, _p(nbr, torch.int32), int(n_out), PREC_FP32, _p(out), _p(st), None, 0,
+                                  c_out, _p(nbr, torch.int32), int(n_out), PREC_FP32 | flag, _p(out), _p(st), None, 0,
                                   _p(n_out_dev), _stream()))
     return out
 
@@ -970,9 +974,11 @@ def conv_backward(features, flt, out_bp, nbr, nbr_in=None, order=None, precision
         with torch.cuda.stream(side):
             d_flt = conv_wgrad(features, out_bp, nbr, precision, dy_image=dy_image)
     if need[0]:
-        if nbr_in is None and getattr(nbr, "_ssc_symmetric", False) and n_in == nbr.shape[1]:
-            # a submanifold table with a centred kernel is its own transpose with the offsets reversed
-            nbr_in, flt = nbr, flt.flip(0)
+        # a submanifold table with a centred kernel is its own transpose with the offsets reversed
+        mirror = (nbr_in is None and getattr(nbr, "_ssc_symmetric", False) and n_in == nbr.shape[1]
+                  and not _use_pairs(flt.shape[0], c_out, c_in, n_in, PREC_TF32))
+        if mirror:
+            nbr_in = nbr
         elif nbr_in is None:
             kept = getattr(nbr, "_ssc_in_major", None)     # layers that share a rulebook share these too
             if kept is not None and kept[0] == n_in:
@@ -988,7 +994,7 @@ def conv_backward(features, flt, out_bp, nbr, nbr_in=None, order=None, precision
                     except Exception:
                         pass
         d_in = conv_forward(out_bp, flt.transpose(1, 2).contiguous(), nbr_in, n_in, precision, row_order=order,
-                            image=dy_image if tf32_in else None)
+                            image=dy_image if tf32_in else None, reversed_table=mirror)
     if forked:
         cur.wait_stream(side)
     elif need[1]:
