@@ -32,7 +32,9 @@ constexpr int TC_SLAB = 32;            // tf32 elements per 128-byte operand row
 constexpr int TC_MAX_STAGES = 8;       // producer warps = ring slots
 constexpr int TC_EPI_WARPS = 4;        // warps 0..3 also run the epilogue (one TMEM lane quarter each)
 constexpr int TC_A_BYTES = TC_M * 128;
+constexpr int TC_ROWS_THREADS = 288;     // conv_fwd_rows_kernel: two groups of four producer warps (or one) and the issuing warp
 constexpr int TC_CTRL_BYTES = 1024;
+constexpr int TC_LIST_BYTES = TC_M * 5;   // a slot's list of present rows: 128 source rows, 128 rows of the tile
 
 struct TcParams {
   int k_slabs;    // ceil(c_in / 32)
@@ -85,6 +87,7 @@ static bool tc_params(int c_in, int c_out, TcParams &p, bool split_n = false, bo
   p.fmt16 = 0;
   p.k_groups = (p.k_slabs + p.sps - 1) / p.sps;
   int stage = p.sps * (TC_A_BYTES + p.b_bytes);
+  // behind the slots: control block, a list of 128 rows (5 bytes each) per slot, alignment slack
   int fixed = TC_CTRL_BYTES + 1024;
   // Resident CTAs hide each other's per-step latencies, so take as many per SM as tensor
   // memory (512 columns) and shared memory (two ring slots each at least) allow, up to four.
@@ -93,6 +96,7 @@ static bool tc_params(int c_in, int c_out, TcParams &p, bool split_n = false, bo
   int ctas = 512 / p.tmem_cols;
   if (ctas > 4) ctas = 4;
   if (one_cta_per_sm) ctas = 1;
+  stage += TC_LIST_BYTES;
   while (ctas > 1 && ((227 * 1024) / ctas - 1024 - fixed) / stage < 2) --ctas;
   p.stages = ((227 * 1024) / ctas - 1024 - fixed) / stage;
   if (p.stages > TC_MAX_STAGES) p.stages = TC_MAX_STAGES;
@@ -193,7 +197,7 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
   uint8_t *act_list = ctrl + 512;                          // [256]
   uint32_t *slot_masks = (uint32_t *)(ctrl + 768);         // [stages][4] rows of the step WITHOUT a neighbour
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
   const int n_warps = blockDim.x >> 5;
   const int mma_warp = n_warps - 1;
   const int m0 = blockIdx.x * TC_M;
@@ -365,6 +369,14 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
         par ^= 1u;
       }
     } else {
+    // The rows of a step that have a neighbour are put into a list first (local row and source row), eight lanes
+    // then fetch the 128-byte line of a listed row: one L1 line and four sectors per row and a request for
+    // four rows per instruction.  With a lane per row every instruction asked L1 for the lines of all
+    // present rows of 32, and a 32-byte sector twice: eight slots of an SM kept its load unit busy.
+    const int list_at = slot * TC_M + q0 * 32;      // the warps of a slot share its 128 entries
+    int32_t *list_src = (int32_t *)(ctrl + TC_CTRL_BYTES) + list_at;
+    uint8_t *list_row = ctrl + TC_CTRL_BYTES + S * TC_M * 4 + list_at;
+    const int sub = lane & 7, grp = lane >> 3;
     if (slot < n_iter) load_rows(slot, nxt);
     for (int j = slot; j < n_iter; j += S) {
       const int act = j / p.k_groups, slab0 = (j - act * p.k_groups) * p.sps;
@@ -373,6 +385,25 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 #pragma unroll
       for (int q = 0; q < 4; ++q) src[q] = nxt[q];
       if (j + S < n_iter) load_rows(j + S, nxt);  // neighbour rows of this warp's next step
+      unsigned have[4];
+      int listed = 0;
+      if (STAGED) {
+        __syncwarp();       // everybody is done with the list of the step before
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          have[q] = __ballot_sync(0xffffffffu, src[q] >= 0);
+          if (src[q] >= 0) {
+            const int at = listed + __popc(have[q] & ((1u << lane) - 1u));
+            list_src[at] = src[q];
+            list_row[at] = (uint8_t)(q * 32 + lane);
+          }
+          listed += __popc(have[q]);
+        }
+        __syncwarp();
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) have[q] = __ballot_sync(0xffffffffu, src[q] >= 0);
+      }
       if (j >= S) {
         if (!mbar_wait_warp(smem_u32(empty_bars + slot), par ^ 1u, abort_flag)) break;
         tc_fence_after();
@@ -389,10 +420,24 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
       }
       uint32_t present = 0;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {  // rows of this step that the MMA must leave alone
-        const unsigned have = __ballot_sync(0xffffffffu, src[q] >= 0);
-        if (lane == 0 && q >= q0 && q < q0 + q_per) slot_masks[slot * 4 + q] = ~have;
-      }
+      for (int q = 0; q < 4; ++q)    // rows of this step that the MMA must leave alone
+        if (lane == 0 && q >= q0 && q < q0 + q_per) slot_masks[slot * 4 + q] = ~have[q];
+      if (STAGED) {
+        present = listed > 0;
+        for (int ss = 0; ss < n_sub; ++ss) {
+          const int ch0 = (slab0 + ss) * TC_SLAB + sub * 4;
+          const bool ok = ch0 < c_in;            // pieces past the last channel are zero-filled
+          const float *fp = features + (ok ? ch0 : 0);
+          const uint32_t a_slab = slot_addr + (uint32_t)(ss * TC_A_BYTES);
+#pragma unroll 4
+          for (int i = grp; i < listed; i += 4) {
+            const uint32_t row = list_row[i];
+            const int s_row = list_src[i];
+            cp_async16_cg(a_slab + (row >> 3) * 1024u + (row & 7u) * 128u + (((uint32_t)sub ^ (row & 7u)) << 4),
+                          fp + (size_t)s_row * c_in, ok ? 16u : 0u);
+          }
+        }
+      } else {
       for (int ss = 0; ss < n_sub; ++ss) {
       const int ch0 = (slab0 + ss) * TC_SLAB;
 #pragma unroll
@@ -404,8 +449,7 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 #pragma unroll
             for (int c = 0; c < 8; ++c) {  // chunks past the last channel are zero-filled
               bool ok = ch0 + c * 4 < c_in;
-              if (STAGED) cp_async16_cg(a_row + ((c ^ sw) << 4), ok ? (const void *)(fp + c * 4) : (const void *)features, ok ? 16u : 0u);
-              else cp_async16(a_row + ((c ^ sw) << 4), ok ? (const void *)(fp + c * 4) : (const void *)features, ok ? 16u : 0u);
+              cp_async16(a_row + ((c ^ sw) << 4), ok ? (const void *)(fp + c * 4) : (const void *)features, ok ? 16u : 0u);
             }
           } else {
 #pragma unroll
@@ -419,6 +463,7 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
           }
           present |= 1u << q;
         }
+      }
       }
       }
       cp_async_commit();
@@ -446,10 +491,9 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
       par ^= 1u;
     }
     }   // one offset per step
-  } else if (warp == mma_warp && lane == 0) {
-    // ================================ MMA issuer ============================================
-    // The issuing thread is the serial bottleneck of the pipeline, so its loop is kept to a
-    // handful of instructions: slot index, parity and descriptor halves are running values.
+  } else if (warp == mma_warp) {
+    // ================================ MMA issuer: the whole warp, one elected lane issues ========
+    // slot index, parity and descriptor halves are running values
     // fp32 accumulator; operand formats: kind::tf32 2 = TF32; kind::f16 0 = fp16, 1 = bf16
     const uint32_t fmt = F16 ? (uint32_t)p.fmt16 : 2u;
     const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.tile_n >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
@@ -458,7 +502,7 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
     uint32_t s = 0, par = 0, a_lo = a_lo0;
     int grp = 0;  // which slab group of its kernel offset the current step is
     for (int it = 0; it < n_iter; ++it) {
-      if (!mbar_wait(fulla0 + s * 8u, par, abort_flag)) break;
+      if (!mbar_wait_uniform(fulla0 + s * 8u, par, abort_flag)) break;
       tc_fence_after();
       const uint4 off = *(const uint4 *)(slot_masks + s * 4u);  // rows to leave untouched
       const int n_sub = min(p.sps, p.k_slabs - grp * p.sps);
@@ -470,20 +514,10 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
         for (int nt = 0; nt < p.nt_cta; ++nt) {
           const uint32_t dn = tmem_base + (uint32_t)(nt * p.tile_n);
           const uint32_t bn = a_lo + (uint32_t)(p.sps * TC_A_BYTES >> 4) + (uint32_t)ss * ((uint32_t)p.b_bytes >> 4) + (uint32_t)nt * n_step;
-          if (n_kk == 4) {   // the common case, straight-line
-            if (F16) {
-              mma_f16_ss_masked(dn, an, bn, idesc, off);
-              mma_f16_ss_masked(dn, an + 2u, bn + 2u, idesc, off);
-              mma_f16_ss_masked(dn, an + 4u, bn + 4u, idesc, off);
-              mma_f16_ss_masked(dn, an + 6u, bn + 6u, idesc, off);
-            } else {
-              mma_tf32_ss_masked(dn, an, bn, idesc, off);
-              mma_tf32_ss_masked(dn, an + 2u, bn + 2u, idesc, off);
-              mma_tf32_ss_masked(dn, an + 4u, bn + 4u, idesc, off);
-              mma_tf32_ss_masked(dn, an + 6u, bn + 6u, idesc, off);
-            }
-          } else {
-            for (int kk = 0; kk < n_kk; ++kk) {
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+              if (kk >= n_kk) break;
               if (F16) mma_f16_ss_masked(dn, an + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
               else mma_tf32_ss_masked(dn, an + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
             }
@@ -491,11 +525,11 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
         }
       }
       if (++grp == p.k_groups) grp = 0;
-      mma_commit(empty0 + s * 8u);
+      if (elect_one()) mma_commit(empty0 + s * 8u);
       a_lo += slot_step;
       if (++s == (uint32_t)S) { s = 0; par ^= 1u; a_lo = a_lo0; }
     }
-    mma_commit(smem_u32(done_bar));  // arrives once everything issued above has retired
+    if (elect_one()) mma_commit(smem_u32(done_bar));  // arrives once everything issued above has retired
   }
 
   // ================================ epilogue: TMEM -> registers -> global ====================
@@ -552,8 +586,300 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
   }
 }
 
+// ---------------------------------------------------------------------------------------------------
+// The kernel for staged operands (TF32-rounded fp32 rows, or fp16 / bf16 rows: F16), one kernel offset and one
+// 128-byte slab per step.  Warps 0-3 produce (and run the epilogue), a lane per output row of the tile; with
+// four ring slots or more (few CTAs per SM) warps 4-7 are a second group that takes every other
+// offset; the last warp issues the MMAs.
+//
+// What bounds it is the way of an operand slot: free -> rows gathered -> multiplied -> free, against the slots that
+// fit an SM (eight of 26 KB for 64 -> 76 channels).  With a warp per slot that built its row lists, waited
+// for its own copies and arrived, that way was 3700 cycles, of which about 2300 were the warp's own
+// 250 dependent instructions.  Hence here:
+//   * the four warps fill every slot together, 32 rows each, four lanes to a row, and work out the source rows
+//     once per kernel offset for all its slabs;
+//   * nobody waits for copies: the copies' completion arrives on the slot's barrier by itself
+//     (cp.async.mbarrier.arrive.noinc), the warps go on to the next free slot, and the issuing warp orders
+//     the landed rows for the tensor core (fence.proxy.async behind the barrier);
+//   * table entries are loaded two offsets ahead.
+// Sums are accumulated in the order of the steps (ascending offset, ascending slab), whatever the tile's
+// other rows need.
+template <bool F16>
+__global__ void __launch_bounds__(TC_ROWS_THREADS)
+conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
+                     const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out, int32_t *status, TcParams p,
+                     const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order) {
+  const int n_rows = live_rows(n_out, n_out_dev);
+  if ((int)blockIdx.x * TC_M >= n_rows) return;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t empty_bars[TC_MAX_STAGES], full_bars[TC_MAX_STAGES], done_bar;
+  __shared__ __align__(16) uint32_t slot_masks[TC_MAX_STAGES * 4];   // rows of the slot's step WITHOUT a neighbour
+  __shared__ uint32_t act_bits[8];
+  __shared__ uint8_t act_list[256];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_word, n_act_s;
+  volatile int *abort_flag = &abort_word;
+  // operand slots need 1024-byte alignment for the 128-byte swizzle
+  uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int stage_bytes = TC_A_BYTES + p.b_bytes;
+  const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
+  const int groups = (int)blockDim.x / 128, mma_warp = groups * 4;   // producer groups of four warps
+  const int quarter = warp & 3;                                      // the 32 rows of the tile a producer warp works on
+  const int m0 = blockIdx.x * TC_M, nt0 = (int)blockIdx.y * p.nt_cta, S = p.stages;
+  auto table = [&](int kap) { return nbr + (size_t)(p.rev ? K - 1 - kap : kap) * n_out; };
+
+  // Rows in a row order were put together by the offsets they use, so that a tile can leave out the others: the
+  // table is scanned for them first.  In any other order nearly every offset has a row among 128, the
+  // scan (8 us when all CTAs of the first wave do it at once) finds nothing, and a step without a
+  // row costs its filter copy but no multiplication.
+  const bool scan = order != nullptr;
+  const int m_tile = m0 + quarter * 32 + lane;    // (producers) this lane's row of the tile
+  int my_row = -1;                                // its column of the table
+  if (warp == mma_warp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)p.tmem_cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  } else {
+    if (tid < 8) act_bits[tid] = 0u;
+    if (tid == 32) {
+      for (int s = 0; s < S; ++s) {
+        mbar_init(smem_u32(empty_bars + s), 1);
+        // 128 arrivals by copies, one per warp for the row mask, one for the filter copy's byte count
+        mbar_init(smem_u32(full_bars + s), 128 + 4 + 1);
+      }
+      mbar_init(smem_u32(&done_bar), 1);
+      *abort_flag = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (m_tile < n_rows) my_row = (order && !p.nbr_by_pos) ? __ldg(order + m_tile) : m_tile;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_slot;
+  if (warp < 4) {
+    // Clear the accumulators: every MMA accumulates, rows without a neighbour at a step are switched off
+    // through the MMA's disable-output-lane mask, so the gathered operand never holds zero rows.
+#pragma unroll 1
+    for (int c0 = 0; c0 < p.n_cta; c0 += 16) {
+      const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
+      asm volatile(
+          "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+          "r"(0u)
+          : "memory");
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  }
+  if (scan) {
+    if (warp < mma_warp) {
+#pragma unroll 1
+      for (int k0 = 9 * (warp >> 2); k0 < K; k0 += 9 * groups) {     // nine loads in flight per lane
+        int v[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) v[i] = (k0 + i < K && my_row >= 0) ? __ldg(table(k0 + i) + my_row) : -1;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+          const unsigned b = __ballot_sync(0xffffffffu, v[i] >= 0);
+          if (lane == 0 && b) atomicOr(&act_bits[(k0 + i) >> 5], 1u << ((k0 + i) & 31));
+        }
+      }
+    }
+    __syncthreads();
+    if (warp == mma_warp) {
+      int n = 0;
+      for (int w = 0; w * 32 < K; ++w) {
+        const uint32_t bits = act_bits[w];
+        if ((bits >> lane) & 1u) act_list[n + __popc(bits & ((1u << lane) - 1u))] = (uint8_t)(w * 32 + lane);
+        n += __popc(bits);
+      }
+      if (lane == 0) n_act_s = n;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const int n_act = scan ? n_act_s : K, n_iter = n_act * p.k_slabs;
+  const uint32_t smem_base = smem_u32(smem);
+
+  if (warp < mma_warp) {
+    // ====================== producers =========================================================
+    // Four lanes per row, eight rows per pass: lane l copies the 16-byte pieces l & 3 and (l & 3) + 4 of the row
+    // 8 * pass + l / 4 of its warp's 32 rows, where that row has a neighbour.
+    const int sub = lane & 3, row8 = lane >> 2;
+    const uint32_t warp_rows = smem_base + (uint32_t)quarter * 4096u + (uint32_t)row8 * 128u;   // row of the warp's first 8-row group
+    const uint32_t piece0 = ((uint32_t)sub ^ (uint32_t)row8) << 4, piece1 = ((uint32_t)(sub + 4) ^ (uint32_t)row8) << 4;
+    auto offset_of = [&](int a) { return scan ? (int)act_list[a] : a; };
+    auto entry = [&](int a) { return (a < n_act && my_row >= 0) ? __ldg(table(offset_of(a)) + my_row) : -1; };
+    // with two groups each takes every other offset
+    const int first = warp >> 2;
+    int src = entry(first), nxt = entry(first + groups);
+    int slot = 0, it_no = first * p.k_slabs;
+    uint32_t par = 1;                             // parity the slot's "empty" barrier has to have passed (first uses: none)
+    auto skip = [&](int steps) {
+      for (slot += steps; slot >= S; slot -= S) par ^= 1u;
+    };
+    skip(it_no);
+    bool alive = true;
+#pragma unroll 1
+    for (int a = first; a < n_act && alive; a += groups) {
+      const int after = entry(a + 2 * groups);
+      const unsigned have = __ballot_sync(0xffffffffu, src >= 0);
+      const float *ptr[4];
+      bool live[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int s = __shfl_sync(0xffffffffu, src, i * 8 + row8);
+        live[i] = s >= 0;
+        ptr[i] = features + (size_t)(s >= 0 ? s : 0) * row_words + sub * 4;
+      }
+      const uint4 *bsrc = packed + (size_t)offset_of(a) * p.k_slabs * (size_t)(p.n_pad * 8) + (size_t)nt0 * (size_t)(p.tile_n * 8);
+#pragma unroll 1
+      for (int slab = 0; slab < p.k_slabs; ++slab) {
+        const uint32_t full = smem_u32(full_bars + slot);
+        if (it_no >= S && !mbar_wait_warp(smem_u32(empty_bars + slot), par, abort_flag)) { alive = false; break; }
+        const uint32_t slot_off = (uint32_t)slot * (uint32_t)stage_bytes;
+        if (lane == 0) {
+          if (quarter == 0) {                     // the pre-packed filter slab of this step: one bulk copy
+            mbar_expect_tx(full, (uint32_t)p.b_bytes);
+            bulk_g2s(smem_base + slot_off + (uint32_t)TC_A_BYTES, bsrc + (size_t)slab * (size_t)(p.n_pad * 8), (uint32_t)p.b_bytes, full);
+          }
+          slot_masks[slot * 4 + quarter] = ~have;
+        }
+        const int words = row_words - slab * TC_SLAB - sub * 4;   // from this lane's first piece to the row's end
+        const uint32_t dst = warp_rows + slot_off;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (live[i]) {                          // pieces past the last channel are zero-filled (and read nothing)
+            cp_async16_cg(dst + (uint32_t)i * 1024u + piece0, words > 0 ? ptr[i] : features, words > 0 ? 16u : 0u);
+            cp_async16_cg(dst + (uint32_t)i * 1024u + piece1, words > 16 ? ptr[i] + 16 : features, words > 16 ? 16u : 0u);
+          }
+          ptr[i] += TC_SLAB;
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
+        if (lane == 0) mbar_arrive(full);         // (releases the row mask)
+        ++it_no;
+        skip(1);
+      }
+      src = nxt;
+      nxt = after;
+      it_no += (groups - 1) * p.k_slabs;
+      skip((groups - 1) * p.k_slabs);
+    }
+    cp_async_wait_all();
+  } else {
+    // ================================ MMA issuer: the whole warp, one elected lane issues ========
+    // fp32 accumulator; operand formats: kind::tf32 2 = TF32; kind::f16 0 = fp16, 1 = bf16
+    const uint32_t fmt = F16 ? (uint32_t)p.fmt16 : 2u;
+    const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.tile_n >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+    const uint32_t a_lo0 = desc_lo(smem_base), slot_step = (uint32_t)stage_bytes >> 4, n_step = (uint32_t)(p.tile_n * 128) >> 4;
+    const uint32_t full0 = smem_u32(full_bars), empty0 = smem_u32(empty_bars);
+    uint32_t s = 0, par = 0, a_lo = a_lo0;
+    int slab = 0;
+    for (int it = 0; it < n_iter; ++it) {
+      if (!mbar_wait_uniform(full0 + s * 8u, par, abort_flag)) break;
+      fence_async_smem();                         // the rows other threads' copies left, for the tensor core
+      tc_fence_after();
+      const uint4 off = *(const uint4 *)(slot_masks + s * 4u);
+      // k-steps that hold real channels (the rest of the last slab is zero on both sides)
+      const int n_kk = slab == p.k_slabs - 1 ? p.last_kk : 4;
+      const bool any = __any_sync(0xffffffffu, (off.x & off.y & off.z & off.w) != 0xffffffffu);
+      for (int nt = 0; nt < (any ? p.nt_cta : 0); ++nt) {
+        const uint32_t dn = tmem_base + (uint32_t)(nt * p.tile_n);
+        const uint32_t bn = a_lo + (uint32_t)(TC_A_BYTES >> 4) + (uint32_t)nt * n_step;
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {
+            if (kk >= n_kk) break;
+            if (F16) mma_f16_ss_masked(dn, a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
+            else mma_tf32_ss_masked(dn, a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
+          }
+        }
+      }
+      if (++slab == p.k_slabs) slab = 0;
+      if (elect_one()) mma_commit(empty0 + s * 8u);
+      a_lo += slot_step;
+      if (++s == (uint32_t)S) { s = 0; par ^= 1u; a_lo = a_lo0; }
+    }
+    if (elect_one()) mma_commit(smem_u32(&done_bar));   // arrives once everything issued above has retired
+  }
+
+  // ================================ epilogue: TMEM -> shared memory -> global ====================
+  if (warp < 4) {
+    __syncwarp();
+    bool ok = __all_sync(0xffffffffu, !*abort_flag);
+    if (ok && n_iter > 0) ok = mbar_wait_warp(smem_u32(&done_bar), 0u, abort_flag);
+    ok = __all_sync(0xffffffffu, ok);             // tcgen05.ld below is warp-collective
+    tc_fence_after();
+    const int m = m_tile < n_rows ? (order ? __ldg(order + m_tile) : m_tile) : -1;
+    const int col0 = nt0 * p.tile_n;              // first output channel of this CTA
+    // 32 columns of the warp's 32 rows at a time go through the warp's share of slot 0 (free now), so that eight
+    // lanes write the 128 contiguous bytes of a row
+    float *blk = (float *)(smem + (size_t)warp * 4096u);
+    const bool vec = (c_out & 3) == 0 && ((uintptr_t)out & 15u) == 0;
+    for (int c0 = 0; c0 < p.n_cta && col0 + c0 < c_out; c0 += 32) {
+      uint32_t r[32];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (ok && n_iter > 0 && c0 + 16 * h < p.n_cta) {
+          const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c0 + 16 * h);
+          uint32_t *q = r + 16 * h;
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+              : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]), "=r"(q[8]),
+                "=r"(q[9]), "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
+              : "r"(taddr)
+              : "memory");
+        } else {
+#pragma unroll
+          for (int q = 0; q < 16; ++q) r[16 * h + q] = 0u;
+        }
+      }
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (vec) {
+        __syncwarp();
+        // piece q of row `lane` at place q ^ (lane & 7): both directions touch every bank once per phase
+#pragma unroll
+        for (int q = 0; q < 8; ++q) *(uint4 *)(blk + lane * 32 + ((q ^ (lane & 7)) << 2)) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+        __syncwarp();
+        const int q = lane & 7, col = col0 + c0 + 4 * q;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int row = 4 * i + (lane >> 3);
+          const int to = __shfl_sync(0xffffffffu, m, row);
+          if (to >= 0 && col < c_out && c0 + 4 * q < p.n_cta)
+            *(uint4 *)(out + (size_t)to * c_out + col) = *(const uint4 *)(blk + row * 32 + ((q ^ (row & 7)) << 2));
+        }
+      } else if (m >= 0) {
+        float *op = out + (size_t)m * c_out + col0 + c0;
+#pragma unroll
+        for (int q = 0; q < 32; ++q)
+          if (col0 + c0 + q < c_out && c0 + q < p.n_cta) op[q] = __uint_as_float(r[q]);
+      }
+    }
+  }
+  // a wait gave up: what was issued still arrives on done_bar (committed on every path) and filter copies land
+  // within microseconds; both before the accumulators and the shared memory are handed back
+  if (*abort_flag) {
+    if (warp == mma_warp && lane == 0 && n_iter > 0) mbar_wait_drain(smem_u32(&done_bar), 0u);
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (tid == 0 && *abort_flag && status) atomicOr(status, 16);
+  if (warp == mma_warp) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols) : "memory");
+  }
+}
+
+// Two producer groups where the ring is deep enough for both.  A group that comes to a slot may find its "empty"
+// barrier at most one phase behind the one it waits for (the wait tells phases apart by their parity only).
+// The group's step before is (groups - 1) * k_slabs + 1 earlier and was let through by a slot freed `stages`
+// before that, so a slot is behind by no more than that as long as k_slabs + 1 <= stages.
+static int rows_threads(const TcParams &p) {
+  return p.stages >= 4 && p.k_slabs + 1 <= p.stages ? TC_ROWS_THREADS : TC_ROWS_THREADS - 128;
+}
+
 static size_t tc_smem_bytes(const TcParams &p) {
-  return (size_t)p.stages * p.sps * (TC_A_BYTES + p.b_bytes) + 1024 /*alignment slack*/ + TC_CTRL_BYTES;
+  return (size_t)p.stages * p.sps * (TC_A_BYTES + p.b_bytes) + 1024 /*alignment slack*/ + TC_CTRL_BYTES + (size_t)p.stages * TC_LIST_BYTES;
 }
 
 // 16-bit operands: filters [K, c_in, c_out] fp32 -> [K][k_slabs][n_pad rows][64 fp16 or bf16], same
@@ -607,11 +933,11 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
     if (rc != SSC_OK) return rc;
   }
   const size_t smem = tc_smem_bytes(p);
-  auto kernel = conv_fwd_tf32_kernel<true, true>;
+  auto kernel = conv_fwd_rows_kernel<true>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(16-bit): smem attribute: %s", cudaGetErrorString(e));
   const dim3 grid2(grid, p.n_tiles / p.nt_cta);
-  { kernel<<<grid2, p.threads, smem, st>>>((const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order); note_launches(1); }
+  { kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_fwd_16");
   return SSC_OK;
 }
@@ -646,11 +972,12 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
     int rc = stage_features(features, n_in, c_in, scratch, st);
     if (rc != SSC_OK) return rc;
   }
-  auto kernel = opk > 1 ? conv_fwd_tf32_kernel<true, false, true> : staged ? conv_fwd_tf32_kernel<true> : conv_fwd_tf32_kernel<false>;
+  const bool rows = staged && opk == 1;
+  auto kernel = opk > 1 ? conv_fwd_tf32_kernel<true, false, true> : rows ? conv_fwd_rows_kernel<false> : conv_fwd_tf32_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
   const dim3 grid2(grid, p.n_tiles / p.nt_cta);
-  { kernel<<<grid2, p.threads, smem, st>>>(staged ? (const float *)scratch : features, staged ? c_pad : c_in, (const uint4 *)packed, K, c_out,
+  { kernel<<<grid2, rows ? rows_threads(p) : p.threads, smem, st>>>(staged ? (const float *)scratch : features, staged ? c_pad : c_in, (const uint4 *)packed, K, c_out,
                                         nbr, n_out, out, status, p, n_out_dev, order); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_fwd_tf32");
   return SSC_OK;

@@ -71,6 +71,25 @@ __device__ __forceinline__ bool mbar_wait_warp_backoff(uint32_t bar, uint32_t pa
   ok = __shfl_sync(0xffffffffu, ok, 0);
   return ok != 0;
 }
+// Roles that issue tensor-core instructions run as a whole warp with warp-uniform control flow, and one elected
+// lane issues: the instructions take their operands from uniform registers, and inside a branch on
+// the lane number the compiler moves every operand there one by one - 150 cycles per tcgen05.mma
+// whatever its size, against 39 (N = 16), 55 (N = 80) and 128 (N = 256) in this form.
+__device__ __forceinline__ int warp_id() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+// Bounded wait of a whole warp; the result is a vote, i.e. warp-uniform.
+__device__ __forceinline__ bool mbar_wait_uniform(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+  for (uint32_t i = 0; i < kSpinLimit; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 1023u) == 1023u && __any_sync(0xffffffffu, *abort_flag)) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
