@@ -76,45 +76,54 @@ struct PlParams {
 // greedily, main strips first, each to the CTA with the least work so far: every CTA starts with a
 // strip that walks its offset's list from the first row (all CTAs sweep the rows together, which keeps
 // gathers and reductions in L2) and the tails fill the CTAs whose offsets were short.
-__global__ void pl_strips_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_ctas,
-                                 int32_t *__restrict__ hdr, int4 *__restrict__ strips, int32_t *__restrict__ owner) {
-  __shared__ int tiles[256];
-  __shared__ int first[257];
-  __shared__ int load_s[PL_MAX_CTAS];
-  __shared__ long long L_s;
-  const int tid = threadIdx.x;
+// What bounds it is the greedy assignment, one strip after the other: with the CTAs' loads spread over a warp
+// each strip cost a scan of all of them from shared memory, 140 us for the 330 strips of a 5^3 layer.
+// A thread now holds the load of one CTA in a register and a block-wide minimum (two shuffle
+// reductions, the lowest CTA wins ties) decides per strip; the first strip of every CTA needs no
+// decision (all loads are zero, so they go to the CTAs in order).
+__global__ void __launch_bounds__(PL_MAX_CTAS)
+pl_strips_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_ctas,
+                 int32_t *__restrict__ hdr, int4 *__restrict__ strips, int32_t *__restrict__ owner) {
+  __shared__ int tiles[256], first[257], tiles_of[PL_MAX_CTAS];
+  __shared__ unsigned best_s[2][PL_MAX_CTAS / 32];
+  __shared__ int L_s;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (hdr[0] > 0 && hdr[1] == K && hdr[2] == n_split && hdr[3] == n_ctas) return;   // built before for this grid
   int T = 0;
   if (tid < K) {
     const int n = starts[tid + 1] - starts[tid];
     T = n > 0 ? (n + PL_M - 1) / PL_M : 0;
   }
-  tiles[tid] = T;
+  if (tid < 256) tiles[tid] = T;
   __syncthreads();
-  if (tid == 0) {
+  if (tid < 32) {
     long long tot = 0;
-    for (int k = 0; k < K; ++k) tot += tiles[k];
-    tot *= n_split;
-    const long long L = (tot + n_ctas - 1) / n_ctas;
-    L_s = L < 1 ? 1 : L;
+    for (int k = tid; k < K; k += 32) tot += tiles[k];
+    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    const long long L = (tot * n_split + n_ctas - 1) / n_ctas;
+    if (tid == 0) L_s = L < 1 ? 1 : (int)L;
   }
   __syncthreads();
-  const int L = (int)L_s;
+  const int L = L_s;
   int mains = 0, tail = 0;
   if (T > 0) {
     if (T > L + L / 2) mains = (T + L / 2) / L;
     else { mains = 1; tail = T > L ? 1 : 0; }
   }
+  if (tid < 256) tiles[tid] = (mains + tail) * n_split;
   __syncthreads();
-  tiles[tid] = (mains + tail) * n_split;
-  __syncthreads();
-  if (tid == 0) {
-    int s = 0;
-    for (int k = 0; k < K; ++k) {
-      first[k] = s;
-      s += tiles[k];
+  if (tid < 32) {
+    int run = 0;
+    for (int k0 = 0; k0 < 256; k0 += 32) {
+      int v = k0 + lane < K ? tiles[k0 + lane] : 0, incl = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+      }
+      first[k0 + lane] = run + incl - v;
+      run += __shfl_sync(0xffffffffu, incl, 31);
     }
-    first[256] = s;
+    if (lane == 0) first[256] = run;
   }
   __syncthreads();
   const int n_strips = first[256];
@@ -132,35 +141,59 @@ __global__ void pl_strips_kernel(const int32_t *__restrict__ starts, int K, int 
     }
   }
   __syncthreads();
-  if (tid < 32) {   // one warp: greedy assignment, main strips (-1) first, then tails (-2)
-    for (int b = tid; b < n_ctas; b += 32) load_s[b] = 0;
-    __syncwarp();
-    for (int pass = -1; pass >= -2; --pass) {
-      for (int s = 0; s < n_strips; ++s) {
-        if (owner[s] != pass) continue;            // warp-uniform
-        int best = 0x7fffffff, arg = 0x7fffffff;
-        for (int b = tid; b < n_ctas; b += 32) {
-          const int v = load_s[b];
-          if (v < best) { best = v; arg = b; }     // ascending b: the lowest index wins ties
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-          const int ob = __shfl_xor_sync(0xffffffffu, best, o), oa = __shfl_xor_sync(0xffffffffu, arg, o);
-          if (ob < best || (ob == best && oa < arg)) { best = ob; arg = oa; }
-        }
-        if (tid == 0) {
-          owner[s] = arg;
-          load_s[arg] = best + strips[s].w;
-        }
-        __syncwarp();
+  // main strips (-1) first, then tails (-2), each to the CTA with the least work so far.  Work and CTA in one word:
+  // a load is at most the number of tiles of a table, which stays below 2^22 for 2^31 / 128 / K pairs.
+  unsigned load = 0;
+  int turn = 0;
+  __shared__ int n_main_s;
+  if (tid < 32) {              // the main strips among the first n_ctas strips of that kind
+    int seen = 0;
+    for (int s0 = 0; s0 < n_strips && seen < n_ctas; s0 += 32) {
+      const int s = s0 + lane;
+      const bool is = s < n_strips && owner[s] == -1;
+      const unsigned b = __ballot_sync(0xffffffffu, is);
+      const int at = seen + __popc(b & ((1u << lane) - 1u));
+      if (is && at < n_ctas) {
+        owner[s] = at;
+        tiles_of[at] = strips[s].w;
       }
+      seen += __popc(b);
     }
-    if (tid == 0) {
-      hdr[1] = K;
-      hdr[2] = n_split;
-      hdr[3] = n_ctas;
-      __threadfence();
-      hdr[0] = n_strips;
+    if (lane == 0) n_main_s = seen < n_ctas ? seen : n_ctas;
+  }
+  __syncthreads();
+  if (tid < n_main_s) load = (unsigned)tiles_of[tid];
+  for (int pass = -1; pass >= -2; --pass) {
+    for (int s0 = 0; s0 < n_strips; s0 += PL_MAX_CTAS) {
+      const int mine = s0 + tid < n_strips ? owner[s0 + tid] : 0, work = s0 + tid < n_strips ? strips[s0 + tid].w : 0;
+      __shared__ int kind_s[PL_MAX_CTAS], work_s[PL_MAX_CTAS];
+      kind_s[tid] = mine;
+      work_s[tid] = work;
+      __syncthreads();
+      const int end = min(PL_MAX_CTAS, n_strips - s0);
+      for (int i = 0; i < end; ++i) {
+        if (kind_s[i] != pass) continue;            // the same for the whole block
+        unsigned v = tid < n_ctas ? (load << 9) | (unsigned)tid : 0xffffffffu;
+        v = __reduce_min_sync(0xffffffffu, v);
+        if (lane == 0) best_s[turn][warp] = v;
+        __syncthreads();
+        unsigned m = lane < PL_MAX_CTAS / 32 ? best_s[turn][lane] : 0xffffffffu;
+        m = __reduce_min_sync(0xffffffffu, m);
+        if ((int)(m & 511u) == tid) {
+          load += (unsigned)work_s[i];
+          owner[s0 + i] = tid;
+        }
+        turn ^= 1;
+      }
+      __syncthreads();
     }
+  }
+  if (tid == 0) {
+    hdr[1] = K;
+    hdr[2] = n_split;
+    hdr[3] = n_ctas;
+    __threadfence();
+    hdr[0] = n_strips;
   }
 }
 
@@ -187,7 +220,7 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
   uint32_t *tmem_slot = (uint32_t *)(final_bar + 1);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
   const int S = p.stages;
   const int mma_warp = S;
   const int n_strips = *n_strips_dev;
@@ -304,30 +337,28 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
     // a wait gave up while a filter copy may still be in flight: let it land before the CTA exits
     if (warp == 0 && lane == 0 && *abort_flag && w_issued > 0) mbar_wait_drain(smem_u32(wfull_bar), (uint32_t)(w_issued - 1) & 1u);
   } else if (warp == mma_warp) {
-    // ==================================== MMA issuer ============================================
-    if (lane == 0) {
-      long long g = 0;
-      int tcount = 0, scount = 0;
-      bool alive = true;
-      for (int si = 0; si < n_strips && alive; ++si) {
-        if (__ldg(owner + si) != (int)blockIdx.x) continue;
-        const int4 sd = __ldg(strips + si);
-        const int n_tiles = sd.w;
-        if (!mbar_wait_backoff(smem_u32(wfull_bar), (uint32_t)scount & 1u, abort_flag, 64)) break;
-        tc_fence_after();
-        for (int ti = 0; ti < n_tiles && alive; ++ti, ++tcount) {
-          const int buf = tcount & 1;
-          if (tcount >= 2) {
-            if (!mbar_wait_backoff(smem_u32(acce_bars + buf), (uint32_t)((tcount >> 1) - 1) & 1u, abort_flag, 64)) { alive = false; break; }
-            tc_fence_after();
-          }
-          const uint32_t d = tmem_base + (uint32_t)(buf * p.acc_cols);
-          for (int s = 0; s < p.k_slabs; ++s, ++g) {
-            const uint32_t slot = (uint32_t)(g % S), par = (uint32_t)(g / S) & 1u;
-            if (!mbar_wait_backoff(smem_u32(full_bars + slot), par, abort_flag, 32)) { alive = false; break; }
-            tc_fence_after();
-            const uint32_t a_lo = desc_lo(a_base + slot * PL_A_BYTES);
-            const uint32_t b_lo = desc_lo(w_base + (uint32_t)s * (uint32_t)p.n_cta * 128u);
+    // ==================================== MMA issuer: the whole warp, one elected lane issues ====
+    int tcount = 0, scount = 0;
+    uint32_t slot = 0, slot_par = 0;
+    bool alive = true;
+    for (int si = 0; si < n_strips && alive; ++si) {
+      if (__ldg(owner + si) != (int)blockIdx.x) continue;
+      const int n_tiles = __ldg(strips + si).w;
+      if (!mbar_wait_uniform(smem_u32(wfull_bar), (uint32_t)scount & 1u, abort_flag)) break;
+      tc_fence_after();
+      for (int ti = 0; ti < n_tiles && alive; ++ti, ++tcount) {
+        const int buf = tcount & 1;
+        if (tcount >= 2) {
+          if (!mbar_wait_uniform(smem_u32(acce_bars + buf), (uint32_t)((tcount >> 1) - 1) & 1u, abort_flag)) { alive = false; break; }
+          tc_fence_after();
+        }
+        const uint32_t d = tmem_base + (uint32_t)(buf * p.acc_cols);
+        for (int s = 0; s < p.k_slabs; ++s) {
+          if (!mbar_wait_uniform(smem_u32(full_bars + slot), slot_par, abort_flag)) { alive = false; break; }
+          tc_fence_after();
+          const uint32_t a_lo = desc_lo(a_base + slot * PL_A_BYTES);
+          const uint32_t b_lo = desc_lo(w_base + (uint32_t)s * (uint32_t)p.n_cta * 128u);
+          if (elect_one()) {
 #pragma unroll
             for (uint32_t kk = 0; kk < 4; ++kk) {
               if (F16) mma_f16_ss(d, a_lo + 2u * kk, b_lo + 2u * kk, p.idesc, (s | (int)kk) != 0 ? 1u : 0u);
@@ -335,15 +366,16 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
             }
             mma_commit(smem_u32(empty_bars + slot));
           }
-          if (alive) mma_commit(smem_u32(accf_bars + buf));
+          if (++slot == (uint32_t)S) { slot = 0; slot_par ^= 1u; }
         }
-        if (alive) mma_commit(smem_u32(wfree_bar));
-        ++scount;
+        if (alive && elect_one()) mma_commit(smem_u32(accf_bars + buf));
       }
-      // everything issued above (on any path) retires before the CTA hands its tensor memory back
-      mma_commit(smem_u32(final_bar));
-      mbar_wait_drain(smem_u32(final_bar), 0u);
+      if (alive && elect_one()) mma_commit(smem_u32(wfree_bar));
+      ++scount;
     }
+    // everything issued above (on any path) retires before the CTA hands its tensor memory back
+    if (elect_one()) mma_commit(smem_u32(final_bar));
+    mbar_wait_drain(smem_u32(final_bar), 0u);
   } else {
     // ==================================== epilogue ==============================================
     // Two warps per quarter of the tensor-memory lanes; they take the 32-column blocks of the
@@ -525,7 +557,7 @@ int conv_fwd_pairs(const void *staged, int c_in, const void *packed, int K, int 
   int32_t *owner = (int32_t *)(strips + max_strips(K));
   cudaError_t e = cudaMemsetAsync(out, 0, (size_t)n_out * c_out * sizeof(float), st);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd_pairs: clearing the output: %s", cudaGetErrorString(e));
-  { pl_strips_kernel<<<1, 256, 0, st>>>(pl.starts, K, p.n_split, n_ctas, hdr, strips, owner); note_launches(1); }
+  { pl_strips_kernel<<<1, PL_MAX_CTAS, 0, st>>>(pl.starts, K, p.n_split, n_ctas, hdr, strips, owner); note_launches(1); }
   SSC_CHECK_LAUNCH("pl_strips");
   const size_t smem = pl_smem_bytes(p);
   auto kernel = p.f16 ? conv_fwd_pairs_kernel<true> : conv_fwd_pairs_kernel<false>;

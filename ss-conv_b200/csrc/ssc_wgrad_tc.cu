@@ -44,31 +44,46 @@ constexpr int WT_K = 32;           // pairs per chunk
 constexpr int WT_MAX_STAGES = 8;
 constexpr int WT_BLOCK = WT_K * 128;   // 32 channels of a chunk's pairs
 
-// One warp per 32 output rows of one kernel offset: which of them have a neighbour.
-__global__ void pair_bitmap_kernel(const int32_t *__restrict__ nbr, int K, int n_out, int words_per_row,
-                                   uint32_t *__restrict__ bitmap) {
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (gw >= (long long)K * words_per_row) return;
-  const int kappa = (int)(gw / words_per_row), r = (int)(gw % words_per_row) * 32 + (int)(threadIdx.x & 31);
-  const bool have = r < n_out && __ldg(nbr + (size_t)kappa * n_out + r) >= 0;
-  const unsigned m = __ballot_sync(0xffffffffu, have);
-  if ((threadIdx.x & 31) == 0) bitmap[gw] = m;
+// Which output rows have a neighbour: a warp makes four words (128 rows) of one kernel offset (blockIdx.y), four
+// loads in flight per lane.  HBM-bound: the table is read once.
+__global__ void __launch_bounds__(256)
+pair_bitmap_kernel(const int32_t *__restrict__ nbr, int n_out, int words_per_row, uint32_t *__restrict__ bitmap) {
+  const int w0 = ((int)blockIdx.x * 8 + (int)(threadIdx.x >> 5)) * 4, lane = threadIdx.x & 31;
+  if (w0 >= words_per_row) return;
+  const int32_t *row = nbr + (size_t)blockIdx.y * n_out;
+  int v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = (w0 + i) * 32 + lane;
+    v[i] = r < n_out ? __ldg(row + r) : -1;
+  }
+  uint32_t mine = 0u;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const unsigned m = __ballot_sync(0xffffffffu, v[i] >= 0);
+    if (lane == i) mine = m;
+  }
+  if (lane < 4 && w0 + lane < words_per_row) bitmap[(size_t)blockIdx.y * words_per_row + w0 + lane] = mine;
 }
 // prefix[w] = number of pairs before word w (over all offsets): the lists of the offsets follow one
-// another in pair_out / pair_in, starts[kappa] is where the list of offset kappa begins.
-__global__ void pair_scatter_kernel(const int32_t *__restrict__ nbr, int K, int n_out, int words_per_row,
-                                    const uint32_t *__restrict__ bitmap, const uint32_t *__restrict__ prefix,
-                                    int32_t *__restrict__ pair_out, int32_t *__restrict__ pair_in, int32_t *__restrict__ starts) {
-  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (gw >= (long long)K * words_per_row) return;
-  const int lane = threadIdx.x & 31;
-  const int kappa = (int)(gw / words_per_row), w = (int)(gw % words_per_row), r = w * 32 + lane;
-  const uint32_t m = bitmap[gw], base = prefix[gw];
-  if (w == 0 && lane == 0) starts[kappa] = (int32_t)base;
-  if ((m >> lane) & 1u) {
-    const uint32_t pos = base + (uint32_t)__popc(m & ((1u << lane) - 1u));
+// another in pair_out / pair_in, starts[kappa] is where the list of offset kappa begins.  A thread takes a
+// word: sparsely filled tables have a few set bits in each (a warp per word spent 96 us on the 22 M
+// entries of a 5^3 layer of 177 k rows, nine tenths of them absent).
+__global__ void __launch_bounds__(256)
+pair_scatter_kernel(const int32_t *__restrict__ nbr, int n_out, int words_per_row,
+                    const uint32_t *__restrict__ bitmap, const uint32_t *__restrict__ prefix,
+                    int32_t *__restrict__ pair_out, int32_t *__restrict__ pair_in, int32_t *__restrict__ starts) {
+  const int w = blockIdx.x * 256 + threadIdx.x, kappa = blockIdx.y;
+  if (w >= words_per_row) return;
+  uint32_t m = __ldg(bitmap + (size_t)kappa * words_per_row + w), pos = __ldg(prefix + (size_t)kappa * words_per_row + w);
+  if (w == 0) starts[kappa] = (int32_t)pos;
+  const int32_t *row = nbr + (size_t)kappa * n_out;
+  while (m != 0u) {
+    const int r = w * 32 + __ffs((int)m) - 1;
+    m &= m - 1u;
     pair_out[pos] = r;
-    pair_in[pos] = __ldg(nbr + (size_t)kappa * n_out + r);
+    pair_in[pos] = __ldg(row + r);
+    ++pos;
   }
 }
 
@@ -137,7 +152,7 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
   volatile int *abort_flag = &abort_word;
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
   const int S = p.stages, mma_warp = S;
   const int co0 = blockIdx.y * WT_M;
   if (tid == 0) {
@@ -255,39 +270,39 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
       par ^= 1u;
     }
   } else if (warp == mma_warp) {
-    // ====================================== MMA issuer =======================================
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(p.n_pad >> 3) << 17) | ((uint32_t)(WT_M >> 4) << 24);
-      int kappa = kappa0, seg = 0;
-      bool alive = true;
-      uint32_t s = 0, par = 0;
-      for (int q = q_begin; q < q_end && alive;) {
-        while (first[kappa + 1] <= q) ++kappa;
-        const int stop = min(q_end, first[kappa + 1]), buf = seg % p.n_buf, use = seg / p.n_buf;
-        if (use > 0) {
-          if (!mbar_wait(smem_u32(acce_bars + buf), (uint32_t)(use - 1) & 1u, abort_flag)) break;
-          tc_fence_after();
-        }
-        const uint32_t d = tmem_base + (uint32_t)buf * p.buf_cols;
-        for (const int q0 = q; q < stop; ++q) {
-          if (!mbar_wait(smem_u32(full_bars + s), par, abort_flag)) { alive = false; break; }
-          tc_fence_after();
-          const uint32_t a_lo = mn_desc_lo(smem_base + s * (uint32_t)p.stage_bytes);
-          const uint32_t b_lo = mn_desc_lo(smem_base + s * (uint32_t)p.stage_bytes + (uint32_t)p.a_bytes);
+    // ====================================== MMA issuer: the whole warp, one elected lane issues =====
+    const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(p.n_pad >> 3) << 17) | ((uint32_t)(WT_M >> 4) << 24);
+    int kappa = kappa0, seg = 0;
+    bool alive = true;
+    uint32_t s = 0, par = 0;
+    for (int q = q_begin; q < q_end && alive;) {
+      while (first[kappa + 1] <= q) ++kappa;
+      const int stop = min(q_end, first[kappa + 1]), buf = seg % p.n_buf, use = seg / p.n_buf;
+      if (use > 0) {
+        if (!mbar_wait_uniform(smem_u32(acce_bars + buf), (uint32_t)(use - 1) & 1u, abort_flag)) break;
+        tc_fence_after();
+      }
+      const uint32_t d = tmem_base + (uint32_t)buf * p.buf_cols;
+      for (const int q0 = q; q < stop; ++q) {
+        if (!mbar_wait_uniform(smem_u32(full_bars + s), par, abort_flag)) { alive = false; break; }
+        tc_fence_after();
+        const uint32_t a_lo = mn_desc_lo(smem_base + s * (uint32_t)p.stage_bytes);
+        const uint32_t b_lo = mn_desc_lo(smem_base + s * (uint32_t)p.stage_bytes + (uint32_t)p.a_bytes);
+        if (elect_one()) {
           mma_tf32_mn(d, a_lo, b_lo, idesc, q > q0 ? 1u : 0u);      // eight pairs per instruction: 1024 bytes apart
           mma_tf32_mn(d, a_lo + 64u, b_lo + 64u, idesc, 1u);
           mma_tf32_mn(d, a_lo + 128u, b_lo + 128u, idesc, 1u);
           mma_tf32_mn(d, a_lo + 192u, b_lo + 192u, idesc, 1u);
           mma_commit(smem_u32(empty_bars + s));
-          if (++s == (uint32_t)S) { s = 0; par ^= 1u; }
         }
-        if (alive) mma_commit(smem_u32(accf_bars + buf));
-        ++seg;
+        if (++s == (uint32_t)S) { s = 0; par ^= 1u; }
       }
-      // everything issued above (on any path) retires before the tensor memory is handed back
-      mma_commit(smem_u32(&done_bar));
-      mbar_wait_drain(smem_u32(&done_bar), 0u);
+      if (alive && elect_one()) mma_commit(smem_u32(accf_bars + buf));
+      ++seg;
     }
+    // everything issued above (on any path) retires before the tensor memory is handed back
+    if (elect_one()) mma_commit(smem_u32(&done_bar));
+    mbar_wait_drain(smem_u32(&done_bar), 0u);
   } else {
     // ====================================== epilogue ===========================================
     const int quarter = warp & 3;
@@ -442,11 +457,11 @@ PairLists pair_lists_view(void *lists, int K, int n_out) {
 // bitmap of the table, popcount scan, scatter: three small launches
 int pair_lists_build(const int32_t *nbr, int K, int n_out, void *lists, PairLists *out, cudaStream_t st) {
   const ListPlan p = plan_lists(lists, K, n_out);
-  { pair_bitmap_kernel<<<ceil_div(p.words * 32, 256), 256, 0, st>>>(nbr, K, n_out, p.wpr, p.bitmap); note_launches(1); }
+  { pair_bitmap_kernel<<<dim3(ceil_div(p.wpr, 32), K), 256, 0, st>>>(nbr, n_out, p.wpr, p.bitmap); note_launches(1); }
   SSC_CHECK_LAUNCH("pair_bitmap");
   int rc = exclusive_scan_u32<true>(p.bitmap, p.words, p.prefix, p.block_sums, p.starts + K, nullptr, st);
   if (rc != 0) return rc;
-  { pair_scatter_kernel<<<ceil_div(p.words * 32, 256), 256, 0, st>>>(nbr, K, n_out, p.wpr, p.bitmap, p.prefix, p.pair_out, p.pair_in, p.starts); note_launches(1); }
+  { pair_scatter_kernel<<<dim3(ceil_div(p.wpr, 256), K), 256, 0, st>>>(nbr, n_out, p.wpr, p.bitmap, p.prefix, p.pair_out, p.pair_in, p.starts); note_launches(1); }
   SSC_CHECK_LAUNCH("pair_scatter");
   if (out) *out = PairLists{p.pair_out, p.pair_in, p.starts};
   return SSC_OK;
