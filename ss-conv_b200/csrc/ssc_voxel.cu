@@ -289,15 +289,18 @@ __global__ void nn_tile_range_kernel(const float4 *__restrict__ known, int m, fl
   }
 }
 
-// 256 queries per block; known points stream through shared memory in tiles of 1024, tiles
-// whose batch-id range cannot match any query of the block are skipped.  Scan order and
-// comparisons equal the exhaustive reference loop (ascending k, strict <).
+// 64 queries per block, four threads per query; known points stream through shared memory in tiles of 1024,
+// tiles whose batch-id range cannot match any query of the block are skipped.  Thread s of a query
+// looks at every fourth point of a tile; the three best of the four are merged by (distance, index), which is
+// the result of the exhaustive reference loop (ascending k, strict <): the smallest index wins ties.
+// A thread per query left each SM with two blocks of one long serial scan: 150 us for 65 k queries.
+constexpr int NN_SPLIT = 4;
 __global__ void __launch_bounds__(256)
 three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known,
                 const float2 *__restrict__ ranges, float *__restrict__ dist2, int32_t *__restrict__ idx) {
   __shared__ float4 tile[NN_TILE];
   __shared__ float qmin_s[8], qmax_s[8];
-  int q = blockIdx.x * 256 + threadIdx.x;
+  const int q = blockIdx.x * (256 / NN_SPLIT) + (int)threadIdx.x / NN_SPLIT, part = threadIdx.x % NN_SPLIT;
   float4 u = q < n ? unknown[q] : make_float4(NAN, 0.f, 0.f, 0.f);
   float lo = q < n ? u.x : INFINITY, hi = q < n ? u.x : -INFINITY;
   for (int o = 16; o > 0; o >>= 1) {
@@ -314,41 +317,73 @@ three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *
     qmin = fminf(qmin, qmin_s[w]);
     qmax = fmaxf(qmax, qmax_s[w]);
   }
-  float best1 = INFINITY, best2 = INFINITY, best3 = INFINITY;
-  int i1 = 0, i2 = 0, i3 = 0;
-  int n_tiles = (m + NN_TILE - 1) / NN_TILE;
+  float best[3] = {INFINITY, INFINITY, INFINITY};
+  int at[3] = {0, 0, 0};
+  // (d, i) into the ordered triple; equal distances stay behind
+  auto take = [&](float d, int i) {
+    if (d < best[0]) {
+      best[2] = best[1]; at[2] = at[1];
+      best[1] = best[0]; at[1] = at[0];
+      best[0] = d; at[0] = i;
+    } else if (d < best[1]) {
+      best[2] = best[1]; at[2] = at[1];
+      best[1] = d; at[1] = i;
+    } else if (d < best[2]) {
+      best[2] = d; at[2] = i;
+    }
+  };
+  const int n_tiles = (m + NN_TILE - 1) / NN_TILE;
   for (int t = 0; t < n_tiles; ++t) {
-    float2 r = ranges[t];
+    const float2 r = ranges[t];
     if (r.y < qmin || r.x > qmax) continue;  // block-uniform
     __syncthreads();
-    int base = t * NN_TILE;
+    const int base = t * NN_TILE;
     for (int i = threadIdx.x; i < NN_TILE; i += 256) tile[i] = base + i < m ? known[base + i] : make_float4(NAN, 0.f, 0.f, 0.f);
     __syncthreads();
-    int cnt = min(NN_TILE, m - base);
+    const int cnt = min(NN_TILE, m - base);
     if (q < n && !(r.y < u.x || r.x > u.x)) {
-      for (int i = 0; i < cnt; ++i) {
-        float4 k = tile[i];
-        if (k.x != u.x) continue;
-        float dx = __fsub_rn(u.y, k.y), dy = __fsub_rn(u.z, k.z), dz = __fsub_rn(u.w, k.w);
+#pragma unroll 4
+      for (int i = part; i < cnt; i += NN_SPLIT) {
+        const float4 k = tile[i];
+        const float dx = __fsub_rn(u.y, k.y), dy = __fsub_rn(u.z, k.z), dz = __fsub_rn(u.w, k.w);
         // the contraction nvcc applies to the reference's dx*dx + dy*dy + dz*dz
         // (interpolate_cuda_kernel.cu:39), checked bit for bit against the reference's own kernel
-        float d = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
-        if (d < best1) {
-          best3 = best2; i3 = i2;
-          best2 = best1; i2 = i1;
-          best1 = d; i1 = base + i;
-        } else if (d < best2) {
-          best3 = best2; i3 = i2;
-          best2 = d; i2 = base + i;
-        } else if (d < best3) {
-          best3 = d; i3 = base + i;
-        }
+        const float d = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+        if (k.x == u.x && d < best[2]) take(d, base + i);
       }
     }
   }
-  if (q < n) {
-    dist2[q * 3 + 0] = best1; dist2[q * 3 + 1] = best2; dist2[q * 3 + 2] = best3;
-    idx[q * 3 + 0] = i1; idx[q * 3 + 1] = i2; idx[q * 3 + 2] = i3;
+  // merge the partners' triples (a slot that was never filled is infinite and loses to everything)
+#pragma unroll
+  for (int o = 1; o < NN_SPLIT; o <<= 1) {
+    float od[3];
+    int oi[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      od[k] = __shfl_xor_sync(0xffffffffu, best[k], o);
+      oi[k] = __shfl_xor_sync(0xffffffffu, at[k], o);
+    }
+    float md[3];
+    int mi[3], a = 0, c = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float da = a == 0 ? best[0] : a == 1 ? best[1] : best[2], dc = c == 0 ? od[0] : c == 1 ? od[1] : od[2];
+      const int ia = a == 0 ? at[0] : a == 1 ? at[1] : at[2], ic = c == 0 ? oi[0] : c == 1 ? oi[1] : oi[2];
+      const bool mine = da < dc || (da == dc && ia <= ic);
+      md[k] = mine ? da : dc;
+      mi[k] = mine ? ia : ic;
+      a += mine ? 1 : 0;
+      c += mine ? 0 : 1;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { best[k] = md[k]; at[k] = mi[k]; }
+  }
+  if (q < n && part == 0) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      dist2[q * 3 + k] = best[k];
+      idx[q * 3 + k] = best[k] == INFINITY ? 0 : at[k];
+    }
   }
 }
 
@@ -425,6 +460,83 @@ extern "C" size_t ssc_p2v_scratch_bytes(int n_point, int batch, const int grid[3
 // Feature steering: every point is moved into the frame of its sample, new_p = (p - t_b) . R_b
 // (/ (s_b + 1e-8)), and every irrep block of its feature row is multiplied from the right by the
 // sample's representation matrix D^l_b.  One thread per (point, output channel or coordinate).
+// Real Wigner-D matrices of the samples' rotations: D^l(R) = Y_l(R v) pinv(Y_l(v)) over fixed directions v (the
+// projection the host tables were made for), in double precision.  Real spherical harmonics at a unit
+// vector (x, y, z): sqrt(2) N P~_l^m(z) Re / Im (x + i y)^m with P~ the Legendre functions without their
+// sin^m factor (standard recurrences in l; no trigonometry).  A block per sample: a thread per direction puts the
+// harmonics of the rotated direction into shared memory, then a thread per matrix element adds them up.
+// dirs / pinv: per order l, 6 (2 l + 1) + 8 directions [S, 3] and the pseudo-inverse [S, 2 l + 1], one order after
+// the other.  axes != 0: the rotation is described in the frame whose polar axis is y (R -> S R S^T).
+__global__ void __launch_bounds__(128)
+steer_matrices_kernel(const float *__restrict__ rot, int orders, const double *__restrict__ dirs,
+                      const double *__restrict__ pinv, int axes, int stride, float *__restrict__ dmats) {
+  extern __shared__ double ys[];                 // per order [S][2 l + 1], as pinv
+  const int b = blockIdx.x;
+  double R[3][3], Q[3][3];
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) R[i][j] = (double)rot[(size_t)b * 9 + i * 3 + j];
+  const double det = R[0][0] * (R[1][1] * R[2][2] - R[1][2] * R[2][1]) - R[0][1] * (R[1][0] * R[2][2] - R[1][2] * R[2][0]) +
+                     R[0][2] * (R[1][0] * R[2][1] - R[1][1] * R[2][0]);
+  const double sign = det > 0.0 ? 1.0 : (det < 0.0 ? -1.0 : 0.0);
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) Q[i][j] = sign * (axes ? R[(i + 2) % 3][(j + 2) % 3] : R[i][j]);
+  int d0 = 0, p0 = 0;
+  for (int l = 0; l < orders; ++l) {
+    const int d = 2 * l + 1, s_cnt = 6 * d + 8;
+    for (int s = (int)threadIdx.x - (d0 / 3) % (int)blockDim.x; s < s_cnt; s += blockDim.x) {   // orders side by side over the threads
+      if (s < 0) continue;
+      const double vx = dirs[d0 + s * 3], vy = dirs[d0 + s * 3 + 1], vz = dirs[d0 + s * 3 + 2];
+      double x = Q[0][0] * vx + Q[0][1] * vy + Q[0][2] * vz, y = Q[1][0] * vx + Q[1][1] * vy + Q[1][2] * vz;
+      double z = Q[2][0] * vx + Q[2][1] * vy + Q[2][2] * vz;
+      z = z > 1.0 ? 1.0 : (z < -1.0 ? -1.0 : z);
+      const double xy = sqrt(x * x + y * y), want = sqrt(1.0 - z * z);   // the azimuth of (x, y) at the polar angle of z
+      if (xy > 0.0) {
+        x *= want / xy;
+        y *= want / xy;
+      } else {
+        x = want;
+        y = 0.0;
+      }
+      double re = 1.0, im = 0.0, pmm = 1.0, fact = (2.0 * l + 1.0) / 12.566370614359172954;   // fact: N^2 of order m
+      for (int m = 0; m <= l; ++m) {
+        if (m > 0) {
+          const double t = re * x - im * y;
+          im = re * y + im * x;
+          re = t;
+          pmm *= 2.0 * m - 1.0;
+          fact /= (double)(l + m) * (double)(l - m + 1);
+        }
+        double p_prev = 0.0, p = pmm;
+        for (int ll = m + 1; ll <= l; ++ll) {
+          const double t = ((2.0 * ll - 1.0) * z * p - (ll + m - 1.0) * p_prev) / (double)(ll - m);
+          p_prev = p;
+          p = t;
+        }
+        const double n = sqrt(fact) * (m > 0 ? 1.4142135623730950488 : 1.0) * p;
+        ys[p0 + s * d + l + m] = n * re;
+        if (m > 0) ys[p0 + s * d + l - m] = n * im;
+      }
+    }
+    d0 += 3 * s_cnt;
+    p0 += s_cnt * d;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < stride; e += blockDim.x) {
+    int l = 0, off = 0;
+    p0 = 0;
+    while (e >= off + (2 * l + 1) * (2 * l + 1)) {
+      off += (2 * l + 1) * (2 * l + 1);
+      p0 += (6 * (2 * l + 1) + 8) * (2 * l + 1);
+      ++l;
+    }
+    const int d = 2 * l + 1, row = (e - off) / d, col = (e - off) - row * d, s_cnt = 6 * d + 8;
+    double acc = 0.0;
+#pragma unroll 8
+    for (int s = 0; s < s_cnt; ++s) acc = fma(ys[p0 + s * d + row], pinv[p0 + s * d + col], acc);
+    dmats[(size_t)b * stride + e] = (float)acc;
+  }
+}
+
 __global__ void steer_kernel(const float *__restrict__ points, const float *__restrict__ feats,
                              const int32_t *__restrict__ ids, const float *__restrict__ rot, const float *__restrict__ trans,
                              const float *__restrict__ scale, const float *__restrict__ dmats, int d_stride,
@@ -455,6 +567,26 @@ __global__ void steer_kernel(const float *__restrict__ points, const float *__re
   float acc = 0.f;
   for (int i = 0; i < d; ++i) acc += feats[(size_t)p * c + start + i] * D[i * d + j];
   new_feats[(size_t)p * c + k] = acc;
+}
+
+extern "C" int ssc_steer_matrices(const float *rot, int batch, int orders, const double *dirs, const double *pinv, int axes,
+                                  float *dmats, void *stream) {
+  SSC_REQUIRE(batch >= 0 && orders >= 1 && orders <= 16, "steer_matrices: bad sizes");
+  if (batch == 0) return SSC_OK;
+  SSC_REQUIRE(rot && dirs && pinv && dmats, "steer_matrices: null pointer");
+  int stride = 0, harmonics = 0;
+  for (int l = 0; l < orders; ++l) {
+    stride += (2 * l + 1) * (2 * l + 1);
+    harmonics += (6 * (2 * l + 1) + 8) * (2 * l + 1);
+  }
+  const size_t smem = (size_t)harmonics * sizeof(double);       // 5 KB for orders 0..3, below 48 KB up to order 8
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(steer_matrices_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "steer_matrices: smem attribute: %s", cudaGetErrorString(e));
+  }
+  { steer_matrices_kernel<<<batch, 128, smem, as_stream(stream)>>>(rot, orders, dirs, pinv, axes, stride, dmats); note_launches(1); }
+  SSC_CHECK_LAUNCH("steer_matrices");
+  return SSC_OK;
 }
 
 extern "C" int ssc_steer_fwd(const float *points, const float *feats, const int32_t *ids, const float *rot,
@@ -559,7 +691,7 @@ extern "C" int ssc_three_nn(int n, int m, const float *unknown, const float *kno
     return fail(SSC_ERR_SCRATCH, "three_nn: scratch %zu < %zu bytes", scratch_bytes, (size_t)n_tiles * sizeof(float2));
   float2 *ranges = (float2 *)scratch;
   { nn_tile_range_kernel<<<n_tiles, 256, 0, st>>>((const float4 *)known, m, ranges); note_launches(1); }
-  { three_nn_kernel<<<ceil_div(n, 256), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, ranges, dist2, idx); note_launches(1); }
+  { three_nn_kernel<<<ceil_div(n, 256 / NN_SPLIT), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, ranges, dist2, idx); note_launches(1); }
   SSC_CHECK_LAUNCH("three_nn");
   return SSC_OK;
 }

@@ -79,6 +79,7 @@ SIGNATURES = {
     "ssc_global_maxpool_bwd": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
     "ssc_voxelize_bwd": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "ssc_three_interpolate_bwd": (c_int, [c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "ssc_steer_matrices": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
     "ssc_steer_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                               c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "ssc_p2v_stats": (c_int, [c_void_p, c_void_p, c_int, _I3, _F3, c_void_p, c_void_p]),
@@ -1174,6 +1175,16 @@ def voxelize_bp(d_output_feats, d_feats, map_rule, mode, n_voxel, max_active, c)
 voxelize_idx = _not_built("voxelize_idx")
 point_recover_fp = _not_built("point_recover_fp")
 point_recover_bp = _not_built("point_recover_bp")
+
+
+def steer_matrices(rot, dirs, pinv, orders, reference_frame):
+    """[B, sum (2l+1)^2] representation matrices of rotations [B, 3, 3] (ssc_steer_matrices); dirs / pinv: the
+    float64 tables of SO3.sample_tables on the same device."""
+    rot = rot.float().contiguous()
+    out = torch.empty((rot.shape[0], sum((2 * l + 1) ** 2 for l in range(orders))), dtype=torch.float32, device=rot.device)
+    _check(lib().ssc_steer_matrices(_p(rot), rot.shape[0], int(orders), _p(dirs, torch.float64), _p(pinv, torch.float64),
+                                    int(bool(reference_frame)), _p(out), _stream()))
+    return out
 
 
 def steer(points, feats, ids, rot, trans, scale, dmats, chan):

@@ -116,6 +116,14 @@ def _sample_dirs(l):
     return _SAMPLE_CACHE[l]
 
 
+def sample_tables(orders):
+    """(dirs, pinv): the sample directions and pseudo-inverses of orders 0 .. orders - 1 behind irr_repr, each as
+    one flat float64 tensor (the tables of the GPU form of D_from_matrix)."""
+    tabs = [_sample_dirs(l) for l in range(orders)]
+    return (torch.from_numpy(np.concatenate([v.reshape(-1) for v, _ in tabs])),
+            torch.from_numpy(np.concatenate([p.reshape(-1) for _, p in tabs])))
+
+
 def irr_repr(order, alpha, beta, gamma, dtype=None):
     """Real Wigner-D matrix of rot(alpha, beta, gamma) in the basis of `spherical_harmonics`:
     the matrix D with Y(R x) = D Y(x) for all x."""
