@@ -942,9 +942,6 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
   return SSC_OK;
 }
 
-// Smallest problem (in 128-row tiles) for which the extra staging launch pays for itself.
-constexpr int kStagingMinTiles = 8;
-
 int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed, int K, int c_out,
                   const int32_t *nbr, int n_out, float *out, int32_t *status, void *scratch, size_t scratch_bytes,
                   const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, cudaStream_t st) {
@@ -967,7 +964,9 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
   // layers with few input channels have their filters packed for several offsets per operand row,
   // which the kernel can only feed from the staged (padded) rows
   if (opk > 1 && !fits) return fail(SSC_ERR_SCRATCH, "conv_fwd(tf32): a layer with %d input channels needs the staging buffer (ssc_conv_scratch_bytes)", c_in);
-  const bool staged = fits && (prestaged || grid >= kStagingMinTiles || opk > 1);
+  // whoever brings a staging buffer gets the kernel that runs on staged rows: also a layer of a few tiles, whose
+  // CTAs are alone on their SMs (512 rows of 120 -> 240 channels: 104 us unstaged)
+  const bool staged = fits;
   if (staged && !prestaged) {
     int rc = stage_features(features, n_in, c_in, scratch, st);
     if (rc != SSC_OK) return rc;

@@ -603,9 +603,10 @@ def _resolve_precision(c_in, c_out, precision=None):
     return mode
 
 
-# Layers with fewer output rows do not stage a TF32-rounded copy of their input rows (the extra
-# launch would cost more than it saves), so no staging buffer is allocated for them.
-STAGING_MIN_ROWS = 8 * 128
+# Output rows from which a call brings a staging buffer (a copy of its input rows, rounded once): always, since
+# the kernel on staged rows is the faster one also for a layer of a few tiles (512 rows of 120 -> 240 channels:
+# 104 us without).  Raise it to save the buffer's memory; the results have the same bits.
+STAGING_MIN_ROWS = 0
 
 # Which tensor-core kernel a convolution call takes: 'auto' (by shape, see _use_pairs), 'rows' (the
 # output-stationary kernel: one CTA per 128 output rows, bitwise repeatable) or 'pairs' (the
@@ -705,15 +706,13 @@ def conv_prepare(features, filters, precision=None):
     filter image and the staged (TF32- or fp16-rounded) copy of the feature rows - queued on the
     current stream (meant to be a side stream running next to the rulebook kernels).  The
     conv_forward call on the same two tensors picks the result up.  Returns False when the call
-    would not use a staged image (exact fp32, small layers)."""
+    would not use a staged image (exact fp32, unstaged layers)."""
     flt = filters.reshape(-1, filters.shape[-2], filters.shape[-1])
     if not (flt.is_contiguous() and features.is_contiguous() and features.dtype == torch.float32):
         return False      # (16-bit features are their own staged image: nothing to prepare but the filters)
     K, c_in, c_out = flt.shape
     mode = _resolve_precision(c_in, c_out, precision)
-    if mode not in _PREC_OF or (mode != "tf32" and c_out > 512):
-        return False
-    if mode == "tf32" and features.shape[0] < STAGING_MIN_ROWS:
+    if mode not in _PREC_OF or (mode != "tf32" and c_out > 512) or (mode == "tf32" and features.shape[0] < STAGING_MIN_ROWS):
         return False
     prec = _PREC_OF[mode]
     packed = pack_filters(flt, prec)
@@ -964,7 +963,7 @@ def conv_backward(features, flt, out_bp, nbr, nbr_in=None, order=None, precision
     tf32_in = need[0] and _resolve_precision(c_out, c_in, precision) == "tf32" and not _use_pairs(
         flt.shape[0], c_out, c_in, n_in, PREC_TF32)
     tf32_flt = need[1] and c_in <= 256 and _resolve_precision(c_in, c_out, precision) in _PREC_OF
-    dy_image = stage_tf32(out_bp) if (tf32_in or tf32_flt) and out_bp.shape[0] >= STAGING_MIN_ROWS else None
+    dy_image = stage_tf32(out_bp) if tf32_in or tf32_flt else None
     # the two gradients do not depend on each other: while a graph is recorded the filter gradient
     # goes to a side stream, so the graph runs it next to the input gradient
     forked = need[0] and need[1] and torch.cuda.is_current_stream_capturing()
