@@ -253,6 +253,10 @@ int ssc_maxpool_fwd(const float *features, int c, const int32_t *nbr, int K, int
                     const int32_t *n_out_dev, void *stream);
 int ssc_avgpool_fwd(const float *features, int c, const int32_t *nbr, int K, int n_out,
                     const int32_t *summaryrf, float *out, const int32_t *n_out_dev, void *stream);
+/* The same on rows stored as fp16 / bf16 (precision; ssc_bn_gate_fwd16): the values are widened, the sums and the
+ * result are fp32.  average 0: maximum. */
+int ssc_pool_fwd16(const void *features, int precision, int average, int c, const int32_t *nbr, int K, int n_out,
+                   const int32_t *summaryrf, float *out, const int32_t *n_out_dev, void *stream);
 /* Replaces indiceSummaryRF (SS_Conv_lib/src/pool/indiceSummaryRF.cu:21-63). */
 int ssc_summary_rf(const int32_t *nbr, int K, int n_out, int32_t *rf, void *stream);
 

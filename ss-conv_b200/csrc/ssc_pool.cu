@@ -1,49 +1,74 @@
 // Sparse max / avg pooling over the output-major neighbour table (one launch, each output
 // row written once) and per-sample global pooling.  All HBM-bound.
+#include <cuda_fp16.h>
+
 #include "ssc_common.cuh"
+#include "ssc_pool_tile.cuh"
 
 namespace ssc {
 
-// MODE 0 = max (output starts at 0), 1 = avg (sum of x / divisor in ascending offset order).
-// One thread per (output row, 4 channels).
-template <int MODE, bool VEC>
-__global__ void pool_fwd_kernel(const float *__restrict__ features, int c, const int32_t *__restrict__ nbr, int K,
-                                int n_out, const int32_t *__restrict__ summaryrf, float *__restrict__ out,
-                                const int32_t *__restrict__ n_out_dev) {
-  int cg = (c + 3) >> 2;
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)live_rows(n_out, n_out_dev) * cg) return;  // n_out stays the row stride of nbr
-  int o = (int)(t / cg);
-  int c0 = (int)(t - (long long)o * cg) * 4;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  float div = 1.f;
-  if (MODE == 1) div = summaryrf ? (float)summaryrf[o] : (float)K;
-  for (int kappa = 0; kappa < K; ++kappa) {
-    int src = __ldg(nbr + (size_t)kappa * n_out + o);
-    if (src < 0) continue;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    const float *fp = features + (size_t)src * c + c0;
-    if (VEC) {
-      float4 f = __ldg((const float4 *)fp);
-      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+// Rows of fp32, fp16 or bf16 (IN = 0, 1, 2) channels, four at a time or one.
+template <int IN, int VEC>
+__device__ __forceinline__ void load_channels(const void *__restrict__ rows, size_t at, float (&v)[VEC]) {
+  if (IN == 0) {
+    const float *p = (const float *)rows + at;
+    if (VEC == 4) {
+      const float4 f = __ldg((const float4 *)p);
+      v[0] = f.x; v[1 % VEC] = f.y; v[2 % VEC] = f.z; v[3 % VEC] = f.w;
     } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (c0 + q < c) v[q] = __ldg(fp + q);
+      v[0] = __ldg(p);
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (MODE == 0) acc[q] = v[q] > acc[q] ? v[q] : acc[q];
-      else acc[q] = acc[q] + v[q] / div;
-    }
-  }
-  float *op = out + (size_t)o * c + c0;
-  if (VEC) {
-    *(float4 *)op = make_float4(acc[0], acc[1], acc[2], acc[3]);
   } else {
+    const uint16_t *p = (const uint16_t *)rows + at;
+    uint16_t h[4];
+    if (VEC == 4) {
+      const uint2 w = __ldg((const uint2 *)p);
+      h[0] = (uint16_t)w.x; h[1] = (uint16_t)(w.x >> 16); h[2] = (uint16_t)w.y; h[3] = (uint16_t)(w.y >> 16);
+    } else {
+      h[0] = __ldg(p);
+    }
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (c0 + q < c) op[q] = acc[q];
+    for (int q = 0; q < VEC; ++q) v[q] = IN == 2 ? __uint_as_float((uint32_t)h[q] << 16) : __half2float(__ushort_as_half(h[q]));
+  }
+}
+
+// MODE 0 = max (output starts at 0), 1 = avg (sum of x / divisor in ascending offset order).
+// A block takes R output rows.  Most table entries are absent (a strided 3^3 pool over surface voxels: 1.5 of 27 per
+// row), and what bounded one thread per (row, 4 channels) walking the table was that walk, done once
+// per channel group: 74 us for 27 offsets of 140 k rows of 76 channels.  Here the block brings its piece of the table into shared memory
+// once, with a presence mask per row, and the threads then visit only what is there: 35 us.
+template <int MODE, int IN, int VEC>
+__global__ void __launch_bounds__(256)
+pool_fwd_kernel(const void *__restrict__ features, int c, const int32_t *__restrict__ nbr, int K,
+                int n_out, const int32_t *__restrict__ summaryrf, float *__restrict__ out,
+                const int32_t *__restrict__ n_out_dev, int R) {
+  extern __shared__ int32_t pool_smem[];
+  const PoolTile tile = pool_tile(nbr, K, n_out, live_rows(n_out, n_out_dev), R, pool_smem);   // n_out: row stride of nbr
+  const uint32_t cg = (uint32_t)(c / VEC), items = (uint32_t)tile.rows * cg;
+  for (uint32_t t = threadIdx.x; t < items; t += 256) {
+    const int r = (int)(t / cg), c0 = (int)(t - (uint32_t)r * cg) * VEC;
+    const int o = tile.first + r;
+    float acc[VEC];
+#pragma unroll
+    for (int q = 0; q < VEC; ++q) acc[q] = 0.f;
+    float div = 1.f;
+    if (MODE == 1) div = summaryrf ? (float)__ldg(summaryrf + o) : (float)K;
+    const float inv = __frcp_rn(div);
+    pool_visit(tile, r, K, [&](int src) {
+      float v[VEC];
+      load_channels<IN, VEC>(features, (size_t)src * c + c0, v);
+#pragma unroll
+      for (int q = 0; q < VEC; ++q) {
+        if (MODE == 0) acc[q] = v[q] > acc[q] ? v[q] : acc[q];
+        else acc[q] = acc[q] + divide_by_count(v[q], div, inv);
+      }
+    });
+    float *op = out + (size_t)o * c + c0;
+    if (VEC == 4) {
+      *(float4 *)op = make_float4(acc[0], acc[1 % VEC], acc[2 % VEC], acc[3 % VEC]);
+    } else {
+      op[0] = acc[0];
+    }
   }
 }
 
@@ -99,13 +124,16 @@ __global__ void global_pool_kernel(const float *__restrict__ feats, const int32_
   }
 }
 
-// offsets[b+1] = number of rows with batch id <= b: histogram, then an in-place scan by one warp.
+// offsets[b+1] = number of rows with batch id <= b: histogram, then an in-place scan by one warp.  Rows of a
+// sample follow one another nearly always: the lanes of a warp with the same id send one atomic (one per
+// row queued up at a single address: 38 us for 138 k rows).
 __global__ void batch_count_kernel(const int4 *__restrict__ indices, int n, int batch, int32_t *offsets,
                                    const int32_t *__restrict__ n_dev) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= live_rows(n, n_dev)) return;
-  int b = indices[i].x;
-  if ((unsigned)b < (unsigned)batch) atomicAdd(offsets + b + 1, 1);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int b = -1;
+  if (i < live_rows(n, n_dev)) b = __ldg((const int32_t *)(indices + i));
+  const unsigned same = __match_any_sync(0xffffffffu, b);
+  if ((unsigned)b < (unsigned)batch && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(offsets + b + 1, __popc(same));
 }
 
 __global__ void batch_scan_kernel(int32_t *offsets, int batch) {
@@ -128,30 +156,45 @@ __global__ void batch_scan_kernel(int32_t *offsets, int batch) {
 
 using namespace ssc;
 
-template <int MODE>
-static int launch_pool(const float *features, int c, const int32_t *nbr, int K, int n_out, const int32_t *rf,
+template <int MODE, int IN>
+static int launch_pool(const void *features, int c, const int32_t *nbr, int K, int n_out, const int32_t *rf,
                        float *out, const int32_t *n_out_dev, void *stream, const char *name) {
   SSC_REQUIRE(c > 0 && K > 0 && n_out >= 0, "%s: bad sizes", name);
   if (n_out == 0) return SSC_OK;
   SSC_REQUIRE(features && nbr && out, "%s: null pointer", name);
-  long long threads = (long long)n_out * ((c + 3) / 4);
-  bool vec = (c % 4 == 0) && (((uintptr_t)features | (uintptr_t)out) % 16 == 0);
-  if (vec)
-    { pool_fwd_kernel<MODE, true><<<ceil_div(threads, 256), 256, 0, as_stream(stream)>>>(features, c, nbr, K, n_out, rf, out, n_out_dev); note_launches(1); }
-  else
-    { pool_fwd_kernel<MODE, false><<<ceil_div(threads, 256), 256, 0, as_stream(stream)>>>(features, c, nbr, K, n_out, rf, out, n_out_dev); note_launches(1); }
+  const bool vec = (c % 4 == 0) && (((uintptr_t)features | (uintptr_t)out) % 16 == 0);
+  const PoolShape p = pool_shape(n_out, K);
+  SSC_REQUIRE(p.rows > 0, "%s: kernel of %d offsets is too large", name, K);
+  if (p.smem > 48 * 1024) {
+    cudaError_t e = vec ? cudaFuncSetAttribute(pool_fwd_kernel<MODE, IN, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem)
+                        : cudaFuncSetAttribute(pool_fwd_kernel<MODE, IN, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "%s: smem attribute: %s", name, cudaGetErrorString(e));
+  }
+  if (vec) pool_fwd_kernel<MODE, IN, 4><<<p.grid, 256, p.smem, as_stream(stream)>>>(features, c, nbr, K, n_out, rf, out, n_out_dev, p.rows);
+  else pool_fwd_kernel<MODE, IN, 1><<<p.grid, 256, p.smem, as_stream(stream)>>>(features, c, nbr, K, n_out, rf, out, n_out_dev, p.rows);
+  note_launches(1);
   SSC_CHECK_LAUNCH(name);
   return SSC_OK;
 }
 
 extern "C" int ssc_maxpool_fwd(const float *features, int c, const int32_t *nbr, int K, int n_out, float *out,
                                const int32_t *n_out_dev, void *stream) {
-  return launch_pool<0>(features, c, nbr, K, n_out, nullptr, out, n_out_dev, stream, "maxpool_fwd");
+  return launch_pool<0, 0>(features, c, nbr, K, n_out, nullptr, out, n_out_dev, stream, "maxpool_fwd");
 }
 
 extern "C" int ssc_avgpool_fwd(const float *features, int c, const int32_t *nbr, int K, int n_out,
                                const int32_t *summaryrf, float *out, const int32_t *n_out_dev, void *stream) {
-  return launch_pool<1>(features, c, nbr, K, n_out, summaryrf, out, n_out_dev, stream, "avgpool_fwd");
+  return launch_pool<1, 0>(features, c, nbr, K, n_out, summaryrf, out, n_out_dev, stream, "avgpool_fwd");
+}
+
+extern "C" int ssc_pool_fwd16(const void *features, int precision, int average, int c, const int32_t *nbr, int K, int n_out,
+                              const int32_t *summaryrf, float *out, const int32_t *n_out_dev, void *stream) {
+  SSC_REQUIRE(precision == SSC_PREC_F16 || precision == SSC_PREC_BF16, "pool_fwd16: precision must be SSC_PREC_F16 or SSC_PREC_BF16");
+  if (precision == SSC_PREC_BF16)
+    return average ? launch_pool<1, 2>(features, c, nbr, K, n_out, summaryrf, out, n_out_dev, stream, "pool_fwd16")
+                   : launch_pool<0, 2>(features, c, nbr, K, n_out, nullptr, out, n_out_dev, stream, "pool_fwd16");
+  return average ? launch_pool<1, 1>(features, c, nbr, K, n_out, summaryrf, out, n_out_dev, stream, "pool_fwd16")
+                 : launch_pool<0, 1>(features, c, nbr, K, n_out, nullptr, out, n_out_dev, stream, "pool_fwd16");
 }
 
 extern "C" int ssc_summary_rf(const int32_t *nbr, int K, int n_out, int32_t *rf, void *stream) {

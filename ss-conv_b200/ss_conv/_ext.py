@@ -85,6 +85,7 @@ SIGNATURES = {
     "ssc_p2v_stats": (c_int, [c_void_p, c_void_p, c_int, _I3, _F3, c_void_p, c_void_p]),
     "ssc_maxpool_fwd": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "ssc_avgpool_fwd": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "ssc_pool_fwd16": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "ssc_summary_rf": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "ssc_global_avgpool_fwd": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "ssc_global_maxpool_fwd": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
@@ -769,9 +770,7 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
     elif mode in _PREC_OF:
         prec = _PREC_OF[mode]
         packed = _packed_filters(filters, prec)
-        # the 16-bit kernels always gather from their staged image
-        # (layers with up to 16 input channels have filters packed for several offsets per operand row,
-        #  which the kernel feeds from the staged rows only)
+        # (the 16-bit kernels and layers with up to 16 input channels know the staged form only)
         stage = prec != PREC_TF32 or n_out >= STAGING_MIN_ROWS or c_in <= 16
         nbytes = lib().ssc_conv_scratch_bytes(features.shape[0], c_in, c_out, prec) if stage else 0
         scratch = torch.empty(nbytes, dtype=torch.uint8, device=features.device) if nbytes else None
@@ -1051,23 +1050,30 @@ def indice_conv_backward_half(features, filters, out_bp, indice_pairs, indice_nu
 
 
 # ================================================================================== pools
-def indice_maxpool_fp32(features, indice_pairs, indice_num, num_act):
-    features = features.contiguous()
-    nbr, n_out_dev = _table_for(indice_pairs, indice_num, int(num_act))
-    out = torch.empty((int(num_act), features.shape[1]), dtype=torch.float32, device=features.device)
-    _check(lib().ssc_maxpool_fwd(_p(features, torch.float32), features.shape[1], _p(nbr), nbr.shape[0], int(num_act),
-                                 _p(out), _p(n_out_dev), _stream()))
-    return out
-
-
-def indice_avgpool_fp32(features, indice_pairs, indice_num, num_act, summaryrf):
+def _pool(features, indice_pairs, indice_num, num_act, average, summaryrf=None):
     features = features.contiguous()
     nbr, n_out_dev = _table_for(indice_pairs, indice_num, int(num_act))
     out = torch.empty((int(num_act), features.shape[1]), dtype=torch.float32, device=features.device)
     rf = None if summaryrf is None else summaryrf.to(torch.int32).contiguous()
-    _check(lib().ssc_avgpool_fwd(_p(features, torch.float32), features.shape[1], _p(nbr), nbr.shape[0], int(num_act),
-                                 _p(rf), _p(out), _p(n_out_dev), _stream()))
+    c, K = features.shape[1], nbr.shape[0]
+    if features.dtype in _PREC_OF_DTYPE:     # rows stored in 16 bits by a gated Activation
+        _check(lib().ssc_pool_fwd16(_p(features), _PREC_OF[_PREC_OF_DTYPE[features.dtype]], int(average), c, _p(nbr), K,
+                                    int(num_act), _p(rf), _p(out), _p(n_out_dev), _stream()))
+    elif average:
+        _check(lib().ssc_avgpool_fwd(_p(features, torch.float32), c, _p(nbr), K, int(num_act), _p(rf), _p(out),
+                                     _p(n_out_dev), _stream()))
+    else:
+        _check(lib().ssc_maxpool_fwd(_p(features, torch.float32), c, _p(nbr), K, int(num_act), _p(out), _p(n_out_dev),
+                                     _stream()))
     return out
+
+
+def indice_maxpool_fp32(features, indice_pairs, indice_num, num_act):
+    return _pool(features, indice_pairs, indice_num, num_act, False)
+
+
+def indice_avgpool_fp32(features, indice_pairs, indice_num, num_act, summaryrf):
+    return _pool(features, indice_pairs, indice_num, num_act, True, summaryrf)
 
 
 def indiceSummaryRF(indice_pairs, indice_num, num_act):
@@ -1082,14 +1088,14 @@ def indice_maxpool_half(features, indice_pairs, indice_num, num_act):
     widened values (a maximum of fp16 values is exact), the result is narrowed again."""
     if features.dtype != torch.half:
         raise TypeError("indice_maxpool_half expects float16 features")
-    return indice_maxpool_fp32(features.float(), indice_pairs, indice_num, num_act).half()
+    return _pool(features, indice_pairs, indice_num, num_act, False).half()
 
 
 def indice_avgpool_half(features, indice_pairs, indice_num, num_act, summaryrf):
     """(SS_Conv_lib/src/ss_conv_ops.h:62) half tensors in and out, sums in fp32, one rounding at the end."""
     if features.dtype != torch.half:
         raise TypeError("indice_avgpool_half expects float16 features")
-    return indice_avgpool_fp32(features.float(), indice_pairs, indice_num, num_act, summaryrf).half()
+    return _pool(features, indice_pairs, indice_num, num_act, True, summaryrf).half()
 def indice_maxpool_backward_fp32(features, out_features, out_bp, indice_pairs, indice_num):
     """(SS_Conv_lib/src/ss_conv_ops.h:58-59) gradient to every input that equals its pooled value."""
     features, out_features, out_bp = features.contiguous(), out_features.contiguous(), out_bp.contiguous()

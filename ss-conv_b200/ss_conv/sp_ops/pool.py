@@ -9,7 +9,7 @@ from .functional import indice_avgpool, indice_maxpool
 
 
 class _SparsePool(nn.Module):
-    _op = None
+    _op = _stored16 = None
 
     def __init__(self, ndim, kernel_size, stride=1, padding=0, dilation=1, subm=False):
         super().__init__()
@@ -28,17 +28,18 @@ class _SparsePool(nn.Module):
         out_shape = shape if self.subm else get_conv_output_size(shape, self.kernel_size, self.stride, self.padding,
                                                                  self.dilation)
         feats_raw, inds_raw, n_in_dev = input.raw()
-        if feats_raw.dtype in (torch.float16, torch.bfloat16):
-            # features stored in 16 bits by a gated Activation: the pools compute in fp32
+        stored16 = feats_raw.dtype in (torch.float16, torch.bfloat16)
+        if stored16 and (torch.is_grad_enabled() and feats_raw.requires_grad or not feats_raw.is_cuda):
             input._features = feats_raw = feats_raw.float()
-        if (_ext.AHEAD and not self.subm and feats_raw.is_cuda and feats_raw.dtype == torch.float32
+            stored16 = False
+        if (_ext.AHEAD and not self.subm and feats_raw.is_cuda and (stored16 or feats_raw.dtype == torch.float32)
                 and not (torch.is_grad_enabled() and feats_raw.requires_grad)):
             ahead, indices_ready = _ext.rulebook_next_to_features(input._rows, lambda: _ext.get_indice_pairs_ahead(
                 inds_raw, input.batch_size, out_shape, list(shape), self.kernel_size, self.stride, self.padding,
                 self.dilation, 0, n_in_dev=n_in_dev))
             if ahead is not None:
                 outids_cap, pairs, pair_num = ahead
-                feats_cap = type(self)._op(feats_raw, pairs, pair_num, pairs.capacity)
+                feats_cap = self._pool(feats_raw, pairs, pair_num, pairs.capacity)
                 out = SparseTensor(feats_cap, outids_cap, out_shape, input.batch_size)
                 out.indice_dict = input.indice_dict
                 out.grid = input.grid
@@ -55,11 +56,17 @@ class _SparsePool(nn.Module):
                 return out
         return self._forward_exact(input, out_shape)
 
+    def _pool(self, features, pairs, pair_num, n_out):
+        """Features stored in 16 bits by a gated Activation are widened as the pool reads them: fp32 sums and result."""
+        if features.dtype in (torch.float16, torch.bfloat16):
+            return self._stored16(features, pairs, pair_num, n_out)
+        return type(self)._op(features, pairs, pair_num, n_out)
+
     def _forward_exact(self, input, out_shape):
         outids, pairs, pair_num = get_indice_pairs(input.indices, input.batch_size, input.spatial_shape,
                                                    self.kernel_size, self.stride, self.padding, self.dilation, 0,
                                                    self.subm, lazy=True)
-        feats = type(self)._op(input.features, pairs, pair_num, outids.shape[0])
+        feats = self._pool(input.features, pairs, pair_num, outids.shape[0])
         out = SparseTensor(feats, outids, out_shape, input.batch_size)
         out.indice_dict = input.indice_dict
         out.grid = input.grid
@@ -69,8 +76,10 @@ class _SparsePool(nn.Module):
 class SparseAvgPool(_SparsePool):
     """out = (sum of present inputs) / kernel volume."""
     _op = staticmethod(indice_avgpool)
+    _stored16 = staticmethod(lambda *a: _ext._pool(*a, True))
 
 
 class SparseMaxPool(_SparsePool):
     """out = max(0, max of present inputs): the output starts from zero."""
     _op = staticmethod(indice_maxpool)
+    _stored16 = staticmethod(lambda *a: _ext._pool(*a, False))

@@ -1,0 +1,117 @@
+"""Kernels and dispatch branches at the sizes where they can go wrong: edges of tiles, remainders, the smallest
+and the largest of a range."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_helpers import dev, gpu_rulebook, random_voxels, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _table(nbr_rows, n_in, K, present, rng):
+    t = rng.randint(0, n_in, (K, nbr_rows)).astype(np.int32)
+    t[rng.rand(K, nbr_rows) >= present] = -1
+    return t
+
+
+@pytest.mark.parametrize("n_in,n_out,c,K,dtype", [(1, 1, 4, 1, torch.float32), (40, 33, 20, 27, torch.float32),
+                                                  (500, 64, 7, 32, torch.float32), (300, 257, 36, 125, torch.float32),
+                                                  (200, 65, 8, 400, torch.float32), (90, 31, 12, 27, torch.float16),
+                                                  (90, 33, 5, 8, torch.bfloat16)])
+def test_pools_at_tile_edges(cuda, n_in, n_out, c, K, dtype):
+    """Pools over arbitrary tables: rows around the 32 of a block, more offsets than a mask word, channels that are no
+    multiple of four, rows stored in 16 bits.  Quotients are correctly rounded (zeros, tiny, huge and infinite
+    values among them), maxima exact, and the sums run in ascending offset order: same bits as the
+    plain loop."""
+    from ss_conv import _ext
+    from ss_conv._ext import lib, _p, _stream, _check
+    rng = np.random.RandomState(K + n_out)
+    t = dev(_table(n_out, n_in, K, 0.3, rng), cuda)
+    x = rng.randn(n_in, c).astype(np.float32)
+    x[rng.rand(n_in, c) < .3] = 0
+    if dtype == torch.float32:
+        x[rng.rand(n_in, c) < .05] *= np.float32(1e-36)
+        x[rng.rand(n_in, c) < .05] *= np.float32(1e32)
+        x[0, 0] = np.inf
+    x = dev(x, cuda).to(dtype)
+    xf = torch.cat([x.float(), torch.zeros(1, c, device=cuda)])           # row -1: absent
+    count = dev(rng.randint(1, 30, n_out).astype(np.int32), cuda)
+    for average, rf in ((False, None), (True, None), (True, count)):
+        out, want = torch.empty(n_out, c, device=cuda), torch.zeros(n_out, c, device=cuda)
+        div = (torch.full((n_out,), K, device=cuda) if rf is None else rf).float()[:, None]
+        for k in range(K):
+            v = xf[t[k].long()]
+            want = torch.where((t[k] >= 0)[:, None], want + v / div if average else torch.maximum(want, v), want)
+        if dtype != torch.float32:
+            _check(lib().ssc_pool_fwd16(_p(x), _ext.PREC_F16 if dtype == torch.float16 else _ext.PREC_BF16, int(average), c,
+                                        _p(t), K, n_out, _p(rf), _p(out), None, _stream()))
+        elif average:
+            _check(lib().ssc_avgpool_fwd(_p(x), c, _p(t), K, n_out, _p(rf), _p(out), None, _stream()))
+        else:
+            _check(lib().ssc_maxpool_fwd(_p(x), c, _p(t), K, n_out, _p(out), None, _stream()))
+        assert torch.equal(out, want)
+        if dtype != torch.float32:
+            continue
+        # gradients: the same table read as [K, rows that receive]
+        g, src = torch.randn(n_in, c, device=cuda), torch.cat([out, out])[:n_out]
+        y = dev(rng.randn(n_in, c).astype(np.float32), cuda).round()
+        xi, d = src.round(), torch.empty(n_out, c, device=cuda)
+        gz, yz, want = torch.cat([g, xf[-1:]]), torch.cat([y, xf[-1:]]), torch.zeros(n_out, c, device=cuda)
+        rf_in = None if rf is None else dev(rng.randint(1, 30, n_in).astype(np.int32), cuda)
+        div = torch.cat([torch.full((n_in,), K, device=cuda) if rf is None else rf_in, torch.ones(1, dtype=torch.int32, device=cuda)])
+        for k in range(K):
+            o, on = t[k].long(), (t[k] >= 0)[:, None]
+            want = torch.where(on, want + gz[o] / div[o].float()[:, None], want) if average else torch.where(on & (yz[o] == xi), want + gz[o], want)
+        if average:
+            _check(lib().ssc_avgpool_bwd(_p(g), c, _p(t), K, n_out, _p(rf_in), _p(d), _stream()))
+        else:
+            _check(lib().ssc_maxpool_bwd(_p(xi), _p(y), _p(g), c, _p(t), K, n_out, _p(d), _stream()))
+        assert torch.equal(d, want)
+
+
+@pytest.mark.parametrize("c_in,c_out,k,n", [(1, 1, 1, 1), (2, 40, 3, 129), (3, 36, 3, 700), (4, 38, 3, 300), (3, 70, 5, 130)])
+def test_fp32_convolution_of_few_input_channels(cuda, c_in, c_out, k, n):
+    """The exact kernel for up to four input channels: rows around a block, output channels that are no multiple
+    of four, more offsets than one pass holds.  Bound: the fp32 error of a sum of present * c_in products, a few ulp."""
+    from ss_conv import _ext
+    import ssconv_oracle as O
+    rng = np.random.RandomState(n)
+    ind = random_voxels(rng, 1, 12, n)
+    feats, W = rng.randn(len(ind), c_in).astype(np.float32), rng.randn(k, k, k, c_in, c_out).astype(np.float32)
+    outids, pairs, num = gpu_rulebook(ind, 1, [12] * 3, k, 1, k // 2, 1, True, cuda)
+    _ext.set_precision("fp32")
+    try:
+        y = _ext.indice_conv_fp32(dev(feats, cuda), dev(W, cuda), pairs, num, outids.shape[0], 0, 1).cpu().numpy()
+    finally:
+        _ext.set_precision("auto")
+    ref = O.indice_conv_f64(feats, W, pairs.cpu().numpy(), num.cpu().numpy(), outids.shape[0])
+    assert rel_err(y, ref) <= 2e-5
+
+
+@pytest.mark.parametrize("orders,batch", [(1, 1), (4, 65), (8, 3)])
+@pytest.mark.parametrize("frame", ["kernel", "reference"])
+def test_steering_matrices_match_the_host_form(cuda, orders, batch, frame):
+    """Representation matrices made on the GPU in double precision against the host's, rounded to fp32: entries are
+    at most 1, so 1e-6 allows for the last bit and the rounding of double-precision sums."""
+    from ss_conv import _ext
+    from ss_conv.utils import SO3
+    rng = np.random.RandomState(orders)
+    q, r = np.linalg.qr(rng.randn(batch, 3, 3))
+    q = q * np.sign(np.linalg.det(q))[:, None, None]
+    q[0] = np.eye(3)
+    rot = torch.from_numpy(q.astype(np.float32))
+    got = _ext.steer_matrices(rot.to(cuda), *(t.to(cuda) for t in SO3.sample_tables(orders)), orders, frame == "reference")
+    want = torch.cat([SO3.D_from_matrix(rot.double(), l, frame).reshape(batch, -1) for l in range(orders)], dim=1)
+    assert float((got.cpu().double() - want.double()).abs().max()) <= 1e-6
+
+
+@pytest.mark.parametrize("n_query,n_known", [(1, 3), (63, 4), (65, 5), (130, 257)])
+def test_three_nearest_with_ties(cuda, n_query, n_known):
+    """Coordinates on a coarse lattice (many equal distances, all exact): the smallest index first among equals."""
+    from ss_conv.sp_ops.functional import three_nn
+    rng = np.random.RandomState(n_known)
+    q, k = (dev(np.concatenate([np.zeros((n, 1)), rng.randint(0, 3, (n, 3))], 1).astype(np.float32), cuda) for n in (n_query, n_known))
+    dist, idx = three_nn(q, k)
+    want, order = torch.sort(((q[:, None] - k[None]) ** 2).sum(-1), dim=1, stable=True)
+    assert torch.equal(dist, want[:, :3].sqrt()) and torch.equal(idx.long(), order[:, :3])
