@@ -1,5 +1,6 @@
 // Irrep-wise BatchNorm (eval: folded per-channel affine; train: statistics) and the gated
 // activation, as single elementwise passes.  HBM-bound.
+#include "ssc_act.cuh"
 #include "ssc_common.cuh"
 #include "ssc_tc_ptx.cuh"
 
@@ -20,12 +21,6 @@ __global__ void bn_fold_kernel(const float *running_mean, const float *running_v
   }
   scale[ch] = sc;
   shift[ch] = sh;
-}
-
-__device__ __forceinline__ float apply_act(float v, int kind) {
-  if (kind == 1) return v > 0.f ? v : 0.f;
-  if (kind == 2) return __frcp_rn(1.0f + expf(-v));   // the correctly rounded reciprocal: the bits of 1.0f / (...)
-  return v;
 }
 
 // One thread per output element (any channel counts / alignment).

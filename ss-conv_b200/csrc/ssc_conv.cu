@@ -352,10 +352,35 @@ extern "C" int ssc_conv_fwd_ordered(const float *features, int n_in, int c_in, c
     SSC_CHECK_LAUNCH("conv_fwd_fp32");
     return SSC_OK;
   }
-  if (precision == SSC_PREC_TF32) return conv_fwd_tf32(features, n_in, c_in, filters, K, c_out, nbr, n_out, out, status, scratch, scratch_bytes, n_out_dev, row_order, prestaged, table_form, st);
+  if (precision == SSC_PREC_TF32) return conv_fwd_tf32(features, n_in, c_in, filters, K, c_out, nbr, n_out, out, status, scratch, scratch_bytes, n_out_dev, row_order, prestaged, table_form, GateEpilogue{}, st);
   if (precision == SSC_PREC_F16 || precision == SSC_PREC_BF16)
-    return conv_fwd_16(features, n_in, c_in, precision == SSC_PREC_BF16, filters, K, c_out, nbr, n_out, out, status, scratch, scratch_bytes, n_out_dev, row_order, prestaged, table_form, st);
+    return conv_fwd_16(features, n_in, c_in, precision == SSC_PREC_BF16, filters, K, c_out, nbr, n_out, out, status, scratch, scratch_bytes, n_out_dev, row_order, prestaged, table_form, GateEpilogue{}, st);
   return fail(SSC_ERR_INVALID, "conv_fwd: unknown precision %d", precision);
+}
+
+extern "C" int ssc_conv_gate_covered(int c_in, int c_out, int c_keep, int precision, int n_out) {
+  return conv_gate_covered(c_in, c_out, c_keep, precision, n_out) ? 1 : 0;
+}
+
+extern "C" int ssc_conv_fwd_gated(const float *features, int n_in, int c_in, const void *filters, int K, int c_out,
+                                  const int32_t *nbr, int n_out, int precision, const float *scale, const float *shift,
+                                  const int32_t *gate_of_channel, int c_keep, int scalar_act, int gate_act, int out_precision,
+                                  void *out, int32_t *status, void *scratch, size_t scratch_bytes, const int32_t *n_out_dev,
+                                  void *stream) {
+  SSC_REQUIRE(c_in > 0 && c_out > 0 && K > 0 && n_in >= 0 && n_out >= 0, "conv_fwd_gated: bad sizes");
+  const bool prestaged = (precision & SSC_CONV_PRESTAGED) != 0;
+  precision &= ~SSC_CONV_PRESTAGED;
+  SSC_REQUIRE(conv_gate_covered(c_in, c_out, c_keep, precision, n_out), "conv_fwd_gated: %d -> %d (%d kept) channels at precision %d are not covered", c_in, c_out, c_keep, precision);
+  SSC_REQUIRE(out_precision == SSC_PREC_FP32 || ((out_precision == SSC_PREC_F16 || out_precision == SSC_PREC_BF16) && c_keep % 8 == 0),
+              "conv_fwd_gated: rows of %d channels cannot be stored at precision %d", c_keep, out_precision);
+  if (n_out == 0) return SSC_OK;
+  SSC_REQUIRE(filters && nbr && out && scratch && gate_of_channel && (scale == nullptr) == (shift == nullptr) && (n_in == 0 || features || prestaged),
+              "conv_fwd_gated: null pointer");
+  const GateEpilogue gate = {scale, shift, gate_of_channel, c_keep, scalar_act, gate_act,
+                             out_precision == SSC_PREC_F16 ? 1 : out_precision == SSC_PREC_BF16 ? 2 : 0};
+  if (precision == SSC_PREC_TF32)
+    return conv_fwd_tf32(features, n_in, c_in, filters, K, c_out, nbr, n_out, (float *)out, status, scratch, scratch_bytes, n_out_dev, nullptr, prestaged, 0, gate, as_stream(stream));
+  return conv_fwd_16(features, n_in, c_in, precision == SSC_PREC_BF16, filters, K, c_out, nbr, n_out, (float *)out, status, scratch, scratch_bytes, n_out_dev, nullptr, prestaged, 0, gate, as_stream(stream));
 }
 
 extern "C" int ssc_conv_fwd(const float *features, int n_in, int c_in, const void *filters, int K, int c_out,

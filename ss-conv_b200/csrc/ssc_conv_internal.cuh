@@ -26,13 +26,24 @@ inline int tf32_offsets_per_row(int c_in) {
 // geometry of the packed filter image [K][k_slabs][n_pad][128 bytes] (ssc_conv_tc.cu)
 bool tc_operand_layout(int c_in_words, int c_out, int *k_slabs, int *n_pad, int *tile_n, int *n_tiles);
 
+// A per-channel affine map (an eval-mode batch norm folded up; scale NULL: none) and the gated activation, applied to
+// the rows of a convolution before they are stored: channels [0, c_keep) are kept, the rest are the gate
+// scalars (ssc_bn_gate_fwd with c_gate_base = c_keep and no biases).
+struct GateEpilogue {
+  const float *scale, *shift;
+  const int32_t *gate_of_channel;   // NULL: the convolution's own rows are stored
+  int c_keep, scalar_act, gate_act;
+  int out16;                        // 0: fp32 rows, 1: fp16, 2: bf16
+};
+bool conv_gate_covered(int c_in, int c_out, int c_keep, int precision, int n_out);
+
 // output-stationary tensor-core kernels (ssc_conv_tc.cu); table_form: SSC_CONV_TABLE_IN_ORDER | SSC_CONV_TABLE_REVERSED
 int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed, int K, int c_out,
                   const int32_t *nbr, int n_out, float *out, int32_t *status, void *scratch, size_t scratch_bytes,
-                  const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, cudaStream_t st);
+                  const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, const GateEpilogue &gate, cudaStream_t st);
 int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void *packed, int K, int c_out,
                 const int32_t *nbr, int n_out, float *out, int32_t *status, void *scratch, size_t scratch_bytes,
-                const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, cudaStream_t st);
+                const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, const GateEpilogue &gate, cudaStream_t st);
 
 // compacted per-offset pair lists of a neighbour table (ssc_wgrad_tc.cu): the lists of the kernel
 // offsets follow one another in pair_out / pair_in (ascending output row inside an offset),

@@ -22,6 +22,7 @@
 // Every wait on an mbarrier is bounded: on expiry the thread records an error in `status`
 // through a shared flag, every other wait then gives up too, and the kernel frees its tensor
 // memory and returns.
+#include "ssc_act.cuh"
 #include "ssc_conv_internal.cuh"
 #include "ssc_tc_ptx.cuh"
 
@@ -604,11 +605,15 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 //   * table entries are loaded two offsets ahead.
 // Sums are accumulated in the order of the steps (ascending offset, ascending slab), whatever the tile's
 // other rows need.
-template <bool F16>
-__global__ void __launch_bounds__(TC_ROWS_THREADS)
+//
+// GATED: batch norm and gated activation on the way out.  As a pass of its own (ssc_bn_gate_fwd) they read and write
+// every row once more: 164 us of the 12 layers of a backbone, 320 us of 24 with bf16 rows.  A row's gate
+// scalars are evaluated first, a lane per row, into shared memory; the arithmetic is that pass's, so are the bits.
+template <bool F16, bool GATED>
+__global__ void __launch_bounds__(TC_ROWS_THREADS, 3)
 conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
                      const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out, int32_t *status, TcParams p,
-                     const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order) {
+                     const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order, GateEpilogue gate) {
   const int n_rows = live_rows(n_out, n_out_dev);
   if ((int)blockIdx.x * TC_M >= n_rows) return;
   extern __shared__ uint8_t smem_raw[];
@@ -803,56 +808,159 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   }
 
   // ================================ epilogue: TMEM -> shared memory -> global ====================
-  if (warp < 4) {
+  // The producer warps again: 32 rows each, with two groups every other 32 columns.
+  if (warp < mma_warp) {
+    const int group = warp >> 2;
     __syncwarp();
+    float4 consts[2];                             // (GATED) scale, shift, gate of the channels this thread hands round
+    auto channel = [&](int ch) {
+      const bool affine = gate.scale != nullptr;
+      return make_float4(affine ? __ldg(gate.scale + ch) : 0.f, affine ? __ldg(gate.shift + ch) : 0.f,
+                         __int_as_float(ch < gate.c_keep ? __ldg(gate.gate_of_channel + ch) : -2), 0.f);
+    };
+    if (GATED) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (tid + 128 * i < c_out) consts[i] = channel(tid + 128 * i);
+    }
     bool ok = __all_sync(0xffffffffu, !*abort_flag);
     if (ok && n_iter > 0) ok = mbar_wait_warp(smem_u32(&done_bar), 0u, abort_flag);
-    ok = __all_sync(0xffffffffu, ok);             // tcgen05.ld below is warp-collective
+    ok = __all_sync(0xffffffffu, ok) && n_iter > 0;   // tcgen05.ld below is warp-collective
     tc_fence_after();
-    const int m = m_tile < n_rows ? (order ? __ldg(order + m_tile) : m_tile) : -1;
+    const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    auto load16 = [&](uint32_t *q, int c0) {
+      if (ok && c0 < p.n_cta) {
+        tmem_ld16(q, acc + (uint32_t)c0);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) q[i] = 0u;
+      }
+    };
     const int col0 = nt0 * p.tile_n;              // first output channel of this CTA
-    // 32 columns of the warp's 32 rows at a time go through the warp's share of slot 0 (free now), so that eight
+    // 32 columns of the warp's 32 rows at a time go through the warp's 4 KB of the slots (free now), so that eight
     // lanes write the 128 contiguous bytes of a row
     float *blk = (float *)(smem + (size_t)warp * 4096u);
-    const bool vec = (c_out & 3) == 0 && ((uintptr_t)out & 15u) == 0;
-    for (int c0 = 0; c0 < p.n_cta && col0 + c0 < c_out; c0 += 32) {
-      uint32_t r[32];
+    const int c_row = GATED ? gate.c_keep : c_out;          // channels of a stored row
+    const bool vec = (c_row & 3) == 0 && ((uintptr_t)out & 15u) == 0;
+    if (GATED) {                                  // one CTA has all channels
+      float4 *chan = (float4 *)(smem + (size_t)groups * 4u * 4096u);   // [c_out]
+      // act(gate g) of row r of the quarter at g * 33 + r, and a last line of ones
+      const int n_gates = c_out - c_row;
+      float *gates = (float *)(chan + c_out) + quarter * 33 * (n_gates + 1);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (ok && n_iter > 0 && c0 + 16 * h < p.n_cta) {
-          const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c0 + 16 * h);
-          uint32_t *q = r + 16 * h;
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]), "=r"(q[8]),
-                "=r"(q[9]), "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
-              : "r"(taddr)
-              : "memory");
-        } else {
+      for (int i = 0; i < 2; ++i)
+        if (tid + 128 * i < c_out && group == 0) chan[tid + 128 * i] = consts[i];
+      for (int ch = tid + 256; ch < c_out && group == 0; ch += 128) chan[ch] = channel(ch);
+      asm volatile("bar.sync 1, %0;" ::"r"(groups * 128) : "memory");
+      if (group == 0) gates[n_gates * 33 + lane] = 1.f;
+      for (int c0 = (c_row & ~15) + 16 * group; c0 < c_out; c0 += 16 * groups) {
+        uint32_t q[16];
+        load16(q, c0);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float v[16];
 #pragma unroll
-          for (int q = 0; q < 16; ++q) r[16 * h + q] = 0u;
+        for (int i = 0; i < 16; ++i) {
+          const float4 k = chan[c0 + i < c_out ? c0 + i : 0];
+          v[i] = __uint_as_float(q[i]);
+          if (gate.scale) v[i] = fmaf(v[i], k.x, k.y);
         }
+        if (gate.gate_act == 2) {                 // (all sixteen side by side: one after the other they are all latency)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = apply_act(v[i], 2);
+        } else if (gate.gate_act == 1) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = apply_act(v[i], 1);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (c0 + i >= c_row && c0 + i < c_out) gates[(c0 + i - c_row) * 33 + lane] = v[i];
       }
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (vec) {
+      if (groups > 1) asm volatile("bar.sync 1, %0;" ::"r"(groups * 128) : "memory");
+      for (int c0 = 32 * group; c0 < c_row; c0 += 32 * groups) {
+        uint32_t r[32];
+        load16(r, c0);
+        load16(r + 16, c0 + 16);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         __syncwarp();
         // piece q of row `lane` at place q ^ (lane & 7): both directions touch every bank once per phase
 #pragma unroll
         for (int q = 0; q < 8; ++q) *(uint4 *)(blk + lane * 32 + ((q ^ (lane & 7)) << 2)) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
         __syncwarp();
-        const int q = lane & 7, col = col0 + c0 + 4 * q;
+        const int q = lane & 7, col = c0 + 4 * q;
+        if (col >= c_row) continue;
+        float sc[4], sh[4];
+        const float *gp[4];
+        bool scalar[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int row = 4 * i + (lane >> 3);
-          const int to = __shfl_sync(0xffffffffu, m, row);
-          if (to >= 0 && col < c_out && c0 + 4 * q < p.n_cta)
-            *(uint4 *)(out + (size_t)to * c_out + col) = *(const uint4 *)(blk + row * 32 + ((q ^ (row & 7)) << 2));
+        for (int j = 0; j < 4; ++j) {
+          const float4 k = chan[col + j < c_out ? col + j : 0];
+          const int g = __float_as_int(k.z);
+          sc[j] = k.x;
+          sh[j] = k.y;
+          scalar[j] = g == -1;
+          gp[j] = gates + (g >= 0 ? g : n_gates) * 33;
         }
-      } else if (m >= 0) {
-        float *op = out + (size_t)m * c_out + col0 + c0;
+#pragma unroll 4
+        for (int i = 0; i < 8; ++i) {
+          const int row = 4 * i + (lane >> 3), to = m0 + quarter * 32 + row;
+          const float4 x = *(const float4 *)(blk + row * 32 + ((q ^ (row & 7)) << 2));
+          float v[4] = {x.x, x.y, x.z, x.w};
+          if (gate.scale) {
 #pragma unroll
-        for (int q = 0; q < 32; ++q)
-          if (col0 + c0 + q < c_out && c0 + q < p.n_cta) op[q] = __uint_as_float(r[q]);
+            for (int j = 0; j < 4; ++j) v[j] = fmaf(v[j], sc[j], sh[j]);
+          }
+          if (gate.scalar_act == 1) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = scalar[j] && !(v[j] > 0.f) ? 0.f : v[j];
+          } else if (gate.scalar_act != 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (scalar[j]) v[j] = apply_act(v[j], gate.scalar_act);
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] *= gp[j][row];
+          if (to >= n_rows) continue;
+          const size_t at = (size_t)to * c_row + col;
+          if (gate.out16 == 0) {
+            if (vec) {
+              *(float4 *)(out + at) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                if (col + j < c_row) out[at + j] = v[j];
+            }
+          } else {                                // c_row is a multiple of eight
+            *(uint2 *)((uint16_t *)out + at) = gate.out16 == 2 ? make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]))
+                                                              : make_uint2(pack_f16x2(v[0], v[1]), pack_f16x2(v[2], v[3]));
+          }
+        }
+      }
+    } else {
+      const int m = m_tile < n_rows ? (order ? __ldg(order + m_tile) : m_tile) : -1;
+      for (int c0 = 32 * group; c0 < p.n_cta && col0 + c0 < c_row; c0 += 32 * groups) {
+        uint32_t r[32];
+        load16(r, c0);
+        load16(r + 16, c0 + 16);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (vec) {
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < 8; ++q) *(uint4 *)(blk + lane * 32 + ((q ^ (lane & 7)) << 2)) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+          __syncwarp();
+          const int q = lane & 7, col = col0 + c0 + 4 * q;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int row = 4 * i + (lane >> 3);
+            const int to = __shfl_sync(0xffffffffu, m, row);
+            if (to >= 0 && col < c_row && c0 + 4 * q < p.n_cta)
+              *(uint4 *)(out + (size_t)to * c_row + col) = *(const uint4 *)(blk + row * 32 + ((q ^ (row & 7)) << 2));
+          }
+        } else if (m >= 0) {
+          float *op = out + (size_t)m * c_row + col0 + c0;
+#pragma unroll
+          for (int q = 0; q < 32; ++q)
+            if (col0 + c0 + q < c_row && c0 + q < p.n_cta) op[q] = __uint_as_float(r[q]);
+        }
       }
     }
   }
@@ -912,19 +1020,41 @@ __global__ void pack_filters_16_kernel(const float *__restrict__ filters, int K,
   packed[block + off] = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
+// The plan of a launch over n_out rows: few row tiles spread the N tiles over CTAs too, and CTAs that are alone on
+// their SM take all of its shared memory.
+static bool rows_params(int words, int c_out, int n_out, TcParams &p, int opk = 1) {
+  const int grid = ceil_div(n_out, TC_M), sms = sm_count();
+  if (!tc_params(words, c_out, p, grid < 2 * sms, false, opk)) return false;
+  return grid * (p.n_tiles / p.nt_cta) > sms || tc_params(words, c_out, p, grid < 2 * sms, true, opk);
+}
+
+// What the gated epilogue needs: 4 KB per producer warp, the channel constants and the gates of 128 rows, in the
+// operand slots that are free by then.
+static bool gate_fits(const TcParams &p, int c_out, int c_keep) {
+  const size_t warps = (size_t)(rows_threads(p) - 32) / 32;
+  return p.nt_cta == p.n_tiles &&
+         warps * 4096 + (size_t)c_out * 16 + (size_t)4 * 33 * 4 * (c_out - c_keep + 1) <= (size_t)p.stages * (TC_A_BYTES + p.b_bytes);
+}
+
+bool conv_gate_covered(int c_in, int c_out, int c_keep, int precision, int n_out) {
+  if (c_in < 1 || c_keep < 1 || c_keep > c_out) return false;
+  const bool tf32 = precision == SSC_PREC_TF32;
+  if (!tf32 && precision != SSC_PREC_F16 && precision != SSC_PREC_BF16) return false;
+  if (tf32 && tf32_offsets_per_row(c_in) > 1) return false;
+  TcParams p;
+  return rows_params(tf32 ? c_in : f16_row_words(c_in), c_out, n_out, p) && gate_fits(p, c_out, c_keep);
+}
+
 int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void *packed, int K, int c_out,
                 const int32_t *nbr, int n_out, float *out, int32_t *status, void *scratch, size_t scratch_bytes,
-                const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, cudaStream_t st) {
+                const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, const GateEpilogue &gate, cudaStream_t st) {
   if (K > 256) return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): kernel volume %d > 256", K);
   const int words = f16_row_words(c_in);
   if (scratch == nullptr || scratch_bytes + 16 < conv_f16_scratch_bytes(n_in, c_in) || ((uintptr_t)scratch & 15u) != 0)
     return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): needs the staging buffer of ssc_conv_scratch_bytes (16-byte aligned)");
   int grid = ceil_div(n_out, TC_M);
-  const int sms = sm_count();
   TcParams p;
-  if (!tc_params(words, c_out, p, grid < 2 * sms))
-    return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): c_out %d / kernel volume %d not supported", c_out, K);
-  if (grid * (p.n_tiles / p.nt_cta) <= sms) tc_params(words, c_out, p, grid < 2 * sms, true);
+  if (!rows_params(words, c_out, n_out, p)) return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): c_out %d / kernel volume %d not supported", c_out, K);
   p.fmt16 = bf16 ? 1 : 0;
   p.nbr_by_pos = ((table_form & SSC_CONV_TABLE_IN_ORDER) && order) ? 1 : 0;
   p.rev = (table_form & SSC_CONV_TABLE_REVERSED) ? 1 : 0;
@@ -933,25 +1063,25 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
     if (rc != SSC_OK) return rc;
   }
   const size_t smem = tc_smem_bytes(p);
-  auto kernel = conv_fwd_rows_kernel<true>;
+  const bool gated = gate.gate_of_channel != nullptr;
+  if (gated && !gate_fits(p, c_out, gate.c_keep)) return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): the gated epilogue does not cover %d -> %d channels", c_out, gate.c_keep);
+  auto kernel = gated ? conv_fwd_rows_kernel<true, true> : conv_fwd_rows_kernel<true, false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(16-bit): smem attribute: %s", cudaGetErrorString(e));
   const dim3 grid2(grid, p.n_tiles / p.nt_cta);
-  { kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order); note_launches(1); }
+  { kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_fwd_16");
   return SSC_OK;
 }
 
 int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed, int K, int c_out,
                   const int32_t *nbr, int n_out, float *out, int32_t *status, void *scratch, size_t scratch_bytes,
-                  const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, cudaStream_t st) {
+                  const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, const GateEpilogue &gate, cudaStream_t st) {
   TcParams p;
   if (K > 256) return fail(SSC_ERR_INVALID, "conv_fwd(tf32): kernel volume %d > 256", K);
   int grid = ceil_div(n_out, TC_M);
-  const bool split_n = grid < 2 * sm_count();   // few row tiles: spread the N tiles over CTAs too
   const int opk = tf32_offsets_per_row(c_in);
-  if (!tc_params(c_in, c_out, p, split_n, false, opk)) return fail(SSC_ERR_INVALID, "conv_fwd(tf32): c_out %d / kernel volume %d not supported", c_out, K);
-  if (grid * (p.n_tiles / p.nt_cta) <= sm_count()) tc_params(c_in, c_out, p, split_n, true, opk);
+  if (!rows_params(c_in, c_out, n_out, p, opk)) return fail(SSC_ERR_INVALID, "conv_fwd(tf32): c_out %d / kernel volume %d not supported", c_out, K);
   p.nbr_by_pos = ((table_form & SSC_CONV_TABLE_IN_ORDER) && order) ? 1 : 0;
   p.rev = (table_form & SSC_CONV_TABLE_REVERSED) ? 1 : 0;
   size_t smem = tc_smem_bytes(p);
@@ -971,13 +1101,22 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
     int rc = stage_features(features, n_in, c_in, scratch, st);
     if (rc != SSC_OK) return rc;
   }
-  const bool rows = staged && opk == 1;
-  auto kernel = opk > 1 ? conv_fwd_tf32_kernel<true, false, true> : rows ? conv_fwd_rows_kernel<false> : conv_fwd_tf32_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
   const dim3 grid2(grid, p.n_tiles / p.nt_cta);
-  { kernel<<<grid2, rows ? rows_threads(p) : p.threads, smem, st>>>(staged ? (const float *)scratch : features, staged ? c_pad : c_in, (const uint4 *)packed, K, c_out,
-                                        nbr, n_out, out, status, p, n_out_dev, order); note_launches(1); }
+  const bool rows = staged && opk == 1, gated = gate.gate_of_channel != nullptr;
+  if (gated && !(rows && gate_fits(p, c_out, gate.c_keep)))
+    return fail(SSC_ERR_INVALID, "conv_fwd(tf32): the gated epilogue does not cover %d -> %d channels without a staging buffer", c_out, gate.c_keep);
+  if (rows) {
+    auto kernel = gated ? conv_fwd_rows_kernel<false, true> : conv_fwd_rows_kernel<false, false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
+    kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, c_pad, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
+  } else {
+    auto kernel = opk > 1 ? conv_fwd_tf32_kernel<true, false, true> : conv_fwd_tf32_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
+    kernel<<<grid2, p.threads, smem, st>>>(staged ? (const float *)scratch : features, staged ? c_pad : c_in, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order);
+  }
+  note_launches(1);
   SSC_CHECK_LAUNCH("conv_fwd_tf32");
   return SSC_OK;
 }

@@ -66,6 +66,10 @@ SIGNATURES = {
     "ssc_nbr_row_order_planes_scratch_bytes": (c_size_t, [_I3, c_int]),
     "ssc_nbr_row_order_planes": (c_int, [c_void_p, _I3, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "ssc_conv_stage": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
+    "ssc_conv_gate_covered": (c_int, [c_int, c_int, c_int, c_int, c_int]),
+    "ssc_conv_fwd_gated": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p,
+                                   c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p,
+                                   c_void_p]),
     "ssc_conv_fwd_ordered": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p,
                                      c_void_p, c_void_p, c_size_t, c_void_p, c_void_p, c_void_p]),
     "ssc_conv_wgrad_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
@@ -725,14 +729,17 @@ def conv_prepare(features, filters, precision=None):
 
 
 def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, row_order=None, algo=None,
-                 table_in_order=False, image=None, reversed_table=False):
+                 table_in_order=False, image=None, reversed_table=False, gate=None):
     """out [n_out, Cout] = sum over offsets of gathered rows times filters (one launch).
     n_out_dev: device word with the exact row count when n_out is only a capacity.
     row_order: permutation of the output rows from nbr_row_order (same result, fewer steps).
     table_in_order: nbr is the table with its columns already in that order (nbr_row_order_planes).
     algo: None (the module setting), 'rows' or 'pairs' (see set_algo).
     image: the features' TF32 image (stage_tf32) where the caller has one already.
-    reversed_table: the neighbours at kernel offset kappa stand in row K - 1 - kappa of nbr."""
+    reversed_table: the neighbours at kernel offset kappa stand in row K - 1 - kappa of nbr.
+    gate: (scale, shift, gate_of_channel, c_keep, scalar_act, gate_act) of a folded batch norm and a gated
+    activation: the rows come out normalised and gated, in the feature storage type, from the
+    convolution's own kernel where that covers the sizes (same bits as bn_gate_forward on its result)."""
     if filters.dim() != 3:
         filters = filters.reshape(-1, filters.shape[-2], filters.shape[-1])
     K, c_in, c_out = filters.shape
@@ -741,16 +748,16 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
     features = features.contiguous()
     if features.dtype in _PREC_OF_DTYPE:
         if c_in % 8 == 0 and c_out <= 512 and row_order is None and not reversed_table:
-            return _conv_forward_stored16(features, filters, nbr, n_out, n_out_dev, algo)
+            return _conv_forward_stored16(features, filters, nbr, n_out, n_out_dev, algo, gate)
         features = features.float()
-    out = torch.empty((n_out, c_out), dtype=torch.float32, device=features.device)
     mode = _resolve_precision(c_in, c_out, precision)
     st = status_word(features.device)
     if mode in ("fp16", "bf16") and c_out > 512:
         mode = "fp32"
     if (mode in _PREC_OF and n_out_dev is None and row_order is None and nbr.shape[1] == n_out and not reversed_table
             and _use_pairs(K, c_in, c_out, n_out, _PREC_OF[mode], algo)):
-        return _conv_forward_pairs(features, filters, nbr, n_out, _PREC_OF[mode], out, st)
+        out = torch.empty((n_out, c_out), dtype=torch.float32, device=features.device)
+        return _gated(_conv_forward_pairs(features, filters, nbr, n_out, _PREC_OF[mode], out, st), gate)
     flag = TABLE_IN_ORDER if (table_in_order and row_order is not None) else 0
     if flag and mode not in _PREC_OF:
         raise ValueError("ssconv_b200: a table in row order needs a tensor-core precision")
@@ -762,7 +769,15 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
         _prepared.clear()
     if image is not None and mode == "tf32":
         ready = (PREC_TF32, _packed_filters(filters, PREC_TF32), image, image.numel())
-    if ready is not None and ready[0] == _PREC_OF.get(mode, -1):
+    prec = _PREC_OF.get(mode, PREC_FP32)
+    if gate is not None and row_order is None and not flag and _gate_covered(c_in, c_out, gate[3], prec, n_out):
+        if ready is None or ready[0] != prec:
+            nbytes = lib().ssc_conv_scratch_bytes(features.shape[0], c_in, c_out, prec)
+            ready = (0, _packed_filters(filters, prec), torch.empty(nbytes, dtype=torch.uint8, device=features.device), nbytes)
+        return _conv_gated(_p(features, torch.float32), features.shape[0], c_in, ready[1], K, c_out, nbr, n_out,
+                           prec | (PRESTAGED if ready[0] else 0), gate, st, _p(ready[2]), ready[3], n_out_dev)
+    out = torch.empty((n_out, c_out), dtype=torch.float32, device=features.device)
+    if ready is not None and ready[0] == prec:
         prec, packed, scratch, nbytes = ready
         _check(lib().ssc_conv_fwd_ordered(_p(features, torch.float32), features.shape[0], c_in, _p(packed), K, c_out,
                                           _p(nbr, torch.int32), int(n_out), prec | PRESTAGED | flag, _p(out), _p(st), _p(scratch),
@@ -782,7 +797,38 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
         _check(lib().ssc_conv_fwd(_p(features, torch.float32), features.shape[0], c_in, _p(filters, torch.float32), K,
                                   c_out, _p(nbr, torch.int32), int(n_out), PREC_FP32 | flag, _p(out), _p(st), None, 0,
                                   _p(n_out_dev), _stream()))
+    return _gated(out, gate)
+
+
+def _gated(out, gate):
+    if gate is None:
+        return out
+    scale, shift, table, c_keep, scalar_act, gate_act = gate
+    return bn_gate_forward(out, scale, shift, table, c_keep, c_keep, scalar_act, gate_act, None, None, storage=_storage)
+
+
+def _gate_covered(c_in, c_out, c_keep, prec, n_out):
+    return prec != PREC_FP32 and bool(lib().ssc_conv_gate_covered(c_in, c_out, c_keep, prec, int(n_out)))
+
+
+def _conv_gated(features, n_in, c_in, packed, K, c_out, nbr, n_out, prec, gate, st, scratch, nbytes, n_out_dev):
+    scale, shift, table, c_keep, scalar_act, gate_act = gate
+    stored = _stored_type(n_out, c_out, c_keep, c_keep)
+    out = torch.empty((n_out, c_keep), dtype=stored or torch.float32, device=nbr.device)
+    _check(lib().ssc_conv_fwd_gated(features, n_in, c_in, _p(packed), K, c_out, _p(nbr, torch.int32), int(n_out), prec,
+                                    _p(scale), _p(shift), _p(table), c_keep, scalar_act, gate_act,
+                                    _PREC_OF[_storage] if stored else PREC_FP32, _p(out), _p(st), scratch, nbytes,
+                                    _p(n_out_dev), _stream()))
     return out
+
+
+def _stored_type(n, c, c_keep, c_gate_base, storage=True):
+    """The 16-bit type gated rows are stored in, None where they stay fp32: no storage type is set (`storage`
+    overrides the setting) or the shapes do not allow 16-byte rows."""
+    storage = _storage if storage is True else storage
+    if storage in _DTYPE_OF and c_keep % 8 == 0 and c % 4 == 0 and c_gate_base % 4 == 0 and n * c_keep // 4 < 2 ** 31:
+        return _DTYPE_OF[storage]
+    return None
 
 
 def _packed_filters(filters, prec):
@@ -799,24 +845,28 @@ def _packed_filters(filters, prec):
     return packed
 
 
-def _conv_forward_stored16(features, filters, nbr, n_out, n_out_dev, algo):
+def _conv_forward_stored16(features, filters, nbr, n_out, n_out_dev, algo, gate=None):
     """Convolution on features stored as fp16 / bf16 rows [n_in, Cin] (Cin a multiple of 8): the rows
     ARE the staged operand image, so the call is the kernel alone."""
     K, c_in, c_out = filters.shape
     prec = _PREC_OF[_PREC_OF_DTYPE[features.dtype]]
-    out = torch.empty((n_out, c_out), dtype=torch.float32, device=features.device)
     st = status_word(features.device)
     packed = _packed_filters(filters, prec)
     nbytes = features.numel() * 2
-    if n_out_dev is None and nbr.shape[1] == n_out and _use_pairs(K, c_in, c_out, n_out, prec, algo):
+    pairs = n_out_dev is None and nbr.shape[1] == n_out and _use_pairs(K, c_in, c_out, n_out, prec, algo)
+    if gate is not None and not pairs and _gate_covered(c_in, c_out, gate[3], prec, n_out):
+        return _conv_gated(None, features.shape[0], c_in, packed, K, c_out, nbr, n_out, prec | PRESTAGED, gate, st,
+                           _p(features), nbytes, n_out_dev)
+    out = torch.empty((n_out, c_out), dtype=torch.float32, device=features.device)
+    if pairs:
         lists = pair_lists(nbr)
         _check(lib().ssc_conv_fwd_pairs(None, features.shape[0], c_in, _p(packed), K, c_out, _p(lists), lists.numel(),
                                         int(n_out), prec | PRESTAGED, _p(out), _p(st), _p(features), nbytes, _stream()))
-        return out
+        return _gated(out, gate)
     _check(lib().ssc_conv_fwd_ordered(None, features.shape[0], c_in, _p(packed), K, c_out, _p(nbr, torch.int32),
                                       int(n_out), prec | PRESTAGED, _p(out), _p(st), _p(features), nbytes, _p(n_out_dev),
                                       None, _stream()))
-    return out
+    return _gated(out, gate)
 
 
 def _conv_forward_pairs(features, filters, nbr, n_out, prec, out, st):
@@ -840,7 +890,7 @@ def _conv_forward_pairs(features, filters, nbr, n_out, prec, out, st):
     return out
 
 
-def indice_conv_fp32(features, filters, indice_pairs, indice_num, num_act_out, inverse, subm):
+def indice_conv_fp32(features, filters, indice_pairs, indice_num, num_act_out, inverse, subm, gate=None):
     """Reference signature (SS_Conv_lib/src/ss_conv_ops.h:43-45); filters [k,k,k,Cin,Cout]
     (a permuted view is accepted).  The submanifold centre needs no special case."""
     if features.dtype != torch.float32 and features.dtype not in _PREC_OF_DTYPE:
@@ -861,7 +911,7 @@ def indice_conv_fp32(features, filters, indice_pairs, indice_num, num_act_out, i
         # an inverse convolution gathers through its partner's table with the roles exchanged: like the
         # input gradient, every output row uses only the offsets of its parity class
         order = nbr_row_order(nbr)
-    return conv_forward(features, flt, nbr, int(num_act_out), n_out_dev=n_out_dev, row_order=order)
+    return conv_forward(features, flt, nbr, int(num_act_out), n_out_dev=n_out_dev, row_order=order, gate=gate)
 
 
 def _not_built(name):
@@ -1276,9 +1326,9 @@ def bn_gate_forward(x, scale, shift, gate_of_channel, c_out, c_gate_base, scalar
     """storage 'fp16' / 'bf16': the result is written in that type (see set_feature_storage) when the
     shapes allow 16-byte rows; otherwise fp32."""
     x = x.contiguous()
-    if (storage in _DTYPE_OF and int(c_out) % 8 == 0 and x.shape[1] % 4 == 0 and int(c_gate_base) % 4 == 0
-            and x.shape[0] * int(c_out) // 4 < 2 ** 31):
-        out = torch.empty((x.shape[0], int(c_out)), dtype=_DTYPE_OF[storage], device=x.device)
+    stored = _stored_type(x.shape[0], x.shape[1], int(c_out), int(c_gate_base), storage)
+    if stored:
+        out = torch.empty((x.shape[0], int(c_out)), dtype=stored, device=x.device)
         _check(lib().ssc_bn_gate_fwd16(_p(x, torch.float32), x.shape[0], x.shape[1], _p(scale), _p(shift),
                                        _p(gate_of_channel), int(c_out), int(c_gate_base), int(scalar_act), int(gate_act),
                                        _p(scalar_bias), _p(gate_bias), _PREC_OF[storage], _p(out), _stream()))

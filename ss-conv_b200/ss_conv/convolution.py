@@ -44,13 +44,13 @@ class Convolution(SparseConvolution):
             self.weight = None
         return super().train(mode)
 
-    def forward(self, input):
+    def forward(self, input, gate=None):
         assert isinstance(input, SparseTensor)
         device = input.raw()[0].device
         if self.kernel.weight.device != device:
             self.kernel.to(device)
         if self.training:
-            return self._sparse_conv(input, self.kernel.filters())
+            return self._sparse_conv(input, self.kernel.filters(), gate)
         if self.weight is None or self.weight.device != device:
             self.weight = self.kernel.filters()
-        return self._sparse_conv(input, self.weight)
+        return self._sparse_conv(input, self.weight, gate)

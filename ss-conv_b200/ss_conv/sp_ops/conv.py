@@ -63,7 +63,7 @@ class SparseConvolution(nn.Module):
                                           self.output_padding)
         return get_conv_output_size(spatial_shape, self.kernel_size, self.stride, self.padding, self.dilation)
 
-    def _sparse_conv(self, input, weight):
+    def _sparse_conv(self, input, weight, gate=None):
         """weight: [kx, ky, kz, Cin, Cout].  Rulebooks are cached in input.indice_dict under
         indice_key; an inverse convolution reuses its partner's rulebook with the pair roles
         exchanged.
@@ -71,7 +71,10 @@ class SparseConvolution(nn.Module):
         A regular (strided / transposed) convolution without an indice_key can run ahead of its
         output count: rulebook and convolution are queued with a guessed row capacity (also on
         an input whose own count is still pending) and the result is a SparseTensor with pending
-        rows; see sp_ops/tensor.py."""
+        rows; see sp_ops/tensor.py.
+
+        gate: a folded batch norm and gated activation to apply to the rows (_ext.conv_forward), while no
+        gradients are recorded."""
         assert isinstance(input, SparseTensor)
         out_spatial_shape = self._output_shape(input.spatial_shape)
         feats_raw, inds_raw, n_in_dev = input.raw()
@@ -96,7 +99,7 @@ class SparseConvolution(nn.Module):
                     _ext._prepared.clear()
             if ahead is not None:
                 outids_cap, pairs, pair_num = ahead
-                out_cap = indice_conv(feats_raw, weight, pairs, pair_num, pairs.capacity)
+                out_cap = self._op(feats_raw, weight, pairs, pair_num, pairs.capacity, gate)
                 if self.bias is not None:
                     out_cap += self.bias
                 out = SparseTensor(out_cap, outids_cap, out_spatial_shape, input.batch_size)
@@ -106,7 +109,7 @@ class SparseConvolution(nn.Module):
                                          self.dilation, self.transposed)
 
                 def redo():
-                    t = self._sparse_conv_exact(input, weight)
+                    t = self._sparse_conv_exact(input, weight, gate)
                     return t.features, t.indices
 
                 out._rows = PendingRows(pairs._n_out_dev, pairs.capacity, input if input.pending() else None, redo,
@@ -132,8 +135,7 @@ class SparseConvolution(nn.Module):
                 if self.indice_key is not None:
                     input.indice_dict[self.indice_key] = (inds_raw, inds_raw, pairs, None, input.spatial_shape)
             if pairs is not None:
-                op = indice_subm_conv if self.subm else indice_conv
-                out_cap = op(feats_raw, weight, pairs, None, pairs.capacity)
+                out_cap = self._op(feats_raw, weight, pairs, None, pairs.capacity, gate)
                 if self.bias is not None:
                     out_cap += self.bias
                 out = SparseTensor(out_cap, inds_raw, out_spatial_shape if self.subm else input.spatial_shape,
@@ -149,14 +151,20 @@ class SparseConvolution(nn.Module):
                     kept = input.find_indice_pair(key)
                     if kept is not None and kept[2] is pairs:
                         input.indice_dict.pop(key)
-                    t = self._sparse_conv_exact(input, weight)
+                    t = self._sparse_conv_exact(input, weight, gate)
                     return t.features, t.indices
 
                 out._rows = PendingRows(n_in_dev, pairs.capacity, input, redo)
                 pairs.count = out._rows.count
                 out._rows.indices_ready = getattr(input._rows, "indices_ready", None)
                 return out
-        return self._sparse_conv_exact(input, weight)
+        return self._sparse_conv_exact(input, weight, gate)
+
+    def _op(self, features, weight, pairs, num, n_out, gate):
+        if gate is not None:
+            return _ext.indice_conv_fp32(features, weight, pairs, num, n_out, int(self.inverse), int(self.subm), gate)
+        op = indice_subm_conv if self.subm else (indice_inverse_conv if self.inverse else indice_conv)
+        return op(features, weight, pairs, num, n_out)
 
     def _cached_rulebook(self, input):
         """The rulebook kept under this layer's key with exact row counts (an entry made on a pending
@@ -174,7 +182,7 @@ class SparseConvolution(nn.Module):
             cached = input.indice_dict[self.indice_key] = (outids, indices, pairs, num, shape)
         return cached
 
-    def _sparse_conv_exact(self, input, weight):
+    def _sparse_conv_exact(self, input, weight, gate=None):
         features, indices = input.features, input.indices
         spatial_shape, batch_size = input.spatial_shape, input.batch_size
         out_spatial_shape = self._output_shape(spatial_shape)
@@ -187,7 +195,7 @@ class SparseConvolution(nn.Module):
             rows = torch.arange(n, dtype=torch.int32, device=features.device)
             pairs = torch.stack([rows, rows]).unsqueeze(0).contiguous()
             num = torch.full((1,), n, dtype=torch.int32, device=features.device)
-            input.features = indice_subm_conv(features, weight, pairs, num, n)
+            input.features = self._op(features, weight, pairs, num, n, gate)
             if self.bias is not None:
                 input.features += self.bias
             return input
@@ -206,8 +214,7 @@ class SparseConvolution(nn.Module):
                 self.output_padding, self.subm, self.transposed, grid=input.grid, lazy=True)
             input.indice_dict[self.indice_key] = (outids, indices, indice_pairs, indice_pair_num, spatial_shape)
 
-        op = indice_subm_conv if self.subm else (indice_inverse_conv if self.inverse else indice_conv)
-        out_features = op(features, weight, indice_pairs, indice_pair_num, outids.shape[0])
+        out_features = self._op(features, weight, indice_pairs, indice_pair_num, outids.shape[0], gate)
         if self.bias is not None:
             out_features += self.bias
         out = SparseTensor(out_features, outids, out_spatial_shape, batch_size)

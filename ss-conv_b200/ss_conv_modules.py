@@ -50,7 +50,26 @@ class SS_Conv(nn.Module):
             self.activation = None
         self.dropout = Dropout(Rs_out, p=dropout_p) if dropout_p is not None and dropout_p > 0 else None
 
+    def _inference_gate(self, x):
+        """The folded batch norm and the activation for the convolution to apply as it stores its rows
+        (_ext.conv_forward), or None: while gradients are recorded or statistics are taken, with biases or
+        an activation the library does not know, with hooks on the modules that would not be called."""
+        bn, act, conv = self.bn, self.activation, self.conv
+        if (torch.is_grad_enabled() or act is None or conv.bias is not None or conv.training or (bn is not None and bn.training)
+                or conv._forward_hooks or act._forward_hooks or act._forward_pre_hooks
+                or (bn is not None and (bn._forward_hooks or bn._forward_pre_hooks)) or not act.fusable_gate()):
+            return None
+        device = x.raw()[0].device
+        if device.type != "cuda":
+            return None
+        table, _, _, scalar_act, gate_act = act.gate_tables(device)
+        return (*(bn.folded_affine(device) if bn is not None else (None, None)), table, act.c_out(), scalar_act, gate_act)
+
     def forward(self, x):
+        gate = self._inference_gate(x)
+        if gate is not None:
+            x = self.conv(x, gate)
+            return x if self.dropout is None else self.dropout(x)
         x = self.conv(x)
         both = self.bn.norm_and_gate(x, self.activation) if self.bn is not None and self.activation is not None else None
         if both is not None:

@@ -115,3 +115,31 @@ def test_three_nearest_with_ties(cuda, n_query, n_known):
     dist, idx = three_nn(q, k)
     want, order = torch.sort(((q[:, None] - k[None]) ** 2).sum(-1), dim=1, stable=True)
     assert torch.equal(dist, want[:, :3].sqrt()) and torch.equal(idx.long(), order[:, :3])
+
+
+@pytest.mark.parametrize("c_in,c_out,c_keep,n,precision,stored", [
+    (17, 11, 9, 1, "tf32", None), (32, 38, 32, 127, "tf32", None), (64, 76, 64, 129, "tf32", "bf16"),
+    (40, 256, 208, 300, "tf32", "fp16"), (24, 16, 16, 200, "tf32", None), (200, 152, 128, 257, "tf32", None),
+    (32, 38, 32, 700, "fp16", "fp16"), (64, 176, 128, 260, "bf16", "bf16"), (30, 19, 16, 33, "bf16", None)])
+@pytest.mark.parametrize("affine", [True, False])
+def test_gated_convolution_has_the_bits_of_the_two_passes(cuda, c_in, c_out, c_keep, n, precision, stored, affine):
+    """Rows around a tile of 128, channels that are no multiple of 4 or 16, one chunk of gates and several, none at
+    all, all result types: exactly the convolution followed by the gate pass."""
+    from ss_conv import _ext
+    rng = np.random.RandomState(n)
+    ind = random_voxels(rng, 1, 10, n)
+    outids, pairs, num = gpu_rulebook(ind, 1, [10] * 3, 3, 1, 1, 1, True, cuda)
+    nbr = _ext.neighbour_table(pairs, num, n)
+    feats, W = dev(rng.randn(n, c_in).astype(np.float32), cuda), dev(rng.randn(27, c_in, c_out).astype(np.float32) * .1, cuda)
+    table = dev(np.where(np.arange(c_keep) < 3, -1, np.arange(c_keep) % max(c_out - c_keep, 1) if c_out > c_keep else -2).astype(np.int32), cuda)
+    scale, shift = (torch.rand(c_out, device=cuda) + .5, torch.randn(c_out, device=cuda)) if affine else (None, None)
+    assert _ext._gate_covered(c_in, c_out, c_keep, _ext._PREC_OF[precision], n)
+    _ext.set_feature_storage(stored)
+    try:
+        got = _ext.conv_forward(feats, W, nbr, n, precision, gate=(scale, shift, table, c_keep, 1, 2))
+        x = _ext.conv_forward(feats, W, nbr, n, precision)
+        want = _ext.bn_gate_forward(x, scale, shift, table, c_keep, c_keep, 1, 2, None, None, storage=stored)
+    finally:
+        _ext.set_feature_storage(None)
+    _ext.check_status(cuda)
+    assert got.dtype == want.dtype and torch.equal(got, want) and float(x.abs().max()) > 0
