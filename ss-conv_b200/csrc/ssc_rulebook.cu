@@ -28,7 +28,7 @@ constexpr long long kDenseCellsPerRow = 512;
 
 struct RulebookScratch {
   unsigned long long *table;
-  int32_t *row_map;      // non-null: dense map in use instead of the hash table
+  int32_t *row_map;      // non-null: dense map (row + 1, 0 = absent) in use instead of the hash table; the bitmap follows it
   long long in_cells;
   uint32_t n_buckets;
   uint32_t *bitmap;
@@ -120,8 +120,7 @@ __global__ void hash_insert_kernel(const int4 *__restrict__ indices, int n, int 
   atomicOr(status, 2);  // table full (cannot happen at load factor <= 0.5)
 }
 
-// Dense alternative to hash_insert_kernel: row_map[flat input cell] = row (largest row wins on
-// duplicate coordinates, as in the hash table).
+// Dense alternative to hash_insert_kernel: row_map[flat input cell] = row + 1 (largest row wins on duplicates).
 __global__ void map_insert_kernel(const int4 *__restrict__ indices, int n, int batch, Geometry g,
                                   int32_t *__restrict__ row_map, int32_t *status, const int32_t *__restrict__ n_dev) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -132,7 +131,7 @@ __global__ void map_insert_kernel(const int4 *__restrict__ indices, int n, int b
     return;
   }
   const long long cell = ((long long)(c.x * g.in_shape[0] + c.y) * g.in_shape[1] + c.z) * g.in_shape[2] + c.w;
-  atomicMax(row_map + cell, j);
+  atomicMax(row_map + cell, j + 1);
 }
 
 // One thread per input row: mark every output cell the row reaches.  Bits that fall into the
@@ -186,7 +185,7 @@ constexpr int kCoarseVolume = 4096;      // cells per sample up to which a direc
 constexpr int kMarkImageWords = 1024;
 __global__ void __launch_bounds__(128)
 mark_outputs_kernel(const int4 *__restrict__ indices, int n, int batch, Geometry g, uint32_t *bitmap,
-                    const int32_t *__restrict__ n_dev) {
+                    const int32_t *__restrict__ n_dev, int32_t *__restrict__ row_map, int32_t *status) {
   __shared__ uint32_t image[kMarkImageWords];
   __shared__ unsigned cell_min, cell_max;
   __shared__ int any_row;
@@ -202,8 +201,12 @@ mark_outputs_kernel(const int4 *__restrict__ indices, int n, int batch, Geometry
   if (j < live) {
     c = indices[j];
     if ((unsigned)c.x < (unsigned)batch && in_range3(c.y, c.z, c.w, g.in_shape)) {
+      if (row_map)                                               // the insertion into the dense map, on the way
+        atomicMax(row_map + (((long long)(c.x * g.in_shape[0] + c.y) * g.in_shape[1] + c.z) * g.in_shape[2] + c.w), j + 1);
       rx = reach_of(g, 0, c.y); ry = reach_of(g, 1, c.z); rz = reach_of(g, 2, c.w);
       ok = rx.n > 0 && ry.n > 0 && rz.n > 0;
+    } else if (row_map) {
+      atomicOr(status, 1);
     }
   }
   const int base_b = c.x * g.out_shape[0];
@@ -392,7 +395,7 @@ lookup_dense_kernel(const int4 *__restrict__ out_indices, int n_out, int batch, 
       for (int kz = 0; kz < g.ksize[2]; ++kz, ++kappa) {
         const int z = coord(2, kz);
         int found = -1;
-        if (base >= 0 && (x | y | z) >= 0) found = __ldg(row_map + plane + z);
+        if (base >= 0 && (x | y | z) >= 0) found = __ldg(row_map + plane + z) - 1;
         if (o < n_out) nbr[(size_t)kappa * n_out + o] = found;
         if (counting) {
           const unsigned hits = __ballot_sync(0xffffffffu, found >= 0);
@@ -576,9 +579,8 @@ static int check_volume(int batch, const int shape[3], const char *what) {
 
 static int build_hash(const int32_t *indices, int n_in, int batch, const Geometry &g, RulebookScratch &s,
                       int32_t *status, cudaStream_t st, const int32_t *n_in_dev = nullptr) {
-  cudaMemsetAsync(s.misc, 0, 256, st);
   if (s.row_map != nullptr) {
-    cudaMemsetAsync(s.row_map, 0xFF, (size_t)s.in_cells * 4, st);
+    cudaMemsetAsync(s.row_map, 0, (size_t)s.in_cells * 4, st);
     if (n_in > 0) {
       { map_insert_kernel<<<ceil_div(n_in, 256), 256, 0, st>>>((const int4 *)indices, n_in, batch, g, s.row_map,
                                                             status ? status : s.misc + 1, n_in_dev); note_launches(1); }
@@ -783,13 +785,21 @@ extern "C" int ssc_rulebook_conv_count(const int32_t *indices, int n_in, int bat
   if (scratch == nullptr || scratch_bytes < s.total)
     return fail(SSC_ERR_SCRATCH, "rulebook_conv_count: scratch %zu < %zu bytes", scratch_bytes, s.total);
   cudaStream_t st = as_stream(stream);
-  if (int e = build_hash(indices, n_in, batch, g, s, status, st, n_in_dev)) return e;
-  cudaMemsetAsync(s.bitmap, 0, (size_t)s.n_words * 4, st);
+  bool simple = true;
+  for (int d = 0; d < 3; ++d) simple = simple && (g.transpose || g.stride[d] == 1 || g.dilation[d] == 1);
+  // with a dense map the marking kernel also fills the map, and one clearing covers map and bitmap: two launches
+  // instead of four before the scan
+  const bool together = simple && s.row_map != nullptr;
+  if (together) {
+    cudaMemsetAsync(s.row_map, 0, (size_t)((char *)(s.bitmap + s.n_words) - (char *)s.row_map), st);
+  } else {
+    if (int e = build_hash(indices, n_in, batch, g, s, status, st, n_in_dev)) return e;
+    cudaMemsetAsync(s.bitmap, 0, (size_t)s.n_words * 4, st);
+  }
   if (n_in > 0) {
-    bool simple = true;
-    for (int d = 0; d < 3; ++d) simple = simple && (g.transpose || g.stride[d] == 1 || g.dilation[d] == 1);
     if (simple) {
-      { mark_outputs_kernel<<<ceil_div(n_in, 128), 128, 0, st>>>((const int4 *)indices, n_in, batch, g, s.bitmap, n_in_dev); note_launches(1); }
+      { mark_outputs_kernel<<<ceil_div(n_in, 128), 128, 0, st>>>((const int4 *)indices, n_in, batch, g, s.bitmap, n_in_dev,
+                                                                together ? s.row_map : nullptr, status ? status : s.misc + 1); note_launches(1); }
     } else {
       { mark_outputs_generic_kernel<<<ceil_div((long long)n_in * g.K, 256), 256, 0, st>>>((const int4 *)indices, n_in, batch, g, s.bitmap, n_in_dev); note_launches(1); }
     }

@@ -25,6 +25,16 @@ c_int, c_size_t, c_void_p, c_float = ctypes.c_int, ctypes.c_size_t, ctypes.c_voi
 _I3 = ctypes.c_int * 3
 _F3 = ctypes.c_float * 3
 
+class Layer(ctypes.Structure):
+    """ssc_layer of the C header."""
+    _fields_ = ([(n, c_void_p) for n in ("indices", "n_in_dev", "out_indices", "n_out_dev", "features", "filters", "scale",
+                                         "shift", "gate_of_channel", "out", "status", "workspace")]
+                + [("workspace_bytes", c_size_t), ("stream", c_void_p)]
+                + [(n, c_int) for n in ("n_in", "n_out", "batch", "op", "stored", "c_in", "c_out", "precision", "c_keep",
+                                        "scalar_act", "gate_act", "out_precision", "transpose")]
+                + [(n, _I3) for n in ("in_shape", "out_shape", "ksize", "stride", "padding", "dilation")])
+
+
 # name -> (restype, argtypes); kept in one table so tests can check it against the header
 SIGNATURES = {
     "ssc_version": (c_int, []),
@@ -66,6 +76,9 @@ SIGNATURES = {
     "ssc_nbr_row_order_planes_scratch_bytes": (c_size_t, [_I3, c_int]),
     "ssc_nbr_row_order_planes": (c_int, [c_void_p, _I3, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "ssc_conv_stage": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
+    "ssc_layer_struct_bytes": (c_size_t, []),
+    "ssc_layer_ahead_bytes": (c_size_t, [c_void_p]),
+    "ssc_layer_ahead": (c_int, [c_void_p]),
     "ssc_conv_gate_covered": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "ssc_conv_fwd_gated": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p,
                                    c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p,
@@ -231,7 +244,7 @@ _scratch_cache = {}
 
 def status_word(device):
     """Per-device int32 that kernels OR error bits into (read it with check_status())."""
-    key = torch.device(device).index
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index
     if key not in _status:
         _status[key] = torch.zeros(1, dtype=torch.int32, device=device)
     return _status[key]
@@ -398,6 +411,77 @@ def get_indice_pairs_ahead(indices, batch_size, out_shape, spatial_shape, ksize,
     _check(L.ssc_rulebook_conv_fill(_p(indices), n_in, int(batch_size), *geo, cap, _p(outids), _p(nbr), None, None,
                                     _p(st), _p(scratch), sbytes, _p(n_out_dev), _stream()))
     return [outids, LazyPairs(nbr, n_in, n_out_dev=n_out_dev, ratio_key=None if n_in_dev is not None else key), None]
+
+
+def layer_plan(in_shape, out_shape, batch_size, ksize, stride, padding, dilation, transpose, op, dtype, c_in, c_out=0,
+               gate=None):
+    """What does not change between the calls of a layer that runs ahead (layer_ahead) on inputs of one
+    shape and type, or None where the layer has to go step by step.  op: 0 convolution, 1 / 2 maximum /
+    average pool; gate: (c_keep, scalar_act, gate_act)."""
+    K = int(ksize[0]) * int(ksize[1]) * int(ksize[2])
+    cells = int(batch_size) * int(out_shape[0]) * int(out_shape[1]) * int(out_shape[2])
+    in_cells = int(batch_size) * int(in_shape[0]) * int(in_shape[1]) * int(in_shape[2])
+    if K > 256 or max(cells, in_cells) >= 2 ** 31 - 1:
+        return None
+    a = Layer()
+    a.batch, a.op, a.c_in, a.c_out, a.transpose = int(batch_size), op, c_in, c_out, int(transpose)
+    for name, v in (("in_shape", in_shape), ("out_shape", out_shape), ("ksize", ksize), ("stride", stride),
+                    ("padding", padding), ("dilation", dilation)):
+        setattr(a, name, _i3(v))
+    if dtype in _PREC_OF_DTYPE:
+        if op == 0 and (c_in % 8 != 0 or c_out > 512):
+            return None
+        a.stored = a.precision = _PREC_OF[_PREC_OF_DTYPE[dtype]]
+    elif dtype != torch.float32:
+        return None
+    elif op == 0:
+        mode = _resolve_precision(c_in, c_out)
+        a.precision = PREC_FP32 if mode in ("fp16", "bf16") and c_out > 512 else _PREC_OF.get(mode, PREC_FP32)
+    c_row, stored = (c_out or c_in), None
+    if gate is not None:
+        a.c_keep, a.scalar_act, a.gate_act = gate
+        c_row, stored = a.c_keep, _stored_type(0, c_out, a.c_keep, a.c_keep)
+        a.out_precision = _PREC_OF[_storage] if stored else PREC_FP32
+    key = _geometry_key(in_shape, ksize, stride, padding, dilation, transpose)
+    return bytes(a), key, K, cells, a.precision, c_row, stored or torch.float32
+
+
+def layer_ahead(plan, indices, n_in_dev, features, weight=None, gate=None):
+    """(rows [cap, c], indices [cap, 4], device word with their count, capacity) of a layer of plan
+    (layer_plan), queued in one call; None when no capacity can be guessed yet.  gate as in conv_forward."""
+    template, key, K, cells, prec, c_row, dtype = plan
+    ratio = _ratio_hint.get(key)
+    n_in = indices.shape[0]
+    if ratio is None or n_in == 0:
+        return None
+    cap = min(n_in * K, cells, int(n_in * ratio * AHEAD_MARGIN) + 1024)
+    if cap * c_row // 4 >= 2 ** 31:
+        return None
+    dev = indices.device
+    a = Layer.from_buffer_copy(template)
+    a.indices, a.features, a.n_in, a.n_out = _p(indices, torch.int32), _p(features), n_in, cap
+    if n_in_dev is not None:
+        a.n_in_dev = n_in_dev.data_ptr()
+    packed = None
+    if weight is not None:
+        flt = _flat_filters(weight)
+        packed = _packed_filters(flt, prec) if prec != PREC_FP32 else flt
+        a.filters = _p(packed)
+        if gate is not None:
+            if gate[0] is not None:
+                a.scale, a.shift = _p(gate[0]), _p(gate[1])
+            a.gate_of_channel = _p(gate[2])
+    outids = torch.empty((cap, 4), dtype=torch.int32, device=dev)
+    n_out_dev = torch.empty(1, dtype=torch.int32, device=dev)
+    out = torch.empty((cap, c_row), dtype=dtype, device=dev)
+    L = lib()
+    at = ctypes.addressof(a)
+    nbytes = L.ssc_layer_ahead_bytes(at)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    a.out_indices, a.n_out_dev, a.out = outids.data_ptr(), n_out_dev.data_ptr(), out.data_ptr()
+    a.workspace, a.workspace_bytes, a.status, a.stream = ws.data_ptr(), nbytes, status_word(dev).data_ptr(), _stream()
+    _check(L.ssc_layer_ahead(at))
+    return out, outids, n_out_dev, cap
 
 
 def get_indice_pairs_subm_ahead(indices_cap, batch_size, spatial_shape, ksize, dilation, n_in_dev):
@@ -890,21 +974,25 @@ def _conv_forward_pairs(features, filters, nbr, n_out, prec, out, st):
     return out
 
 
+def _flat_filters(filters):
+    """Contiguous [K, Cin, Cout] form of filters [k, k, k, Cin, Cout], kept with the tensor until it changes."""
+    cached = getattr(filters, "_ssc_flat", None)
+    if cached is not None and cached[0] == filters._version:
+        return cached[1]
+    flt = filters.reshape(-1, filters.shape[-2], filters.shape[-1]).contiguous()  # no copy when already contiguous
+    try:
+        filters._ssc_flat = (filters._version, flt)
+    except Exception:
+        pass
+    return flt
+
+
 def indice_conv_fp32(features, filters, indice_pairs, indice_num, num_act_out, inverse, subm, gate=None):
     """Reference signature (SS_Conv_lib/src/ss_conv_ops.h:43-45); filters [k,k,k,Cin,Cout]
     (a permuted view is accepted).  The submanifold centre needs no special case."""
     if features.dtype != torch.float32 and features.dtype not in _PREC_OF_DTYPE:
         raise TypeError("indice_conv_fp32 expects float32 features (or features stored in fp16 / bf16 by this library)")
-    c_in, c_out = filters.shape[-2], filters.shape[-1]
-    cached = getattr(filters, "_ssc_flat", None)
-    if cached is not None and cached[0] == filters._version:
-        flt = cached[1]
-    else:
-        flt = filters.reshape(-1, c_in, c_out).contiguous()  # no copy when already contiguous
-        try:
-            filters._ssc_flat = (filters._version, flt)
-        except Exception:
-            pass
+    flt = _flat_filters(filters)
     nbr, n_out_dev = _table_for(indice_pairs, indice_num, int(num_act_out), bool(inverse))
     order = None
     if inverse and n_out_dev is None and int(num_act_out) >= ROW_ORDER_MIN_ROWS and nbr.shape[0] > 1:

@@ -6,7 +6,7 @@ import torch
 import torch.nn as nn
 from torch.nn.parameter import Parameter
 
-from .tensor import PendingRows, SparseTensor
+from .tensor import PendingRows, SparseTensor, run_ahead
 from .ops import get_conv_output_size, get_deconv_output_size, get_indice_pairs, _per_dim
 from .. import _ext
 from .functional import indice_conv, indice_inverse_conv, indice_subm_conv
@@ -81,6 +81,10 @@ class SparseConvolution(nn.Module):
         if (_ext.AHEAD and not self.conv1x1 and not self.subm and not self.inverse and self.indice_key is None
                 and feats_raw.is_cuda and feats_raw.dtype in _FEATURE_DTYPES
                 and not (torch.is_grad_enabled() and (feats_raw.requires_grad or weight.requires_grad))):
+            if self.bias is None and not torch.cuda.is_current_stream_capturing():
+                out = run_ahead(self, input, 0, out_spatial_shape, int(self.transposed), self._sparse_conv_exact, weight, gate)
+                if out is not None:
+                    return out
             # While a CUDA graph is being recorded, the part of the convolution call that does not
             # need the rulebook (filter packing, staging of the feature rows) goes to a side stream:
             # the graph then runs it next to the rulebook kernels, which leave most of the GPU idle.

@@ -3,13 +3,13 @@ import torch
 import torch.nn as nn
 
 from .. import _ext
-from .tensor import PendingRows, SparseTensor
+from .tensor import PendingRows, SparseTensor, run_ahead
 from .ops import get_conv_output_size, get_indice_pairs, _per_dim
 from .functional import indice_avgpool, indice_maxpool
 
 
 class _SparsePool(nn.Module):
-    _op = _stored16 = None
+    _op = _stored16 = _code = None
 
     def __init__(self, ndim, kernel_size, stride=1, padding=0, dilation=1, subm=False):
         super().__init__()
@@ -34,6 +34,10 @@ class _SparsePool(nn.Module):
             stored16 = False
         if (_ext.AHEAD and not self.subm and feats_raw.is_cuda and (stored16 or feats_raw.dtype == torch.float32)
                 and not (torch.is_grad_enabled() and feats_raw.requires_grad)):
+            if not torch.cuda.is_current_stream_capturing():
+                out = run_ahead(self, input, self._code, out_shape, 0, lambda x: self._forward_exact(x, out_shape))
+                if out is not None:
+                    return out
             ahead, indices_ready = _ext.rulebook_next_to_features(input._rows, lambda: _ext.get_indice_pairs_ahead(
                 inds_raw, input.batch_size, out_shape, list(shape), self.kernel_size, self.stride, self.padding,
                 self.dilation, 0, n_in_dev=n_in_dev))
@@ -76,10 +80,12 @@ class _SparsePool(nn.Module):
 class SparseAvgPool(_SparsePool):
     """out = (sum of present inputs) / kernel volume."""
     _op = staticmethod(indice_avgpool)
+    _code = 2                     # as in _ext.layer_plan
     _stored16 = staticmethod(lambda *a: _ext._pool(*a, True))
 
 
 class SparseMaxPool(_SparsePool):
     """out = max(0, max of present inputs): the output starts from zero."""
     _op = staticmethod(indice_maxpool)
+    _code = 1
     _stored16 = staticmethod(lambda *a: _ext._pool(*a, False))

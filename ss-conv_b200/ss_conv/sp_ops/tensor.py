@@ -199,3 +199,41 @@ class SparseTensor(object):
     @property
     def sparity(self):
         return self.indices.shape[0] / np.prod(self.spatial_shape) / self.batch_size
+
+
+def run_ahead(layer, input, op, out_shape, transpose, exact, weight=None, gate=None):
+    """The output of a strided layer without an indice_key queued in one library call with its count still on
+    the device (_ext.layer_ahead), or None where it has to be queued step by step.  layer: the module (its
+    kernel_size, stride, padding, dilation; it keeps the plans); op as in _ext.layer_plan;
+    exact(input, ...) recomputes the layer on exact row counts."""
+    feats, inds, n_in_dev = input.raw()
+    if not (feats.is_contiguous() and inds.is_contiguous()):
+        return None
+    shape = tuple(input.spatial_shape)
+    key = (shape, input.batch_size, feats.dtype, _ext._precision, _ext._storage, gate[3:] if gate is not None else None)
+    plans = layer.__dict__.setdefault("_ahead_plans", {})
+    plan = plans.get(key)
+    if plan is None:
+        if len(plans) > 64:
+            plans.clear()
+        c_in, c_out = (weight.shape[-2], weight.shape[-1]) if weight is not None else (feats.shape[1], 0)
+        plan = plans[key] = _ext.layer_plan(shape, out_shape, input.batch_size, layer.kernel_size, layer.stride, layer.padding,
+                                            layer.dilation, transpose, op, feats.dtype, c_in, c_out, key[-1]) or False
+    if not plan or (weight is not None and feats.shape[1] != weight.shape[-2]):
+        return None
+    made = _ext.layer_ahead(plan, inds, n_in_dev, feats, weight, gate)
+    if made is None:
+        return None
+    rows, indices, n_out_dev, capacity = made
+    out = SparseTensor(rows, indices, out_shape, input.batch_size)
+    out.indice_dict = input.indice_dict
+    out.grid = input.grid
+
+    def redo():
+        t = exact(input) if weight is None else exact(input, weight, gate)
+        return t.features, t.indices
+
+    ratio_key = plan[1]
+    out._rows = PendingRows(n_out_dev, capacity, input if n_in_dev is not None else None, redo,
+                            lambda n: _ext._note_ratio(ratio_key, input.features.shape[0], n))
+    return out

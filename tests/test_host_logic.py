@@ -30,6 +30,12 @@ def test_library_exports_every_declared_symbol():
     assert _ext.lib().ssc_has_tcgen05() == 1
 
 
+def test_layer_structure_has_the_size_of_the_librarys():
+    import ctypes
+    from ss_conv import _ext
+    assert _ext.lib().ssc_layer_struct_bytes() == ctypes.sizeof(_ext.Layer)
+
+
 def test_argument_errors_without_gpu():
     """Size queries and argument validation run on the host only."""
     from ss_conv import _ext
