@@ -4,6 +4,7 @@
 
 #include "ssc_common.cuh"
 #include "ssc_pool_tile.cuh"
+#include "ssc_scan.cuh"
 
 namespace ssc {
 
@@ -187,6 +188,35 @@ __global__ void batch_scan_kernel(int32_t *offsets, int batch) {
   }
 }
 
+// The three steps for few rows, in one block: what bounds them there is the launches.
+constexpr int kOffsetsRows = 16384, kOffsetsBatch = 4096;
+__global__ void __launch_bounds__(1024)
+batch_offsets_small_kernel(const int4 *__restrict__ indices, int n, int batch, int32_t *__restrict__ offsets,
+                           const int32_t *__restrict__ n_dev) {
+  __shared__ int hist[kOffsetsBatch];
+  __shared__ uint32_t sums[33];
+  for (int i = threadIdx.x; i < batch; i += 1024) hist[i] = 0;
+  __syncthreads();
+  const int live = live_rows(n, n_dev);
+  for (int r0 = 0; r0 < live; r0 += 1024) {
+    const int r = r0 + (int)threadIdx.x;
+    const int b = r < live ? __ldg(&indices[r].x) : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, b);
+    if ((unsigned)b < (unsigned)batch && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(hist + b, __popc(same));
+  }
+  __syncthreads();
+  uint32_t running = 0;
+  for (int b0 = 0; b0 < batch; b0 += 1024) {
+    const int b = b0 + (int)threadIdx.x;
+    const uint32_t v = b < batch ? (uint32_t)hist[b] : 0u;
+    uint32_t total;
+    const uint32_t before = block_exclusive_scan(v, sums, &total);
+    if (b < batch) offsets[b + 1] = (int32_t)(running + before + v);
+    running += total;
+  }
+  if (threadIdx.x == 0) offsets[0] = 0;
+}
+
 }  // namespace ssc
 
 using namespace ssc;
@@ -275,6 +305,12 @@ extern "C" int ssc_batch_offsets(const int32_t *indices, int n, int batch, int32
                                  void *stream) {
   SSC_REQUIRE(n >= 0 && batch >= 1 && offsets, "batch_offsets: bad arguments");
   cudaStream_t st = as_stream(stream);
+  if (n <= kOffsetsRows && batch <= kOffsetsBatch) {
+    batch_offsets_small_kernel<<<1, 1024, 0, st>>>((const int4 *)indices, n, batch, offsets, n_dev);
+    note_launches(1);
+    SSC_CHECK_LAUNCH("batch_offsets");
+    return SSC_OK;
+  }
   cudaMemsetAsync(offsets, 0, (size_t)(batch + 1) * 4, st);
   if (n > 0) { batch_count_kernel<<<ceil_div(n, 256), 256, 0, st>>>((const int4 *)indices, n, batch, offsets, n_dev); note_launches(1); }
   { batch_scan_kernel<<<1, 32, 0, st>>>(offsets, batch); note_launches(1); }

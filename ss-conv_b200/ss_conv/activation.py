@@ -131,9 +131,17 @@ class Activation(nn.Module):
                             torch.tensor(length or [0], dtype=torch.int32, device=device))
         return self._ranges[1], self._ranges[2]
 
+    def _codes(self):
+        """(scalar act code, gate act code) as _act_code gives them."""
+        known = self.__dict__.get("_known_codes")
+        if known is None or known[0] is not self._scalar_fn or known[1] is not self._gate_fn:
+            known = self.__dict__["_known_codes"] = (
+                self._scalar_fn, self._gate_fn, (_act_code(self._scalar_fn if self.scalar_act is not None else None),
+                                                 _act_code(self._gate_fn if self.gate_act is not None else None)))
+        return known[2]
+
     def fusable(self):
-        return _act_code(self._scalar_fn if self.scalar_act is not None else None) is not None and \
-            _act_code(self._gate_fn if self.gate_act is not None else None) is not None
+        return None not in self._codes()
 
     def c_out(self):
         return Rs2dim(self.Rs)
@@ -149,9 +157,7 @@ class Activation(nn.Module):
 
     def gate_tables(self, device):
         """(gate_of_channel, field_start, field_len, scalar act code, gate act code)."""
-        return (self._gate_table(device), *self._field_ranges(device),
-                _act_code(self._scalar_fn) if self.scalar_act is not None else 0,
-                _act_code(self._gate_fn) if self.gate_act is not None else 0)
+        return (self._gate_table(device), *self._field_ranges(device), *self._codes())
 
     def forward(self, input):
         if self.scalar_act is None and self.gate_act is None:
@@ -168,8 +174,7 @@ class Activation(nn.Module):
         recording = torch.is_grad_enabled() and (y.requires_grad or
                                                  (self.training and any(p.requires_grad for p in self.parameters())))
         if self.fusable() and y.is_cuda and not recording:
-            s_code = _act_code(self._scalar_fn) if self.scalar_act is not None else 0
-            g_code = _act_code(self._gate_fn) if self.gate_act is not None else 0
+            s_code, g_code = self._codes()
             s_bias = None
             if self.scalar_act is not None and self.scalar_act.bias is not None:
                 s_bias = torch.zeros(C, dtype=torch.float32, device=y.device)
@@ -180,8 +185,7 @@ class Activation(nn.Module):
         no_bias = (self.scalar_act is None or self.scalar_act.bias is None) and \
             (self.gate_act is None or self.gate_act.bias is None)
         if self.fusable() and y.is_cuda and y.dtype == torch.float32 and no_bias and scale is None and y.shape[0] > 0:
-            s_code = _act_code(self._scalar_fn) if self.scalar_act is not None else 0
-            g_code = _act_code(self._gate_fn) if self.gate_act is not None else 0
+            s_code, g_code = self._codes()
             return _GateFn.apply(y, self, s_code, g_code)     # recording: the library's kernels forward and backward
         return self._gate_composite(y if scale is None else y * scale + shift)
 

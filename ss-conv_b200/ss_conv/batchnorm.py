@@ -101,20 +101,24 @@ class BatchNorm(nn.Module):
 
     def folded_affine(self, device, mean=None, var=None):
         """(scale, shift) per channel for the given statistics (default: running buffers)."""
-        field, scalar = self._device_tables(device)
-        running = mean is None and var is None
-        mean = self.running_mean if mean is None else mean
-        var = self.running_var if var is None else var
-        w = self.weight.detach() if self.affine else None
-        b = self.bias.detach() if self.affine else None
         # the fold of the running buffers is kept until one of its inputs changes (in-place updates bump
         # a tensor's version, moves and reloads change its address): an eval-mode network folds once
-        key = None
+        running = mean is None and var is None
+        w, b = (self._parameters["weight"], self._parameters["bias"]) if self.affine else (None, None)
         if running:
-            key = tuple((t.data_ptr(), t._version) for t in (mean, var, w, b) if t is not None) + (str(device), self.eps)
-            kept = getattr(self, "_folded", None)
+            mean, var = self._buffers["running_mean"], self._buffers["running_var"]
+            key = (mean.data_ptr(), mean._version, var.data_ptr(), var._version, device, self.eps)
+            if w is not None:
+                key += (w.data_ptr(), w._version, b.data_ptr(), b._version)
+            kept = self.__dict__.get("_folded")
             if kept is not None and kept[0] == key:
                 return kept[1]
+        else:
+            key = None
+            mean = self.running_mean if mean is None else mean
+            var = self.running_var if var is None else var
+        field, scalar = self._device_tables(device)
+        w, b = (None if w is None else w.detach()), (None if b is None else b.detach())
         if mean.numel() == 0:
             mean = None
             b = None

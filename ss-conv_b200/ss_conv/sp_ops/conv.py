@@ -76,15 +76,15 @@ class SparseConvolution(nn.Module):
         gate: a folded batch norm and gated activation to apply to the rows (_ext.conv_forward), while no
         gradients are recorded."""
         assert isinstance(input, SparseTensor)
-        out_spatial_shape = self._output_shape(input.spatial_shape)
         feats_raw, inds_raw, n_in_dev = input.raw()
         if (_ext.AHEAD and not self.conv1x1 and not self.subm and not self.inverse and self.indice_key is None
                 and feats_raw.is_cuda and feats_raw.dtype in _FEATURE_DTYPES
                 and not (torch.is_grad_enabled() and (feats_raw.requires_grad or weight.requires_grad))):
             if self.bias is None and not torch.cuda.is_current_stream_capturing():
-                out = run_ahead(self, input, 0, out_spatial_shape, int(self.transposed), self._sparse_conv_exact, weight, gate)
+                out = run_ahead(self, input, 0, self._output_shape, int(self.transposed), self._sparse_conv_exact, weight, gate)
                 if out is not None:
                     return out
+            out_spatial_shape = self._output_shape(input.spatial_shape)
             # While a CUDA graph is being recorded, the part of the convolution call that does not
             # need the rulebook (filter packing, staging of the feature rows) goes to a side stream:
             # the graph then runs it next to the rulebook kernels, which leave most of the GPU idle.
@@ -142,8 +142,7 @@ class SparseConvolution(nn.Module):
                 out_cap = self._op(feats_raw, weight, pairs, None, pairs.capacity, gate)
                 if self.bias is not None:
                     out_cap += self.bias
-                out = SparseTensor(out_cap, inds_raw, out_spatial_shape if self.subm else input.spatial_shape,
-                                   input.batch_size)
+                out = SparseTensor(out_cap, inds_raw, input.spatial_shape, input.batch_size)
                 out.indice_dict = input.indice_dict
                 out.grid = input.grid
                 key = self.indice_key

@@ -90,8 +90,8 @@ def _global_pool_function(native_fp, native_bp):
             n, c = feats.size()
             feats = feats.contiguous()
             proposals_offset = proposals_offset.contiguous().int()
-            out = torch.zeros((n_prop, c), dtype=torch.float32, device=feats.device)
-            maxidx = torch.zeros((n_prop, c), dtype=torch.int32, device=feats.device)
+            out = torch.empty((n_prop, c), dtype=torch.float32, device=feats.device)     # every element is written
+            maxidx = torch.empty((n_prop, c), dtype=torch.int32, device=feats.device)    # (by the maximum only)
             native_fp(feats, proposals_offset, out, maxidx, n_prop, c)
             ctx.for_backwards = (maxidx, proposals_offset, n)
             return out

@@ -35,7 +35,7 @@ class _SparsePool(nn.Module):
         if (_ext.AHEAD and not self.subm and feats_raw.is_cuda and (stored16 or feats_raw.dtype == torch.float32)
                 and not (torch.is_grad_enabled() and feats_raw.requires_grad)):
             if not torch.cuda.is_current_stream_capturing():
-                out = run_ahead(self, input, self._code, out_shape, 0, lambda x: self._forward_exact(x, out_shape))
+                out = run_ahead(self, input, self._code, lambda _: out_shape, 0, lambda x: self._forward_exact(x, out_shape))
                 if out is not None:
                     return out
             ahead, indices_ready = _ext.rulebook_next_to_features(input._rows, lambda: _ext.get_indice_pairs_ahead(

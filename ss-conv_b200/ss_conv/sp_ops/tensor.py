@@ -90,6 +90,7 @@ class SparseTensor(object):
         self._features = features
         self._indices = indices if indices.dtype == torch.int32 else indices.int()
         self._rows = None
+        self._cut = None          # exact row count the buffers still have to be cut down to, see resolve
         self._recomputed = False  # contents replaced when the pending count was read back, see resolve
         self._affine = None       # (scale, shift) of an eval-mode batch norm not applied yet, see _flush_affine
         self.spatial_shape = spatial_shape
@@ -112,26 +113,40 @@ class SparseTensor(object):
         aff, self._affine = self._affine, None
         return aff
 
+    def _trim(self):
+        """Cuts the buffers of a resolved count down to it: the inner tensors of a network are resolved with
+        its last one, but nobody looks at most of them."""
+        n, self._cut = self._cut, None
+        self._features, self._indices = self._features[:n], self._indices[:n]
+
     @property
     def features(self):
         self._flush_affine()
         if self._rows is not None:
             self.resolve()
+        if self._cut is not None:
+            self._trim()
         return self._features
 
     @features.setter
     def features(self, value):
         self._affine = None
+        if self._cut is not None:
+            self._trim()
         self._features = value
 
     @property
     def indices(self):
         if self._rows is not None:
             self.resolve()
+        if self._cut is not None:
+            self._trim()
         return self._indices
 
     @indices.setter
     def indices(self, value):
+        if self._cut is not None:
+            self._trim()
         self._indices = value if value.dtype == torch.int32 else value.int()
 
     def pending(self):
@@ -140,7 +155,10 @@ class SparseTensor(object):
     def raw(self):
         """(features, indices, n_dev): the buffers as they are; n_dev is None for an exact tensor,
         else the device word with the number of meaningful rows."""
-        self._flush_affine()
+        if self._affine is not None:
+            self._flush_affine()
+        if self._cut is not None:
+            self._trim()
         return self._features, self._indices, (self._rows.n_dev if self._rows is not None else None)
 
     def resolve(self):
@@ -160,7 +178,8 @@ class SparseTensor(object):
             r.note(n)
         self._rows = None
         if not parent_changed and n <= r.capacity:
-            self._features, self._indices = self._features[:n], self._indices[:n]
+            if n != self._features.shape[0] or n != self._indices.shape[0]:
+                self._cut = n
             return False
         with torch.set_grad_enabled(r.grad):
             feats, inds = r.redo()
@@ -201,15 +220,15 @@ class SparseTensor(object):
         return self.indices.shape[0] / np.prod(self.spatial_shape) / self.batch_size
 
 
-def run_ahead(layer, input, op, out_shape, transpose, exact, weight=None, gate=None):
+def run_ahead(layer, input, op, output_shape, transpose, exact, weight=None, gate=None):
     """The output of a strided layer without an indice_key queued in one library call with its count still on
     the device (_ext.layer_ahead), or None where it has to be queued step by step.  layer: the module (its
-    kernel_size, stride, padding, dilation; it keeps the plans); op as in _ext.layer_plan;
-    exact(input, ...) recomputes the layer on exact row counts."""
+    kernel_size, stride, padding, dilation; it keeps the plans); op as in _ext.layer_plan; output_shape(shape)
+    gives the spatial shape of its output, exact(input, ...) recomputes the layer on exact row counts."""
     feats, inds, n_in_dev = input.raw()
     if not (feats.is_contiguous() and inds.is_contiguous()):
         return None
-    shape = tuple(input.spatial_shape)
+    shape = tuple(input.spatial_shape)          # (a list, or an array)
     key = (shape, input.batch_size, feats.dtype, _ext._precision, _ext._storage, gate[3:] if gate is not None else None)
     plans = layer.__dict__.setdefault("_ahead_plans", {})
     plan = plans.get(key)
@@ -217,15 +236,17 @@ def run_ahead(layer, input, op, out_shape, transpose, exact, weight=None, gate=N
         if len(plans) > 64:
             plans.clear()
         c_in, c_out = (weight.shape[-2], weight.shape[-1]) if weight is not None else (feats.shape[1], 0)
-        plan = plans[key] = _ext.layer_plan(shape, out_shape, input.batch_size, layer.kernel_size, layer.stride, layer.padding,
-                                            layer.dilation, transpose, op, feats.dtype, c_in, c_out, key[-1]) or False
-    if not plan or (weight is not None and feats.shape[1] != weight.shape[-2]):
+        out_shape = output_shape(input.spatial_shape)
+        plan = plans[key] = (_ext.layer_plan(shape, out_shape, input.batch_size, layer.kernel_size, layer.stride, layer.padding,
+                                             layer.dilation, transpose, op, feats.dtype, c_in, c_out, key[-1]), tuple(out_shape))
+    plan, out_shape = plan
+    if plan is None or (weight is not None and feats.shape[1] != weight.shape[-2]):
         return None
     made = _ext.layer_ahead(plan, inds, n_in_dev, feats, weight, gate)
     if made is None:
         return None
     rows, indices, n_out_dev, capacity = made
-    out = SparseTensor(rows, indices, out_shape, input.batch_size)
+    out = SparseTensor(rows, indices, list(out_shape), input.batch_size)
     out.indice_dict = input.indice_dict
     out.grid = input.grid
 

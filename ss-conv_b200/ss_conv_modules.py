@@ -54,16 +54,19 @@ class SS_Conv(nn.Module):
         """The folded batch norm and the activation for the convolution to apply as it stores its rows
         (_ext.conv_forward), or None: while gradients are recorded or statistics are taken, with biases or
         an activation the library does not know, with hooks on the modules that would not be called."""
-        bn, act, conv = self.bn, self.activation, self.conv
-        if (torch.is_grad_enabled() or act is None or conv.bias is not None or conv.training or (bn is not None and bn.training)
-                or conv._forward_hooks or act._forward_hooks or act._forward_pre_hooks
-                or (bn is not None and (bn._forward_hooks or bn._forward_pre_hooks)) or not act.fusable_gate()):
+        if torch.is_grad_enabled():
+            return None
+        parts = self._modules
+        bn, act, conv = parts.get("bn"), parts.get("activation"), parts["conv"]
+        if (act is None or conv.training or conv._parameters["bias"] is not None or conv._forward_hooks or act._forward_hooks
+                or act._forward_pre_hooks or (bn is not None and (bn.training or bn._forward_hooks or bn._forward_pre_hooks))
+                or not act.fusable_gate()):
             return None
         device = x.raw()[0].device
         if device.type != "cuda":
             return None
-        table, _, _, scalar_act, gate_act = act.gate_tables(device)
-        return (*(bn.folded_affine(device) if bn is not None else (None, None)), table, act.c_out(), scalar_act, gate_act)
+        scale, shift = bn.folded_affine(device) if bn is not None else (None, None)
+        return (scale, shift, act._gate_table(device), act.c_out(), *act._codes())
 
     def forward(self, x):
         gate = self._inference_gate(x)

@@ -143,3 +143,16 @@ def test_gated_convolution_has_the_bits_of_the_two_passes(cuda, c_in, c_out, c_k
         _ext.set_feature_storage(None)
     _ext.check_status(cuda)
     assert got.dtype == want.dtype and torch.equal(got, want) and float(x.abs().max()) > 0
+
+
+@pytest.mark.parametrize("n,batch", [(0, 1), (1, 3), (1025, 1024), (16384, 4096), (16385, 7), (300, 4097)])
+def test_batch_offsets_at_the_sizes_of_the_one_block_form(cuda, n, batch):
+    """Rows in any order, samples without rows, ids outside the batch (counted nowhere): a plain histogram's prefix."""
+    from ss_conv import _ext
+    b = np.random.RandomState(n).randint(-1, batch + 1, n)
+    ind = np.zeros((n, 4), np.int32)
+    ind[:, 0] = b
+    got = _ext.batch_offsets(dev(ind, cuda), batch)
+    inside = b[(b >= 0) & (b < batch)]
+    want = np.concatenate([[0], np.cumsum(np.bincount(inside, minlength=batch))])
+    assert got.cpu().numpy().tolist() == want.tolist()
