@@ -364,14 +364,14 @@ int ssc_conv_fwd_ordered(const float *features, int n_in, int c_in, const void *
 /* ssc_conv_fwd followed by ssc_bn_gate_fwd / ssc_bn_gate_fwd16 (c_gate_base = c_keep, no biases) as one kernel, with
  * their results bit for bit: out [n_out, c_keep] = gate(scale * conv + shift), fp32 or (out_precision SSC_PREC_F16 /
  * SSC_PREC_BF16, c_keep a multiple of eight) 16-bit rows.  scale / shift may both be NULL.  `precision` is a
- * tensor-core one (SSC_CONV_PRESTAGED may be or'ed in), `scratch` is needed.  ssc_conv_gate_covered: 1 where the
+ * tensor-core one (SSC_CONV_PRESTAGED may be or'ed in), `scratch` is needed, row_order as in ssc_conv_fwd_ordered.  ssc_conv_gate_covered: 1 where the
  * sizes are covered (TF32 with c_in <= 16 is not, nor are more than 256 channels of few rows). */
 int ssc_conv_gate_covered(int c_in, int c_out, int c_keep, int precision, int n_out);
 int ssc_conv_fwd_gated(const float *features, int n_in, int c_in, const void *filters, int K, int c_out,
                        const int32_t *nbr, int n_out, int precision, const float *scale, const float *shift,
                        const int32_t *gate_of_channel, int c_keep, int scalar_act, int gate_act, int out_precision,
                        void *out, int32_t *status, void *scratch, size_t scratch_bytes, const int32_t *n_out_dev,
-                       void *stream);
+                       const int32_t *row_order, void *stream);
 size_t ssc_conv_wgrad_scratch_bytes(int K, int c_in, int c_out, int n_out);
 int ssc_conv_wgrad(const float *features, int c_in, const float *out_grad, int c_out, const int32_t *nbr,
                    int K, int n_out, int precision, float *d_filters, int32_t *status, void *scratch,

@@ -366,7 +366,7 @@ extern "C" int ssc_conv_fwd_gated(const float *features, int n_in, int c_in, con
                                   const int32_t *nbr, int n_out, int precision, const float *scale, const float *shift,
                                   const int32_t *gate_of_channel, int c_keep, int scalar_act, int gate_act, int out_precision,
                                   void *out, int32_t *status, void *scratch, size_t scratch_bytes, const int32_t *n_out_dev,
-                                  void *stream) {
+                                  const int32_t *row_order, void *stream) {
   SSC_REQUIRE(c_in > 0 && c_out > 0 && K > 0 && n_in >= 0 && n_out >= 0, "conv_fwd_gated: bad sizes");
   const bool prestaged = (precision & SSC_CONV_PRESTAGED) != 0;
   precision &= ~SSC_CONV_PRESTAGED;
@@ -379,8 +379,8 @@ extern "C" int ssc_conv_fwd_gated(const float *features, int n_in, int c_in, con
   const GateEpilogue gate = {scale, shift, gate_of_channel, c_keep, scalar_act, gate_act,
                              out_precision == SSC_PREC_F16 ? 1 : out_precision == SSC_PREC_BF16 ? 2 : 0};
   if (precision == SSC_PREC_TF32)
-    return conv_fwd_tf32(features, n_in, c_in, filters, K, c_out, nbr, n_out, (float *)out, status, scratch, scratch_bytes, n_out_dev, nullptr, prestaged, 0, gate, as_stream(stream));
-  return conv_fwd_16(features, n_in, c_in, precision == SSC_PREC_BF16, filters, K, c_out, nbr, n_out, (float *)out, status, scratch, scratch_bytes, n_out_dev, nullptr, prestaged, 0, gate, as_stream(stream));
+    return conv_fwd_tf32(features, n_in, c_in, filters, K, c_out, nbr, n_out, (float *)out, status, scratch, scratch_bytes, n_out_dev, row_order, prestaged, 0, gate, as_stream(stream));
+  return conv_fwd_16(features, n_in, c_in, precision == SSC_PREC_BF16, filters, K, c_out, nbr, n_out, (float *)out, status, scratch, scratch_bytes, n_out_dev, row_order, prestaged, 0, gate, as_stream(stream));
 }
 
 extern "C" int ssc_conv_fwd(const float *features, int n_in, int c_in, const void *filters, int K, int c_out,

@@ -902,7 +902,7 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
         }
 #pragma unroll 4
         for (int i = 0; i < 8; ++i) {
-          const int row = 4 * i + (lane >> 3), to = m0 + quarter * 32 + row;
+          const int row = 4 * i + (lane >> 3), at_row = m0 + quarter * 32 + row;
           const float4 x = *(const float4 *)(blk + row * 32 + ((q ^ (row & 7)) << 2));
           float v[4] = {x.x, x.y, x.z, x.w};
           if (gate.scale) {
@@ -919,8 +919,8 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) v[j] *= gp[j][row];
-          if (to >= n_rows) continue;
-          const size_t at = (size_t)to * c_row + col;
+          if (at_row >= n_rows) continue;
+          const size_t at = (size_t)(order ? __ldg(order + at_row) : at_row) * c_row + col;
           if (gate.out16 == 0) {
             if (vec) {
               *(float4 *)(out + at) = make_float4(v[0], v[1], v[2], v[3]);

@@ -68,7 +68,7 @@ extern "C" int ssc_layer_ahead(const ssc_layer *layer) {
   const int precision = a.precision | (a.stored ? SSC_CONV_PRESTAGED : 0);
   if (gate_fused(a))
     return ssc_conv_fwd_gated(rows, a.n_in, a.c_in, a.filters, K, a.c_out, nbr, a.n_out, precision, a.scale, a.shift, a.gate_of_channel,
-                              a.c_keep, a.scalar_act, a.gate_act, a.out_precision, a.out, a.status, image, image_bytes, a.n_out_dev, a.stream);
+                              a.c_keep, a.scalar_act, a.gate_act, a.out_precision, a.out, a.status, image, image_bytes, a.n_out_dev, nullptr, a.stream);
   float *conv = a.gate_of_channel ? (float *)(ws + s.rows) : (float *)a.out;
   rc = ssc_conv_fwd(rows, a.n_in, a.c_in, a.filters, K, a.c_out, nbr, a.n_out, precision, conv, a.status,
                     a.precision == SSC_PREC_FP32 ? nullptr : image, a.precision == SSC_PREC_FP32 ? 0 : image_bytes, a.n_out_dev, a.stream);

@@ -82,7 +82,7 @@ SIGNATURES = {
     "ssc_conv_gate_covered": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "ssc_conv_fwd_gated": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p,
                                    c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p,
-                                   c_void_p]),
+                                   c_void_p, c_void_p]),
     "ssc_conv_fwd_ordered": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p,
                                      c_void_p, c_void_p, c_size_t, c_void_p, c_void_p, c_void_p]),
     "ssc_conv_wgrad_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
@@ -410,7 +410,9 @@ def get_indice_pairs_ahead(indices, batch_size, out_shape, spatial_shape, ksize,
     # they are computed only if somebody turns the handle into reference-format pair lists
     _check(L.ssc_rulebook_conv_fill(_p(indices), n_in, int(batch_size), *geo, cap, _p(outids), _p(nbr), None, None,
                                     _p(st), _p(scratch), sbytes, _p(n_out_dev), _stream()))
-    return [outids, LazyPairs(nbr, n_in, n_out_dev=n_out_dev, ratio_key=None if n_in_dev is not None else key), None]
+    pairs = LazyPairs(nbr, n_in, n_out_dev=n_out_dev, ratio_key=None if n_in_dev is not None else key)
+    pairs.regular = True
+    return [outids, pairs, None]
 
 
 def layer_plan(in_shape, out_shape, batch_size, ksize, stride, padding, dilation, transpose, op, dtype, c_in, c_out=0,
@@ -552,6 +554,9 @@ class LazyPairs(object):
     (indexing, .cpu(), arithmetic ...) gets the real tensor, built on first use by
     ssc_pairs_from_nbr."""
 
+    regular = False      # built ahead for a strided layer: other rows than the input's
+    _inverse = None
+
     def __init__(self, nbr, n_in, n_out_dev=None, ratio_key=None):
         self._nbr_cap = nbr                  # [K, capacity]; capacity == n_out unless built ahead
         self.capacity = int(nbr.shape[1])
@@ -594,6 +599,13 @@ class LazyPairs(object):
             self.capacity = n
         return self._nbr_cap
 
+    def inverse_table(self):
+        """The table [K, n_in] of the exchanged roles, kept with the handle: for every (offset, input row) the
+        output row.  Needs no exact count: rows past it have no neighbours."""
+        if self._inverse is None:
+            self._inverse = input_major_table(self._nbr_cap, self._n_in)
+        return self._inverse
+
     def to(self, *args, **kwargs):
         return self
 
@@ -633,8 +645,11 @@ def _table_for(pairs, num, n_out, inverse=False):
 def neighbour_table(pairs, num, n_out, inverse=False):
     """nbr [K, n_out] for a reference-format rulebook (cached on the pair tensor when possible)."""
     if isinstance(pairs, LazyPairs):
-        if not inverse and pairs._ssc_nbr.shape[1] == n_out:
-            return pairs._ssc_nbr
+        nbr = pairs._ssc_nbr
+        if not inverse and nbr.shape[1] == n_out:
+            return nbr
+        if inverse and pairs._n_in == n_out:
+            return pairs.inverse_table()
         pairs = pairs.materialize()
     nbr = getattr(pairs, "_ssc_nbr", None)
     if nbr is not None and not inverse and nbr.shape[1] == n_out and nbr.device == pairs.device:
@@ -854,12 +869,12 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
     if image is not None and mode == "tf32":
         ready = (PREC_TF32, _packed_filters(filters, PREC_TF32), image, image.numel())
     prec = _PREC_OF.get(mode, PREC_FP32)
-    if gate is not None and row_order is None and not flag and _gate_covered(c_in, c_out, gate[3], prec, n_out):
+    if gate is not None and not flag and _gate_covered(c_in, c_out, gate[3], prec, n_out):
         if ready is None or ready[0] != prec:
             nbytes = lib().ssc_conv_scratch_bytes(features.shape[0], c_in, c_out, prec)
             ready = (0, _packed_filters(filters, prec), torch.empty(nbytes, dtype=torch.uint8, device=features.device), nbytes)
         return _conv_gated(_p(features, torch.float32), features.shape[0], c_in, ready[1], K, c_out, nbr, n_out,
-                           prec | (PRESTAGED if ready[0] else 0), gate, st, _p(ready[2]), ready[3], n_out_dev)
+                           prec | (PRESTAGED if ready[0] else 0), gate, st, _p(ready[2]), ready[3], n_out_dev, row_order)
     out = torch.empty((n_out, c_out), dtype=torch.float32, device=features.device)
     if ready is not None and ready[0] == prec:
         prec, packed, scratch, nbytes = ready
@@ -895,14 +910,14 @@ def _gate_covered(c_in, c_out, c_keep, prec, n_out):
     return prec != PREC_FP32 and bool(lib().ssc_conv_gate_covered(c_in, c_out, c_keep, prec, int(n_out)))
 
 
-def _conv_gated(features, n_in, c_in, packed, K, c_out, nbr, n_out, prec, gate, st, scratch, nbytes, n_out_dev):
+def _conv_gated(features, n_in, c_in, packed, K, c_out, nbr, n_out, prec, gate, st, scratch, nbytes, n_out_dev, row_order=None):
     scale, shift, table, c_keep, scalar_act, gate_act = gate
     stored = _stored_type(n_out, c_out, c_keep, c_keep)
     out = torch.empty((n_out, c_keep), dtype=stored or torch.float32, device=nbr.device)
     _check(lib().ssc_conv_fwd_gated(features, n_in, c_in, _p(packed), K, c_out, _p(nbr, torch.int32), int(n_out), prec,
                                     _p(scale), _p(shift), _p(table), c_keep, scalar_act, gate_act,
                                     _PREC_OF[_storage] if stored else PREC_FP32, _p(out), _p(st), scratch, nbytes,
-                                    _p(n_out_dev), _stream()))
+                                    _p(n_out_dev), _p(row_order), _stream()))
     return out
 
 

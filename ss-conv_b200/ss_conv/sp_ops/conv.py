@@ -68,7 +68,7 @@ class SparseConvolution(nn.Module):
         indice_key; an inverse convolution reuses its partner's rulebook with the pair roles
         exchanged.
 
-        A regular (strided / transposed) convolution without an indice_key can run ahead of its
+        A regular (strided / transposed) convolution (with an indice_key: on exact rows) can run ahead of its
         output count: rulebook and convolution are queued with a guessed row capacity (also on
         an input whose own count is still pending) and the result is a SparseTensor with pending
         rows; see sp_ops/tensor.py.
@@ -77,10 +77,13 @@ class SparseConvolution(nn.Module):
         gradients are recorded."""
         assert isinstance(input, SparseTensor)
         feats_raw, inds_raw, n_in_dev = input.raw()
-        if (_ext.AHEAD and not self.conv1x1 and not self.subm and not self.inverse and self.indice_key is None
+        key = self.indice_key
+        if (_ext.AHEAD and not self.conv1x1 and not self.subm and not self.inverse
+                and (key is None or (n_in_dev is None and key not in input.indice_dict
+                                     and not torch.cuda.is_current_stream_capturing()))
                 and feats_raw.is_cuda and feats_raw.dtype in _FEATURE_DTYPES
                 and not (torch.is_grad_enabled() and (feats_raw.requires_grad or weight.requires_grad))):
-            if self.bias is None and not torch.cuda.is_current_stream_capturing():
+            if key is None and self.bias is None and not torch.cuda.is_current_stream_capturing():
                 out = run_ahead(self, input, 0, self._output_shape, int(self.transposed), self._sparse_conv_exact, weight, gate)
                 if out is not None:
                     return out
@@ -103,21 +106,23 @@ class SparseConvolution(nn.Module):
                     _ext._prepared.clear()
             if ahead is not None:
                 outids_cap, pairs, pair_num = ahead
+                if key is not None:
+                    input.indice_dict[key] = (outids_cap, inds_raw, pairs, None, input.spatial_shape)
                 out_cap = self._op(feats_raw, weight, pairs, pair_num, pairs.capacity, gate)
                 if self.bias is not None:
                     out_cap += self.bias
                 out = SparseTensor(out_cap, outids_cap, out_spatial_shape, input.batch_size)
                 out.indice_dict = input.indice_dict
                 out.grid = input.grid
-                key = _ext._geometry_key(input.spatial_shape, self.kernel_size, self.stride, self.padding,
-                                         self.dilation, self.transposed)
+                ratio_key = _ext._geometry_key(input.spatial_shape, self.kernel_size, self.stride, self.padding,
+                                               self.dilation, self.transposed)
 
                 def redo():
                     t = self._sparse_conv_exact(input, weight, gate)
                     return t.features, t.indices
 
                 out._rows = PendingRows(pairs._n_out_dev, pairs.capacity, input if input.pending() else None, redo,
-                                        lambda n: _ext._note_ratio(key, input.features.shape[0], n))
+                                        lambda n: _ext._note_ratio(ratio_key, input.features.shape[0], n))
                 pairs.count = out._rows.count
                 out._rows.indices_ready = indices_ready   # the next layer's rulebook may start here
                 return out
@@ -128,16 +133,16 @@ class SparseConvolution(nn.Module):
             # keeps the row set of its input: on an input whose count is still on the device it works
             # on the capacity-sized buffers and hands the pending count on (so a whole stack of such
             # layers - a module of the Plain backbones - queues without a host round trip).
-            cached = input.find_indice_pair(self.indice_key)
+            cached = input.find_indice_pair(key)
             pairs = None
             if cached is not None and isinstance(cached[2], _ext.LazyPairs) and cached[2].pending() \
-                    and cached[2].capacity == inds_raw.shape[0]:
+                    and not cached[2].regular and cached[2].capacity == inds_raw.shape[0]:
                 pairs = cached[2]
             elif cached is None and self.subm:
                 pairs = _ext.get_indice_pairs_subm_ahead(inds_raw, input.batch_size, list(input.spatial_shape),
                                                          self.kernel_size, self.dilation, n_in_dev)
-                if self.indice_key is not None:
-                    input.indice_dict[self.indice_key] = (inds_raw, inds_raw, pairs, None, input.spatial_shape)
+                if key is not None:
+                    input.indice_dict[key] = (inds_raw, inds_raw, pairs, None, input.spatial_shape)
             if pairs is not None:
                 out_cap = self._op(feats_raw, weight, pairs, None, pairs.capacity, gate)
                 if self.bias is not None:
@@ -145,7 +150,6 @@ class SparseConvolution(nn.Module):
                 out = SparseTensor(out_cap, inds_raw, input.spatial_shape, input.batch_size)
                 out.indice_dict = input.indice_dict
                 out.grid = input.grid
-                key = self.indice_key
 
                 def redo():
                     # the table the pending rows were built on is void; one that an earlier layer of
@@ -161,7 +165,42 @@ class SparseConvolution(nn.Module):
                 pairs.count = out._rows.count
                 out._rows.indices_ready = getattr(input._rows, "indices_ready", None)
                 return out
+        if self.inverse and _ext.AHEAD and input.pending() and not self.conv1x1:
+            out = self._inverse_ahead(input, feats_raw, inds_raw, weight, gate)
+            if out is not None:
+                return out
         return self._sparse_conv_exact(input, weight, gate)
+
+    def _inverse_ahead(self, input, feats, inds, weight, gate):
+        """An inverse convolution whose partner ran ahead: it gathers through the exchanged table, whose rows are
+        the partner's input rows, so the number of the input's own rows is not needed.  None where it does not
+        apply."""
+        cached = input.find_indice_pair(self.indice_key)
+        if (cached is None or not isinstance(cached[2], _ext.LazyPairs) or not cached[2].regular or not cached[2].pending()
+                or cached[0] is not inds or not feats.is_cuda or feats.dtype not in _FEATURE_DTYPES
+                or torch.cuda.is_current_stream_capturing()
+                or (torch.is_grad_enabled() and (feats.requires_grad or weight.requires_grad))):
+            return None
+        _, outids, pairs, _, out_spatial_shape = cached
+        assert pairs.shape[0] == np.prod(self.kernel_size), "inverse conv must have same kernel size as its couple conv"
+        n = outids.shape[0]
+        table = pairs.inverse_table()
+        order = _ext.nbr_row_order(table) if n >= _ext.ROW_ORDER_MIN_ROWS and table.shape[0] > 1 else None
+        rows = _ext.conv_forward(feats, _ext._flat_filters(weight), table, n, row_order=order, gate=gate)
+        if self.bias is not None:
+            rows += self.bias
+        out = SparseTensor(rows, outids, out_spatial_shape, input.batch_size)
+        out.indice_dict = input.indice_dict
+        out.grid = input.grid
+
+        def redo():
+            t = self._sparse_conv_exact(input, weight, gate)
+            return t.features, t.indices
+
+        # its count is known, but its rows are void if those of its input are
+        out._rows = PendingRows(torch.full((1,), n, dtype=torch.int32, device=feats.device), n, input, redo)
+        out._rows.count.value = n
+        return out
 
     def _op(self, features, weight, pairs, num, n_out, gate):
         if gate is not None:
@@ -180,8 +219,10 @@ class SparseConvolution(nn.Module):
         if n is None:                                  # built for rows that did not fit: void
             input.indice_dict.pop(self.indice_key)
             return None
-        if outids.shape[0] != n:                       # a table on pending rows has as many outputs as inputs
-            outids, indices = outids[:n], indices[:n]
+        if outids.shape[0] != n:
+            if not pairs.regular:                      # a table on pending rows has as many outputs as inputs
+                indices = indices[:n]
+            outids = outids[:n]
             cached = input.indice_dict[self.indice_key] = (outids, indices, pairs, num, shape)
         return cached
 

@@ -143,6 +143,9 @@ def test_gated_convolution_has_the_bits_of_the_two_passes(cuda, c_in, c_out, c_k
         _ext.set_feature_storage(None)
     _ext.check_status(cuda)
     assert got.dtype == want.dtype and torch.equal(got, want) and float(x.abs().max()) > 0
+    if stored is None:                              # rows scattered by a row order: the same rows
+        order = torch.randperm(n, device=cuda, dtype=torch.int32)
+        assert torch.equal(_ext.conv_forward(feats, W, nbr, n, precision, row_order=order, gate=(scale, shift, table, c_keep, 1, 2)), want)
 
 
 @pytest.mark.parametrize("n,batch", [(0, 1), (1, 3), (1025, 1024), (16384, 4096), (16385, 7), (300, 4097)])

@@ -2,8 +2,11 @@
 relies on the rulebook cached by the module's first block (SS_Conv_lib/ss_conv/sp_ops/conv.py:124-136)
 gives the exact pass's result also when a capacity guess was too small, and when the counts are read
 back in the middle of the stack (batch statistics in training mode do that)."""
+import numpy as np
 import pytest
 import torch
+
+from gpu_helpers import dev, random_voxels
 
 pytestmark = pytest.mark.gpu
 
@@ -59,3 +62,41 @@ def test_counts_read_back_inside_the_stack(cuda):
         assert torch.equal(got[1], ref[1])
         assert torch.equal(got[0], ref[0])
     _ext.check_status(cuda)
+
+
+@pytest.mark.parametrize("overflow", [False, True])
+def test_inverse_convolution_behind_a_pending_partner(cuda, overflow):
+    """Encode and decode under one indice_key without a read-back in between, with a capacity that fits and with one
+    that does not (both layers are then recomputed): the rows of the exact path, and the shared rulebook entry
+    ends up exact."""
+    from ss_conv import _ext
+    from ss_conv.sp_ops.tensor import SparseTensor
+    from ss_conv_modules import SS_Conv
+    import torch.nn as nn
+    torch.manual_seed(3)
+    act = (torch.relu, torch.sigmoid)
+    net = nn.Sequential(SS_Conv((4,) * 4, (4,) * 4, 3, stride=2, padding=1, activation=act, indice_key="level"),
+                        SS_Conv((4,) * 4, (4,) * 4, 3, inverse=True, activation=act, indice_key="level"),
+                        SS_Conv((4,) * 4, (4,) * 4, 3, padding=1, subm=True, activation=act)).to(cuda).eval()
+    rng = np.random.RandomState(4)
+    ind = dev(random_voxels(rng, 3, 24, 4000), cuda)
+    feats = torch.randn(ind.shape[0], 64, device=cuda)
+
+    def run():
+        y = net(SparseTensor(feats, ind, [24] * 3, 3))
+        return y.features.clone(), y.indices.clone(), net[0].conv._cached_rulebook(y)
+
+    with torch.no_grad():
+        ahead, _ext.AHEAD = _ext.AHEAD, False
+        try:
+            want = run()
+        finally:
+            _ext.AHEAD = ahead
+        run()                                        # (learns the ratio)
+        if overflow:
+            for k in list(_ext._ratio_hint):
+                _ext._ratio_hint[k] = 1e-3
+        got = run()
+    _ext.check_status(cuda)
+    assert torch.equal(got[1], want[1]) and torch.equal(got[0], want[0])
+    assert torch.equal(got[2][0], want[2][0]) and torch.equal(got[2][1], want[2][1])
