@@ -33,7 +33,7 @@ constexpr int TC_SLAB = 32;            // tf32 elements per 128-byte operand row
 constexpr int TC_MAX_STAGES = 8;       // producer warps = ring slots
 constexpr int TC_EPI_WARPS = 4;        // warps 0..3 also run the epilogue (one TMEM lane quarter each)
 constexpr int TC_A_BYTES = TC_M * 128;
-constexpr int TC_ROWS_THREADS = 288;     // conv_fwd_rows_kernel: two groups of four producer warps (or one) and the issuing warp
+constexpr int TC_ROWS_THREADS = 288;     // conv_fwd_rows_kernel: two groups of four producer warps and the issuing warp
 constexpr int TC_CTRL_BYTES = 1024;
 constexpr int TC_LIST_BYTES = TC_M * 5;   // a slot's list of present rows: 128 source rows, 128 rows of the tile
 
@@ -588,10 +588,28 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 }
 
 // ---------------------------------------------------------------------------------------------------
+// (from >= 0) the two 16-byte pieces of a row that a lane copies, OFF bytes into its part of the slot; predicated
+// instead of branched around: a branch per row is what the copies themselves cost.
+template <int OFF>
+__device__ __forceinline__ void copy_row_pieces(int from, uint32_t dst0, uint32_t dst1, const float *src) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %0, 0;\n\t"
+      "@p cp.async.cg.shared.global [%1+%4], [%3], 16;\n\t"
+      "@p cp.async.cg.shared.global [%2+%4], [%3+64], 16;\n\t}" ::"r"(from), "r"(dst0), "r"(dst1), "l"(src), "n"(OFF)
+      : "memory");
+}
+// (one lane) a word for the issuing warp and the arrival that releases it.
+__device__ __forceinline__ void store_and_arrive(bool on, uint32_t at, uint32_t word, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t"
+      "@p st.shared.u32 [%1], %2;\n\t"
+      "@p mbarrier.arrive.shared::cta.b64 _, [%3];\n\t}" ::"r"((uint32_t)on), "r"(at), "r"(word), "r"(bar)
+      : "memory");
+}
+
 // The kernel for staged operands (TF32-rounded fp32 rows, or fp16 / bf16 rows: F16), one kernel offset and one
-// 128-byte slab per step.  Warps 0-3 produce (and run the epilogue), a lane per output row of the tile; with
-// four ring slots or more (few CTAs per SM) warps 4-7 are a second group that takes every other
-// offset; the last warp issues the MMAs.
+// 128-byte slab per step.  Warps 0-3 and 4-7 are two groups of producers, each of which fills every other slot
+// (and they run the epilogue), a lane per output row of the tile; the last warp issues the MMAs.
 //
 // What bounds it is the way of an operand slot: free -> rows gathered -> multiplied -> free, against the slots that
 // fit an SM (eight of 26 KB for 64 -> 76 channels).  With a warp per slot that built its row lists, waited
@@ -610,7 +628,7 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 // every row once more: 164 us of the 12 layers of a backbone, 320 us of 24 with bf16 rows.  A row's gate
 // scalars are evaluated first, a lane per row, into shared memory; the arithmetic is that pass's, so are the bits.
 template <bool F16, bool GATED>
-__global__ void __launch_bounds__(TC_ROWS_THREADS, 3)
+__global__ void __launch_bounds__(TC_ROWS_THREADS, 4)
 conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
                      const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out, int32_t *status, TcParams p,
                      const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order, GateEpilogue gate) {
@@ -628,7 +646,7 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int stage_bytes = TC_A_BYTES + p.b_bytes;
   const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
-  const int groups = (int)blockDim.x / 128, mma_warp = groups * 4;   // producer groups of four warps
+  constexpr int groups = 2, mma_warp = groups * 4;                   // producer groups of four warps
   const int quarter = warp & 3;                                      // the 32 rows of the tile a producer warp works on
   const int m0 = blockIdx.x * TC_M, nt0 = (int)blockIdx.y * p.nt_cta, S = p.stages;
   auto table = [&](int kap) { return nbr + (size_t)(p.rev ? K - 1 - kap : kap) * n_out; };
@@ -708,66 +726,77 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   if (warp < mma_warp) {
     // ====================== producers =========================================================
     // Four lanes per row, eight rows per pass: lane l copies the 16-byte pieces l & 3 and (l & 3) + 4 of the row
-    // 8 * pass + l / 4 of its warp's 32 rows, where that row has a neighbour.
+    // 8 * pass + l / 4 of its warp's 32 rows, where that row has a neighbour.  Step `it` is slab it % k_slabs of the
+    // it / k_slabs-th offset; each group takes every other step.  A group that comes to a slot may find its
+    // "empty" barrier at most one phase behind the one it waits for (the wait tells phases apart by their parity
+    // only): its step before, it - 2, was let through when step it - 2 - S had been multiplied, and a phase behind
+    // means step it - 2 S, which came no later as long as there are two slots.
     const int sub = lane & 3, row8 = lane >> 2;
     const uint32_t warp_rows = smem_base + (uint32_t)quarter * 4096u + (uint32_t)row8 * 128u;   // row of the warp's first 8-row group
     const uint32_t piece0 = ((uint32_t)sub ^ (uint32_t)row8) << 4, piece1 = ((uint32_t)(sub + 4) ^ (uint32_t)row8) << 4;
     auto offset_of = [&](int a) { return scan ? (int)act_list[a] : a; };
     auto entry = [&](int a) { return (a < n_act && my_row >= 0) ? __ldg(table(offset_of(a)) + my_row) : -1; };
-    // with two groups each takes every other offset
-    const int first = warp >> 2;
-    int src = entry(first), nxt = entry(first + groups);
-    int slot = 0, it_no = first * p.k_slabs;
+    int a0 = 0, slab = warp >> 2;                  // offset (number in the list) and slab of this group's step
+    auto forward = [&](int &a, int &s) {
+      for (s += groups; s >= p.k_slabs; s -= p.k_slabs) ++a;
+    };
+    for (; slab >= p.k_slabs; slab -= p.k_slabs) ++a0;
+    int a1 = a0, s1 = slab;                       // the group's next step
+    forward(a1, s1);
+    int src = entry(a0), nxt = a1 == a0 ? src : entry(a1);
+    int slot = 0;
     uint32_t par = 1;                             // parity the slot's "empty" barrier has to have passed (first uses: none)
     auto skip = [&](int steps) {
       for (slot += steps; slot >= S; slot -= S) par ^= 1u;
     };
-    skip(it_no);
-    bool alive = true;
+    skip(warp >> 2);
+    const float *lane_piece = features + sub * 4;
 #pragma unroll 1
-    for (int a = first; a < n_act && alive; a += groups) {
-      const int after = entry(a + 2 * groups);
+    for (int it = warp >> 2; it < n_iter; it += groups) {
+      int a2 = a1, s2 = s1;
+      forward(a2, s2);
+      const int after = a2 == a1 ? nxt : entry(a2);
       const unsigned have = __ballot_sync(0xffffffffu, src >= 0);
       const float *ptr[4];
-      bool live[4];
+      int from[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int s = __shfl_sync(0xffffffffu, src, i * 8 + row8);
-        live[i] = s >= 0;
-        ptr[i] = features + (size_t)(s >= 0 ? s : 0) * row_words + sub * 4;
+        from[i] = __shfl_sync(0xffffffffu, src, i * 8 + row8);
+        ptr[i] = lane_piece + (size_t)(uint32_t)max(from[i], 0) * (uint32_t)row_words + slab * TC_SLAB;
       }
-      const uint4 *bsrc = packed + (size_t)offset_of(a) * p.k_slabs * (size_t)(p.n_pad * 8) + (size_t)nt0 * (size_t)(p.tile_n * 8);
-#pragma unroll 1
-      for (int slab = 0; slab < p.k_slabs; ++slab) {
-        const uint32_t full = smem_u32(full_bars + slot);
-        if (it_no >= S && !mbar_wait_warp(smem_u32(empty_bars + slot), par, abort_flag)) { alive = false; break; }
-        const uint32_t slot_off = (uint32_t)slot * (uint32_t)stage_bytes;
-        if (lane == 0) {
-          if (quarter == 0) {                     // the pre-packed filter slab of this step: one bulk copy
-            mbar_expect_tx(full, (uint32_t)p.b_bytes);
-            bulk_g2s(smem_base + slot_off + (uint32_t)TC_A_BYTES, bsrc + (size_t)slab * (size_t)(p.n_pad * 8), (uint32_t)p.b_bytes, full);
-          }
-          slot_masks[slot * 4 + quarter] = ~have;
-        }
+      const uint32_t full = smem_u32(full_bars + slot), slot_off = (uint32_t)slot * (uint32_t)stage_bytes;
+      if (it >= S && !mbar_wait_uniform(smem_u32(empty_bars + slot), par, abort_flag)) break;
+      if (quarter == 0 && elect_one()) {          // the pre-packed filter slab of this step: one bulk copy
+        mbar_expect_tx(full, (uint32_t)p.b_bytes);
+        bulk_g2s(smem_base + slot_off + (uint32_t)TC_A_BYTES,
+                 packed + ((size_t)offset_of(a0) * p.k_slabs + slab) * (size_t)(p.n_pad * 8) + (size_t)nt0 * (size_t)(p.tile_n * 8),
+                 (uint32_t)p.b_bytes, full);
+      }
+      const uint32_t dst0 = warp_rows + slot_off + piece0, dst1 = warp_rows + slot_off + piece1;
+      if ((slab + 1) * TC_SLAB <= row_words) {
+        copy_row_pieces<0>(from[0], dst0, dst1, ptr[0]);
+        copy_row_pieces<1024>(from[1], dst0, dst1, ptr[1]);
+        copy_row_pieces<2048>(from[2], dst0, dst1, ptr[2]);
+        copy_row_pieces<3072>(from[3], dst0, dst1, ptr[3]);
+      } else {                                    // pieces past the last channel are zero-filled (and read nothing)
         const int words = row_words - slab * TC_SLAB - sub * 4;   // from this lane's first piece to the row's end
-        const uint32_t dst = warp_rows + slot_off;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          if (live[i]) {                          // pieces past the last channel are zero-filled (and read nothing)
-            cp_async16_cg(dst + (uint32_t)i * 1024u + piece0, words > 0 ? ptr[i] : features, words > 0 ? 16u : 0u);
-            cp_async16_cg(dst + (uint32_t)i * 1024u + piece1, words > 16 ? ptr[i] + 16 : features, words > 16 ? 16u : 0u);
+          if (from[i] >= 0) {
+            cp_async16_cg(dst0 + (uint32_t)i * 1024u, words > 0 ? ptr[i] : features, words > 0 ? 16u : 0u);
+            cp_async16_cg(dst1 + (uint32_t)i * 1024u, words > 16 ? ptr[i] + 16 : features, words > 16 ? 16u : 0u);
           }
-          ptr[i] += TC_SLAB;
         }
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
-        if (lane == 0) mbar_arrive(full);         // (releases the row mask)
-        ++it_no;
-        skip(1);
       }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
+      store_and_arrive(lane == 0, smem_u32(slot_masks + slot * 4 + quarter), ~have, full);
+      a0 = a1;
+      slab = s1;
+      a1 = a2;
+      s1 = s2;
       src = nxt;
       nxt = after;
-      it_no += (groups - 1) * p.k_slabs;
-      skip((groups - 1) * p.k_slabs);
+      skip(groups);
     }
     cp_async_wait_all();
   } else {
@@ -875,7 +904,7 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
         for (int i = 0; i < 16; ++i)
           if (c0 + i >= c_row && c0 + i < c_out) gates[(c0 + i - c_row) * 33 + lane] = v[i];
       }
-      if (groups > 1) asm volatile("bar.sync 1, %0;" ::"r"(groups * 128) : "memory");
+      asm volatile("bar.sync 1, %0;" ::"r"(groups * 128) : "memory");
       for (int c0 = 32 * group; c0 < c_row; c0 += 32 * groups) {
         uint32_t r[32];
         load16(r, c0);
@@ -978,14 +1007,6 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   }
 }
 
-// Two producer groups where the ring is deep enough for both.  A group that comes to a slot may find its "empty"
-// barrier at most one phase behind the one it waits for (the wait tells phases apart by their parity only).
-// The group's step before is (groups - 1) * k_slabs + 1 earlier and was let through by a slot freed `stages`
-// before that, so a slot is behind by no more than that as long as k_slabs + 1 <= stages.
-static int rows_threads(const TcParams &p) {
-  return p.stages >= 4 && p.k_slabs + 1 <= p.stages ? TC_ROWS_THREADS : TC_ROWS_THREADS - 128;
-}
-
 static size_t tc_smem_bytes(const TcParams &p) {
   return (size_t)p.stages * p.sps * (TC_A_BYTES + p.b_bytes) + 1024 /*alignment slack*/ + TC_CTRL_BYTES + (size_t)p.stages * TC_LIST_BYTES;
 }
@@ -1031,7 +1052,7 @@ static bool rows_params(int words, int c_out, int n_out, TcParams &p, int opk = 
 // What the gated epilogue needs: 4 KB per producer warp, the channel constants and the gates of 128 rows, in the
 // operand slots that are free by then.
 static bool gate_fits(const TcParams &p, int c_out, int c_keep) {
-  const size_t warps = (size_t)(rows_threads(p) - 32) / 32;
+  const size_t warps = (TC_ROWS_THREADS - 32) / 32;
   return p.nt_cta == p.n_tiles &&
          warps * 4096 + (size_t)c_out * 16 + (size_t)4 * 33 * 4 * (c_out - c_keep + 1) <= (size_t)p.stages * (TC_A_BYTES + p.b_bytes);
 }
@@ -1069,7 +1090,7 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(16-bit): smem attribute: %s", cudaGetErrorString(e));
   const dim3 grid2(grid, p.n_tiles / p.nt_cta);
-  { kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate); note_launches(1); }
+  { kernel<<<grid2, TC_ROWS_THREADS, smem, st>>>((const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_fwd_16");
   return SSC_OK;
 }
@@ -1109,7 +1130,7 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
     auto kernel = gated ? conv_fwd_rows_kernel<false, true> : conv_fwd_rows_kernel<false, false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
-    kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, c_pad, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
+    kernel<<<grid2, TC_ROWS_THREADS, smem, st>>>((const float *)scratch, c_pad, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
   } else {
     auto kernel = opk > 1 ? conv_fwd_tf32_kernel<true, false, true> : conv_fwd_tf32_kernel<false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
