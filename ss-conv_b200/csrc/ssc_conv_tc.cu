@@ -33,7 +33,6 @@ constexpr int TC_SLAB = 32;            // tf32 elements per 128-byte operand row
 constexpr int TC_MAX_STAGES = 8;       // producer warps = ring slots
 constexpr int TC_EPI_WARPS = 4;        // warps 0..3 also run the epilogue (one TMEM lane quarter each)
 constexpr int TC_A_BYTES = TC_M * 128;
-constexpr int TC_ROWS_THREADS = 288;     // conv_fwd_rows_kernel: two groups of four producer warps and the issuing warp
 constexpr int TC_CTRL_BYTES = 1024;
 constexpr int TC_LIST_BYTES = TC_M * 5;   // a slot's list of present rows: 128 source rows, 128 rows of the tile
 
@@ -45,6 +44,7 @@ struct TcParams {
   int tmem_cols;  // power of two >= max(32, n_pad)
   int stages;     // operand ring depth = number of producer warps (>= 4)
   int threads;    // (max(n_prod, 4) + 1) * 32
+  int ctas;       // CTAs that share an SM
   int n_prod;     // producer warps: a multiple of the slots (several warps share a slot's rows)
   int b_bytes;    // n_pad * 128
   int sps;        // 32-channel slabs per ring slot (a step covers sps slabs of one kernel offset)
@@ -101,6 +101,7 @@ static bool tc_params(int c_in, int c_out, TcParams &p, bool split_n = false, bo
   while (ctas > 1 && ((227 * 1024) / ctas - 1024 - fixed) / stage < 2) --ctas;
   p.stages = ((227 * 1024) / ctas - 1024 - fixed) / stage;
   if (p.stages > TC_MAX_STAGES) p.stages = TC_MAX_STAGES;
+  p.ctas = ctas;
   if (p.stages < 2) return false;
   // producer warps: one per slot with four or more slots, else the slots' rows are split over four warps
   p.n_prod = p.stages < TC_EPI_WARPS ? (TC_EPI_WARPS / p.stages) * p.stages : p.stages;
@@ -588,14 +589,26 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 }
 
 // ---------------------------------------------------------------------------------------------------
-// (from >= 0) the two 16-byte pieces of a row that a lane copies, OFF bytes into its part of the slot; predicated
-// instead of branched around: a branch per row is what the copies themselves cost.
+// The two 16-byte pieces a lane copies of row `from` (none if negative) of rows `stride` bytes apart, OFF bytes into its
+// part of the slot.  Predicated instead of branched around, and addressed by one multiply-add: the
+// instructions around the copies are what the producers' time goes into.
 template <int OFF>
-__device__ __forceinline__ void copy_row_pieces(int from, uint32_t dst0, uint32_t dst1, const float *src) {
+__device__ __forceinline__ void copy_row_pieces(int from, uint32_t dst0, uint32_t dst1, const char *base, uint32_t stride) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %0, 0;\n\t"
-      "@p cp.async.cg.shared.global [%1+%4], [%3], 16;\n\t"
-      "@p cp.async.cg.shared.global [%2+%4], [%3+64], 16;\n\t}" ::"r"(from), "r"(dst0), "r"(dst1), "l"(src), "n"(OFF)
+      "{\n\t.reg .pred p;\n\t.reg .b64 a;\n\tsetp.ge.s32 p, %0, 0;\n\tmad.wide.u32 a, %0, %4, %3;\n\t"
+      "@p cp.async.cg.shared.global [%1+%5], [a], 16;\n\t"
+      "@p cp.async.cg.shared.global [%2+%5], [a+64], 16;\n\t}" ::"r"(from), "r"(dst0), "r"(dst1), "l"(base), "r"(stride), "n"(OFF)
+      : "memory");
+}
+// The same where a piece may lie past the row's end: it is zero-filled then, and its (base, stride) lead somewhere valid.
+template <int OFF>
+__device__ __forceinline__ void copy_row_ends(int from, uint32_t dst0, uint32_t dst1, const char *base0, uint32_t stride0, uint32_t bytes0,
+                                              const char *base1, uint32_t stride1, uint32_t bytes1) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ge.s32 p, %0, 0;\n\tmad.wide.u32 a, %0, %4, %3;\n\tmad.wide.u32 b, %0, %6, %5;\n\t"
+      "@p cp.async.cg.shared.global [%1+%9], [a], 16, %7;\n\t"
+      "@p cp.async.cg.shared.global [%2+%9], [b], 16, %8;\n\t}" ::"r"(from), "r"(dst0), "r"(dst1), "l"(base0), "r"(stride0),
+      "l"(base1), "r"(stride1), "r"(bytes0), "r"(bytes1), "n"(OFF)
       : "memory");
 }
 // (one lane) a word for the issuing warp and the arrival that releases it.
@@ -608,8 +621,8 @@ __device__ __forceinline__ void store_and_arrive(bool on, uint32_t at, uint32_t 
 }
 
 // The kernel for staged operands (TF32-rounded fp32 rows, or fp16 / bf16 rows: F16), one kernel offset and one
-// 128-byte slab per step.  Warps 0-3 and 4-7 are two groups of producers, each of which fills every other slot
-// (and they run the epilogue), a lane per output row of the tile; the last warp issues the MMAs.
+// 128-byte slab per step.  GROUPS of four warps produce, a lane per output row of the tile (and run the epilogue); two
+// groups fill every other slot each.  The last warp issues the MMAs.
 //
 // What bounds it is the way of an operand slot: free -> rows gathered -> multiplied -> free, against the slots that
 // fit an SM (eight of 26 KB for 64 -> 76 channels).  With a warp per slot that built its row lists, waited
@@ -627,8 +640,8 @@ __device__ __forceinline__ void store_and_arrive(bool on, uint32_t at, uint32_t 
 // GATED: batch norm and gated activation on the way out.  As a pass of its own (ssc_bn_gate_fwd) they read and write
 // every row once more: 164 us of the 12 layers of a backbone, 320 us of 24 with bf16 rows.  A row's gate
 // scalars are evaluated first, a lane per row, into shared memory; the arithmetic is that pass's, so are the bits.
-template <bool F16, bool GATED>
-__global__ void __launch_bounds__(TC_ROWS_THREADS, 4)
+template <bool F16, bool GATED, int GROUPS>
+__global__ void __launch_bounds__(GROUPS * 128 + 32, GROUPS == 1 ? 4 : 2)
 conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
                      const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out, int32_t *status, TcParams p,
                      const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order, GateEpilogue gate) {
@@ -646,7 +659,7 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int stage_bytes = TC_A_BYTES + p.b_bytes;
   const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
-  constexpr int groups = 2, mma_warp = groups * 4;                   // producer groups of four warps
+  constexpr int groups = GROUPS, mma_warp = groups * 4;              // producer groups of four warps
   const int quarter = warp & 3;                                      // the 32 rows of the tile a producer warp works on
   const int m0 = blockIdx.x * TC_M, nt0 = (int)blockIdx.y * p.nt_cta, S = p.stages;
   auto table = [&](int kap) { return nbr + (size_t)(p.rev ? K - 1 - kap : kap) * n_out; };
@@ -727,76 +740,72 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
     // ====================== producers =========================================================
     // Four lanes per row, eight rows per pass: lane l copies the 16-byte pieces l & 3 and (l & 3) + 4 of the row
     // 8 * pass + l / 4 of its warp's 32 rows, where that row has a neighbour.  Step `it` is slab it % k_slabs of the
-    // it / k_slabs-th offset; each group takes every other step.  A group that comes to a slot may find its
+    // it / k_slabs-th offset; of two groups each takes every other step.  A group that comes to a slot may find its
     // "empty" barrier at most one phase behind the one it waits for (the wait tells phases apart by their parity
     // only): its step before, it - 2, was let through when step it - 2 - S had been multiplied, and a phase behind
     // means step it - 2 S, which came no later as long as there are two slots.
-    const int sub = lane & 3, row8 = lane >> 2;
+    const int sub = lane & 3, row8 = lane >> 2, group = warp >> 2;
     const uint32_t warp_rows = smem_base + (uint32_t)quarter * 4096u + (uint32_t)row8 * 128u;   // row of the warp's first 8-row group
-    const uint32_t piece0 = ((uint32_t)sub ^ (uint32_t)row8) << 4, piece1 = ((uint32_t)(sub + 4) ^ (uint32_t)row8) << 4;
+    const uint32_t first0 = warp_rows + (((uint32_t)sub ^ (uint32_t)row8) << 4), first1 = warp_rows + (((uint32_t)(sub + 4) ^ (uint32_t)row8) << 4);
+    const uint32_t full0 = smem_u32(full_bars), empty0 = smem_u32(empty_bars), masks0 = smem_u32(slot_masks + quarter);
+    const uint32_t b_to = smem_base + (uint32_t)TC_A_BYTES, row_bytes = (uint32_t)row_words * 4u;
+    const char *lane_rows = (const char *)features + sub * 16;
+    const char *b_from = (const char *)packed + (size_t)nt0 * (size_t)(p.tile_n * 128);
+    const bool in_rows = my_row >= 0, lead = lane == 0;
+    const int32_t *my_entries = nbr + (p.rev ? (size_t)(K - 1) * n_out : 0) + max(my_row, 0);
+    const int k_slabs = p.k_slabs, offset_step = p.rev ? -n_out : n_out, last = n_act - 1;
     auto offset_of = [&](int a) { return scan ? (int)act_list[a] : a; };
-    auto entry = [&](int a) { return (a < n_act && my_row >= 0) ? __ldg(table(offset_of(a)) + my_row) : -1; };
-    int a0 = 0, slab = warp >> 2;                  // offset (number in the list) and slab of this group's step
-    auto forward = [&](int &a, int &s) {
-      for (s += groups; s >= p.k_slabs; s -= p.k_slabs) ++a;
+    auto entry = [&](int a) {                     // (past the last offset: anything, it is not used)
+      const int v = __ldg(my_entries + (long long)offset_of(min(a, last)) * offset_step);
+      return in_rows ? v : -1;
     };
-    for (; slab >= p.k_slabs; slab -= p.k_slabs) ++a0;
-    int a1 = a0, s1 = slab;                       // the group's next step
-    forward(a1, s1);
-    int src = entry(a0), nxt = a1 == a0 ? src : entry(a1);
-    int slot = 0;
+    // a group's offsets and, of each, its slabs
+    const int a_step = groups == 2 && k_slabs == 1 ? 2 : 1;
+    int src = -1, nxt = -1, a = a_step == 2 ? group : 0;
+    if (n_act > 0) { src = entry(a); nxt = entry(a + a_step); }
+    int slot = group;                             // (two slots at least)
     uint32_t par = 1;                             // parity the slot's "empty" barrier has to have passed (first uses: none)
-    auto skip = [&](int steps) {
-      for (slot += steps; slot >= S; slot -= S) par ^= 1u;
-    };
-    skip(warp >> 2);
-    const float *lane_piece = features + sub * 4;
+    bool alive = true;
 #pragma unroll 1
-    for (int it = warp >> 2; it < n_iter; it += groups) {
-      int a2 = a1, s2 = s1;
-      forward(a2, s2);
-      const int after = a2 == a1 ? nxt : entry(a2);
+    for (; a < n_act && alive; a += a_step) {
+      const int after = entry(a + 2 * a_step);
       const unsigned have = __ballot_sync(0xffffffffu, src >= 0);
-      const float *ptr[4];
       int from[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        from[i] = __shfl_sync(0xffffffffu, src, i * 8 + row8);
-        ptr[i] = lane_piece + (size_t)(uint32_t)max(from[i], 0) * (uint32_t)row_words + slab * TC_SLAB;
-      }
-      const uint32_t full = smem_u32(full_bars + slot), slot_off = (uint32_t)slot * (uint32_t)stage_bytes;
-      if (it >= S && !mbar_wait_uniform(smem_u32(empty_bars + slot), par, abort_flag)) break;
-      if (quarter == 0 && elect_one()) {          // the pre-packed filter slab of this step: one bulk copy
-        mbar_expect_tx(full, (uint32_t)p.b_bytes);
-        bulk_g2s(smem_base + slot_off + (uint32_t)TC_A_BYTES,
-                 packed + ((size_t)offset_of(a0) * p.k_slabs + slab) * (size_t)(p.n_pad * 8) + (size_t)nt0 * (size_t)(p.tile_n * 8),
-                 (uint32_t)p.b_bytes, full);
-      }
-      const uint32_t dst0 = warp_rows + slot_off + piece0, dst1 = warp_rows + slot_off + piece1;
-      if ((slab + 1) * TC_SLAB <= row_words) {
-        copy_row_pieces<0>(from[0], dst0, dst1, ptr[0]);
-        copy_row_pieces<1024>(from[1], dst0, dst1, ptr[1]);
-        copy_row_pieces<2048>(from[2], dst0, dst1, ptr[2]);
-        copy_row_pieces<3072>(from[3], dst0, dst1, ptr[3]);
-      } else {                                    // pieces past the last channel are zero-filled (and read nothing)
-        const int words = row_words - slab * TC_SLAB - sub * 4;   // from this lane's first piece to the row's end
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (from[i] >= 0) {
-            cp_async16_cg(dst0 + (uint32_t)i * 1024u, words > 0 ? ptr[i] : features, words > 0 ? 16u : 0u);
-            cp_async16_cg(dst1 + (uint32_t)i * 1024u, words > 16 ? ptr[i] + 16 : features, words > 16 ? 16u : 0u);
-          }
+      for (int i = 0; i < 4; ++i) from[i] = __shfl_sync(0xffffffffu, src, i * 8 + row8);
+      const int kappa = offset_of(a);
+#pragma unroll 1
+      for (int slab = groups == 1 || a_step == 2 ? 0 : (group ^ (a & k_slabs)) & 1; slab < k_slabs; slab += groups) {
+        const uint32_t full = full0 + (uint32_t)slot * 8u, slot_off = (uint32_t)slot * (uint32_t)stage_bytes;
+        if (a * k_slabs + slab >= S && !mbar_wait_uniform(empty0 + (uint32_t)slot * 8u, par, abort_flag)) { alive = false; break; }
+        if (quarter == 0 && elect_one()) {        // the pre-packed filter slab of this step: one bulk copy
+          mbar_expect_tx(full, (uint32_t)p.b_bytes);
+          bulk_g2s(b_to + slot_off, b_from + (size_t)(uint32_t)(kappa * k_slabs + slab) * (uint32_t)(p.n_pad * 128), (uint32_t)p.b_bytes, full);
         }
+        const uint32_t dst0 = first0 + slot_off, dst1 = first1 + slot_off;
+        const char *base = lane_rows + slab * 128;
+        if ((slab + 1) * TC_SLAB <= row_words) {
+          copy_row_pieces<0>(from[0], dst0, dst1, base, row_bytes);
+          copy_row_pieces<1024>(from[1], dst0, dst1, base, row_bytes);
+          copy_row_pieces<2048>(from[2], dst0, dst1, base, row_bytes);
+          copy_row_pieces<3072>(from[3], dst0, dst1, base, row_bytes);
+        } else {                                  // the last slab of a row that does not fill it
+          const int words = row_words - slab * TC_SLAB - sub * 4;   // from this lane's first piece to the row's end
+          const uint32_t bytes0 = words > 0 ? 16u : 0u, bytes1 = words > 16 ? 16u : 0u;
+          const char *base0 = bytes0 ? base : (const char *)features, *base1 = bytes1 ? base + 64 : (const char *)features;
+          const uint32_t stride0 = bytes0 ? row_bytes : 0u, stride1 = bytes1 ? row_bytes : 0u;
+          copy_row_ends<0>(from[0], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
+          copy_row_ends<1024>(from[1], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
+          copy_row_ends<2048>(from[2], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
+          copy_row_ends<3072>(from[3], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
+        store_and_arrive(lead, masks0 + (uint32_t)slot * 16u, ~have, full);
+        slot += groups;
+        if (slot >= S) { slot -= S; par ^= 1u; }
       }
-      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
-      store_and_arrive(lane == 0, smem_u32(slot_masks + slot * 4 + quarter), ~have, full);
-      a0 = a1;
-      slab = s1;
-      a1 = a2;
-      s1 = s2;
       src = nxt;
       nxt = after;
-      skip(groups);
     }
     cp_async_wait_all();
   } else {
@@ -1049,10 +1058,24 @@ static bool rows_params(int words, int c_out, int n_out, TcParams &p, int opk = 
   return grid * (p.n_tiles / p.nt_cta) > sms || tc_params(words, c_out, p, grid < 2 * sms, true, opk);
 }
 
+// Producer groups.  Three or four CTAs on an SM have producers enough between them, and a second group in each would leave
+// its threads 56 registers, which costs more instructions than it brings; one or two CTAs need both (64 -> 76
+// channels, four CTAs: 95 us with two groups, 88 with one; 128 -> 152 bf16 channels, two CTAs: 77 and 83).
+static int rows_groups(const TcParams &p) { return p.ctas > 2 ? 1 : 2; }
+
+using RowsKernel = void (*)(const float *, int, const uint4 *, int, int, const int32_t *, int, float *, int32_t *, TcParams, const int32_t *,
+                            const int32_t *, GateEpilogue);
+template <bool F16>
+static RowsKernel rows_kernel(const TcParams &p, bool gated) {
+  if (rows_groups(p) == 1) return gated ? conv_fwd_rows_kernel<F16, true, 1> : conv_fwd_rows_kernel<F16, false, 1>;
+  return gated ? conv_fwd_rows_kernel<F16, true, 2> : conv_fwd_rows_kernel<F16, false, 2>;
+}
+static int rows_threads(const TcParams &p) { return rows_groups(p) * 128 + 32; }
+
 // What the gated epilogue needs: 4 KB per producer warp, the channel constants and the gates of 128 rows, in the
 // operand slots that are free by then.
 static bool gate_fits(const TcParams &p, int c_out, int c_keep) {
-  const size_t warps = (TC_ROWS_THREADS - 32) / 32;
+  const size_t warps = (size_t)rows_groups(p) * 4;
   return p.nt_cta == p.n_tiles &&
          warps * 4096 + (size_t)c_out * 16 + (size_t)4 * 33 * 4 * (c_out - c_keep + 1) <= (size_t)p.stages * (TC_A_BYTES + p.b_bytes);
 }
@@ -1086,11 +1109,11 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
   const size_t smem = tc_smem_bytes(p);
   const bool gated = gate.gate_of_channel != nullptr;
   if (gated && !gate_fits(p, c_out, gate.c_keep)) return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): the gated epilogue does not cover %d -> %d channels", c_out, gate.c_keep);
-  auto kernel = gated ? conv_fwd_rows_kernel<true, true> : conv_fwd_rows_kernel<true, false>;
+  const RowsKernel kernel = rows_kernel<true>(p, gated);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(16-bit): smem attribute: %s", cudaGetErrorString(e));
   const dim3 grid2(grid, p.n_tiles / p.nt_cta);
-  { kernel<<<grid2, TC_ROWS_THREADS, smem, st>>>((const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate); note_launches(1); }
+  { kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_fwd_16");
   return SSC_OK;
 }
@@ -1127,10 +1150,10 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
   if (gated && !(rows && gate_fits(p, c_out, gate.c_keep)))
     return fail(SSC_ERR_INVALID, "conv_fwd(tf32): the gated epilogue does not cover %d -> %d channels without a staging buffer", c_out, gate.c_keep);
   if (rows) {
-    auto kernel = gated ? conv_fwd_rows_kernel<false, true> : conv_fwd_rows_kernel<false, false>;
+    const RowsKernel kernel = rows_kernel<false>(p, gated);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
-    kernel<<<grid2, TC_ROWS_THREADS, smem, st>>>((const float *)scratch, c_pad, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
+    kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, c_pad, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
   } else {
     auto kernel = opk > 1 ? conv_fwd_tf32_kernel<true, false, true> : conv_fwd_tf32_kernel<false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
