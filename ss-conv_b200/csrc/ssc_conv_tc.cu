@@ -589,15 +589,14 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 }
 
 // ---------------------------------------------------------------------------------------------------
-// The two 16-byte pieces a lane copies of row `from` (none if negative) of rows `stride` bytes apart, OFF bytes into its
-// part of the slot.  Predicated instead of branched around, and addressed by one multiply-add: the
-// instructions around the copies are what the producers' time goes into.
+// The two 16-byte pieces a lane copies of a row (none if `from` is negative), OFF bytes into its part of the slot;
+// predicated instead of branched around: the instructions around the copies are what the producers' time goes into.
 template <int OFF>
-__device__ __forceinline__ void copy_row_pieces(int from, uint32_t dst0, uint32_t dst1, const char *base, uint32_t stride) {
+__device__ __forceinline__ void copy_row_pieces(int from, uint32_t dst0, uint32_t dst1, const char *at) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 a;\n\tsetp.ge.s32 p, %0, 0;\n\tmad.wide.u32 a, %0, %4, %3;\n\t"
-      "@p cp.async.cg.shared.global [%1+%5], [a], 16;\n\t"
-      "@p cp.async.cg.shared.global [%2+%5], [a+64], 16;\n\t}" ::"r"(from), "r"(dst0), "r"(dst1), "l"(base), "r"(stride), "n"(OFF)
+      "{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %0, 0;\n\t"
+      "@p cp.async.cg.shared.global [%1+%4], [%3], 16;\n\t"
+      "@p cp.async.cg.shared.global [%2+%4], [%3+64], 16;\n\t}" ::"r"(from), "r"(dst0), "r"(dst1), "l"(at), "n"(OFF)
       : "memory");
 }
 // The same where a piece may lie past the row's end: it is zero-filled then, and its (base, stride) lead somewhere valid.
@@ -777,18 +776,20 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
 #pragma unroll 1
       for (int slab = groups == 1 || a_step == 2 ? 0 : (group ^ (a & k_slabs)) & 1; slab < k_slabs; slab += groups) {
         const uint32_t full = full0 + (uint32_t)slot * 8u, slot_off = (uint32_t)slot * (uint32_t)stage_bytes;
+        const char *base = lane_rows + slab * 128, *at[4];      // (ready before the slot is: nothing but the copies behind the wait)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) at[i] = base + (unsigned long long)(uint32_t)from[i] * row_bytes;
         if (a * k_slabs + slab >= S && !mbar_wait_uniform(empty0 + (uint32_t)slot * 8u, par, abort_flag)) { alive = false; break; }
         if (quarter == 0 && elect_one()) {        // the pre-packed filter slab of this step: one bulk copy
           mbar_expect_tx(full, (uint32_t)p.b_bytes);
           bulk_g2s(b_to + slot_off, b_from + (size_t)(uint32_t)(kappa * k_slabs + slab) * (uint32_t)(p.n_pad * 128), (uint32_t)p.b_bytes, full);
         }
         const uint32_t dst0 = first0 + slot_off, dst1 = first1 + slot_off;
-        const char *base = lane_rows + slab * 128;
         if ((slab + 1) * TC_SLAB <= row_words) {
-          copy_row_pieces<0>(from[0], dst0, dst1, base, row_bytes);
-          copy_row_pieces<1024>(from[1], dst0, dst1, base, row_bytes);
-          copy_row_pieces<2048>(from[2], dst0, dst1, base, row_bytes);
-          copy_row_pieces<3072>(from[3], dst0, dst1, base, row_bytes);
+          copy_row_pieces<0>(from[0], dst0, dst1, at[0]);
+          copy_row_pieces<1024>(from[1], dst0, dst1, at[1]);
+          copy_row_pieces<2048>(from[2], dst0, dst1, at[2]);
+          copy_row_pieces<3072>(from[3], dst0, dst1, at[3]);
         } else {                                  // the last slab of a row that does not fill it
           const int words = row_words - slab * TC_SLAB - sub * 4;   // from this lane's first piece to the row's end
           const uint32_t bytes0 = words > 0 ? 16u : 0u, bytes1 = words > 16 ? 16u : 0u;
@@ -852,8 +853,8 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
     __syncwarp();
     float4 consts[2];                             // (GATED) scale, shift, gate of the channels this thread hands round
     auto channel = [&](int ch) {
-      const bool affine = gate.scale != nullptr;
-      return make_float4(affine ? __ldg(gate.scale + ch) : 0.f, affine ? __ldg(gate.shift + ch) : 0.f,
+      const bool bn = gate.scale != nullptr;
+      return make_float4(bn ? __ldg(gate.scale + ch) : 0.f, bn ? __ldg(gate.shift + ch) : 0.f,
                          __int_as_float(ch < gate.c_keep ? __ldg(gate.gate_of_channel + ch) : -2), 0.f);
     };
     if (GATED) {
@@ -884,6 +885,7 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
       float4 *chan = (float4 *)(smem + (size_t)groups * 4u * 4096u);   // [c_out]
       // act(gate g) of row r of the quarter at g * 33 + r, and a last line of ones
       const int n_gates = c_out - c_row;
+      const bool affine = gate.scale != nullptr, whole = vec && order == nullptr && m0 + TC_M <= n_rows;
       float *gates = (float *)(chan + c_out) + quarter * 33 * (n_gates + 1);
 #pragma unroll
       for (int i = 0; i < 2; ++i)
@@ -924,8 +926,7 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
 #pragma unroll
         for (int q = 0; q < 8; ++q) *(uint4 *)(blk + lane * 32 + ((q ^ (lane & 7)) << 2)) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
         __syncwarp();
-        const int q = lane & 7, col = c0 + 4 * q;
-        if (col >= c_row) continue;
+        const int q = lane & 7, row4 = lane >> 3, col = c0 + 4 * q;
         float sc[4], sh[4];
         const float *gp[4];
         bool scalar[4];
@@ -936,40 +937,64 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
           sc[j] = k.x;
           sh[j] = k.y;
           scalar[j] = g == -1;
-          gp[j] = gates + (g >= 0 ? g : n_gates) * 33;
+          gp[j] = gates + (g >= 0 ? g : n_gates) * 33 + row4;
         }
-#pragma unroll 4
-        for (int i = 0; i < 8; ++i) {
-          const int row = 4 * i + (lane >> 3), at_row = m0 + quarter * 32 + row;
-          const float4 x = *(const float4 *)(blk + row * 32 + ((q ^ (row & 7)) << 2));
+        const bool scalars = __any_sync(0xffffffffu, scalar[0] || scalar[1] || scalar[2] || scalar[3]) && gate.scalar_act != 0;
+        if (col >= c_row) continue;
+        // rows 4 i + row4 of the warp's 32: the swizzle of even and odd i, the rest are constants
+        const float *even = blk + row4 * 32 + ((q ^ row4) << 2), *odd = blk + row4 * 32 + ((q ^ row4 ^ 4) << 2);
+        const int row0 = m0 + quarter * 32 + row4;
+        auto finished = [&](int i, bool act) {
+          const float4 x = *(const float4 *)((i & 1 ? odd : even) + i * 128);
           float v[4] = {x.x, x.y, x.z, x.w};
-          if (gate.scale) {
+          if (affine) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) v[j] = fmaf(v[j], sc[j], sh[j]);
           }
-          if (gate.scalar_act == 1) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = scalar[j] && !(v[j] > 0.f) ? 0.f : v[j];
-          } else if (gate.scalar_act != 0) {
+          if (act) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
               if (scalar[j]) v[j] = apply_act(v[j], gate.scalar_act);
           }
+          return make_float4(v[0] * gp[0][4 * i], v[1] * gp[1][4 * i], v[2] * gp[2][4 * i], v[3] * gp[3][4 * i]);
+        };
+        if (!scalars && whole && gate.out16 == 0) {          // most columns of most tiles
+          float *to = out + (size_t)row0 * c_row + col;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) v[j] *= gp[j][row];
-          if (at_row >= n_rows) continue;
-          const size_t at = (size_t)(order ? __ldg(order + at_row) : at_row) * c_row + col;
-          if (gate.out16 == 0) {
-            if (vec) {
-              *(float4 *)(out + at) = make_float4(v[0], v[1], v[2], v[3]);
+          for (int i = 0; i < 8; ++i, to += 4 * c_row) *(float4 *)to = finished(i, false);
+        } else if (!scalars && whole) {
+          uint16_t *to = (uint16_t *)out + (size_t)row0 * c_row + col;
+          if (gate.out16 == 2) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i, to += 4 * c_row) {
+              const float4 v = finished(i, false);
+              *(uint2 *)to = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i, to += 4 * c_row) {
+              const float4 v = finished(i, false);
+              *(uint2 *)to = make_uint2(pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w));
+            }
+          }
+        } else {
+#pragma unroll 2
+          for (int i = 0; i < 8; ++i) {
+            const int at_row = row0 + 4 * i;
+            const float4 v = finished(i, scalars);
+            if (at_row >= n_rows) continue;
+            const size_t at = (size_t)(order ? __ldg(order + at_row) : at_row) * c_row + col;
+            if (gate.out16 != 0) {                // c_row is a multiple of eight
+              *(uint2 *)((uint16_t *)out + at) = gate.out16 == 2 ? make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w))
+                                                                : make_uint2(pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w));
+            } else if (vec) {
+              *(float4 *)(out + at) = v;
             } else {
+              const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
               for (int j = 0; j < 4; ++j)
-                if (col + j < c_row) out[at + j] = v[j];
+                if (col + j < c_row) out[at + j] = e[j];
             }
-          } else {                                // c_row is a multiple of eight
-            *(uint2 *)((uint16_t *)out + at) = gate.out16 == 2 ? make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]))
-                                                              : make_uint2(pack_f16x2(v[0], v[1]), pack_f16x2(v[2], v[3]));
           }
         }
       }
@@ -1051,11 +1076,14 @@ __global__ void pack_filters_16_kernel(const float *__restrict__ filters, int K,
 }
 
 // The plan of a launch over n_out rows: few row tiles spread the N tiles over CTAs too, and CTAs that are alone on
-// their SM take all of its shared memory.
+// their SM take all of its shared memory.  Row tiles that fit the SMs by themselves but not with their N tiles
+// spread stay whole: a few SMs with two CTAs would make all wait for rings of half the depth (79 row tiles
+// of 256 -> 304 bf16 channels: 62 us spread).
 static bool rows_params(int words, int c_out, int n_out, TcParams &p, int opk = 1) {
   const int grid = ceil_div(n_out, TC_M), sms = sm_count();
-  if (!tc_params(words, c_out, p, grid < 2 * sms, false, opk)) return false;
-  return grid * (p.n_tiles / p.nt_cta) > sms || tc_params(words, c_out, p, grid < 2 * sms, true, opk);
+  if (!tc_params(words, c_out, p, false, grid <= sms, opk)) return false;
+  if (p.n_tiles == 1 || grid >= 2 * sms || (grid <= sms && grid * p.n_tiles > sms)) return true;
+  return tc_params(words, c_out, p, true, grid * p.n_tiles <= sms, opk);
 }
 
 // Producer groups.  Three or four CTAs on an SM have producers enough between them, and a second group in each would leave
