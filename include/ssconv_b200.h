@@ -441,6 +441,23 @@ int ssc_steer_fwd(const float *points, const float *feats, const int32_t *ids, c
                   const int32_t *chan, int n, int c, int n_sample, float *new_points, float *new_feats,
                   void *stream);
 
+/* Points outside the grid dropped from a batch whose ids ascend without gaps from 0 to n_sample - 1, as
+ * SS_Conv_lib/ss_conv/sp_ops/voxelize.py:38-84 does it with masks, two torch.unique and a sort: rows in their order,
+ * a sample that loses all its points keeps one at the origin with zero features.  The outputs have room for
+ * n_point rows; counts_dev[0] = rows written, [1] = samples left without points; flag [n_sample] = 1.0 for the
+ * others, 0.0 for these. */
+size_t ssc_p2v_keep_scratch_bytes(int n_point, int n_sample);
+int ssc_p2v_keep(const float *points, const int32_t *batch_ids, const float *feats, int n_point, int c, int n_sample,
+                 const int grid[3], const float unit[3], float *new_points, int32_t *new_ids, float *new_feats,
+                 float *flag, int32_t *counts_dev, void *scratch, size_t scratch_bytes, void *stream);
+
+/* The rows (batch id, x, y, z) ssc_three_nn takes, of voxel centres (index * unit - extent / 2 + unit / 2) and of
+ * points, and the interpolation weights (1 / (d + 1e-8), normalised) of its squared distances
+ * (SS_Conv_lib/ss_conv/sp_ops/voxelize.py:125-162). */
+int ssc_voxel_centres(const int32_t *indices, int n, const float unit[3], const float extent[3], float *rows, void *stream);
+int ssc_point_rows(const float *points, const int32_t *ids, int n, float *rows, void *stream);
+int ssc_nn_weights(const float *dist2, int n, float *weight, void *stream);
+
 /* One pass over a point batch telling the host which path Point2Voxel can take
  * (SS_Conv_lib/ss_conv/sp_ops/voxelize.py:38-84 answers the same questions with two torch.unique
  * calls, a sort and three read-backs): stats_dev[0] = points outside the grid, [1] = places where

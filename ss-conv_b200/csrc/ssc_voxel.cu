@@ -123,6 +123,16 @@ __global__ void p2v_mark_kernel(const float *__restrict__ points, const int32_t 
   atomicOr(bitmap + (flat >> 5), 1u << (flat & 31));
 }
 
+__device__ __forceinline__ bool point_inside(const float *__restrict__ p, const VoxelGrid &g) {
+  bool out = false;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int c = (int)__fdiv_rn(__fadd_rn(p[d], g.half[d]), g.unit[d]);
+    out = out || fabsf(p[d]) > g.half[d] || (unsigned)c >= (unsigned)g.grid[d];
+  }
+  return !out;
+}
+
 // What the host needs to know about a point batch before voxelizing it, in one pass:
 // stats[0] points outside the grid (|p| > half extent or cell index out of range),
 // stats[1] positions where the batch id decreases, stats[2] positions where it changes,
@@ -132,12 +142,7 @@ __global__ void p2v_stats_kernel(const float *__restrict__ points, const int32_t
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool out = false, down = false, change = false;
   if (i < n) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const float p = points[i * 3 + d];
-      const int c = (int)__fdiv_rn(__fadd_rn(p, g.half[d]), g.unit[d]);
-      out = out || fabsf(p) > g.half[d] || (unsigned)c >= (unsigned)g.grid[d];
-    }
+    out = !point_inside(points + i * 3, g);
     if (i > 0) {
       const int a = batch_ids[i - 1], b = batch_ids[i];
       down = b < a;
@@ -150,6 +155,63 @@ __global__ void p2v_stats_kernel(const float *__restrict__ points, const int32_t
     if (n_out) atomicAdd(stats + 0, n_out);
     if (n_down) atomicAdd(stats + 1, n_down);
     if (n_change) atomicAdd(stats + 2, n_change);
+  }
+}
+
+// Dropping the points outside the grid from a batch whose ids ascend without gaps from 0: a sample that loses all
+// its points keeps a single one, at the origin and with zero features, where its first point stood.
+__global__ void __launch_bounds__(256)
+p2v_kept_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, int n, VoxelGrid g, int n_sample,
+                int32_t *__restrict__ kept) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  int b = -1;
+  if (i < n && point_inside(points + (size_t)i * 3, g)) b = __ldg(batch_ids + i);
+  const unsigned same = __match_any_sync(0xffffffffu, b);
+  if ((unsigned)b < (unsigned)n_sample && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(kept + b, __popc(same));
+}
+// A bit per point: it stays, itself or as its sample's stand-in.  flag [n_sample]: 1 for samples with points left.
+__global__ void __launch_bounds__(256)
+p2v_stays_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, int n, VoxelGrid g, int n_sample,
+                 const int32_t *__restrict__ kept, uint32_t *__restrict__ bitmap, float *__restrict__ flag, int32_t *__restrict__ n_empty) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  bool stays = false, empty = false;
+  if (i < n) {
+    const int b = __ldg(batch_ids + i);
+    empty = (i == 0 || __ldg(batch_ids + i - 1) != b) && (unsigned)b < (unsigned)n_sample && __ldg(kept + b) == 0;
+    stays = empty || point_inside(points + (size_t)i * 3, g);
+  }
+  const unsigned word = __ballot_sync(0xffffffffu, stays), lost = __ballot_sync(0xffffffffu, empty);
+  if ((threadIdx.x & 31) == 0 && i < n) bitmap[i >> 5] = word;
+  if ((threadIdx.x & 31) == 0 && lost) atomicAdd(n_empty, __popc(lost));
+  if (i < n_sample) flag[i] = __ldg(kept + i) > 0 ? 1.f : 0.f;
+}
+// VEC channels per thread; HBM-bound.
+template <int VEC>
+__global__ void __launch_bounds__(256)
+p2v_gather_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, const float *__restrict__ feats, int n, int c,
+                  VoxelGrid g, const uint32_t *__restrict__ bitmap, const uint32_t *__restrict__ prefix,
+                  float *__restrict__ new_points, int32_t *__restrict__ new_ids, float *__restrict__ new_feats) {
+  const uint32_t groups = (uint32_t)(c / VEC);
+  const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (t >= (long long)n * groups) return;
+  const int i = t < 0x7fffffffll ? (int)((uint32_t)t / groups) : (int)(t / groups);
+  const int q = (int)(t - (long long)i * groups);
+  const uint32_t bits = __ldg(bitmap + (i >> 5));
+  if (!((bits >> (i & 31)) & 1u)) return;
+  const size_t to = __ldg(prefix + (i >> 5)) + (uint32_t)__popc(bits & ((1u << (i & 31)) - 1u));
+  const float *p = points + (size_t)i * 3;
+  const bool real = point_inside(p, g);
+  if (VEC == 4) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (real) v = __ldg((const float4 *)(feats + (size_t)i * c) + q);
+    ((float4 *)(new_feats + to * c))[q] = v;
+  } else {
+    new_feats[to * c + q] = real ? __ldg(feats + (size_t)i * c + q) : 0.f;
+  }
+  if (q == 0) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) new_points[to * 3 + d] = real ? p[d] : 0.f;
+    new_ids[to] = __ldg(batch_ids + i);
   }
 }
 
@@ -387,6 +449,34 @@ three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *
   }
 }
 
+// Rows (batch id, x, y, z) as three_nn takes them, and the interpolation weights from its squared distances:
+// element for element the torch expressions of Voxel2Point, a dozen launches of a few microseconds otherwise.
+__global__ void __launch_bounds__(256)
+voxel_centres_kernel(const int4 *__restrict__ indices, int n, float3 unit, float3 half_extent, float3 half_unit, float4 *__restrict__ out) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  const int4 v = __ldg(indices + i);
+  out[i] = make_float4((float)v.x, __fadd_rn(__fsub_rn(__fmul_rn((float)v.y, unit.x), half_extent.x), half_unit.x),
+                       __fadd_rn(__fsub_rn(__fmul_rn((float)v.z, unit.y), half_extent.y), half_unit.y),
+                       __fadd_rn(__fsub_rn(__fmul_rn((float)v.w, unit.z), half_extent.z), half_unit.z));
+}
+__global__ void __launch_bounds__(256)
+point_rows_kernel(const float *__restrict__ points, const int32_t *__restrict__ ids, int n, float4 *__restrict__ out) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < n) out[i] = make_float4((float)__ldg(ids + i), __ldg(points + (size_t)i * 3), __ldg(points + (size_t)i * 3 + 1), __ldg(points + (size_t)i * 3 + 2));
+}
+__global__ void __launch_bounds__(256)
+nn_weights_kernel(const float *__restrict__ dist2, int n, float *__restrict__ weight) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  float r[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) r[k] = __fdiv_rn(1.f, __fadd_rn(__fsqrt_rn(__ldg(dist2 + (size_t)i * 3 + k)), 1e-8f));
+  const float s = __fadd_rn(__fadd_rn(r[0], r[2]), r[1]);      // (the order of torch.sum)
+#pragma unroll
+  for (int k = 0; k < 3; ++k) weight[(size_t)i * 3 + k] = __fdiv_rn(r[k], s);
+}
+
 __global__ void three_interpolate_kernel(int c, int n, const float *__restrict__ points,
                                          const int32_t *__restrict__ idx, const float *__restrict__ weight,
                                          float *__restrict__ out) {
@@ -614,6 +704,72 @@ extern "C" int ssc_p2v_stats(const float *points, const int32_t *batch_ids, int 
   fill_grid(g, grid, unit);
   { p2v_stats_kernel<<<ceil_div(n_point, 256), 256, 0, st>>>(points, batch_ids, n_point, g, stats_dev); note_launches(1); }
   SSC_CHECK_LAUNCH("p2v_stats");
+  return SSC_OK;
+}
+
+extern "C" size_t ssc_p2v_keep_scratch_bytes(int n_point, int n_sample) {
+  const size_t words = (size_t)(n_point > 0 ? n_point : 1) / 32 + 1;
+  return align_up((size_t)n_sample * 4, 256) + 2 * align_up(words * 4, 256) + align_up((words / 1024 + 3) * 4, 256);
+}
+
+extern "C" int ssc_p2v_keep(const float *points, const int32_t *batch_ids, const float *feats, int n_point, int c, int n_sample,
+                            const int grid[3], const float unit[3], float *new_points, int32_t *new_ids, float *new_feats,
+                            float *flag, int32_t *counts_dev, void *scratch, size_t scratch_bytes, void *stream) {
+  SSC_REQUIRE(n_point >= 1 && c >= 1 && n_sample >= 1 && n_sample <= n_point && grid && unit, "p2v_keep: bad sizes");
+  SSC_REQUIRE(points && batch_ids && feats && new_points && new_ids && new_feats && flag && counts_dev, "p2v_keep: null pointer");
+  if (!scratch || scratch_bytes < ssc_p2v_keep_scratch_bytes(n_point, n_sample)) return fail(SSC_ERR_SCRATCH, "p2v_keep: scratch too small");
+  cudaStream_t st = as_stream(stream);
+  VoxelGrid g;
+  fill_grid(g, grid, unit);
+  const size_t words = (size_t)(n_point + 31) / 32, room = align_up(((size_t)n_point / 32 + 1) * 4, 256);
+  int32_t *kept = (int32_t *)scratch;
+  uint32_t *bitmap = (uint32_t *)((char *)scratch + align_up((size_t)n_sample * 4, 256)), *prefix = (uint32_t *)((char *)bitmap + room);
+  uint32_t *sums = (uint32_t *)((char *)prefix + room);
+  cudaMemsetAsync(kept, 0, (size_t)n_sample * 4, st);
+  cudaMemsetAsync(counts_dev, 0, 8, st);
+  const int blocks = ceil_div(n_point, 256);
+  p2v_kept_kernel<<<blocks, 256, 0, st>>>(points, batch_ids, n_point, g, n_sample, kept);
+  p2v_stays_kernel<<<blocks, 256, 0, st>>>(points, batch_ids, n_point, g, n_sample, kept, bitmap, flag, counts_dev + 1);
+  note_launches(2);
+  if (int e = exclusive_scan_u32<true>(bitmap, (long long)words, prefix, sums, counts_dev, nullptr, st)) return e;
+  if (c % 4 == 0 && (((uintptr_t)feats | (uintptr_t)new_feats) & 15u) == 0)
+    p2v_gather_kernel<4><<<ceil_div((long long)n_point * (c / 4), 256), 256, 0, st>>>(points, batch_ids, feats, n_point, c, g, bitmap, prefix, new_points, new_ids, new_feats);
+  else
+    p2v_gather_kernel<1><<<ceil_div((long long)n_point * c, 256), 256, 0, st>>>(points, batch_ids, feats, n_point, c, g, bitmap, prefix, new_points, new_ids, new_feats);
+  note_launches(1);
+  SSC_CHECK_LAUNCH("p2v_keep");
+  return SSC_OK;
+}
+
+extern "C" int ssc_voxel_centres(const int32_t *indices, int n, const float unit[3], const float extent[3], float *rows, void *stream) {
+  SSC_REQUIRE(n >= 0 && unit && extent, "voxel_centres: bad arguments");
+  if (n == 0) return SSC_OK;
+  SSC_REQUIRE(indices && rows, "voxel_centres: null pointer");
+  voxel_centres_kernel<<<ceil_div(n, 256), 256, 0, as_stream(stream)>>>((const int4 *)indices, n, make_float3(unit[0], unit[1], unit[2]),
+                                                                        make_float3(0.5f * extent[0], 0.5f * extent[1], 0.5f * extent[2]),
+                                                                        make_float3(0.5f * unit[0], 0.5f * unit[1], 0.5f * unit[2]), (float4 *)rows);
+  note_launches(1);
+  SSC_CHECK_LAUNCH("voxel_centres");
+  return SSC_OK;
+}
+
+extern "C" int ssc_point_rows(const float *points, const int32_t *ids, int n, float *rows, void *stream) {
+  SSC_REQUIRE(n >= 0, "point_rows: bad size");
+  if (n == 0) return SSC_OK;
+  SSC_REQUIRE(points && ids && rows, "point_rows: null pointer");
+  point_rows_kernel<<<ceil_div(n, 256), 256, 0, as_stream(stream)>>>(points, ids, n, (float4 *)rows);
+  note_launches(1);
+  SSC_CHECK_LAUNCH("point_rows");
+  return SSC_OK;
+}
+
+extern "C" int ssc_nn_weights(const float *dist2, int n, float *weight, void *stream) {
+  SSC_REQUIRE(n >= 0, "nn_weights: bad size");
+  if (n == 0) return SSC_OK;
+  SSC_REQUIRE(dist2 && weight, "nn_weights: null pointer");
+  nn_weights_kernel<<<ceil_div(n, 256), 256, 0, as_stream(stream)>>>(dist2, n, weight);
+  note_launches(1);
+  SSC_CHECK_LAUNCH("nn_weights");
   return SSC_OK;
 }
 

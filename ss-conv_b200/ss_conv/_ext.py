@@ -110,6 +110,12 @@ SIGNATURES = {
     "ssc_voxel2point_map": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "ssc_voxelize_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "ssc_p2v_scratch_bytes": (c_size_t, [c_int, c_int, _I3]),
+    "ssc_p2v_keep_scratch_bytes": (c_size_t, [c_int, c_int]),
+    "ssc_p2v_keep": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, _I3, _F3, c_void_p, c_void_p, c_void_p,
+                             c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
+    "ssc_voxel_centres": (c_int, [c_void_p, c_int, _F3, _F3, c_void_p, c_void_p]),
+    "ssc_point_rows": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
+    "ssc_nn_weights": (c_int, [c_void_p, c_int, c_void_p, c_void_p]),
     "ssc_p2v_count": (c_int, [c_void_p, c_void_p, c_int, c_int, _I3, _F3, c_void_p, c_void_p, c_void_p, c_size_t,
                               c_void_p]),
     "ssc_p2v_fill": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, _I3, _F3, c_int, c_int, c_void_p,
@@ -1364,6 +1370,45 @@ def p2v_stats(points, batch_ids, grid, unit):
     _check(lib().ssc_p2v_stats(_p(points, torch.float32), _p(batch_ids, torch.int32), points.shape[0], _i3(grid),
                                _F3(*[float(u) for u in unit]), _p(stats), _stream()))
     return read_counts([stats[k:k + 1] for k in range(4)])
+
+
+def p2v_keep(points, feats, batch_ids, n_sample, n_outside, grid, unit):
+    """(points, feats, ids, flag, number of samples left without points) of a batch with ids 0 .. n_sample - 1 in
+    ascending order, n_outside of whose points lie outside the grid and are dropped (ssc_p2v_keep)."""
+    n, c = feats.shape
+    cap, dev = n - int(n_outside) + int(n_sample), points.device
+    new_points = torch.empty((cap, 3), dtype=torch.float32, device=dev)
+    new_feats = torch.empty((cap, c), dtype=torch.float32, device=dev)
+    new_ids = torch.empty(cap, dtype=torch.int32, device=dev)
+    flag = torch.empty(n_sample, dtype=torch.float32, device=dev)
+    counts = torch.empty(2, dtype=torch.int32, device=dev)
+    nbytes = int(lib().ssc_p2v_keep_scratch_bytes(n, int(n_sample)))
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    _check(lib().ssc_p2v_keep(_p(points, torch.float32), _p(batch_ids, torch.int32), _p(feats, torch.float32), n, c, int(n_sample),
+                              _i3(grid), _F3(*[float(u) for u in unit]), _p(new_points), _p(new_ids), _p(new_feats), _p(flag),
+                              _p(counts), _p(scratch), nbytes, _stream()))
+    m, empty = read_counts([counts[:1], counts[1:]])
+    return new_points[:m], new_feats[:m], new_ids[:m], flag, empty
+
+
+def voxel_centres(indices, unit, extent):
+    """Rows (batch, x, y, z) of the centres of voxels `indices` [M, 4] (fp32 unit and extent)."""
+    out = torch.empty((indices.shape[0], 4), dtype=torch.float32, device=indices.device)
+    _check(lib().ssc_voxel_centres(_p(indices, torch.int32), indices.shape[0], _F3(*unit), _F3(*extent), _p(out), _stream()))
+    return out
+
+
+def point_rows(points, ids):
+    """Rows (id, x, y, z)."""
+    out = torch.empty((points.shape[0], 4), dtype=torch.float32, device=points.device)
+    _check(lib().ssc_point_rows(_p(points, torch.float32), _p(ids, torch.int32), points.shape[0], _p(out), _stream()))
+    return out
+
+
+def nn_weights(dist2):
+    out = torch.empty_like(dist2)
+    _check(lib().ssc_nn_weights(_p(dist2, torch.float32), dist2.shape[0], _p(out), _stream()))
+    return out
 
 
 def point2voxel(points, feats, batch_ids, batch_size, grid, unit, mode, ahead=False):

@@ -77,16 +77,25 @@ class Point2Voxel(nn.Module):
                 n_outside, n_down, n_change, last_id = 0, 0, self.trusted_batch_size - 1, self.trusted_batch_size - 1
             else:
                 n_outside, n_down, n_change, last_id = _ext.p2v_stats(point_cloud, ids32, grid_i, unit_f)
+            if (n_outside > 0 and n_down == 0 and last_id == n_change and feature.is_cuda and feature.dtype == torch.float32
+                    and feature.shape[0] == point_cloud.shape[0] and C > 0
+                    and not (torch.is_grad_enabled() and (feature.requires_grad or point_cloud.requires_grad))):
+                # sorted ids without gaps and points outside the grid: they are dropped by the library, after
+                # which the batch is one of the common case
+                pts, fts, ids32, flag, n_empty = _ext.p2v_keep(point_cloud, feature.contiguous(), ids32, n_change + 1, n_outside,
+                                                               grid_i, unit_f)
+                flag._ssc_any = n_empty <= n_change          # (host knowledge of flag.sum() > 0)
+                sparse = self._voxels(pts, fts, ids32, last_id + 1, grid_i, unit_f)
+                return pts, sparse, ids32 if batch_ids.dtype == torch.int32 else ids32.to(batch_ids.dtype), flag
             if n_outside == 0 and n_down == 0 and last_id >= 0:
                 B1 = n_change + 1
                 fts = feature.float().contiguous()
                 if _ext.AHEAD and not (torch.is_grad_enabled() and feature.requires_grad):
                     # the voxel count stays on the device too: buffers sized by the point count
-                    vox, _inverse, vfeat, m_dev = _ext.point2voxel(point_cloud, fts, ids32, max(last_id + 1, B1), grid_i,
-                                                                   unit_f, self.voxelization_mode, ahead=True)
-                    sparse = SparseTensor(vfeat, vox, self.voxel_num_limit.astype(np.int64), B1)
-                    sparse._rows = PendingRows(m_dev, vox.shape[0], None, None)
-                    return point_cloud, sparse, batch_ids, torch.ones(B1, dtype=torch.float32, device=device)
+                    sparse = self._voxels(point_cloud, fts, ids32, B1, grid_i, unit_f, max(last_id + 1, B1))
+                    flag = torch.ones(B1, dtype=torch.float32, device=device)
+                    flag._ssc_any = True
+                    return point_cloud, sparse, batch_ids, flag
                 vox, _inverse, vfeat = _ext.point2voxel(point_cloud, fts, ids32, max(last_id + 1, B1), grid_i, unit_f,
                                                         self.voxelization_mode)
                 if torch.is_grad_enabled() and feature.requires_grad:
@@ -130,6 +139,14 @@ class Point2Voxel(nn.Module):
         sparse = SparseTensor(vfeat, vox, self.voxel_num_limit.astype(np.int64), B1)
         return pts, sparse, ids, flag
 
+    def _voxels(self, points, feats, ids32, batch_size, grid_i, unit_f, span=None):
+        """The voxel tensor of a sorted batch inside the grid; its voxel count stays on the device where it may."""
+        made = _ext.point2voxel(points, feats, ids32, span or batch_size, grid_i, unit_f, self.voxelization_mode, ahead=_ext.AHEAD)
+        sparse = SparseTensor(made[2], made[0], self.voxel_num_limit.astype(np.int64), batch_size)
+        if _ext.AHEAD:
+            sparse._rows = PendingRows(made[3], made[0].shape[0], None, None)
+        return sparse
+
 
 class Voxel2Point(nn.Module):
     """Features at arbitrary points by inverse-distance interpolation of the three nearest
@@ -146,6 +163,13 @@ class Voxel2Point(nn.Module):
         if point_cloud is None:
             return vx_points[:, 1:].contiguous(), vx_feats, vx_points[:, 0].contiguous()
         assert batch_ids is not None
+        if (point_cloud.is_cuda and point_cloud.dtype == torch.float32 and batch_ids.dtype in (torch.int32, torch.int64)
+                and vx_feats.is_cuda and vx_feats.dtype == torch.float32):
+            rows = _ext.point_rows(point_cloud.detach().contiguous(), batch_ids.int().contiguous())
+            dist2 = torch.empty((rows.shape[0], 3), dtype=torch.float32, device=rows.device)
+            idx = torch.empty((rows.shape[0], 3), dtype=torch.int32, device=rows.device)
+            _ext.three_nn(rows.shape[0], vx_points.shape[0], rows, vx_points, dist2, idx)
+            return three_interpolate(vx_feats, idx, _ext.nn_weights(dist2))
         points = torch.cat([batch_ids.float().unsqueeze(1), point_cloud], dim=1)
         return self._get_point_feats(points, vx_points, vx_feats)
 
@@ -156,6 +180,9 @@ class Voxel2Point(nn.Module):
             unit_np, extent_np = self.voxel_extent / shape, self.voxel_extent
         else:
             unit_np, extent_np = self.unit_voxel_extent, self.unit_voxel_extent * shape
+        if feat.is_cuda and sparse_tensor.indices.shape[0] > 0:
+            return _ext.voxel_centres(sparse_tensor.indices.contiguous(), [float(v) for v in unit_np],
+                                      [float(v) for v in extent_np]), feat
         unit = torch.tensor(unit_np, dtype=torch.float32, device=feat.device)
         extent = torch.tensor(extent_np, dtype=torch.float32, device=feat.device)
         centres = sparse_tensor.indices.float()

@@ -129,7 +129,8 @@ class Feature_Steering_Module(nn.Module):
                 feats = self.v2p(feats, points, ids)
         new_points, new_feats = self.steer(points, feats, ids, r, t, s)
         valid_points, valid_feats, valid_ids, flag = self.p2v(new_points, new_feats, ids)
-        if torch.sum(flag) > 0:
+        any_left = getattr(flag, "_ssc_any", None)        # (what the voxelizer already knows on the host)
+        if torch.sum(flag) > 0 if any_left is None else any_left:
             valid_feats = self.conv1(valid_feats)
             valid_feats = self.conv2(valid_feats)
         return valid_points, valid_feats, valid_ids, flag

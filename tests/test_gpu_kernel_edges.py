@@ -159,3 +159,23 @@ def test_batch_offsets_at_the_sizes_of_the_one_block_form(cuda, n, batch):
     inside = b[(b >= 0) & (b < batch)]
     want = np.concatenate([[0], np.cumsum(np.bincount(inside, minlength=batch))])
     assert got.cpu().numpy().tolist() == want.tolist()
+
+
+@pytest.mark.parametrize("n,batch,c,far", [(1, 1, 3, 0.0), (33, 1, 4, 0.5), (700, 5, 7, 0.3), (2049, 3, 64, 0.02), (300, 40, 4, 0.8), (64, 2, 5, 1.0)])
+def test_points_outside_the_grid_are_dropped_as_the_torch_steps_do(cuda, n, batch, c, far):
+    """Samples that lose all their points (one at the origin stays), rows around a word of 32, channels that are no
+    multiple of four: exactly the mask / unique / sort form, which 16-bit ids still take."""
+    from ss_conv.sp_ops.voxelize import Point2Voxel
+    rng = np.random.RandomState(n)
+    ids = np.sort(np.concatenate([np.arange(batch), rng.randint(0, batch, n - batch if n > batch else 0)]))[:max(n, batch)]
+    pts = rng.rand(len(ids), 3).astype(np.float32) - 0.5
+    pts[rng.rand(len(ids)) < far] *= 4
+    pts[ids == batch - 1] += 3                       # one sample entirely outside
+    feats = dev(rng.randn(len(ids), c).astype(np.float32), cuda)
+    p2v = Point2Voxel([8] * 3, [0.125] * 3, 4)
+    got = p2v(dev(pts, cuda), feats, dev(ids.astype(np.int64), cuda))
+    want = p2v(dev(pts, cuda), feats, dev(ids.astype(np.int16), cuda))
+    assert got[2].dtype == torch.int64 and torch.equal(got[2], want[2].long())
+    assert torch.equal(got[0], want[0]) and torch.equal(got[3], want[3])
+    assert torch.equal(got[1].indices, want[1].indices) and torch.equal(got[1].features, want[1].features)
+    assert got[3]._ssc_any == bool(want[3].sum() > 0)
