@@ -1,4 +1,4 @@
-"""Build libssconv_b200.so (the C-ABI CUDA library) in-tree for sm_100a with nvcc.
+"""Build libssconv_b200.so (the C-ABI CUDA library, sm_100a, nvcc) and its Python bindings (g++) in-tree.
 
 Usage: python ss-conv_b200/build.py [--force] [--verbose]
 The shared library is written next to the Python package (ss_conv/libssconv_b200.so) so that
@@ -12,6 +12,7 @@ from concurrent.futures import ThreadPoolExecutor
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "ss_conv", "libssconv_b200.so")
+BINDINGS = os.path.join(HERE, "ss_conv", "_host.so")
 SOURCES = ["ssc_error.cu", "ssc_rulebook.cu", "ssc_conv.cu", "ssc_conv_tc.cu", "ssc_conv_stage.cu", "ssc_conv_pairs.cu", "ssc_backward.cu", "ssc_order.cu", "ssc_wgrad_tc.cu", "ssc_pool.cu", "ssc_layer.cu", "ssc_voxel.cu",
            "ssc_bnact.cu", "ssc_ceiling.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -25,11 +26,36 @@ def _nvcc():
 
 
 def _newest_input():
-    files = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(HERE, "..", "include", "ssconv_b200.h")]
+    files = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if not f.endswith(".cpp")] + [os.path.join(HERE, "..", "include", "ssconv_b200.h")]
     return max(os.path.getmtime(f) for f in files if os.path.exists(f))
 
 
+def build_bindings(force=False):
+    """ss_conv/_host.so: needs the headers of Python and torch, no GPU toolkit."""
+    inputs = [os.path.join(CSRC, "ssc_host.cpp"), os.path.join(HERE, "..", "include", "ssconv_b200.h")]
+    if os.path.exists(BINDINGS) and not force and os.path.getmtime(BINDINGS) >= max(os.path.getmtime(f) for f in inputs):
+        return BINDINGS
+    import sysconfig
+    import torch
+    base = os.path.join(os.path.dirname(torch.__file__), "include")
+    cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", inputs[0], "-o", BINDINGS, "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+           "-I" + base, "-I" + os.path.join(base, "torch", "csrc", "api", "include"), "-I" + sysconfig.get_paths()["include"], "-I" + cuda,
+           "-L" + os.path.dirname(LIB), "-lssconv_b200", "-Wl,-rpath,$ORIGIN",
+           "-L" + os.path.join(os.path.dirname(torch.__file__), "lib"), "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed on ssc_host.cpp:\n" + r.stderr[-6000:])
+    return BINDINGS
+
+
 def build(force=False, verbose=False):
+    lib = build_library(force, verbose)
+    build_bindings(force)
+    return lib
+
+
+def build_library(force=False, verbose=False):
     sources = [s for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
     if os.path.exists(LIB) and not force and os.path.getmtime(LIB) >= _newest_input():
         return LIB

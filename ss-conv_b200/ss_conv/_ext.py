@@ -13,6 +13,11 @@ import os
 
 import torch
 
+try:
+    from . import _host                  # the C ABI's bindings (csrc/ssc_host.cpp)
+except ImportError:
+    _host = None
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # SSCONV_B200_LIB selects another build of the same library (e.g. a debug build)
 LIB_PATH = os.environ.get("SSCONV_B200_LIB", os.path.join(_HERE, "libssconv_b200.so"))
@@ -51,8 +56,8 @@ SIGNATURES = {
                                         c_void_p, c_void_p]),
     "ssc_rulebook_conv_count": (c_int, [c_void_p, c_int, c_int, _I3, _I3, _I3, _I3, _I3, _I3, c_int, c_void_p,
                                         c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
-    "ssc_rulebook_conv_fill": (c_int, [c_void_p, c_int, c_int, _I3, _I3, _I3, _I3, _I3, _I3, c_int, c_int, c_void_p,
-                                       c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
+    "ssc_rulebook_conv_fill": (c_int, [c_void_p, c_int, c_int, _I3, _I3, _I3, _I3, _I3, _I3, c_int, c_int, c_void_p, c_void_p,
+                                       c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "ssc_pairs_to_nbr": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "ssc_pairs_from_nbr_scratch_bytes": (c_size_t, [c_int, c_int]),
     "ssc_pairs_from_nbr": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
@@ -149,12 +154,16 @@ _lib_handle = None
 
 
 def lib():
-    """The loaded C-ABI library; raises if it has not been built."""
+    """The library's functions; raises if it has not been built.  They are called through the bindings module,
+    or through ctypes when SSCONV_B200_LIB names another build of the library."""
     global _lib_handle
     if _lib_handle is None:
-        if not os.path.exists(LIB_PATH):
-            raise RuntimeError("libssconv_b200.so is missing: run `python ss-conv_b200/build.py` "
+        if not os.path.exists(LIB_PATH) or (_host is None and "SSCONV_B200_LIB" not in os.environ):
+            raise RuntimeError("libssconv_b200.so or its bindings _host.so are missing: run `python ss-conv_b200/build.py` "
                                "(there is no CPU or PyTorch fallback)")
+        if "SSCONV_B200_LIB" not in os.environ:
+            _lib_handle = _host
+            return _host
         h = ctypes.CDLL(LIB_PATH)
         for name, (res, args) in SIGNATURES.items():
             fn = getattr(h, name)
@@ -224,6 +233,14 @@ def _p(t, dtype=None):
     if not t.is_contiguous():
         raise ValueError("tensor must be contiguous")
     return t.data_ptr()  # ctypes turns the int into a void* (NULL must be passed as None)
+
+
+def _empty(shape, dtype, device):
+    return torch.empty(shape, dtype=dtype, device=device)
+
+
+if _host is not None:
+    _p, _empty = _host.ptr, _host.empty      # the same, without the interpreter
 
 
 def _stream():
@@ -320,13 +337,13 @@ def build_rulebook(indices, batch_size, out_shape, spatial_shape, ksize, stride,
             _scratch_cache.clear()
         sbytes = _scratch_cache[skey] = max(int(L.ssc_rulebook_scratch_bytes(n_in, int(batch_size), _i3(spatial_shape),
                                                                              _i3(grid), K)), 256)
-    scratch = torch.empty(sbytes, dtype=torch.uint8, device=dev)
-    small = torch.empty(K + 1, dtype=torch.int32, device=dev)   # [indice_num (K) | n_out]
+    scratch = _empty(sbytes, torch.uint8, dev)
+    small = _empty(K + 1, torch.int32, dev)   # [indice_num (K) | n_out]
     num = small[:K]
-    pairs = torch.empty((K, 2, n_in), dtype=torch.int32, device=dev) if want_pairs else None
+    pairs = _empty((K, 2, n_in), torch.int32, dev) if want_pairs else None
     st = status_word(dev)
     if subm:
-        nbr = torch.empty((K, n_in), dtype=torch.int32, device=dev)
+        nbr = _empty((K, n_in), torch.int32, dev)
         _check(L.ssc_rulebook_subm(_p(indices), n_in, int(batch_size), _i3(spatial_shape), _i3(ksize), _i3(dilation),
                                    _p(nbr), _p(pairs), _p(num), _p(st), _p(scratch), scratch.numel(), _stream()))
         nbr._ssc_symmetric = all(int(k) == 1 or (int(k) % 2 == 1 and int(d) == 1) for k, d in zip(ksize, dilation))
@@ -336,8 +353,8 @@ def build_rulebook(indices, batch_size, out_shape, spatial_shape, ksize, stride,
     _check(L.ssc_rulebook_conv_count(_p(indices), n_in, int(batch_size), *geo, _p(n_out_dev), _p(st), _p(scratch),
                                      scratch.numel(), None, _stream()))
     n_out = read_count(n_out_dev)  # the one host sync of a regular rulebook (the status word comes with it)
-    outids = torch.empty((n_out, 4), dtype=torch.int32, device=dev)
-    nbr = torch.empty((K, n_out), dtype=torch.int32, device=dev)
+    outids = _empty((n_out, 4), torch.int32, dev)
+    nbr = _empty((K, n_out), torch.int32, dev)
     _check(L.ssc_rulebook_conv_fill(_p(indices), n_in, int(batch_size), *geo, n_out, _p(outids), _p(nbr), _p(pairs),
                                     _p(num), _p(st), _p(scratch), scratch.numel(), None, _stream()))
     _note_ratio(_geometry_key(spatial_shape, ksize, stride, padding, dilation, transpose), n_in, n_out)
@@ -404,14 +421,14 @@ def get_indice_pairs_ahead(indices, batch_size, out_shape, spatial_shape, ksize,
             _scratch_cache.clear()
         sbytes = _scratch_cache[skey] = max(int(L.ssc_rulebook_scratch_bytes(n_in, int(batch_size), _i3(spatial_shape),
                                                                              _i3(out_shape), K)), 256)
-    scratch = torch.empty(sbytes, dtype=torch.uint8, device=dev)
-    n_out_dev = torch.empty(1, dtype=torch.int32, device=dev)
+    scratch = _empty(sbytes, torch.uint8, dev)
+    n_out_dev = _empty(1, torch.int32, dev)
     st = status_word(dev)
     geo = (_i3(spatial_shape), _i3(out_shape), _i3(ksize), _i3(stride), _i3(padding), _i3(dilation), int(transpose))
     _check(L.ssc_rulebook_conv_count(_p(indices), n_in, int(batch_size), *geo, _p(n_out_dev), _p(st), _p(scratch),
                                      sbytes, _p(n_in_dev), _stream()))
-    outids = torch.empty((cap, 4), dtype=torch.int32, device=dev)
-    nbr = torch.empty((K, cap), dtype=torch.int32, device=dev)
+    outids = _empty((cap, 4), torch.int32, dev)
+    nbr = _empty((K, cap), torch.int32, dev)
     # the per-offset pair counts (indice_num) are not needed by the kernels that consume the table:
     # they are computed only if somebody turns the handle into reference-format pair lists
     _check(L.ssc_rulebook_conv_fill(_p(indices), n_in, int(batch_size), *geo, cap, _p(outids), _p(nbr), None, None,
@@ -479,13 +496,13 @@ def layer_ahead(plan, indices, n_in_dev, features, weight=None, gate=None):
             if gate[0] is not None:
                 a.scale, a.shift = _p(gate[0]), _p(gate[1])
             a.gate_of_channel = _p(gate[2])
-    outids = torch.empty((cap, 4), dtype=torch.int32, device=dev)
-    n_out_dev = torch.empty(1, dtype=torch.int32, device=dev)
-    out = torch.empty((cap, c_row), dtype=dtype, device=dev)
+    outids = _empty((cap, 4), torch.int32, dev)
+    n_out_dev = _empty(1, torch.int32, dev)
+    out = _empty((cap, c_row), dtype, dev)
     L = lib()
     at = ctypes.addressof(a)
     nbytes = L.ssc_layer_ahead_bytes(at)
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    ws = _empty(nbytes, torch.uint8, dev)
     a.out_indices, a.n_out_dev, a.out = outids.data_ptr(), n_out_dev.data_ptr(), out.data_ptr()
     a.workspace, a.workspace_bytes, a.status, a.stream = ws.data_ptr(), nbytes, status_word(dev).data_ptr(), _stream()
     _check(L.ssc_layer_ahead(at))
@@ -510,8 +527,8 @@ def get_indice_pairs_subm_ahead(indices_cap, batch_size, spatial_shape, ksize, d
     if sbytes is None:
         sbytes = _scratch_cache[skey] = max(int(L.ssc_rulebook_scratch_bytes(cap, int(batch_size), _i3(spatial_shape),
                                                                              _i3(spatial_shape), K)), 256)
-    scratch = torch.empty(sbytes, dtype=torch.uint8, device=dev)
-    nbr = torch.empty((K, cap), dtype=torch.int32, device=dev)
+    scratch = _empty(sbytes, torch.uint8, dev)
+    nbr = _empty((K, cap), torch.int32, dev)
     _check(L.ssc_rulebook_subm_ahead(_p(indices_cap, torch.int32), cap, int(batch_size), _i3(spatial_shape), _i3(ksize),
                                      _i3(dilation), _p(nbr), _p(status_word(dev)), _p(scratch), sbytes, _p(n_in_dev),
                                      _stream()))
@@ -619,10 +636,10 @@ class LazyPairs(object):
         if self._tensor is None:
             nbr = self._ssc_nbr
             K, n_out = nbr.shape
-            pairs = torch.empty((K, 2, self._n_in), dtype=torch.int32, device=nbr.device)
-            num = torch.empty(K, dtype=torch.int32, device=nbr.device)
+            pairs = _empty((K, 2, self._n_in), torch.int32, nbr.device)
+            num = _empty(K, torch.int32, nbr.device)
             nbytes = int(lib().ssc_pairs_from_nbr_scratch_bytes(K, n_out))
-            scratch = torch.empty(nbytes, dtype=torch.uint8, device=nbr.device)
+            scratch = _empty(nbytes, torch.uint8, nbr.device)
             _check(lib().ssc_pairs_from_nbr(_p(nbr), K, n_out, self._n_in, _p(pairs), _p(num), _p(scratch), nbytes,
                                             _stream()))
             pairs._ssc_nbr = nbr
@@ -666,7 +683,7 @@ def neighbour_table(pairs, num, n_out, inverse=False):
         return cached
     pairs = pairs.contiguous()
     K, _, n_cols = pairs.shape
-    nbr = torch.empty((K, n_out), dtype=torch.int32, device=pairs.device)
+    nbr = _empty((K, n_out), torch.int32, pairs.device)
     _check(lib().ssc_pairs_to_nbr(_p(pairs, torch.int32), _p(num.to(pairs.device), torch.int32), K, n_cols, int(n_out),
                                   int(bool(inverse)), _p(nbr), _stream()))
     try:
@@ -678,7 +695,7 @@ def neighbour_table(pairs, num, n_out, inverse=False):
 
 # ============================================================== materialisation and conv
 def materialize(weight, basis, block_table, n_blocks_in, out_field, in_field, c_out, c_in, K):
-    flt = torch.empty((K, c_in, c_out), dtype=torch.float32, device=weight.device)
+    flt = _empty((K, c_in, c_out), torch.float32, weight.device)
     _check(lib().ssc_materialize(_p(weight, torch.float32), _p(basis, torch.float32), _p(block_table, torch.int32),
                                  int(n_blocks_in), _p(out_field, torch.int32), _p(in_field, torch.int32), int(c_out),
                                  int(c_in), int(K), _p(flt), _stream()))
@@ -687,7 +704,7 @@ def materialize(weight, basis, block_table, n_blocks_in, out_field, in_field, c_
 
 def materialize_backward(d_filters, basis, block_table, n_blocks_in, out_field, in_field, out_start, in_start, max_pair, c_out,
                          c_in, K, n_weight):
-    d_w = torch.empty(n_weight, dtype=torch.float32, device=d_filters.device)
+    d_w = _empty(n_weight, torch.float32, d_filters.device)
     _check(lib().ssc_materialize_bwd(_p(d_filters, torch.float32), _p(basis, torch.float32), _p(block_table, torch.int32),
                                      int(n_blocks_in), _p(out_field, torch.int32), _p(in_field, torch.int32),
                                      _p(out_start, torch.int32), out_start.numel(), _p(in_start, torch.int32),
@@ -701,7 +718,7 @@ def pack_filters(filters_kio, prec=PREC_TF32):
     nbytes = lib().ssc_conv_packed_bytes(K, c_in, c_out, prec)
     if nbytes == 0:
         raise ValueError("channel count not supported by the tensor-core path")
-    packed = torch.empty(int(nbytes), dtype=torch.uint8, device=filters_kio.device)
+    packed = _empty(int(nbytes), torch.uint8, filters_kio.device)
     _check(lib().ssc_conv_pack_filters(_p(filters_kio, torch.float32), K, c_in, c_out, prec, _p(packed), _stream()))
     return packed
 
@@ -756,7 +773,7 @@ def pair_lists(nbr):
         return kept
     K, n_out = nbr.shape
     nbytes = int(lib().ssc_conv_pairs_list_bytes(K, n_out))
-    lists = torch.empty(nbytes, dtype=torch.uint8, device=nbr.device)
+    lists = _empty(nbytes, torch.uint8, nbr.device)
     _check(lib().ssc_conv_pairs_build(_p(nbr, torch.int32), K, n_out, _p(lists), nbytes, _stream()))
     if not torch.cuda.is_current_stream_capturing():
         try:
@@ -827,7 +844,7 @@ def conv_prepare(features, filters, precision=None):
     prec = _PREC_OF[mode]
     packed = pack_filters(flt, prec)
     nbytes = int(lib().ssc_conv_scratch_bytes(features.shape[0], c_in, c_out, prec))
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=features.device)
+    scratch = _empty(nbytes, torch.uint8, features.device)
     _check(lib().ssc_conv_stage(_p(features, torch.float32), features.shape[0], c_in, prec, _p(scratch), nbytes, _stream()))
     _prepared[(features.data_ptr(), flt.data_ptr())] = (prec, packed, scratch, nbytes)
     return True
@@ -861,7 +878,7 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
         mode = "fp32"
     if (mode in _PREC_OF and n_out_dev is None and row_order is None and nbr.shape[1] == n_out and not reversed_table
             and _use_pairs(K, c_in, c_out, n_out, _PREC_OF[mode], algo)):
-        out = torch.empty((n_out, c_out), dtype=torch.float32, device=features.device)
+        out = _empty((n_out, c_out), torch.float32, features.device)
         return _gated(_conv_forward_pairs(features, filters, nbr, n_out, _PREC_OF[mode], out, st), gate)
     flag = TABLE_IN_ORDER if (table_in_order and row_order is not None) else 0
     if flag and mode not in _PREC_OF:
@@ -878,10 +895,10 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
     if gate is not None and not flag and _gate_covered(c_in, c_out, gate[3], prec, n_out):
         if ready is None or ready[0] != prec:
             nbytes = lib().ssc_conv_scratch_bytes(features.shape[0], c_in, c_out, prec)
-            ready = (0, _packed_filters(filters, prec), torch.empty(nbytes, dtype=torch.uint8, device=features.device), nbytes)
+            ready = (0, _packed_filters(filters, prec), _empty(nbytes, torch.uint8, features.device), nbytes)
         return _conv_gated(_p(features, torch.float32), features.shape[0], c_in, ready[1], K, c_out, nbr, n_out,
                            prec | (PRESTAGED if ready[0] else 0), gate, st, _p(ready[2]), ready[3], n_out_dev, row_order)
-    out = torch.empty((n_out, c_out), dtype=torch.float32, device=features.device)
+    out = _empty((n_out, c_out), torch.float32, features.device)
     if ready is not None and ready[0] == prec:
         prec, packed, scratch, nbytes = ready
         _check(lib().ssc_conv_fwd_ordered(_p(features, torch.float32), features.shape[0], c_in, _p(packed), K, c_out,
@@ -893,7 +910,7 @@ def conv_forward(features, filters, nbr, n_out, precision=None, n_out_dev=None, 
         # (the 16-bit kernels and layers with up to 16 input channels know the staged form only)
         stage = prec != PREC_TF32 or n_out >= STAGING_MIN_ROWS or c_in <= 16
         nbytes = lib().ssc_conv_scratch_bytes(features.shape[0], c_in, c_out, prec) if stage else 0
-        scratch = torch.empty(nbytes, dtype=torch.uint8, device=features.device) if nbytes else None
+        scratch = _empty(nbytes, torch.uint8, features.device) if nbytes else None
         _check(lib().ssc_conv_fwd_ordered(_p(features, torch.float32), features.shape[0], c_in, _p(packed), K, c_out,
                                           _p(nbr, torch.int32), int(n_out), prec | flag, _p(out), _p(st), _p(scratch), nbytes,
                                           _p(n_out_dev), _p(row_order), _stream()))
@@ -919,7 +936,7 @@ def _gate_covered(c_in, c_out, c_keep, prec, n_out):
 def _conv_gated(features, n_in, c_in, packed, K, c_out, nbr, n_out, prec, gate, st, scratch, nbytes, n_out_dev, row_order=None):
     scale, shift, table, c_keep, scalar_act, gate_act = gate
     stored = _stored_type(n_out, c_out, c_keep, c_keep)
-    out = torch.empty((n_out, c_keep), dtype=stored or torch.float32, device=nbr.device)
+    out = _empty((n_out, c_keep), stored or torch.float32, nbr.device)
     _check(lib().ssc_conv_fwd_gated(features, n_in, c_in, _p(packed), K, c_out, _p(nbr, torch.int32), int(n_out), prec,
                                     _p(scale), _p(shift), _p(table), c_keep, scalar_act, gate_act,
                                     _PREC_OF[_storage] if stored else PREC_FP32, _p(out), _p(st), scratch, nbytes,
@@ -962,7 +979,7 @@ def _conv_forward_stored16(features, filters, nbr, n_out, n_out_dev, algo, gate=
     if gate is not None and not pairs and _gate_covered(c_in, c_out, gate[3], prec, n_out):
         return _conv_gated(None, features.shape[0], c_in, packed, K, c_out, nbr, n_out, prec | PRESTAGED, gate, st,
                            _p(features), nbytes, n_out_dev)
-    out = torch.empty((n_out, c_out), dtype=torch.float32, device=features.device)
+    out = _empty((n_out, c_out), torch.float32, features.device)
     if pairs:
         lists = pair_lists(nbr)
         _check(lib().ssc_conv_fwd_pairs(None, features.shape[0], c_in, _p(packed), K, c_out, _p(lists), lists.numel(),
@@ -988,7 +1005,7 @@ def _conv_forward_pairs(features, filters, nbr, n_out, prec, out, st):
     else:
         packed = _packed_filters(filters, prec)
         nbytes = int(lib().ssc_conv_scratch_bytes(features.shape[0], c_in, c_out, prec))
-        scratch = torch.empty(nbytes, dtype=torch.uint8, device=features.device)
+        scratch = _empty(nbytes, torch.uint8, features.device)
     lists = pair_lists(nbr)
     _check(lib().ssc_conv_fwd_pairs(_p(features, torch.float32), features.shape[0], c_in, _p(packed), K, c_out, _p(lists),
                                     lists.numel(), int(n_out), prec | flag, _p(out), _p(st), _p(scratch), nbytes, _stream()))
@@ -1034,7 +1051,7 @@ def _not_built(name):
 def input_major_table(nbr, n_in):
     """nbr_in [K, n_in]: for every (offset, input row) the output row it contributes to, or -1."""
     K, n_out = nbr.shape
-    nbr_in = torch.empty((K, int(n_in)), dtype=torch.int32, device=nbr.device)
+    nbr_in = _empty((K, int(n_in)), torch.int32, nbr.device)
     _check(lib().ssc_nbr_transpose(_p(nbr, torch.int32), K, n_out, int(n_in), _p(nbr_in), _stream()))
     return nbr_in
 
@@ -1057,9 +1074,9 @@ def nbr_row_order_planes(nbr, ksize, n_rows_dev=None, with_table=False):
     nbytes = int(lib().ssc_nbr_row_order_planes_scratch_bytes(_i3(ks), n))
     if nbytes == 0:
         return None
-    order = torch.empty(n, dtype=torch.int32, device=nbr.device)
+    order = _empty(n, torch.int32, nbr.device)
     moved = torch.empty_like(nbr) if with_table else None
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=nbr.device)
+    scratch = _empty(nbytes, torch.uint8, nbr.device)
     _check(lib().ssc_nbr_row_order_planes(_p(nbr, torch.int32), _i3(ks), n, _p(order), _p(moved), _p(scratch), nbytes,
                                           _p(n_rows_dev), _stream()))
     return (order, moved) if with_table else order
@@ -1072,8 +1089,8 @@ def nbr_row_order(nbr):
     nbytes = int(lib().ssc_nbr_row_order_scratch_bytes(K, n))
     if nbytes == 0 or n == 0:
         return None
-    order = torch.empty(n, dtype=torch.int32, device=nbr.device)
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=nbr.device)
+    order = _empty(n, torch.int32, nbr.device)
+    scratch = _empty(nbytes, torch.uint8, nbr.device)
     _check(lib().ssc_nbr_row_order(_p(nbr, torch.int32), K, n, _p(order), _p(scratch), nbytes, _stream()))
     return order
 
@@ -1082,7 +1099,7 @@ def stage_tf32(rows):
     """The TF32 operand image of fp32 rows [n, C] (ssc_conv_stage): a flat byte buffer."""
     n, c = rows.shape
     nbytes = int(lib().ssc_conv_scratch_bytes(n, c, c, PREC_TF32))
-    image = torch.empty(nbytes, dtype=torch.uint8, device=rows.device)
+    image = _empty(nbytes, torch.uint8, rows.device)
     _check(lib().ssc_conv_stage(_p(rows, torch.float32), n, c, PREC_TF32, _p(image), nbytes, _stream()))
     return image
 
@@ -1095,9 +1112,9 @@ def conv_wgrad(features, out_grad, nbr, precision=None, x_image=None, dy_image=N
     c_in, c_out = features.shape[1], out_grad.shape[1]
     # the filter gradient has no 16-bit form: 'fp16' / 'bf16' take the TF32 kernel
     mode = PREC_TF32 if _resolve_precision(c_in, c_out, precision) in _PREC_OF else PREC_FP32
-    d_flt = torch.empty((K, c_in, c_out), dtype=torch.float32, device=features.device)
+    d_flt = _empty((K, c_in, c_out), torch.float32, features.device)
     nbytes = int(lib().ssc_conv_wgrad_scratch_bytes(K, c_in, c_out, n_out))
-    scratch = torch.empty(max(nbytes, 4), dtype=torch.uint8, device=features.device)
+    scratch = _empty(max(nbytes, 4), torch.uint8, features.device)
     lists = pair_lists(nbr) if n_out > 0 and (mode == PREC_TF32 or c_in <= 16) else None
     x, dy = _p(features, torch.float32), _p(out_grad, torch.float32)
     if mode == PREC_TF32 and c_in <= 256:
@@ -1212,7 +1229,7 @@ def indice_conv_backward_half(features, filters, out_bp, indice_pairs, indice_nu
 def _pool(features, indice_pairs, indice_num, num_act, average, summaryrf=None):
     features = features.contiguous()
     nbr, n_out_dev = _table_for(indice_pairs, indice_num, int(num_act))
-    out = torch.empty((int(num_act), features.shape[1]), dtype=torch.float32, device=features.device)
+    out = _empty((int(num_act), features.shape[1]), torch.float32, features.device)
     rf = None if summaryrf is None else summaryrf.to(torch.int32).contiguous()
     c, K = features.shape[1], nbr.shape[0]
     if features.dtype in _PREC_OF_DTYPE:     # rows stored in 16 bits by a gated Activation
@@ -1237,7 +1254,7 @@ def indice_avgpool_fp32(features, indice_pairs, indice_num, num_act, summaryrf):
 
 def indiceSummaryRF(indice_pairs, indice_num, num_act):
     nbr = neighbour_table(indice_pairs, indice_num, int(num_act))
-    rf = torch.empty(int(num_act), dtype=torch.int32, device=nbr.device)
+    rf = _empty(int(num_act), torch.int32, nbr.device)
     _check(lib().ssc_summary_rf(_p(nbr), nbr.shape[0], int(num_act), _p(rf), _stream()))
     return rf
 
@@ -1314,7 +1331,7 @@ def global_maxpool_bp(d_feats, offsets, maxidx, d_out, n_proposal, c):
 def batch_offsets(indices, batch_size, n_dev=None):
     """Row offsets [B+1] (int32, on device) of the samples of an indices tensor, no host sync.
     n_dev: device word with the exact row count when the tensor's length is only a capacity."""
-    off = torch.empty(int(batch_size) + 1, dtype=torch.int32, device=indices.device)
+    off = _empty(int(batch_size) + 1, torch.int32, indices.device)
     _check(lib().ssc_batch_offsets(_p(indices.contiguous(), torch.int32), indices.shape[0], int(batch_size), _p(off),
                                    _p(n_dev), _stream()))
     return off
@@ -1345,7 +1362,7 @@ def steer_matrices(rot, dirs, pinv, orders, reference_frame):
     """[B, sum (2l+1)^2] representation matrices of rotations [B, 3, 3] (ssc_steer_matrices); dirs / pinv: the
     float64 tables of SO3.sample_tables on the same device."""
     rot = rot.float().contiguous()
-    out = torch.empty((rot.shape[0], sum((2 * l + 1) ** 2 for l in range(orders))), dtype=torch.float32, device=rot.device)
+    out = _empty((rot.shape[0], sum((2 * l + 1) ** 2 for l in range(orders))), torch.float32, rot.device)
     _check(lib().ssc_steer_matrices(_p(rot), rot.shape[0], int(orders), _p(dirs, torch.float64), _p(pinv, torch.float64),
                                     int(bool(reference_frame)), _p(out), _stream()))
     return out
@@ -1354,8 +1371,8 @@ def steer_matrices(rot, dirs, pinv, orders, reference_frame):
 def steer(points, feats, ids, rot, trans, scale, dmats, chan):
     """(new_points [N,3], new_feats [N,C]) of the feature-steering change of frame (one launch)."""
     n, c = feats.shape
-    new_points = torch.empty((n, 3), dtype=torch.float32, device=feats.device)
-    new_feats = torch.empty((n, c), dtype=torch.float32, device=feats.device)
+    new_points = _empty((n, 3), torch.float32, feats.device)
+    new_feats = _empty((n, c), torch.float32, feats.device)
     _check(lib().ssc_steer_fwd(_p(points, torch.float32), _p(feats, torch.float32), _p(ids, torch.int32),
                                _p(rot, torch.float32), _p(trans, torch.float32), _p(scale), _p(dmats, torch.float32),
                                dmats.shape[1], _p(chan, torch.int32), n, c, rot.shape[0], _p(new_points), _p(new_feats),
@@ -1366,7 +1383,7 @@ def steer(points, feats, ids, rot, trans, scale, dmats, chan):
 def p2v_stats(points, batch_ids, grid, unit):
     """[n outside the grid, n places where batch_ids decreases, n places where it changes, last id]
     of a point batch (one kernel, one read-back)."""
-    stats = torch.empty(4, dtype=torch.int32, device=points.device)
+    stats = _empty(4, torch.int32, points.device)
     _check(lib().ssc_p2v_stats(_p(points, torch.float32), _p(batch_ids, torch.int32), points.shape[0], _i3(grid),
                                _F3(*[float(u) for u in unit]), _p(stats), _stream()))
     return read_counts([stats[k:k + 1] for k in range(4)])
@@ -1377,13 +1394,13 @@ def p2v_keep(points, feats, batch_ids, n_sample, n_outside, grid, unit):
     ascending order, n_outside of whose points lie outside the grid and are dropped (ssc_p2v_keep)."""
     n, c = feats.shape
     cap, dev = n - int(n_outside) + int(n_sample), points.device
-    new_points = torch.empty((cap, 3), dtype=torch.float32, device=dev)
-    new_feats = torch.empty((cap, c), dtype=torch.float32, device=dev)
-    new_ids = torch.empty(cap, dtype=torch.int32, device=dev)
-    flag = torch.empty(n_sample, dtype=torch.float32, device=dev)
-    counts = torch.empty(2, dtype=torch.int32, device=dev)
+    new_points = _empty((cap, 3), torch.float32, dev)
+    new_feats = _empty((cap, c), torch.float32, dev)
+    new_ids = _empty(cap, torch.int32, dev)
+    flag = _empty(n_sample, torch.float32, dev)
+    counts = _empty(2, torch.int32, dev)
     nbytes = int(lib().ssc_p2v_keep_scratch_bytes(n, int(n_sample)))
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    scratch = _empty(nbytes, torch.uint8, dev)
     _check(lib().ssc_p2v_keep(_p(points, torch.float32), _p(batch_ids, torch.int32), _p(feats, torch.float32), n, c, int(n_sample),
                               _i3(grid), _F3(*[float(u) for u in unit]), _p(new_points), _p(new_ids), _p(new_feats), _p(flag),
                               _p(counts), _p(scratch), nbytes, _stream()))
@@ -1393,14 +1410,14 @@ def p2v_keep(points, feats, batch_ids, n_sample, n_outside, grid, unit):
 
 def voxel_centres(indices, unit, extent):
     """Rows (batch, x, y, z) of the centres of voxels `indices` [M, 4] (fp32 unit and extent)."""
-    out = torch.empty((indices.shape[0], 4), dtype=torch.float32, device=indices.device)
+    out = _empty((indices.shape[0], 4), torch.float32, indices.device)
     _check(lib().ssc_voxel_centres(_p(indices, torch.int32), indices.shape[0], _F3(*unit), _F3(*extent), _p(out), _stream()))
     return out
 
 
 def point_rows(points, ids):
     """Rows (id, x, y, z)."""
-    out = torch.empty((points.shape[0], 4), dtype=torch.float32, device=points.device)
+    out = _empty((points.shape[0], 4), torch.float32, points.device)
     _check(lib().ssc_point_rows(_p(points, torch.float32), _p(ids, torch.int32), points.shape[0], _p(out), _stream()))
     return out
 
@@ -1423,16 +1440,16 @@ def point2voxel(points, feats, batch_ids, batch_size, grid, unit, mode, ahead=Fa
     batch_ids = batch_ids.contiguous().to(torch.int32)
     n = points.shape[0]
     sbytes = L.ssc_p2v_scratch_bytes(n, int(batch_size), _i3(grid))
-    scratch = torch.empty(max(int(sbytes), 256), dtype=torch.uint8, device=dev)
-    m_dev = torch.empty(1, dtype=torch.int32, device=dev)
+    scratch = _empty(max(int(sbytes), 256), torch.uint8, dev)
+    m_dev = _empty(1, torch.int32, dev)
     st = status_word(dev)
     unit3 = _F3(*[float(u) for u in unit])
     _check(L.ssc_p2v_count(_p(points), _p(batch_ids), n, int(batch_size), _i3(grid), unit3, _p(m_dev), _p(st),
                            _p(scratch), scratch.numel(), _stream()))
     m = n if ahead else read_count(m_dev)
-    vox = torch.empty((m, 4), dtype=torch.int32, device=dev)
-    inverse = torch.empty(n, dtype=torch.int32, device=dev)
-    vfeat = torch.empty((m, feats.shape[1]), dtype=torch.float32, device=dev)
+    vox = _empty((m, 4), torch.int32, dev)
+    inverse = _empty(n, torch.int32, dev)
+    vfeat = _empty((m, feats.shape[1]), torch.float32, dev)
     _check(L.ssc_p2v_fill(_p(points), _p(batch_ids), _p(feats), n, feats.shape[1], int(batch_size), _i3(grid), unit3,
                           int(mode), m, _p(vox), _p(inverse), _p(vfeat), _p(scratch), scratch.numel(), _stream()))
     if ahead:
@@ -1443,7 +1460,7 @@ def point2voxel(points, feats, batch_ids, batch_size, grid, unit, mode, ahead=Fa
 def three_nn(n, m, unknown, known, dist2, idx):
     L = lib()
     sbytes = max(int(L.ssc_three_nn_scratch_bytes(int(m))), 256)
-    scratch = torch.empty(sbytes, dtype=torch.uint8, device=unknown.device)
+    scratch = _empty(sbytes, torch.uint8, unknown.device)
     _check(L.ssc_three_nn(int(n), int(m), _p(unknown, torch.float32), _p(known, torch.float32),
                           _p(dist2, torch.float32), _p(idx, torch.int32), _p(scratch), scratch.numel(), _stream()))
 
@@ -1462,7 +1479,7 @@ def three_interpolate_bp(c, n, m, grad_out, idx, weight, grad_points):
 # ================================================================ BatchNorm / activation
 def bn_fold(running_mean, running_var, weight, bias, field_of_channel, scalar_of_channel, eps):
     c = field_of_channel.numel()
-    scale = torch.empty(c, dtype=torch.float32, device=running_var.device)
+    scale = _empty(c, torch.float32, running_var.device)
     shift = torch.empty_like(scale)
     _check(lib().ssc_bn_fold(_p(running_mean), _p(running_var), _p(weight), _p(bias), _p(field_of_channel, torch.int32),
                              _p(scalar_of_channel, torch.int32), c, float(eps), _p(scale), _p(shift), _stream()))
@@ -1476,12 +1493,12 @@ def bn_gate_forward(x, scale, shift, gate_of_channel, c_out, c_gate_base, scalar
     x = x.contiguous()
     stored = _stored_type(x.shape[0], x.shape[1], int(c_out), int(c_gate_base), storage)
     if stored:
-        out = torch.empty((x.shape[0], int(c_out)), dtype=stored, device=x.device)
+        out = _empty((x.shape[0], int(c_out)), stored, x.device)
         _check(lib().ssc_bn_gate_fwd16(_p(x, torch.float32), x.shape[0], x.shape[1], _p(scale), _p(shift),
                                        _p(gate_of_channel), int(c_out), int(c_gate_base), int(scalar_act), int(gate_act),
                                        _p(scalar_bias), _p(gate_bias), _PREC_OF[storage], _p(out), _stream()))
         return out
-    out = torch.empty((x.shape[0], int(c_out)), dtype=torch.float32, device=x.device)
+    out = _empty((x.shape[0], int(c_out)), torch.float32, x.device)
     _check(lib().ssc_bn_gate_fwd(_p(x, torch.float32), x.shape[0], x.shape[1], _p(scale), _p(shift),
                                  _p(gate_of_channel), int(c_out), int(c_gate_base), int(scalar_act), int(gate_act),
                                  _p(scalar_bias), _p(gate_bias), _p(out), _stream()))
@@ -1495,10 +1512,10 @@ def bn_train(x, field_of_channel, scalar_of_channel, n_field, n_scalar, weight, 
     running.mul_(1 - momentum).add_(momentum * batch)."""
     x = x.contiguous()
     n, c = x.shape
-    flat = torch.empty(n_scalar + n_field + 3 * c, dtype=torch.float32, device=x.device)
+    flat = _empty(n_scalar + n_field + 3 * c, torch.float32, x.device)
     scale, shift, chan_mean, mean, var = flat.split([c, c, c, n_scalar, n_field])   # (the first ones 16-byte aligned)
     nbytes = int(lib().ssc_bn_scratch_bytes(n, c))
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    scratch = _empty(nbytes, torch.uint8, x.device)
     _check(lib().ssc_bn_train(_p(x, torch.float32), n, c, _p(field_of_channel, torch.int32),
                               _p(scalar_of_channel, torch.int32), int(n_field), int(n_scalar), _p(weight), _p(bias),
                               float(eps), float(momentum), _p(running_mean), _p(running_var), mean.data_ptr() or flat.data_ptr(), _p(var),
@@ -1516,10 +1533,10 @@ def bn_gate_backward(x, gout, field_of_channel, scalar_of_channel, n_field, n_sc
     x, gout = x.contiguous(), gout.contiguous()
     n, c = x.shape
     gx = torch.empty_like(x)
-    d_w = torch.empty(n_field, dtype=torch.float32, device=x.device)
-    d_b = torch.empty(max(n_scalar, 1), dtype=torch.float32, device=x.device)
+    d_w = _empty(n_field, torch.float32, x.device)
+    d_b = _empty(max(n_scalar, 1), torch.float32, x.device)
     nbytes = int(lib().ssc_bn_scratch_bytes(n, c))
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    scratch = _empty(nbytes, torch.uint8, x.device)
     table, start, length, s_act, g_act = gate if gate is not None else (None, None, None, 0, 0)
     _check(lib().ssc_bn_gate_bwd(_p(x, torch.float32), _p(gout, torch.float32), n, c, gout.shape[1],
                                  _p(field_of_channel, torch.int32), _p(scalar_of_channel, torch.int32), int(n_field),
@@ -1535,10 +1552,10 @@ def bn_backward(x, gy, field_of_channel, scalar_of_channel, n_field, n_scalar, m
     x, gy = x.contiguous(), gy.contiguous()
     n, c = x.shape
     gx = torch.empty_like(x)
-    d_w = torch.empty(n_field, dtype=torch.float32, device=x.device)
-    d_b = torch.empty(max(n_scalar, 1), dtype=torch.float32, device=x.device)
+    d_w = _empty(n_field, torch.float32, x.device)
+    d_b = _empty(max(n_scalar, 1), torch.float32, x.device)
     nbytes = int(lib().ssc_bn_scratch_bytes(n, c))
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    scratch = _empty(nbytes, torch.uint8, x.device)
     mean_c = None if n_scalar == 0 else mean.contiguous()
     _check(lib().ssc_bn_bwd(_p(x, torch.float32), _p(gy, torch.float32), n, c, _p(field_of_channel, torch.int32),
                             _p(scalar_of_channel, torch.int32), int(n_field), int(n_scalar), _p(mean_c),
@@ -1566,5 +1583,5 @@ def scatter_add_rate(out, rows, steps, lanes_per_row=8, warps_per_sm=16):
     rows = rows.to(torch.int32).contiguous()
     nbytes = ctypes.c_ulonglong(0)
     _check(lib().ssc_scatter_add_rate(_p(out), int(out.shape[1]), _p(rows, torch.int32), int(rows.numel()), int(steps),
-                                      int(lanes_per_row), int(warps_per_sm), ctypes.byref(nbytes), _stream()))
+                                      int(lanes_per_row), int(warps_per_sm), ctypes.addressof(nbytes), _stream()))
     return int(nbytes.value)

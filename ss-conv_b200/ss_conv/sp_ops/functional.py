@@ -90,8 +90,8 @@ def _global_pool_function(native_fp, native_bp):
             n, c = feats.size()
             feats = feats.contiguous()
             proposals_offset = proposals_offset.contiguous().int()
-            out = torch.empty((n_prop, c), dtype=torch.float32, device=feats.device)     # every element is written
-            maxidx = torch.empty((n_prop, c), dtype=torch.int32, device=feats.device)    # (by the maximum only)
+            out = _ext._empty((n_prop, c), torch.float32, feats.device)     # every element is written
+            maxidx = _ext._empty((n_prop, c), torch.int32, feats.device)    # (by the maximum only)
             native_fp(feats, proposals_offset, out, maxidx, n_prop, c)
             ctx.for_backwards = (maxidx, proposals_offset, n)
             return out
@@ -156,8 +156,8 @@ class ThreeNN(Function):
         """unknown [N,4], known [M,4] rows (batch,x,y,z) -> (distance [N,3], index [N,3])."""
         unknown, known = unknown.contiguous(), known.contiguous()
         n, m = unknown.size(0), known.size(0)
-        dist2 = torch.empty((n, 3), dtype=torch.float32, device=unknown.device)
-        idx = torch.empty((n, 3), dtype=torch.int32, device=unknown.device)
+        dist2 = _ext._empty((n, 3), torch.float32, unknown.device)
+        idx = _ext._empty((n, 3), torch.int32, unknown.device)
         _ext.three_nn(n, m, unknown, known, dist2, idx)
         return torch.sqrt(dist2), idx
 
@@ -174,7 +174,7 @@ class ThreeInterpolate(Function):
         m, c = features.size()
         n = idx.size(0)
         ctx.three_interpolate_for_backward = (idx, weight, m)
-        out = torch.empty((n, c), dtype=torch.float32, device=features.device)
+        out = _ext._empty((n, c), torch.float32, features.device)
         _ext.three_interpolate_fp(c, m, n, features, idx, weight, out)
         return out
 

@@ -166,8 +166,8 @@ class Voxel2Point(nn.Module):
         if (point_cloud.is_cuda and point_cloud.dtype == torch.float32 and batch_ids.dtype in (torch.int32, torch.int64)
                 and vx_feats.is_cuda and vx_feats.dtype == torch.float32):
             rows = _ext.point_rows(point_cloud.detach().contiguous(), batch_ids.int().contiguous())
-            dist2 = torch.empty((rows.shape[0], 3), dtype=torch.float32, device=rows.device)
-            idx = torch.empty((rows.shape[0], 3), dtype=torch.int32, device=rows.device)
+            dist2 = _ext._empty((rows.shape[0], 3), torch.float32, rows.device)
+            idx = _ext._empty((rows.shape[0], 3), torch.int32, rows.device)
             _ext.three_nn(rows.shape[0], vx_points.shape[0], rows, vx_points, dist2, idx)
             return three_interpolate(vx_feats, idx, _ext.nn_weights(dist2))
         points = torch.cat([batch_ids.float().unsqueeze(1), point_cloud], dim=1)

@@ -30,6 +30,26 @@ def test_library_exports_every_declared_symbol():
     assert _ext.lib().ssc_has_tcgen05() == 1
 
 
+def test_bindings_cover_every_function_and_check_their_arguments():
+    from ss_conv import _ext
+    assert _ext._host is not None and _ext.lib() is _ext._host
+    for name, (_, args) in _ext.SIGNATURES.items():
+        with pytest.raises(TypeError):
+            getattr(_ext._host, name)(*[0] * (len(args) + 1))
+    with pytest.raises(RuntimeError):                 # no CPU tensors
+        _ext._p(torch.zeros(3))
+    assert _ext._p(None) is None
+    with pytest.raises(OverflowError):
+        _ext.lib().ssc_pairs_from_nbr_scratch_bytes(2 ** 40, 1)
+    assert _ext.lib().ssc_layer_ahead(None) == 1 and b"null pointer" in _ext.lib().ssc_last_error()
+    where = (ctypes.c_void_p * 1)()                    # a c_void_p is the pointer, an array is pointed to
+    assert _ext.lib().ssc_layer_ahead_bytes(ctypes.c_void_p(None)) == 0
+    assert _ext.lib().ssc_read_words(where, -1, ctypes.c_void_p(None), None) == 1
+    assert _ext._empty((2, 0, 3), torch.int32, torch.device("cpu")).shape == (2, 0, 3)
+    with pytest.raises(RuntimeError):
+        _ext._empty((-1,), torch.int32, torch.device("cpu"))
+
+
 def test_layer_structure_has_the_size_of_the_librarys():
     import ctypes
     from ss_conv import _ext
