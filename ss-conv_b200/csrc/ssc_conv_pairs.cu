@@ -17,15 +17,17 @@
 //     only operand traffic per tile is the gathered rows.  All strips walk their lists from the
 //     first row to the last at the same pace, so at any time the CTAs of the grid read and update
 //     the same window of rows: the gathers and the reductions hit L2.
-//   * warps 0 .. S-1: producers.  Warp w owns ring slot w: two lanes per row (each 32-byte sector
-//     is asked for once), 16-byte cp.async copies of the row's 128-byte slab from the staged operand
-//     image (TF32-rounded fp32, fp16 or bf16) into the K-major 128-byte-swizzled operand layout,
-//     then one arrival per lane on the slot's "full" mbarrier.
-//   * warp S: tensor-memory allocation and the MMA-issuing thread: tcgen05.mma M=128, N<=256,
+//   * warps 0 .. 3: producers.  They fill every ring slot together, 32 pairs each, four lanes to a row:
+//     16-byte cp.async copies of the row's 128-byte slab from the staged operand image (TF32-rounded
+//     fp32, fp16 or bf16) into the K-major 128-byte-swizzled operand layout.  Nobody waits for
+//     copies: their completion arrives on the slot's "full" mbarrier by itself, and the issuing warp
+//     orders the rows for the tensor core.  (A warp per slot that waited for its own copies let
+//     a slot turn round in 5000 cycles: 1240 us for 2.2 M pairs of 256 -> 256 channels.)
+//   * warp 4: the filter matrix of each strip, tensor-memory allocation and the MMA-issuing thread: tcgen05.mma M=128, N<=256,
 //     accumulating over the slabs of a tile in one of TWO accumulator buffers, tcgen05.commit to
 //     the slot's "empty" barrier and, after the last slab, to the buffer's "accumulator full"
 //     barrier.
-//   * warps S+1 .. S+8: epilogue, two per quarter of the tensor-memory lanes (they take the
+//   * warps 5 .. 12: epilogue, two per quarter of the tensor-memory lanes (they take the
 //     32-column blocks in turn).  tcgen05.ld (lane = pair), a transposition through shared memory,
 //     16 rows at a time, so that eight neighbouring lanes hold the 128 contiguous bytes of one
 //     output row, then red.global.add.v4.f32: the reductions reach L2 as whole 128-byte lines.
@@ -44,7 +46,8 @@ constexpr int PL_M = 128;                 // pairs per tile
 constexpr int PL_A_BYTES = PL_M * 128;    // one gathered slab
 constexpr int PL_MAX_STAGES = 6;
 constexpr int PL_EPI_WARPS = 8;
-constexpr int PL_STG_ROW = 144;           // bytes per row of the epilogue's transpose block (128 + 16 pad)
+constexpr int PL_PRODUCERS = 4;           // producer warps
+constexpr int PL_STG_ROW = 128;           // bytes per row of the epilogue's transpose block (pieces swizzled by the row)
 constexpr int PL_STG_BYTES = PL_EPI_WARPS * 16 * PL_STG_ROW;
 constexpr int PL_CTRL_BYTES = 1024;
 constexpr int PL_MAX_CTAS = 320;
@@ -57,7 +60,7 @@ struct PlParams {
   int n_split;      // ranges of output channels (each a strip of its own)
   int n_cta;        // output channels per CTA = n_pad / n_split: multiple of 16, <= 256
   int acc_cols;     // tensor-memory columns of one accumulator buffer (power of two >= n_cta, >= 32)
-  int stages;       // ring slots = producer warps
+  int stages;       // ring slots
   int w_bytes;      // k_slabs * n_cta * 128: the resident filter matrix
   int threads;
   int ctas_per_sm;
@@ -198,7 +201,7 @@ pl_strips_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_c
 }
 
 template <bool F16>
-__global__ void __launch_bounds__((PL_MAX_STAGES + 1 + PL_EPI_WARPS) * 32, 1)
+__global__ void __launch_bounds__((PL_PRODUCERS + 1 + PL_EPI_WARPS) * 32, 1)
 conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict__ packed, int c_out,
                       const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in,
                       const int32_t *__restrict__ starts, const int4 *__restrict__ strips,
@@ -222,12 +225,12 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
 
   const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
   const int S = p.stages;
-  const int mma_warp = S;
+  constexpr int mma_warp = PL_PRODUCERS;
   const int n_strips = *n_strips_dev;
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(smem_u32(full_bars + s), 32);
+      mbar_init(smem_u32(full_bars + s), PL_PRODUCERS * 32);    // arrivals by copies
       mbar_init(smem_u32(empty_bars + s), 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -252,98 +255,86 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t a_base = smem_u32(a_smem), w_base = smem_u32(w_smem);
 
-  // Every role walks the same strips and keeps the same counters: g = ring steps so far (slot
-  // g % S, use g / S), tcount = tiles so far (buffer tcount % 2), scount = strips so far.
-  if (warp < S) {
+  // Every role walks the same strips and keeps the same counters: ring slot and its parity, tcount = tiles so far
+  // (buffer tcount % 2), scount = strips so far.
+  if (warp < PL_PRODUCERS) {
     // ==================================== producers =============================================
-    // Two lanes per row: lanes 2j and 2j+1 copy neighbouring 16-byte chunks, i.e. one whole 32-byte
-    // sector per pair of lanes and instruction (one lane per row would ask for every sector twice,
-    // once per half).  Pass p of a step covers rows 16 p .. 16 p + 15; a lane copies four chunks
-    // (2 cc + its parity, cc = 0..3) of its row in each of the eight passes.
-    const int lrow = lane >> 1, lpar = lane & 1;
-    const uint32_t sw = (uint32_t)(lrow & 7);             // row & 7 (16 p keeps the low three bits)
-    const uint32_t row_off0 = (uint32_t)(lrow >> 3) * 1024u + sw * 128u;   // + p * 2048
-    const uint32_t slot_addr = a_base + (uint32_t)warp * PL_A_BYTES;
-    long long g = 0;
-    int scount = 0, w_issued = 0;
+    // Lane l copies the 16-byte pieces l & 3 and (l & 3) + 4 of rows 8 * pass + l / 4 of its warp's 32, four passes;
+    // the input rows of the tile after this one are on their way meanwhile.
+    const int sub = lane & 3, row8 = lane >> 2;
+    const uint32_t warp_rows = a_base + (uint32_t)warp * 4096u + (uint32_t)row8 * 128u;
+    const uint32_t first0 = warp_rows + (((uint32_t)sub ^ (uint32_t)row8) << 4), first1 = warp_rows + (((uint32_t)(sub + 4) ^ (uint32_t)row8) << 4);
+    const uint32_t full0 = smem_u32(full_bars), empty0 = smem_u32(empty_bars), row_bytes = (uint32_t)p.row_words * 4u;
+    const char *lane_rows = (const char *)staged + sub * 16;
+    const int k_slabs = p.k_slabs, slab_words = p.slab_words;
+    int slot = 0;
+    uint32_t par = 1;                                     // (a fresh barrier counts as passed with parity 1)
     bool alive = true;
     for (int si = 0; si < n_strips && alive; ++si) {
       if (__ldg(owner + si) != (int)blockIdx.x) continue;
       const int4 sd = __ldg(strips + si);
-      const int kappa = sd.x / p.n_split, half = sd.x - kappa * p.n_split;
+      const int kappa = sd.x / p.n_split;
       const int list0 = __ldg(starts + kappa), n_pairs = __ldg(starts + kappa + 1) - list0;
       const int n_tiles = sd.w;
-      if (warp == 0 && lane == 0) {
-        // the strip's filter matrix: one bulk copy per slab, after the MMAs of the last strip retired
-        bool ok = true;
-        if (scount > 0) ok = mbar_wait_backoff(smem_u32(wfree_bar), (uint32_t)(scount - 1) & 1u, abort_flag, 128);
-        if (ok) {
-          const uint32_t bar = smem_u32(wfull_bar), slab_bytes = (uint32_t)p.n_cta * 128u;
-          mbar_expect_tx(bar, (uint32_t)p.w_bytes);
-          for (int s = 0; s < p.k_slabs; ++s) {
-            const uint4 *src = packed + ((size_t)kappa * p.k_slabs + s) * (size_t)(p.n_pad * 8) + (size_t)half * (size_t)(p.n_cta * 8);
-            bulk_g2s(w_base + (uint32_t)s * slab_bytes, src, slab_bytes, bar);
-          }
-          ++w_issued;
-        }
-      }
-      const long long n_steps = (long long)n_tiles * p.k_slabs;
-      // input rows of step q (the same for every slab of a tile)
-      auto load_rows = [&](long long q, int *dst) {
-        const int ti = (int)(q / p.k_slabs);
-        const int row0 = (sd.y + ti * sd.z) * PL_M;       // position of the tile in the offset's list
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          const int j = row0 + r * 16 + lrow;
-          dst[r] = j < n_pairs ? __ldg(pair_in + list0 + j) : -1;
-        }
+      auto row_of = [&](int ti) {                         // input row of this lane's pair
+        const int j = (sd.y + ti * sd.z) * PL_M + warp * 32 + lane;
+        return ti < n_tiles && j < n_pairs ? __ldg(pair_in + list0 + j) : -1;
       };
-      // first step of this strip that falls on this warp's slot
-      long long q = ((long long)warp - g % S + S) % S;
-      int src[8], nxt[8];
-      if (q < n_steps) load_rows(q, nxt);
-      for (; q < n_steps; q += S) {
-        const int ti = (int)(q / p.k_slabs), slab = (int)(q - (long long)ti * p.k_slabs);
+      int src = row_of(0);
+      for (int ti = 0; ti < n_tiles && alive; ++ti) {
+        const int next = row_of(ti + 1);
+        int from[4];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) src[r] = nxt[r];
-        if (q + S < n_steps) load_rows(q + S, nxt);       // in flight while this step waits and copies
-        const long long use = (g + q) / S;
-        if (use > 0) {
-          if (!mbar_wait_warp_backoff(smem_u32(empty_bars + warp), (uint32_t)(use - 1) & 1u, abort_flag, 32)) { alive = false; break; }
-          tc_fence_after();
-        }
-        const int w0 = slab * 32;                          // first 4-byte word of the slab
+        for (int i = 0; i < 4; ++i) from[i] = __shfl_sync(0xffffffffu, src, i * 8 + row8);
+#pragma unroll 1
+        for (int slab = 0; slab < k_slabs; ++slab) {
+          const char *base = lane_rows + slab * 128, *at[4];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          if (src[r] >= 0) {
-            const float *fp = staged + (size_t)src[r] * p.row_words + w0;
-            const uint32_t a_row = slot_addr + row_off0 + (uint32_t)r * 2048u;
-#pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {   // chunks past the last real word are zero-filled
-              const int c = 2 * cc + lpar;
-              const bool ok = w0 + c * 4 < p.slab_words;
-              cp_async16_cg(a_row + (((uint32_t)c ^ sw) << 4), ok ? (const void *)(fp + c * 4) : (const void *)staged, ok ? 16u : 0u);
-            }
+          for (int i = 0; i < 4; ++i) at[i] = base + (unsigned long long)(uint32_t)from[i] * row_bytes;
+          const uint32_t full = full0 + (uint32_t)slot * 8u, slot_off = (uint32_t)slot * (uint32_t)PL_A_BYTES;
+          if (!mbar_wait_uniform(empty0 + (uint32_t)slot * 8u, par, abort_flag)) { alive = false; break; }
+          const uint32_t dst0 = first0 + slot_off, dst1 = first1 + slot_off;
+          if ((slab + 1) * 32 <= slab_words) {
+            copy_row_pieces<0>(from[0], dst0, dst1, at[0]);
+            copy_row_pieces<1024>(from[1], dst0, dst1, at[1]);
+            copy_row_pieces<2048>(from[2], dst0, dst1, at[2]);
+            copy_row_pieces<3072>(from[3], dst0, dst1, at[3]);
+          } else {                                        // the last slab of a row that does not fill it
+            const int words = slab_words - slab * 32 - sub * 4;
+            const uint32_t bytes0 = words > 0 ? 16u : 0u, bytes1 = words > 16 ? 16u : 0u;
+            const char *base0 = bytes0 ? base : (const char *)staged, *base1 = bytes1 ? base + 64 : (const char *)staged;
+            const uint32_t stride0 = bytes0 ? row_bytes : 0u, stride1 = bytes1 ? row_bytes : 0u;
+            copy_row_ends<0>(from[0], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
+            copy_row_ends<1024>(from[1], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
+            copy_row_ends<2048>(from[2], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
+            copy_row_ends<3072>(from[3], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
           }
+          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
+          if (++slot == S) { slot = 0; par ^= 1u; }
         }
-        cp_async_commit();
-        cp_async_wait_all();
-        fence_async_smem();
-        mbar_arrive(smem_u32(full_bars + warp));
+        src = next;
       }
-      g += n_steps;
-      ++scount;
     }
-    // a wait gave up while a filter copy may still be in flight: let it land before the CTA exits
-    if (warp == 0 && lane == 0 && *abort_flag && w_issued > 0) mbar_wait_drain(smem_u32(wfull_bar), (uint32_t)(w_issued - 1) & 1u);
+    cp_async_wait_all();
   } else if (warp == mma_warp) {
     // ==================================== MMA issuer: the whole warp, one elected lane issues ====
-    int tcount = 0, scount = 0;
+    int tcount = 0, scount = 0, w_issued = 0;
     uint32_t slot = 0, slot_par = 0;
     bool alive = true;
     for (int si = 0; si < n_strips && alive; ++si) {
       if (__ldg(owner + si) != (int)blockIdx.x) continue;
-      const int n_tiles = __ldg(strips + si).w;
+      const int4 sd = __ldg(strips + si);
+      const int n_tiles = sd.w, kappa = sd.x / p.n_split, half = sd.x - kappa * p.n_split;
+      // the strip's filter matrix: one bulk copy per slab, after the MMAs of the last strip retired
+      if (scount > 0 && !mbar_wait_uniform(smem_u32(wfree_bar), (uint32_t)(scount - 1) & 1u, abort_flag)) break;
+      if (elect_one()) {
+        const uint32_t bar = smem_u32(wfull_bar), slab_bytes = (uint32_t)p.n_cta * 128u;
+        mbar_expect_tx(bar, (uint32_t)p.w_bytes);
+        for (int s = 0; s < p.k_slabs; ++s)
+          bulk_g2s(w_base + (uint32_t)s * slab_bytes,
+                   packed + ((size_t)kappa * p.k_slabs + s) * (size_t)(p.n_pad * 8) + (size_t)half * (size_t)(p.n_cta * 8), slab_bytes, bar);
+      }
+      ++w_issued;
       if (!mbar_wait_uniform(smem_u32(wfull_bar), (uint32_t)scount & 1u, abort_flag)) break;
       tc_fence_after();
       for (int ti = 0; ti < n_tiles && alive; ++ti, ++tcount) {
@@ -355,6 +346,7 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
         const uint32_t d = tmem_base + (uint32_t)(buf * p.acc_cols);
         for (int s = 0; s < p.k_slabs; ++s) {
           if (!mbar_wait_uniform(smem_u32(full_bars + slot), slot_par, abort_flag)) { alive = false; break; }
+          fence_async_smem();                             // the rows other threads' copies left, for the tensor core
           tc_fence_after();
           const uint32_t a_lo = desc_lo(a_base + slot * PL_A_BYTES);
           const uint32_t b_lo = desc_lo(w_base + (uint32_t)s * (uint32_t)p.n_cta * 128u);
@@ -376,6 +368,8 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
     // everything issued above (on any path) retires before the CTA hands its tensor memory back
     if (elect_one()) mma_commit(smem_u32(final_bar));
     mbar_wait_drain(smem_u32(final_bar), 0u);
+    // a wait gave up while a filter copy may still be in flight: let it land before the CTA exits
+    if (*abort_flag && w_issued > 0) mbar_wait_drain(smem_u32(wfull_bar), (uint32_t)(w_issued - 1) & 1u);
   } else {
     // ==================================== epilogue ==============================================
     // Two warps per quarter of the tensor-memory lanes; they take the 32-column blocks of the
@@ -439,7 +433,7 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
             if ((lane >> 4) == h) {
 #pragma unroll
               for (int q = 0; q < 8; ++q)
-                *(uint4 *)(blk + (lane & 15) * PL_STG_ROW + q * 16) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                *(uint4 *)(blk + (lane & 15) * PL_STG_ROW + ((q ^ (lane & 7)) << 4)) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             }
             __syncwarp();
             const int c_local = blk_i * 32 + sub * 4;       // column within the strip's range
@@ -448,7 +442,7 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
             for (int i = 0; i < 4; ++i) {
               const int row = 4 * i + grp;
               const int orow = __shfl_sync(0xffffffffu, my_out, 16 * h + row);
-              const float4 x = *(const float4 *)(blk + row * PL_STG_ROW + sub * 16);
+              const float4 x = *(const float4 *)(blk + row * PL_STG_ROW + ((sub ^ (row & 7)) << 4));
               if (orow >= 0 && c_local < cols) {
                 float *dst = out + (size_t)orow * c_out + cc;
                 if (vec_ok) {
@@ -524,12 +518,12 @@ static bool pl_params(int c_in, int c_out, int precision, PlParams &p) {
   if (p.n_split == 0 || p.n_cta < 16) return false;
   p.acc_cols = 32;
   while (p.acc_cols < p.n_cta) p.acc_cols <<= 1;
-  p.ctas_per_sm = 1;      // 13 to 15 warps with ~100 registers each: one persistent CTA per SM
+  p.ctas_per_sm = 1;      // 13 warps with ~120 registers each: one persistent CTA per SM
   const size_t b = budget;
   p.stages = (int)((b - p.w_bytes) / PL_A_BYTES);
   if (p.stages > PL_MAX_STAGES) p.stages = PL_MAX_STAGES;
   if (p.stages < 3) return false;
-  p.threads = (p.stages + 1 + PL_EPI_WARPS) * 32;
+  p.threads = (PL_PRODUCERS + 1 + PL_EPI_WARPS) * 32;
   const uint32_t fmt = is16 ? (precision == SSC_PREC_BF16 ? 1u : 0u) : 2u;
   p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.n_cta >> 3) << 17) | ((uint32_t)(PL_M >> 4) << 24);
   return true;

@@ -589,27 +589,6 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 }
 
 // ---------------------------------------------------------------------------------------------------
-// The two 16-byte pieces a lane copies of a row (none if `from` is negative), OFF bytes into its part of the slot;
-// predicated instead of branched around: the instructions around the copies are what the producers' time goes into.
-template <int OFF>
-__device__ __forceinline__ void copy_row_pieces(int from, uint32_t dst0, uint32_t dst1, const char *at) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %0, 0;\n\t"
-      "@p cp.async.cg.shared.global [%1+%4], [%3], 16;\n\t"
-      "@p cp.async.cg.shared.global [%2+%4], [%3+64], 16;\n\t}" ::"r"(from), "r"(dst0), "r"(dst1), "l"(at), "n"(OFF)
-      : "memory");
-}
-// The same where a piece may lie past the row's end: it is zero-filled then, and its (base, stride) lead somewhere valid.
-template <int OFF>
-__device__ __forceinline__ void copy_row_ends(int from, uint32_t dst0, uint32_t dst1, const char *base0, uint32_t stride0, uint32_t bytes0,
-                                              const char *base1, uint32_t stride1, uint32_t bytes1) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ge.s32 p, %0, 0;\n\tmad.wide.u32 a, %0, %4, %3;\n\tmad.wide.u32 b, %0, %6, %5;\n\t"
-      "@p cp.async.cg.shared.global [%1+%9], [a], 16, %7;\n\t"
-      "@p cp.async.cg.shared.global [%2+%9], [b], 16, %8;\n\t}" ::"r"(from), "r"(dst0), "r"(dst1), "l"(base0), "r"(stride0),
-      "l"(base1), "r"(stride1), "r"(bytes0), "r"(bytes1), "n"(OFF)
-      : "memory");
-}
 // (one lane) a word for the issuing warp and the arrival that releases it.
 __device__ __forceinline__ void store_and_arrive(bool on, uint32_t at, uint32_t word, uint32_t bar) {
   asm volatile(
