@@ -79,16 +79,14 @@ struct PlParams {
 // greedily, main strips first, each to the CTA with the least work so far: every CTA starts with a
 // strip that walks its offset's list from the first row (all CTAs sweep the rows together, which keeps
 // gathers and reductions in L2) and the tails fill the CTAs whose offsets were short.
-// What bounds it is the greedy assignment, one strip after the other: with the CTAs' loads spread over a warp
-// each strip cost a scan of all of them from shared memory, 140 us for the 330 strips of a 5^3 layer.
-// A thread now holds the load of one CTA in a register and a block-wide minimum (two shuffle
-// reductions, the lowest CTA wins ties) decides per strip; the first strip of every CTA needs no
-// decision (all loads are zero, so they go to the CTAs in order).
+// What bounds it is the greedy assignment, one strip after the other: with the CTAs' loads in shared memory each
+// strip cost a scan of all of them, 140 us for the 330 strips of a 5^3 layer; with a load per thread of the
+// block and two barriers per strip 30 us.  One warp now holds ten loads per lane in registers (the lowest
+// CTA wins ties); the first strip of every CTA needs no decision (all loads are zero, so they go in order).
 __global__ void __launch_bounds__(PL_MAX_CTAS)
 pl_strips_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_ctas,
                  int32_t *__restrict__ hdr, int4 *__restrict__ strips, int32_t *__restrict__ owner) {
   __shared__ int tiles[256], first[257], tiles_of[PL_MAX_CTAS];
-  __shared__ unsigned best_s[2][PL_MAX_CTAS / 32];
   __shared__ int L_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (hdr[0] > 0 && hdr[1] == K && hdr[2] == n_split && hdr[3] == n_ctas) return;   // built before for this grid
@@ -146,8 +144,6 @@ pl_strips_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_c
   __syncthreads();
   // main strips (-1) first, then tails (-2), each to the CTA with the least work so far.  Work and CTA in one word:
   // a load is at most the number of tiles of a table, which stays below 2^22 for 2^31 / 128 / K pairs.
-  unsigned load = 0;
-  int turn = 0;
   __shared__ int n_main_s;
   if (tid < 32) {              // the main strips among the first n_ctas strips of that kind
     int seen = 0;
@@ -165,32 +161,34 @@ pl_strips_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_c
     if (lane == 0) n_main_s = seen < n_ctas ? seen : n_ctas;
   }
   __syncthreads();
-  if (tid < n_main_s) load = (unsigned)tiles_of[tid];
-  for (int pass = -1; pass >= -2; --pass) {
-    for (int s0 = 0; s0 < n_strips; s0 += PL_MAX_CTAS) {
-      const int mine = s0 + tid < n_strips ? owner[s0 + tid] : 0, work = s0 + tid < n_strips ? strips[s0 + tid].w : 0;
-      __shared__ int kind_s[PL_MAX_CTAS], work_s[PL_MAX_CTAS];
-      kind_s[tid] = mine;
-      work_s[tid] = work;
-      __syncthreads();
-      const int end = min(PL_MAX_CTAS, n_strips - s0);
-      for (int i = 0; i < end; ++i) {
-        if (kind_s[i] != pass) continue;            // the same for the whole block
-        unsigned v = tid < n_ctas ? (load << 9) | (unsigned)tid : 0xffffffffu;
-        v = __reduce_min_sync(0xffffffffu, v);
-        if (lane == 0) best_s[turn][warp] = v;
-        __syncthreads();
-        unsigned m = lane < PL_MAX_CTAS / 32 ? best_s[turn][lane] : 0xffffffffu;
-        m = __reduce_min_sync(0xffffffffu, m);
-        if ((int)(m & 511u) == tid) {
-          load += (unsigned)work_s[i];
-          owner[s0 + i] = tid;
+  if (warp == 0) {
+    constexpr int PER = PL_MAX_CTAS / 32;
+    unsigned key[PER];                              // of CTA 32 j + lane
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int cta = j * 32 + lane;
+      key[j] = cta < n_ctas ? ((cta < n_main_s ? (unsigned)tiles_of[cta] : 0u) << 9) | (unsigned)cta : 0xffffffffu;
+    }
+    for (int pass = -1; pass >= -2; --pass) {
+      for (int s0 = 0; s0 < n_strips; s0 += 32) {
+        const int s = s0 + lane, kind = s < n_strips ? owner[s] : 0, work = s < n_strips ? strips[s].w : 0;
+        int to = kind;
+        for (unsigned left = __ballot_sync(0xffffffffu, kind == pass); left != 0u; left &= left - 1u) {
+          const int i = __ffs((int)left) - 1;
+          unsigned m = key[0];
+#pragma unroll
+          for (int j = 1; j < PER; ++j) m = min(m, key[j]);
+          m = __reduce_min_sync(0xffffffffu, m);
+          const unsigned add = (unsigned)__shfl_sync(0xffffffffu, work, i) << 9;
+#pragma unroll
+          for (int j = 0; j < PER; ++j) key[j] += key[j] == m ? add : 0u;
+          if (lane == i) to = (int)(m & 511u);
         }
-        turn ^= 1;
+        if (kind == pass) owner[s] = to;
       }
-      __syncthreads();
     }
   }
+  __syncthreads();
   if (tid == 0) {
     hdr[1] = K;
     hdr[2] = n_split;
@@ -198,6 +196,17 @@ pl_strips_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_c
     __threadfence();
     hdr[0] = n_strips;
   }
+}
+
+// A lane's piece of two rows (none of a negative one), OFF bytes into its part of the slot.
+template <int OFF>
+__device__ __forceinline__ void copy_rows(int a, int b, uint32_t dst0, uint32_t dst1, const char *base, uint32_t stride, uint32_t bytes) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 s, t;\n\tsetp.ge.s32 p, %0, 0;\n\tsetp.ge.s32 q, %1, 0;\n\t"
+      "mad.wide.u32 s, %0, %5, %4;\n\tmad.wide.u32 t, %1, %5, %4;\n\t"
+      "@p cp.async.cg.shared.global [%2+%7], [s], 16, %6;\n\t"
+      "@q cp.async.cg.shared.global [%3+%7], [t], 16, %6;\n\t}" ::"r"(a), "r"(b), "r"(dst0), "r"(dst1), "l"(base), "r"(stride), "r"(bytes), "n"(OFF)
+      : "memory");
 }
 
 template <bool F16>
@@ -259,13 +268,15 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
   // (buffer tcount % 2), scount = strips so far.
   if (warp < PL_PRODUCERS) {
     // ==================================== producers =============================================
-    // Lane l copies the 16-byte pieces l & 3 and (l & 3) + 4 of rows 8 * pass + l / 4 of its warp's 32, four passes;
-    // the input rows of the tile after this one are on their way meanwhile.
-    const int sub = lane & 3, row8 = lane >> 2;
-    const uint32_t warp_rows = a_base + (uint32_t)warp * 4096u + (uint32_t)row8 * 128u;
-    const uint32_t first0 = warp_rows + (((uint32_t)sub ^ (uint32_t)row8) << 4), first1 = warp_rows + (((uint32_t)(sub + 4) ^ (uint32_t)row8) << 4);
+    // Lane l copies the 16-byte piece l & 7 of rows 4 * pass + l / 8 of its warp's 32, eight passes: a row's 128 bytes are
+    // one request (with four lanes to a row they are two, and the way out of the SM, which the reductions
+    // share, was what bound the kernel).  The input rows of the next tile are on their way meanwhile.
+    const int piece = lane & 7, row4 = lane >> 3;
+    const uint32_t warp_rows = a_base + (uint32_t)warp * 4096u;
+    const uint32_t first0 = warp_rows + (uint32_t)row4 * 128u + (uint32_t)((piece ^ row4) << 4);
+    const uint32_t first1 = warp_rows + (uint32_t)(row4 + 4) * 128u + (uint32_t)((piece ^ row4 ^ 4) << 4);
     const uint32_t full0 = smem_u32(full_bars), empty0 = smem_u32(empty_bars), row_bytes = (uint32_t)p.row_words * 4u;
-    const char *lane_rows = (const char *)staged + sub * 16;
+    const char *lane_rows = (const char *)staged + piece * 16;
     const int k_slabs = p.k_slabs, slab_words = p.slab_words;
     int slot = 0;
     uint32_t par = 1;                                     // (a fresh barrier counts as passed with parity 1)
@@ -283,32 +294,21 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
       int src = row_of(0);
       for (int ti = 0; ti < n_tiles && alive; ++ti) {
         const int next = row_of(ti + 1);
-        int from[4];
+        int from[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) from[i] = __shfl_sync(0xffffffffu, src, i * 8 + row8);
+        for (int i = 0; i < 8; ++i) from[i] = __shfl_sync(0xffffffffu, src, i * 4 + row4);
 #pragma unroll 1
         for (int slab = 0; slab < k_slabs; ++slab) {
-          const char *base = lane_rows + slab * 128, *at[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) at[i] = base + (unsigned long long)(uint32_t)from[i] * row_bytes;
+          // pieces past the last channel are zero-filled (and read nothing)
+          const uint32_t bytes = slab * 32 + piece * 4 < slab_words ? 16u : 0u, stride = bytes ? row_bytes : 0u;
+          const char *base = bytes ? lane_rows + slab * 128 : (const char *)staged;
           const uint32_t full = full0 + (uint32_t)slot * 8u, slot_off = (uint32_t)slot * (uint32_t)PL_A_BYTES;
           if (!mbar_wait_uniform(empty0 + (uint32_t)slot * 8u, par, abort_flag)) { alive = false; break; }
           const uint32_t dst0 = first0 + slot_off, dst1 = first1 + slot_off;
-          if ((slab + 1) * 32 <= slab_words) {
-            copy_row_pieces<0>(from[0], dst0, dst1, at[0]);
-            copy_row_pieces<1024>(from[1], dst0, dst1, at[1]);
-            copy_row_pieces<2048>(from[2], dst0, dst1, at[2]);
-            copy_row_pieces<3072>(from[3], dst0, dst1, at[3]);
-          } else {                                        // the last slab of a row that does not fill it
-            const int words = slab_words - slab * 32 - sub * 4;
-            const uint32_t bytes0 = words > 0 ? 16u : 0u, bytes1 = words > 16 ? 16u : 0u;
-            const char *base0 = bytes0 ? base : (const char *)staged, *base1 = bytes1 ? base + 64 : (const char *)staged;
-            const uint32_t stride0 = bytes0 ? row_bytes : 0u, stride1 = bytes1 ? row_bytes : 0u;
-            copy_row_ends<0>(from[0], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
-            copy_row_ends<1024>(from[1], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
-            copy_row_ends<2048>(from[2], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
-            copy_row_ends<3072>(from[3], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
-          }
+          copy_rows<0>(from[0], from[1], dst0, dst1, base, stride, bytes);
+          copy_rows<1024>(from[2], from[3], dst0, dst1, base, stride, bytes);
+          copy_rows<2048>(from[4], from[5], dst0, dst1, base, stride, bytes);
+          copy_rows<3072>(from[6], from[7], dst0, dst1, base, stride, bytes);
           asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
           if (++slot == S) { slot = 0; par ^= 1u; }
         }
