@@ -402,159 +402,184 @@ bn_finish_var_kernel(const float *__restrict__ part, int row_blocks, int n, int 
 //   ks = r w, ka = w r^3 A / N, kg = r w G / N (ka = kg = 0 with running statistics).
 // y and g are recomputed from x and go in both passes (PASS 0 adds up A and G, PASS 1 writes gx), so neither
 // is ever stored: 2 reads of x and go and one write of gx per backward, instead of four tensors more.
-// A block takes R whole rows at a time into shared memory, evaluates every gate once, then walks the
-// channels.  PASS 0: block = one chain of rows (the order of the sums is that of the batch statistics
-// above), thread = channels.  PASS 1: R consecutive rows (a straight copy).  Without a gate table g = go
-// (batch norm alone); without ks gx = g (activation alone).  HBM-bound.
+// A block takes R whole rows at a time into shared memory, every warp the rows w, w + 8, ... on its own: it copies them
+// (the next tile's are on their way while it works on this one), evaluates their gates and turns go into g.
+// PASS 0: block = one chain of rows (the order of the sums is that of the batch statistics above); the
+// warps meet and a thread adds up its channels' rows.  PASS 1: R consecutive rows, and the warp writes gx.
+// Without a gate table g = go (batch norm alone); without ks gx = g (activation alone).  Issue-bound, hence: the
+// per-channel constants stand in shared memory as two 16-byte words, a sigmoid is evaluated once for value and
+// slope, a lane works on two rows of its gate at a time (with constants read from global memory per
+// element a row of 76 channels took 400 warp instructions: 33 + 38 us for 61 k rows).
 struct BnGateBwd {
   const float *x, *go;
   int n, c, c_out, n_gates, rows, chains;      // rows = R
   const float *scale, *shift, *mu;             // per channel (may be NULL: identity / zero)
   const int32_t *gate_of_channel, *field_start, *field_len;
   int s_act, g_act;
-  int vec;                                     // both row lengths and pointers allow 16-byte copies
 };
 
 constexpr int kBwdMaxAcc = 4;                  // channels of a thread in PASS 0
 
-__device__ __forceinline__ float act_grad(float v, int kind) {
+// Slope of the activation at v, `value` there given (the sigmoid's slope follows from it).
+__device__ __forceinline__ float act_grad(float v, float value, int kind) {
   if (kind == 1) return v > 0.f ? 1.f : 0.f;
-  if (kind == 2) {
-    const float sg = 1.0f / (1.0f + expf(-v));
-    return sg * (1.f - sg);
-  }
+  if (kind == 2) return value * (1.f - value);
   return 1.f;
 }
+__host__ __device__ constexpr size_t align4(size_t floats) { return (floats + 3) & ~(size_t)3; }
 
-template <int PASS>
+template <int VEC>
+__device__ __forceinline__ void copy_floats(float *dst, const float *src) {      // VEC floats, asynchronously
+  const uint32_t to = smem_u32(dst);
+  if (VEC == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(src) : "memory");
+  else if (VEC == 2) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(src) : "memory");
+}
+
+template <int PASS, int VEC>
 __global__ void __launch_bounds__(256)
 bn_gate_bwd_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
                    float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
   extern __shared__ __align__(16) float sm[];
-  float *xs = sm, *gs = xs + (size_t)p.rows * p.c, *as = gs + (size_t)p.rows * p.c_out, *gg = as + (size_t)p.rows * p.n_gates;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int row_step = PASS == 0 ? p.chains : 1;                 // distance of a tile's rows
-  const int first = PASS == 0 ? (int)blockIdx.x : (int)blockIdx.x * p.rows;
-  const int tile_step = PASS == 0 ? p.rows * p.chains : (int)gridDim.x * p.rows;
-  // PASS 1: channels over threads, rows of the tile over the lanes that are left when the row is short
-  const int lanes = PASS == 0 || p.c >= nt ? 1 : nt / p.c;
-  const int ch_step = p.c >= nt || PASS == 0 ? nt : p.c;
-  const int ch_block = PASS == 0 ? (int)blockIdx.y * nt * kBwdMaxAcc : 0;
-  const int ch_first = ch_block + tid % ch_step, lane = tid / ch_step;
+  const int R = p.rows, c = p.c, c_out = p.c_out, n_gates = p.n_gates;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const size_t buffer = (size_t)R * (c + c_out);                   // x rows, then go rows
+  float *as = sm + 2 * buffer, *gg = as + (size_t)R * n_gates;
+  // the block's rows are PASS 0 blockIdx.x, + chains, ..., PASS 1 R consecutive ones of every gridDim.x tiles: `row` of
+  // its tile's first and `left` how many follow
+  const int row_step = PASS == 0 ? p.chains : 1;
+  const int tile_step = PASS == 0 ? R * p.chains : R * (int)gridDim.x;
+  auto load = [&](int row, int rows, int buf) {
+    float *xs = sm + buf * buffer, *gs = xs + (size_t)R * c;
+    for (int r = warp; r < rows; r += 8) {
+      const size_t at = (size_t)(row + r * row_step);
+      for (int i = lane * VEC; i < c; i += 32 * VEC) copy_floats<VEC>(xs + r * c + i, p.x + at * c + i);
+      for (int i = lane * VEC; i < c_out; i += 32 * VEC) copy_floats<VEC>(gs + r * c_out + i, p.go + at * c_out + i);
+    }
+    cp_async_commit();
+  };
+  // gates over the lanes: several rows at a time where a row has few
+  const bool few = n_gates > 0 && n_gates <= 32;
+  const int per = few ? 32 / n_gates : 1, lane_row = few ? lane / n_gates : 0, lane_gate = few ? lane % n_gates : lane;
+  const bool affine = p.scale != nullptr;
+  // constants of a channel: (scale, shift, mean, gate: -3 itself a gate scalar, -2 copy, -1 scalar), (ks, ka, kg)
+  float4 *chan = (float4 *)(sm + align4(2 * buffer + 2 * (size_t)R * n_gates)), *coef = chan + c;
+  for (int ch = tid; ch < c; ch += 256) {
+    const int gate = p.gate_of_channel ? (ch < c_out ? __ldg(p.gate_of_channel + ch) : -3) : -2;
+    chan[ch] = make_float4(affine ? __ldg(p.scale + ch) : 1.f, affine ? __ldg(p.shift + ch) : 0.f, p.mu ? __ldg(p.mu + ch) : 0.f, __int_as_float(gate));
+    if (PASS == 1) coef[ch] = ks ? make_float4(__ldg(ks + ch), __ldg(ka + ch), __ldg(kg + ch), 0.f) : make_float4(1.f, 0.f, 0.f, 0.f);
+  }
+  __syncthreads();
   float sum_a[kBwdMaxAcc], sum_g[kBwdMaxAcc];
 #pragma unroll
   for (int i = 0; i < kBwdMaxAcc; ++i) sum_a[i] = sum_g[i] = 0.f;
-  for (int r0 = first; r0 < p.n; r0 += tile_step) {
-    const int rows = min(p.rows, (p.n - r0 + row_step - 1) / row_step);
-    if (p.vec) {
-      const int cx = p.c >> 2, cg = p.c_out >> 2;
-      if (PASS == 1) {
-        for (int i = tid; i < rows * cx; i += nt) ((float4 *)xs)[i] = __ldg((const float4 *)(p.x + (size_t)r0 * p.c) + i);
-        for (int i = tid; i < rows * cg; i += nt) ((float4 *)gs)[i] = __ldg((const float4 *)(p.go + (size_t)r0 * p.c_out) + i);
-      } else {
-        for (int i = tid; i < rows * cx; i += nt) {
-          const int r = i / cx;
-          ((float4 *)xs)[i] = __ldg((const float4 *)(p.x + (size_t)(r0 + r * row_step) * p.c) + (i - r * cx));
-        }
-        for (int i = tid; i < rows * cg; i += nt) {
-          const int r = i / cg;
-          ((float4 *)gs)[i] = __ldg((const float4 *)(p.go + (size_t)(r0 + r * row_step) * p.c_out) + (i - r * cg));
-        }
-      }
-    } else {
-      for (int i = tid; i < rows * p.c; i += nt) {
-        const int r = i / p.c;
-        xs[i] = __ldg(p.x + (size_t)(r0 + r * row_step) * p.c + (i - r * p.c));
-      }
-      for (int i = tid; i < rows * p.c_out; i += nt) {
-        const int r = i / p.c_out;
-        gs[i] = __ldg(p.go + (size_t)(r0 + r * row_step) * p.c_out + (i - r * p.c_out));
-      }
-    }
-    __syncthreads();
-    if (p.n_gates > 0) {
-      for (int i = tid; i < rows * p.n_gates; i += nt) {
-        const int r = i / p.n_gates, j = i - r * p.n_gates;
-        const float *xr = xs + r * p.c, *gr = gs + r * p.c_out;
-        const int cg = p.c_out + j;
-        float v = xr[cg];
-        if (p.scale) v = fmaf(v, p.scale[cg], p.shift[cg]);
-        const int s0 = p.field_start[j], len = p.field_len[j];
-        float acc = 0.f;
-        for (int q = 0; q < len; ++q) {
-          float y = xr[s0 + q];
-          if (p.scale) y = fmaf(y, p.scale[s0 + q], p.shift[s0 + q]);
-          acc = fmaf(gr[s0 + q], y, acc);
-        }
-        as[i] = apply_act(v, p.g_act);
-        gg[i] = acc * act_grad(v, p.g_act);
-      }
-      __syncthreads();
-    }
-    // g of a channel of a row; its gate's value and the gate scalars' gradients stand in shared memory
-    auto gradient = [&](int r, int ch, int gate, float x, float sc, float sh) -> float {
-      if (gate == -3) return gg[r * p.n_gates + ch - p.c_out];
-      float g = gs[r * p.c_out + ch];
-      if (gate == -1) g *= act_grad(p.scale ? fmaf(x, sc, sh) : x, p.s_act);
-      else if (gate >= 0) g *= as[r * p.n_gates + gate];
-      return g;
-    };
-    if (PASS == 0) {
-      // all threads turn go into g in place, then a thread adds up the rows of its channels in order: the
-      // chain is two shared-memory loads and two additions per row
-      if (p.gate_of_channel) {
-        const int per = p.c_out >= nt ? 1 : nt / p.c_out, step = p.c_out >= nt ? nt : p.c_out;
-        if (tid / step < per)
-          for (int ch = tid % step; ch < p.c_out; ch += step) {
-            const int gate = p.gate_of_channel[ch];
-            if (gate < -1) continue;
-            const float sc = p.scale ? p.scale[ch] : 1.f, sh = p.scale ? p.shift[ch] : 0.f;
-            for (int r = tid / step; r < rows; r += per) gs[r * p.c_out + ch] = gradient(r, ch, gate, xs[r * p.c + ch], sc, sh);
+  const int ch_block = PASS == 0 ? (int)blockIdx.y * 256 * kBwdMaxAcc : 0;
+
+  const int first = PASS == 0 ? (int)blockIdx.x : (int)blockIdx.x * R;
+  int left = PASS == 0 ? (p.n - first + p.chains - 1) / p.chains : 0;      // PASS 0: rows of the chain still to come
+  auto rows_at = [&](int row, int in_chain) { return max(0, min(R, PASS == 0 ? in_chain : p.n - row)); };
+  int buf = 0, rows = rows_at(first, left);
+  load(first, rows, 0);
+  for (int r0 = first; rows > 0; r0 += tile_step, buf ^= 1) {
+    const int next = r0 > p.n - tile_step ? 0 : rows_at(r0 + tile_step, left - R);   // (r0 + tile_step stays below n)
+    load(r0 + tile_step, next, buf ^ 1);                           // (nothing behind the last tile)
+    cp_async_wait(1);
+    __syncwarp();
+    float *xs = sm + buf * buffer, *gs = xs + (size_t)R * c;
+    if (lane_row < per) {
+      for (int j = lane_gate; j < n_gates; j += 32) {
+        const float4 kc = chan[c_out + j];
+        const int s0 = __ldg(p.field_start + j), len = __ldg(p.field_len + j);
+        for (int r = warp + 8 * lane_row; r < rows; r += 16 * per) {
+          const int r2 = r + 8 * per < rows ? r + 8 * per : r;
+          const float *xa = xs + r * c, *xb = xs + r2 * c, *ga = gs + r * c_out + s0, *gb = gs + r2 * c_out + s0;
+          float va = xa[c_out + j], vb = xb[c_out + j], acc_a = 0.f, acc_b = 0.f;
+          if (affine) {
+            va = fmaf(va, kc.x, kc.y);
+            vb = fmaf(vb, kc.x, kc.y);
           }
-        __syncthreads();
+          for (int q = 0; q < len; ++q) {
+            const float2 k = *(const float2 *)(chan + s0 + q);
+            float ya = xa[s0 + q], yb = xb[s0 + q];
+            if (affine) {
+              ya = fmaf(ya, k.x, k.y);
+              yb = fmaf(yb, k.x, k.y);
+            }
+            acc_a = fmaf(ga[q], ya, acc_a);
+            acc_b = fmaf(gb[q], yb, acc_b);
+          }
+          const float fa = apply_act(va, p.g_act), fb = apply_act(vb, p.g_act);
+          as[r * n_gates + j] = fa;
+          gg[r * n_gates + j] = acc_a * act_grad(va, fa, p.g_act);
+          if (r2 != r) {
+            as[r2 * n_gates + j] = fb;
+            gg[r2 * n_gates + j] = acc_b * act_grad(vb, fb, p.g_act);
+          }
+        }
       }
+    }
+    __syncwarp();
+    // go of a channel into g; gates' values and the gate scalars' gradients stand in shared memory
+    for (int ch0 = 0; ch0 < (PASS == 0 ? c_out : c); ch0 += 32) {
+      const int ch = ch0 + lane;
+      const bool in = ch < (PASS == 0 ? c_out : c);
+      const float4 kc = chan[in ? ch : 0];
+      const int gate = in ? __float_as_int(kc.w) : -2;
+      const bool scalars = __any_sync(0xffffffffu, gate == -1);
+      // where g comes from and what it is multiplied by (nothing: gate < 0)
+      const float *from = gate == -3 ? gg + (ch - c_out) : gs + ch, *by = as + (gate >= 0 ? gate : 0);
+      const int step = gate == -3 ? n_gates : c_out;
+      if (!in || (PASS == 0 && gate < -1)) continue;
+      const float4 kd = PASS == 1 ? coef[ch] : make_float4(0.f, 0.f, 0.f, 0.f);
+      float *to = PASS == 1 ? gx + (size_t)(r0 + warp) * c + ch : gs + warp * c_out + ch;
+#pragma unroll 4
+      for (int r = warp; r < rows; r += 8) {
+        const float x = PASS == 1 || scalars ? xs[r * c + ch] : 0.f;
+        float g = from[r * step];
+        if (gate >= 0) g *= by[r * n_gates];
+        if (scalars && gate == -1) {
+          const float y = affine ? fmaf(x, kc.x, kc.y) : x;
+          g *= act_grad(y, p.s_act == 2 ? apply_act(y, 2) : 0.f, p.s_act);
+        }
+        *to = PASS == 0 ? g : ks ? kd.x * g - kd.y * (x - kc.z) - kd.z : g;
+        to += PASS == 1 ? 8 * (size_t)c : 8 * (size_t)c_out;
+      }
+    }
+    if (PASS == 0) {
+      __syncthreads();
 #pragma unroll
       for (int i = 0; i < kBwdMaxAcc; ++i) {
-        const int ch = ch_first + i * ch_step;
-        if (ch < p.c) {
-          const float mu = p.mu ? p.mu[ch] : 0.f;
-          const float *gp = ch < p.c_out ? gs + ch : gg + (ch - p.c_out), *xp = xs + ch;
-          const int gstep = ch < p.c_out ? p.c_out : p.n_gates;
+        const int ch = ch_block + tid + i * 256;
+        if (ch < c) {
+          const float mu = chan[ch].z;
+          const float *gp = ch < c_out ? gs + ch : gg + (ch - c_out), *xp = xs + ch;
+          const int gstep = ch < c_out ? c_out : n_gates;
           float s = sum_g[i], a = sum_a[i];
 #pragma unroll 8
           for (int r = 0; r < rows; ++r) {
             const float g = gp[r * gstep];
             s += g;
-            a = fmaf(g, xp[r * p.c] - mu, a);
+            a = fmaf(g, xp[r * c] - mu, a);
           }
           sum_g[i] = s;
           sum_a[i] = a;
         }
       }
-    } else if (lane < lanes) {
-      for (int ch = ch_first; ch < p.c; ch += ch_step) {
-        const float mu = p.mu ? p.mu[ch] : 0.f;
-        const float sc = p.scale ? p.scale[ch] : 1.f, sh = p.scale ? p.shift[ch] : 0.f;
-        const int gate = p.gate_of_channel ? (ch < p.c_out ? p.gate_of_channel[ch] : -3) : -2;
-        const float k_s = ks ? ks[ch] : 1.f, k_a = ks ? ka[ch] : 0.f, k_g = ks ? kg[ch] : 0.f;
-#pragma unroll 4
-        for (int r = lane; r < rows; r += lanes) {
-          const float x = xs[r * p.c + ch];
-          const float g = gradient(r, ch, gate, x, sc, sh);
-          gx[(size_t)(r0 + r) * p.c + ch] = ks ? k_s * g - k_a * (x - mu) - k_g : g;
-        }
-        if (p.c < nt) break;
-      }
+      __syncthreads();
+    } else {
+      __syncwarp();
     }
-    __syncthreads();
+    left -= R;
+    rows = next;
   }
+  cp_async_wait_all();
   if (PASS == 0) {
 #pragma unroll
     for (int i = 0; i < kBwdMaxAcc; ++i) {
-      const int ch = ch_first + i * ch_step;
-      if (ch < p.c) {
-        part_a[(size_t)blockIdx.x * p.c + ch] = sum_a[i];
-        part_g[(size_t)blockIdx.x * p.c + ch] = sum_g[i];
+      const int ch = ch_block + tid + i * 256;
+      if (ch < c) {
+        part_a[(size_t)blockIdx.x * c + ch] = sum_a[i];
+        part_g[(size_t)blockIdx.x * c + ch] = sum_g[i];
       }
     }
   }
@@ -738,33 +763,41 @@ extern "C" int ssc_bn_stats(const float *x, int n, int c, const int32_t *field_o
                       mean, var, var + n_field, nullptr, nullptr, scratch, scratch_bytes, stream);
 }
 
-// Rows per tile of the backward kernels: as many as 32 KB of shared memory hold (up to seven blocks per SM), no
-// more than a chain has.
-static int bwd_tile_rows(int c, int c_out, int n_gates, size_t *smem) {
-  const size_t per_row = (size_t)(c + c_out + 2 * n_gates) * sizeof(float);
-  int rows = (int)(32 * 1024 / per_row);
-  rows = rows >= 8 ? (rows & ~3) : (rows < 1 ? 1 : rows);     // multiples of four keep the copies 16-byte aligned
-  if (rows > 32) rows = 32;
-  *smem = rows * per_row;
+// Rows per tile of the backward kernels: a multiple of eight (a row per warp), as many as 44 KB of shared memory hold
+// twice (five blocks per SM); fewer where eight rows do not fit.
+static int bwd_tile_rows(int c, int c_out, int n_gates, int most, size_t *smem) {
+  const size_t per_row = (size_t)(2 * (c + c_out) + 2 * n_gates) * sizeof(float), fixed = (size_t)c * 32 + 16;
+  int rows = most;
+  while (rows > 8 && rows * per_row + fixed > 44 * 1024) rows -= 8;
+  while (rows > 1 && rows * per_row + fixed > 200 * 1024) --rows;
+  *smem = rows * per_row + fixed;
   return rows;
+}
+
+template <int PASS, int VEC>
+static int launch_bwd_vec(const BnGateBwd &p, size_t smem, const float *ks, const float *ka, const float *kg, float *gx, float *part_a, float *part_g, cudaStream_t st) {
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(bn_gate_bwd_kernel<PASS, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "bn_gate_bwd: smem attribute: %s", cudaGetErrorString(e));
+  }
+  int blocks = PASS == 0 ? p.chains : ceil_div(p.n, p.rows);
+  if (PASS == 1 && blocks > 5 * 148) blocks = 5 * 148;
+  bn_gate_bwd_kernel<PASS, VEC><<<dim3(blocks, PASS == 0 ? ceil_div(p.c, 256 * kBwdMaxAcc) : 1), 256, smem, st>>>(p, ks, ka, kg, gx, part_a, part_g);
+  note_launches(1);
+  SSC_CHECK_LAUNCH("bn_gate_bwd");
+  return SSC_OK;
 }
 
 template <int PASS>
 static int launch_bwd(BnGateBwd p, const float *ks, const float *ka, const float *kg, float *gx, float *part_a, float *part_g, cudaStream_t st) {
   size_t smem;
-  p.rows = bwd_tile_rows(p.c, p.c_out, p.n_gates, &smem);
+  p.rows = bwd_tile_rows(p.c, p.c_out, p.n_gates, PASS == 0 ? 32 : 64, &smem);
   p.chains = 8 * bn_row_blocks(p.n);
-  p.vec = (p.c & 3) == 0 && (p.c_out & 3) == 0 && (((uintptr_t)p.x | (uintptr_t)p.go) & 15u) == 0;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(bn_gate_bwd_kernel<PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "bn_gate_bwd: smem attribute: %s", cudaGetErrorString(e));
-  }
-  const int threads = 256;
-  int blocks = PASS == 0 ? p.chains : ceil_div(p.n, p.rows);
-  if (PASS == 1 && blocks > 8 * 148) blocks = 8 * 148;
-  { bn_gate_bwd_kernel<PASS><<<dim3(blocks, PASS == 0 ? ceil_div(p.c, threads * kBwdMaxAcc) : 1), threads, smem, st>>>(p, ks, ka, kg, gx, part_a, part_g); note_launches(1); }
-  SSC_CHECK_LAUNCH("bn_gate_bwd");
-  return SSC_OK;
+  const int odd = p.c | p.c_out;
+  const uintptr_t at = (uintptr_t)p.x | (uintptr_t)p.go;
+  if ((odd & 3) == 0 && (at & 15u) == 0) return launch_bwd_vec<PASS, 4>(p, smem, ks, ka, kg, gx, part_a, part_g, st);
+  if ((odd & 1) == 0 && (at & 7u) == 0) return launch_bwd_vec<PASS, 2>(p, smem, ks, ka, kg, gx, part_a, part_g, st);
+  return launch_bwd_vec<PASS, 1>(p, smem, ks, ka, kg, gx, part_a, part_g, st);
 }
 
 extern "C" int ssc_bn_gate_bwd(const float *x, const float *gout, int n, int c, int c_out, const int32_t *field_of_channel,
@@ -782,7 +815,7 @@ extern "C" int ssc_bn_gate_bwd(const float *x, const float *gout, int n, int c, 
   float *part_a = (float *)scratch, *part_g = part_a + (size_t)8 * rb * c;
   float *ks = part_g + (size_t)8 * rb * c, *ka = ks + c, *kg = ka + c;
   BnGateBwd p = {x, gout, n, c, c_out, gate_of_channel ? c - c_out : 0, 0, 0, scale, shift, chan_mean, gate_of_channel, field_start, field_len,
-                 scalar_act, gate_act, 0};
+                 scalar_act, gate_act};
   if (int e = launch_bwd<0>(p, nullptr, nullptr, nullptr, nullptr, part_a, part_g, st)) return e;
   { bn_bwd_finish_kernel<<<n_field, kFinishThreads, 0, st>>>(part_a, part_g, rb, n, c, field_of_channel, scalar_of_channel, var, weight, eps,
                                                            training, ks, ka, kg, d_weight, d_bias); note_launches(1); }
@@ -811,6 +844,6 @@ extern "C" int ssc_gate_bwd(const float *x, const float *gy, int n, int c_total,
   if (n == 0) return SSC_OK;
   SSC_REQUIRE(x && gy && gx && gate_of_channel && (c_total == c_out || (field_start && field_len)), "gate_bwd: null pointer");
   BnGateBwd p = {x, gy, n, c_total, c_out, c_total - c_out, 0, 0, nullptr, nullptr, nullptr, gate_of_channel, field_start, field_len,
-                 scalar_act, gate_act, 0};
+                 scalar_act, gate_act};
   return launch_bwd<1>(p, nullptr, nullptr, nullptr, gx, nullptr, nullptr, as_stream(stream));
 }

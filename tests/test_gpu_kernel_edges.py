@@ -179,3 +179,36 @@ def test_points_outside_the_grid_are_dropped_as_the_torch_steps_do(cuda, n, batc
     assert torch.equal(got[0], want[0]) and torch.equal(got[3], want[3])
     assert torch.equal(got[1].indices, want[1].indices) and torch.equal(got[1].features, want[1].features)
     assert got[3]._ssc_any == bool(want[3].sum() > 0)
+
+
+@pytest.mark.parametrize("Rs,n", [([(1, 0)], 1), ([(2, 0), (3, 1)], 9), ([(4, 0), (4, 1), (4, 2), (4, 3)], 520), ([(2, 0), (2, 1), (2, 2), (2, 3)], 4999),
+                                  ([(40, 0), (40, 1)], 70), ([(300, 0), (200, 1)], 33)])
+@pytest.mark.parametrize("training", [True, False])
+def test_norm_and_gate_gradients_at_tile_edges(cuda, Rs, n, training):
+    """One row and a few more than a tile, channels that are odd, even and multiples of four, no gates, more gates than
+    lanes, more channels than threads: against the float64 composite.  Every term carries a few roundings of fp32
+    and sums of n terms stay within n ulp of the sum of magnitudes: 1e-4 of the largest entry."""
+    import copy
+    from ss_conv.activation import Activation
+    from ss_conv.batchnorm import BatchNorm
+    from ss_conv.sp_ops.tensor import SparseTensor
+    torch.manual_seed(n)
+    n_gates = sum(m for m, l in Rs if l > 0)
+    gated = Rs + ([(n_gates, 0)] if n_gates else [])
+    c, c_out = (sum(m * (2 * l + 1) for m, l in r) for r in (gated, Rs))
+    bn, act = BatchNorm(gated).to(cuda), Activation(Rs, (torch.relu, torch.sigmoid), bias=False, checkpoint=False).to(cuda)
+    with torch.no_grad():
+        bn.weight.uniform_(0.5, 1.5)
+        bn.bias.normal_(0, 0.3)
+    bn.train(training)
+    bn64, act64 = copy.deepcopy(bn).double().cpu(), copy.deepcopy(act).double().cpu()
+    x = (torch.randn(n, c, device=cuda) + 0.2).requires_grad_(True)
+    coef = torch.randn(n, c_out, device=cuda)
+    both = bn.norm_and_gate(SparseTensor(x, torch.zeros(n, 4, dtype=torch.int32, device=cuda), [8] * 3, 1), act)
+    (both.features * coef).sum().backward()
+    x64 = x.detach().double().cpu().requires_grad_(True)
+    (act64._gate_composite(bn64._differentiable(x64)) * coef.double().cpu()).sum().backward()
+    scale = max(float(x64.grad.abs().max()), 1e-3)
+    assert float((x.grad.cpu().double() - x64.grad).abs().max()) <= 1e-4 * scale
+    for got, want in ((bn.weight.grad, bn64.weight.grad), (bn.bias.grad, bn64.bias.grad)):
+        assert float((got.cpu().double() - want).abs().max()) <= 1e-4 * max(float(want.abs().max()), 1.0)
