@@ -139,6 +139,12 @@ int ssc_rulebook_conv_fill(const int32_t *indices, int n_in, int batch, const in
                            int32_t *out_indices, int32_t *nbr, int32_t *pairs,
                            int32_t *indice_num, int32_t *status, void *scratch,
                            size_t scratch_bytes, const int32_t *n_out_dev, void *stream);
+/* Both phases back to back with the capacity n_out, without pair lists: the exact count stays in n_out_dev (fewer
+ * launches than the two calls). */
+int ssc_rulebook_conv_ahead(const int32_t *indices, int n_in, int batch, const int in_shape[3], const int out_shape[3],
+                            const int ksize[3], const int stride[3], const int padding[3], const int dilation[3],
+                            int transpose, int n_out, int32_t *out_indices, int32_t *nbr, int32_t *n_out_dev,
+                            int32_t *status, void *scratch, size_t scratch_bytes, const int32_t *n_in_dev, void *stream);
 
 /* Neighbour table from a reference-format rulebook (indicePairs [K,2,n_cols], indiceNum [K]):
  * nbr[kappa][pairs[kappa][1-swap][i]] = pairs[kappa][swap][i].  swap = 1 is the "inverse"

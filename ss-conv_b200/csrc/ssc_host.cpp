@@ -178,10 +178,26 @@ PyObject *empty(PyObject *, PyObject *const *args, Py_ssize_t n) {
   }
 }
 
+// head(tensor, n): its first n rows, tensor[:n].
+PyObject *head(PyObject *, PyObject *const *args, Py_ssize_t n) {
+  if (n != 2 || !THPVariable_Check(args[0])) {
+    PyErr_SetString(PyExc_TypeError, "head(tensor, n)");
+    return nullptr;
+  }
+  const long long rows = PyLong_AsLongLong(args[1]);
+  if (rows == -1 && PyErr_Occurred()) return nullptr;
+  try {
+    return THPVariable_Wrap(THPVariable_Unpack(args[0]).narrow(0, 0, rows));
+  } catch (const std::exception &e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+
 #define SSC_FUNCTIONS \
   X(ssc_version) X(ssc_last_error) X(ssc_has_tcgen05) X(ssc_kernel_launches) X(ssc_read_words) \
   X(ssc_rulebook_scratch_bytes) X(ssc_rulebook_subm) X(ssc_rulebook_subm_static) X(ssc_rulebook_subm_ahead) \
-  X(ssc_rulebook_conv_count) X(ssc_rulebook_conv_fill) X(ssc_pairs_to_nbr) X(ssc_pairs_from_nbr_scratch_bytes) \
+  X(ssc_rulebook_conv_count) X(ssc_rulebook_conv_fill) X(ssc_rulebook_conv_ahead) X(ssc_pairs_to_nbr) X(ssc_pairs_from_nbr_scratch_bytes) \
   X(ssc_pairs_from_nbr) X(ssc_materialize) X(ssc_materialize_bwd) X(ssc_conv_packed_bytes) X(ssc_conv_pack_filters) \
   X(ssc_conv_scratch_bytes) X(ssc_conv_fwd) X(ssc_conv_pairs_list_bytes) X(ssc_conv_pairs_supported) \
   X(ssc_conv_pairs_build) X(ssc_conv_fwd_pairs) X(ssc_nbr_transpose) X(ssc_nbr_row_order_scratch_bytes) \
@@ -200,6 +216,7 @@ PyObject *empty(PyObject *, PyObject *const *args, Py_ssize_t n) {
 #define X(name) {#name, (PyCFunction)(void (*)())entry<&name>, METH_FASTCALL, nullptr},
 PyMethodDef methods[] = {{"ptr", (PyCFunction)(void (*)())ptr, METH_FASTCALL, "device pointer of a contiguous CUDA tensor"},
                          {"empty", (PyCFunction)(void (*)())empty, METH_FASTCALL, "torch.empty(shape, dtype, device)"},
+                         {"head", (PyCFunction)(void (*)())head, METH_FASTCALL, "tensor[:n]"},
                          SSC_FUNCTIONS{nullptr, nullptr, 0, nullptr}};
 #undef X
 

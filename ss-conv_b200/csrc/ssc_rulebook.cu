@@ -11,6 +11,7 @@
 // Submanifold convolution skips 2-4 (outputs are the inputs).
 // Everything is integer work bound by HBM/L2 traffic; no tensor cores involved.
 #include "ssc_common.cuh"
+#include "ssc_conv_internal.cuh"
 #include "ssc_scan.cuh"
 
 namespace ssc {
@@ -347,6 +348,50 @@ static void launch_decode(const uint32_t *bitmap, const uint32_t *word_prefix, l
     { decode_outputs_bits_kernel<<<ceil_div(n_words * 32, 256), 256, 0, st>>>(bitmap, word_prefix, n_words, g, n_out, out_indices); note_launches(1); }
   } else {
     { decode_outputs_kernel<<<ceil_div(n_words, 256), 256, 0, st>>>(bitmap, word_prefix, n_words, g, n_out, out_indices); note_launches(1); }
+  }
+}
+
+// Count, ranks and coordinates of the set bits in one launch, for bitmaps of up to kRankedWords words: what bounds
+// the three or five kernels otherwise is their launches (17 us for 32 k words, of which 6 between them).  A
+// block takes WORDS words; the bits before them it counts itself, from L2: few words where that is little.
+constexpr int kRankedWords = 1 << 15;
+template <int WORDS>
+__global__ void __launch_bounds__(256)
+rank_decode_kernel(const uint32_t *__restrict__ bitmap, int n_words, Geometry g, int n_out, int4 *__restrict__ out_indices,
+                   int32_t *__restrict__ total_dev) {
+  __shared__ uint32_t smem[33], word_s[WORDS], prefix_s[WORDS];
+  const int w0 = (int)blockIdx.x * WORDS;
+  uint32_t before = 0;
+  const uint4 *quads = (const uint4 *)bitmap;                 // (256-byte aligned; w0 is a multiple of four)
+#pragma unroll 8
+  for (int q = threadIdx.x; q < w0 / 4; q += 256) {
+    const uint4 v = __ldg(quads + q);
+    before += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+  }
+  const uint32_t mine = (int)threadIdx.x < WORDS && w0 + (int)threadIdx.x < n_words ? __ldg(bitmap + w0 + threadIdx.x) : 0u;
+  uint32_t base, in_block;
+  block_exclusive_scan(before, smem, &base);
+  const uint32_t ex = block_exclusive_scan(__popc(mine), smem, &in_block);
+  if (threadIdx.x < WORDS) {
+    word_s[threadIdx.x] = mine;
+    prefix_s[threadIdx.x] = base + ex;
+  }
+  __syncthreads();
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total_dev = (int32_t)(base + in_block);
+  const int yz = g.out_shape[1] * g.out_shape[2], vol = g.out_shape[0] * yz, bit = threadIdx.x & 31;
+#pragma unroll 4
+  for (int w = threadIdx.x >> 5; w < WORDS; w += 8) {
+    const uint32_t bits = word_s[w];
+    if (!((bits >> bit) & 1u)) continue;
+    const uint32_t rank = prefix_s[w] + (uint32_t)__popc(bits & ((1u << bit) - 1u));
+    if ((int)rank >= n_out) continue;
+    const uint32_t flat = (uint32_t)(w0 + w) * 32u + (uint32_t)bit;
+    const int b = (int)(flat / (uint32_t)vol);
+    int r = (int)(flat - (uint32_t)b * (uint32_t)vol);
+    const int x = r / yz;
+    r -= x * yz;
+    const int y = r / g.out_shape[2];
+    out_indices[rank] = make_int4(b, x, y, r - y * g.out_shape[2]);
   }
 }
 
@@ -768,23 +813,20 @@ extern "C" int ssc_rulebook_subm_ahead(const int32_t *indices, int n_cap, int ba
   return SSC_OK;
 }
 
-extern "C" int ssc_rulebook_conv_count(const int32_t *indices, int n_in, int batch, const int in_shape[3],
-                                       const int out_shape[3], const int ksize[3], const int stride[3],
-                                       const int padding[3], const int dilation[3], int transpose,
-                                       int32_t *n_out_dev, int32_t *status, void *scratch,
-                                       size_t scratch_bytes, const int32_t *n_in_dev, void *stream) {
-  SSC_REQUIRE(n_in >= 0 && in_shape && out_shape && ksize && stride && padding && dilation && n_out_dev,
-              "rulebook_conv_count: bad arguments");
-  Geometry g;
-  SSC_REQUIRE(fill_geometry(g, in_shape, out_shape, ksize, stride, padding, dilation, transpose) == 0,
-              "rulebook_conv_count: bad geometry");
-  SSC_REQUIRE(g.K <= 256, "rulebook_conv_count: kernel volume %d > 256", g.K);
-  if (int e = check_volume(batch, in_shape, "rulebook_conv_count(in)")) return e;
-  if (int e = check_volume(batch, out_shape, "rulebook_conv_count(out)")) return e;
-  RulebookScratch s = carve(scratch, n_in, batch, in_shape, out_shape, g.K);
+namespace ssc {
+
+// Output cells of a regular rulebook in the bitmap, input rows in the map or table; scratch carved into s, geometry into g.
+static int mark_outputs(const char *who, const int32_t *indices, int n_in, int batch, const int in_shape[3], const int out_shape[3],
+                        const int ksize[3], const int stride[3], const int padding[3], const int dilation[3], int transpose,
+                        int32_t *status, void *scratch, size_t scratch_bytes, const int32_t *n_in_dev, cudaStream_t st,
+                        RulebookScratch &s, Geometry &g) {
+  SSC_REQUIRE(fill_geometry(g, in_shape, out_shape, ksize, stride, padding, dilation, transpose) == 0, "%s: bad geometry", who);
+  SSC_REQUIRE(g.K <= 256, "%s: kernel volume %d > 256", who, g.K);
+  if (int e = check_volume(batch, in_shape, who)) return e;
+  if (int e = check_volume(batch, out_shape, who)) return e;
+  s = carve(scratch, n_in, batch, in_shape, out_shape, g.K);
   if (scratch == nullptr || scratch_bytes < s.total)
-    return fail(SSC_ERR_SCRATCH, "rulebook_conv_count: scratch %zu < %zu bytes", scratch_bytes, s.total);
-  cudaStream_t st = as_stream(stream);
+    return fail(SSC_ERR_SCRATCH, "%s: scratch %zu < %zu bytes", who, scratch_bytes, s.total);
   bool simple = true;
   for (int d = 0; d < 3; ++d) simple = simple && (g.transpose || g.stride[d] == 1 || g.dilation[d] == 1);
   // with a dense map the marking kernel also fills the map, and one clearing covers map and bitmap: two launches
@@ -805,6 +847,46 @@ extern "C" int ssc_rulebook_conv_count(const int32_t *indices, int n_in, int bat
     }
     SSC_CHECK_LAUNCH("mark_outputs");
   }
+  return 0;
+}
+
+int rulebook_conv_ahead(const int32_t *indices, int n_in, int batch, const int in_shape[3], const int out_shape[3], const int ksize[3],
+                        const int stride[3], const int padding[3], const int dilation[3], int transpose, int n_out,
+                        int32_t *out_indices, int32_t *nbr, int32_t *n_out_dev, int32_t *status, void *scratch, size_t scratch_bytes,
+                        const int32_t *n_in_dev, cudaStream_t st) {
+  RulebookScratch s;
+  Geometry g;
+  if (int e = mark_outputs("rulebook_conv_ahead", indices, n_in, batch, in_shape, out_shape, ksize, stride, padding, dilation, transpose, status,
+                           scratch, scratch_bytes, n_in_dev, st, s, g)) return e;
+  SSC_REQUIRE((long long)n_out <= s.out_cap, "rulebook_conv_ahead: n_out %d exceeds the possible maximum", n_out);
+  if (s.n_words <= kRankedWords) {
+    const int n = (int)s.n_words;
+    if (n <= 8192) rank_decode_kernel<32><<<ceil_div(n, 32), 256, 0, st>>>(s.bitmap, n, g, n_out, (int4 *)out_indices, n_out_dev);
+    else rank_decode_kernel<128><<<ceil_div(n, 128), 256, 0, st>>>(s.bitmap, n, g, n_out, (int4 *)out_indices, n_out_dev);
+    note_launches(1);
+    SSC_CHECK_LAUNCH("rank_decode");
+  } else {
+    if (int e = exclusive_scan_u32<true>(s.bitmap, s.n_words, s.word_prefix, s.block_sums, s.misc, n_out_dev, st)) return e;
+    launch_decode(s.bitmap, s.word_prefix, s.n_words, g, n_out, (int4 *)out_indices, st);
+    SSC_CHECK_LAUNCH("decode_outputs");
+  }
+  return lookup_and_compact(out_indices, n_out, n_in, batch, g, s, nbr, nullptr, nullptr, st, n_out_dev);
+}
+
+}  // namespace ssc
+
+extern "C" int ssc_rulebook_conv_count(const int32_t *indices, int n_in, int batch, const int in_shape[3],
+                                       const int out_shape[3], const int ksize[3], const int stride[3],
+                                       const int padding[3], const int dilation[3], int transpose,
+                                       int32_t *n_out_dev, int32_t *status, void *scratch,
+                                       size_t scratch_bytes, const int32_t *n_in_dev, void *stream) {
+  SSC_REQUIRE(n_in >= 0 && in_shape && out_shape && ksize && stride && padding && dilation && n_out_dev,
+              "rulebook_conv_count: bad arguments");
+  RulebookScratch s;
+  Geometry g;
+  cudaStream_t st = as_stream(stream);
+  if (int e = mark_outputs("rulebook_conv_count", indices, n_in, batch, in_shape, out_shape, ksize, stride, padding, dilation, transpose, status,
+                           scratch, scratch_bytes, n_in_dev, st, s, g)) return e;
   if (int e = exclusive_scan_u32<true>(s.bitmap, s.n_words, s.word_prefix, s.block_sums, s.misc, n_out_dev, st)) return e;
   SSC_CHECK_LAUNCH("rulebook_conv_count");
   return SSC_OK;
@@ -837,6 +919,16 @@ extern "C" int ssc_rulebook_conv_fill(const int32_t *indices, int n_in, int batc
   if (int e = lookup_and_compact(out_indices, n_out, n_in, batch, g, s, nbr, pairs, indice_num, st, n_out_dev)) return e;
   SSC_CHECK_LAUNCH("rulebook_conv_fill");
   return SSC_OK;
+}
+
+extern "C" int ssc_rulebook_conv_ahead(const int32_t *indices, int n_in, int batch, const int in_shape[3], const int out_shape[3],
+                                       const int ksize[3], const int stride[3], const int padding[3], const int dilation[3],
+                                       int transpose, int n_out, int32_t *out_indices, int32_t *nbr, int32_t *n_out_dev,
+                                       int32_t *status, void *scratch, size_t scratch_bytes, const int32_t *n_in_dev, void *stream) {
+  SSC_REQUIRE(n_in > 0 && n_out > 0 && indices && in_shape && out_shape && ksize && stride && padding && dilation && out_indices && nbr && n_out_dev,
+              "rulebook_conv_ahead: bad arguments");
+  return rulebook_conv_ahead(indices, n_in, batch, in_shape, out_shape, ksize, stride, padding, dilation, transpose, n_out, out_indices, nbr,
+                             n_out_dev, status, scratch, scratch_bytes, n_in_dev, as_stream(stream));
 }
 
 extern "C" int ssc_pairs_to_nbr(const int32_t *pairs, const int32_t *indice_num, int K, int n_cols, int n_out,

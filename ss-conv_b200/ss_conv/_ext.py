@@ -58,6 +58,8 @@ SIGNATURES = {
                                         c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "ssc_rulebook_conv_fill": (c_int, [c_void_p, c_int, c_int, _I3, _I3, _I3, _I3, _I3, _I3, c_int, c_int, c_void_p, c_void_p,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
+    "ssc_rulebook_conv_ahead": (c_int, [c_void_p, c_int, c_int, _I3, _I3, _I3, _I3, _I3, _I3, c_int, c_int, c_void_p, c_void_p,
+                                        c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "ssc_pairs_to_nbr": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "ssc_pairs_from_nbr_scratch_bytes": (c_size_t, [c_int, c_int]),
     "ssc_pairs_from_nbr": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
@@ -239,8 +241,12 @@ def _empty(shape, dtype, device):
     return torch.empty(shape, dtype=dtype, device=device)
 
 
+def _head(t, n):
+    return t[:n]
+
+
 if _host is not None:
-    _p, _empty = _host.ptr, _host.empty      # the same, without the interpreter
+    _p, _empty, _head = _host.ptr, _host.empty, _host.head      # the same, without the interpreter
 
 
 def _stream():
@@ -425,14 +431,19 @@ def get_indice_pairs_ahead(indices, batch_size, out_shape, spatial_shape, ksize,
     n_out_dev = _empty(1, torch.int32, dev)
     st = status_word(dev)
     geo = (_i3(spatial_shape), _i3(out_shape), _i3(ksize), _i3(stride), _i3(padding), _i3(dilation), int(transpose))
-    _check(L.ssc_rulebook_conv_count(_p(indices), n_in, int(batch_size), *geo, _p(n_out_dev), _p(st), _p(scratch),
-                                     sbytes, _p(n_in_dev), _stream()))
     outids = _empty((cap, 4), torch.int32, dev)
     nbr = _empty((K, cap), torch.int32, dev)
     # the per-offset pair counts (indice_num) are not needed by the kernels that consume the table:
     # they are computed only if somebody turns the handle into reference-format pair lists
-    _check(L.ssc_rulebook_conv_fill(_p(indices), n_in, int(batch_size), *geo, cap, _p(outids), _p(nbr), None, None,
-                                    _p(st), _p(scratch), sbytes, _p(n_out_dev), _stream()))
+    if torch.cuda.is_current_stream_capturing():
+        # a recorded graph keeps the phases' own kernels: its nodes follow one another without a launch to save
+        _check(L.ssc_rulebook_conv_count(_p(indices), n_in, int(batch_size), *geo, _p(n_out_dev), _p(st), _p(scratch), sbytes,
+                                         _p(n_in_dev), _stream()))
+        _check(L.ssc_rulebook_conv_fill(_p(indices), n_in, int(batch_size), *geo, cap, _p(outids), _p(nbr), None, None,
+                                        _p(st), _p(scratch), sbytes, _p(n_out_dev), _stream()))
+    else:
+        _check(L.ssc_rulebook_conv_ahead(_p(indices), n_in, int(batch_size), *geo, cap, _p(outids), _p(nbr), _p(n_out_dev), _p(st),
+                                         _p(scratch), sbytes, _p(n_in_dev), _stream()))
     pairs = LazyPairs(nbr, n_in, n_out_dev=n_out_dev, ratio_key=None if n_in_dev is not None else key)
     pairs.regular = True
     return [outids, pairs, None]
@@ -1405,7 +1416,7 @@ def p2v_keep(points, feats, batch_ids, n_sample, n_outside, grid, unit):
                               _i3(grid), _F3(*[float(u) for u in unit]), _p(new_points), _p(new_ids), _p(new_feats), _p(flag),
                               _p(counts), _p(scratch), nbytes, _stream()))
     m, empty = read_counts([counts[:1], counts[1:]])
-    return new_points[:m], new_feats[:m], new_ids[:m], flag, empty
+    return _head(new_points, m), _head(new_feats, m), _head(new_ids, m), flag, empty
 
 
 def voxel_centres(indices, unit, extent):

@@ -117,7 +117,7 @@ class SparseTensor(object):
         """Cuts the buffers of a resolved count down to it: the inner tensors of a network are resolved with
         its last one, but nobody looks at most of them."""
         n, self._cut = self._cut, None
-        self._features, self._indices = self._features[:n], self._indices[:n]
+        self._features, self._indices = _ext._head(self._features, n), _ext._head(self._indices, n)
 
     @property
     def features(self):

@@ -212,3 +212,26 @@ def test_norm_and_gate_gradients_at_tile_edges(cuda, Rs, n, training):
     assert float((x.grad.cpu().double() - x64.grad).abs().max()) <= 1e-4 * scale
     for got, want in ((bn.weight.grad, bn64.weight.grad), (bn.bias.grad, bn64.bias.grad)):
         assert float((got.cpu().double() - want).abs().max()) <= 1e-4 * max(float(want.abs().max()), 1.0)
+
+
+@pytest.mark.parametrize("batch,grid,per", [(1, 3, 5), (1, 16, 300), (3, 17, 900), (8, 32, 700), (2, 64, 3000), (40, 32, 400)])
+def test_rulebook_in_one_go_equals_the_two_phases(cuda, batch, grid, per):
+    """Bitmaps of one word, around the 128 words of a block, at the most words of the one-launch form and above, with
+    room for more rows than there are and for fewer."""
+    from ss_conv import _ext
+    from ss_conv.sp_ops.ops import get_conv_output_size
+    rng = np.random.RandomState(per)
+    ind = dev(random_voxels(rng, batch, grid, per), cuda)
+    shape, geo = [grid] * 3, ([3] * 3, [1] * 3 if grid == 32 and batch == 40 else [2] * 3, [1] * 3, [1] * 3)
+    out_shape = get_conv_output_size(shape, *geo)
+    want = _ext.build_rulebook(ind, batch, out_shape, shape, *geo, False, False)
+    n = want[0].shape[0]
+    key = _ext._geometry_key(shape, *geo, 0)
+    for ratio in (float(n) / ind.shape[0] * 1.2, 0.0):
+        _ext._ratio_hint[key] = ratio
+        outids, pairs, _ = _ext.get_indice_pairs_ahead(ind, batch, out_shape, shape, *geo, 0)
+        rows = min(n, pairs.capacity)
+        assert int(pairs._n_out_dev.item()) == n
+        assert torch.equal(outids[:rows], want[0][:rows]) and torch.equal(pairs._nbr_cap[:, :rows], want[1][:, :rows])
+    _ext._ratio_hint.pop(key)
+    _ext.check_status(cuda)
