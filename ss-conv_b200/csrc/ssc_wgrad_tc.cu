@@ -395,32 +395,49 @@ conv_wgrad_small_kernel(const float *__restrict__ features, int c_in, const floa
   }
 }
 
-// d_filters[kappa] = sum of the offset's partials, in a fixed order.  grid (elements / 32, K), block 32 elements x
-// 8 slices: slice s adds every eighth share (the centre offset has most of them), the slices are added
-// one after the other.
+// d_filters[kappa] = sum of the offset's partials, in a fixed order.  grid (x, K), block 32 groups of VEC elements x 8
+// slices: slice s adds every eighth share (the centre offset has most of them), the slices are added one after
+// the other.  A block goes on to further elements: where its shares lie costs it more than adding them up
+// (with 32 elements per block 16 us for 27 x 64 x 76, nine tenths of it that).
+template <int VEC>
 __global__ void __launch_bounds__(256)
 wgrad_reduce_shares_kernel(const float *__restrict__ partial, const int32_t *__restrict__ starts, int K, int shares, int elems,
                            float *__restrict__ out) {
   __shared__ int first[257];
-  __shared__ float sm[8][33];
+  __shared__ float sm[8][32 * VEC + 1];
   chunk_prefix(starts, K, first);
   const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
-  const int kappa = blockIdx.y, e = blockIdx.x * 32 + lane, total = first[K];
-  float s = 0.f;
-  if (e < elems && first[kappa + 1] > first[kappa]) {
-    const int lo = share_of(first[kappa], total, shares), hi = share_of(first[kappa + 1] - 1, total, shares);
-    const bool gaps = total < shares;            // shares without a chunk wrote nothing
-    const float *p = partial + ((size_t)lo + slice + kappa) * elems + e;
-#pragma unroll 4
-    for (int b = lo + slice; b <= hi; b += 8, p += (size_t)8 * elems)
-      if (!gaps || share_begin(b + 1, total, shares) > share_begin(b, total, shares)) s += __ldg(p);
-  }
-  sm[slice][lane] = s;
-  __syncthreads();
-  if (slice == 0 && e < elems) {
+  const int kappa = blockIdx.y, total = first[K];
+  const bool any = first[kappa + 1] > first[kappa], gaps = total < shares;      // gaps: shares without a chunk wrote nothing
+  const int lo = any ? share_of(first[kappa], total, shares) : 0, hi = any ? share_of(first[kappa + 1] - 1, total, shares) : -1;
+  for (int e0 = (int)blockIdx.x * 32 * VEC; e0 < elems; e0 += (int)gridDim.x * 32 * VEC) {
+    const int e = e0 + lane * VEC;
+    float s[VEC];
 #pragma unroll
-    for (int k = 1; k < 8; ++k) s += sm[k][lane];
-    out[(size_t)kappa * elems + e] = s;
+    for (int q = 0; q < VEC; ++q) s[q] = 0.f;
+    if (e < elems) {
+      const float *p = partial + ((size_t)lo + slice + kappa) * elems + e;
+#pragma unroll 4
+      for (int b = lo + slice; b <= hi; b += 8, p += (size_t)8 * elems) {
+        if (gaps && share_begin(b + 1, total, shares) <= share_begin(b, total, shares)) continue;
+        if (VEC == 4) {
+          const float4 v = __ldg((const float4 *)p);
+          s[0] += v.x; s[1 % VEC] += v.y; s[2 % VEC] += v.z; s[3 % VEC] += v.w;
+        } else {
+          s[0] += __ldg(p);
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < VEC; ++q) sm[slice][lane * VEC + q] = s[q];
+    __syncthreads();
+    for (int i = threadIdx.x; i < 32 * VEC && e0 + i < elems; i += 256) {
+      float r = sm[0][i];
+#pragma unroll
+      for (int k = 1; k < 8; ++k) r += sm[k][i];
+      out[(size_t)kappa * elems + e0 + i] = r;
+    }
+    __syncthreads();
   }
 }
 
@@ -547,7 +564,12 @@ int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int
     return -1;
   }
   const int elems = c_in * c_out;
-  { wgrad_reduce_shares_kernel<<<dim3(ceil_div(elems, 32), K), 256, 0, st>>>(partial, pl.starts, K, p.shares, elems, d_filters); note_launches(1); }
+  const bool vec = (elems & 3) == 0 && ((uintptr_t)partial & 15u) == 0;
+  const int tiles = ceil_div(elems, vec ? 128 : 32), most = ceil_div(8 * sm_count(), K);      // one wave of blocks
+  const dim3 grid(tiles < most ? tiles : most, K);
+  if (vec) wgrad_reduce_shares_kernel<4><<<grid, 256, 0, st>>>(partial, pl.starts, K, p.shares, elems, d_filters);
+  else wgrad_reduce_shares_kernel<1><<<grid, 256, 0, st>>>(partial, pl.starts, K, p.shares, elems, d_filters);
+  note_launches(1);
   SSC_CHECK_LAUNCH("conv_wgrad_reduce");
   return SSC_OK;
 }
