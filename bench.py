@@ -13,7 +13,7 @@ value   : inputs resident in HBM, CUDA-event timed; the --steps-long region is r
 e2e     : the same step through the public ss_conv API starting from pinned HOST buffers
           (H2D of indices+features and D2H of the pooled features of every step inside the timed
           region; ss_conv.pipeline.HostStream overlaps the copies of neighbouring steps)
-roofline: dominant call (stage_features_kernel + conv_fwd_tf32_kernel): algorithmic bytes / its
+roofline: dominant call (stage_features_kernel + conv_fwd_rows_kernel): algorithmic bytes / its
           CUDA-event time
 layers  : the other layer configurations (cfg1, stage 2 of the cfg3 backbone, the wide cfg5 layer):
           rulebook and convolution call, useful TFLOP/s against the tensor-pipe peak
@@ -50,7 +50,7 @@ CFG2 = dict(name="cfg2: SS-Conv (4,4,4,4)->(4,4,4,4)+12 gates, k3 s2 p1, batch 3
 #   --clock-control none -k regex:"stage_features|conv_fwd_tf32" -c 8 python bench.py --only conv --steps 1
 # (staging: 61.4 MB read + 10.9 MB written back, most of the staged image stays in L2;
 #  convolution: 76.0 MB read + 1.0 MB written)
-NCU_DRAM_BYTES = {"stage_features_kernel": 72.3e6, "conv_fwd_tf32_kernel": 77.0e6}
+NCU_DRAM_BYTES = {"stage_features_kernel": 72.3e6, "conv_fwd_rows_kernel": 77.0e6}
 ROTATE = 4    # distinct input batches cycled through so the working set exceeds the 126 MB L2
 REGIONS = 25  # repetitions of the --steps-long timed region; the median region is reported
 
@@ -375,7 +375,7 @@ def layer_numbers(name, ind, batch, V, k, stride, pad, subm, c_in, c_out, precis
             _ext.pair_lists(nbr)          # built once per table (kept with it), like the table itself
         ms = graph_ms(lambda: _ext.conv_forward(feats, W, nbr, n_out, prec), reps=15)
         peak_t = peak_bf16 if prec in ("bf16", "fp16") else peak_bf16 / 2
-        entry = {"conv_call_ms": ms, "kernel": "pair-list (conv_fwd_pairs_kernel)" if uses_pairs else "output-stationary (conv_fwd_tf32_kernel)",
+        entry = {"conv_call_ms": ms, "kernel": "pair-list (conv_fwd_pairs_kernel)" if uses_pairs else "output-stationary (conv_fwd_rows_kernel)",
                  "voxels_per_s": n_in / (ms * 1e-3), "useful_tflops": flops / (ms * 1e-3) / 1e12,
                  "frac_of_tensor_peak": flops / (ms * 1e-3) / 1e12 / peak_t, "tensor_peak_tflops": peak_t,
                  "frac_of_hbm_peak": alg_bytes / (ms * 1e-3) / 1e9 / peak_hbm}
@@ -766,7 +766,7 @@ def run_ours(args):
     torch.cuda.synchronize()
     serial_s = time.perf_counter() - t0
 
-    # ---- dominant call alone: stage_features_kernel + conv_fwd_tf32_kernel, recorded as a small CUDA
+    # ---- dominant call alone: stage_features_kernel + conv_fwd_rows_kernel, recorded as a small CUDA
     # graph per input batch so that the CUDA events around a replay see device time only
     from ss_conv.sp_ops.ops import get_indice_pairs
     prepared = []
@@ -855,7 +855,7 @@ def run_ours(args):
     if e2e16 is not None and e2e16_s > 0:
         e2e16["value"] = vox_e2e / e2e16_s
     if rank == 0:
-        traffic = NCU_DRAM_BYTES["stage_features_kernel"] + NCU_DRAM_BYTES["conv_fwd_tf32_kernel"]
+        traffic = NCU_DRAM_BYTES["stage_features_kernel"] + NCU_DRAM_BYTES["conv_fwd_rows_kernel"]
         line = {
             "metric": "active voxels/sec per SS-Conv layer", "value": voxels / (ms * 1e-3), "unit": "voxels/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps,
@@ -886,11 +886,11 @@ def run_ours(args):
                     "serial_value": vox_e2e / serial_s, "bf16_upload": e2e16},
             "gpu_launches": int(launches),
             "clocks": clk.summary(),
-            "roofline": {"bound": "hbm", "kernel": "stage_features_kernel + conv_fwd_tf32_kernel", "achieved": achieved,
+            "roofline": {"bound": "hbm", "kernel": "stage_features_kernel + conv_fwd_rows_kernel", "achieved": achieved,
                          "peak": peak_hbm, "unit": "GB/s", "frac": achieved / peak_hbm, "traffic": traffic,
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the two kernels of the timed call on the "
                                            "cfg2 inputs (staging %.1f MB + convolution %.1f MB per launch)"
-                                           % (NCU_DRAM_BYTES["stage_features_kernel"] / 1e6, NCU_DRAM_BYTES["conv_fwd_tf32_kernel"] / 1e6),
+                                           % (NCU_DRAM_BYTES["stage_features_kernel"] / 1e6, NCU_DRAM_BYTES["conv_fwd_rows_kernel"] / 1e6),
                          "peak_source": peak_src,
                          "kernel_ms": kern_ms, "algorithmic_bytes": alg_bytes,
                          "tensor_tflops": flops / (kern_ms * 1e-3) / 1e12,
