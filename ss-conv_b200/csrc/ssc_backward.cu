@@ -99,46 +99,39 @@ __global__ void wgrad_reduce_kernel(const float *__restrict__ partial, int split
 // MODE 0: max pool (gradient goes to every input equal to the pooled value), 1: avg pool.  A block takes R input
 // rows with their piece of the table in shared memory, as in the forward pass (one thread per row and
 // channel group walking the table: 48 us for 27 offsets of 60 k rows of 76 channels).
-template <int MODE, int VEC>
+template <int MODE, int PIECE>
 __global__ void __launch_bounds__(256)
 pool_bwd_kernel(const float *__restrict__ features, const float *__restrict__ out_features,
                 const float *__restrict__ out_grad, int c, const int32_t *__restrict__ nbr_in, int K,
                 int n_in, const int32_t *__restrict__ summaryrf, float *__restrict__ d_in, int R) {
   extern __shared__ int32_t pool_smem[];
-  const PoolTile tile = pool_tile(nbr_in, K, n_in, n_in, R, pool_smem);
-  const uint32_t cg = (uint32_t)(c / VEC), items = (uint32_t)tile.rows * cg;
-  auto load = [&](const float *p, float (&v)[VEC]) {
-    if (VEC == 4) {
-      const float4 f = __ldg((const float4 *)p);
-      v[0] = f.x; v[1 % VEC] = f.y; v[2 % VEC] = f.z; v[3 % VEC] = f.w;
-    } else {
-      v[0] = __ldg(p);
-    }
+  struct Item {
+    Channels g, y;
+    float div;
   };
+  const PoolTile tile = pool_tile(nbr_in, K, n_in, n_in, R, pool_smem);
+  const uint32_t cg = (uint32_t)(c + 3) / 4, items = (uint32_t)tile.rows * cg;
   for (uint32_t t = threadIdx.x; t < items; t += 256) {
-    const int r = (int)(t / cg), c0 = (int)(t - (uint32_t)r * cg) * VEC;
+    const int r = (int)(t / cg), c0 = (int)(t - (uint32_t)r * cg) * 4, valid = c - c0;
     const size_t at = (size_t)(tile.first + r) * c + c0;
-    float x[VEC], acc[VEC];
+    Channels x, acc = {{0.f, 0.f, 0.f, 0.f}};
+    if (MODE == 0) load_rows<PIECE>(features + at, valid, x);
+    pool_visit<1, Item>(tile, r, K,
+        [&](int o, Item &v) {
+          load_rows<PIECE>(out_grad + (size_t)o * c + c0, valid, v.g);
+          if (MODE == 0) load_rows<PIECE>(out_features + (size_t)o * c + c0, valid, v.y);
+          else v.div = summaryrf ? (float)__ldg(summaryrf + o) : (float)K;
+        },
+        [&](int, const Item &v) {
+          if (MODE == 1) {
+            add_quotients(acc, v.g, v.div, __frcp_rn(v.div));
+          } else {
 #pragma unroll
-    for (int q = 0; q < VEC; ++q) x[q] = acc[q] = 0.f;
-    if (MODE == 0) load(features + at, x);
-    pool_visit(tile, r, K, [&](int o) {
-      float g[VEC], y[VEC];
-      load(out_grad + (size_t)o * c + c0, g);
-      if (MODE == 0) load(out_features + (size_t)o * c + c0, y);
-      const float div = MODE == 1 ? (summaryrf ? (float)__ldg(summaryrf + o) : (float)K) : 1.f;
-      const float inv = __frcp_rn(div);
-#pragma unroll
-      for (int q = 0; q < VEC; ++q) {
-        if (MODE == 0) {
-          if (y[q] == x[q]) acc[q] += g[q];
-        } else {
-          acc[q] += divide_by_count(g[q], div, inv);
-        }
-      }
-    });
-    if (VEC == 4) *(float4 *)(d_in + at) = make_float4(acc[0], acc[1 % VEC], acc[2 % VEC], acc[3 % VEC]);
-    else d_in[at] = acc[0];
+            for (int q = 0; q < 4; ++q)
+              if (v.y.v[q] == x.v[q]) acc.v[q] += v.g.v[q];
+          }
+        });
+    store_rows<PIECE>(d_in + at, valid, acc);
   }
 }
 
@@ -320,16 +313,15 @@ static int launch_pool_bwd(const float *features, const float *out_features, con
   SSC_REQUIRE(c > 0 && K > 0 && n_in >= 0, "%s: bad sizes", name);
   if (n_in == 0) return SSC_OK;
   SSC_REQUIRE(out_grad && nbr_in && d_in && (MODE == 1 || (features && out_features)), "%s: null pointer", name);
-  const bool vec = (c % 4 == 0) && (((uintptr_t)features | (uintptr_t)out_features | (uintptr_t)out_grad | (uintptr_t)d_in) % 16 == 0);
   const PoolShape p = pool_shape(n_in, K);
   SSC_REQUIRE(p.rows > 0, "%s: kernel of %d offsets is too large", name, K);
+  const int piece = pool_piece(c, (uintptr_t)features | (uintptr_t)out_features | (uintptr_t)out_grad | (uintptr_t)d_in);
+  auto kernel = piece == 4 ? pool_bwd_kernel<MODE, 4> : piece == 2 ? pool_bwd_kernel<MODE, 2> : pool_bwd_kernel<MODE, 1>;
   if (p.smem > 48 * 1024) {
-    cudaError_t e = vec ? cudaFuncSetAttribute(pool_bwd_kernel<MODE, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem)
-                        : cudaFuncSetAttribute(pool_bwd_kernel<MODE, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "%s: smem attribute: %s", name, cudaGetErrorString(e));
   }
-  if (vec) pool_bwd_kernel<MODE, 4><<<p.grid, 256, p.smem, as_stream(stream)>>>(features, out_features, out_grad, c, nbr_in, K, n_in, rf, d_in, p.rows);
-  else pool_bwd_kernel<MODE, 1><<<p.grid, 256, p.smem, as_stream(stream)>>>(features, out_features, out_grad, c, nbr_in, K, n_in, rf, d_in, p.rows);
+  kernel<<<p.grid, 256, p.smem, as_stream(stream)>>>(features, out_features, out_grad, c, nbr_in, K, n_in, rf, d_in, p.rows);
   note_launches(1);
   SSC_CHECK_LAUNCH(name);
   return SSC_OK;

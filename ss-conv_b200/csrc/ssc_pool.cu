@@ -8,104 +8,104 @@
 
 namespace ssc {
 
-// Rows of fp32, fp16 or bf16 (IN = 0, 1, 2) channels, four at a time or one.
-template <int IN, int VEC>
-__device__ __forceinline__ void load_channels(const void *__restrict__ rows, size_t at, float (&v)[VEC]) {
+// Rows of fp32, fp16 or bf16 (IN = 0, 1, 2) channels.
+template <int IN, int PIECE>
+__device__ __forceinline__ void load_channels(const void *__restrict__ rows, size_t at, int valid, Channels &x) {
   if (IN == 0) {
-    const float *p = (const float *)rows + at;
-    if (VEC == 4) {
-      const float4 f = __ldg((const float4 *)p);
-      v[0] = f.x; v[1 % VEC] = f.y; v[2 % VEC] = f.z; v[3 % VEC] = f.w;
-    } else {
-      v[0] = __ldg(p);
-    }
-  } else {
-    const uint16_t *p = (const uint16_t *)rows + at;
-    uint16_t h[4];
-    if (VEC == 4) {
-      const uint2 w = __ldg((const uint2 *)p);
-      h[0] = (uint16_t)w.x; h[1] = (uint16_t)(w.x >> 16); h[2] = (uint16_t)w.y; h[3] = (uint16_t)(w.y >> 16);
-    } else {
-      h[0] = __ldg(p);
-    }
-#pragma unroll
-    for (int q = 0; q < VEC; ++q) v[q] = IN == 2 ? __uint_as_float((uint32_t)h[q] << 16) : __half2float(__ushort_as_half(h[q]));
+    load_rows<PIECE>((const float *)rows + at, valid, x);
+    return;
   }
+  const uint16_t *p = (const uint16_t *)rows + at;
+  uint16_t h[4];
+  if (PIECE == 4) {
+    const uint2 w = __ldg((const uint2 *)p);
+    h[0] = (uint16_t)w.x; h[1] = (uint16_t)(w.x >> 16); h[2] = (uint16_t)w.y; h[3] = (uint16_t)(w.y >> 16);
+  } else if (PIECE == 2) {
+    const uint32_t w = __ldg((const uint32_t *)p), u = valid > 2 ? __ldg((const uint32_t *)p + 1) : 0u;
+    h[0] = (uint16_t)w; h[1] = (uint16_t)(w >> 16); h[2] = (uint16_t)u; h[3] = (uint16_t)(u >> 16);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) h[q] = q < valid ? __ldg(p + q) : (uint16_t)0;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) x.v[q] = IN == 2 ? __uint_as_float((uint32_t)h[q] << 16) : __half2float(__ushort_as_half(h[q]));
 }
 
 // MODE 0 = max (output starts at 0), 1 = avg (sum of x / divisor in ascending offset order).
-// A block takes R output rows.  Most table entries are absent (a strided 3^3 pool over surface voxels: 1.5 of 27 per
-// row), and what bounded one thread per (row, 4 channels) walking the table was that walk, done once
+template <int MODE>
+__device__ __forceinline__ void pool_add(Channels &acc, const Channels &x, float div, float inv) {
+  if (MODE == 1) {
+    add_quotients(acc, x, div, inv);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc.v[q] = x.v[q] > acc.v[q] ? x.v[q] : acc.v[q];
+  }
+}
+
+// A block takes R output rows.  Most table entries are absent (a strided 3^3 pool over surface voxels: 1.5 to 11 of 27
+// per row), and what bounded one thread per (row, 4 channels) walking the table was that walk, done once
 // per channel group: 74 us for 27 offsets of 140 k rows of 76 channels.  Here the block brings its piece of the table into shared memory
-// once, with a presence mask per row, and the threads then visit only what is there: 35 us.
-template <int MODE, int IN, int VEC>
+// once, with a presence mask per row, and the threads then visit only
+// what is there, two rows in flight (169 k rows with 11 of 27 present, 76 channels: max 94 us, with one row 100, with four 104).
+template <int MODE, int IN, int PIECE>
 __global__ void __launch_bounds__(256)
 pool_fwd_kernel(const void *__restrict__ features, int c, const int32_t *__restrict__ nbr, int K,
                 int n_out, const int32_t *__restrict__ summaryrf, float *__restrict__ out,
                 const int32_t *__restrict__ n_out_dev, int R) {
   extern __shared__ int32_t pool_smem[];
   const PoolTile tile = pool_tile(nbr, K, n_out, live_rows(n_out, n_out_dev), R, pool_smem);   // n_out: row stride of nbr
-  const uint32_t cg = (uint32_t)(c / VEC), items = (uint32_t)tile.rows * cg;
+  const uint32_t cg = (uint32_t)(c + 3) / 4, items = (uint32_t)tile.rows * cg;
   for (uint32_t t = threadIdx.x; t < items; t += 256) {
-    const int r = (int)(t / cg), c0 = (int)(t - (uint32_t)r * cg) * VEC;
+    const int r = (int)(t / cg), c0 = (int)(t - (uint32_t)r * cg) * 4, valid = c - c0;
     const int o = tile.first + r;
-    float acc[VEC];
-#pragma unroll
-    for (int q = 0; q < VEC; ++q) acc[q] = 0.f;
-    float div = 1.f;
-    if (MODE == 1) div = summaryrf ? (float)__ldg(summaryrf + o) : (float)K;
-    const float inv = __frcp_rn(div);
-    pool_visit(tile, r, K, [&](int src) {
-      float v[VEC];
-      load_channels<IN, VEC>(features, (size_t)src * c + c0, v);
-#pragma unroll
-      for (int q = 0; q < VEC; ++q) {
-        if (MODE == 0) acc[q] = v[q] > acc[q] ? v[q] : acc[q];
-        else acc[q] = acc[q] + divide_by_count(v[q], div, inv);
-      }
-    });
-    float *op = out + (size_t)o * c + c0;
-    if (VEC == 4) {
-      *(float4 *)op = make_float4(acc[0], acc[1 % VEC], acc[2 % VEC], acc[3 % VEC]);
-    } else {
-      op[0] = acc[0];
-    }
+    Channels acc = {{0.f, 0.f, 0.f, 0.f}};
+    const float div = MODE == 1 ? (summaryrf ? (float)__ldg(summaryrf + o) : (float)K) : 1.f, inv = __frcp_rn(div);
+    pool_visit<2, Channels>(tile, r, K,
+        [&](int src, Channels &x) { load_channels<IN, PIECE>(features, (size_t)src * c + c0, valid, x); },
+        [&](int, const Channels &x) { pool_add<MODE>(acc, x, div, inv); });
+    store_rows<PIECE>(out + (size_t)o * c + c0, valid, acc);
   }
 }
 
 // The same for kernels of up to eight offsets (pools of 2^3 windows, most of whose entries are present): one
-// thread per (row, VEC channels), all entries loaded at once.  The tiles above take 12.8 us for 38 k rows of
-// 64 channels and eight offsets, this 8 us.
-template <int MODE, int IN, int VEC>
+// thread per (row, 4 channels), all entries loaded at once and G rows at a time; G = 4, or 1 for fewer
+// than four offsets, where threads in flight count for more (544 k rows, one offset, 76 channels: 71 us
+// for 102; 119 k rows, eight offsets: avg 58 us for 78, offset by offset).
+template <int MODE, int IN, int PIECE, int G>
 __global__ void __launch_bounds__(256)
 pool_fwd_few_kernel(const void *__restrict__ features, int c, const int32_t *__restrict__ nbr, int K, int n_out,
                     const int32_t *__restrict__ summaryrf, float *__restrict__ out, const int32_t *__restrict__ n_out_dev) {
-  const uint32_t cg = (uint32_t)(c / VEC);
+  const uint32_t cg = (uint32_t)(c + 3) / 4;
   const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
   if (t >= (long long)live_rows(n_out, n_out_dev) * cg) return;
   const int o = t < 0x7fffffffll ? (int)((uint32_t)t / cg) : (int)(t / cg);
-  const int c0 = (int)(t - (long long)o * cg) * VEC;
-  int src[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) src[k] = k < K ? __ldg(nbr + (size_t)k * n_out + o) : -1;
-  float acc[VEC];
-#pragma unroll
-  for (int q = 0; q < VEC; ++q) acc[q] = 0.f;
+  const int c0 = (int)(t - (long long)o * cg) * 4, valid = c - c0;
   const float div = MODE == 1 ? (summaryrf ? (float)__ldg(summaryrf + o) : (float)K) : 1.f, inv = __frcp_rn(div);
+  Channels acc = {{0.f, 0.f, 0.f, 0.f}};
+  if (G == 1) {
+    for (int k = 0; k < K; ++k) {
+      const int src = __ldg(nbr + (size_t)k * n_out + o);
+      if (src < 0) continue;
+      Channels x;
+      load_channels<IN, PIECE>(features, (size_t)src * c + c0, valid, x);
+      pool_add<MODE>(acc, x, div, inv);
+    }
+  } else {
+    int src[8];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    if (src[k] < 0) continue;
-    float v[VEC];
-    load_channels<IN, VEC>(features, (size_t)src[k] * c + c0, v);
+    for (int k = 0; k < 8; ++k) src[k] = k < K ? __ldg(nbr + (size_t)k * n_out + o) : -1;
 #pragma unroll
-    for (int q = 0; q < VEC; ++q) {
-      if (MODE == 0) acc[q] = v[q] > acc[q] ? v[q] : acc[q];
-      else acc[q] = acc[q] + divide_by_count(v[q], div, inv);
+    for (int k0 = 0; k0 < 8; k0 += G) {
+      Channels x[G];
+#pragma unroll
+      for (int k = 0; k < G; ++k)
+        if (src[k0 + k] >= 0) load_channels<IN, PIECE>(features, (size_t)src[k0 + k] * c + c0, valid, x[k]);
+#pragma unroll
+      for (int k = 0; k < G; ++k)
+        if (src[k0 + k] >= 0) pool_add<MODE>(acc, x[k], div, inv);
     }
   }
-  float *op = out + (size_t)o * c + c0;
-  if (VEC == 4) *(float4 *)op = make_float4(acc[0], acc[1 % VEC], acc[2 % VEC], acc[3 % VEC]);
-  else op[0] = acc[0];
+  store_rows<PIECE>(out + (size_t)o * c + c0, valid, acc);
 }
 
 __global__ void summary_rf_kernel(const int32_t *__restrict__ nbr, int K, int n_out, int32_t *__restrict__ rf) {
@@ -221,33 +221,37 @@ batch_offsets_small_kernel(const int4 *__restrict__ indices, int n, int batch, i
 
 using namespace ssc;
 
+template <int MODE, int IN, int PIECE>
+static int launch_pool_as(const void *features, int c, const int32_t *nbr, int K, int n_out, const int32_t *rf,
+                          float *out, const int32_t *n_out_dev, void *stream, const char *name) {
+  cudaStream_t st = as_stream(stream);
+  if (K <= 8) {
+    const int blocks = ceil_div((long long)n_out * ((c + 3) / 4), 256);
+    if (K >= 4) pool_fwd_few_kernel<MODE, IN, PIECE, 4><<<blocks, 256, 0, st>>>(features, c, nbr, K, n_out, rf, out, n_out_dev);
+    else pool_fwd_few_kernel<MODE, IN, PIECE, 1><<<blocks, 256, 0, st>>>(features, c, nbr, K, n_out, rf, out, n_out_dev);
+  } else {
+    const PoolShape p = pool_shape(n_out, K);
+    SSC_REQUIRE(p.rows > 0, "%s: kernel of %d offsets is too large", name, K);
+    if (p.smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(pool_fwd_kernel<MODE, IN, PIECE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+      if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "%s: smem attribute: %s", name, cudaGetErrorString(e));
+    }
+    pool_fwd_kernel<MODE, IN, PIECE><<<p.grid, 256, p.smem, st>>>(features, c, nbr, K, n_out, rf, out, n_out_dev, p.rows);
+  }
+  note_launches(1);
+  SSC_CHECK_LAUNCH(name);
+  return SSC_OK;
+}
+
 template <int MODE, int IN>
 static int launch_pool(const void *features, int c, const int32_t *nbr, int K, int n_out, const int32_t *rf,
                        float *out, const int32_t *n_out_dev, void *stream, const char *name) {
   SSC_REQUIRE(c > 0 && K > 0 && n_out >= 0, "%s: bad sizes", name);
   if (n_out == 0) return SSC_OK;
   SSC_REQUIRE(features && nbr && out, "%s: null pointer", name);
-  const bool vec = (c % 4 == 0) && (((uintptr_t)features | (uintptr_t)out) % 16 == 0);
-  if (K <= 8) {
-    const int blocks = ceil_div((long long)n_out * (vec ? c / 4 : c), 256);
-    if (vec) pool_fwd_few_kernel<MODE, IN, 4><<<blocks, 256, 0, as_stream(stream)>>>(features, c, nbr, K, n_out, rf, out, n_out_dev);
-    else pool_fwd_few_kernel<MODE, IN, 1><<<blocks, 256, 0, as_stream(stream)>>>(features, c, nbr, K, n_out, rf, out, n_out_dev);
-    note_launches(1);
-    SSC_CHECK_LAUNCH(name);
-    return SSC_OK;
-  }
-  const PoolShape p = pool_shape(n_out, K);
-  SSC_REQUIRE(p.rows > 0, "%s: kernel of %d offsets is too large", name, K);
-  if (p.smem > 48 * 1024) {
-    cudaError_t e = vec ? cudaFuncSetAttribute(pool_fwd_kernel<MODE, IN, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem)
-                        : cudaFuncSetAttribute(pool_fwd_kernel<MODE, IN, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
-    if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "%s: smem attribute: %s", name, cudaGetErrorString(e));
-  }
-  if (vec) pool_fwd_kernel<MODE, IN, 4><<<p.grid, 256, p.smem, as_stream(stream)>>>(features, c, nbr, K, n_out, rf, out, n_out_dev, p.rows);
-  else pool_fwd_kernel<MODE, IN, 1><<<p.grid, 256, p.smem, as_stream(stream)>>>(features, c, nbr, K, n_out, rf, out, n_out_dev, p.rows);
-  note_launches(1);
-  SSC_CHECK_LAUNCH(name);
-  return SSC_OK;
+  const int piece = pool_piece(c, (uintptr_t)features | (uintptr_t)out);
+  auto launch = piece == 4 ? launch_pool_as<MODE, IN, 4> : piece == 2 ? launch_pool_as<MODE, IN, 2> : launch_pool_as<MODE, IN, 1>;
+  return launch(features, c, nbr, K, n_out, rf, out, n_out_dev, stream, name);
 }
 
 extern "C" int ssc_maxpool_fwd(const float *features, int c, const int32_t *nbr, int K, int n_out, float *out,

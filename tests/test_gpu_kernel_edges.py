@@ -18,7 +18,9 @@ def _table(nbr_rows, n_in, K, present, rng):
 @pytest.mark.parametrize("n_in,n_out,c,K,dtype", [(1, 1, 4, 1, torch.float32), (40, 33, 20, 27, torch.float32),
                                                   (500, 64, 7, 32, torch.float32), (300, 257, 36, 125, torch.float32),
                                                   (200, 65, 8, 400, torch.float32), (90, 31, 12, 27, torch.float16),
-                                                  (90, 33, 5, 8, torch.bfloat16)])
+                                                  (90, 33, 5, 8, torch.bfloat16), (50, 37, 30, 8, torch.float32),
+                                                  (60, 40, 6, 3, torch.float32), (300, 65, 38, 27, torch.float32),
+                                                  (90, 33, 10, 27, torch.float16), (90, 40, 30, 2, torch.bfloat16)])
 def test_pools_at_tile_edges(cuda, n_in, n_out, c, K, dtype):
     """Pools over arbitrary tables: rows around the 32 of a block, more offsets than a mask word, channels that are no
     multiple of four, rows stored in 16 bits.  Quotients are correctly rounded (zeros, tiny, huge and infinite
