@@ -50,6 +50,14 @@ unsigned long long ssc_kernel_launches(void);
 /* out[i] = *words[i] for n int32 device words, read after everything queued on `stream` so far; waits
  * for them.  (The reference reads counts back with .item() / .cpu().) */
 int ssc_read_words(const int32_t *const *words, int n, int32_t *out, void *stream);
+/* A row count posted to the host by the kernel that finds it, so that whoever needs it waits for that kernel
+ * and not for all that was queued since.  ssc_count_open: a mapped place for one count (NULL: none to be had), to be
+ * handed to ssc_rulebook_conv_ahead or ssc_layer once, never while a graph is recorded.  ssc_count_wait:
+ * out = {count, status word at that time, 1}, or {0, 0, 0} where everything on `stream` is done and no count has
+ * come (it was posted on another stream, or not at all); the place stays open.  ssc_count_close gives it back. */
+void *ssc_count_open(void);
+int ssc_count_wait(void *place, int *out, void *stream);
+int ssc_count_close(void *place);
 /* 1 if the tcgen05 tensor-core kernels were compiled in (always for sm_100a builds). */
 int ssc_has_tcgen05(void);
 
@@ -140,11 +148,11 @@ int ssc_rulebook_conv_fill(const int32_t *indices, int n_in, int batch, const in
                            int32_t *indice_num, int32_t *status, void *scratch,
                            size_t scratch_bytes, const int32_t *n_out_dev, void *stream);
 /* Both phases back to back with the capacity n_out, without pair lists: the exact count stays in n_out_dev (fewer
- * launches than the two calls). */
+ * launches than the two calls).  place: of ssc_count_open, or NULL. */
 int ssc_rulebook_conv_ahead(const int32_t *indices, int n_in, int batch, const int in_shape[3], const int out_shape[3],
                             const int ksize[3], const int stride[3], const int padding[3], const int dilation[3],
                             int transpose, int n_out, int32_t *out_indices, int32_t *nbr, int32_t *n_out_dev,
-                            int32_t *status, void *scratch, size_t scratch_bytes, const int32_t *n_in_dev, void *stream);
+                            int32_t *status, void *scratch, size_t scratch_bytes, const int32_t *n_in_dev, void *place, void *stream);
 
 /* Neighbour table from a reference-format rulebook (indicePairs [K,2,n_cols], indiceNum [K]):
  * nbr[kappa][pairs[kappa][1-swap][i]] = pairs[kappa][swap][i].  swap = 1 is the "inverse"
@@ -299,7 +307,7 @@ typedef struct ssc_layer {
   int32_t *status;
   void *workspace;
   size_t workspace_bytes;
-  void *stream;
+  void *place, *stream;   /* place: of ssc_count_open, or NULL */
   int n_in, n_out, batch, op, stored, c_in, c_out, precision, c_keep, scalar_act, gate_act, out_precision, transpose;
   int in_shape[3], out_shape[3], ksize[3], stride[3], padding[3], dilation[3];
 } ssc_layer;

@@ -80,4 +80,22 @@ inline uint32_t hash_buckets_for(int n) {
 int bitmap_decode(const uint32_t *bitmap, const uint32_t *word_prefix, long long n_words, const int shape[3],
                   int n_out, int32_t *out_indices, cudaStream_t st);
 
+// A count for the host (ssc_count_open): status word and count, then the number the host watches for.
+struct CountPost {
+  int32_t *host;        // null: nobody asked
+  int32_t seq;
+};
+CountPost next_post(void *place);
+void launch_post(const CountPost &post, const int32_t *n_dev, const int32_t *status, cudaStream_t st);
+
+#ifdef __CUDACC__
+static __device__ __forceinline__ void post_count(const CountPost &post, int32_t count, const int32_t *status) {
+  volatile int32_t *dst = post.host;
+  dst[1] = status != nullptr ? *(const volatile int32_t *)status : 0;
+  dst[2] = count;
+  __threadfence_system();
+  dst[0] = post.seq;
+}
+#endif
+
 }  // namespace ssc

@@ -45,12 +45,6 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
                 const int32_t *nbr, int n_out, float *out, int32_t *status, void *scratch, size_t scratch_bytes,
                 const int32_t *n_out_dev, const int32_t *order, bool prestaged, int table_form, const GateEpilogue &gate, cudaStream_t st);
 
-// ssc_rulebook_conv_count and ssc_rulebook_conv_fill with the capacity n_out, back to back (ssc_rulebook.cu)
-int rulebook_conv_ahead(const int32_t *indices, int n_in, int batch, const int in_shape[3], const int out_shape[3], const int ksize[3],
-                        const int stride[3], const int padding[3], const int dilation[3], int transpose, int n_out,
-                        int32_t *out_indices, int32_t *nbr, int32_t *n_out_dev, int32_t *status, void *scratch, size_t scratch_bytes,
-                        const int32_t *n_in_dev, cudaStream_t st);
-
 // compacted per-offset pair lists of a neighbour table (ssc_wgrad_tc.cu): the lists of the kernel
 // offsets follow one another in pair_out / pair_in (ascending output row inside an offset),
 // starts[kappa] .. starts[kappa + 1] is the range of offset kappa, starts[K] the number of pairs.

@@ -1,5 +1,6 @@
 // Error reporting, identification and the read-back of device words.
 #include <stdarg.h>
+#include <deque>
 #include <mutex>
 #include <vector>
 #if defined(__x86_64__)
@@ -99,8 +100,90 @@ int read_some(const int32_t *const *words, int n, int32_t *out, cudaStream_t st)
   give_slot(s);
   return SSC_OK;
 }
+
+// Places for posted counts.  A place that was given back may still be written by a kernel that nobody waited for: it is
+// taken again only when its last number has arrived, the longest given back first.
+struct CountPlace {
+  int32_t *host;      // [number, status, count]
+  int32_t seq;        // number of the last post
+};
+std::mutex g_places_lock;
+std::deque<CountPlace *> g_places;
+constexpr int kPlacesPerPage = 64;
+
+bool arrived(const CountPlace *p) { return __atomic_load_n(p->host, __ATOMIC_ACQUIRE) == p->seq; }
+
+__global__ void post_count_kernel(const int32_t *n_dev, const int32_t *status, CountPost post) {
+  post_count(post, *n_dev, status);
+}
 }  // namespace
+
+CountPost next_post(void *place) {
+  CountPlace *p = (CountPlace *)place;
+  if (p == nullptr) return {nullptr, 0};
+  p->seq = p->seq == 0x7fffffff ? 1 : p->seq + 1;
+  return {p->host, p->seq};
+}
+
+void launch_post(const CountPost &post, const int32_t *n_dev, const int32_t *status, cudaStream_t st) {
+  if (post.host == nullptr) return;
+  post_count_kernel<<<1, 1, 0, st>>>(n_dev, status, post);
+  note_launches(1);
+}
 }  // namespace ssc
+
+extern "C" void *ssc_count_open(void) {
+  using namespace ssc;
+  std::lock_guard<std::mutex> hold(g_places_lock);
+  for (size_t tries = g_places.size() < 4 ? g_places.size() : 4; tries > 0; --tries) {
+    CountPlace *p = g_places.front();
+    g_places.pop_front();
+    if (arrived(p)) return p;
+    g_places.push_back(p);
+  }
+  char *page = nullptr;
+  if (cudaHostAlloc((void **)&page, kPlacesPerPage * 64, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  memset(page, 0, kPlacesPerPage * 64);
+  for (int i = 0; i < kPlacesPerPage; ++i) g_places.push_front(new CountPlace{(int32_t *)(page + 64 * i), 0});
+  CountPlace *p = g_places.front();
+  g_places.pop_front();
+  return p;
+}
+
+extern "C" int ssc_count_wait(void *place, int *out, void *stream) {
+  using namespace ssc;
+  SSC_REQUIRE(place && out, "count_wait: null pointer");
+  const CountPlace *p = (const CountPlace *)place;
+  out[0] = out[1] = out[2] = 0;
+  for (unsigned spin = 1; !arrived(p); ++spin) {
+#if defined(__x86_64__)
+    _mm_pause();
+#endif
+    if ((spin & 0x3ffu) != 0) continue;
+    const cudaError_t e = cudaStreamQuery(as_stream(stream));
+    if (e == cudaErrorNotReady) {
+      (void)cudaGetLastError();
+    } else if (e != cudaSuccess) {
+      return fail(SSC_ERR_CUDA, "count_wait: %s", cudaGetErrorString(e));
+    } else if (!arrived(p)) {
+      return SSC_OK;
+    }
+  }
+  out[0] = p->host[2];
+  out[1] = p->host[1];
+  out[2] = 1;
+  return SSC_OK;
+}
+
+extern "C" int ssc_count_close(void *place) {
+  SSC_REQUIRE(place, "count_close: null pointer");
+  std::lock_guard<std::mutex> hold(ssc::g_places_lock);
+  ssc::g_places.push_back((ssc::CountPlace *)place);
+  return SSC_OK;
+}
 
 extern "C" int ssc_read_words(const int32_t *const *words, int n, int32_t *out, void *stream) {
   SSC_REQUIRE(n >= 0 && (n == 0 || (words && out)), "read_words: bad arguments");

@@ -51,7 +51,7 @@ extern "C" int ssc_layer_ahead(const ssc_layer *layer) {
   int32_t *nbr = (int32_t *)(ws + s.table);
   const int K = a.ksize[0] * a.ksize[1] * a.ksize[2];
   int rc = ssc_rulebook_conv_ahead(a.indices, a.n_in, a.batch, a.in_shape, a.out_shape, a.ksize, a.stride, a.padding, a.dilation, a.transpose,
-                                   a.n_out, a.out_indices, nbr, a.n_out_dev, a.status, ws, s.rulebook_bytes, a.n_in_dev, a.stream);
+                                   a.n_out, a.out_indices, nbr, a.n_out_dev, a.status, ws, s.rulebook_bytes, a.n_in_dev, a.place, a.stream);
   if (rc != SSC_OK) return rc;
   if (a.op != 0) {
     if (a.stored != 0) return ssc_pool_fwd16(a.features, a.stored, a.op == 2, a.c_in, nbr, K, a.n_out, nullptr, (float *)a.out, a.n_out_dev, a.stream);

@@ -10,6 +10,7 @@ variants of convolution and pools); only the functions the reference's own Pytho
 """
 import ctypes
 import os
+import threading
 
 import torch
 
@@ -34,7 +35,7 @@ class Layer(ctypes.Structure):
     """ssc_layer of the C header."""
     _fields_ = ([(n, c_void_p) for n in ("indices", "n_in_dev", "out_indices", "n_out_dev", "features", "filters", "scale",
                                          "shift", "gate_of_channel", "out", "status", "workspace")]
-                + [("workspace_bytes", c_size_t), ("stream", c_void_p)]
+                + [("workspace_bytes", c_size_t), ("place", c_void_p), ("stream", c_void_p)]
                 + [(n, c_int) for n in ("n_in", "n_out", "batch", "op", "stored", "c_in", "c_out", "precision", "c_keep",
                                         "scalar_act", "gate_act", "out_precision", "transpose")]
                 + [(n, _I3) for n in ("in_shape", "out_shape", "ksize", "stride", "padding", "dilation")])
@@ -47,6 +48,9 @@ SIGNATURES = {
     "ssc_has_tcgen05": (c_int, []),
     "ssc_kernel_launches": (ctypes.c_ulonglong, []),
     "ssc_read_words": (c_int, [ctypes.POINTER(c_void_p), c_int, ctypes.POINTER(c_int), c_void_p]),
+    "ssc_count_open": (c_void_p, []),
+    "ssc_count_wait": (c_int, [c_void_p, ctypes.POINTER(c_int), c_void_p]),
+    "ssc_count_close": (c_int, [c_void_p]),
     "ssc_rulebook_scratch_bytes": (c_size_t, [c_int, c_int, _I3, _I3, c_int]),
     "ssc_rulebook_subm": (c_int, [c_void_p, c_int, c_int, _I3, _I3, _I3, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_void_p, c_size_t, c_void_p]),
@@ -59,7 +63,7 @@ SIGNATURES = {
     "ssc_rulebook_conv_fill": (c_int, [c_void_p, c_int, c_int, _I3, _I3, _I3, _I3, _I3, _I3, c_int, c_int, c_void_p, c_void_p,
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "ssc_rulebook_conv_ahead": (c_int, [c_void_p, c_int, c_int, _I3, _I3, _I3, _I3, _I3, _I3, c_int, c_int, c_void_p, c_void_p,
-                                        c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
+                                        c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p, c_void_p]),
     "ssc_pairs_to_nbr": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "ssc_pairs_from_nbr_scratch_bytes": (c_size_t, [c_int, c_int]),
     "ssc_pairs_from_nbr": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
@@ -307,6 +311,47 @@ def read_counts(words):
     One small kernel writes the words into mapped host memory and the host watches for them there: a
     copy engine and a stream synchronisation per read cost several times as much."""
     dev = words[0].device
+    posted = [getattr(w, "_ssc_post", None) for w in words]
+    rest = [w for w, p in zip(words, posted) if p is None]
+    if len(rest) == len(words):
+        return _read_words(words, dev)
+    # counts that their kernels post themselves: no waiting for what was queued behind those
+    others = iter(_read_words(rest, dev) if rest else ())
+    values = [next(others) if p is None else p.wait(dev) for p in posted]
+    return [_read_words([w], dev)[0] if v is None else v for w, v in zip(words, values)]
+
+
+class CountPost(object):
+    """A place in mapped host memory to which the kernel that finds a row count posts it (ssc_count_open), and
+    the value once it has come.  What the status word reports after that kernel surfaces with the next count
+    that is read, as it does behind layers on exact rows."""
+
+    __slots__ = ("place", "value", "lock")
+
+    def __init__(self):
+        self.place, self.value, self.lock = lib().ssc_count_open(), None, threading.Lock()
+
+    def wait(self, device):
+        """The count, or None where it has to be read from its device word."""
+        with self.lock:
+            if self.value is None and self.place:
+                out = (c_int * 3)()
+                _check(lib().ssc_count_wait(self.place, out, _stream()))
+                if out[2]:
+                    self.value = out[0]
+                    self._close()
+                    raise_on_status(out[1], device)
+            return self.value
+
+    def _close(self):
+        place, self.place = self.place, None
+        if place and lib is not None:
+            lib().ssc_count_close(place)
+
+    __del__ = _close
+
+
+def _read_words(words, dev):
     n = len(words) + 1
     ptrs = (c_void_p * n)(*[_p(w, torch.int32) for w in words], _p(status_word(dev)))
     out = (c_int * n)()
@@ -442,8 +487,9 @@ def get_indice_pairs_ahead(indices, batch_size, out_shape, spatial_shape, ksize,
         _check(L.ssc_rulebook_conv_fill(_p(indices), n_in, int(batch_size), *geo, cap, _p(outids), _p(nbr), None, None,
                                         _p(st), _p(scratch), sbytes, _p(n_out_dev), _stream()))
     else:
+        post = n_out_dev._ssc_post = CountPost()
         _check(L.ssc_rulebook_conv_ahead(_p(indices), n_in, int(batch_size), *geo, cap, _p(outids), _p(nbr), _p(n_out_dev), _p(st),
-                                         _p(scratch), sbytes, _p(n_in_dev), _stream()))
+                                         _p(scratch), sbytes, _p(n_in_dev), post.place, _stream()))
     pairs = LazyPairs(nbr, n_in, n_out_dev=n_out_dev, ratio_key=None if n_in_dev is not None else key)
     pairs.regular = True
     return [outids, pairs, None]
@@ -515,6 +561,8 @@ def layer_ahead(plan, indices, n_in_dev, features, weight=None, gate=None):
     nbytes = L.ssc_layer_ahead_bytes(at)
     ws = _empty(nbytes, torch.uint8, dev)
     a.out_indices, a.n_out_dev, a.out = outids.data_ptr(), n_out_dev.data_ptr(), out.data_ptr()
+    post = n_out_dev._ssc_post = CountPost()
+    a.place = post.place
     a.workspace, a.workspace_bytes, a.status, a.stream = ws.data_ptr(), nbytes, status_word(dev).data_ptr(), _stream()
     _check(L.ssc_layer_ahead(at))
     return out, outids, n_out_dev, cap

@@ -100,3 +100,36 @@ def test_inverse_convolution_behind_a_pending_partner(cuda, overflow):
     _ext.check_status(cuda)
     assert torch.equal(got[1], want[1]) and torch.equal(got[0], want[0])
     assert torch.equal(got[2][0], want[2][0]) and torch.equal(got[2][1], want[2][1])
+
+
+@pytest.mark.parametrize("batch,grid,per", [(1, 4, 1), (2, 32, 500), (2, 200, 3000)])
+def test_counts_are_posted_before_what_is_queued_behind_them(cuda, batch, grid, per):
+    """The count of a strided layer arrives without waiting for the work behind it (bitmaps of one word, of one launch
+    and beyond the 32 k words of one), through places of which many were given up unread, and again
+    where the reading stream is not the one it was posted on."""
+    from ss_conv import _ext
+    from ss_conv.pool import MaxPool
+    from ss_conv.sp_ops.tensor import SparseTensor
+    rng = np.random.RandomState(grid)
+    inds = dev(random_voxels(rng, batch, grid, per), cuda)
+    feats = torch.randn(inds.shape[0], 8, device=cuda)
+    pool = MaxPool(2, stride=2)
+    want = torch.unique(torch.cat([inds[:, :1], inds[:, 1:] // 2], 1), dim=0)
+    with torch.no_grad():
+        pool(SparseTensor(feats, inds, [grid] * 3, batch)).features      # the first call learns the ratio
+        for _ in range(200):
+            pool(SparseTensor(feats, inds, [grid] * 3, batch))           # nobody looks
+        y = pool(SparseTensor(feats, inds, [grid] * 3, batch))
+        torch.cuda._sleep(100000000)                                     # some 50 ms
+        behind = torch.cuda.Event()
+        behind.record()
+        n = y.features.shape[0]
+        early = not behind.query()
+        assert n == want.shape[0] and torch.equal(y.indices, want.int())
+        assert early or not _ext.AHEAD
+        z = pool(SparseTensor(feats, inds, [grid] * 3, batch))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            assert z.features.shape[0] == n
+        assert torch.equal(z.features, y.features)
+    _ext.check_status(cuda)
