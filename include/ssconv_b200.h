@@ -58,6 +58,8 @@ int ssc_read_words(const int32_t *const *words, int n, int32_t *out, void *strea
 void *ssc_count_open(void);
 int ssc_count_wait(void *place, int *out, void *stream);
 int ssc_count_close(void *place);
+/* Posts *n_dev (and *status) to a place from a kernel of its own, behind what is queued on `stream`. */
+int ssc_count_post(const int32_t *n_dev, const int32_t *status, void *place, void *stream);
 /* 1 if the tcgen05 tensor-core kernels were compiled in (always for sm_100a builds). */
 int ssc_has_tcgen05(void);
 

@@ -178,6 +178,13 @@ extern "C" int ssc_count_wait(void *place, int *out, void *stream) {
   return SSC_OK;
 }
 
+extern "C" int ssc_count_post(const int32_t *n_dev, const int32_t *status, void *place, void *stream) {
+  SSC_REQUIRE(n_dev && place, "count_post: null pointer");
+  ssc::launch_post(ssc::next_post(place), n_dev, status, ssc::as_stream(stream));
+  SSC_CHECK_LAUNCH("count_post");
+  return SSC_OK;
+}
+
 extern "C" int ssc_count_close(void *place) {
   SSC_REQUIRE(place, "count_close: null pointer");
   std::lock_guard<std::mutex> hold(ssc::g_places_lock);

@@ -51,6 +51,7 @@ SIGNATURES = {
     "ssc_count_open": (c_void_p, []),
     "ssc_count_wait": (c_int, [c_void_p, ctypes.POINTER(c_int), c_void_p]),
     "ssc_count_close": (c_int, [c_void_p]),
+    "ssc_count_post": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p]),
     "ssc_rulebook_scratch_bytes": (c_size_t, [c_int, c_int, _I3, _I3, c_int]),
     "ssc_rulebook_subm": (c_int, [c_void_p, c_int, c_int, _I3, _I3, _I3, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_void_p, c_size_t, c_void_p]),
@@ -1505,6 +1506,10 @@ def point2voxel(points, feats, batch_ids, batch_size, grid, unit, mode, ahead=Fa
     unit3 = _F3(*[float(u) for u in unit])
     _check(L.ssc_p2v_count(_p(points), _p(batch_ids), n, int(batch_size), _i3(grid), unit3, _p(m_dev), _p(st),
                            _p(scratch), scratch.numel(), _stream()))
+    if ahead and not torch.cuda.is_current_stream_capturing():
+        post = m_dev._ssc_post = CountPost()
+        if post.place:
+            _check(L.ssc_count_post(_p(m_dev), _p(st), post.place, _stream()))
     m = n if ahead else read_count(m_dev)
     vox = _empty((m, 4), torch.int32, dev)
     inverse = _empty(n, torch.int32, dev)
