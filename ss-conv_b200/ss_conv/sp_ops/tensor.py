@@ -229,18 +229,23 @@ def run_ahead(layer, input, op, output_shape, transpose, exact, weight=None, gat
     if not (feats.is_contiguous() and inds.is_contiguous()):
         return None
     shape = tuple(input.spatial_shape)          # (a list, or an array)
-    key = (shape, input.batch_size, feats.dtype, _ext._precision, _ext._storage, gate[3:] if gate is not None else None)
+    c_in, c_out = (weight.shape[-2], weight.shape[-1]) if weight is not None else (feats.shape[1], 0)
+    if feats.shape[1] != c_in:
+        return None
+    # everything a plan is made from: one pool may serve rows of several widths, a layer's geometry may be changed
+    gated = gate[3:] if gate is not None else None
+    key = (shape, input.batch_size, feats.dtype, _ext._precision, _ext._storage, gated, c_in, c_out, transpose, *layer.kernel_size,
+           *layer.stride, *layer.padding, *layer.dilation, *getattr(layer, "output_padding", ()))
     plans = layer.__dict__.setdefault("_ahead_plans", {})
     plan = plans.get(key)
     if plan is None:
         if len(plans) > 64:
             plans.clear()
-        c_in, c_out = (weight.shape[-2], weight.shape[-1]) if weight is not None else (feats.shape[1], 0)
         out_shape = output_shape(input.spatial_shape)
         plan = plans[key] = (_ext.layer_plan(shape, out_shape, input.batch_size, layer.kernel_size, layer.stride, layer.padding,
-                                             layer.dilation, transpose, op, feats.dtype, c_in, c_out, key[-1]), tuple(out_shape))
+                                             layer.dilation, transpose, op, feats.dtype, c_in, c_out, gated), tuple(out_shape))
     plan, out_shape = plan
-    if plan is None or (weight is not None and feats.shape[1] != weight.shape[-2]):
+    if plan is None:
         return None
     made = _ext.layer_ahead(plan, inds, n_in_dev, feats, weight, gate)
     if made is None:

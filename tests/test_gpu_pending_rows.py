@@ -133,3 +133,27 @@ def test_counts_are_posted_before_what_is_queued_behind_them(cuda, batch, grid, 
             assert z.features.shape[0] == n
         assert torch.equal(z.features, y.features)
     _ext.check_status(cuda)
+
+
+@pytest.mark.parametrize("widths", [(76, 16, 76), (16, 76, 5)])
+def test_one_pool_serves_rows_of_several_widths(cuda, widths):
+    """A pool has no parameters: networks share one between stages.  Every call against the exact path, the row ratio
+    known from the first on."""
+    from ss_conv import _ext
+    from ss_conv.pool import AvgPool
+    from ss_conv.sp_ops.tensor import SparseTensor
+    rng = np.random.RandomState(5)
+    inds = dev(random_voxels(rng, 2, 20, 900), cuda)
+    pool = AvgPool(3, stride=2, padding=1)
+    with torch.no_grad():
+        for c in widths:
+            x = SparseTensor(torch.randn(inds.shape[0], c, device=cuda), inds, [20] * 3, 2)
+            ahead, _ext.AHEAD = _ext.AHEAD, False
+            try:
+                want = pool(x)
+            finally:
+                _ext.AHEAD = ahead
+            got = pool(x)
+            assert got.pending() == _ext.AHEAD
+            assert torch.equal(got.features, want.features) and torch.equal(got.indices, want.indices)
+    _ext.check_status(cuda)

@@ -56,6 +56,32 @@ def test_layer_structure_has_the_size_of_the_librarys():
     assert _ext.lib().ssc_layer_struct_bytes() == ctypes.sizeof(_ext.Layer)
 
 
+def test_plans_of_layers_that_run_ahead_follow_their_input(monkeypatch):
+    """One pool on rows of several widths, and a layer whose geometry is changed: the plan handed to the library has the
+    present channel counts and sizes."""
+    from ss_conv import _ext
+    from ss_conv.pool import MaxPool
+    from ss_conv.sp_ops.conv import SparseConvolution
+    from ss_conv.sp_ops.tensor import SparseTensor, run_ahead
+    seen = []
+
+    def layer_ahead(plan, inds, n_in_dev, feats, weight=None, gate=None):
+        seen.append((_ext.Layer.from_buffer_copy(plan[0]), plan[5]))
+
+    monkeypatch.setattr(_ext, "layer_ahead", layer_ahead)
+    pool = MaxPool(2, stride=2)
+    for c in (64, 32, 64, 7):
+        run_ahead(pool, SparseTensor(torch.zeros(10, c), torch.zeros(10, 4, dtype=torch.int32), [8] * 3, 1), 1,
+                  lambda _: [4] * 3, 0, None)
+    assert [(a.c_in, c_row) for a, c_row in seen] == [(64, 64), (32, 32), (64, 64), (7, 7)]
+    conv = SparseConvolution(3, 16, 8, 3, stride=2, padding=1, bias=False)
+    for weight, stride in ((conv.weight, 2), (torch.zeros(3, 3, 3, 16, 24), 2), (conv.weight, 1)):
+        conv.stride = [stride] * 3
+        run_ahead(conv, SparseTensor(torch.zeros(10, 16), torch.zeros(10, 4, dtype=torch.int32), [8] * 3, 1), 0,
+                  conv._output_shape, 0, None, weight)
+    assert [(a.c_out, c_row, a.stride[0], a.out_shape[2]) for a, c_row in seen[4:]] == [(8, 8, 2, 4), (24, 24, 2, 4), (8, 8, 1, 8)]
+
+
 def test_argument_errors_without_gpu():
     """Size queries and argument validation run on the host only."""
     from ss_conv import _ext
