@@ -549,7 +549,7 @@ def layer_ahead(plan, indices, n_in_dev, features, weight=None, gate=None):
     if weight is not None:
         flt = _flat_filters(weight)
         packed = _packed_filters(flt, prec) if prec != PREC_FP32 else flt
-        a.filters = _p(packed)
+        a.filters = _p(packed, torch.float32 if prec == PREC_FP32 else torch.uint8)
         if gate is not None:
             if gate[0] is not None:
                 a.scale, a.shift = _p(gate[0]), _p(gate[1])

@@ -177,7 +177,7 @@ class SparseConvolution(nn.Module):
         apply."""
         cached = input.find_indice_pair(self.indice_key)
         if (cached is None or not isinstance(cached[2], _ext.LazyPairs) or not cached[2].regular or not cached[2].pending()
-                or cached[0] is not inds or not feats.is_cuda or feats.dtype not in _FEATURE_DTYPES
+                or cached[0] is not inds or not feats.is_cuda or feats.dtype not in _FEATURE_DTYPES or weight.dtype != torch.float32
                 or torch.cuda.is_current_stream_capturing()
                 or (torch.is_grad_enabled() and (feats.requires_grad or weight.requires_grad))):
             return None

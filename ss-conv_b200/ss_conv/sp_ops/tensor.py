@@ -226,8 +226,8 @@ def run_ahead(layer, input, op, output_shape, transpose, exact, weight=None, gat
     kernel_size, stride, padding, dilation; it keeps the plans); op as in _ext.layer_plan; output_shape(shape)
     gives the spatial shape of its output, exact(input, ...) recomputes the layer on exact row counts."""
     feats, inds, n_in_dev = input.raw()
-    if not (feats.is_contiguous() and inds.is_contiguous()):
-        return None
+    if not (feats.is_contiguous() and inds.is_contiguous()) or (weight is not None and weight.dtype != torch.float32):
+        return None                             # (16-bit filters have entry points of their own)
     shape = tuple(input.spatial_shape)          # (a list, or an array)
     c_in, c_out = (weight.shape[-2], weight.shape[-1]) if weight is not None else (feats.shape[1], 0)
     if feats.shape[1] != c_in:

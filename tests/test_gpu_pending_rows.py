@@ -157,3 +157,39 @@ def test_one_pool_serves_rows_of_several_widths(cuda, widths):
             assert got.pending() == _ext.AHEAD
             assert torch.equal(got.features, want.features) and torch.equal(got.indices, want.indices)
     _ext.check_status(cuda)
+
+
+def test_half_filters_keep_their_entry_points(cuda):
+    """Half rows and half filters go through indice_conv_half whether or not the row ratio is known, strided and inverse;
+    half filters on fp32 rows are refused (never read as fp32)."""
+    from ss_conv import _ext
+    from ss_conv.sp_ops.conv import SparseConvolution
+    from ss_conv.sp_ops.tensor import SparseTensor
+    torch.manual_seed(1)
+    rng = np.random.RandomState(6)
+    inds = dev(random_voxels(rng, 2, 16, 700), cuda)
+    plain = SparseConvolution(3, 16, 24, 3, stride=2, padding=1, bias=False).to(cuda).half()
+    down = SparseConvolution(3, 16, 24, 3, stride=2, padding=1, bias=False, indice_key="k").to(cuda).half()
+    up = SparseConvolution(3, 24, 8, 3, inverse=True, bias=False, indice_key="k").to(cuda).half()
+    feats = torch.randn(inds.shape[0], 16, device=cuda)
+
+    def run(f):
+        a = plain(SparseTensor(f, inds, [16] * 3, 2))
+        b = up(down(SparseTensor(f, inds, [16] * 3, 2)))
+        return a.features, b.features
+
+    with torch.no_grad():
+        ahead, _ext.AHEAD = _ext.AHEAD, False
+        try:
+            want = run(feats.half())
+        finally:
+            _ext.AHEAD = ahead
+        for _ in range(2):
+            for got, ref in zip(run(feats.half()), want):
+                assert got.dtype == torch.half and torch.equal(got, ref)
+        few = SparseConvolution(3, 8, 8, 3, stride=2, padding=1, bias=False).to(cuda).half()
+        for layer, c in ((plain, 16), (few, 8)):
+            for _ in range(2):
+                with pytest.raises(TypeError):
+                    layer(SparseTensor(feats[:, :c].contiguous(), inds, [16] * 3, 2))
+    _ext.check_status(cuda)

@@ -80,6 +80,10 @@ def test_plans_of_layers_that_run_ahead_follow_their_input(monkeypatch):
         run_ahead(conv, SparseTensor(torch.zeros(10, 16), torch.zeros(10, 4, dtype=torch.int32), [8] * 3, 1), 0,
                   conv._output_shape, 0, None, weight)
     assert [(a.c_out, c_row, a.stride[0], a.out_shape[2]) for a, c_row in seen[4:]] == [(8, 8, 2, 4), (24, 24, 2, 4), (8, 8, 1, 8)]
+    x = SparseTensor(torch.zeros(10, 16), torch.zeros(10, 4, dtype=torch.int32), [8] * 3, 1)
+    for dtype in (torch.float16, torch.bfloat16, torch.float64):      # left to the entry points that look at the type
+        assert run_ahead(conv, x, 0, conv._output_shape, 0, None, conv.weight.to(dtype)) is None
+    assert len(seen) == 7
 
 
 def test_argument_errors_without_gpu():
