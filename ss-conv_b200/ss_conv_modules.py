@@ -8,6 +8,7 @@ import numpy as np
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from ss_conv import _ext
 from ss_conv.activation import Activation
@@ -20,6 +21,14 @@ from ss_conv.utils import SO3
 from ss_conv.utils.kernel import gaussian_window_wrapper
 
 radial_window = partial(gaussian_window_wrapper, mode="compromise", border_dist=0, sigma=0.6)
+
+
+def _unwatched(module, kind):
+    """The module is one of this package's own, and nothing waits for it to be called: what fuses it with its neighbours
+    must not pass by a subclass, a replaced forward or a hook of any kind."""
+    return (type(module) is kind and "forward" not in module.__dict__
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+            and not _has_any_global_hook())
 
 
 class SS_Conv(nn.Module):
@@ -53,13 +62,13 @@ class SS_Conv(nn.Module):
     def _inference_gate(self, x):
         """The folded batch norm and the activation for the convolution to apply as it stores its rows
         (_ext.conv_forward), or None: while gradients are recorded or statistics are taken, with biases or
-        an activation the library does not know, with hooks on the modules that would not be called."""
+        an activation the library does not know, with modules that have to be called (_unwatched)."""
         if torch.is_grad_enabled():
             return None
         parts = self._modules
         bn, act, conv = parts.get("bn"), parts.get("activation"), parts["conv"]
-        if (act is None or conv.training or conv._parameters["bias"] is not None or conv._forward_hooks or act._forward_hooks
-                or act._forward_pre_hooks or (bn is not None and (bn.training or bn._forward_hooks or bn._forward_pre_hooks))
+        if (act is None or not _unwatched(conv, Convolution) or conv.training or conv._parameters["bias"] is not None
+                or not _unwatched(act, Activation) or (bn is not None and (bn.training or not _unwatched(bn, BatchNorm)))
                 or not act.fusable_gate()):
             return None
         device = x.raw()[0].device
@@ -74,7 +83,9 @@ class SS_Conv(nn.Module):
             x = self.conv(x, gate)
             return x if self.dropout is None else self.dropout(x)
         x = self.conv(x)
-        both = self.bn.norm_and_gate(x, self.activation) if self.bn is not None and self.activation is not None else None
+        both = None
+        if _unwatched(self.bn, BatchNorm) and _unwatched(self.activation, Activation):
+            both = self.bn.norm_and_gate(x, self.activation)
         if both is not None:
             x = both
         else:

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import ssconv_oracle as O
-from gpu_helpers import dev, rel_err
+from gpu_helpers import dev, random_voxels, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -580,3 +580,43 @@ def test_eval_batchnorm_refolds_when_its_buffers_change(cuda):
         bn.weight.fill_(2.0)
     c = run()
     assert torch.allclose(c, 2.0 * b, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("training", [True, False])
+@pytest.mark.parametrize("hook", ["register_forward_hook", "register_forward_pre_hook", "global", "pre-hook of the convolution"])
+def test_hooks_inside_a_block_fire(cuda, training, hook):
+    """Hooks on a block's norm, activation and convolution, and hooks on all modules, fire in training and in inference
+    alike, and the rows are those of the block without hooks (the fused passes have the bits of the
+    single ones)."""
+    from ss_conv.sp_ops.tensor import SparseTensor
+    from ss_conv_modules import SS_Conv
+    torch.manual_seed(2)
+    block = SS_Conv((4, 4), (4, 4), 3, padding=1, subm=True, activation=(torch.relu, torch.sigmoid)).to(cuda).train(training)
+    inds = dev(random_voxels(np.random.RandomState(3), 1, 12, 300), cuda)
+    feats = torch.randn(inds.shape[0], 16, device=cuda)
+
+    def run():
+        state = {k: v.clone() for k, v in block.state_dict().items()}
+        with torch.set_grad_enabled(training):
+            y = block(SparseTensor(feats.clone().requires_grad_(training), inds, [12] * 3, 1)).features
+            if training:
+                y.sum().backward()
+        block.load_state_dict(state)
+        return y.detach()
+
+    want, seen = run(), set()
+    if hook == "global":
+        handles = [torch.nn.modules.module.register_module_forward_hook(lambda m, a, y: seen.add(m) and None)]
+        got = run()
+        assert {block.conv, block.bn, block.activation} <= seen
+    elif hook.startswith("pre-hook"):
+        handles = [block.conv.register_forward_pre_hook(lambda m, a: seen.add(len(a)) or a[0])]
+        got = run()
+        assert seen == {1}
+    else:
+        handles = [getattr(m, hook)(lambda m, *a: seen.add(m) and None) for m in (block.bn, block.activation)]
+        got = run()
+        assert seen == {block.bn, block.activation}
+    for h in handles:
+        h.remove()
+    assert torch.equal(got, want)

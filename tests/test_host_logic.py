@@ -86,6 +86,28 @@ def test_plans_of_layers_that_run_ahead_follow_their_input(monkeypatch):
     assert len(seen) == 7
 
 
+def test_a_block_calls_submodules_that_were_replaced():
+    """Foreign modules in the place of a block's own are called, with and without recorded gradients."""
+    import torch.nn as nn
+    from ss_conv_modules import SS_Conv
+    calls = []
+
+    class Foreign(nn.Module):
+        def forward(self, x):
+            calls.append(self)
+            return x + 1
+
+    for mode in (True, False):
+        for name in ("bn", "activation"):
+            block = SS_Conv((2, 2), (2, 2), 3, padding=1, activation=(torch.relu, torch.sigmoid)).train(mode)
+            block.conv = Foreign()
+            block.bn = block.activation = Foreign()
+            setattr(block, name, None)
+            with torch.set_grad_enabled(mode):
+                assert float(block(torch.zeros(1))) == 2
+    assert len(calls) == 8
+
+
 def test_argument_errors_without_gpu():
     """Size queries and argument validation run on the host only."""
     from ss_conv import _ext
