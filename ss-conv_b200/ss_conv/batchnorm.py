@@ -104,7 +104,10 @@ class BatchNorm(nn.Module):
         # the fold of the running buffers is kept until one of its inputs changes (in-place updates bump
         # a tensor's version, moves and reloads change its address): an eval-mode network folds once
         running = mean is None and var is None
-        w, b = (self._parameters["weight"], self._parameters["bias"]) if self.affine else (None, None)
+        # (straight from the dictionary; replicas and parametrised modules hold them as other attributes)
+        w, b = self._parameters.get("weight"), self._parameters.get("bias")
+        if self.affine and (w is None or b is None):
+            w, b = self.weight, self.bias
         if running:
             mean, var = self._buffers["running_mean"], self._buffers["running_var"]
             key = (mean.data_ptr(), mean._version, var.data_ptr(), var._version, device, self.eps)
@@ -124,7 +127,7 @@ class BatchNorm(nn.Module):
             b = None
         folded = _ext.bn_fold(mean, var, w, b, field, scalar, self.eps)
         if key is not None:
-            self._folded = (key, folded)
+            self._folded = (key, folded, (mean, var, w, b))     # (held, so that no other tensor takes their addresses)
         return folded
 
     def _running(self):

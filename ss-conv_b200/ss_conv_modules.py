@@ -67,7 +67,7 @@ class SS_Conv(nn.Module):
             return None
         parts = self._modules
         bn, act, conv = parts.get("bn"), parts.get("activation"), parts["conv"]
-        if (act is None or not _unwatched(conv, Convolution) or conv.training or conv._parameters["bias"] is not None
+        if (act is None or not _unwatched(conv, Convolution) or conv.training or conv.bias is not None
                 or not _unwatched(act, Activation) or (bn is not None and (bn.training or not _unwatched(bn, BatchNorm)))
                 or not act.fusable_gate()):
             return None

@@ -108,6 +108,39 @@ def test_a_block_calls_submodules_that_were_replaced():
     assert len(calls) == 8
 
 
+def test_folded_norms_of_replicas_and_parametrised_modules(monkeypatch):
+    """Affine parameters that are not in the module's own dictionary: replicas of torch.nn.DataParallel, parametrised
+    weights."""
+    import torch.nn as nn
+    from ss_conv import _ext
+    from ss_conv.batchnorm import BatchNorm
+    from ss_conv.convolution import Convolution
+    from ss_conv_modules import SS_Conv
+    monkeypatch.setattr(_ext, "bn_fold", lambda mean, var, w, b, field, scalar, eps: (w.clone(), b.clone()))
+    bn = BatchNorm([(2, 0), (1, 1)])
+    replica = bn._replicate_for_data_parallel()
+    replica.weight, replica.bias = torch.full((3,), 2.0), torch.full((2,), 3.0)
+    w, b = replica.folded_affine(torch.device("cpu"))
+    assert w.tolist() == [2.0] * 3 and b.tolist() == [3.0] * 2
+
+    class Twice(nn.Module):
+        def forward(self, x):
+            return 2 * x
+
+    nn.utils.parametrize.register_parametrization(bn, "weight", Twice())
+    for k in range(4):            # (every look at the weight is a new tensor, often where the last one was)
+        with torch.no_grad():
+            bn.parametrizations.weight.original.fill_(1.0 + k)
+            assert bn.folded_affine(torch.device("cpu"))[0].tolist() == [2.0 + 2 * k] * 3
+    block = SS_Conv((2, 2), (2, 2), 3, padding=1, activation=(torch.relu, torch.sigmoid), bias=True).eval()
+    replica = block._replicate_for_data_parallel()
+    replica._modules = dict(block._modules, conv=block.conv._replicate_for_data_parallel())
+    replica.conv.bias = block.conv.bias.detach()
+    assert type(replica.conv) is Convolution
+    with torch.no_grad():
+        assert replica._inference_gate(None) is None          # a bias: the gate cannot be applied by the convolution
+
+
 def test_argument_errors_without_gpu():
     """Size queries and argument validation run on the host only."""
     from ss_conv import _ext
