@@ -35,8 +35,7 @@ class _BatchNormFn(torch.autograd.Function):
         w = None if weight is None else weight.detach().contiguous()
         b = None if (bias is None or n_scalar == 0) else bias.detach().contiguous()
         if training:
-            mean, var, chan_mean, scale, shift = _ext.bn_train(x, field, scalar, n_field, n_scalar, w, b, module.eps,
-                                                               module.momentum, *module._running())
+            mean, var, chan_mean, scale, shift = module._batch_statistics(x, field, scalar, w, b)
         else:
             mean, var, chan_mean = module.running_mean.clone(), module.running_var.clone(), None
             scale, shift = _ext.bn_fold(mean if n_scalar > 0 else None, var, w, b, field, scalar, module.eps)
@@ -130,10 +129,19 @@ class BatchNorm(nn.Module):
             self._folded = (key, folded, (mean, var, w, b))     # (held, so that no other tensor takes their addresses)
         return folded
 
-    def _running(self):
-        """The running buffers for an in-place update by the library."""
+    def _batch_statistics(self, x, field, scalar, w, b):
+        """_ext.bn_train of rows x; the running buffers are updated by the library where they are what its kernels write,
+        else (a module in another floating-point type) by the torch operations."""
         self._folded = None
-        return (self.running_mean if self.running_mean.numel() else None), self.running_var
+        mean, var = self.running_mean, self.running_var
+        direct = all(t.dtype == torch.float32 and t.device == x.device and t.is_contiguous() for t in (mean, var))
+        out = _ext.bn_train(x, field, scalar, var.numel(), mean.numel(), w, b, self.eps, self.momentum,
+                            *((mean if mean.numel() else None, var) if direct else (None, None)))
+        if not direct:
+            with torch.no_grad():
+                for running, batch in ((mean, out[0]), (var, out[1])):
+                    running.mul_(1 - self.momentum).add_(self.momentum * batch)
+        return out
 
     def _differentiable(self, x):
         """The layer as a composite of torch ops, used while autograd is recording so that
@@ -215,9 +223,7 @@ class BatchNorm(nn.Module):
             if self.reduce != 'mean':
                 raise ValueError("Invalid reduce option {}".format(self.reduce))
             w, b = (self.weight.detach(), self.bias.detach()) if self.affine else (None, None)
-            scale, shift = _ext.bn_train(x, field, scalar, self.running_var.numel(), self.running_mean.numel(), w,
-                                         b if self.running_mean.numel() else None, self.eps, self.momentum,
-                                         *self._running())[3:]
+            scale, shift = self._batch_statistics(x, field, scalar, w, b if self.running_mean.numel() else None)[3:]
         else:
             scale, shift = self.folded_affine(x.device)
 

@@ -237,3 +237,23 @@ def test_rulebook_in_one_go_equals_the_two_phases(cuda, batch, grid, per):
         assert torch.equal(outids[:rows], want[0][:rows]) and torch.equal(pairs._nbr_cap[:, :rows], want[1][:, :rows])
     _ext._ratio_hint.pop(key)
     _ext.check_status(cuda)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float64])
+@pytest.mark.parametrize("record", [True, False])
+def test_training_norm_with_running_buffers_of_another_type(cuda, dtype, record):
+    """The same rows as with fp32 buffers, and buffers that are the fp32 ones' values in their own type (one rounding of
+    each step)."""
+    from ss_conv.batchnorm import BatchNorm
+    from ss_conv.sp_ops.tensor import SparseTensor
+    Rs = [(3, 0), (2, 1)]
+    x = torch.randn(200, 9, device=cuda) + 0.3
+    outs = []
+    for t in (torch.float32, dtype):
+        bn = BatchNorm(Rs, affine=False).to(cuda).to(t)
+        with torch.set_grad_enabled(record):
+            y = bn(SparseTensor(x.clone().requires_grad_(record), torch.zeros(200, 4, dtype=torch.int32, device=cuda), [8] * 3, 1))
+        outs.append((y.features.detach(), bn.running_mean, bn.running_var))
+    assert torch.equal(outs[0][0], outs[1][0])
+    for a, b in zip(outs[0][1:], outs[1][1:]):
+        assert b.dtype == dtype and torch.allclose(a.double(), b.double(), rtol=4 * torch.finfo(torch.float16).eps if dtype == torch.float16 else 1e-6, atol=1e-4)

@@ -141,6 +141,27 @@ def test_folded_norms_of_replicas_and_parametrised_modules(monkeypatch):
         assert replica._inference_gate(None) is None          # a bias: the gate cannot be applied by the convolution
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.float64])
+def test_running_statistics_of_other_types_stay_with_torch(monkeypatch, dtype):
+    """Only fp32 buffers are handed to the library, which writes fp32; others take torch's own update, and take it once."""
+    from ss_conv import _ext
+    from ss_conv.batchnorm import BatchNorm
+    given = []
+
+    def bn_train(x, field, scalar, n_field, n_scalar, w, b, eps, momentum, running_mean=None, running_var=None):
+        given.append((running_mean, running_var))
+        return torch.full((n_scalar,), 4.0), torch.full((n_field,), 3.0), None, None, None
+
+    monkeypatch.setattr(_ext, "bn_train", bn_train)
+    bn = BatchNorm([(2, 0), (1, 1)], momentum=0.5, affine=False).to(dtype)
+    bn._batch_statistics(torch.zeros(5, 5), None, None, None, None)
+    if dtype == torch.float32:
+        assert given == [(bn.running_mean, bn.running_var)]
+    else:
+        assert given == [(None, None)]
+        assert bn.running_mean.tolist() == [2.0] * 2 and bn.running_var.tolist() == [2.0] * 3
+
+
 def test_argument_errors_without_gpu():
     """Size queries and argument validation run on the host only."""
     from ss_conv import _ext
