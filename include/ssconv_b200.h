@@ -394,7 +394,8 @@ int ssc_conv_wgrad(const float *features, int c_in, const float *out_grad, int c
                    size_t scratch_bytes, void *stream);
 /* The same with the table's compacted pair lists already in hand (ssc_conv_pairs_build; layers that share a
  * rulebook share them): nothing is built per call.  lists NULL: built in scratch, as ssc_conv_wgrad does.
- * OR'ed into `precision` = SSC_PREC_TF32 (c_in <= 256): `features` / `out_grad` is the image ssc_conv_stage
+ * Tables of more than 256 offsets have no lists (NULL): those take the exact fp32 kernel.
+ * OR'ed into `precision` = SSC_PREC_TF32 (c_in <= 256, K <= 256): `features` / `out_grad` is the image ssc_conv_stage
  * made of it (rows padded to a multiple of four floats), so its rows need no rounding again. */
 #define SSC_WGRAD_X_STAGED 0x400
 #define SSC_WGRAD_DY_STAGED 0x800

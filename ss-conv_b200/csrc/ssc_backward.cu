@@ -260,7 +260,7 @@ extern "C" size_t ssc_conv_wgrad_scratch_bytes(int K, int c_in, int c_out, int n
 extern "C" int ssc_conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int c_out, const int32_t *nbr, int K,
                                     int n_out, void *lists, size_t list_bytes, int precision, float *d_filters,
                                     int32_t *status, void *scratch, size_t scratch_bytes, void *stream) {
-  SSC_REQUIRE(K >= 1 && K <= 256 && c_in >= 1 && c_out >= 1 && n_out >= 0 && d_filters, "conv_wgrad: bad arguments");
+  SSC_REQUIRE(K >= 1 && c_in >= 1 && c_out >= 1 && n_out >= 0 && d_filters, "conv_wgrad: bad arguments");
   cudaStream_t st = as_stream(stream);
   const long long elems = (long long)K * c_in * c_out;
   if (n_out == 0) {
@@ -276,7 +276,7 @@ extern "C" int ssc_conv_wgrad_lists(const float *features, int c_in, const float
   const int staged = ((precision & SSC_WGRAD_X_STAGED) ? 1 : 0) | ((precision & SSC_WGRAD_DY_STAGED) ? 2 : 0);
   const bool tf32 = (precision & ~(SSC_WGRAD_X_STAGED | SSC_WGRAD_DY_STAGED)) == SSC_PREC_TF32;
   SSC_REQUIRE(staged == 0 || (tf32 && conv_wgrad_lists_partial_bytes(K, c_in, c_out, n_out, true) > 0),
-              "conv_wgrad: staged operands need TF32 and at most 256 input channels");
+              "conv_wgrad: staged operands need TF32, at most 256 input channels and 256 offsets");
   if (conv_wgrad_lists_partial_bytes(K, c_in, c_out, n_out, tf32) > 0) {
     PairLists pl;
     if (lists) {

@@ -503,6 +503,7 @@ struct WgradPlan {
 static WgradPlan wgrad_plan(int K, int c_in, int c_out, int n_out, bool tf32) {
   WgradPlan p;
   memset(&p, 0, sizeof(p));
+  if (K > 256) return p;               // (chunk_prefix keeps the offsets in shared memory)
   // never more shares than the table could hold chunks
   const long long most = (long long)K * ceil_div(n_out > 0 ? n_out : 1, WT_K);
   if (tf32) {
@@ -543,7 +544,8 @@ size_t conv_wgrad_lists_partial_bytes(int K, int c_in, int c_out, int n_out, boo
 }
 
 // staged: bit 0 / 1: features / out_grad are TF32 images (ssc_conv_stage: rows padded to a multiple of four floats).
-// Returns -1 when the shape is not covered (the caller then uses the CUDA-core kernel over the table).
+// Returns -1 when the shape is not covered (conv_wgrad_lists_partial_bytes is 0: the caller then uses the CUDA-core kernel
+// over the table).
 int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int c_out, const PairLists &pl, int K, int n_out,
                      bool tf32, int staged, float *partial, float *d_filters, int32_t *status, cudaStream_t st) {
   const WgradPlan p = wgrad_plan(K, c_in, c_out, n_out, tf32);

@@ -1175,9 +1175,10 @@ def conv_wgrad(features, out_grad, nbr, precision=None, x_image=None, dy_image=N
     d_flt = _empty((K, c_in, c_out), torch.float32, features.device)
     nbytes = int(lib().ssc_conv_wgrad_scratch_bytes(K, c_in, c_out, n_out))
     scratch = _empty(max(nbytes, 4), torch.uint8, features.device)
-    lists = pair_lists(nbr) if n_out > 0 and (mode == PREC_TF32 or c_in <= 16) else None
+    # (tables of more than 256 offsets have no lists: the exact kernel works on the table itself)
+    lists = pair_lists(nbr) if n_out > 0 and K <= 256 and (mode == PREC_TF32 or c_in <= 16) else None
     x, dy = _p(features, torch.float32), _p(out_grad, torch.float32)
-    if mode == PREC_TF32 and c_in <= 256:
+    if mode == PREC_TF32 and c_in <= 256 and K <= 256:
         if x_image is not None:
             x, mode = _p(x_image), mode | WGRAD_X_STAGED
         if dy_image is not None:

@@ -257,3 +257,21 @@ def test_training_norm_with_running_buffers_of_another_type(cuda, dtype, record)
     assert torch.equal(outs[0][0], outs[1][0])
     for a, b in zip(outs[0][1:], outs[1][1:]):
         assert b.dtype == dtype and torch.allclose(a.double(), b.double(), rtol=4 * torch.finfo(torch.float16).eps if dtype == torch.float16 else 1e-6, atol=1e-4)
+
+
+@pytest.mark.parametrize("K,c_in,c_out", [(256, 3, 8), (257, 3, 8), (343, 20, 7)])
+def test_gradients_over_tables_of_many_offsets(cuda, K, c_in, c_out):
+    """Around the 256 offsets up to which pair lists are made.  Sums of at most 90 products: a few ulp of the largest."""
+    from ss_conv import _ext
+    rng = np.random.RandomState(K)
+    n_in, n_out = 90, 70
+    t = np.stack([rng.permutation(n_in)[:n_out] for _ in range(K)]).astype(np.int32)      # an input once per offset
+    t[rng.rand(K, n_out) < .7] = -1
+    x, W, g = (rng.randn(*s).astype(np.float32) for s in ((n_in, c_in), (K, c_in, c_out), (n_out, c_out)))
+    d_in, d_w = _ext.conv_backward(dev(x, cuda), dev(W, cuda), dev(g, cuda), dev(t, cuda), precision="fp32")
+    want_in, want_w = np.zeros((n_in, c_in)), np.zeros(W.shape)
+    for k in range(K):
+        o = np.nonzero(t[k] >= 0)[0]
+        np.add.at(want_in, t[k][o], g[o].astype(np.float64) @ W[k].T)
+        want_w[k] = x[t[k][o]].astype(np.float64).T @ g[o]
+    assert rel_err(d_in.cpu().numpy(), want_in) <= 1e-5 and rel_err(d_w.cpu().numpy(), want_w) <= 1e-5

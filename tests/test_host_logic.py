@@ -162,6 +162,14 @@ def test_running_statistics_of_other_types_stay_with_torch(monkeypatch, dtype):
         assert bn.running_mean.tolist() == [2.0] * 2 and bn.running_var.tolist() == [2.0] * 3
 
 
+def test_filter_gradients_of_large_kernels_are_not_refused():
+    """Tables of more than 256 offsets (a 7^3 kernel) come from rulebooks made elsewhere: only the missing rows are an error."""
+    from ss_conv import _ext
+    assert _ext.lib().ssc_conv_wgrad_scratch_bytes(343, 3, 8, 10) > 0
+    assert _ext.lib().ssc_conv_wgrad(None, 3, None, 8, None, 343, 10, _ext.PREC_FP32, 8, None, None, 0, None) == 1
+    assert b"null pointer" in _ext.lib().ssc_last_error()
+
+
 def test_argument_errors_without_gpu():
     """Size queries and argument validation run on the host only."""
     from ss_conv import _ext
