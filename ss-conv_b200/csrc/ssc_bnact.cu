@@ -585,6 +585,51 @@ bn_gate_bwd_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__res
   }
 }
 
+// The same for rows of which not even one fits shared memory twice with its constants (more than about 4800
+// channels): a thread per channel, everything read where it lies.  Same sums in the same order.
+template <int PASS>
+__global__ void __launch_bounds__(256)
+bn_gate_bwd_wide_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
+                        float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
+  const int ch = (int)(blockIdx.y * 256 + threadIdx.x);
+  if (ch >= p.c) return;
+  auto normed = [&](const float *xr, int k) { return p.scale ? fmaf(__ldg(xr + k), __ldg(p.scale + k), __ldg(p.shift + k)) : __ldg(xr + k); };
+  const int gate = p.gate_of_channel ? (ch < p.c_out ? __ldg(p.gate_of_channel + ch) : -3) : -2;
+  const float mu = p.mu ? __ldg(p.mu + ch) : 0.f;
+  float sum_a = 0.f, sum_g = 0.f;
+  const int step = PASS == 0 ? p.chains : (int)gridDim.x;
+  for (long long r = blockIdx.x; r < p.n; r += step) {
+    const float *xr = p.x + (size_t)r * p.c, *gr = p.go + (size_t)r * p.c_out;
+    float g;
+    if (gate == -3) {
+      const int s0 = __ldg(p.field_start + ch - p.c_out), len = __ldg(p.field_len + ch - p.c_out);
+      float acc = 0.f;
+      for (int q = 0; q < len; ++q) acc = fmaf(__ldg(gr + s0 + q), normed(xr, s0 + q), acc);
+      const float v = normed(xr, ch);
+      g = acc * act_grad(v, apply_act(v, p.g_act), p.g_act);
+    } else {
+      g = __ldg(gr + ch);
+      if (gate >= 0) {
+        g *= apply_act(normed(xr, p.c_out + gate), p.g_act);
+      } else if (gate == -1) {
+        const float y = normed(xr, ch);
+        g *= act_grad(y, p.s_act == 2 ? apply_act(y, 2) : 0.f, p.s_act);
+      }
+    }
+    const float d = __ldg(xr + ch) - mu;
+    if (PASS == 0) {
+      sum_g += g;
+      sum_a = fmaf(g, d, sum_a);
+    } else {
+      gx[(size_t)r * p.c + ch] = ks ? __ldg(ks + ch) * g - __ldg(ka + ch) * d - __ldg(kg + ch) : g;
+    }
+  }
+  if (PASS == 0) {
+    part_a[(size_t)blockIdx.x * p.c + ch] = sum_a;
+    part_g[(size_t)blockIdx.x * p.c + ch] = sum_g;
+  }
+}
+
 // Block per field: A and G from the chains, the field's coefficients and parameter gradients.
 __global__ void __launch_bounds__(kFinishThreads)
 bn_bwd_finish_kernel(const float *__restrict__ part_a, const float *__restrict__ part_g, int row_blocks, int n, int c,
@@ -793,6 +838,13 @@ static int launch_bwd(BnGateBwd p, const float *ks, const float *ka, const float
   size_t smem;
   p.rows = bwd_tile_rows(p.c, p.c_out, p.n_gates, PASS == 0 ? 32 : 64, &smem);
   p.chains = 8 * bn_row_blocks(p.n);
+  if (smem > 227 * 1024) {
+    const int blocks = PASS == 0 ? p.chains : (p.n < 4 * 148 ? p.n : 4 * 148);
+    bn_gate_bwd_wide_kernel<PASS><<<dim3(blocks, ceil_div(p.c, 256)), 256, 0, st>>>(p, ks, ka, kg, gx, part_a, part_g);
+    note_launches(1);
+    SSC_CHECK_LAUNCH("bn_gate_bwd");
+    return SSC_OK;
+  }
   const int odd = p.c | p.c_out;
   const uintptr_t at = (uintptr_t)p.x | (uintptr_t)p.go;
   if ((odd & 3) == 0 && (at & 15u) == 0) return launch_bwd_vec<PASS, 4>(p, smem, ks, ka, kg, gx, part_a, part_g, st);

@@ -275,3 +275,33 @@ def test_gradients_over_tables_of_many_offsets(cuda, K, c_in, c_out):
         np.add.at(want_in, t[k][o], g[o].astype(np.float64) @ W[k].T)
         want_w[k] = x[t[k][o]].astype(np.float64).T @ g[o]
     assert rel_err(d_in.cpu().numpy(), want_in) <= 1e-5 and rel_err(d_w.cpu().numpy(), want_w) <= 1e-5
+
+
+@pytest.mark.parametrize("Rs,n", [([(3500, 0), (300, 1)], 5), ([(4001, 0), (1500, 1)], 70), ([(9001, 0)], 3)])
+@pytest.mark.parametrize("training", [True, False])
+def test_norm_and_gate_gradients_of_very_wide_rows(cuda, Rs, n, training):
+    """Below and above the width of which a row with its constants fits shared memory, norm and gate together and the
+    gate alone: the float64 composite, with the bound of the test at tile edges."""
+    import copy
+    from ss_conv.activation import Activation
+    from ss_conv.batchnorm import BatchNorm
+    from ss_conv.sp_ops.tensor import SparseTensor
+    torch.manual_seed(n)
+    n_gates = sum(m for m, l in Rs if l > 0)
+    gated = Rs + ([(n_gates, 0)] if n_gates else [])
+    c, c_out = (sum(m * (2 * l + 1) for m, l in r) for r in (gated, Rs))
+    bn, act = BatchNorm(gated).to(cuda).train(training), Activation(Rs, (torch.relu, torch.sigmoid), bias=False, checkpoint=False).to(cuda)
+    bn64, act64 = copy.deepcopy(bn).double().cpu(), copy.deepcopy(act).double().cpu()
+    coef, base = torch.randn(n, c_out, device=cuda), torch.randn(n, c, device=cuda) + 0.2
+
+    def close(got, want):
+        assert float((got.cpu().double() - want).abs().max()) <= 1e-4 * max(float(want.abs().max()), 1e-3)
+
+    for alone in (False, True):
+        x, x64 = base.clone().requires_grad_(True), base.double().cpu().requires_grad_(True)
+        t = SparseTensor(x, torch.zeros(n, 4, dtype=torch.int32, device=cuda), [8] * 3, 1)
+        ((act(t) if alone else bn.norm_and_gate(t, act)).features * coef).sum().backward()
+        (act64._gate_composite(x64 if alone else bn64._differentiable(x64)) * coef.double().cpu()).sum().backward()
+        close(x.grad, x64.grad)
+    close(bn.weight.grad, bn64.weight.grad)
+    close(bn.bias.grad, bn64.bias.grad)
