@@ -1477,7 +1477,9 @@ def voxel_centres(indices, unit, extent):
 
 
 def point_rows(points, ids):
-    """Rows (id, x, y, z)."""
+    """Rows (id, x, y, z) of points [n, 3] and ids [n]."""
+    if points.dim() != 2 or points.shape[1] != 3 or ids.shape != points.shape[:1]:
+        raise ValueError("points must be [n, 3] with one batch id each (got %s and %s)" % (tuple(points.shape), tuple(ids.shape)))
     out = _empty((points.shape[0], 4), torch.float32, points.device)
     _check(lib().ssc_point_rows(_p(points, torch.float32), _p(ids, torch.int32), points.shape[0], _p(out), _stream()))
     return out

@@ -326,3 +326,15 @@ def test_scatter_add_rate_kernel_adds_what_it_reports(cuda):
         idx = torch.arange(positions, device=cuda) % rows.numel()
         expect = torch.bincount(rows[idx].long(), minlength=n_rows).float()
         assert torch.equal(out, expect[:, None].expand(n_rows, width)), (lanes, warps)
+
+
+def test_points_and_batch_ids_of_different_lengths_are_refused(cuda):
+    from ss_conv.sp_ops.tensor import SparseTensor
+    from ss_conv.sp_ops.voxelize import Voxel2Point
+    x = SparseTensor(torch.randn(4, 8, device=cuda), torch.zeros(4, 4, dtype=torch.int32, device=cuda), [8] * 3, 1)
+    v2p = Voxel2Point(voxel_extent=[1.0] * 3, unit_voxel_extent=None)
+    points = torch.zeros(10, 3, device=cuda)
+    assert v2p(x, points, torch.zeros(10, dtype=torch.int64, device=cuda)).shape == (10, 8)
+    for ids in (torch.zeros(9, dtype=torch.int64, device=cuda), torch.zeros(10, 1, dtype=torch.int32, device=cuda)):
+        with pytest.raises((ValueError, RuntimeError)):
+            v2p(x, points, ids)

@@ -170,6 +170,14 @@ def test_filter_gradients_of_large_kernels_are_not_refused():
     assert b"null pointer" in _ext.lib().ssc_last_error()
 
 
+@pytest.mark.parametrize("points,ids", [((5, 3), (4,)), ((5, 3), (5, 1)), ((5, 2), (5,)), ((15,), (5,))])
+def test_point_rows_look_at_their_shapes(points, ids):
+    """The kernel reads three coordinates and one id per point: anything else is refused before it runs."""
+    from ss_conv import _ext
+    with pytest.raises(ValueError):
+        _ext.point_rows(torch.zeros(points), torch.zeros(ids, dtype=torch.int32))
+
+
 def test_argument_errors_without_gpu():
     """Size queries and argument validation run on the host only."""
     from ss_conv import _ext
