@@ -444,9 +444,13 @@ size_t ssc_p2v_scratch_bytes(int n_point, int batch, const int grid[3]);
  * rotations rot [batch, 3, 3] (an improper one is first multiplied by -1), as rotation_utils.py:424-447
  * computes them on the host: D^l(R) = Y_l(R v) pinv(Y_l(v)), in double precision.  dirs, pinv: for every order
  * one after the other, S = 6 (2 l + 1) + 8 unit directions [S, 3] and the pseudo-inverse [S, 2 l + 1] of their
- * harmonics [2 l + 1, S].  axes: 1 = the reference's frame (polar axis y), 0 = the filter basis' own. */
+ * harmonics [2 l + 1, S].  axes: 1 = the reference's frame (polar axis y), 0 = the filter basis' own.
+ * ssc_steer_matrices64: of rotations in double precision. */
+#define SSC_STEER_MAX_ORDERS 15
 int ssc_steer_matrices(const float *rot, int batch, int orders, const double *dirs, const double *pinv, int axes,
                        float *dmats, void *stream);
+int ssc_steer_matrices64(const double *rot, int batch, int orders, const double *dirs, const double *pinv, int axes,
+                         float *dmats, void *stream);
 /* Feature steering (Feature_Steering_Module._transform_points / _transform_feats,
  * Common_utils/ss_conv_modules.py:198-224): new_points[p] = (points[p] - trans[b]) . rot[b]
  * (divided by scale[b] + 1e-8 when scale is given), new_feats[p, block] = feats[p, block] . D_b for

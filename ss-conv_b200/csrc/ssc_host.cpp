@@ -206,7 +206,7 @@ PyObject *head(PyObject *, PyObject *const *args, Py_ssize_t n) {
   X(ssc_layer_struct_bytes) X(ssc_layer_ahead_bytes) X(ssc_layer_ahead) X(ssc_conv_gate_covered) \
   X(ssc_conv_fwd_gated) X(ssc_conv_fwd_ordered) X(ssc_conv_wgrad_scratch_bytes) X(ssc_conv_wgrad) \
   X(ssc_conv_wgrad_lists) X(ssc_maxpool_bwd) X(ssc_avgpool_bwd) X(ssc_global_avgpool_bwd) X(ssc_global_maxpool_bwd) \
-  X(ssc_voxelize_bwd) X(ssc_three_interpolate_bwd) X(ssc_steer_matrices) X(ssc_steer_fwd) X(ssc_p2v_stats) \
+  X(ssc_voxelize_bwd) X(ssc_three_interpolate_bwd) X(ssc_steer_matrices) X(ssc_steer_matrices64) X(ssc_steer_fwd) X(ssc_p2v_stats) \
   X(ssc_maxpool_fwd) X(ssc_avgpool_fwd) X(ssc_pool_fwd16) X(ssc_summary_rf) X(ssc_global_avgpool_fwd) \
   X(ssc_global_maxpool_fwd) X(ssc_batch_offsets) X(ssc_voxel2point_map) X(ssc_voxelize_fwd) X(ssc_p2v_scratch_bytes) \
   X(ssc_p2v_keep_scratch_bytes) X(ssc_p2v_keep) X(ssc_voxel_centres) X(ssc_point_rows) X(ssc_nn_weights) \

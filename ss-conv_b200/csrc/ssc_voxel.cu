@@ -557,8 +557,10 @@ extern "C" size_t ssc_p2v_scratch_bytes(int n_point, int batch, const int grid[3
 // harmonics of the rotated direction into shared memory, then a thread per matrix element adds them up.
 // dirs / pinv: per order l, 6 (2 l + 1) + 8 directions [S, 3] and the pseudo-inverse [S, 2 l + 1], one order after
 // the other.  axes != 0: the rotation is described in the frame whose polar axis is y (R -> S R S^T).
+// T: the rotations as the caller has them, fp32 or double (rounded to fp32 first they cost 4e-8 per entry and order).
+template <typename T>
 __global__ void __launch_bounds__(128)
-steer_matrices_kernel(const float *__restrict__ rot, int orders, const double *__restrict__ dirs,
+steer_matrices_kernel(const T *__restrict__ rot, int orders, const double *__restrict__ dirs,
                       const double *__restrict__ pinv, int axes, int stride, float *__restrict__ dmats) {
   extern __shared__ double ys[];                 // per order [S][2 l + 1], as pinv
   const int b = blockIdx.x;
@@ -659,9 +661,9 @@ __global__ void steer_kernel(const float *__restrict__ points, const float *__re
   new_feats[(size_t)p * c + k] = acc;
 }
 
-extern "C" int ssc_steer_matrices(const float *rot, int batch, int orders, const double *dirs, const double *pinv, int axes,
-                                  float *dmats, void *stream) {
-  SSC_REQUIRE(batch >= 0 && orders >= 1 && orders <= 16, "steer_matrices: bad sizes");
+template <typename T>
+static int steer_matrices(const T *rot, int batch, int orders, const double *dirs, const double *pinv, int axes, float *dmats, void *stream) {
+  SSC_REQUIRE(batch >= 0 && orders >= 1 && orders <= SSC_STEER_MAX_ORDERS, "steer_matrices: bad sizes");
   if (batch == 0) return SSC_OK;
   SSC_REQUIRE(rot && dirs && pinv && dmats, "steer_matrices: null pointer");
   int stride = 0, harmonics = 0;
@@ -671,12 +673,22 @@ extern "C" int ssc_steer_matrices(const float *rot, int batch, int orders, const
   }
   const size_t smem = (size_t)harmonics * sizeof(double);       // 5 KB for orders 0..3, below 48 KB up to order 8
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(steer_matrices_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(steer_matrices_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "steer_matrices: smem attribute: %s", cudaGetErrorString(e));
   }
-  { steer_matrices_kernel<<<batch, 128, smem, as_stream(stream)>>>(rot, orders, dirs, pinv, axes, stride, dmats); note_launches(1); }
+  { steer_matrices_kernel<T><<<batch, 128, smem, as_stream(stream)>>>(rot, orders, dirs, pinv, axes, stride, dmats); note_launches(1); }
   SSC_CHECK_LAUNCH("steer_matrices");
   return SSC_OK;
+}
+
+extern "C" int ssc_steer_matrices(const float *rot, int batch, int orders, const double *dirs, const double *pinv, int axes,
+                                  float *dmats, void *stream) {
+  return steer_matrices(rot, batch, orders, dirs, pinv, axes, dmats, stream);
+}
+
+extern "C" int ssc_steer_matrices64(const double *rot, int batch, int orders, const double *dirs, const double *pinv, int axes,
+                                    float *dmats, void *stream) {
+  return steer_matrices(rot, batch, orders, dirs, pinv, axes, dmats, stream);
 }
 
 extern "C" int ssc_steer_fwd(const float *points, const float *feats, const int32_t *ids, const float *rot,

@@ -109,6 +109,7 @@ SIGNATURES = {
     "ssc_voxelize_bwd": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "ssc_three_interpolate_bwd": (c_int, [c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "ssc_steer_matrices": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
+    "ssc_steer_matrices64": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
     "ssc_steer_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                               c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "ssc_p2v_stats": (c_int, [c_void_p, c_void_p, c_int, _I3, _F3, c_void_p, c_void_p]),
@@ -1419,13 +1420,21 @@ point_recover_fp = _not_built("point_recover_fp")
 point_recover_bp = _not_built("point_recover_bp")
 
 
+STEER_MAX_ORDERS = 15        # SSC_STEER_MAX_ORDERS: what a block's harmonics leave room for in shared memory
+
+
 def steer_matrices(rot, dirs, pinv, orders, reference_frame):
     """[B, sum (2l+1)^2] representation matrices of rotations [B, 3, 3] (ssc_steer_matrices); dirs / pinv: the
-    float64 tables of SO3.sample_tables on the same device."""
-    rot = rot.float().contiguous()
+    float64 tables of SO3.sample_tables on the same device.  Rotations in double precision are taken as they are."""
+    if rot.numel() != 9 * rot.shape[0]:
+        raise ValueError("rotations must be [B, 3, 3] (got %s)" % (tuple(rot.shape),))
+    if rot.dtype != torch.float64:
+        rot = rot.float()
+    rot = rot.contiguous()
     out = _empty((rot.shape[0], sum((2 * l + 1) ** 2 for l in range(orders))), torch.float32, rot.device)
-    _check(lib().ssc_steer_matrices(_p(rot), rot.shape[0], int(orders), _p(dirs, torch.float64), _p(pinv, torch.float64),
-                                    int(bool(reference_frame)), _p(out), _stream()))
+    fn = lib().ssc_steer_matrices64 if rot.dtype == torch.float64 else lib().ssc_steer_matrices
+    _check(fn(_p(rot), rot.shape[0], int(orders), _p(dirs, torch.float64), _p(pinv, torch.float64), int(bool(reference_frame)),
+              _p(out), _stream()))
     return out
 
 

@@ -149,10 +149,11 @@ class Feature_Steering_Module(nn.Module):
     def sample_matrices(self, r):
         """[B, sum (2l+1)^2]: the representation matrices D^l(r_b) of every order, back to back.  On the GPU one
         kernel in double precision; a loop over samples and orders on the host took 9 ms for 64 samples."""
-        if r.is_cuda:
-            if self._tables is None or self._tables[0].device != r.device:
-                self._tables = tuple(t.to(r.device) for t in SO3.sample_tables(len(self.irrep)))
-            return _ext.steer_matrices(r.detach(), *self._tables, len(self.irrep), self.frame == "reference")
+        if r.is_cuda and len(self.irrep) <= _ext.STEER_MAX_ORDERS:
+            tables = self.__dict__.get("_tables")
+            if tables is None or tables[0].device != r.device:
+                tables = self._tables = tuple(t.to(r.device) for t in SO3.sample_tables(len(self.irrep)))
+            return _ext.steer_matrices(r.detach(), *tables, len(self.irrep), self.frame == "reference")
         blocks = [SO3.D_from_matrix(r.detach().double().cpu(), l, self.frame).reshape(r.shape[0], -1)
                   for l in range(len(self.irrep))]
         return torch.cat(blocks, dim=1).float()
@@ -168,9 +169,9 @@ class Feature_Steering_Module(nn.Module):
                 s = s[:, 0] if s.size(1) == 1 else torch.norm(s, dim=1)
             scale = s.contiguous().to(dev)
         dmats = self.sample_matrices(r).to(dev).contiguous()
-        if self._chan.device != dev:
-            self._chan = self._chan.to(dev)
         chan = self._chan
+        if chan.device != dev:
+            chan = self._chan = chan.to(dev)
         return _ext.steer(points.float().contiguous(), feats.float().contiguous(), ids.int().contiguous(),
                           r.detach().float().contiguous().to(dev), t.detach().float().contiguous().to(dev), scale, dmats,
                           chan)

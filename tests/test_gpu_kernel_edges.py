@@ -108,6 +108,27 @@ def test_steering_matrices_match_the_host_form(cuda, orders, batch, frame):
     assert float((got.cpu().double() - want.double()).abs().max()) <= 1e-6
 
 
+@pytest.mark.parametrize("orders", [4, 15, 16])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.float16])
+def test_steering_matrices_take_rotations_as_they_are(cuda, orders, dtype):
+    """Rotations in double precision are not rounded first (the matrix of rotations rounded to fp32 is off by their
+    rounding times the order); orders beyond the kernel's go through the host form.  The result is
+    that of the host rounded to fp32: half an ulp of entries up to 1 and what double sums lose, 1e-7."""
+    from ss_conv.utils import SO3
+    from ss_conv_modules import Feature_Steering_Module
+    rng = np.random.RandomState(orders)
+    q = np.linalg.qr(rng.randn(5, 3, 3))[0]
+    rot = torch.from_numpy(q * np.sign(np.linalg.det(q))[:, None, None]).to(dtype)
+    net = Feature_Steering_Module((1,) + (0,) * (orders - 1) if orders > 4 else (1,) * 4, origin_voxel_extent=[1.0] * 3)
+    got = net.sample_matrices(rot.to(cuda))
+    want = torch.cat([SO3.D_from_matrix(rot.double(), l, net.frame).reshape(5, -1) for l in range(orders)], dim=1)
+    assert got.dtype == torch.float32
+    assert float((got.cpu().double() - want).abs().max()) <= 1e-7
+    if orders == 4:
+        with pytest.raises((ValueError, RuntimeError)):
+            net.sample_matrices(rot[0].to(cuda))
+
+
 @pytest.mark.parametrize("n_query,n_known", [(1, 3), (63, 4), (65, 5), (130, 257)])
 def test_three_nearest_with_ties(cuda, n_query, n_known):
     """Coordinates on a coarse lattice (many equal distances, all exact): the smallest index first among equals."""
