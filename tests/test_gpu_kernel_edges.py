@@ -72,6 +72,33 @@ def test_pools_at_tile_edges(cuda, n_in, n_out, c, K, dtype):
         assert torch.equal(d, want)
 
 
+@pytest.mark.parametrize("K,c", [(27, 8), (27, 6), (8, 5)])
+def test_average_pools_divide_by_any_count(cuda, K, c):
+    """Counts are an argument of the entry points: 0, negative ones and ones beyond the range of the corrected quotient
+    give the bits of a division, infinities and NaNs included."""
+    from ss_conv import _ext
+    from ss_conv._ext import lib, _p, _stream, _check
+    rng = np.random.RandomState(K + c)
+    n_in, n_out = 60, 40
+    t = dev(_table(n_out, n_in, K, 0.5, rng), cuda)
+    x = rng.randn(n_in, c).astype(np.float32)
+    x[rng.rand(n_in, c) < .3] = 0
+    x = dev(x, cuda)
+    special = np.array([0, -3, 1, 2 ** 20, 2 ** 20 + 1, 2 ** 31 - 1], np.int32)
+    for backward in (False, True):
+        count = dev(special[rng.randint(0, 6, n_in if backward else n_out)], cuda)
+        out, want = torch.empty(n_out, c, device=cuda), torch.zeros(n_out, c, device=cuda)
+        for k in range(K):
+            div = (count[t[k].clamp(min=0).long()] if backward else count).float()[:, None]
+            want = torch.where((t[k] >= 0)[:, None], want + x[t[k].clamp(min=0).long()] / div, want)
+        if backward:
+            _check(lib().ssc_avgpool_bwd(_p(x), c, _p(t), K, n_out, _p(count), _p(out), _stream()))
+        else:
+            _check(lib().ssc_avgpool_fwd(_p(x), c, _p(t), K, n_out, _p(count), _p(out), None, _stream()))
+        assert not bool(want.isfinite().all()) and torch.equal(out.isnan(), want.isnan())
+        assert torch.equal(out.nan_to_num(7.0, 8.0, 9.0), want.nan_to_num(7.0, 8.0, 9.0))
+
+
 @pytest.mark.parametrize("c_in,c_out,k,n", [(1, 1, 1, 1), (2, 40, 3, 129), (3, 36, 3, 700), (4, 38, 3, 300), (3, 70, 5, 130)])
 def test_fp32_convolution_of_few_input_channels(cuda, c_in, c_out, k, n):
     """The exact kernel for up to four input channels: rows around a block, output channels that are no multiple
