@@ -352,6 +352,16 @@ class CountPost(object):
 
     __del__ = _close
 
+    def __deepcopy__(self, memo):         # a copied tensor's count is the same count
+        return self
+
+    def __reduce__(self):                 # elsewhere it is read from the device word
+        return _no_post, ()
+
+
+def _no_post():
+    return None
+
 
 def _read_words(words, dev):
     n = len(words) + 1

@@ -178,6 +178,23 @@ def test_point_rows_look_at_their_shapes(points, ids):
         _ext.point_rows(torch.zeros(points), torch.zeros(ids, dtype=torch.int32))
 
 
+def test_tensors_with_posted_counts_can_be_copied_and_saved():
+    """A pending SparseTensor carries its count's place: deep copies share it, a saved one reads the device word."""
+    import copy
+    import io
+    from ss_conv import _ext
+    from ss_conv.sp_ops.tensor import PendingRows, SparseTensor
+    n = torch.zeros(1, dtype=torch.int32)
+    n._ssc_post = _ext.CountPost()
+    x = SparseTensor(torch.zeros(4, 2), torch.zeros(4, 4, dtype=torch.int32), [4] * 3, 1)
+    x._rows = PendingRows(n, 4, None, None)
+    assert copy.deepcopy(x)._rows.n_dev._ssc_post is n._ssc_post
+    file = io.BytesIO()
+    torch.save(x, file)
+    file.seek(0)
+    assert torch.load(file, weights_only=False)._rows.n_dev._ssc_post is None
+
+
 def test_argument_errors_without_gpu():
     """Size queries and argument validation run on the host only."""
     from ss_conv import _ext
