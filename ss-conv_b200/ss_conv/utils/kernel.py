@@ -156,16 +156,17 @@ class SE3Kernel(torch.nn.Module):
                     print("{} -> {} : {} basis elements".format(l_in, l_out, len(basis)))
                 self.register_buffer(name, basis.type(torch.get_default_dtype()))
         self.weight = torch.nn.Parameter(torch.cat(weights))
-        self._packed = None  # (device, blob, block_table, out_field, in_field)
+        self._packed = None  # (device, blob, block_table, out_field, in_field, out_start, in_start)
 
     def __repr__(self):
         return "{} ({} -> {}, size={})".format(self.__class__.__name__, self.Rs_in, self.Rs_out, self.size)
 
     # ------------------------------------------------------------------ device-side tables
     def _tables(self, device):
-        """Basis blob + index tables for the materialisation kernel, cached per device."""
-        if self._packed is not None and self._packed[0] == device:
-            return self._packed[1:]
+        """Basis blob + index tables for the materialisation kernel and its adjoint, cached per device."""
+        packed = self._packed
+        if packed is not None and packed[0] == device and len(packed) == 7:      # (saved modules may hold fewer)
+            return packed[1:]
         K = self.size ** 3
         blobs, table, boff, woff = [], [], 0, 0
         for i, (m_out, _) in enumerate(self.Rs_out):
@@ -186,10 +187,9 @@ class SE3Kernel(torch.nn.Module):
                     for c in range(self.dims_in[j])]
         blob = (torch.cat(blobs) if blobs else torch.zeros(1)).to(device)
         ints = lambda v: torch.tensor(v, dtype=torch.int32, device=device).reshape(-1)  # noqa: E731
-        packed = (device, blob, ints(table), ints(out_field), ints(in_field))
+        packed = (device, blob, ints(table), ints(out_field), ints(in_field),
+                  ints([k for k, f in enumerate(out_field) if f[2] == 0]), ints([k for k, f in enumerate(in_field) if f[2] == 0]))
         self._packed = packed
-        self._starts = (ints([k for k, f in enumerate(out_field) if f[2] == 0]),
-                        ints([k for k, f in enumerate(in_field) if f[2] == 0]))
         return packed[1:]
 
     def _apply(self, fn, *args, **kwargs):
@@ -205,7 +205,7 @@ class SE3Kernel(torch.nn.Module):
         return self._materialize(weight)
 
     def _materialize(self, weight):
-        blob, table, out_field, in_field = self._tables(weight.device)
+        blob, table, out_field, in_field = self._tables(weight.device)[:4]
         K = self.size ** 3
         flt = _ext.materialize(weight.detach().contiguous(), blob, table, len(self.Rs_in), out_field, in_field,
                                self.n_out, self.n_in, K)
@@ -214,8 +214,8 @@ class SE3Kernel(torch.nn.Module):
     def _weight_grad(self, g):
         """Adjoint of the (linear) materialisation: g [k,k,k,Cin,Cout] -> gradient of the flat
         weight vector (weights of block (i,j) are laid out [m_out, m_in, n_basis])."""
-        blob, table, out_field, in_field = self._tables(g.device)
-        return _ext.materialize_backward(g.float(), blob, table, len(self.Rs_in), out_field, in_field, *self._starts,
+        blob, table, *fields = self._tables(g.device)
+        return _ext.materialize_backward(g.float(), blob, table, len(self.Rs_in), *fields,
                                          max(self.dims_out) * max(self.dims_in), self.n_out, self.n_in, self.size ** 3,
                                          self.weight.numel()).to(self.weight.dtype)
 

@@ -195,6 +195,23 @@ def test_tensors_with_posted_counts_can_be_copied_and_saved():
     assert torch.load(file, weights_only=False)._rows.n_dev._ssc_post is None
 
 
+def test_kernels_saved_with_fewer_tables_are_completed(monkeypatch):
+    """Index tables travel with a pickled module: one saved before the adjoint had tables of its own gets them on first use,
+    and the tables of a device are taken as one."""
+    import pickle
+    from ss_conv import _ext
+    from ss_conv.utils.kernel import SE3Kernel
+    kernel = SE3Kernel([(1, 0), (1, 1)], [(2, 0), (1, 1)], 3)
+    full = kernel._tables(torch.device("cpu"))
+    assert [t.tolist() for t in full[4:]] == [[0, 1, 2], [0, 1]]
+    kernel._packed = kernel._packed[:5]
+    kernel = pickle.loads(pickle.dumps(kernel))
+    seen = []
+    monkeypatch.setattr(_ext, "materialize_backward", lambda *a: seen.append(a) or torch.zeros(a[-1]))
+    kernel._weight_grad(torch.zeros(3, 3, 3, 4, 5))
+    assert all(torch.equal(a, b) for a, b in zip(seen[0][4:8], full[2:]))
+
+
 def test_argument_errors_without_gpu():
     """Size queries and argument validation run on the host only."""
     from ss_conv import _ext
