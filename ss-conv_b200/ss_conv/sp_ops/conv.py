@@ -6,7 +6,7 @@ import torch
 import torch.nn as nn
 from torch.nn.parameter import Parameter
 
-from .tensor import PendingRows, SparseTensor, run_ahead
+from .tensor import PendingRows, RunsAhead, SparseTensor, run_ahead
 from .ops import get_conv_output_size, get_deconv_output_size, get_indice_pairs, _per_dim
 from .. import _ext
 from .functional import indice_conv, indice_inverse_conv, indice_subm_conv
@@ -16,7 +16,7 @@ from .functional import indice_conv, indice_inverse_conv, indice_subm_conv
 _FEATURE_DTYPES = (torch.float32, torch.float16, torch.bfloat16)
 
 
-class SparseConvolution(nn.Module):
+class SparseConvolution(RunsAhead, nn.Module):
     def __init__(self, ndim, in_channels, out_channels, kernel_size=3, stride=1, padding=0, dilation=1, groups=1,
                  bias=True, subm=False, output_padding=0, transposed=False, inverse=False, indice_key=None):
         super().__init__()

@@ -3,12 +3,12 @@ import torch
 import torch.nn as nn
 
 from .. import _ext
-from .tensor import PendingRows, SparseTensor, run_ahead
+from .tensor import PendingRows, RunsAhead, SparseTensor, run_ahead
 from .ops import get_conv_output_size, get_indice_pairs, _per_dim
 from .functional import indice_avgpool, indice_maxpool
 
 
-class _SparsePool(nn.Module):
+class _SparsePool(RunsAhead, nn.Module):
     _op = _stored16 = _code = None
 
     def __init__(self, ndim, kernel_size, stride=1, padding=0, dilation=1, subm=False):

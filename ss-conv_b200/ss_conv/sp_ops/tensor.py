@@ -220,6 +220,14 @@ class SparseTensor(object):
         return self.indices.shape[0] / np.prod(self.spatial_shape) / self.batch_size
 
 
+class RunsAhead(object):
+    """Mixin of the layers that run_ahead keeps plans on: they stay out of copies and saved modules (a plan is the memory of
+    a structure of this build of the library, and made again in microseconds)."""
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_ahead_plans"}
+
+
 def run_ahead(layer, input, op, output_shape, transpose, exact, weight=None, gate=None):
     """The output of a strided layer without an indice_key queued in one library call with its count still on
     the device (_ext.layer_ahead), or None where it has to be queued step by step.  layer: the module (its

@@ -59,6 +59,8 @@ def test_layer_structure_has_the_size_of_the_librarys():
 def test_plans_of_layers_that_run_ahead_follow_their_input(monkeypatch):
     """One pool on rows of several widths, and a layer whose geometry is changed: the plan handed to the library has the
     present channel counts and sizes."""
+    import copy
+    import pickle
     from ss_conv import _ext
     from ss_conv.pool import MaxPool
     from ss_conv.sp_ops.conv import SparseConvolution
@@ -80,6 +82,10 @@ def test_plans_of_layers_that_run_ahead_follow_their_input(monkeypatch):
         run_ahead(conv, SparseTensor(torch.zeros(10, 16), torch.zeros(10, 4, dtype=torch.int32), [8] * 3, 1), 0,
                   conv._output_shape, 0, None, weight)
     assert [(a.c_out, c_row, a.stride[0], a.out_shape[2]) for a, c_row in seen[4:]] == [(8, 8, 2, 4), (24, 24, 2, 4), (8, 8, 1, 8)]
+    for layer in (pool, conv):                     # plans do not travel with copies and saved modules
+        assert layer._ahead_plans
+        for other in (copy.deepcopy(layer), pickle.loads(pickle.dumps(layer))):
+            assert not hasattr(other, "_ahead_plans") and other.stride == layer.stride
     x = SparseTensor(torch.zeros(10, 16), torch.zeros(10, 4, dtype=torch.int32), [8] * 3, 1)
     for dtype in (torch.float16, torch.bfloat16, torch.float64):      # left to the entry points that look at the type
         assert run_ahead(conv, x, 0, conv._output_shape, 0, None, conv.weight.to(dtype)) is None
