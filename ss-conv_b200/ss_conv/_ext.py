@@ -714,8 +714,13 @@ class LazyPairs(object):
             _check(lib().ssc_pairs_from_nbr(_p(nbr), K, n_out, self._n_in, _p(pairs), _p(num), _p(scratch), nbytes,
                                             _stream()))
             pairs._ssc_nbr = nbr
-            self._tensor = pairs
+            self._tensor, self._num = pairs, num
         return self._tensor
+
+    def pair_counts(self):
+        """indice_num [K]: the number of pairs of every kernel offset."""
+        self.materialize()
+        return self._num
 
     def __getattr__(self, name):  # only reached for attributes this class does not define
         return getattr(self.materialize(), name)

@@ -6,7 +6,7 @@ import torch
 import torch.nn as nn
 from torch.nn.parameter import Parameter
 
-from .tensor import PendingRows, RunsAhead, SparseTensor, run_ahead
+from .tensor import PendingRows, PendingRulebook, RunsAhead, SparseTensor, run_ahead
 from .ops import get_conv_output_size, get_deconv_output_size, get_indice_pairs, _per_dim
 from .. import _ext
 from .functional import indice_conv, indice_inverse_conv, indice_subm_conv
@@ -107,7 +107,10 @@ class SparseConvolution(RunsAhead, nn.Module):
             if ahead is not None:
                 outids_cap, pairs, pair_num = ahead
                 if key is not None:
-                    input.indice_dict[key] = (outids_cap, inds_raw, pairs, None, input.spatial_shape)
+                    # (the entry must not hold the input, whose dictionary holds the entry)
+                    geometry = (inds_raw, input.batch_size, input.spatial_shape, input.grid)
+                    input.indice_dict[key] = PendingRulebook((outids_cap, inds_raw, pairs, None, input.spatial_shape),
+                                                             lambda: self._build_rulebook(*geometry))
                 out_cap = self._op(feats_raw, weight, pairs, pair_num, pairs.capacity, gate)
                 if self.bias is not None:
                     out_cap += self.bias
@@ -133,7 +136,7 @@ class SparseConvolution(RunsAhead, nn.Module):
             # keeps the row set of its input: on an input whose count is still on the device it works
             # on the capacity-sized buffers and hands the pending count on (so a whole stack of such
             # layers - a module of the Plain backbones - queues without a host round trip).
-            cached = input.find_indice_pair(key)
+            cached = input.raw_indice_pair(key)
             pairs = None
             if cached is not None and isinstance(cached[2], _ext.LazyPairs) and cached[2].pending() \
                     and not cached[2].regular and cached[2].capacity == inds_raw.shape[0]:
@@ -142,7 +145,7 @@ class SparseConvolution(RunsAhead, nn.Module):
                 pairs = _ext.get_indice_pairs_subm_ahead(inds_raw, input.batch_size, list(input.spatial_shape),
                                                          self.kernel_size, self.dilation, n_in_dev)
                 if key is not None:
-                    input.indice_dict[key] = (inds_raw, inds_raw, pairs, None, input.spatial_shape)
+                    input.indice_dict[key] = PendingRulebook((inds_raw, inds_raw, pairs, None, input.spatial_shape))
             if pairs is not None:
                 out_cap = self._op(feats_raw, weight, pairs, None, pairs.capacity, gate)
                 if self.bias is not None:
@@ -155,7 +158,7 @@ class SparseConvolution(RunsAhead, nn.Module):
                     # the table the pending rows were built on is void; one that an earlier layer of
                     # this key has rebuilt since is the one to use (a layer that is not submanifold
                     # itself could not build it)
-                    kept = input.find_indice_pair(key)
+                    kept = input.raw_indice_pair(key)
                     if kept is not None and kept[2] is pairs:
                         input.indice_dict.pop(key)
                     t = self._sparse_conv_exact(input, weight, gate)
@@ -175,7 +178,7 @@ class SparseConvolution(RunsAhead, nn.Module):
         """An inverse convolution whose partner ran ahead: it gathers through the exchanged table, whose rows are
         the partner's input rows, so the number of the input's own rows is not needed.  None where it does not
         apply."""
-        cached = input.find_indice_pair(self.indice_key)
+        cached = input.raw_indice_pair(self.indice_key)
         if (cached is None or not isinstance(cached[2], _ext.LazyPairs) or not cached[2].regular or not cached[2].pending()
                 or cached[0] is not inds or not feats.is_cuda or feats.dtype not in _FEATURE_DTYPES or weight.dtype != torch.float32
                 or torch.cuda.is_current_stream_capturing()
@@ -209,22 +212,20 @@ class SparseConvolution(RunsAhead, nn.Module):
         return op(features, weight, pairs, num, n_out)
 
     def _cached_rulebook(self, input):
-        """The rulebook kept under this layer's key with exact row counts (an entry made on a pending
-        row count holds capacity-sized coordinates until somebody asks), or None."""
-        cached = input.find_indice_pair(self.indice_key)
-        if cached is None or not isinstance(cached[2], _ext.LazyPairs):
-            return cached
-        outids, indices, pairs, num, shape = cached
-        n = pairs.resolve()
-        if n is None:                                  # built for rows that did not fit: void
+        """The rulebook kept under this layer's key with exact rows (its pair counts may be None), or None."""
+        kept = input.indice_dict.get(self.indice_key) if self.indice_key is not None else None
+        if not isinstance(kept, PendingRulebook):
+            return kept
+        rows = kept.rows()
+        if rows is None:                               # built for rows that did not fit: void
             input.indice_dict.pop(self.indice_key)
-            return None
-        if outids.shape[0] != n:
-            if not pairs.regular:                      # a table on pending rows has as many outputs as inputs
-                indices = indices[:n]
-            outids = outids[:n]
-            cached = input.indice_dict[self.indice_key] = (outids, indices, pairs, num, shape)
-        return cached
+        return rows
+
+    def _build_rulebook(self, indices, batch_size, shape, grid):
+        """The entry of `indice_dict` for this layer on exact rows."""
+        outids, pairs, num = get_indice_pairs(indices, batch_size, shape, self.kernel_size, self.stride, self.padding,
+                                              self.dilation, self.output_padding, self.subm, self.transposed, grid=grid, lazy=True)
+        return outids, indices, pairs, num, shape
 
     def _sparse_conv_exact(self, input, weight, gate=None):
         features, indices = input.features, input.indices
@@ -253,10 +254,8 @@ class SparseConvolution(RunsAhead, nn.Module):
         elif self.indice_key is not None and cached is not None:
             outids, _, indice_pairs, indice_pair_num, _ = cached
         else:
-            outids, indice_pairs, indice_pair_num = get_indice_pairs(
-                indices, batch_size, spatial_shape, self.kernel_size, self.stride, self.padding, self.dilation,
-                self.output_padding, self.subm, self.transposed, grid=input.grid, lazy=True)
-            input.indice_dict[self.indice_key] = (outids, indices, indice_pairs, indice_pair_num, spatial_shape)
+            entry = input.indice_dict[self.indice_key] = self._build_rulebook(indices, batch_size, spatial_shape, input.grid)
+            outids, _, indice_pairs, indice_pair_num, _ = entry
 
         out_features = self._op(features, weight, indice_pairs, indice_pair_num, outids.shape[0], gate)
         if self.bias is not None:

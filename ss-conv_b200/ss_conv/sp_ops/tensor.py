@@ -81,6 +81,51 @@ class PendingRows(object):
         self.family[:] = [c for c in self.family if c.value is None]
 
 
+class PendingRulebook(object):
+    """The entry (outids, indices, indice_pairs, indice_pair_num, spatial_shape) of `indice_dict` for a rulebook whose
+    row count was on the device when it was made.  `raw` is what there is without waiting: capacity-sized
+    coordinates, no pair counts.  Looked at as the tuple it stands for, it is exact: the count is read back, the
+    pair counts are taken from the lists.  A rulebook whose output did not fit its capacity is built again
+    (rebuild); one on pending rows that did not fit (no rebuild) is void until those are recomputed."""
+
+    __slots__ = ("raw", "rebuild", "_rows", "_entry")
+
+    def __init__(self, raw, rebuild=None):
+        self.raw, self.rebuild, self._rows, self._entry = raw, rebuild, None, None
+
+    def rows(self):
+        """The entry with exact rows, its pair counts may be None still; None where it is void."""
+        if self._rows is None:
+            outids, indices, pairs, num, shape = self.raw
+            n = pairs.resolve()
+            if n is None:
+                self._rows = self.rebuild() if self.rebuild is not None else None
+            elif outids.shape[0] != n:
+                # (a table on pending rows has as many outputs as inputs)
+                self._rows = (_ext._head(outids, n), indices if pairs.regular else _ext._head(indices, n), pairs, num, shape)
+            else:
+                self._rows = self.raw
+        return self._rows
+
+    def exact(self):
+        if self._entry is None:
+            rows = self.rows()
+            if rows is None:
+                raise RuntimeError("the rows this rulebook was made on did not fit and have not been recomputed yet")
+            outids, indices, pairs, num, shape = rows
+            self._entry = (outids, indices, pairs, pairs.pair_counts() if num is None else num, shape)
+        return self._entry
+
+    def __iter__(self):
+        return iter(self.exact())
+
+    def __getitem__(self, i):
+        return self.exact()[i]
+
+    def __len__(self):
+        return 5
+
+
 class SparseTensor(object):
     """features [N,C] float32, indices [N,4] int32 rows (batch,x,y,z), the dense spatial shape,
     the batch size, and `indice_dict`, the per-key rulebook cache shared along a network:
@@ -194,9 +239,19 @@ class SparseTensor(object):
         return np.prod(self.spatial_shape)
 
     def find_indice_pair(self, key):
+        """(outids, indices, indice_pairs, indice_pair_num, spatial_shape) kept under `key`, on exact rows, or None."""
         if key is None:
             return None
-        return self.indice_dict.get(key, None)
+        kept = self.indice_dict.get(key, None)
+        if isinstance(kept, PendingRulebook) and kept.rows() is None:
+            self.resolve()
+            kept = self.indice_dict.get(key, None)
+        return kept.exact() if isinstance(kept, PendingRulebook) else kept
+
+    def raw_indice_pair(self, key):
+        """The same without waiting for the device: a rulebook made on pending rows as it stands (PendingRulebook.raw)."""
+        kept = self.indice_dict.get(key, None) if key is not None else None
+        return kept.raw if isinstance(kept, PendingRulebook) else kept
 
     def dense(self, channels_first=True):
         shape = [self.batch_size] + list(self.spatial_shape) + [self.features.shape[1]]

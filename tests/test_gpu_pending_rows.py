@@ -193,3 +193,72 @@ def test_half_filters_keep_their_entry_points(cuda):
                 with pytest.raises(TypeError):
                     layer(SparseTensor(feats[:, :c].contiguous(), inds, [16] * 3, 2))
     _ext.check_status(cuda)
+
+
+@pytest.mark.parametrize("overflow", [False, True])
+@pytest.mark.parametrize("direct", [False, True])
+def test_rulebooks_found_under_a_key_are_exact(cuda, overflow, direct):
+    """find_indice_pair and indice_dict give coordinates, pair lists and pair counts of the exact rows, asked on the
+    input or on the output, whether the layer ran ahead, whether its capacity fitted; so does the entry of
+    a submanifold layer on pending rows."""
+    from ss_conv import _ext
+    from ss_conv.sp_ops.conv import SparseConvolution
+    from ss_conv.sp_ops.tensor import SparseTensor
+    torch.manual_seed(2)
+    rng = np.random.RandomState(8)
+    inds = dev(random_voxels(rng, 2, 20, 2500), cuda)
+    feats = torch.randn(inds.shape[0], 16, device=cuda)
+    plain = SparseConvolution(3, 16, 16, 3, stride=2, padding=1, bias=False).to(cuda)
+    down = SparseConvolution(3, 16, 24, 3, stride=2, padding=1, bias=False, indice_key="down").to(cuda)
+    subm = SparseConvolution(3, 16, 16, 3, padding=1, subm=True, bias=False, indice_key="subm").to(cuda)
+
+    def run(ratio=None):
+        x = SparseTensor(feats, inds, [20] * 3, 2)
+        plain(x)                                                      # (learns the ratio of this geometry)
+        for k in _ext._ratio_hint if ratio else ():
+            _ext._ratio_hint[k] = ratio
+        y, z = down(x), subm(plain(SparseTensor(feats, inds, [20] * 3, 2)))
+        return x, y, z
+
+    def exact(e):
+        return e[0], e[1], e[2].materialize() if isinstance(e[2], _ext.LazyPairs) else e[2], e[3]
+
+    with torch.no_grad():
+        ahead, _ext.AHEAD = _ext.AHEAD, False
+        try:
+            x, y, z = run()
+            want = [exact(t.find_indice_pair(k)) for t, k in ((x, "down"), (z, "subm"))]
+        finally:
+            _ext.AHEAD = ahead
+        for asked in (0, 1):
+            x, y, z = run(1e-4 if overflow else None)
+            assert y.pending() == z.pending() == _ext.AHEAD
+            found = [t.indice_dict[k] if direct and not (overflow and k == "subm") else t.find_indice_pair(k)
+                     for t, k in (((x, y)[asked], "down"), (z, "subm"))]
+            for e, ref in zip(found, want):
+                assert len(e) == 5 and all(torch.equal(a, b) for a, b in zip(exact(e)[:2] + exact(e)[3:], ref[:2] + ref[3:]))
+                for k, n in enumerate(ref[3].tolist()):       # (the lists behind their counts are undefined)
+                    assert torch.equal(exact(e)[2][k, :, :n], ref[2][k, :, :n])
+            assert torch.equal(y.indices, want[0][0]) and torch.equal(z.indices, want[1][0])
+    _ext.check_status(cuda)
+
+
+def test_kept_rulebooks_do_not_hold_their_input(cuda):
+    """A pass leaves nothing behind that only the cycle collector frees."""
+    import gc
+    import weakref
+    from ss_conv.sp_ops.conv import SparseConvolution
+    from ss_conv.sp_ops.tensor import SparseTensor
+    inds = dev(random_voxels(np.random.RandomState(9), 1, 16, 500), cuda)
+    down = SparseConvolution(3, 8, 8, 3, stride=2, padding=1, bias=False, indice_key="down").to(cuda)
+    gc.disable()
+    try:
+        with torch.no_grad():
+            for _ in range(2):
+                x = SparseTensor(torch.randn(inds.shape[0], 8, device=cuda), inds, [16] * 3, 1)
+                y, gone = down(x), weakref.ref(x)
+                y.features
+                del x, y
+                assert gone() is None
+    finally:
+        gc.enable()
