@@ -4,6 +4,7 @@ Usage: python ss-conv_b200/build.py [--force] [--verbose]
 The shared library is written next to the Python package (ss_conv/libssconv_b200.so) so that
 it travels with the source tree; no JIT cache is involved.
 """
+import importlib.metadata
 import os
 import subprocess
 import sys
@@ -13,6 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "ss_conv", "libssconv_b200.so")
 BINDINGS = os.path.join(HERE, "ss_conv", "_host.so")
+MADE_FOR = os.path.join(HERE, "build", "_host.versions")
 SOURCES = ["ssc_error.cu", "ssc_rulebook.cu", "ssc_conv.cu", "ssc_conv_tc.cu", "ssc_conv_stage.cu", "ssc_conv_pairs.cu", "ssc_backward.cu", "ssc_order.cu", "ssc_wgrad_tc.cu", "ssc_pool.cu", "ssc_layer.cu", "ssc_voxel.cu",
            "ssc_bnact.cu", "ssc_ceiling.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -30,10 +32,23 @@ def _newest_input():
     return max(os.path.getmtime(f) for f in files if os.path.exists(f))
 
 
+def _versions():
+    """What the bindings are bound to besides their sources."""
+    return "python %s, torch %s" % (sys.version, importlib.metadata.version("torch"))
+
+
+def bindings_current(inputs):
+    """The bindings are newer than their sources and made for this Python and this torch."""
+    if not (os.path.exists(BINDINGS) and os.path.exists(MADE_FOR)):
+        return False
+    with open(MADE_FOR) as f:
+        return f.read() == _versions() and os.path.getmtime(BINDINGS) >= max(os.path.getmtime(i) for i in inputs)
+
+
 def build_bindings(force=False):
     """ss_conv/_host.so: needs the headers of Python and torch, no GPU toolkit."""
     inputs = [os.path.join(CSRC, "ssc_host.cpp"), os.path.join(HERE, "..", "include", "ssconv_b200.h")]
-    if os.path.exists(BINDINGS) and not force and os.path.getmtime(BINDINGS) >= max(os.path.getmtime(f) for f in inputs):
+    if not force and bindings_current(inputs):
         return BINDINGS
     import sysconfig
     import torch
@@ -46,6 +61,9 @@ def build_bindings(force=False):
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed on ssc_host.cpp:\n" + r.stderr[-6000:])
+    os.makedirs(os.path.dirname(MADE_FOR), exist_ok=True)
+    with open(MADE_FOR, "w") as f:
+        f.write(_versions())
     return BINDINGS
 
 

@@ -14,10 +14,11 @@ import threading
 
 import torch
 
+_host_error = None
 try:
     from . import _host                  # the C ABI's bindings (csrc/ssc_host.cpp)
-except ImportError:
-    _host = None
+except ImportError as _e:                # not built, or built for another Python or torch: lib() says which
+    _host, _host_error = None, _e
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # SSCONV_B200_LIB selects another build of the same library (e.g. a debug build)
@@ -167,8 +168,8 @@ def lib():
     global _lib_handle
     if _lib_handle is None:
         if not os.path.exists(LIB_PATH) or (_host is None and "SSCONV_B200_LIB" not in os.environ):
-            raise RuntimeError("libssconv_b200.so or its bindings _host.so are missing: run `python ss-conv_b200/build.py` "
-                               "(there is no CPU or PyTorch fallback)")
+            raise RuntimeError("libssconv_b200.so or its bindings _host.so are missing or do not load (%s): run "
+                               "`python ss-conv_b200/build.py` (there is no CPU or PyTorch fallback)" % (_host_error,)) from _host_error
         if "SSCONV_B200_LIB" not in os.environ:
             _lib_handle = _host
             return _host

@@ -218,6 +218,33 @@ def test_kernels_saved_with_fewer_tables_are_completed(monkeypatch):
     assert all(torch.equal(a, b) for a, b in zip(seen[0][4:8], full[2:]))
 
 
+def test_bindings_of_another_python_or_torch_are_rebuilt_and_named(monkeypatch, tmp_path):
+    """build.py looks at the versions the bindings were made for; lib() passes on why they did not load."""
+    import importlib.util
+    from ss_conv import _ext
+    spec = importlib.util.spec_from_file_location("ssconv_build_under_test", os.path.join(os.path.dirname(os.path.dirname(_ext.__file__)), "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    source, made_for = tmp_path / "s.cpp", tmp_path / "versions"
+    source.write_text("")
+    binary = tmp_path / "b.so"
+    binary.write_text("")
+    monkeypatch.setattr(build, "BINDINGS", str(binary))
+    monkeypatch.setattr(build, "MADE_FOR", str(made_for))
+    assert not build.bindings_current([str(source)])            # nobody knows what they were made for
+    made_for.write_text(build._versions())
+    assert build.bindings_current([str(source)])
+    made_for.write_text(build._versions().replace("torch ", "torch 1."))
+    assert not build.bindings_current([str(source)])
+    monkeypatch.setattr(_ext, "_lib_handle", None)
+    monkeypatch.setattr(_ext, "_host", None)
+    monkeypatch.setattr(_ext, "_host_error", ImportError("undefined symbol"))
+    monkeypatch.delenv("SSCONV_B200_LIB", raising=False)
+    with pytest.raises(RuntimeError, match="undefined symbol") as raised:
+        _ext.lib()
+    assert raised.value.__cause__ is _ext._host_error
+
+
 def test_argument_errors_without_gpu():
     """Size queries and argument validation run on the host only."""
     from ss_conv import _ext
