@@ -236,7 +236,8 @@ __device__ __forceinline__ void cp_async_wait(int n) {
     default: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
   }
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+// All of the thread's copies, committed to a group or not (copies that arrive on a barrier by themselves never are).
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // The two 16-byte pieces a lane copies of a row (none if `from` is negative), OFF bytes into its part of the slot;
 // predicated instead of branched around: the instructions around the copies are what the producers' time goes into.
