@@ -60,6 +60,10 @@ int ssc_count_wait(void *place, int *out, void *stream);
 int ssc_count_close(void *place);
 /* Posts *n_dev (and *status) to a place from a kernel of its own, behind what is queued on `stream`. */
 int ssc_count_post(const int32_t *n_dev, const int32_t *status, void *place, void *stream);
+/* A word in mapped host memory, one for the process, that a kernel whose bounded wait ran out sets to non-zero after it has
+ * set its status word (16).  The host may look at it at any time without waiting and clears it itself.  Kernels
+ * launched before the first call, and everything where NULL is returned, have no alarm. */
+int32_t *ssc_alarm_open(void);
 /* 1 if the tcgen05 tensor-core kernels were compiled in (always for sm_100a builds). */
 int ssc_has_tcgen05(void);
 

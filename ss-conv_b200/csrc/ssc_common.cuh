@@ -80,6 +80,9 @@ inline uint32_t hash_buckets_for(int n) {
 int bitmap_decode(const uint32_t *bitmap, const uint32_t *word_prefix, long long n_words, const int shape[3],
                   int n_out, int32_t *out_indices, cudaStream_t st);
 
+// The process's alarm (ssc_alarm_open), null while nobody has opened it.
+int32_t *alarm_word();
+
 // A count for the host (ssc_count_open): status word and count, then the number the host watches for.
 struct CountPost {
   int32_t *host;        // null: nobody asked
@@ -89,6 +92,16 @@ CountPost next_post(void *place);
 void launch_post(const CountPost &post, const int32_t *n_dev, const int32_t *status, cudaStream_t st);
 
 #ifdef __CUDACC__
+// (one thread) a bounded wait ran out and the output is incomplete: status bit 16, then the alarm, which the host sees
+// without reading anything back.
+static __device__ __forceinline__ void report_expired(int32_t *status, int32_t *alarm) {
+  if (status != nullptr) atomicOr(status, 16);
+  if (alarm != nullptr) {
+    __threadfence_system();
+    *(volatile int32_t *)alarm = 16;
+  }
+}
+
 static __device__ __forceinline__ void post_count(const CountPost &post, int32_t count, const int32_t *status) {
   volatile int32_t *dst = post.host;
   dst[1] = status != nullptr ? *(const volatile int32_t *)status : 0;

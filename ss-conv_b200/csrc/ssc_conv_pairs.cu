@@ -65,6 +65,7 @@ struct PlParams {
   int threads;
   int ctas_per_sm;
   uint32_t idesc;
+  int32_t *alarm;   // mapped host word that tells of an expired wait (may be NULL)
   int f16;          // kind::f16 (fp16 / bf16 operands) instead of kind::tf32
 };
 
@@ -480,7 +481,7 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
 
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && *abort_flag && status) atomicOr(status, 16);
+  if (tid == 0 && *abort_flag) report_expired(status, p.alarm);
   if (warp == mma_warp) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(2 * p.acc_cols))
                  : "memory");
@@ -544,6 +545,7 @@ int conv_fwd_pairs(const void *staged, int c_in, const void *packed, int K, int 
   PlParams p;
   if (K > 256 || !pl_params(c_in, c_out, precision, p))
     return fail(SSC_ERR_INVALID, "conv_fwd_pairs: shape (c_in %d, c_out %d, kernel volume %d) not covered by the pair-list kernel", c_in, c_out, K);
+  p.alarm = alarm_word();
   int n_ctas = sm_count() * p.ctas_per_sm;
   if (n_ctas > PL_MAX_CTAS) n_ctas = PL_MAX_CTAS;
   int32_t *hdr = (int32_t *)strip_mem;

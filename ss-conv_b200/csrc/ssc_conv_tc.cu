@@ -55,6 +55,7 @@ struct TcParams {
   int last_kk;    // MMA k-steps (32 bytes of K each) that hold real channels in the LAST slab: 1..4
   int opk;        // kernel offsets per 128-byte operand row: 1, or 32 / c_pad for TF32 layers with c_pad = 4, 8, 16
   int rev;        // 1: the table's row of kernel offset kappa is K - 1 - kappa (the transpose of a centred submanifold table)
+  int32_t *alarm; // mapped host word that tells of an expired wait (may be NULL)
   int nbr_by_pos; // 1: the table's columns are already in the order of `order` (column j <-> output row order[j])
                   // channels (a first layer with 3 input channels packs 8 offsets into one step)
 };
@@ -66,6 +67,7 @@ static bool tc_params(int c_in, int c_out, TcParams &p, bool split_n = false, bo
   p.opk = opk;
   p.nbr_by_pos = 0;
   p.rev = 0;
+  p.alarm = nullptr;
   if (opk > 1) {     // grouped offsets: one full slab per group of offsets
     p.k_slabs = 1;
     p.last_kk = 4;
@@ -581,7 +583,7 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
   if (warp == mma_warp && lane == 0 && *abort_flag && n_iter > 0) mbar_wait_drain(smem_u32(done_bar), 0u);
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && *abort_flag && status) atomicOr(status, 16);
+  if (tid == 0 && *abort_flag) report_expired(status, p.alarm);
   if (warp == mma_warp) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols)
                  : "memory");
@@ -1014,7 +1016,7 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && *abort_flag && status) atomicOr(status, 16);
+  if (tid == 0 && *abort_flag) report_expired(status, p.alarm);
   if (warp == mma_warp) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols) : "memory");
   }
@@ -1109,6 +1111,7 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
   p.fmt16 = bf16 ? 1 : 0;
   p.nbr_by_pos = ((table_form & SSC_CONV_TABLE_IN_ORDER) && order) ? 1 : 0;
   p.rev = (table_form & SSC_CONV_TABLE_REVERSED) ? 1 : 0;
+  p.alarm = alarm_word();
   if (!prestaged) {
     int rc = stage_features_16(features, n_in, c_in, bf16, scratch, st);
     if (rc != SSC_OK) return rc;
@@ -1135,6 +1138,7 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
   if (!rows_params(c_in, c_out, n_out, p, opk)) return fail(SSC_ERR_INVALID, "conv_fwd(tf32): c_out %d / kernel volume %d not supported", c_out, K);
   p.nbr_by_pos = ((table_form & SSC_CONV_TABLE_IN_ORDER) && order) ? 1 : 0;
   p.rev = (table_form & SSC_CONV_TABLE_REVERSED) ? 1 : 0;
+  p.alarm = alarm_word();
   size_t smem = tc_smem_bytes(p);
   // With a staging buffer the feature rows are rounded to TF32 once, up front, instead of after
   // every gather (a row is gathered about K/2 times).

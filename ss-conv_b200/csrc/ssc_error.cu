@@ -26,6 +26,12 @@ static unsigned long long g_launches = 0;
 void note_launches(int n) { __atomic_fetch_add(&g_launches, (unsigned long long)n, __ATOMIC_RELAXED); }
 unsigned long long launches() { return __atomic_load_n(&g_launches, __ATOMIC_RELAXED); }
 
+// Kernels that give up set this word too, besides their status word: row counts are posted to the host before the
+// convolution behind them has run, so nothing that is read back tells of it in time.  Mapped host memory, kept
+// for the life of the process (recorded graphs hold its address).
+static int32_t *g_alarm = nullptr;
+int32_t *alarm_word() { return __atomic_load_n(&g_alarm, __ATOMIC_ACQUIRE); }
+
 // Read-back of a few device words.  What bounds it is latency: through a device-to-host copy and a stream
 // synchronisation one word costs 20 - 25 us after the last kernel (staging of the pageable
 // destination, copy engine start, completion interrupt path); a one-warp kernel that stores the
@@ -200,6 +206,21 @@ extern "C" int ssc_read_words(const int32_t *const *words, int n, int32_t *out, 
     if (int e = ssc::read_some(words + i, m, out + i, ssc::as_stream(stream))) return e;
   }
   return SSC_OK;
+}
+
+extern "C" int32_t *ssc_alarm_open(void) {
+  using namespace ssc;
+  std::lock_guard<std::mutex> hold(g_places_lock);
+  if (alarm_word() == nullptr) {
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
+    memset(p, 0, 64);
+    __atomic_store_n(&g_alarm, (int32_t *)p, __ATOMIC_RELEASE);
+  }
+  return alarm_word();
 }
 
 extern "C" int ssc_version(void) { return 100; }

@@ -95,6 +95,7 @@ PyObject *result(long long v) { return PyLong_FromLongLong(v); }
 PyObject *result(unsigned long v) { return PyLong_FromUnsignedLong(v); }
 PyObject *result(unsigned long long v) { return PyLong_FromUnsignedLongLong(v); }
 PyObject *result(void *v) { return PyLong_FromVoidPtr(v); }
+PyObject *result(int32_t *v) { return PyLong_FromVoidPtr(v); }
 PyObject *result(const char *v) { return PyBytes_FromString(v ? v : ""); }
 
 template <auto Fn, typename R, typename... A, size_t... I>
@@ -196,7 +197,7 @@ PyObject *head(PyObject *, PyObject *const *args, Py_ssize_t n) {
 }
 
 #define SSC_FUNCTIONS \
-  X(ssc_version) X(ssc_last_error) X(ssc_has_tcgen05) X(ssc_kernel_launches) X(ssc_read_words) X(ssc_count_open) X(ssc_count_wait) X(ssc_count_close) X(ssc_count_post) \
+  X(ssc_version) X(ssc_last_error) X(ssc_has_tcgen05) X(ssc_kernel_launches) X(ssc_read_words) X(ssc_count_open) X(ssc_count_wait) X(ssc_count_close) X(ssc_count_post) X(ssc_alarm_open) \
   X(ssc_rulebook_scratch_bytes) X(ssc_rulebook_subm) X(ssc_rulebook_subm_static) X(ssc_rulebook_subm_ahead) \
   X(ssc_rulebook_conv_count) X(ssc_rulebook_conv_fill) X(ssc_rulebook_conv_ahead) X(ssc_pairs_to_nbr) X(ssc_pairs_from_nbr_scratch_bytes) \
   X(ssc_pairs_from_nbr) X(ssc_materialize) X(ssc_materialize_bwd) X(ssc_conv_packed_bytes) X(ssc_conv_pack_filters) \

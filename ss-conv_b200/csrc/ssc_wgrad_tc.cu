@@ -132,6 +132,7 @@ struct WtParams {
   int x_round, y_round;        // 1: rows still to be rounded to TF32
   int n_pad, a_bytes, stage_bytes, stages, n_buf;
   uint32_t buf_cols;
+  int32_t *alarm;              // mapped host word that tells of an expired wait (may be NULL)
 };
 
 // smem descriptor halves of an MN-major operand: 32-channel blocks WT_BLOCK bytes apart (leading offset), four
@@ -347,7 +348,7 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && *abort_flag && status) atomicOr(status, 16);
+  if (tid == 0 && *abort_flag) report_expired(status, p.alarm);
   if (warp == mma_warp) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.buf_cols * (uint32_t)p.n_buf) : "memory");
   }
@@ -553,7 +554,7 @@ int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int
     cudaError_t e = cudaFuncSetAttribute(conv_wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_wgrad(tf32): smem attribute: %s", cudaGetErrorString(e));
     const WtParams w = {features, out_grad, c_in, c_out, (staged & 1) ? (c_in + 3) & ~3 : c_in, (staged & 2) ? (c_out + 3) & ~3 : c_out,
-                        (staged & 1) ? 0 : 1, (staged & 2) ? 0 : 1, p.n_pad, p.a_bytes, p.stage_bytes, p.stages, p.n_buf, p.buf_cols};
+                        (staged & 1) ? 0 : 1, (staged & 2) ? 0 : 1, p.n_pad, p.a_bytes, p.stage_bytes, p.stages, p.n_buf, p.buf_cols, alarm_word()};
     { conv_wgrad_tc_kernel<<<dim3(p.shares, p.co_blocks), (p.stages + 5) * 32, p.smem, st>>>(w, pl.pair_out, pl.pair_in, pl.starts, K, partial, status); note_launches(1); }
     SSC_CHECK_LAUNCH("conv_wgrad_tc");
   } else if (p.small) {

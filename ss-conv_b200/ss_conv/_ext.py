@@ -53,6 +53,7 @@ SIGNATURES = {
     "ssc_count_wait": (c_int, [c_void_p, ctypes.POINTER(c_int), c_void_p]),
     "ssc_count_close": (c_int, [c_void_p]),
     "ssc_count_post": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p]),
+    "ssc_alarm_open": (c_void_p, []),
     "ssc_rulebook_scratch_bytes": (c_size_t, [c_int, c_int, _I3, _I3, c_int]),
     "ssc_rulebook_subm": (c_int, [c_void_p, c_int, c_int, _I3, _I3, _I3, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_void_p, c_size_t, c_void_p]),
@@ -229,6 +230,8 @@ def _check(rc):
         if rc == 1:
             raise ValueError("ssconv_b200: " + msg)
         raise RuntimeError("ssconv_b200 (code %d): %s" % (rc, msg))
+    if _alarm is not None and _alarm.value:
+        _raise_on_alarm()
 
 
 def _p(t, dtype=None):
@@ -275,6 +278,7 @@ def _i3(v):
 
 
 _status = {}
+_alarm = None          # the process's alarm word (ssc_alarm_open): a kernel gave up somewhere, looked at in every call
 _scratch_cache = {}
 
 
@@ -282,8 +286,32 @@ def status_word(device):
     """Per-device int32 that kernels OR error bits into (read it with check_status())."""
     key = (device if isinstance(device, torch.device) else torch.device(device)).index
     if key not in _status:
+        _open_alarm()
         _status[key] = torch.zeros(1, dtype=torch.int32, device=device)
     return _status[key]
+
+
+def _open_alarm():
+    global _alarm
+    if _alarm is None and not torch.cuda.is_current_stream_capturing():
+        where = lib().ssc_alarm_open()
+        _alarm = c_int.from_address(where) if where else None
+
+
+def _raise_on_alarm():
+    """A kernel's bounded wait ran out at some time before this call: its output, handed out or not, is incomplete.  The
+    status words of all devices say what there is to say and are cleared."""
+    if torch.cuda.is_current_stream_capturing():
+        return                                      # (they cannot be read now; the alarm stays)
+    _alarm.value = 0
+    bits = 0
+    for word in list(_status.values()):
+        v = int(word.item())
+        if v:
+            word.zero_()
+            bits |= v
+    if bits:                                        # (else somebody has read and raised it since)
+        raise RuntimeError("ssconv_b200 kernel status 0x%x (%s)" % (bits, _STATUS_TEXT))
 
 
 def check_status(device=None):
@@ -308,9 +336,10 @@ def raise_on_status(value, device):
 
 
 def read_counts(words):
-    """Host values of device row counts (int32 words of one device).  The per-device status word rides
-    along in the same read-back, so a kernel that gave up (bounded wait, full hash, bad coordinate)
-    surfaces here, where the host waits for the device anyway, instead of handing out partial results.
+    """Host values of device row counts (int32 words of one device).  The per-device status word rides along, as it
+    stood when the count was found: bad coordinates and a full hash surface here, with the rows they spoil.  A
+    convolution behind a posted count is still running then; if one gives up (a bounded wait inside it runs
+    out), the next call into the library, this one included, raises (_raise_on_alarm).
     One small kernel writes the words into mapped host memory and the host watches for them there: a
     copy engine and a stream synchronisation per read cost several times as much."""
     dev = words[0].device
@@ -326,8 +355,7 @@ def read_counts(words):
 
 class CountPost(object):
     """A place in mapped host memory to which the kernel that finds a row count posts it (ssc_count_open), and
-    the value once it has come.  What the status word reports after that kernel surfaces with the next count
-    that is read, as it does behind layers on exact rows."""
+    the value once it has come."""
 
     __slots__ = ("place", "value", "lock")
 

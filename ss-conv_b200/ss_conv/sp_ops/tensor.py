@@ -216,7 +216,7 @@ class SparseTensor(object):
         if _capture_log is not None:
             raise RuntimeError("a row count cannot be read back while a CUDA graph is being recorded: this layer "
                                "needs exact row counts and cannot be part of a captured chain")
-        r.read()                            # the kernel status word is checked in the same read-back
+        r.read()                            # (raises what the status word reports, see _ext.read_counts)
         parent_changed = r.parent.resolve() if r.parent is not None else False
         n = r.count.value
         if r.note is not None and not parent_changed:

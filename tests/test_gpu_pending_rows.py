@@ -262,3 +262,39 @@ def test_kept_rulebooks_do_not_hold_their_input(cuda):
                 assert gone() is None
     finally:
         gc.enable()
+
+
+def test_a_kernel_that_gives_up_behind_a_posted_count_is_reported(cuda):
+    """The status word and the alarm as such a kernel leaves them, behind the kernel that posted the count: the next look at
+    the rows raises, once; so does any other call; a status word alone is what check_status is for."""
+    from ss_conv import _ext
+    from ss_conv.pool import MaxPool
+    from ss_conv.sp_ops.tensor import SparseTensor
+    inds = dev(random_voxels(np.random.RandomState(3), 2, 16, 300), cuda)
+    feats = torch.randn(inds.shape[0], 8, device=cuda)
+    pool = MaxPool(2, stride=2)
+
+    def run():
+        return pool(SparseTensor(feats, inds, [16] * 3, 2))
+
+    def expire(alarm=True):
+        torch.cuda.synchronize()
+        _ext.status_word(cuda).fill_(16)
+        _ext._alarm.value = 16 if alarm else 0
+
+    with torch.no_grad():
+        n = run().features.shape[0]
+        y = run()
+        expire()
+        with pytest.raises(RuntimeError, match="0x10"):
+            y.features
+        assert y.features.shape[0] == n and int(_ext.status_word(cuda)) == 0
+        expire()
+        with pytest.raises(RuntimeError, match="0x10"):
+            run()
+        assert run().features.shape[0] == n
+        y = run()
+        expire(alarm=False)
+        with pytest.raises(RuntimeError, match="0x10"):
+            _ext.check_status(cuda)
+        assert y.features.shape[0] == n

@@ -245,6 +245,25 @@ def test_bindings_of_another_python_or_torch_are_rebuilt_and_named(monkeypatch, 
     assert raised.value.__cause__ is _ext._host_error
 
 
+def test_an_alarm_is_raised_once_by_the_next_call(monkeypatch):
+    """A kernel that gives up sets the alarm besides its status word: whatever call comes next raises what the status words
+    report and clears them.  While a graph is recorded nothing can be read, so the alarm stays."""
+    from ss_conv import _ext
+    capturing = [True]
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    monkeypatch.setattr(_ext, "_alarm", ctypes.c_int(16))
+    monkeypatch.setattr(_ext, "_status", {0: torch.zeros(1, dtype=torch.int32), 1: torch.tensor([16], dtype=torch.int32)})
+    _ext._check(0)
+    capturing[0] = False
+    with pytest.raises(RuntimeError, match="0x10"):
+        _ext._check(0)
+    assert _ext._alarm.value == 0 and int(_ext._status[1]) == 0
+    _ext._check(0)
+    _ext._alarm.value = 16                        # reported since by somebody who read the status word
+    _ext._check(0)
+    assert _ext._alarm.value == 0
+
+
 def test_argument_errors_without_gpu():
     """Size queries and argument validation run on the host only."""
     from ss_conv import _ext
