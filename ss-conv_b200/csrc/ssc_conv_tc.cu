@@ -1,23 +1,20 @@
 // Output-stationary gather-GEMM on the 5th-generation tensor cores (tcgen05, sm_100a).
 //
-// One CTA owns 128 consecutive output rows and runs a warp-specialised pipeline over the
-// steps (kernel offset with a neighbour in the tile) x (32-channel slab of the input).  The
-// operand ring has one slot per producer warp:
-//   * producer warp w owns ring slot w and prepares the steps w, w+S, w+2S, ...: each lane
-//     looks up the neighbour rows of its four output rows and pulls the 128-byte slab of every
-//     present feature row with cp.async straight into the K-major 128-byte-swizzled operand
-//     layout; rows without a neighbour stay zero (a slot row is cleared again only if it held
-//     data before).  When its copies have landed the lane rounds its rows fp32 -> TF32 (round
-//     to nearest) in place and arrives on the slot's "A full" mbarrier.  Lane 0 also brings in
-//     the pre-packed filter slab (already TF32, already in operand layout) with one bulk
-//     asynchronous copy that completes on the "B full" mbarrier.  The global-memory latency
-//     of a step is paid inside one warp while the other warps work on the neighbouring steps.
-//   * one MMA warp: a single thread waits for both barriers of a slot, issues tcgen05.mma
-//     (M=128, N<=256, K=8 per instruction) accumulating in tensor memory (fp32), and commits
-//     the group to the slot's "empty" mbarrier, which lets the owner refill the slot.
-// There is no CTA-wide barrier inside the loop.  Accumulators stay in TMEM across all
-// offsets; four warps then read them with tcgen05.ld and write each output row exactly once
-// (no scatter atomics, deterministic order).
+// One CTA owns 128 output rows (consecutive ones, or those of a row order) and runs a warp-specialised pipeline over the
+// steps (kernel offset) x (128-byte slab of the input's channels); the operand ring has up to eight slots:
+//   * producer warps fetch the rows' neighbours into the slot, in the K-major 128-byte-swizzled operand layout;
+//     the pre-packed filter slab (already rounded, already in operand layout) comes with one bulk
+//     asynchronous copy, and both arrive on the slot's "full" mbarrier.
+//   * one MMA warp waits for it, issues tcgen05.mma (M=128, N<=256), accumulating in tensor memory (fp32),
+//     rows without a neighbour switched off by the output-lane mask, and commits the group to the slot's
+//     "empty" mbarrier, which frees the slot.
+// There is no CTA-wide barrier inside the loop.  Accumulators stay in tensor memory across all offsets; the
+// producer warps then read them with tcgen05.ld and write each output row exactly once (no scatter
+// atomics, one stated order of the sums).
+// Two kernels share this plan.  conv_fwd_rows_kernel is the one the layers run: rows staged once (rounded to TF32, or
+// fp16 / bf16), four warps to a slot.  conv_fwd_tf32_kernel takes what it does not cover: layers of up to 16
+// input channels, several offsets per operand row (GROUPED), and fp32 rows without a staging buffer, rounded
+// in shared memory (callers that bring no scratch); a producer warp per slot there.
 //
 // Every wait on an mbarrier is bounded: on expiry the thread records an error in `status`
 // through a shared flag, every other wait then gives up too, and the kernel frees its tensor
@@ -34,7 +31,6 @@ constexpr int TC_MAX_STAGES = 8;       // producer warps = ring slots
 constexpr int TC_EPI_WARPS = 4;        // warps 0..3 also run the epilogue (one TMEM lane quarter each)
 constexpr int TC_A_BYTES = TC_M * 128;
 constexpr int TC_CTRL_BYTES = 1024;
-constexpr int TC_LIST_BYTES = TC_M * 5;   // a slot's list of present rows: 128 source rows, 128 rows of the tile
 
 struct TcParams {
   int k_slabs;    // ceil(c_in / 32)
@@ -90,7 +86,7 @@ static bool tc_params(int c_in, int c_out, TcParams &p, bool split_n = false, bo
   p.fmt16 = 0;
   p.k_groups = (p.k_slabs + p.sps - 1) / p.sps;
   int stage = p.sps * (TC_A_BYTES + p.b_bytes);
-  // behind the slots: control block, a list of 128 rows (5 bytes each) per slot, alignment slack
+  // behind the slots: control block, alignment slack
   int fixed = TC_CTRL_BYTES + 1024;
   // Resident CTAs hide each other's per-step latencies, so take as many per SM as tensor
   // memory (512 columns) and shared memory (two ring slots each at least) allow, up to four.
@@ -99,7 +95,6 @@ static bool tc_params(int c_in, int c_out, TcParams &p, bool split_n = false, bo
   int ctas = 512 / p.tmem_cols;
   if (ctas > 4) ctas = 4;
   if (one_cta_per_sm) ctas = 1;
-  stage += TC_LIST_BYTES;
   while (ctas > 1 && ((227 * 1024) / ctas - 1024 - fixed) / stage < 2) --ctas;
   p.stages = ((227 * 1024) / ctas - 1024 - fixed) / stage;
   if (p.stages > TC_MAX_STAGES) p.stages = TC_MAX_STAGES;
@@ -171,9 +166,9 @@ __global__ void pack_filters_tf32_grouped_kernel(const float *__restrict__ filte
 
 // Warps 0 .. n_prod-1 are producers (warp w <-> ring slot w; with fewer than four slots the
 // spare warps only help in the prologue and epilogue), the last warp issues the MMAs.
-// F16: the staged image and the filter slabs hold fp16 (64 channels per 128-byte row); the
-// gather is the same byte-for-byte, `c_in` is then the row length in 4-byte units.
-template <bool STAGED, bool F16 = false, bool GROUPED = false>
+// GROUPED: staged rows of few channels, several kernel offsets per operand row; else fp32 rows as they are, rounded
+// in shared memory.
+template <bool GROUPED>
 __global__ void __launch_bounds__((TC_MAX_STAGES + 1) * 32)
 conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *__restrict__ packed, int K,
                      int c_out, const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out,
@@ -373,14 +368,6 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
         par ^= 1u;
       }
     } else {
-    // The rows of a step that have a neighbour are put into a list first (local row and source row), eight lanes
-    // then fetch the 128-byte line of a listed row: one L1 line and four sectors per row and a request for
-    // four rows per instruction.  With a lane per row every instruction asked L1 for the lines of all
-    // present rows of 32, and a 32-byte sector twice: eight slots of an SM kept its load unit busy.
-    const int list_at = slot * TC_M + q0 * 32;      // the warps of a slot share its 128 entries
-    int32_t *list_src = (int32_t *)(ctrl + TC_CTRL_BYTES) + list_at;
-    uint8_t *list_row = ctrl + TC_CTRL_BYTES + S * TC_M * 4 + list_at;
-    const int sub = lane & 7, grp = lane >> 3;
     if (slot < n_iter) load_rows(slot, nxt);
     for (int j = slot; j < n_iter; j += S) {
       const int act = j / p.k_groups, slab0 = (j - act * p.k_groups) * p.sps;
@@ -390,24 +377,8 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
       for (int q = 0; q < 4; ++q) src[q] = nxt[q];
       if (j + S < n_iter) load_rows(j + S, nxt);  // neighbour rows of this warp's next step
       unsigned have[4];
-      int listed = 0;
-      if (STAGED) {
-        __syncwarp();       // everybody is done with the list of the step before
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          have[q] = __ballot_sync(0xffffffffu, src[q] >= 0);
-          if (src[q] >= 0) {
-            const int at = listed + __popc(have[q] & ((1u << lane) - 1u));
-            list_src[at] = src[q];
-            list_row[at] = (uint8_t)(q * 32 + lane);
-          }
-          listed += __popc(have[q]);
-        }
-        __syncwarp();
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) have[q] = __ballot_sync(0xffffffffu, src[q] >= 0);
-      }
+      for (int q = 0; q < 4; ++q) have[q] = __ballot_sync(0xffffffffu, src[q] >= 0);
       if (j >= S) {
         if (!mbar_wait_warp(smem_u32(empty_bars + slot), par ^ 1u, abort_flag)) break;
         tc_fence_after();
@@ -426,22 +397,6 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 #pragma unroll
       for (int q = 0; q < 4; ++q)    // rows of this step that the MMA must leave alone
         if (lane == 0 && q >= q0 && q < q0 + q_per) slot_masks[slot * 4 + q] = ~have[q];
-      if (STAGED) {
-        present = listed > 0;
-        for (int ss = 0; ss < n_sub; ++ss) {
-          const int ch0 = (slab0 + ss) * TC_SLAB + sub * 4;
-          const bool ok = ch0 < c_in;            // pieces past the last channel are zero-filled
-          const float *fp = features + (ok ? ch0 : 0);
-          const uint32_t a_slab = slot_addr + (uint32_t)(ss * TC_A_BYTES);
-#pragma unroll 4
-          for (int i = grp; i < listed; i += 4) {
-            const uint32_t row = list_row[i];
-            const int s_row = list_src[i];
-            cp_async16_cg(a_slab + (row >> 3) * 1024u + (row & 7u) * 128u + (((uint32_t)sub ^ (row & 7u)) << 4),
-                          fp + (size_t)s_row * c_in, ok ? 16u : 0u);
-          }
-        }
-      } else {
       for (int ss = 0; ss < n_sub; ++ss) {
       const int ch0 = (slab0 + ss) * TC_SLAB;
 #pragma unroll
@@ -469,14 +424,13 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
         }
       }
       }
-      }
       cp_async_commit();
       cp_async_wait(0);
       // copies landed: round the gathered rows to TF32 in place
-      for (int ss = 0; ss < (STAGED ? 0 : n_sub); ++ss)
+      for (int ss = 0; ss < n_sub; ++ss)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        if (!STAGED && (present & (1u << q))) {
+        if (present & (1u << q)) {
           uint8_t *row = slot_ptr + (size_t)ss * TC_A_BYTES + row_off[q];
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
@@ -497,10 +451,8 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
     }   // one offset per step
   } else if (warp == mma_warp) {
     // ================================ MMA issuer: the whole warp, one elected lane issues ========
-    // slot index, parity and descriptor halves are running values
-    // fp32 accumulator; operand formats: kind::tf32 2 = TF32; kind::f16 0 = fp16, 1 = bf16
-    const uint32_t fmt = F16 ? (uint32_t)p.fmt16 : 2u;
-    const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.tile_n >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+    // slot index, parity and descriptor halves are running values; fp32 accumulator, TF32 operands
+    const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(p.tile_n >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
     const uint32_t a_lo0 = desc_lo(smem_base), slot_step = (uint32_t)stage_bytes >> 4, n_step = (uint32_t)(p.tile_n * 128) >> 4;
     const uint32_t fulla0 = smem_u32(fulla_bars), empty0 = smem_u32(empty_bars);
     uint32_t s = 0, par = 0, a_lo = a_lo0;
@@ -522,8 +474,7 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
               if (kk >= n_kk) break;
-              if (F16) mma_f16_ss_masked(dn, an + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
-              else mma_tf32_ss_masked(dn, an + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
+              mma_tf32_ss_masked(dn, an + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
             }
           }
         }
@@ -1023,7 +974,7 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
 }
 
 static size_t tc_smem_bytes(const TcParams &p) {
-  return (size_t)p.stages * p.sps * (TC_A_BYTES + p.b_bytes) + 1024 /*alignment slack*/ + TC_CTRL_BYTES + (size_t)p.stages * TC_LIST_BYTES;
+  return (size_t)p.stages * p.sps * (TC_A_BYTES + p.b_bytes) + 1024 /*alignment slack*/ + TC_CTRL_BYTES;
 }
 
 // 16-bit operands: filters [K, c_in, c_out] fp32 -> [K][k_slabs][n_pad rows][64 fp16 or bf16], same
@@ -1166,7 +1117,7 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
     kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, c_pad, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
   } else {
-    auto kernel = opk > 1 ? conv_fwd_tf32_kernel<true, false, true> : conv_fwd_tf32_kernel<false>;
+    auto kernel = opk > 1 ? conv_fwd_tf32_kernel<true> : conv_fwd_tf32_kernel<false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
     kernel<<<grid2, p.threads, smem, st>>>(staged ? (const float *)scratch : features, staged ? c_pad : c_in, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order);

@@ -765,11 +765,6 @@ extern "C" int ssc_rulebook_subm_static(const int32_t *indices, int n_in, int ba
   return SSC_OK;
 }
 
-namespace ssc {
-}  // namespace ssc
-
-using namespace ssc;
-
 extern "C" size_t ssc_rulebook_scratch_bytes(int n_in, int batch, const int in_shape[3], const int out_shape[3], int K) {
   if (n_in < 0 || batch < 1 || K < 1 || !in_shape || !out_shape) return 0;
   return carve(nullptr, n_in, batch, in_shape, out_shape, K).total;

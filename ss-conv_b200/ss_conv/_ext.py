@@ -837,7 +837,8 @@ def _resolve_precision(c_in, c_out, precision=None):
 
 # Output rows from which a call brings a staging buffer (a copy of its input rows, rounded once): always, since
 # the kernel on staged rows is the faster one also for a layer of a few tiles (512 rows of 120 -> 240 channels:
-# 104 us without).  Raise it to save the buffer's memory; the results have the same bits.
+# 104 us without).  Raise it to save the buffer's memory where layers are queued step by step; the results have the
+# same bits.  (Layers queued in one call always stage.)
 STAGING_MIN_ROWS = 0
 
 # Which tensor-core kernel a convolution call takes: 'auto' (by shape, see _use_pairs), 'rows' (the
@@ -891,7 +892,7 @@ def pair_lists(nbr):
 PRESTAGED = 0x100
 TABLE_IN_ORDER = 0x200
 TABLE_REVERSED = 0x1000
-WGRAD_X_STAGED, WGRAD_DY_STAGED = 0x400, 0x800
+WGRAD_DY_STAGED = 0x800
 # (features.data_ptr(), filters.data_ptr()) -> (prec, packed, scratch, nbytes) left by conv_prepare for the
 # conv_forward call that follows on the same tensors
 _prepared = {}
@@ -1209,10 +1210,10 @@ def stage_tf32(rows):
     return image
 
 
-def conv_wgrad(features, out_grad, nbr, precision=None, x_image=None, dy_image=None):
+def conv_wgrad(features, out_grad, nbr, precision=None, dy_image=None):
     """d_filters [K, Cin, Cout] = sum over output rows of gathered input rows (outer) out_grad rows
-    (tensor cores with TF32 operands or exact fp32, chosen like the forward pass).  x_image / dy_image:
-    the operands' TF32 images (stage_tf32) where the caller has them."""
+    (tensor cores with TF32 operands or exact fp32, chosen like the forward pass).  dy_image:
+    the TF32 image of out_grad (stage_tf32) where the caller has it."""
     K, n_out = nbr.shape
     c_in, c_out = features.shape[1], out_grad.shape[1]
     # the filter gradient has no 16-bit form: 'fp16' / 'bf16' take the TF32 kernel
@@ -1223,11 +1224,8 @@ def conv_wgrad(features, out_grad, nbr, precision=None, x_image=None, dy_image=N
     # (tables of more than 256 offsets have no lists: the exact kernel works on the table itself)
     lists = pair_lists(nbr) if n_out > 0 and K <= 256 and (mode == PREC_TF32 or c_in <= 16) else None
     x, dy = _p(features, torch.float32), _p(out_grad, torch.float32)
-    if mode == PREC_TF32 and c_in <= 256 and K <= 256:
-        if x_image is not None:
-            x, mode = _p(x_image), mode | WGRAD_X_STAGED
-        if dy_image is not None:
-            dy, mode = _p(dy_image), mode | WGRAD_DY_STAGED
+    if mode == PREC_TF32 and c_in <= 256 and K <= 256 and dy_image is not None:
+        dy, mode = _p(dy_image), mode | WGRAD_DY_STAGED
     _check(lib().ssc_conv_wgrad_lists(x, c_in, dy, c_out, _p(nbr, torch.int32), K, n_out, _p(lists),
                                       lists.numel() if lists is not None else 0, mode, _p(d_flt),
                                       _p(status_word(features.device)), _p(scratch), nbytes, _stream()))
@@ -1663,24 +1661,6 @@ def bn_gate_backward(x, gout, field_of_channel, scalar_of_channel, n_field, n_sc
                                  _p(scale), _p(shift), _p(chan_mean), _p(var), _p(weight), float(eps),
                                  int(bool(training)), _p(table), _p(start), _p(length), int(s_act), int(g_act), _p(gx),
                                  _p(d_w), _p(d_b), _p(scratch), nbytes, _stream()))
-    return gx, d_w, d_b[:n_scalar]
-
-
-def bn_backward(x, gy, field_of_channel, scalar_of_channel, n_field, n_scalar, mean, var, weight, eps, training):
-    """(gx [n, c], d_weight [n_field], d_bias [n_scalar]) of y = (x - mean) * weight / sqrt(var + eps) + bias;
-    training: mean / var are the batch statistics of x and the gradient flows through them."""
-    x, gy = x.contiguous(), gy.contiguous()
-    n, c = x.shape
-    gx = torch.empty_like(x)
-    d_w = _empty(n_field, torch.float32, x.device)
-    d_b = _empty(max(n_scalar, 1), torch.float32, x.device)
-    nbytes = int(lib().ssc_bn_scratch_bytes(n, c))
-    scratch = _empty(nbytes, torch.uint8, x.device)
-    mean_c = None if n_scalar == 0 else mean.contiguous()
-    _check(lib().ssc_bn_bwd(_p(x, torch.float32), _p(gy, torch.float32), n, c, _p(field_of_channel, torch.int32),
-                            _p(scalar_of_channel, torch.int32), int(n_field), int(n_scalar), _p(mean_c),
-                            _p(var.contiguous()), _p(weight), float(eps), int(bool(training)), _p(gx), _p(d_w), _p(d_b),
-                            _p(scratch), nbytes, _stream()))
     return gx, d_w, d_b[:n_scalar]
 
 

@@ -283,7 +283,7 @@ def test_training_step_through_conv_bn_gate(cuda):
 @pytest.mark.parametrize("training", [True, False])
 def test_batchnorm_and_gate_backward_kernels(cuda, training):
     """BatchNorm and the gated activation under autograd run the library's kernels in both
-    directions (ssc_bn_stats / ssc_bn_bwd / ssc_gate_bwd).  Gradients of the input and of the affine
+    directions (ssc_bn_train / ssc_bn_gate_bwd / ssc_gate_bwd).  Gradients of the input and of the affine
     parameters, the outputs and the updated running statistics against the same layers evaluated as a
     float64 composite of torch ops on the CPU (what the reference's autograd would compute,
     SS_Conv_lib/ss_conv/batchnorm.py:49-136, activation.py:55-100)."""

@@ -353,3 +353,45 @@ def test_norm_and_gate_gradients_of_very_wide_rows(cuda, Rs, n, training):
         close(x.grad, x64.grad)
     close(bn.weight.grad, bn64.weight.grad)
     close(bn.bias.grad, bn64.bias.grad)
+
+
+@pytest.mark.parametrize("n,training", [(1, True), (700, True), (700, False)])
+def test_norm_entry_points_for_c_callers(cuda, n, training):
+    """ssc_bn_stats and ssc_bn_bwd, which the layers no longer call, give the bits of the joined forms the layers do call."""
+    from ss_conv import _ext
+    from ss_conv._ext import lib, _p, _stream, _check
+    from ss_conv.batchnorm import _channel_tables
+    field, scalar = (torch.tensor(v, dtype=torch.int32, device=cuda) for v in _channel_tables([(3, 0), (2, 1), (1, 2)]))
+    c, n_field, n_scalar = 14, 6, 3
+    x, g, w = torch.randn(n, c, device=cuda) + 0.2, torch.randn(n, c, device=cuda), torch.rand(n_field, device=cuda) + 0.5
+    scratch = torch.empty(lib().ssc_bn_scratch_bytes(n, c), dtype=torch.uint8, device=cuda)
+    mean, var = torch.empty(n_scalar, device=cuda), torch.empty(n_field + c, device=cuda)
+    _check(lib().ssc_bn_stats(_p(x), n, c, _p(field), _p(scalar), n_field, n_scalar, _p(mean), _p(var), _p(scratch),
+                              scratch.numel(), _stream()))
+    m, v, chan_mean, scale, shift = _ext.bn_train(x, field, scalar, n_field, n_scalar, w, None, 1e-5, 0.1)
+    assert torch.equal(mean, m) and torch.equal(var[:n_field], v)
+    want = _ext.bn_gate_backward(x, g, field, scalar, n_field, n_scalar, scale, shift, chan_mean, v, w, 1e-5, training)
+    got = torch.empty_like(x), torch.empty(n_field, device=cuda), torch.empty(n_scalar, device=cuda)
+    _check(lib().ssc_bn_bwd(_p(x), _p(g), n, c, _p(field), _p(scalar), n_field, n_scalar, _p(mean), _p(var), _p(w), 1e-5,
+                            int(training), *(_p(t) for t in got), _p(scratch), scratch.numel(), _stream()))
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("c_in,c_out,n", [(16, 8, 1), (18, 22, 130), (64, 76, 400)])
+def test_filter_gradient_of_staged_operands(cuda, c_in, c_out, n):
+    """Operands that are rounded and padded already (the flags of ssc_conv_wgrad_lists, alone and together) give the bits of
+    those that the kernel rounds itself."""
+    from ss_conv import _ext
+    from ss_conv._ext import lib, _p, _stream, _check
+    rng = np.random.RandomState(n)
+    t = dev(_table(n, n, 27, 0.4, rng), cuda)
+    x, g = torch.randn(n, c_in, device=cuda), torch.randn(n, c_out, device=cuda)
+    want = _ext.conv_wgrad(x, g, t, precision="tf32")
+    lists, scratch = _ext.pair_lists(t), torch.empty(lib().ssc_conv_wgrad_scratch_bytes(27, c_in, c_out, n), dtype=torch.uint8, device=cuda)
+    for flags in (0x400, 0x800, 0xC00):
+        got = torch.empty_like(want)
+        a, b = (_ext.stage_tf32(v) if flags & f else v for v, f in ((x, 0x400), (g, 0x800)))
+        _check(lib().ssc_conv_wgrad_lists(_p(a), c_in, _p(b), c_out, _p(t), 27, n, _p(lists), lists.numel(), _ext.PREC_TF32 | flags,
+                                          _p(got), _p(_ext.status_word(cuda)), _p(scratch), scratch.numel(), _stream()))
+        assert torch.equal(got, want)
+    _ext.check_status(cuda)
