@@ -152,8 +152,9 @@ class Activation(nn.Module):
     def fusable_gate(self):
         """relu / sigmoid / identity without biases, at least one of them an activation: what the
         library's gate kernels cover in both directions."""
-        acts = [a for a in (self.scalar_act, self.gate_act) if a is not None]
-        return bool(acts) and all(a.bias is None for a in acts) and self.fusable()
+        scalar, gate = self._modules.get("scalar_act"), self._modules.get("gate_act")
+        return ((scalar is not None or gate is not None) and (scalar is None or scalar.bias is None)
+                and (gate is None or gate.bias is None) and self.fusable())
 
     def gate_tables(self, device):
         """(gate_of_channel, field_start, field_len, scalar act code, gate act code)."""

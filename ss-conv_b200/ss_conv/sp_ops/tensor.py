@@ -1,4 +1,6 @@
 """Sparse voxel tensor (interface of SS_Conv_lib/ss_conv/sp_ops/tensor.py:22-69)."""
+import copy
+
 import numpy as np
 import torch
 
@@ -279,6 +281,8 @@ class RunsAhead(object):
     """Mixin of the layers that run_ahead keeps plans on: they stay out of copies and saved modules (a plan is the memory of
     a structure of this build of the library, and made again in microseconds)."""
 
+    output_padding = ()
+
     def __getstate__(self):
         return {k: v for k, v in self.__dict__.items() if k != "_ahead_plans"}
 
@@ -292,22 +296,28 @@ def run_ahead(layer, input, op, output_shape, transpose, exact, weight=None, gat
     if not (feats.is_contiguous() and inds.is_contiguous()) or (weight is not None and weight.dtype != torch.float32):
         return None                             # (16-bit filters have entry points of their own)
     shape = tuple(input.spatial_shape)          # (a list, or an array)
-    c_in, c_out = (weight.shape[-2], weight.shape[-1]) if weight is not None else (feats.shape[1], 0)
-    if feats.shape[1] != c_in:
-        return None
+    c_in, c_out = feats.shape[1], 0
+    if weight is not None:
+        size = weight.shape
+        c_out = size[-1]
+        if size[-2] != c_in:
+            return None
     # everything a plan is made from: one pool may serve rows of several widths, a layer's geometry may be changed
     gated = gate[3:] if gate is not None else None
-    key = (shape, input.batch_size, feats.dtype, _ext._precision, _ext._storage, gated, c_in, c_out, transpose, *layer.kernel_size,
-           *layer.stride, *layer.padding, *layer.dilation, *getattr(layer, "output_padding", ()))
-    plans = layer.__dict__.setdefault("_ahead_plans", {})
-    plan = plans.get(key)
-    if plan is None:
+    key = (shape, input.batch_size, feats.dtype, _ext._precision, _ext._storage, gated, c_in, c_out, transpose)
+    geometry = (layer.kernel_size, layer.stride, layer.padding, layer.dilation, layer.output_padding)
+    plans = layer.__dict__.get("_ahead_plans")
+    if plans is None:
+        plans = layer.__dict__.setdefault("_ahead_plans", {})
+    kept = plans.get(key)
+    if kept is None or kept[2] != geometry:
         if len(plans) > 64:
             plans.clear()
         out_shape = output_shape(input.spatial_shape)
-        plan = plans[key] = (_ext.layer_plan(shape, out_shape, input.batch_size, layer.kernel_size, layer.stride, layer.padding,
-                                             layer.dilation, transpose, op, feats.dtype, c_in, c_out, gated), tuple(out_shape))
-    plan, out_shape = plan
+        kept = plans[key] = (_ext.layer_plan(shape, out_shape, input.batch_size, layer.kernel_size, layer.stride, layer.padding,
+                                             layer.dilation, transpose, op, feats.dtype, c_in, c_out, gated),
+                             tuple(out_shape), tuple(copy.copy(v) for v in geometry))
+    plan, out_shape, _ = kept
     if plan is None:
         return None
     made = _ext.layer_ahead(plan, inds, n_in_dev, feats, weight, gate)

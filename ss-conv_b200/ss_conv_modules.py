@@ -25,10 +25,9 @@ radial_window = partial(gaussian_window_wrapper, mode="compromise", border_dist=
 
 def _unwatched(module, kind):
     """The module is one of this package's own, and nothing waits for it to be called: what fuses it with its neighbours
-    must not pass by a subclass, a replaced forward or a hook of any kind."""
+    must not pass by a subclass, a replaced forward or a hook of any kind (hooks on all modules: _has_any_global_hook)."""
     return (type(module) is kind and "forward" not in module.__dict__
-            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
-            and not _has_any_global_hook())
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks))
 
 
 class SS_Conv(nn.Module):
@@ -67,10 +66,10 @@ class SS_Conv(nn.Module):
             return None
         parts = self._modules
         bn, act, conv = parts.get("bn"), parts.get("activation"), parts["conv"]
-        if (act is None or not _unwatched(conv, Convolution) or conv.training or conv.bias is not None
+        if (act is None or not _unwatched(conv, Convolution) or conv.training or conv._parameters.get("bias", 0) is not None
                 or not _unwatched(act, Activation) or (bn is not None and (bn.training or not _unwatched(bn, BatchNorm)))
-                or not act.fusable_gate()):
-            return None
+                or not act.fusable_gate() or _has_any_global_hook()):
+            return None                      # (a replica's bias is not among its parameters)
         device = x.raw()[0].device
         if device.type != "cuda":
             return None
@@ -84,7 +83,7 @@ class SS_Conv(nn.Module):
             return x if self.dropout is None else self.dropout(x)
         x = self.conv(x)
         both = None
-        if _unwatched(self.bn, BatchNorm) and _unwatched(self.activation, Activation):
+        if _unwatched(self.bn, BatchNorm) and _unwatched(self.activation, Activation) and not _has_any_global_hook():
             both = self.bn.norm_and_gate(x, self.activation)
         if both is not None:
             x = both
