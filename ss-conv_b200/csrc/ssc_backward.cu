@@ -96,7 +96,8 @@ __global__ void wgrad_reduce_kernel(const float *__restrict__ partial, int split
   out[e] = s;
 }
 
-// MODE 0: max pool (gradient goes to every input equal to the pooled value), 1: avg pool.  A block takes R input
+// MODE 0: max pool (gradient goes to every input equal to the pooled value), 1: avg pool over K, 2: avg pool over the
+// outputs' counts, which may be any.  A block takes R input
 // rows with their piece of the table in shared memory, as in the forward pass (one thread per row and
 // channel group walking the table: 48 us for 27 offsets of 60 k rows of 76 channels).
 template <int MODE, int PIECE>
@@ -107,7 +108,7 @@ pool_bwd_kernel(const float *__restrict__ features, const float *__restrict__ ou
   extern __shared__ int32_t pool_smem[];
   struct Item {
     Channels g, y;
-    float div;
+    int32_t count;
   };
   const PoolTile tile = pool_tile(nbr_in, K, n_in, n_in, R, pool_smem);
   const uint32_t cg = (uint32_t)(c + 3) / 4, items = (uint32_t)tile.rows * cg;
@@ -120,11 +121,17 @@ pool_bwd_kernel(const float *__restrict__ features, const float *__restrict__ ou
         [&](int o, Item &v) {
           load_rows<PIECE>(out_grad + (size_t)o * c + c0, valid, v.g);
           if (MODE == 0) load_rows<PIECE>(out_features + (size_t)o * c + c0, valid, v.y);
-          else v.div = summaryrf ? (float)__ldg(summaryrf + o) : (float)K;
+          else v.count = MODE == 2 || summaryrf ? __ldg(summaryrf + o) : K;     // (a constant count made MODE 1 6 % slower)
         },
         [&](int, const Item &v) {
-          if (MODE == 1) {
-            add_quotients(acc, v.g, v.div, __frcp_rn(v.div));
+          if (MODE != 0) {
+            const float div = (float)v.count;
+            if (MODE == 1 || whole_count(v.count)) {
+              add_quotients(acc, v.g, div, __frcp_rn(div));
+            } else {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) acc.v[q] += v.g.v[q] / div;
+            }
           } else {
 #pragma unroll
             for (int q = 0; q < 4; ++q)
@@ -312,7 +319,7 @@ static int launch_pool_bwd(const float *features, const float *out_features, con
                            const char *name) {
   SSC_REQUIRE(c > 0 && K > 0 && n_in >= 0, "%s: bad sizes", name);
   if (n_in == 0) return SSC_OK;
-  SSC_REQUIRE(out_grad && nbr_in && d_in && (MODE == 1 || (features && out_features)), "%s: null pointer", name);
+  SSC_REQUIRE(out_grad && nbr_in && d_in && (MODE != 0 || (features && out_features)), "%s: null pointer", name);
   const PoolShape p = pool_shape(n_in, K);
   SSC_REQUIRE(p.rows > 0, "%s: kernel of %d offsets is too large", name, K);
   const int piece = pool_piece(c, (uintptr_t)features | (uintptr_t)out_features | (uintptr_t)out_grad | (uintptr_t)d_in);
@@ -334,7 +341,8 @@ extern "C" int ssc_maxpool_bwd(const float *features, const float *out_features,
 
 extern "C" int ssc_avgpool_bwd(const float *out_grad, int c, const int32_t *nbr_in, int K, int n_in,
                                const int32_t *summaryrf, float *d_in, void *stream) {
-  return launch_pool_bwd<1>(nullptr, nullptr, out_grad, c, nbr_in, K, n_in, summaryrf, d_in, stream, "avgpool_bwd");
+  auto launch = summaryrf ? launch_pool_bwd<2> : launch_pool_bwd<1>;
+  return launch(nullptr, nullptr, out_grad, c, nbr_in, K, n_in, summaryrf, d_in, stream, "avgpool_bwd");
 }
 
 extern "C" int ssc_global_avgpool_bwd(const float *d_out, const int32_t *offsets, int n_samples, int c, int n_rows,

@@ -108,6 +108,35 @@ pool_fwd_few_kernel(const void *__restrict__ features, int c, const int32_t *__r
   store_rows<PIECE>(out + (size_t)o * c + c0, valid, acc);
 }
 
+// The rows of an average pool whose counts the kernels above do not take (whole_count), once more by plain division: a warp
+// looks at the counts of 32 rows, nearly all of which have nothing to do.  Looked for in the kernels themselves, even
+// once per row, they cost 3 to 10 % of every average pool (83 k rows of 8 offsets and 76 channels 43.9 -> 45.6 us, with a
+// row's test in front of its loop 47.5; 134 k rows of 27 92.2 -> 95.1 and 101.3); this runs only where a caller
+// brings counts.
+template <int IN>
+__global__ void __launch_bounds__(256)
+pool_divided_rows_kernel(const void *__restrict__ features, int c, const int32_t *__restrict__ nbr, int K, int n_out,
+                         const int32_t *__restrict__ summaryrf, float *__restrict__ out, const int32_t *__restrict__ n_out_dev) {
+  const int lane = threadIdx.x & 31, row0 = (int)(blockIdx.x * 256 + (threadIdx.x & ~31u)), n_rows = live_rows(n_out, n_out_dev);
+  const int count = lane < n_rows - row0 ? __ldg(summaryrf + row0 + lane) : 1;
+  for (unsigned left = __ballot_sync(0xffffffffu, !whole_count(count)); left != 0u; left &= left - 1u) {
+    const int r = __ffs((int)left) - 1, o = row0 + r;
+    const float div = (float)__shfl_sync(0xffffffffu, count, r);
+    for (int ch = lane; ch < c; ch += 32) {
+      float acc = 0.f;
+      for (int k = 0; k < K; ++k) {
+        const int src = __ldg(nbr + (size_t)k * n_out + o);
+        if (src < 0) continue;
+        Channels x;
+        load_channels<IN, 1>(features, (size_t)src * c + ch, 1, x);
+        acc += x.v[0] / div;
+      }
+      out[(size_t)o * c + ch] = acc;
+    }
+    __syncwarp();
+  }
+}
+
 __global__ void summary_rf_kernel(const int32_t *__restrict__ nbr, int K, int n_out, int32_t *__restrict__ rf) {
   int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= n_out) return;
@@ -239,6 +268,10 @@ static int launch_pool_as(const void *features, int c, const int32_t *nbr, int K
     pool_fwd_kernel<MODE, IN, PIECE><<<p.grid, 256, p.smem, st>>>(features, c, nbr, K, n_out, rf, out, n_out_dev, p.rows);
   }
   note_launches(1);
+  if (MODE == 1 && rf != nullptr) {
+    pool_divided_rows_kernel<IN><<<ceil_div(n_out, 256), 256, 0, st>>>(features, c, nbr, K, n_out, rf, out, n_out_dev);
+    note_launches(1);
+  }
   SSC_CHECK_LAUNCH(name);
   return SSC_OK;
 }

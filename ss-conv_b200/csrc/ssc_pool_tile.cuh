@@ -117,14 +117,13 @@ static __device__ __forceinline__ void store_rows(float *__restrict__ p, int val
   }
 }
 
-// acc += x / d for a count d, with r = 1 / d rounded to nearest: correctly rounded, as x / d is.  Two corrections by the
-// exact remainder (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990: a quotient
-// within an ulp, corrected by r times its remainder, is the correctly rounded one) for whole d of 1 .. 2^20; sizes
-// whose remainder might not be representable, infinities and NaNs are divided, and so is everything by any other
-// d (counts are the caller's: 0 gives an infinity).  Half of the values behind a ReLU are zeros, on which a
-// division costs more: three average pools took 182 us with it, 105 us without.
+// acc += x / d for a count d (whole_count) with r = 1 / d rounded to nearest: correctly rounded, as x / d is.  Two
+// corrections by the exact remainder (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000", 1990: a quotient within an ulp, corrected by r times its remainder, is the correctly rounded
+// one); sizes whose remainder might not be representable, infinities and NaNs are divided.  Half of the values
+// behind a ReLU are zeros, on which a division costs more: three average pools took 182 us with it, 105 us without.
 static __device__ __forceinline__ void add_quotients(Channels &acc, const Channels &x, float d, float r) {
-  bool fast = d >= 1.f && d <= 1048576.f;
+  bool fast = true;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const float a = fabsf(x.v[q]);
@@ -142,5 +141,8 @@ static __device__ __forceinline__ void add_quotients(Channels &acc, const Channe
     for (int q = 0; q < 4; ++q) acc.v[q] += x.v[q] / d;
   }
 }
+
+// What add_quotients takes.  Counts are the caller's: all others are divided by (0 gives an infinity).
+static __device__ __forceinline__ bool whole_count(int32_t d) { return (uint32_t)(d - 1) < (1u << 20); }
 
 }  // namespace ssc
