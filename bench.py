@@ -47,9 +47,9 @@ CFG2 = dict(name="cfg2: SS-Conv (4,4,4,4)->(4,4,4,4)+12 gates, k3 s2 p1, batch 3
             batch=32, V=64, n_pts=16384, irreps=(4, 4, 4, 4), k=3, stride=2, pad=1, pool_k=2, pool_s=2)
 # DRAM bytes per launch of the two kernels of the cfg2 convolution call (dram__bytes_read.sum +
 # dram__bytes_write.sum), from:  ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum
-#   --clock-control none -k regex:"stage_features|conv_fwd_tf32" -c 8 python bench.py --only conv --steps 1
+#   --clock-control none -k regex:"stage_features|conv_fwd_rows" -c 8 python bench.py --only conv --steps 1
 # (staging: 61.4 MB read + 10.9 MB written back, most of the staged image stays in L2;
-#  convolution: 76.0 MB read + 1.0 MB written)
+#  convolution: 76.0 MB read + 1.0 to 1.4 MB written)
 NCU_DRAM_BYTES = {"stage_features_kernel": 72.3e6, "conv_fwd_rows_kernel": 77.0e6}
 ROTATE = 4    # distinct input batches cycled through so the working set exceeds the 126 MB L2
 REGIONS = 25  # repetitions of the --steps-long timed region; the median region is reported

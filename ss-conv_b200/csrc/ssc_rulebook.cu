@@ -24,7 +24,8 @@ constexpr int kChunk = 1024;  // outputs per block in lookup / fill
 constexpr long long kDenseMaxCells = 1ll << 26;     // 256 MiB of row map at most
 // A lookup in the map is one load, in the hash table a probe chain: what the map costs more is its clearing, 0.3 ns
 // per 1000 bytes.  Measured over one 5^3 and several 3^3 layers, lookups and clearing together, the map wins at 64,
-// 150 and 400 cells per row (610 + 64 -> 129 us, 119 + 42 -> 63 us); it loses its lead near 1000.
+// 150 and 400 cells per row (610 + 64 -> 129 us, 119 + 42 -> 63 us); it loses its lead near 1000.  In memory it costs up
+// to 2 KB of scratch per input row, 256 MB at most, where the table takes 16 to 32 bytes per row.
 constexpr long long kDenseCellsPerRow = 512;
 
 struct RulebookScratch {

@@ -1,6 +1,7 @@
 """Native-op module of the B200 build: the names the reference exports from its pybind11
 extension `ss_conv._ext` (SS_Conv_lib/src/ss_conv_ops_api.cpp:15-55), implemented as thin
-ctypes calls into the C-ABI CUDA library libssconv_b200.so (include/ssconv_b200.h).
+calls into the C-ABI CUDA library libssconv_b200.so (include/ssconv_b200.h): through the bindings
+module `_host` (csrc/ssc_host.cpp), or through ctypes where SSCONV_B200_LIB names another build.
 
 PyTorch is used only to allocate device memory and to supply the current CUDA stream.  There
 is no CPU path: every function raises if the library is missing or a tensor is not on a CUDA
@@ -522,7 +523,8 @@ def get_indice_pairs_ahead(indices, batch_size, out_shape, spatial_shape, ksize,
     # the per-offset pair counts (indice_num) are not needed by the kernels that consume the table:
     # they are computed only if somebody turns the handle into reference-format pair lists
     if torch.cuda.is_current_stream_capturing():
-        # a recorded graph keeps the phases' own kernels: its nodes follow one another without a launch to save
+        # a recorded graph keeps the phases' own kernels: without launches to save and a count to post, the one-launch
+        # form is worth nothing there (the replay of four strided stages at batch 256: 414 us, with it 411)
         _check(L.ssc_rulebook_conv_count(_p(indices), n_in, int(batch_size), *geo, _p(n_out_dev), _p(st), _p(scratch), sbytes,
                                          _p(n_in_dev), _stream()))
         _check(L.ssc_rulebook_conv_fill(_p(indices), n_in, int(batch_size), *geo, cap, _p(outids), _p(nbr), None, None,
@@ -1170,9 +1172,11 @@ def nbr_row_order_planes(nbr, ksize, n_rows_dev=None, with_table=False):
     (for conv_forward(row_order=...)); None for kernels it does not cover.  n_rows_dev: device word
     with the live row count when n is a capacity.  with_table: also return the table with its
     columns moved into that order (for conv_forward(..., table_in_order=True)).
-    Opt-in: on a 64 -> 76 channel layer of 129 k surface rows the call drops from 0.154 to 0.129 ms
-    (45 % fewer steps, the long tiles first) and the ordering takes 0.044 ms, so it pays from the
-    third layer that shares a table on; the layers do not ask for it themselves."""
+    Opt-in, and rarely worth it: the ordering takes 48 to 60 us.  Strided layers of 134 k surface rows that share a table
+    gain it back after 21 calls at 64 -> 76 channels (82.8 -> 79.9 us) and after four at 128 -> 152 bf16 (118.8 ->
+    100.5); submanifold layers of 15 k to 245 k rows and 2 to 10 neighbours a row are slower in this order
+    (41.0 -> 43.0, 155.7 -> 175.1 us; neighbouring rows no longer share cache lines) but for the narrowest
+    (32 -> 38: 41.0 -> 36.9).  The layers do not ask for it themselves."""
     K, n = nbr.shape
     ks = [int(v) for v in ksize]
     if len(ks) != 3 or ks[0] * ks[1] * ks[2] != K or n == 0:
