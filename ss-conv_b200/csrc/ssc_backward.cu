@@ -325,7 +325,7 @@ static int launch_pool_bwd(const float *features, const float *out_features, con
   const int piece = pool_piece(c, (uintptr_t)features | (uintptr_t)out_features | (uintptr_t)out_grad | (uintptr_t)d_in);
   auto kernel = piece == 4 ? pool_bwd_kernel<MODE, 4> : piece == 2 ? pool_bwd_kernel<MODE, 2> : pool_bwd_kernel<MODE, 1>;
   if (p.smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    cudaError_t e = allow_smem((const void *)kernel, p.smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "%s: smem attribute: %s", name, cudaGetErrorString(e));
   }
   kernel<<<p.grid, 256, p.smem, as_stream(stream)>>>(features, out_features, out_grad, c, nbr_in, K, n_in, rf, d_in, p.rows);

@@ -822,7 +822,7 @@ static int bwd_tile_rows(int c, int c_out, int n_gates, int most, size_t *smem) 
 template <int PASS, int VEC>
 static int launch_bwd_vec(const BnGateBwd &p, size_t smem, const float *ks, const float *ka, const float *kg, float *gx, float *part_a, float *part_g, cudaStream_t st) {
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(bn_gate_bwd_kernel<PASS, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void *)bn_gate_bwd_kernel<PASS, VEC>, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "bn_gate_bwd: smem attribute: %s", cudaGetErrorString(e));
   }
   int blocks = PASS == 0 ? p.chains : ceil_div(p.n, p.rows);

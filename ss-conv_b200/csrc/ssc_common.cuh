@@ -16,6 +16,9 @@ int fail(int code, const char *fmt, ...);
 // Kernel-launch bookkeeping behind ssc_kernel_launches().
 void note_launches(int n);
 
+// Lets a kernel have `bytes` of dynamic shared memory on the current device, for this launch and all others.
+cudaError_t allow_smem(const void *kernel, size_t bytes);
+
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
 #define SSC_CHECK_LAUNCH(name)                                                     \

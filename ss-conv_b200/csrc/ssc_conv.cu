@@ -265,7 +265,7 @@ static int launch_fp32_small(const float *features, int c_in, const float *filte
   const dim3 grid(blocks < most ? blocks : most, ceil_div(c_out, NJ * 32));
   auto kernel = staged ? conv_fwd_fp32_small_kernel<NJ, true> : conv_fwd_fp32_small_kernel<NJ, false>;
   if (staged && smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void *)kernel, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(fp32): smem attribute: %s", cudaGetErrorString(e));
   }
   { kernel<<<grid, SM_WARPS * 32, staged ? smem : 0, st>>>(features, c_in, filters, K, c_out, nbr, n_out, rev, out, n_out_dev); note_launches(1); }
@@ -299,7 +299,7 @@ extern "C" int ssc_materialize_bwd(const float *d_filters, const float *basis, c
   const size_t need = (size_t)K * max_pair * sizeof(float);
   const int staged = need <= 200 * 1024 ? 1 : 0;
   if (staged && need > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(materialize_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+    cudaError_t e = allow_smem((const void *)materialize_bwd_kernel, need);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "materialize_bwd: smem attribute: %s", cudaGetErrorString(e));
   }
   { materialize_bwd_kernel<<<dim3(n_in, n_out), kMatBwdThreads, staged ? need : 0, as_stream(stream)>>>(

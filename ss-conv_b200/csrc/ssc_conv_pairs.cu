@@ -557,7 +557,7 @@ int conv_fwd_pairs(const void *staged, int c_in, const void *packed, int K, int 
   SSC_CHECK_LAUNCH("pl_strips");
   const size_t smem = pl_smem_bytes(p);
   auto kernel = p.f16 ? conv_fwd_pairs_kernel<true> : conv_fwd_pairs_kernel<false>;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = allow_smem((const void *)kernel, smem);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd_pairs: smem attribute: %s", cudaGetErrorString(e));
   { kernel<<<n_ctas, p.threads, smem, st>>>((const float *)staged, (const uint4 *)packed, c_out, pl.pair_out, pl.pair_in, pl.starts,
                                           strips, owner, hdr, out, status, p); note_launches(1); }

@@ -1071,7 +1071,7 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
   const bool gated = gate.gate_of_channel != nullptr;
   if (gated && !gate_fits(p, c_out, gate.c_keep)) return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): the gated epilogue does not cover %d -> %d channels", c_out, gate.c_keep);
   const RowsKernel kernel = rows_kernel<true>(p, gated);
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem((const void *)kernel, smem);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(16-bit): smem attribute: %s", cudaGetErrorString(e));
   const dim3 grid2(grid, p.n_tiles / p.nt_cta);
   { kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate); note_launches(1); }
@@ -1113,12 +1113,12 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
     return fail(SSC_ERR_INVALID, "conv_fwd(tf32): the gated epilogue does not cover %d -> %d channels without a staging buffer", c_out, gate.c_keep);
   if (rows) {
     const RowsKernel kernel = rows_kernel<false>(p, gated);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void *)kernel, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
     kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, c_pad, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
   } else {
     auto kernel = opk > 1 ? conv_fwd_tf32_kernel<true> : conv_fwd_tf32_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void *)kernel, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
     kernel<<<grid2, p.threads, smem, st>>>(staged ? (const float *)scratch : features, staged ? c_pad : c_in, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order);
   }

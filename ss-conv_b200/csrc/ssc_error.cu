@@ -1,7 +1,9 @@
 // Error reporting, identification and the read-back of device words.
 #include <stdarg.h>
 #include <deque>
+#include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
 #if defined(__x86_64__)
 #include <immintrin.h>
@@ -25,6 +27,23 @@ int fail(int code, const char *fmt, ...) {
 static unsigned long long g_launches = 0;
 void note_launches(int n) { __atomic_fetch_add(&g_launches, (unsigned long long)n, __ATOMIC_RELAXED); }
 unsigned long long launches() { return __atomic_load_n(&g_launches, __ATOMIC_RELAXED); }
+
+// The limit is the kernel's, not the launch's, and calls of other sizes set it too: set by every call to what that call
+// needs, one thread could take it away from another between its setting and its launch ("invalid argument", or "too many
+// resources requested": four threads on one network, once in some thousand passes).  So it only ever grows.
+cudaError_t allow_smem(const void *kernel, size_t bytes) {
+  static std::mutex lock;
+  static std::map<std::pair<int, const void *>, size_t> allowed;
+  int dev = 0;
+  if (cudaError_t e = cudaGetDevice(&dev)) return e;
+  std::lock_guard<std::mutex> hold(lock);
+  size_t &have = allowed[{dev, kernel}];
+  if (bytes <= have) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) have = bytes;
+  else (void)cudaGetLastError();
+  return e;
+}
 
 // Kernels that give up set this word too, besides their status word: row counts are posted to the host before the
 // convolution behind them has run, so nothing that is read back tells of it in time.  Mapped host memory, kept

@@ -262,7 +262,7 @@ static int launch_pool_as(const void *features, int c, const int32_t *nbr, int K
     const PoolShape p = pool_shape(n_out, K);
     SSC_REQUIRE(p.rows > 0, "%s: kernel of %d offsets is too large", name, K);
     if (p.smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(pool_fwd_kernel<MODE, IN, PIECE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+      cudaError_t e = allow_smem((const void *)pool_fwd_kernel<MODE, IN, PIECE>, p.smem);
       if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "%s: smem attribute: %s", name, cudaGetErrorString(e));
     }
     pool_fwd_kernel<MODE, IN, PIECE><<<p.grid, 256, p.smem, st>>>(features, c, nbr, K, n_out, rf, out, n_out_dev, p.rows);

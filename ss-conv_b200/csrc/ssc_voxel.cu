@@ -673,7 +673,7 @@ static int steer_matrices(const T *rot, int batch, int orders, const double *dir
   }
   const size_t smem = (size_t)harmonics * sizeof(double);       // 5 KB for orders 0..3, below 48 KB up to order 8
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(steer_matrices_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void *)steer_matrices_kernel<T>, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "steer_matrices: smem attribute: %s", cudaGetErrorString(e));
   }
   { steer_matrices_kernel<T><<<batch, 128, smem, as_stream(stream)>>>(rot, orders, dirs, pinv, axes, stride, dmats); note_launches(1); }

@@ -551,7 +551,7 @@ int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int
                      bool tf32, int staged, float *partial, float *d_filters, int32_t *status, cudaStream_t st) {
   const WgradPlan p = wgrad_plan(K, c_in, c_out, n_out, tf32);
   if (p.tc) {
-    cudaError_t e = cudaFuncSetAttribute(conv_wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    cudaError_t e = allow_smem((const void *)conv_wgrad_tc_kernel, p.smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_wgrad(tf32): smem attribute: %s", cudaGetErrorString(e));
     const WtParams w = {features, out_grad, c_in, c_out, (staged & 1) ? (c_in + 3) & ~3 : c_in, (staged & 2) ? (c_out + 3) & ~3 : c_out,
                         (staged & 1) ? 0 : 1, (staged & 2) ? 0 : 1, p.n_pad, p.a_bytes, p.stage_bytes, p.stages, p.n_buf, p.buf_cols, alarm_word()};

@@ -298,3 +298,49 @@ def test_a_kernel_that_gives_up_behind_a_posted_count_is_reported(cuda):
         with pytest.raises(RuntimeError, match="0x10"):
             _ext.check_status(cuda)
         assert y.features.shape[0] == n
+
+
+def test_threads_run_layers_of_several_sizes_at_a_time(cuda):
+    """Threads with streams of their own queue layers whose kernels are the same and whose shared memory is not (widths,
+    row counts, a shared network on batches of several sizes): every result is that of the single thread."""
+    import threading
+    import torch.nn as nn
+    from ss_conv import _ext
+    from ss_conv.pool import AvgPool
+    from ss_conv.sp_ops.tensor import SparseTensor
+    from ss_conv_modules import SS_Conv
+    torch.manual_seed(0)
+    act = dict(padding=1, activation=(torch.relu, torch.sigmoid))
+    net = nn.Sequential(SS_Conv((4, 4), (4, 4), 3, stride=2, **act), AvgPool(3, stride=2, padding=1),
+                        SS_Conv((4, 4), (8, 8), 3, stride=2, indice_key="k", **act),
+                        SS_Conv((8, 8), (16, 16), 3, inverse=True, activation=(torch.relu, torch.sigmoid), indice_key="k")).to(cuda).eval()
+    batches = []
+    for s in range(12):
+        inds = dev(random_voxels(np.random.RandomState(s), 3, 20 + 4 * (s % 2), (100, 1300, 20, 9000)[s % 4]), cuda)
+        batches.append((inds, torch.randn(inds.shape[0], 16, device=cuda), [20 + 4 * (s % 2)] * 3))
+
+    def run(k):
+        inds, feats, grid = batches[k]
+        with torch.no_grad():
+            return net(SparseTensor(feats, inds, grid, 3)).features
+
+    want, wrong = [run(k) for k in range(12)], []
+    torch.cuda.synchronize()
+
+    def work(seed):
+        rng = np.random.RandomState(seed)
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for k in rng.randint(0, 12, 150):
+                    if not torch.equal(run(k), want[k]):
+                        wrong.append(k)
+        except Exception as e:
+            wrong.append(e)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    _ext.check_status(cuda)
