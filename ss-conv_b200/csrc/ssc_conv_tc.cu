@@ -19,9 +19,7 @@
 // Every wait on an mbarrier is bounded: on expiry the thread records an error in `status`
 // through a shared flag, every other wait then gives up too, and the kernel frees its tensor
 // memory and returns.
-#include "ssc_act.cuh"
-#include "ssc_conv_internal.cuh"
-#include "ssc_tc_ptx.cuh"
+#include "ssc_conv_epilogue.cuh"
 
 namespace ssc {
 
@@ -784,15 +782,10 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
     const int group = warp >> 2;
     __syncwarp();
     float4 consts[2];                             // (GATED) scale, shift, gate of the channels this thread hands round
-    auto channel = [&](int ch) {
-      const bool bn = gate.scale != nullptr;
-      return make_float4(bn ? __ldg(gate.scale + ch) : 0.f, bn ? __ldg(gate.shift + ch) : 0.f,
-                         __int_as_float(ch < gate.c_keep ? __ldg(gate.gate_of_channel + ch) : -2), 0.f);
-    };
     if (GATED) {
 #pragma unroll
       for (int i = 0; i < 2; ++i)
-        if (tid + 128 * i < c_out) consts[i] = channel(tid + 128 * i);
+        if (tid + 128 * i < c_out) consts[i] = gate_channel(gate, tid + 128 * i);
     }
     bool ok = __all_sync(0xffffffffu, !*abort_flag);
     if (ok && n_iter > 0) ok = mbar_wait_warp(smem_u32(&done_bar), 0u, abort_flag);
@@ -817,146 +810,20 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
       float4 *chan = (float4 *)(smem + (size_t)groups * 4u * 4096u);   // [c_out]
       // act(gate g) of row r of the quarter at g * 33 + r, and a last line of ones
       const int n_gates = c_out - c_row;
-      const bool affine = gate.scale != nullptr, whole = vec && order == nullptr && m0 + TC_M <= n_rows;
+      const bool whole = vec && order == nullptr && m0 + TC_M <= n_rows;
       float *gates = (float *)(chan + c_out) + quarter * 33 * (n_gates + 1);
 #pragma unroll
       for (int i = 0; i < 2; ++i)
         if (tid + 128 * i < c_out && group == 0) chan[tid + 128 * i] = consts[i];
-      for (int ch = tid + 256; ch < c_out && group == 0; ch += 128) chan[ch] = channel(ch);
+      for (int ch = tid + 256; ch < c_out && group == 0; ch += 128) chan[ch] = gate_channel(gate, ch);
       asm volatile("bar.sync 1, %0;" ::"r"(groups * 128) : "memory");
       if (group == 0) gates[n_gates * 33 + lane] = 1.f;
-      for (int c0 = (c_row & ~15) + 16 * group; c0 < c_out; c0 += 16 * groups) {
-        uint32_t q[16];
-        load16(q, c0);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        float v[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float4 k = chan[c0 + i < c_out ? c0 + i : 0];
-          v[i] = __uint_as_float(q[i]);
-          if (gate.scale) v[i] = fmaf(v[i], k.x, k.y);
-        }
-        if (gate.gate_act == 2) {                 // (all sixteen side by side: one after the other they are all latency)
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = apply_act(v[i], 2);
-        } else if (gate.gate_act == 1) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = apply_act(v[i], 1);
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (c0 + i >= c_row && c0 + i < c_out) gates[(c0 + i - c_row) * 33 + lane] = v[i];
-      }
+      gate_scalars(load16, gate, chan, gates, c_out, lane, (c_row & ~15) + 16 * group, 16 * groups);
       asm volatile("bar.sync 1, %0;" ::"r"(groups * 128) : "memory");
-      for (int c0 = 32 * group; c0 < c_row; c0 += 32 * groups) {
-        uint32_t r[32];
-        load16(r, c0);
-        load16(r + 16, c0 + 16);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        __syncwarp();
-        // piece q of row `lane` at place q ^ (lane & 7): both directions touch every bank once per phase
-#pragma unroll
-        for (int q = 0; q < 8; ++q) *(uint4 *)(blk + lane * 32 + ((q ^ (lane & 7)) << 2)) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-        __syncwarp();
-        const int q = lane & 7, row4 = lane >> 3, col = c0 + 4 * q;
-        float sc[4], sh[4];
-        const float *gp[4];
-        bool scalar[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 k = chan[col + j < c_out ? col + j : 0];
-          const int g = __float_as_int(k.z);
-          sc[j] = k.x;
-          sh[j] = k.y;
-          scalar[j] = g == -1;
-          gp[j] = gates + (g >= 0 ? g : n_gates) * 33 + row4;
-        }
-        const bool scalars = __any_sync(0xffffffffu, scalar[0] || scalar[1] || scalar[2] || scalar[3]) && gate.scalar_act != 0;
-        if (col >= c_row) continue;
-        // rows 4 i + row4 of the warp's 32: the swizzle of even and odd i, the rest are constants
-        const float *even = blk + row4 * 32 + ((q ^ row4) << 2), *odd = blk + row4 * 32 + ((q ^ row4 ^ 4) << 2);
-        const int row0 = m0 + quarter * 32 + row4;
-        auto finished = [&](int i, bool act) {
-          const float4 x = *(const float4 *)((i & 1 ? odd : even) + i * 128);
-          float v[4] = {x.x, x.y, x.z, x.w};
-          if (affine) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = fmaf(v[j], sc[j], sh[j]);
-          }
-          if (act) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (scalar[j]) v[j] = apply_act(v[j], gate.scalar_act);
-          }
-          return make_float4(v[0] * gp[0][4 * i], v[1] * gp[1][4 * i], v[2] * gp[2][4 * i], v[3] * gp[3][4 * i]);
-        };
-        if (!scalars && whole && gate.out16 == 0) {          // most columns of most tiles
-          float *to = out + (size_t)row0 * c_row + col;
-#pragma unroll
-          for (int i = 0; i < 8; ++i, to += 4 * c_row) *(float4 *)to = finished(i, false);
-        } else if (!scalars && whole) {
-          uint16_t *to = (uint16_t *)out + (size_t)row0 * c_row + col;
-          if (gate.out16 == 2) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i, to += 4 * c_row) {
-              const float4 v = finished(i, false);
-              *(uint2 *)to = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i, to += 4 * c_row) {
-              const float4 v = finished(i, false);
-              *(uint2 *)to = make_uint2(pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w));
-            }
-          }
-        } else {
-#pragma unroll 2
-          for (int i = 0; i < 8; ++i) {
-            const int at_row = row0 + 4 * i;
-            const float4 v = finished(i, scalars);
-            if (at_row >= n_rows) continue;
-            const size_t at = (size_t)(order ? __ldg(order + at_row) : at_row) * c_row + col;
-            if (gate.out16 != 0) {                // c_row is a multiple of eight
-              *(uint2 *)((uint16_t *)out + at) = gate.out16 == 2 ? make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w))
-                                                                : make_uint2(pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w));
-            } else if (vec) {
-              *(float4 *)(out + at) = v;
-            } else {
-              const float e[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (col + j < c_row) out[at + j] = e[j];
-            }
-          }
-        }
-      }
+      store_gated(load16, gate, chan, gates, blk, out, c_out, m0 + quarter * 32, n_rows, order, whole, vec, lane, 32 * group, 32 * groups);
     } else {
       const int m = m_tile < n_rows ? (order ? __ldg(order + m_tile) : m_tile) : -1;
-      for (int c0 = 32 * group; c0 < p.n_cta && col0 + c0 < c_row; c0 += 32 * groups) {
-        uint32_t r[32];
-        load16(r, c0);
-        load16(r + 16, c0 + 16);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (vec) {
-          __syncwarp();
-#pragma unroll
-          for (int q = 0; q < 8; ++q) *(uint4 *)(blk + lane * 32 + ((q ^ (lane & 7)) << 2)) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-          __syncwarp();
-          const int q = lane & 7, col = col0 + c0 + 4 * q;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int row = 4 * i + (lane >> 3);
-            const int to = __shfl_sync(0xffffffffu, m, row);
-            if (to >= 0 && col < c_row && c0 + 4 * q < p.n_cta)
-              *(uint4 *)(out + (size_t)to * c_row + col) = *(const uint4 *)(blk + row * 32 + ((q ^ (row & 7)) << 2));
-          }
-        } else if (m >= 0) {
-          float *op = out + (size_t)m * c_row + col0 + c0;
-#pragma unroll
-          for (int q = 0; q < 32; ++q)
-            if (col0 + c0 + q < c_row && c0 + q < p.n_cta) op[q] = __uint_as_float(r[q]);
-        }
-      }
+      store_plain(load16, blk, out, m, col0, p.n_cta, c_row, vec, lane, 32 * group, 32 * groups);
     }
   }
   // a wait gave up: what was issued still arrives on done_bar (committed on every path) and filter copies land
