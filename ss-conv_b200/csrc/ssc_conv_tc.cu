@@ -748,30 +748,37 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
     const uint32_t full0 = smem_u32(full_bars), empty0 = smem_u32(empty_bars);
     uint32_t s = 0, par = 0, a_lo = a_lo0;
     int slab = 0;
+    bool ready = false;
     for (int it = 0; it < n_iter; ++it) {
-      if (!mbar_wait_uniform(full0 + s * 8u, par, abort_flag)) break;
+      if (!ready && !mbar_wait_uniform(full0 + s * 8u, par, abort_flag)) break;
       fence_async_smem();                         // the rows other threads' copies left, for the tensor core
       tc_fence_after();
       const uint4 off = *(const uint4 *)(slot_masks + s * 4u);
       // k-steps that hold real channels (the rest of the last slab is zero on both sides)
       const int n_kk = slab == p.k_slabs - 1 ? p.last_kk : 4;
       const bool any = __any_sync(0xffffffffu, (off.x & off.y & off.z & off.w) != 0xffffffffu);
+      const uint32_t an = a_lo, done = empty0 + s * 8u;
+      a_lo += slot_step;
+      if (++s == (uint32_t)S) { s = 0; par ^= 1u; a_lo = a_lo0; }
+      // A CTA alone on its SM has a deep ring, and this warp's chain of instructions is what bounds a step (440 cycles undisturbed,
+      // whatever the products): the next step's barrier is looked at before this one's products are issued.  (16 k rows
+      // 32 -> 38: 15.0 -> 14.1 us; 15 k rows 256 -> 304 bf16: 61.2 -> 60.2.  With two or four CTAs the look comes too early: +1 to 2 %.)
+      const bool passed = GROUPS == 2 && p.ctas == 1 && mbar_test_wait(full0 + s * 8u, par);
       for (int nt = 0; nt < (any ? p.nt_cta : 0); ++nt) {
         const uint32_t dn = tmem_base + (uint32_t)(nt * p.tile_n);
-        const uint32_t bn = a_lo + (uint32_t)(TC_A_BYTES >> 4) + (uint32_t)nt * n_step;
+        const uint32_t bn = an + (uint32_t)(TC_A_BYTES >> 4) + (uint32_t)nt * n_step;
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
             if (kk >= n_kk) break;
-            if (F16) mma_f16_ss_masked(dn, a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
-            else mma_tf32_ss_masked(dn, a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
+            if (F16) mma_f16_ss_masked(dn, an + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
+            else mma_tf32_ss_masked(dn, an + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
           }
         }
       }
       if (++slab == p.k_slabs) slab = 0;
-      if (elect_one()) mma_commit(empty0 + s * 8u);
-      a_lo += slot_step;
-      if (++s == (uint32_t)S) { s = 0; par ^= 1u; a_lo = a_lo0; }
+      if (elect_one()) mma_commit(done);
+      ready = GROUPS == 2 && __all_sync(0xffffffffu, passed);
     }
     if (elect_one()) mma_commit(smem_u32(&done_bar));   // arrives once everything issued above has retired
   }
