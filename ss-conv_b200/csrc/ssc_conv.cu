@@ -163,107 +163,125 @@ conv_fwd_fp32_kernel(const float *__restrict__ features, int c_in, const float *
   }
 }
 
+// Two floats in a register pair, and a * b + c of both halves, each correctly rounded (fmaf of each).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 halves(f32x2 v) {
+  float2 h;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(h.x), "=f"(h.y) : "l"(v));
+  return h;
+}
+__device__ __forceinline__ f32x2 fma_pair(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
 // The same sums for up to four input channels (a first layer on point features), in the same order: per output
 // element fused multiply-adds over ascending offsets and channels, present neighbours only.
-// A warp takes eight output rows at a time; lanes hold NJ output channels each (lane, lane + 32, ...), the
-// filters stand in shared memory.  All 28 x 8 table entries of a pass, then all present input rows, are
-// loaded at once, a lane per (offset, row); they reach the other lanes by shuffles.  Bound by instruction
-// issue (about 200 per row of 6 neighbours and 64 channels).  The tiled kernel above pads the
-// channels to 16 and multiplies absent rows: 399 us for 215 k rows of 3 -> 48 channels.
-constexpr int SM_WARPS = 8, SM_ROWS = 8;
-template <int NJ, bool STAGED>
+// A lane has an output row and CB of its channels, two to a register pair; the filters stand in shared memory, where all
+// lanes read the same word at a time.  Table entries and input rows of nine offsets are in flight together.  Bound by
+// issue: a warp runs through every offset that one of its 32 rows has.  215 k rows of 3 -> 36 channels, 6 neighbours
+// a row: 64 us; 83 with a warp per eight rows and a lane per channel, where a row took 200 instructions, as many
+// shuffles as multiply-adds.  (Two rows to a lane and zeros for absent neighbours: 92; three offsets in flight: 76;
+// blocks of four warps, each with its copy of the filters: 71.)
+constexpr int SM_WARPS = 8, SM_AHEAD = 9;
+template <int CB, bool STAGED>
 __global__ void __launch_bounds__(SM_WARPS * 32)
 conv_fwd_fp32_small_kernel(const float *__restrict__ features, int c_in, const float *__restrict__ filters, int K,
                            int c_out, const int32_t *__restrict__ nbr, int n_out, int rev, float *__restrict__ out,
                            const int32_t *__restrict__ n_out_dev) {
-  extern __shared__ float ws[];               // [K][c_in][NJ * 32]
+  extern __shared__ __align__(16) float ws[];   // [K][c_in][CB]
   const int n_rows = live_rows(n_out, n_out_dev);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.y * NJ * 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.y * CB;
+  if ((int)blockIdx.x * SM_WARPS * 32 >= n_rows) return;
   if (STAGED) {
-    for (int i = threadIdx.x; i < K * c_in * NJ * 32; i += SM_WARPS * 32) {
-      const int ch = i % (NJ * 32), kc = i / (NJ * 32);
+    for (int i = threadIdx.x; i < K * c_in * CB; i += SM_WARPS * 32) {
+      const int ch = i % CB, kc = i / CB;
       ws[i] = n0 + ch < c_out ? __ldg(filters + (size_t)kc * c_out + n0 + ch) : 0.f;
     }
     __syncthreads();
   }
-  for (int m0 = ((int)blockIdx.x * SM_WARPS + warp) * SM_ROWS; m0 < n_rows; m0 += (int)gridDim.x * SM_WARPS * SM_ROWS) {
-    float acc[SM_ROWS][NJ];
+  const bool vec = (c_out & 3) == 0 && ((uintptr_t)out & 15u) == 0;
+  for (int m0 = ((int)blockIdx.x * SM_WARPS + warp) * 32; m0 < n_rows; m0 += (int)gridDim.x * SM_WARPS * 32) {
+    const int row = m0 + lane;
+    f32x2 acc[CB / 2];
 #pragma unroll
-    for (int r = 0; r < SM_ROWS; ++r)
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) acc[r][j] = 0.f;
-    const int my_row = m0 + (lane & 7);
+    for (int j = 0; j < CB / 2; ++j) acc[j] = 0ull;
 #pragma unroll 1
-    for (int k0 = 0; k0 < K; k0 += 28) {
-      int idx[7];
-      float x[7][4];
+    for (int k0 = 0; k0 < K; k0 += SM_AHEAD) {
+      int idx[SM_AHEAD];
+      float x[SM_AHEAD][4];
 #pragma unroll
-      for (int t = 0; t < 7; ++t) {            // entry (offset k0 + 4 t + lane / 8, row lane % 8)
-        const int k = k0 + 4 * t + (lane >> 3);
-        idx[t] = (k < K && my_row < n_rows) ? __ldg(nbr + (size_t)(rev ? K - 1 - k : k) * n_out + my_row) : -1;
+      for (int i = 0; i < SM_AHEAD; ++i) {
+        const int k = k0 + i;
+        idx[i] = (k < K && row < n_rows) ? __ldg(nbr + (size_t)(rev ? K - 1 - k : k) * n_out + row) : -1;
       }
 #pragma unroll
-      for (int t = 0; t < 7; ++t) {
-        const float *fp = features + (size_t)(idx[t] >= 0 ? idx[t] : 0) * c_in;
+      for (int i = 0; i < SM_AHEAD; ++i) {
+        const float *fp = features + (size_t)(idx[i] >= 0 ? idx[i] : 0) * c_in;
         if (c_in == 4) {
-          const float4 f = idx[t] >= 0 ? __ldg((const float4 *)fp) : make_float4(0.f, 0.f, 0.f, 0.f);
-          x[t][0] = f.x; x[t][1] = f.y; x[t][2] = f.z; x[t][3] = f.w;
+          const float4 f = idx[i] >= 0 ? __ldg((const float4 *)fp) : make_float4(0.f, 0.f, 0.f, 0.f);
+          x[i][0] = f.x; x[i][1] = f.y; x[i][2] = f.z; x[i][3] = f.w;
         } else {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) x[t][c] = (c < c_in && idx[t] >= 0) ? __ldg(fp + c) : 0.f;
+          for (int c = 0; c < 4; ++c) x[i][c] = (c < c_in && idx[i] >= 0) ? __ldg(fp + c) : 0.f;
         }
       }
 #pragma unroll
-      for (int t = 0; t < 7; ++t) {
-        const unsigned have = __ballot_sync(0xffffffffu, idx[t] >= 0);
-#pragma unroll 1
-        for (int q = 0; q < 4; ++q) {
-          const unsigned m = (have >> (8 * q)) & 255u;
-          if (m == 0u) continue;
-          const int k = k0 + 4 * t + q;
-          float w[4][NJ];
+      for (int i = 0; i < SM_AHEAD; ++i) {
+        if (idx[i] < 0) continue;
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
+        for (int c = 0; c < 4; ++c) {
+          if (c >= c_in) break;
+          const f32x2 xx = pair_of(x[i][c], x[i][c]);
+          if (STAGED) {
+            const ulonglong2 *w = (const ulonglong2 *)(ws + ((size_t)(k0 + i) * c_in + c) * CB);
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-              if (STAGED) w[c][j] = c < c_in ? ws[((size_t)k * c_in + c) * (NJ * 32) + j * 32 + lane] : 0.f;
-              else w[c][j] = (c < c_in && n0 + j * 32 + lane < c_out) ? __ldg(filters + ((size_t)k * c_in + c) * c_out + n0 + j * 32 + lane) : 0.f;
+            for (int j = 0; j < CB / 2; j += 2) {
+              const ulonglong2 v = w[j / 2];
+              acc[j] = fma_pair(xx, v.x, acc[j]);
+              acc[j + 1] = fma_pair(xx, v.y, acc[j + 1]);
             }
+          } else {
+            const float *w = filters + ((size_t)(k0 + i) * c_in + c) * c_out + n0;
 #pragma unroll
-          for (int r = 0; r < SM_ROWS; ++r) {
-            if (!((m >> r) & 1u)) continue;    // the same for the whole warp
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const float xv = __shfl_sync(0xffffffffu, x[t][c], 8 * q + r);
-              if (c < c_in) {
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) acc[r][j] = fmaf(xv, w[c][j], acc[r][j]);
-              }
-            }
+            for (int j = 0; j < CB / 2; ++j)
+              acc[j] = fma_pair(xx, pair_of(n0 + 2 * j < c_out ? __ldg(w + 2 * j) : 0.f, n0 + 2 * j + 1 < c_out ? __ldg(w + 2 * j + 1) : 0.f), acc[j]);
           }
         }
       }
     }
+    if (row >= n_rows) continue;
+    float *to = out + (size_t)row * c_out + n0;
 #pragma unroll
-    for (int r = 0; r < SM_ROWS; ++r) {
-      if (m0 + r >= n_rows) break;
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const int ch = n0 + j * 32 + lane;
-        if (ch < c_out) out[(size_t)(m0 + r) * c_out + ch] = acc[r][j];
+    for (int j = 0; j < CB / 2; j += 2) {
+      const int ch = n0 + 2 * j;
+      const float2 a = halves(acc[j]), b = halves(acc[j + 1]);
+      if (vec) {
+        if (ch < c_out) *(float4 *)(to + 2 * j) = make_float4(a.x, a.y, b.x, b.y);
+      } else {
+        if (ch < c_out) to[2 * j] = a.x;
+        if (ch + 1 < c_out) to[2 * j + 1] = a.y;
+        if (ch + 2 < c_out) to[2 * j + 2] = b.x;
+        if (ch + 3 < c_out) to[2 * j + 3] = b.y;
       }
     }
   }
 }
 
-template <int NJ>
+template <int CB>
 static int launch_fp32_small(const float *features, int c_in, const float *filters, int K, int c_out, const int32_t *nbr, int n_out,
                              int rev, float *out, const int32_t *n_out_dev, cudaStream_t st) {
-  const size_t smem = (size_t)K * c_in * NJ * 32 * sizeof(float);
+  const size_t smem = (size_t)K * c_in * CB * sizeof(float);
   const bool staged = smem <= 100 * 1024;     // two blocks per SM at least; larger filter sets are read through L1
-  const int blocks = ceil_div(n_out, SM_WARPS * SM_ROWS), most = sm_count() * 3;
-  const dim3 grid(blocks < most ? blocks : most, ceil_div(c_out, NJ * 32));
-  auto kernel = staged ? conv_fwd_fp32_small_kernel<NJ, true> : conv_fwd_fp32_small_kernel<NJ, false>;
+  const int blocks = ceil_div(n_out, SM_WARPS * 32), most = sm_count() * 2;
+  const dim3 grid(blocks < most ? blocks : most, ceil_div(c_out, CB));
+  auto kernel = staged ? conv_fwd_fp32_small_kernel<CB, true> : conv_fwd_fp32_small_kernel<CB, false>;
   if (staged && smem > 48 * 1024) {
     cudaError_t e = allow_smem((const void *)kernel, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(fp32): smem attribute: %s", cudaGetErrorString(e));
@@ -343,9 +361,12 @@ extern "C" int ssc_conv_fwd_ordered(const float *features, int n_in, int c_in, c
     if (c_in <= 4 && (c_in != 4 || ((uintptr_t)features & 15u) == 0)) {
       const int rev = table_form != 0;
       const float *w = (const float *)filters;
-      if (c_out <= 32) return launch_fp32_small<1>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
-      if (c_out <= 64) return launch_fp32_small<2>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
-      return launch_fp32_small<3>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+      const int per = ceil_div(c_out, ceil_div(c_out, 48));          // channels of a lane
+      if (per <= 16) return launch_fp32_small<16>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+      if (per <= 24) return launch_fp32_small<24>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+      if (per <= 32) return launch_fp32_small<32>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+      if (per <= 40) return launch_fp32_small<40>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+      return launch_fp32_small<48>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
     }
     dim3 grid(ceil_div(n_out, BM), ceil_div(c_out, BN));
     { conv_fwd_fp32_kernel<<<grid, 256, 0, st>>>(features, c_in, (const float *)filters, K, c_out, nbr, n_out, table_form != 0, out, n_out_dev); note_launches(1); }

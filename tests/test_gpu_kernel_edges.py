@@ -118,6 +118,27 @@ def test_fp32_convolution_of_few_input_channels(cuda, c_in, c_out, k, n):
     assert rel_err(y, ref) <= 2e-5
 
 
+@pytest.mark.parametrize("c_in", [1, 3, 4])
+@pytest.mark.parametrize("c_out", [16, 17, 25, 33, 41, 48, 49, 97])
+@pytest.mark.parametrize("K,n", [(1, 31), (9, 33), (10, 257), (125, 300)])
+def test_fp32_convolution_by_lanes_of_rows(cuda, c_in, c_out, K, n):
+    """Channels of a lane (16, 24, 32, 40, 48, several passes over the rows, filters too large for shared memory), offsets around the
+    nine in flight, rows around a warp and a block.  Every term is rounded once, so |error| <= terms * 2^-24 * sum |x w|;
+    a filter that is not a number reaches the rows that have its offset and no others."""
+    from ss_conv import _ext
+    rng = np.random.RandomState(K + c_out)
+    t = _table(n, 200, K, 0.4, rng)
+    x, w = rng.randn(200, c_in), rng.randn(K, c_in, c_out)
+    x, w = x.astype(np.float32), w.astype(np.float32)
+    got = _ext.conv_forward(dev(x, cuda), dev(w, cuda), dev(t, cuda), n, "fp32").cpu().numpy().astype(np.float64)
+    g = np.where((t >= 0)[:, :, None], x[t], 0).astype(np.float64)
+    want, size = np.einsum("knc,kco->no", g, w.astype(np.float64)), np.einsum("knc,kco->no", abs(g), abs(w).astype(np.float64))
+    assert (abs(got - want) <= K * c_in * 2.0 ** -24 * size).all()
+    w[K // 2, 0, c_out - 1] = np.nan
+    got = _ext.conv_forward(dev(x, cuda), dev(w, cuda), dev(t, cuda), n, "fp32").cpu().numpy()
+    assert (np.isnan(got[:, -1]) == (t[K // 2] >= 0)).all() and np.isfinite(got[:, :-1]).all()
+
+
 @pytest.mark.parametrize("orders,batch", [(1, 1), (4, 65), (8, 3)])
 @pytest.mark.parametrize("frame", ["kernel", "reference"])
 def test_steering_matrices_match_the_host_form(cuda, orders, batch, frame):
