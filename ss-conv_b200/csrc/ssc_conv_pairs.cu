@@ -84,9 +84,8 @@ struct PlParams {
 // strip cost a scan of all of them, 140 us for the 330 strips of a 5^3 layer; with a load per thread of the
 // block and two barriers per strip 30 us.  One warp now holds ten loads per lane in registers (the lowest
 // CTA wins ties); the first strip of every CTA needs no decision (all loads are zero, so they go in order).
-__global__ void __launch_bounds__(PL_MAX_CTAS)
-pl_strips_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_ctas,
-                 int32_t *__restrict__ hdr, int4 *__restrict__ strips, int32_t *__restrict__ owner) {
+__device__ __forceinline__ void deal_strips(const int32_t *__restrict__ starts, int K, int n_split, int n_ctas,
+                                            int32_t *__restrict__ hdr, int4 *__restrict__ strips, int32_t *__restrict__ owner) {
   __shared__ int tiles[256], first[257], tiles_of[PL_MAX_CTAS];
   __shared__ int L_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -197,6 +196,33 @@ pl_strips_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_c
     __threadfence();
     hdr[0] = n_strips;
   }
+}
+
+// What the persistent kernel needs beforehand, in one launch: the strip table (block 0: 16 us of one block's
+// serial work), the operand image of the rows (n_stage pieces of 16 bytes, as ssc_conv_stage.cu writes it; 0 where it is there
+// already) and a cleared output.  The last two are bound by memory, and the strips come in their shadow.
+// (42 k rows 192 -> 192 bf16: 9 + 7 + 16 us one after the other, 22 like this; the whole layer 246 -> 232.)
+template <bool F16>
+__global__ void __launch_bounds__(PL_MAX_CTAS)
+pl_prepare_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_ctas, int32_t *__restrict__ hdr, int4 *__restrict__ strips,
+                  int32_t *__restrict__ owner, const float4 *__restrict__ rows, long long n_stage, int bf16, uint4 *__restrict__ staged,
+                  float4 *__restrict__ out, long long n_clear) {
+  if (blockIdx.x == 0) {
+    deal_strips(starts, K, n_split, n_ctas, hdr, strips, owner);
+    return;
+  }
+  const long long first = (long long)(blockIdx.x - 1) * PL_MAX_CTAS + threadIdx.x, step = (long long)(gridDim.x - 1) * PL_MAX_CTAS;
+  for (long long i = first; i < n_stage; i += step) {
+    if (F16) {
+      const float4 a = __ldg(rows + 2 * i), b = __ldg(rows + 2 * i + 1);
+      staged[i] = bf16 ? make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w))
+                       : make_uint4(pack_f16x2(a.x, a.y), pack_f16x2(a.z, a.w), pack_f16x2(b.x, b.y), pack_f16x2(b.z, b.w));
+    } else {
+      const float4 v = __ldg(rows + i);
+      staged[i] = make_uint4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
+    }
+  }
+  for (long long i = first; i < n_clear; i += step) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // A lane's piece of two rows (none of a negative one), OFF bytes into its part of the slot.
@@ -540,7 +566,8 @@ static size_t max_strips(int K) { return (size_t)PL_MAX_CTAS + 16 * (size_t)K + 
 size_t conv_pairs_strip_bytes(int K) { return 256 + max_strips(K) * (sizeof(int4) + sizeof(int32_t)); }
 
 // `staged`: the operand image of the feature rows (ssc_conv_stage); `strip_mem`: conv_pairs_strip_bytes(K) bytes.
-int conv_fwd_pairs(const void *staged, int c_in, const void *packed, int K, int c_out, int precision,
+// rows: the features to be staged, null where `staged` holds their image.
+int conv_fwd_pairs(const float *rows, int n_in, void *staged, int c_in, const void *packed, int K, int c_out, int precision,
                    const PairLists &pl, int n_out, float *out, int32_t *status, void *strip_mem, cudaStream_t st) {
   PlParams p;
   if (K > 256 || !pl_params(c_in, c_out, precision, p))
@@ -551,10 +578,30 @@ int conv_fwd_pairs(const void *staged, int c_in, const void *packed, int K, int 
   int32_t *hdr = (int32_t *)strip_mem;
   int4 *strips = (int4 *)((uint8_t *)strip_mem + 256);
   int32_t *owner = (int32_t *)(strips + max_strips(K));
-  cudaError_t e = cudaMemsetAsync(out, 0, (size_t)n_out * c_out * sizeof(float), st);
-  if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd_pairs: clearing the output: %s", cudaGetErrorString(e));
-  { pl_strips_kernel<<<1, PL_MAX_CTAS, 0, st>>>(pl.starts, K, p.n_split, n_ctas, hdr, strips, owner); note_launches(1); }
-  SSC_CHECK_LAUNCH("pl_strips");
+  // the image in 16-byte pieces where rows and image have no padding (else by the general kernel), the output likewise
+  const bool bf16 = precision == SSC_PREC_BF16;
+  const int per_piece = p.f16 ? 8 : 4;
+  long long n_stage = 0, n_clear = 0;
+  cudaError_t e;
+  if (rows != nullptr && n_in > 0) {
+    if (c_in % per_piece == 0 && (((uintptr_t)rows | (uintptr_t)staged) & 15u) == 0) {
+      n_stage = (long long)n_in * c_in / per_piece;
+    } else {
+      const int rc = p.f16 ? stage_features_16(rows, n_in, c_in, bf16, staged, st) : stage_features(rows, n_in, c_in, staged, st);
+      if (rc != SSC_OK) return rc;
+    }
+  }
+  if (((uintptr_t)out & 15u) == 0 && ((long long)n_out * c_out & 3) == 0) {
+    n_clear = (long long)n_out * c_out / 4;
+  } else {
+    e = cudaMemsetAsync(out, 0, (size_t)n_out * c_out * sizeof(float), st);
+    if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd_pairs: clearing the output: %s", cudaGetErrorString(e));
+  }
+  const int want = ceil_div(n_stage > n_clear ? n_stage : n_clear, PL_MAX_CTAS * 2), most = sm_count() * 6;
+  const int blocks = 1 + (want < most ? want : most);
+  auto prepare = p.f16 ? pl_prepare_kernel<true> : pl_prepare_kernel<false>;
+  { prepare<<<blocks, PL_MAX_CTAS, 0, st>>>(pl.starts, K, p.n_split, n_ctas, hdr, strips, owner, (const float4 *)rows, n_stage, bf16 ? 1 : 0, (uint4 *)staged, (float4 *)out, n_clear); note_launches(1); }
+  SSC_CHECK_LAUNCH("pl_prepare");
   const size_t smem = pl_smem_bytes(p);
   auto kernel = p.f16 ? conv_fwd_pairs_kernel<true> : conv_fwd_pairs_kernel<false>;
   e = allow_smem((const void *)kernel, smem);
@@ -604,12 +651,7 @@ extern "C" int ssc_conv_fwd_pairs(const float *features, int n_in, int c_in, con
   SSC_REQUIRE(scratch_bytes + 16 >= ssc_conv_scratch_bytes(n_in, c_in, c_out, precision) && ((uintptr_t)scratch & 15u) == 0,
               "conv_fwd_pairs: staging buffer too small or not 16-byte aligned");
   cudaStream_t st = as_stream(stream);
-  if (!prestaged) {
-    int rc = precision == SSC_PREC_TF32 ? stage_features(features, n_in, c_in, scratch, st)
-                                        : stage_features_16(features, n_in, c_in, precision == SSC_PREC_BF16, scratch, st);
-    if (rc != SSC_OK) return rc;
-  }
   const PairLists pl = pair_lists_view(lists, K, n_out);
   void *strip_mem = (uint8_t *)lists + align_up(pair_lists_bytes(K, n_out), 256);
-  return conv_fwd_pairs(scratch, c_in, packed, K, c_out, precision, pl, n_out, out, status, strip_mem, st);
+  return conv_fwd_pairs(prestaged ? nullptr : features, n_in, scratch, c_in, packed, K, c_out, precision, pl, n_out, out, status, strip_mem, st);
 }

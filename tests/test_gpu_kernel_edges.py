@@ -139,6 +139,23 @@ def test_fp32_convolution_by_lanes_of_rows(cuda, c_in, c_out, K, n):
     assert (np.isnan(got[:, -1]) == (t[K // 2] >= 0)).all() and np.isfinite(got[:, :-1]).all()
 
 
+@pytest.mark.parametrize("precision", ["tf32", "bf16", "fp16"])
+@pytest.mark.parametrize("c_in,c_out,n", [(128, 128, 1), (132, 136, 129), (134, 130, 300), (192, 130, 77)])
+def test_pair_lists_prepared_in_one_launch(cuda, precision, c_in, c_out, n):
+    """Rows staged and outputs cleared next to the strip table, and by the general kernels where rows or outputs are no whole
+    16-byte pieces.  Same operands and fp32 sums as the output-stationary kernel, in another order."""
+    from ss_conv import _ext
+    if not _ext.lib().ssc_conv_pairs_supported(c_in, c_out, _ext._PREC_OF[precision]):
+        pytest.skip("shape not covered by the pair-list kernel")
+    rng = np.random.RandomState(n)
+    t = dev(_table(n, 150, 27, 0.3, rng), cuda)
+    x = dev(rng.randn(150, c_in).astype(np.float32), cuda)
+    w = dev((rng.randn(27, c_in, c_out) * 0.1).astype(np.float32), cuda)
+    rows = _ext.conv_forward(x, w, t, n, precision, algo="rows")
+    pairs = _ext.conv_forward(x, w, t, n, precision, algo="pairs")
+    assert rel_err(pairs.cpu(), rows.cpu()) <= 5e-5
+
+
 @pytest.mark.parametrize("orders,batch", [(1, 1), (4, 65), (8, 3)])
 @pytest.mark.parametrize("frame", ["kernel", "reference"])
 def test_steering_matrices_match_the_host_form(cuda, orders, batch, frame):
