@@ -405,6 +405,9 @@ rank_decode_kernel(const uint32_t *__restrict__ bitmap, int n_words, Geometry g,
 // are decoded once; every offset costs a few integer operations, one load from the row map and
 // one coalesced store.
 // Block = kChunk rows; counts per (offset, chunk) are only produced when chunk_counts is given.
+// N = ksize[1] = ksize[2] (0: any): the N x N loads of a thread are all in flight together, where the general form waits for
+// one after the other (1.1 M rows 3^3: 69 -> 47 us, 177 k rows 5^3: 47 -> 34, 140 k rows 3^3: 12.4 -> 8.8, 16 k rows: 4.7 -> 3.0).
+template <int N>
 __global__ void __launch_bounds__(256)
 lookup_dense_kernel(const int4 *__restrict__ out_indices, int n_out, int batch, Geometry g,
                     const int32_t *__restrict__ row_map, int32_t *__restrict__ nbr,
@@ -440,17 +443,37 @@ lookup_dense_kernel(const int4 *__restrict__ out_indices, int n_out, int batch, 
   {
     const int kx = (int)blockIdx.y;
     const int x = coord(0, kx);
-    for (int ky = 0; ky < g.ksize[1]; ++ky) {
-      const int y = coord(1, ky);
-      const long long plane = ((long long)(base * g.in_shape[0] + x) * g.in_shape[1] + y) * g.in_shape[2];
-      for (int kz = 0; kz < g.ksize[2]; ++kz, ++kappa) {
-        const int z = coord(2, kz);
-        int found = -1;
-        if (base >= 0 && (x | y | z) >= 0) found = __ldg(row_map + plane + z) - 1;
-        if (o < n_out) nbr[(size_t)kappa * n_out + o] = found;
-        if (counting) {
-          const unsigned hits = __ballot_sync(0xffffffffu, found >= 0);
-          if ((threadIdx.x & 31) == 0 && hits) atomicAdd(cnt + kappa, __popc(hits));
+    auto keep = [&](int found) {
+      if (o < n_out) nbr[(size_t)kappa * n_out + o] = found;
+      if (counting) {
+        const unsigned hits = __ballot_sync(0xffffffffu, found >= 0);
+        if ((threadIdx.x & 31) == 0 && hits) atomicAdd(cnt + kappa, __popc(hits));
+      }
+      ++kappa;
+    };
+    if (N > 0) {
+      int z[N > 0 ? N : 1], found[N > 0 ? N * N : 1];
+#pragma unroll
+      for (int kz = 0; kz < N; ++kz) z[kz] = coord(2, kz);
+#pragma unroll
+      for (int ky = 0; ky < N; ++ky) {
+        const int y = coord(1, ky);
+        const int32_t *line = row_map + ((long long)(base * g.in_shape[0] + x) * g.in_shape[1] + y) * g.in_shape[2];
+        const bool in = base >= 0 && (x | y) >= 0;
+#pragma unroll
+        for (int kz = 0; kz < N; ++kz) found[ky * N + kz] = in && z[kz] >= 0 ? __ldg(line + z[kz]) : 0;
+      }
+#pragma unroll
+      for (int i = 0; i < N * N; ++i) keep(found[i] - 1);
+    } else {
+      for (int ky = 0; ky < g.ksize[1]; ++ky) {
+        const int y = coord(1, ky);
+        const long long plane = ((long long)(base * g.in_shape[0] + x) * g.in_shape[1] + y) * g.in_shape[2];
+        for (int kz = 0; kz < g.ksize[2]; ++kz) {
+          const int z = coord(2, kz);
+          int found = -1;
+          if (base >= 0 && (x | y | z) >= 0) found = __ldg(row_map + plane + z) - 1;
+          keep(found);
         }
       }
     }
@@ -658,7 +681,9 @@ static int lookup_and_compact(const int32_t *out_indices, int n_out, int n_in, i
     int32_t *counts = indice_num != nullptr ? s.chunk_counts : nullptr;
     if (counts) cudaMemsetAsync(counts, 0, (size_t)n_chunks * K * 4, st);
     const dim3 lgrid(ceil_div(n_out > 0 ? n_out : 1, 256), g.ksize[0]);
-    { lookup_dense_kernel<<<lgrid, 256, K * sizeof(int32_t), st>>>(
+    const int side = g.ksize[1] == g.ksize[2] ? g.ksize[1] : 0;
+    auto lookup = side == 3 ? lookup_dense_kernel<3> : side == 5 ? lookup_dense_kernel<5> : side == 2 ? lookup_dense_kernel<2> : lookup_dense_kernel<0>;
+    { lookup<<<lgrid, 256, K * sizeof(int32_t), st>>>(
           (const int4 *)out_indices, n_out, batch, g, s.row_map, nbr, counts, n_chunks, n_out_dev); note_launches(1); }
   } else {
     dim3 grid(n_chunks, K);
