@@ -22,18 +22,19 @@ int sm_count() {
   return sms;
 }
 
-__global__ void stage_features_kernel(const float4 *__restrict__ in, long long n_vec, long long total_vec,
-                                      uint4 *__restrict__ out) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long step = (long long)gridDim.x * blockDim.x;
-  for (; i < total_vec; i += step) {
-    uint4 o = make_uint4(0u, 0u, 0u, 0u);
-    if (i < n_vec) {
-      float4 v = __ldg(in + i);
-      o = make_uint4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
-    }
-    out[i] = o;
-  }
+// Rows without padding: STAGE_VECS 16-byte pieces per thread, all loads before the first store.  With one at a time a thread
+// waited for memory four times over (121 k rows of 64: 6.4 -> 5.1 us; 1.1 M rows: 111 -> 100).
+constexpr int STAGE_VECS = 4;
+__global__ void __launch_bounds__(256)
+stage_features_kernel(const float4 *__restrict__ in, long long total_vec, uint4 *__restrict__ out) {
+  const long long first = (long long)blockIdx.x * (256 * STAGE_VECS) + threadIdx.x;
+  float4 v[STAGE_VECS];
+#pragma unroll
+  for (int q = 0; q < STAGE_VECS; ++q)
+    if (first + q * 256 < total_vec) v[q] = __ldg(in + first + q * 256);
+#pragma unroll
+  for (int q = 0; q < STAGE_VECS; ++q)
+    if (first + q * 256 < total_vec) out[first + q * 256] = make_uint4(to_tf32(v[q].x), to_tf32(v[q].y), to_tf32(v[q].z), to_tf32(v[q].w));
 }
 
 // Channel counts that are not a multiple of four: rows padded with zeros to c_pad floats.
@@ -68,20 +69,17 @@ size_t conv_tf32_scratch_bytes(int n_in, int c_in) {
 
 int stage_features(const float *features, int n_in, int c_in, void *staged, cudaStream_t st) {
   const int c_pad = (c_in + 3) & ~3;
-  const int max_blocks = sm_count() * 16;
   if (n_in == 0) return SSC_OK;
   if (c_pad == c_in && ((uintptr_t)features & 15u) == 0) {
-    const long long n_vec = (long long)n_in * c_in / 4, total_vec = n_vec;
-    int blocks = ceil_div(total_vec, 256 * 4);
-    if (blocks > max_blocks) blocks = max_blocks;
-    { stage_features_kernel<<<blocks, 256, 0, st>>>((const float4 *)features, n_vec, total_vec, (uint4 *)staged); note_launches(1); }
+    const long long total_vec = (long long)n_in * c_in / 4;
+    { stage_features_kernel<<<ceil_div(total_vec, 256 * STAGE_VECS), 256, 0, st>>>((const float4 *)features, total_vec, (uint4 *)staged); note_launches(1); }
   } else if (c_pad <= 1024) {
     const int groups = c_pad >> 2, rows = 256 / groups;
     { stage_features_padded_rows_kernel<<<ceil_div(n_in, rows), dim3(groups, rows), 0, st>>>(features, n_in, c_in, (uint4 *)staged); note_launches(1); }
   } else {
     const long long total = (long long)n_in * c_pad;
     int blocks = ceil_div(total, 256 * 4);
-    if (blocks > max_blocks) blocks = max_blocks;
+    if (blocks > sm_count() * 16) blocks = sm_count() * 16;
     { stage_features_padded_kernel<<<blocks, 256, 0, st>>>(features, n_in, c_in, c_pad, total, (uint32_t *)staged); note_launches(1); }
   }
   SSC_CHECK_LAUNCH("stage_features");
@@ -113,12 +111,19 @@ __global__ void stage_features_16_kernel(const float *__restrict__ in, long long
 template <bool BF16>
 __global__ void __launch_bounds__(256)
 stage_features_16_vec_kernel(const float4 *__restrict__ in, long long total, uint4 *__restrict__ out) {
-  const long long step = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
-    const float4 a = __ldg(in + 2 * i), b = __ldg(in + 2 * i + 1);
-    out[i] = BF16 ? make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w))
-                  : make_uint4(pack_f16x2(a.x, a.y), pack_f16x2(a.z, a.w), pack_f16x2(b.x, b.y), pack_f16x2(b.z, b.w));
-  }
+  const long long first = (long long)blockIdx.x * (256 * STAGE_VECS) + threadIdx.x;
+  float4 a[STAGE_VECS], b[STAGE_VECS];
+#pragma unroll
+  for (int q = 0; q < STAGE_VECS; ++q)
+    if (first + q * 256 < total) {
+      a[q] = __ldg(in + 2 * (first + q * 256));
+      b[q] = __ldg(in + 2 * (first + q * 256) + 1);
+    }
+#pragma unroll
+  for (int q = 0; q < STAGE_VECS; ++q)
+    if (first + q * 256 < total)
+      out[first + q * 256] = BF16 ? make_uint4(pack_bf16x2(a[q].x, a[q].y), pack_bf16x2(a[q].z, a[q].w), pack_bf16x2(b[q].x, b[q].y), pack_bf16x2(b[q].z, b[q].w))
+                                  : make_uint4(pack_f16x2(a[q].x, a[q].y), pack_f16x2(a[q].z, a[q].w), pack_f16x2(b[q].x, b[q].y), pack_f16x2(b[q].z, b[q].w));
 }
 
 size_t conv_f16_scratch_bytes(int n_in, int c_in) { return (size_t)n_in * (size_t)f16_row_words(c_in) * 4 + 16; }
@@ -128,8 +133,7 @@ int stage_features_16(const float *features, int n_in, int c_in, bool bf16, void
   const int words = f16_row_words(c_in);
   if ((c_in & 7) == 0 && (((uintptr_t)features | (uintptr_t)staged) & 15u) == 0) {
     const long long total = (long long)n_in * c_in / 8;
-    int vb = ceil_div(total, 256 * 2);
-    if (vb > sm_count() * 16) vb = sm_count() * 16;
+    const int vb = ceil_div(total, 256 * STAGE_VECS);
     if (bf16) stage_features_16_vec_kernel<true><<<vb, 256, 0, st>>>((const float4 *)features, total, (uint4 *)staged);
     else stage_features_16_vec_kernel<false><<<vb, 256, 0, st>>>((const float4 *)features, total, (uint4 *)staged);
     note_launches(1);
