@@ -319,132 +319,117 @@ static void fill_grid(VoxelGrid &g, const int grid[3], const float unit[3]) {
 }
 
 // ----------------------------------------------------------------------- three_nn
-constexpr int NN_TILE = 1024;
+// Known points in tiles of 1024 (ranges: batch ids of a tile) and chunks of 32 (chunks: batch ids and x coordinates of a
+// chunk; points in grid order, as the voxelizer and the rulebook give them, have a slab of few x).
+constexpr int NN_CHUNK = 32, NN_TILE = 32 * NN_CHUNK;
 
-__global__ void nn_tile_range_kernel(const float4 *__restrict__ known, int m, float2 *ranges) {
-  __shared__ float smin[8], smax[8];
-  int tile = blockIdx.x;
-  float lo = INFINITY, hi = -INFINITY;
-  for (int i = threadIdx.x; i < NN_TILE; i += blockDim.x) {
-    int k = tile * NN_TILE + i;
+__global__ void __launch_bounds__(256)
+nn_ranges_kernel(const float4 *__restrict__ known, int m, float2 *__restrict__ ranges, float4 *__restrict__ chunks) {
+  __shared__ float lo_s[NN_TILE / NN_CHUNK], hi_s[NN_TILE / NN_CHUNK];
+  const int lane = threadIdx.x & 31;
+  for (int c = threadIdx.x >> 5; c < NN_TILE / NN_CHUNK; c += 8) {
+    const int k = blockIdx.x * NN_TILE + c * NN_CHUNK + lane;
+    float4 r = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
     if (k < m) {
-      float b = known[k].x;
-      lo = fminf(lo, b);
-      hi = fmaxf(hi, b);
+      const float4 p = known[k];
+      // (fminf and fmaxf pass over a coordinate that is not a number: such a point is nobody's neighbour)
+      r = make_float4(fminf(INFINITY, p.x), fmaxf(-INFINITY, p.x), fminf(INFINITY, p.y), fmaxf(-INFINITY, p.y));
     }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fminf(lo, __shfl_down_sync(0xffffffffu, lo, o));
-    hi = fmaxf(hi, __shfl_down_sync(0xffffffffu, hi, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    smin[threadIdx.x >> 5] = lo;
-    smax[threadIdx.x >> 5] = hi;
+    for (int o = 16; o > 0; o >>= 1) {
+      r.x = fminf(r.x, __shfl_xor_sync(0xffffffffu, r.x, o));
+      r.y = fmaxf(r.y, __shfl_xor_sync(0xffffffffu, r.y, o));
+      r.z = fminf(r.z, __shfl_xor_sync(0xffffffffu, r.z, o));
+      r.w = fmaxf(r.w, __shfl_xor_sync(0xffffffffu, r.w, o));
+    }
+    if (lane == 0) {
+      chunks[blockIdx.x * (NN_TILE / NN_CHUNK) + c] = r;
+      lo_s[c] = r.x;
+      hi_s[c] = r.y;
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (blockDim.x >> 5); ++w) {
-      lo = fminf(lo, smin[w]);
-      hi = fmaxf(hi, smax[w]);
+  if (threadIdx.x < 32) {
+    float lo = lo_s[lane], hi = hi_s[lane];
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     }
-    ranges[tile] = make_float2(lo, hi);
+    if (lane == 0) ranges[blockIdx.x] = make_float2(lo, hi);
   }
 }
 
-// 64 queries per block, four threads per query; known points stream through shared memory in tiles of 1024,
-// tiles whose batch-id range cannot match any query of the block are skipped.  Thread s of a query
-// looks at every fourth point of a tile; the three best of the four are merged by (distance, index), which is
-// the result of the exhaustive reference loop (ascending k, strict <): the smallest index wins ties.
-// A thread per query left each SM with two blocks of one long serial scan: 150 us for 65 k queries.
-constexpr int NN_SPLIT = 4;
+// A warp per query.  Its lanes look at the ranges of 32 tiles at a time, then at the 32 chunks of a tile that can hold points of
+// the query's sample: first at the points of the chunks nearest in x, then of those whose distance in x alone does not
+// exceed the third best so far.  That distance, rounded like the points' own, is never more than theirs: every rounding
+// involved is monotonic.  Each lane keeps its three best by (distance, index); the three best of the warp by that order are
+// the result of the exhaustive reference loop (ascending index, strict <).
+// 65 k queries among 1000 points each: 80 us (a chain of trips to L1 and votes per query); 132 with four
+// threads per query that looked at every point of the sample.
+constexpr int NN_QUERIES = 4;                     // of a warp, one after the other
 __global__ void __launch_bounds__(256)
 three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known,
-                const float2 *__restrict__ ranges, float *__restrict__ dist2, int32_t *__restrict__ idx) {
-  __shared__ float4 tile[NN_TILE];
-  __shared__ float qmin_s[8], qmax_s[8];
-  const int q = blockIdx.x * (256 / NN_SPLIT) + (int)threadIdx.x / NN_SPLIT, part = threadIdx.x % NN_SPLIT;
-  float4 u = q < n ? unknown[q] : make_float4(NAN, 0.f, 0.f, 0.f);
-  float lo = q < n ? u.x : INFINITY, hi = q < n ? u.x : -INFINITY;
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fminf(lo, __shfl_down_sync(0xffffffffu, lo, o));
-    hi = fmaxf(hi, __shfl_down_sync(0xffffffffu, hi, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    qmin_s[threadIdx.x >> 5] = lo;
-    qmax_s[threadIdx.x >> 5] = hi;
-  }
-  __syncthreads();
-  float qmin = qmin_s[0], qmax = qmax_s[0];
-  for (int w = 1; w < 8; ++w) {
-    qmin = fminf(qmin, qmin_s[w]);
-    qmax = fmaxf(qmax, qmax_s[w]);
-  }
-  float best[3] = {INFINITY, INFINITY, INFINITY};
-  int at[3] = {0, 0, 0};
-  // (d, i) into the ordered triple; equal distances stay behind
-  auto take = [&](float d, int i) {
-    if (d < best[0]) {
-      best[2] = best[1]; at[2] = at[1];
-      best[1] = best[0]; at[1] = at[0];
-      best[0] = d; at[0] = i;
-    } else if (d < best[1]) {
-      best[2] = best[1]; at[2] = at[1];
-      best[1] = d; at[1] = i;
-    } else if (d < best[2]) {
-      best[2] = d; at[2] = i;
-    }
-  };
-  const int n_tiles = (m + NN_TILE - 1) / NN_TILE;
-  for (int t = 0; t < n_tiles; ++t) {
-    const float2 r = ranges[t];
-    if (r.y < qmin || r.x > qmax) continue;  // block-uniform
-    __syncthreads();
-    const int base = t * NN_TILE;
-    for (int i = threadIdx.x; i < NN_TILE; i += 256) tile[i] = base + i < m ? known[base + i] : make_float4(NAN, 0.f, 0.f, 0.f);
-    __syncthreads();
-    const int cnt = min(NN_TILE, m - base);
-    if (q < n && !(r.y < u.x || r.x > u.x)) {
-#pragma unroll 4
-      for (int i = part; i < cnt; i += NN_SPLIT) {
-        const float4 k = tile[i];
-        const float dx = __fsub_rn(u.y, k.y), dy = __fsub_rn(u.z, k.z), dz = __fsub_rn(u.w, k.w);
-        // the contraction nvcc applies to the reference's dx*dx + dy*dy + dz*dz
-        // (interpolate_cuda_kernel.cu:39), checked bit for bit against the reference's own kernel
-        const float d = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
-        if (k.x == u.x && d < best[2]) take(d, base + i);
+                const float2 *__restrict__ ranges, const float4 *__restrict__ chunks, float *__restrict__ dist2, int32_t *__restrict__ idx) {
+  const int lane = threadIdx.x & 31, n_tiles = (m + NN_TILE - 1) / NN_TILE, n_chunks = (m + NN_CHUNK - 1) / NN_CHUNK;
+  const int q0 = ((int)blockIdx.x * 8 + ((int)threadIdx.x >> 5)) * NN_QUERIES;
+  for (int q = q0; q < min(q0 + NN_QUERIES, n); ++q) {
+    const float4 u = __ldg(unknown + q);
+    float d0 = INFINITY, d1 = INFINITY, d2 = INFINITY;
+    int i0 = 0, i1 = 0, i2 = 0;
+    auto before = [](float d, int i, float e, int j) { return d < e || (d == e && i < j); };
+    auto look_at = [&](int chunk) {
+      const int i = chunk * NN_CHUNK + lane;
+      if (i >= m) return;
+      const float4 k = __ldg(known + i);
+      const float dx = __fsub_rn(u.y, k.y), dy = __fsub_rn(u.z, k.z), dz = __fsub_rn(u.w, k.w);
+      // the contraction nvcc applies to the reference's dx*dx + dy*dy + dz*dz
+      // (interpolate_cuda_kernel.cu:39), checked bit for bit against the reference's own kernel
+      const float d = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+      if (k.x == u.x && d < INFINITY && before(d, i, d2, i2)) {
+        if (before(d, i, d1, i1)) {
+          d2 = d1; i2 = i1;
+          if (before(d, i, d0, i0)) { d1 = d0; i1 = i0; d0 = d; i0 = i; }
+          else { d1 = d; i1 = i; }
+        } else {
+          d2 = d; i2 = i;
+        }
+      }
+    };
+    // (distances are not negative: their order is that of their bits)
+    auto third_best = [&]() {
+      uint32_t a = __float_as_uint(d0), b = __float_as_uint(d1), c = __float_as_uint(d2), least = 0u;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        least = __reduce_min_sync(0xffffffffu, a);
+        const int first = __ffs((int)__ballot_sync(0xffffffffu, a == least)) - 1;
+        if (lane == first) { a = b; b = c; c = 0x7f800000u; }
+      }
+      return __uint_as_float(least);
+    };
+    for (int t0 = 0; t0 < n_tiles; t0 += 32) {
+      const float2 r = t0 + lane < n_tiles ? __ldg(ranges + t0 + lane) : make_float2(INFINITY, -INFINITY);
+      for (unsigned tiles = __ballot_sync(0xffffffffu, r.x <= u.x && u.x <= r.y); tiles != 0u; tiles &= tiles - 1u) {
+        const int c0 = (t0 + __ffs((int)tiles) - 1) * (NN_TILE / NN_CHUNK);
+        const float4 c = c0 + lane < n_chunks ? __ldg(chunks + c0 + lane) : make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
+        const bool may = c.x <= u.x && u.x <= c.y;
+        const float off = fmaxf(0.f, fmaxf(__fsub_rn(c.z, u.y), __fsub_rn(u.y, c.w)));
+        const float least = may ? __fmul_rn(off, off) : INFINITY;     // no point of the chunk is nearer
+        const uint32_t nearest = __reduce_min_sync(0xffffffffu, __float_as_uint(least));
+        const bool near = may && __float_as_uint(least) == nearest;
+        for (unsigned left = __ballot_sync(0xffffffffu, near); left != 0u; left &= left - 1u) look_at(c0 + __ffs((int)left) - 1);
+        const float limit = third_best();
+        for (unsigned left = __ballot_sync(0xffffffffu, may && !near && least <= limit); left != 0u; left &= left - 1u) look_at(c0 + __ffs((int)left) - 1);
       }
     }
-  }
-  // merge the partners' triples (a slot that was never filled is infinite and loses to everything)
-#pragma unroll
-  for (int o = 1; o < NN_SPLIT; o <<= 1) {
-    float od[3];
-    int oi[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      od[k] = __shfl_xor_sync(0xffffffffu, best[k], o);
-      oi[k] = __shfl_xor_sync(0xffffffffu, at[k], o);
-    }
-    float md[3];
-    int mi[3], a = 0, c = 0;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float da = a == 0 ? best[0] : a == 1 ? best[1] : best[2], dc = c == 0 ? od[0] : c == 1 ? od[1] : od[2];
-      const int ia = a == 0 ? at[0] : a == 1 ? at[1] : at[2], ic = c == 0 ? oi[0] : c == 1 ? oi[1] : oi[2];
-      const bool mine = da < dc || (da == dc && ia <= ic);
-      md[k] = mine ? da : dc;
-      mi[k] = mine ? ia : ic;
-      a += mine ? 1 : 0;
-      c += mine ? 0 : 1;
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) { best[k] = md[k]; at[k] = mi[k]; }
-  }
-  if (q < n && part == 0) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      dist2[q * 3 + k] = best[k];
-      idx[q * 3 + k] = best[k] == INFINITY ? 0 : at[k];
+      const uint32_t least = __reduce_min_sync(0xffffffffu, __float_as_uint(d0));
+      const bool best = __float_as_uint(d0) == least;
+      const uint32_t at = __reduce_min_sync(0xffffffffu, best ? (uint32_t)i0 : 0xffffffffu);
+      if (lane == 0) {
+        dist2[q * 3 + k] = __uint_as_float(least);
+        idx[q * 3 + k] = least == 0x7f800000u ? 0 : (int32_t)at;
+      }
+      if (best && (uint32_t)i0 == at) { d0 = d1; i0 = i1; d1 = d2; i1 = i2; d2 = INFINITY; i2 = 0; }
     }
   }
 }
@@ -844,8 +829,11 @@ extern "C" int ssc_p2v_fill(const float *points, const int32_t *batch_ids, const
   return SSC_OK;
 }
 
+// [tiles] ranges, [tiles x chunks of a tile] chunk ranges; 16 bytes to align them
+static size_t nn_tiles(int m) { return (size_t)ceil_div(m > 0 ? m : 1, NN_TILE); }
+
 extern "C" size_t ssc_three_nn_scratch_bytes(int m) {
-  return (size_t)ceil_div(m > 0 ? m : 1, NN_TILE) * sizeof(float2);
+  return nn_tiles(m) * ((NN_TILE / NN_CHUNK) * sizeof(float4) + sizeof(float2)) + 16;
 }
 
 extern "C" int ssc_three_nn(int n, int m, const float *unknown, const float *known, float *dist2, int32_t *idx,
@@ -854,12 +842,12 @@ extern "C" int ssc_three_nn(int n, int m, const float *unknown, const float *kno
   if (n == 0) return SSC_OK;
   SSC_REQUIRE(unknown && dist2 && idx && (m == 0 || known), "three_nn: null pointer");
   cudaStream_t st = as_stream(stream);
-  int n_tiles = ceil_div(m > 0 ? m : 1, NN_TILE);
-  if (!scratch || scratch_bytes < (size_t)n_tiles * sizeof(float2))
-    return fail(SSC_ERR_SCRATCH, "three_nn: scratch %zu < %zu bytes", scratch_bytes, (size_t)n_tiles * sizeof(float2));
-  float2 *ranges = (float2 *)scratch;
-  { nn_tile_range_kernel<<<n_tiles, 256, 0, st>>>((const float4 *)known, m, ranges); note_launches(1); }
-  { three_nn_kernel<<<ceil_div(n, 256 / NN_SPLIT), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, ranges, dist2, idx); note_launches(1); }
+  if (!scratch || scratch_bytes < ssc_three_nn_scratch_bytes(m))
+    return fail(SSC_ERR_SCRATCH, "three_nn: scratch %zu < %zu bytes", scratch_bytes, ssc_three_nn_scratch_bytes(m));
+  float4 *chunks = (float4 *)(((uintptr_t)scratch + 15) & ~(uintptr_t)15);
+  float2 *ranges = (float2 *)(chunks + nn_tiles(m) * (NN_TILE / NN_CHUNK));
+  { nn_ranges_kernel<<<(int)nn_tiles(m), 256, 0, st>>>((const float4 *)known, m, ranges, chunks); note_launches(1); }
+  { three_nn_kernel<<<ceil_div(n, 8 * NN_QUERIES), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, ranges, chunks, dist2, idx); note_launches(1); }
   SSC_CHECK_LAUNCH("three_nn");
   return SSC_OK;
 }

@@ -205,6 +205,27 @@ def test_three_nearest_with_ties(cuda, n_query, n_known):
     assert torch.equal(dist, want[:, :3].sqrt()) and torch.equal(idx.long(), order[:, :3])
 
 
+@pytest.mark.parametrize("n_query,known_of", [(5, [0, 1, 2]), (70, [31, 32, 33, 1024]), (40, [1000, 2100, 7]), (33, [1] * 70)])
+@pytest.mark.parametrize("in_order", [True, False])
+def test_three_nearest_passes_over_far_chunks(cuda, n_query, known_of, in_order):
+    """Samples of fewer points than three, around a chunk and a tile of the known points, in grid order and shuffled; queries inside,
+    outside and far from them.  Coordinates are small multiples of 1/4: distances are exact, many equal, and the
+    smallest index comes first among equals; where a sample has too few points the rest is (inf, 0)."""
+    from ss_conv.sp_ops.functional import three_nn
+    rng = np.random.RandomState(n_query)
+    k = np.concatenate([np.concatenate([np.full((n, 1), b), np.sort(rng.randint(-20, 20, (n, 1)), axis=0) / 4, rng.randint(-8, 8, (n, 2)) / 4], 1)
+                        for b, n in enumerate(known_of)]).astype(np.float32)
+    if not in_order:
+        k = k[rng.permutation(len(k))]
+    q = np.concatenate([rng.randint(0, len(known_of), (n_query, 1)), rng.randint(-24, 24, (n_query, 3)) / 4 * rng.choice([1, 1, 8], (n_query, 1))], 1)
+    q, k = dev(q.astype(np.float32), cuda), dev(k, cuda)
+    dist, idx = three_nn(q, k)
+    d = torch.where(q[:, None, 0] == k[None, :, 0], ((q[:, None, 1:] - k[None, :, 1:]) ** 2).sum(-1), torch.full((), float("inf"), device=cuda))
+    want, order = torch.sort(torch.cat([d, torch.full((n_query, 3), float("inf"), device=cuda)], 1), dim=1, stable=True)
+    want, order = want[:, :3], torch.where(want[:, :3].isinf(), 0, order[:, :3])
+    assert torch.equal(dist, want.sqrt()) and torch.equal(idx.long(), order)
+
+
 @pytest.mark.parametrize("c_in,c_out,c_keep,n,precision,stored", [
     (17, 11, 9, 1, "tf32", None), (32, 38, 32, 127, "tf32", None), (64, 76, 64, 129, "tf32", "bf16"),
     (40, 256, 208, 300, "tf32", "fp16"), (24, 16, 16, 200, "tf32", None), (200, 152, 128, 257, "tf32", None),
