@@ -358,8 +358,11 @@ static void launch_decode(const uint32_t *bitmap, const uint32_t *word_prefix, l
 // The last block posts the count to the host (post): who needs it waits for this kernel, not for the convolution behind
 // it (a layer of 3 k rows 92 -> 69 us per call, an encoder and decoder pair of 90 k rows 301 -> 240).
 constexpr int kRankedWords = 1 << 15;
+// 512 threads: twice the words of the count before them in flight, half the words to decode one after the other (32 k words
+// 11.5 -> 9.3 us, 8 k words 6.6 -> 6.1).
+constexpr int kRankThreads = 512;
 template <int WORDS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kRankThreads)
 rank_decode_kernel(const uint32_t *__restrict__ bitmap, int n_words, Geometry g, int n_out, int4 *__restrict__ out_indices,
                    int32_t *__restrict__ total_dev, const int32_t *__restrict__ status, CountPost post) {
   __shared__ uint32_t smem[33], word_s[WORDS], prefix_s[WORDS];
@@ -367,7 +370,7 @@ rank_decode_kernel(const uint32_t *__restrict__ bitmap, int n_words, Geometry g,
   uint32_t before = 0;
   const uint4 *quads = (const uint4 *)bitmap;                 // (256-byte aligned; w0 is a multiple of four)
 #pragma unroll 8
-  for (int q = threadIdx.x; q < w0 / 4; q += 256) {
+  for (int q = threadIdx.x; q < w0 / 4; q += kRankThreads) {
     const uint4 v = __ldg(quads + q);
     before += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
   }
@@ -386,7 +389,7 @@ rank_decode_kernel(const uint32_t *__restrict__ bitmap, int n_words, Geometry g,
   }
   const int yz = g.out_shape[1] * g.out_shape[2], vol = g.out_shape[0] * yz, bit = threadIdx.x & 31;
 #pragma unroll 4
-  for (int w = threadIdx.x >> 5; w < WORDS; w += 8) {
+  for (int w = threadIdx.x >> 5; w < WORDS; w += kRankThreads / 32) {
     const uint32_t bits = word_s[w];
     if (!((bits >> bit) & 1u)) continue;
     const uint32_t rank = prefix_s[w] + (uint32_t)__popc(bits & ((1u << bit) - 1u));
@@ -888,8 +891,8 @@ static int rulebook_conv_ahead(const int32_t *indices, int n_in, int batch, cons
   const CountPost post = next_post(place);
   if (s.n_words <= kRankedWords) {
     const int n = (int)s.n_words;
-    if (n <= 8192) rank_decode_kernel<32><<<ceil_div(n, 32), 256, 0, st>>>(s.bitmap, n, g, n_out, (int4 *)out_indices, n_out_dev, status, post);
-    else rank_decode_kernel<128><<<ceil_div(n, 128), 256, 0, st>>>(s.bitmap, n, g, n_out, (int4 *)out_indices, n_out_dev, status, post);
+    if (n <= 8192) rank_decode_kernel<32><<<ceil_div(n, 32), kRankThreads, 0, st>>>(s.bitmap, n, g, n_out, (int4 *)out_indices, n_out_dev, status, post);
+    else rank_decode_kernel<128><<<ceil_div(n, 128), kRankThreads, 0, st>>>(s.bitmap, n, g, n_out, (int4 *)out_indices, n_out_dev, status, post);
     note_launches(1);
     SSC_CHECK_LAUNCH("rank_decode");
   } else {
