@@ -95,6 +95,34 @@ CountPost next_post(void *place);
 void launch_post(const CountPost &post, const int32_t *n_dev, const int32_t *status, cudaStream_t st);
 
 #ifdef __CUDACC__
+// Two floats in a register pair; operations on both halves at once, each correctly rounded.
+typedef unsigned long long f32x2;
+static __device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+static __device__ __forceinline__ float2 halves(f32x2 v) {
+  float2 h;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(h.x), "=f"(h.y) : "l"(v));
+  return h;
+}
+static __device__ __forceinline__ f32x2 fma_pair(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+static __device__ __forceinline__ f32x2 mul_pair(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+static __device__ __forceinline__ f32x2 add_pair(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // (one thread) a bounded wait ran out and the output is incomplete: status bit 16, then the alarm, which the host sees
 // without reading anything back.
 static __device__ __forceinline__ void report_expired(int32_t *status, int32_t *alarm) {

@@ -163,24 +163,6 @@ conv_fwd_fp32_kernel(const float *__restrict__ features, int c_in, const float *
   }
 }
 
-// Two floats in a register pair, and a * b + c of both halves, each correctly rounded (fmaf of each).
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
-  f32x2 v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-  return v;
-}
-__device__ __forceinline__ float2 halves(f32x2 v) {
-  float2 h;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(h.x), "=f"(h.y) : "l"(v));
-  return h;
-}
-__device__ __forceinline__ f32x2 fma_pair(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
 // The same sums for up to four input channels (a first layer on point features), in the same order: per output
 // element fused multiply-adds over ascending offsets and channels, present neighbours only.
 // A lane has an output row and CB of its channels, two to a register pair; the filters stand in shared memory, where all

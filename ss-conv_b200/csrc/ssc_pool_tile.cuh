@@ -130,11 +130,15 @@ static __device__ __forceinline__ void add_quotients(Channels &acc, const Channe
     fast = fast && (a == 0.f || (a > 8.0779357e-28f && a < 1.2676506e30f));      // 2^-90, 2^100
   }
   if (fast) {
+    const f32x2 rr = pair_of(r, r), dd = pair_of(-d, -d);        // (two channels per instruction: 138 k rows of 27 offsets 42.5 -> 40.6 us)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float y = x.v[q] * r;
-      y = fmaf(fmaf(-d, y, x.v[q]), r, y);
-      acc.v[q] += fmaf(fmaf(-d, y, x.v[q]), r, y);
+    for (int q = 0; q < 4; q += 2) {
+      const f32x2 xx = pair_of(x.v[q], x.v[q + 1]);
+      f32x2 y = mul_pair(xx, rr);
+      y = fma_pair(fma_pair(dd, y, xx), rr, y);
+      const float2 sum = halves(add_pair(pair_of(acc.v[q], acc.v[q + 1]), fma_pair(fma_pair(dd, y, xx), rr, y)));
+      acc.v[q] = sum.x;
+      acc.v[q + 1] = sum.y;
     }
   } else {
 #pragma unroll
