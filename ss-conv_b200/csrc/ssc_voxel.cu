@@ -342,7 +342,7 @@ nn_ranges_kernel(const float4 *__restrict__ known, int m, float2 *__restrict__ r
       r.w = fmaxf(r.w, __shfl_xor_sync(0xffffffffu, r.w, o));
     }
     if (lane == 0) {
-      chunks[blockIdx.x * (NN_TILE / NN_CHUNK) + c] = r;
+      if (chunks != nullptr) chunks[blockIdx.x * (NN_TILE / NN_CHUNK) + c] = r;
       lo_s[c] = r.x;
       hi_s[c] = r.y;
     }
@@ -409,7 +409,8 @@ three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *
       const float2 r = t0 + lane < n_tiles ? __ldg(ranges + t0 + lane) : make_float2(INFINITY, -INFINITY);
       for (unsigned tiles = __ballot_sync(0xffffffffu, r.x <= u.x && u.x <= r.y); tiles != 0u; tiles &= tiles - 1u) {
         const int c0 = (t0 + __ffs((int)tiles) - 1) * (NN_TILE / NN_CHUNK);
-        const float4 c = c0 + lane < n_chunks ? __ldg(chunks + c0 + lane) : make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
+        float4 c = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
+        if (c0 + lane < n_chunks) c = chunks != nullptr ? __ldg(chunks + c0 + lane) : make_float4(-INFINITY, INFINITY, -INFINITY, INFINITY);
         const bool may = c.x <= u.x && u.x <= c.y;
         const float off = fmaxf(0.f, fmaxf(__fsub_rn(c.z, u.y), __fsub_rn(u.y, c.w)));
         const float least = may ? __fmul_rn(off, off) : INFINITY;     // no point of the chunk is nearer
@@ -842,10 +843,15 @@ extern "C" int ssc_three_nn(int n, int m, const float *unknown, const float *kno
   if (n == 0) return SSC_OK;
   SSC_REQUIRE(unknown && dist2 && idx && (m == 0 || known), "three_nn: null pointer");
   cudaStream_t st = as_stream(stream);
-  if (!scratch || scratch_bytes < ssc_three_nn_scratch_bytes(m))
-    return fail(SSC_ERR_SCRATCH, "three_nn: scratch %zu < %zu bytes", scratch_bytes, ssc_three_nn_scratch_bytes(m));
-  float4 *chunks = (float4 *)(((uintptr_t)scratch + 15) & ~(uintptr_t)15);
-  float2 *ranges = (float2 *)(chunks + nn_tiles(m) * (NN_TILE / NN_CHUNK));
+  // a buffer for the tiles' ranges alone will do: every chunk of a tile is looked at then
+  if (!scratch || scratch_bytes < nn_tiles(m) * sizeof(float2))
+    return fail(SSC_ERR_SCRATCH, "three_nn: scratch %zu < %zu bytes", scratch_bytes, nn_tiles(m) * sizeof(float2));
+  float4 *chunks = nullptr;
+  float2 *ranges = (float2 *)scratch;
+  if (scratch_bytes >= ssc_three_nn_scratch_bytes(m)) {
+    chunks = (float4 *)(((uintptr_t)scratch + 15) & ~(uintptr_t)15);
+    ranges = (float2 *)(chunks + nn_tiles(m) * (NN_TILE / NN_CHUNK));
+  }
   { nn_ranges_kernel<<<(int)nn_tiles(m), 256, 0, st>>>((const float4 *)known, m, ranges, chunks); note_launches(1); }
   { three_nn_kernel<<<ceil_div(n, 8 * NN_QUERIES), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, ranges, chunks, dist2, idx); note_launches(1); }
   SSC_CHECK_LAUNCH("three_nn");

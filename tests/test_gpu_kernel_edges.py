@@ -224,6 +224,11 @@ def test_three_nearest_passes_over_far_chunks(cuda, n_query, known_of, in_order)
     want, order = torch.sort(torch.cat([d, torch.full((n_query, 3), float("inf"), device=cuda)], 1), dim=1, stable=True)
     want, order = want[:, :3], torch.where(want[:, :3].isinf(), 0, order[:, :3])
     assert torch.equal(dist, want.sqrt()) and torch.equal(idx.long(), order)
+    # a buffer for the tiles' ranges alone
+    from ss_conv._ext import lib, _check, _p, _stream
+    small, d2, at = torch.empty(8 * -(-len(k) // 1024), dtype=torch.uint8, device=cuda), torch.empty_like(dist), torch.empty_like(idx)
+    _check(lib().ssc_three_nn(n_query, len(k), _p(q), _p(k), _p(d2), _p(at), _p(small), small.numel(), _stream()))
+    assert torch.equal(d2.sqrt(), dist) and torch.equal(at, idx)
 
 
 @pytest.mark.parametrize("c_in,c_out,c_keep,n,precision,stored", [
