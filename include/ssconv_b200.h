@@ -502,9 +502,9 @@ int ssc_p2v_fill(const float *points, const int32_t *batch_ids, const float *fea
  * (SS_Conv_lib/src/voxelize/interpolate_cuda_kernel.cu:8-55, 79-101): unknown [N,4] and
  * known [M,4] are (batch,x,y,z) float rows; dist2 [N,3] squared distances, idx [N,3].
  * Same neighbours and tie order as the reference's exhaustive scan.  scratch (device,
- * ssc_three_nn_scratch_bytes(m) bytes) holds the batch-id ranges of the 1024-row tiles and
- * of the 32-row chunks of `known`, the chunks' ranges of x too, which let a query pass over what cannot be near;
- * 8 bytes per tile, for the batch-id ranges alone, are accepted too. */
+ * ssc_three_nn_scratch_bytes(m) bytes) holds the ranges of batch ids and x of the 1024-row tiles and
+ * the 32-row chunks of `known`, which let a query pass over what cannot be near, and how much that would be;
+ * smaller buffers from 8 bytes per tile, for the batch-id ranges alone, are accepted too. */
 size_t ssc_three_nn_scratch_bytes(int m);
 int ssc_three_nn(int n, int m, const float *unknown, const float *known, float *dist2,
                  int32_t *idx, void *scratch, size_t scratch_bytes, void *stream);

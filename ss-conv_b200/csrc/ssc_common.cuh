@@ -83,6 +83,9 @@ inline uint32_t hash_buckets_for(int n) {
 int bitmap_decode(const uint32_t *bitmap, const uint32_t *word_prefix, long long n_words, const int shape[3],
                   int n_out, int32_t *out_indices, cudaStream_t st);
 
+// SMs of the current device (ssc_conv_stage.cu).
+int sm_count();
+
 // The process's alarm (ssc_alarm_open), null while nobody has opened it.
 int32_t *alarm_word();
 

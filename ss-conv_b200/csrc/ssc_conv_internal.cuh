@@ -4,8 +4,6 @@
 
 namespace ssc {
 
-int sm_count();
-
 // staged operand images (ssc_conv_stage.cu)
 size_t conv_tf32_scratch_bytes(int n_in, int c_in);
 size_t conv_f16_scratch_bytes(int n_in, int c_in);

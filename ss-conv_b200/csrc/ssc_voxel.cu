@@ -323,68 +323,201 @@ static void fill_grid(VoxelGrid &g, const int grid[3], const float unit[3]) {
 // chunk; points in grid order, as the voxelizer and the rulebook give them, have a slab of few x).
 constexpr int NN_CHUNK = 32, NN_TILE = 32 * NN_CHUNK;
 
-__global__ void __launch_bounds__(256)
-nn_ranges_kernel(const float4 *__restrict__ known, int m, float2 *__restrict__ ranges, float4 *__restrict__ chunks) {
-  __shared__ float lo_s[NN_TILE / NN_CHUNK], hi_s[NN_TILE / NN_CHUNK];
-  const int lane = threadIdx.x & 31;
-  for (int c = threadIdx.x >> 5; c < NN_TILE / NN_CHUNK; c += 8) {
-    const int k = blockIdx.x * NN_TILE + c * NN_CHUNK + lane;
-    float4 r = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
-    if (k < m) {
-      const float4 p = known[k];
-      // (fminf and fmaxf pass over a coordinate that is not a number: such a point is nobody's neighbour)
-      r = make_float4(fminf(INFINITY, p.x), fmaxf(-INFINITY, p.x), fminf(INFINITY, p.y), fmaxf(-INFINITY, p.y));
-    }
+// A tile's ranges of batch ids and x.  shares: how many of its chunks, of 1024, a point of it lies in by their ranges of
+// batch ids and x, on average of 32 points: a few tens in grid order, 1024 where nothing can be passed over.
+constexpr int NN_SHARES = 1024;
+
+__global__ void __launch_bounds__(NN_TILE)
+nn_ranges_kernel(const float4 *__restrict__ known, int m, float2 *__restrict__ ranges, float4 *__restrict__ chunks, float4 *__restrict__ tiles,
+                 int32_t *__restrict__ shares) {
+  __shared__ float4 chunk_s[32];
+  __shared__ int in_s[32];
+  const int lane = threadIdx.x & 31, c = threadIdx.x >> 5, k = blockIdx.x * NN_TILE + (int)threadIdx.x;
+  const float4 p = k < m ? __ldg(known + k) : make_float4(NAN, NAN, NAN, NAN);
+  auto widen = [](float4 r) {
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       r.x = fminf(r.x, __shfl_xor_sync(0xffffffffu, r.x, o));
       r.y = fmaxf(r.y, __shfl_xor_sync(0xffffffffu, r.y, o));
       r.z = fminf(r.z, __shfl_xor_sync(0xffffffffu, r.z, o));
       r.w = fmaxf(r.w, __shfl_xor_sync(0xffffffffu, r.w, o));
     }
-    if (lane == 0) {
-      if (chunks != nullptr) chunks[blockIdx.x * (NN_TILE / NN_CHUNK) + c] = r;
-      lo_s[c] = r.x;
-      hi_s[c] = r.y;
-    }
+    return r;
+  };
+  // (fminf and fmaxf pass over a coordinate that is not a number: such a point is nobody's neighbour)
+  const float4 r = widen(make_float4(fminf(INFINITY, p.x), fmaxf(-INFINITY, p.x), fminf(INFINITY, p.y), fmaxf(-INFINITY, p.y)));
+  if (lane == 0) {
+    chunk_s[c] = r;
+    if (chunks != nullptr) chunks[blockIdx.x * (NN_TILE / NN_CHUNK) + c] = r;
   }
   __syncthreads();
-  if (threadIdx.x < 32) {
-    float lo = lo_s[lane], hi = hi_s[lane];
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  const float4 other = chunk_s[lane];
+  const int middle = min(max(m - (k - lane), 1), NN_CHUNK) / 2;           // of the chunk's points
+  const float sample = __shfl_sync(0xffffffffu, p.x, middle), x = __shfl_sync(0xffffffffu, p.y, middle);
+  const unsigned in = __ballot_sync(0xffffffffu, other.x <= sample && sample <= other.y && other.z <= x && x <= other.w);
+  if (lane == 0) in_s[c] = __popc(in);
+  __syncthreads();
+  if (c == 0) {
+    const int all = __reduce_add_sync(0xffffffffu, in_s[lane]), have = min((m - (int)blockIdx.x * NN_TILE + NN_CHUNK - 1) / NN_CHUNK, 32);
+    const float4 t = widen(other);
+    if (lane == 0) {
+      ranges[blockIdx.x] = make_float2(t.x, t.y);
+      if (chunks != nullptr) {
+        tiles[blockIdx.x] = t;
+        shares[blockIdx.x] = have > 0 ? NN_SHARES * all / (have * have) : 0;
+      }
     }
-    if (lane == 0) ranges[blockIdx.x] = make_float2(lo, hi);
   }
 }
 
-// A warp per query.  Its lanes look at the ranges of 32 tiles at a time, then at the 32 chunks of a tile that can hold points of
-// the query's sample: first at the points of the chunks nearest in x, then of those whose distance in x alone does not
-// exceed the third best so far.  That distance, rounded like the points' own, is never more than theirs: every rounding
-// involved is monotonic.  Each lane keeps its three best by (distance, index); the three best of the warp by that order are
-// the result of the exhaustive reference loop (ascending index, strict <).
-// 65 k queries among 1000 points each: 80 us (a chain of trips to L1 and votes per query); 132 with four
-// threads per query that looked at every point of the sample.
+// The contraction nvcc applies to the reference's dx*dx + dy*dy + dz*dz
+// (interpolate_cuda_kernel.cu:39), checked bit for bit against the reference's own kernel.
+__device__ __forceinline__ float nn_dist2(const float4 &u, const float4 &k) {
+  const float dx = __fsub_rn(u.y, k.y), dy = __fsub_rn(u.z, k.z), dz = __fsub_rn(u.w, k.w);
+  return __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+}
+
+// Where most points have to be looked at: SPLIT threads per query; known points stream through shared memory in
+// tiles of 1024, tiles whose batch-id range cannot match any query of the block are skipped.  Thread s of a query
+// looks at every SPLIT-th point of a tile; the three best of them are merged by (distance, index), which is
+// the result of the exhaustive reference loop (ascending k, strict <): the smallest index wins ties.
+template <int SPLIT>
+__device__ __forceinline__ void nn_by_tiles(int first, int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known,
+                                            const float2 *__restrict__ ranges, float *__restrict__ dist2, int32_t *__restrict__ idx) {
+  __shared__ float4 tile[NN_TILE];
+  __shared__ float qmin_s[8], qmax_s[8];
+  const int q = first + (int)threadIdx.x / SPLIT, part = threadIdx.x % SPLIT;
+  float4 u = q < n ? unknown[q] : make_float4(NAN, 0.f, 0.f, 0.f);
+  float lo = q < n ? u.x : INFINITY, hi = q < n ? u.x : -INFINITY;
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fminf(lo, __shfl_down_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_down_sync(0xffffffffu, hi, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    qmin_s[threadIdx.x >> 5] = lo;
+    qmax_s[threadIdx.x >> 5] = hi;
+  }
+  __syncthreads();
+  float qmin = qmin_s[0], qmax = qmax_s[0];
+  for (int w = 1; w < 8; ++w) {
+    qmin = fminf(qmin, qmin_s[w]);
+    qmax = fmaxf(qmax, qmax_s[w]);
+  }
+  float best[3] = {INFINITY, INFINITY, INFINITY};
+  int at[3] = {0, 0, 0};
+  // (d, i) into the ordered triple; equal distances stay behind
+  auto take = [&](float d, int i) {
+    if (d < best[0]) {
+      best[2] = best[1]; at[2] = at[1];
+      best[1] = best[0]; at[1] = at[0];
+      best[0] = d; at[0] = i;
+    } else if (d < best[1]) {
+      best[2] = best[1]; at[2] = at[1];
+      best[1] = d; at[1] = i;
+    } else if (d < best[2]) {
+      best[2] = d; at[2] = i;
+    }
+  };
+  const int n_tiles = (m + NN_TILE - 1) / NN_TILE;
+  for (int t = 0; t < n_tiles; ++t) {
+    const float2 r = ranges[t];
+    if (r.y < qmin || r.x > qmax) continue;  // block-uniform
+    __syncthreads();
+    const int base = t * NN_TILE;
+    for (int i = threadIdx.x; i < NN_TILE; i += 256) tile[i] = base + i < m ? known[base + i] : make_float4(NAN, 0.f, 0.f, 0.f);
+    __syncthreads();
+    const int cnt = min(NN_TILE, m - base);
+    if (q < n && !(r.y < u.x || r.x > u.x)) {
+#pragma unroll 4
+      for (int i = part; i < cnt; i += SPLIT) {
+        const float4 k = tile[i];
+        const float d = nn_dist2(u, k);
+        if (k.x == u.x && d < best[2]) take(d, base + i);
+      }
+    }
+  }
+  // merge the partners' triples (a slot that was never filled is infinite and loses to everything)
+#pragma unroll
+  for (int o = 1; o < SPLIT; o <<= 1) {
+    float od[3];
+    int oi[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      od[k] = __shfl_xor_sync(0xffffffffu, best[k], o);
+      oi[k] = __shfl_xor_sync(0xffffffffu, at[k], o);
+    }
+    float md[3];
+    int mi[3], a = 0, c = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float da = a == 0 ? best[0] : a == 1 ? best[1] : best[2], dc = c == 0 ? od[0] : c == 1 ? od[1] : od[2];
+      const int ia = a == 0 ? at[0] : a == 1 ? at[1] : at[2], ic = c == 0 ? oi[0] : c == 1 ? oi[1] : oi[2];
+      const bool mine = da < dc || (da == dc && ia <= ic);
+      md[k] = mine ? da : dc;
+      mi[k] = mine ? ia : ic;
+      a += mine ? 1 : 0;
+      c += mine ? 0 : 1;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { best[k] = md[k]; at[k] = mi[k]; }
+  }
+  if (q < n && part == 0) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      dist2[q * 3 + k] = best[k];
+      idx[q * 3 + k] = best[k] == INFINITY ? 0 : at[k];
+    }
+  }
+}
+
+// Where ranges of x are narrow: a warp per query.  Its lanes look at the ranges of 32 tiles at a time, then at the 32 chunks of a
+// tile that can hold points of the query's sample: first at the points of the chunks nearest in x, then of those whose distance in
+// x alone does not exceed the third best so far.  That distance, rounded like the points' own, is never more than theirs:
+// every rounding involved is monotonic.  Of several tiles the nearest in x comes first: in order, each of those before it
+// would hold the best so far and be looked at whole (4096 queries among 40 k points in order: 1170 us, 586 by tiles, 102 like this).
+// Each lane keeps its three best by (distance, index); the three best of the warp by that order are the result of the
+// exhaustive reference loop.
+
+// The tiles that can hold points of a sample: all within [first, end), multiples of 32.  share: how many of 1024 of their
+// chunks a point of the first of them lies in.
+struct NnSpan {
+  float sample;
+  int first, end, share;
+};
+__device__ __forceinline__ NnSpan nn_span(float sample, int n_tiles, const float4 *__restrict__ tiles, const int32_t *__restrict__ shares) {
+  const int lane = threadIdx.x & 31;
+  NnSpan s = {sample, 0, 0, 0};
+  for (int t0 = 0; t0 < n_tiles; t0 += 32) {
+    const bool there = t0 + lane < n_tiles;
+    const float4 r = there ? __ldg(tiles + t0 + lane) : make_float4(INFINITY, -INFINITY, 0.f, 0.f);
+    const int share = there ? __ldg(shares + t0 + lane) : 0;
+    const bool mine = r.x <= sample && sample <= r.y;
+    const int have = __popc(__ballot_sync(0xffffffffu, mine));
+    if (have == 0) continue;
+    if (s.end == 0) {
+      s.first = t0;
+      s.share = __reduce_add_sync(0xffffffffu, mine ? share : 0) / have;
+    }
+    s.end = t0 + 32;
+  }
+  return s;
+}
+
 constexpr int NN_QUERIES = 4;                     // of a warp, one after the other
-__global__ void __launch_bounds__(256)
-three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known,
-                const float2 *__restrict__ ranges, const float4 *__restrict__ chunks, float *__restrict__ dist2, int32_t *__restrict__ idx) {
+__device__ __forceinline__ void nn_by_warps(int q0, float4 next, NnSpan span, int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known,
+                                            const float4 *__restrict__ chunks, const float4 *__restrict__ tiles, const int32_t *__restrict__ shares,
+                                            float *__restrict__ dist2, int32_t *__restrict__ idx) {
   const int lane = threadIdx.x & 31, n_tiles = (m + NN_TILE - 1) / NN_TILE, n_chunks = (m + NN_CHUNK - 1) / NN_CHUNK;
-  const int q0 = ((int)blockIdx.x * 8 + ((int)threadIdx.x >> 5)) * NN_QUERIES;
   for (int q = q0; q < min(q0 + NN_QUERIES, n); ++q) {
-    const float4 u = __ldg(unknown + q);
-    float d0 = INFINITY, d1 = INFINITY, d2 = INFINITY;
+    const float4 u = next;
+    next = __ldg(unknown + min(q + 1, n - 1));    // (on its way while this one is looked for)
+    if (u.x != span.sample) span = nn_span(u.x, n_tiles, tiles, shares);
+    float d0 = INFINITY, d1 = INFINITY, d2 = INFINITY, limit = INFINITY;       // limit: no less than the warp's third best
     int i0 = 0, i1 = 0, i2 = 0;
     auto before = [](float d, int i, float e, int j) { return d < e || (d == e && i < j); };
-    auto look_at = [&](int chunk) {
-      const int i = chunk * NN_CHUNK + lane;
-      if (i >= m) return;
-      const float4 k = __ldg(known + i);
-      const float dx = __fsub_rn(u.y, k.y), dy = __fsub_rn(u.z, k.z), dz = __fsub_rn(u.w, k.w);
-      // the contraction nvcc applies to the reference's dx*dx + dy*dy + dz*dz
-      // (interpolate_cuda_kernel.cu:39), checked bit for bit against the reference's own kernel
-      const float d = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
-      if (k.x == u.x && d < INFINITY && before(d, i, d2, i2)) {
+    auto take = [&](const float4 &k, int i) {
+      const float d = nn_dist2(u, k);
+      if (k.x == u.x && d <= limit && d < INFINITY && before(d, i, d2, i2)) {
         if (before(d, i, d1, i1)) {
           d2 = d1; i2 = i1;
           if (before(d, i, d0, i0)) { d1 = d0; i1 = i0; d0 = d; i0 = i; }
@@ -394,31 +527,76 @@ three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *
         }
       }
     };
+    const float4 none = make_float4(NAN, 0.f, 0.f, 0.f);
+    auto look_at = [&](int c0, unsigned left) {
+      for (; (left & (left - 1u)) != 0u;) {
+        const int a = (c0 + __ffs((int)left) - 1) * NN_CHUNK + lane;
+        left &= left - 1u;
+        const int b = (c0 + __ffs((int)left) - 1) * NN_CHUNK + lane;
+        left &= left - 1u;
+        const float4 ka = a < m ? __ldg(known + a) : none, kb = b < m ? __ldg(known + b) : none;
+        take(ka, a);
+        take(kb, b);
+      }
+      if (left != 0u) {
+        const int a = (c0 + __ffs((int)left) - 1) * NN_CHUNK + lane;
+        take(a < m ? __ldg(known + a) : none, a);
+      }
+    };
     // (distances are not negative: their order is that of their bits)
     auto third_best = [&]() {
       uint32_t a = __float_as_uint(d0), b = __float_as_uint(d1), c = __float_as_uint(d2), least = 0u;
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
         least = __reduce_min_sync(0xffffffffu, a);
-        const int first = __ffs((int)__ballot_sync(0xffffffffu, a == least)) - 1;
-        if (lane == first) { a = b; b = c; c = 0x7f800000u; }
+        const int holder = __ffs((int)__ballot_sync(0xffffffffu, a == least)) - 1;
+        if (lane == holder) { a = b; b = c; c = 0x7f800000u; }
       }
       return __uint_as_float(least);
     };
-    for (int t0 = 0; t0 < n_tiles; t0 += 32) {
-      const float2 r = t0 + lane < n_tiles ? __ldg(ranges + t0 + lane) : make_float2(INFINITY, -INFINITY);
-      for (unsigned tiles = __ballot_sync(0xffffffffu, r.x <= u.x && u.x <= r.y); tiles != 0u; tiles &= tiles - 1u) {
-        const int c0 = (t0 + __ffs((int)tiles) - 1) * (NN_TILE / NN_CHUNK);
-        float4 c = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
-        if (c0 + lane < n_chunks) c = chunks != nullptr ? __ldg(chunks + c0 + lane) : make_float4(-INFINITY, INFINITY, -INFINITY, INFINITY);
-        const bool may = c.x <= u.x && u.x <= c.y;
-        const float off = fmaxf(0.f, fmaxf(__fsub_rn(c.z, u.y), __fsub_rn(u.y, c.w)));
-        const float least = may ? __fmul_rn(off, off) : INFINITY;     // no point of the chunk is nearer
-        const uint32_t nearest = __reduce_min_sync(0xffffffffu, __float_as_uint(least));
-        const bool near = may && __float_as_uint(least) == nearest;
-        for (unsigned left = __ballot_sync(0xffffffffu, near); left != 0u; left &= left - 1u) look_at(c0 + __ffs((int)left) - 1);
-        const float limit = third_best();
-        for (unsigned left = __ballot_sync(0xffffffffu, may && !near && least <= limit); left != 0u; left &= left - 1u) look_at(c0 + __ffs((int)left) - 1);
+    // the square of the distance in x to the nearest point with lo <= x <= hi
+    auto least_of = [&](float lo, float hi) {
+      const float off = fmaxf(0.f, fmaxf(__fsub_rn(lo, u.y), __fsub_rn(u.y, hi)));
+      return __fmul_rn(off, off);
+    };
+    bool stale = false;                           // points were taken since `limit` was found
+    auto look_in = [&](int tile) {
+      const int c0 = tile * (NN_TILE / NN_CHUNK);
+      const float4 c = c0 + lane < n_chunks ? __ldg(chunks + c0 + lane) : make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
+      const bool may = c.x <= u.x && u.x <= c.y;
+      const float least = may ? least_of(c.z, c.w) : INFINITY;
+      const uint32_t nearest = __reduce_min_sync(0xffffffffu, __float_as_uint(least));
+      const bool near = may && __float_as_uint(least) == nearest;
+      look_at(c0, __ballot_sync(0xffffffffu, near));
+      limit = third_best();
+      const unsigned rest = __ballot_sync(0xffffffffu, may && !near && least <= limit);
+      look_at(c0, rest);
+      stale = rest != 0u;
+    };
+    int home = -1, n_mine = 0;
+    float nearest = INFINITY;
+    for (int t0 = span.first; t0 < span.end; t0 += 32) {
+      const float4 r = t0 + lane < n_tiles ? __ldg(tiles + t0 + lane) : make_float4(INFINITY, -INFINITY, 0.f, 0.f);
+      const bool mine = r.x <= u.x && u.x <= r.y;
+      const unsigned have = __ballot_sync(0xffffffffu, mine);
+      if (have == 0u) continue;
+      n_mine += __popc(have);
+      const float least = mine ? least_of(r.z, r.w) : INFINITY;
+      const float here = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(least)));
+      if (home >= 0 && !(here < nearest)) continue;
+      nearest = here;
+      home = t0 + __ffs((int)__ballot_sync(0xffffffffu, mine && least == here)) - 1;
+    }
+    if (home >= 0) look_in(home);
+    for (int t0 = span.first; n_mine > 1 && t0 < span.end; t0 += 32) {
+      const float4 r = t0 + lane < n_tiles ? __ldg(tiles + t0 + lane) : make_float4(INFINITY, -INFINITY, 0.f, 0.f);
+      const bool mine = r.x <= u.x && u.x <= r.y && t0 + lane != home;
+      const float least = mine ? least_of(r.z, r.w) : INFINITY;
+      for (unsigned left = __ballot_sync(0xffffffffu, mine && least <= limit); left != 0u; left &= left - 1u) {
+        const int t = __ffs((int)left) - 1;
+        if (stale) limit = third_best();
+        stale = false;
+        if (__shfl_sync(0xffffffffu, least, t) <= limit) look_in(t0 + t);
       }
     }
 #pragma unroll
@@ -433,6 +611,48 @@ three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *
       if (best && (uint32_t)i0 == at) { d0 = d1; i0 = i1; d1 = d2; i1 = i2; d2 = INFINITY; i2 = 0; }
     }
   }
+}
+
+// A group's queries all go the way that suits the first one's sample: by warps where a point of its tiles lies in up to three eighths of
+// their chunks, by tiles where more of them would have to be looked at anyhow, at twice the instructions per point.  (64 samples of
+// 4096 queries and 1024 points, us: in grid order 147 by warps, 269 by tiles; in any order 484 and 251.  By warps at a half already:
+// 24 samples of 1000 each in any order 78, like this 55.)
+constexpr int NN_MOST = 3 * NN_SHARES / 8;
+// Up to 256 points are no matter of chunks (100 k queries among 20: 10.7 us by tiles at once, 15.4 with ranges and a second kernel).
+constexpr int NN_FEW = 8 * NN_CHUNK;
+template <int GROUP>
+__device__ __forceinline__ NnSpan nn_group(int first, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ tiles, const int32_t *__restrict__ shares) {
+  return nn_span(__ldg(&unknown[first / GROUP * GROUP].x), (m + NN_TILE - 1) / NN_TILE, tiles, shares);
+}
+
+// Few queries: 32 to a block, whichever way they go.
+__global__ void __launch_bounds__(256)
+three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known, const float2 *__restrict__ ranges,
+                const float4 *__restrict__ chunks, const float4 *__restrict__ tiles, const int32_t *__restrict__ shares, float *__restrict__ dist2,
+                int32_t *__restrict__ idx) {
+  const int first = (int)blockIdx.x * 32, q0 = first + ((int)threadIdx.x >> 5) * NN_QUERIES;
+  const float4 own = __ldg(unknown + min(q0, n - 1));
+  NnSpan span = {0.f, 0, 0, NN_SHARES};
+  if (chunks != nullptr) span = nn_group<32>(first, m, unknown, tiles, shares);
+  if (span.share <= NN_MOST) nn_by_warps(q0, own, span, n, m, unknown, known, chunks, tiles, shares, dist2, idx);
+  else nn_by_tiles<8>(first, n, m, unknown, known, ranges, dist2, idx);
+}
+
+// Many: each way has its own kernel, which passes over the other's groups of 64.
+__global__ void __launch_bounds__(256)
+three_nn_warps_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known, const float4 *__restrict__ chunks,
+                      const float4 *__restrict__ tiles, const int32_t *__restrict__ shares, float *__restrict__ dist2, int32_t *__restrict__ idx) {
+  const int first = (int)blockIdx.x * 32, q0 = first + ((int)threadIdx.x >> 5) * NN_QUERIES;
+  const float4 own = __ldg(unknown + min(q0, n - 1));
+  const NnSpan span = nn_group<64>(first, m, unknown, tiles, shares);
+  if (span.share <= NN_MOST) nn_by_warps(q0, own, span, n, m, unknown, known, chunks, tiles, shares, dist2, idx);
+}
+__global__ void __launch_bounds__(256)
+three_nn_tiles_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known, const float2 *__restrict__ ranges,
+                      const float4 *__restrict__ tiles, const int32_t *__restrict__ shares, float *__restrict__ dist2, int32_t *__restrict__ idx) {
+  const int first = (int)blockIdx.x * 64;
+  if (tiles != nullptr && nn_group<64>(first, m, unknown, tiles, shares).share <= NN_MOST) return;
+  nn_by_tiles<4>(first, n, m, unknown, known, ranges, dist2, idx);
 }
 
 // Rows (batch id, x, y, z) as three_nn takes them, and the interpolation weights from its squared distances:
@@ -830,11 +1050,11 @@ extern "C" int ssc_p2v_fill(const float *points, const int32_t *batch_ids, const
   return SSC_OK;
 }
 
-// [tiles] ranges, [tiles x chunks of a tile] chunk ranges; 16 bytes to align them
+// [tiles x chunks of a tile] chunk ranges, [tiles] ranges of batch ids and x, [tiles] of batch ids, [tiles] shares; 16 bytes to align them
 static size_t nn_tiles(int m) { return (size_t)ceil_div(m > 0 ? m : 1, NN_TILE); }
 
 extern "C" size_t ssc_three_nn_scratch_bytes(int m) {
-  return nn_tiles(m) * ((NN_TILE / NN_CHUNK) * sizeof(float4) + sizeof(float2)) + 16;
+  return nn_tiles(m) * ((NN_TILE / NN_CHUNK + 1) * sizeof(float4) + sizeof(float2) + sizeof(int32_t)) + 16;
 }
 
 extern "C" int ssc_three_nn(int n, int m, const float *unknown, const float *known, float *dist2, int32_t *idx,
@@ -843,17 +1063,28 @@ extern "C" int ssc_three_nn(int n, int m, const float *unknown, const float *kno
   if (n == 0) return SSC_OK;
   SSC_REQUIRE(unknown && dist2 && idx && (m == 0 || known), "three_nn: null pointer");
   cudaStream_t st = as_stream(stream);
-  // a buffer for the tiles' ranges alone will do: every chunk of a tile is looked at then
+  // a buffer for the tiles' ranges alone will do: every point of a tile is looked at then
   if (!scratch || scratch_bytes < nn_tiles(m) * sizeof(float2))
     return fail(SSC_ERR_SCRATCH, "three_nn: scratch %zu < %zu bytes", scratch_bytes, nn_tiles(m) * sizeof(float2));
-  float4 *chunks = nullptr;
+  float4 *chunks = nullptr, *tiles = nullptr;
   float2 *ranges = (float2 *)scratch;
-  if (scratch_bytes >= ssc_three_nn_scratch_bytes(m)) {
+  int32_t *shares = nullptr;
+  if (m > NN_FEW && scratch_bytes >= ssc_three_nn_scratch_bytes(m)) {
     chunks = (float4 *)(((uintptr_t)scratch + 15) & ~(uintptr_t)15);
-    ranges = (float2 *)(chunks + nn_tiles(m) * (NN_TILE / NN_CHUNK));
+    tiles = chunks + nn_tiles(m) * (NN_TILE / NN_CHUNK);
+    ranges = (float2 *)(tiles + nn_tiles(m));
+    shares = (int32_t *)(ranges + nn_tiles(m));
   }
-  { nn_ranges_kernel<<<(int)nn_tiles(m), 256, 0, st>>>((const float4 *)known, m, ranges, chunks); note_launches(1); }
-  { three_nn_kernel<<<ceil_div(n, 8 * NN_QUERIES), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, ranges, chunks, dist2, idx); note_launches(1); }
+  { nn_ranges_kernel<<<(int)nn_tiles(m), NN_TILE, 0, st>>>((const float4 *)known, m, ranges, chunks, tiles, shares); note_launches(1); }
+  // 32 queries to a block fill the SMs up to 256 queries per SM; beyond, by tiles, a tile's way to shared memory and the merging pay
+  // for 64 only (64 k queries in any order 131 us in one kernel, 123 in two; in grid order 77 and 79.  20 k: 309 and 357).
+  if (n < sm_count() * 256) {
+    { three_nn_kernel<<<ceil_div(n, 32), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, ranges, chunks, tiles, shares, dist2, idx); note_launches(1); }
+  } else {
+    { three_nn_tiles_kernel<<<ceil_div(n, 64), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, ranges, tiles, shares, dist2, idx); note_launches(1); }
+    if (chunks != nullptr)
+      { three_nn_warps_kernel<<<ceil_div(n, 32), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, chunks, tiles, shares, dist2, idx); note_launches(1); }
+  }
   SSC_CHECK_LAUNCH("three_nn");
   return SSC_OK;
 }

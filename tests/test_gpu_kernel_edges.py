@@ -205,7 +205,8 @@ def test_three_nearest_with_ties(cuda, n_query, n_known):
     assert torch.equal(dist, want[:, :3].sqrt()) and torch.equal(idx.long(), order[:, :3])
 
 
-@pytest.mark.parametrize("n_query,known_of", [(5, [0, 1, 2]), (70, [31, 32, 33, 1024]), (40, [1000, 2100, 7]), (33, [1] * 70)])
+@pytest.mark.parametrize("n_query,known_of", [(5, [0, 1, 2]), (70, [31, 32, 33, 1024]), (40, [1000, 2100, 7]), (33, [1] * 70), (257, [35000, 3]),
+                                              (38000, [300, 31, 500]), (50001, [200, 57])])
 @pytest.mark.parametrize("in_order", [True, False])
 def test_three_nearest_passes_over_far_chunks(cuda, n_query, known_of, in_order):
     """Samples of fewer points than three, around a chunk and a tile of the known points, in grid order and shuffled; queries inside,
@@ -224,11 +225,66 @@ def test_three_nearest_passes_over_far_chunks(cuda, n_query, known_of, in_order)
     want, order = torch.sort(torch.cat([d, torch.full((n_query, 3), float("inf"), device=cuda)], 1), dim=1, stable=True)
     want, order = want[:, :3], torch.where(want[:, :3].isinf(), 0, order[:, :3])
     assert torch.equal(dist, want.sqrt()) and torch.equal(idx.long(), order)
-    # a buffer for the tiles' ranges alone
+    # buffers for the tiles' ranges alone, and of a size in between
     from ss_conv._ext import lib, _check, _p, _stream
-    small, d2, at = torch.empty(8 * -(-len(k) // 1024), dtype=torch.uint8, device=cuda), torch.empty_like(dist), torch.empty_like(idx)
-    _check(lib().ssc_three_nn(n_query, len(k), _p(q), _p(k), _p(d2), _p(at), _p(small), small.numel(), _stream()))
-    assert torch.equal(d2.sqrt(), dist) and torch.equal(at, idx)
+    for nbytes in (8 * -(-len(k) // 1024), 520 * -(-len(k) // 1024) + 16):
+        small, d2, at = torch.empty(nbytes, dtype=torch.uint8, device=cuda), torch.empty_like(dist), torch.empty_like(idx)
+        _check(lib().ssc_three_nn(n_query, len(k), _p(q), _p(k), _p(d2), _p(at), _p(small), small.numel(), _stream()))
+        assert torch.equal(d2.sqrt(), dist) and torch.equal(at, idx)
+
+
+@pytest.mark.parametrize("n_query", [50, 40000])
+@pytest.mark.parametrize("in_order", [True, False])
+def test_three_nearest_of_coordinates_that_are_no_numbers(cuda, n_query, in_order):
+    """A known point with a coordinate or batch id that is not a number, or infinitely far, is nobody's neighbour; a query with one has
+    none at all; infinite distances count as none.  The other distances are exact (small multiples of 1/4)."""
+    from ss_conv.sp_ops.functional import three_nn
+    rng = np.random.RandomState(n_query)
+    k = np.concatenate([rng.randint(0, 3, (700, 1)), rng.randint(-20, 20, (700, 3)) / 4], 1).astype(np.float32)
+    q = np.concatenate([rng.randint(0, 3, (n_query, 1)), rng.randint(-20, 20, (n_query, 3)) / 4], 1).astype(np.float32)
+    if in_order:
+        k = k[np.lexsort((k[:, 1], k[:, 0]))]
+    bad = np.array([np.nan, np.inf, -np.inf], np.float32)
+    for row, v in enumerate(bad):
+        for col in range(4):
+            k[row * 40 + col::229, col] = v
+            q[3 + row * 4 + col::61, col] = v
+    k[320:352, 1] = np.nan                                          # a whole chunk
+    q, k = dev(q, cuda), dev(k, cuda)
+    dist, idx = three_nn(q, k)
+    d = ((q[:, None, 1:] - k[None, :, 1:]) ** 2).sum(-1)
+    d = torch.where((q[:, None, 0] == k[None, :, 0]) & (d < float("inf")), d, torch.full((), float("inf"), device=cuda))
+    want, order = torch.sort(d, dim=1, stable=True)
+    want = want[:, :3]
+    assert torch.equal(dist, want.sqrt()) and torch.equal(idx.long(), torch.where(want.isinf(), 0, order[:, :3]))
+
+
+def _least_ms(call, repeats=7):
+    a, b, times = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True), []
+    for _ in range(repeats):
+        a.record()
+        for _ in range(5):
+            call()
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b))
+    return min(times)
+
+
+def test_three_nearest_in_any_order_cost_what_looking_at_all_costs(cuda):
+    """Shuffled points, of which nothing can be passed over, took 2.2 times as long as points in grid order (now 1.4: bound 1.8), and
+    points in order of a sample of many tiles as long as shuffled ones (0.9; now 0.4: bound 0.65)."""
+    from ss_conv import _ext
+    rng = np.random.RandomState(0)
+    for batch, n_query, n_known, bound in ((64, 4096, 1024, lambda ordered, shuffled: shuffled <= 1.8 * ordered),
+                                           (1, 4096, 40000, lambda ordered, shuffled: ordered <= 0.65 * shuffled)):
+        def points(n):
+            return np.concatenate([np.repeat(np.arange(batch), n)[:, None], rng.uniform(-.5, .5, (batch * n, 3))], 1).astype(np.float32)
+        q, k = points(n_query), points(n_known)
+        d, i = torch.empty(len(q), 3, device=cuda), torch.empty(len(q), 3, dtype=torch.int32, device=cuda)
+        q = dev(q, cuda)
+        took = [_least_ms(lambda: _ext.three_nn(len(q), len(k), q, known, d, i)) for known in (dev(k[np.lexsort((k[:, 1], k[:, 0]))], cuda), dev(k, cuda))]
+        assert bound(*took), took
 
 
 @pytest.mark.parametrize("c_in,c_out,c_keep,n,precision,stored", [
