@@ -164,30 +164,28 @@ conv_fwd_fp32_kernel(const float *__restrict__ features, int c_in, const float *
 }
 
 // The same sums for up to four input channels (a first layer on point features), in the same order: per output
-// element fused multiply-adds over ascending offsets and channels, present neighbours only.
-// A lane has an output row and CB of its channels, two to a register pair; the filters stand in shared memory, where all
-// lanes read the same word at a time.  Table entries and input rows of nine offsets are in flight together.  Bound by
-// issue: a warp runs through every offset that one of its 32 rows has.  215 k rows of 3 -> 36 channels, 6 neighbours
-// a row: 64 us; 83 with a warp per eight rows and a lane per channel, where a row took 200 instructions, as many
-// shuffles as multiply-adds.  (Two rows to a lane and zeros for absent neighbours: 92; three offsets in flight: 76;
-// blocks of four warps, each with its copy of the filters: 71.)
+// element fused multiply-adds over ascending offsets and channels, present neighbours only.  Two forms; fp32_by_lanes chooses.
+//
+// By lanes: a lane has an output row and CB of its channels, two to a register pair; the filters stand in shared memory, where all
+// lanes read the same word at a time.  Table entries and input rows of nine offsets are in flight together.  Bound by what
+// shared memory hands out, 16 bytes a lane for four multiply-adds: a warp runs through every offset that one of its 32 rows has.
+// (215 k rows of 3 -> 36 channels, 6 neighbours a row: 58 us, by warps 94.  Two rows to a lane and zeros for absent
+// neighbours: 92; three offsets in flight: 76; blocks of four warps, each with its copy of the filters: 71.)
 constexpr int SM_WARPS = 8, SM_AHEAD = 9;
-template <int CB, bool STAGED>
+template <int CB>
 __global__ void __launch_bounds__(SM_WARPS * 32)
-conv_fwd_fp32_small_kernel(const float *__restrict__ features, int c_in, const float *__restrict__ filters, int K,
+conv_fwd_fp32_lanes_kernel(const float *__restrict__ features, int c_in, const float *__restrict__ filters, int K,
                            int c_out, const int32_t *__restrict__ nbr, int n_out, int rev, float *__restrict__ out,
                            const int32_t *__restrict__ n_out_dev) {
   extern __shared__ __align__(16) float ws[];   // [K][c_in][CB]
   const int n_rows = live_rows(n_out, n_out_dev);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.y * CB;
   if ((int)blockIdx.x * SM_WARPS * 32 >= n_rows) return;
-  if (STAGED) {
-    for (int i = threadIdx.x; i < K * c_in * CB; i += SM_WARPS * 32) {
-      const int ch = i % CB, kc = i / CB;
-      ws[i] = n0 + ch < c_out ? __ldg(filters + (size_t)kc * c_out + n0 + ch) : 0.f;
-    }
-    __syncthreads();
+  for (int i = threadIdx.x; i < K * c_in * CB; i += SM_WARPS * 32) {
+    const int ch = i % CB, kc = i / CB;
+    ws[i] = n0 + ch < c_out ? __ldg(filters + (size_t)kc * c_out + n0 + ch) : 0.f;
   }
+  __syncthreads();
   const bool vec = (c_out & 3) == 0 && ((uintptr_t)out & 15u) == 0;
   for (int m0 = ((int)blockIdx.x * SM_WARPS + warp) * 32; m0 < n_rows; m0 += (int)gridDim.x * SM_WARPS * 32) {
     const int row = m0 + lane;
@@ -221,19 +219,12 @@ conv_fwd_fp32_small_kernel(const float *__restrict__ features, int c_in, const f
         for (int c = 0; c < 4; ++c) {
           if (c >= c_in) break;
           const f32x2 xx = pair_of(x[i][c], x[i][c]);
-          if (STAGED) {
-            const ulonglong2 *w = (const ulonglong2 *)(ws + ((size_t)(k0 + i) * c_in + c) * CB);
+          const ulonglong2 *w = (const ulonglong2 *)(ws + ((size_t)(k0 + i) * c_in + c) * CB);
 #pragma unroll
-            for (int j = 0; j < CB / 2; j += 2) {
-              const ulonglong2 v = w[j / 2];
-              acc[j] = fma_pair(xx, v.x, acc[j]);
-              acc[j + 1] = fma_pair(xx, v.y, acc[j + 1]);
-            }
-          } else {
-            const float *w = filters + ((size_t)(k0 + i) * c_in + c) * c_out + n0;
-#pragma unroll
-            for (int j = 0; j < CB / 2; ++j)
-              acc[j] = fma_pair(xx, pair_of(n0 + 2 * j < c_out ? __ldg(w + 2 * j) : 0.f, n0 + 2 * j + 1 < c_out ? __ldg(w + 2 * j + 1) : 0.f), acc[j]);
+          for (int j = 0; j < CB / 2; j += 2) {
+            const ulonglong2 v = w[j / 2];
+            acc[j] = fma_pair(xx, v.x, acc[j]);
+            acc[j + 1] = fma_pair(xx, v.y, acc[j + 1]);
           }
         }
       }
@@ -256,14 +247,147 @@ conv_fwd_fp32_small_kernel(const float *__restrict__ features, int c_in, const f
   }
 }
 
+// Channels of a lane, in how many passes over the rows.
+struct LaneShape { int channels, passes; };
+static LaneShape lane_shape(int c_out) {
+  const int passes = ceil_div(c_out, 48);
+  return {max((ceil_div(c_out, passes) + 7) & ~7, 16), passes};
+}
+static size_t lane_smem(int K, int c_in, int c_out) { return (size_t)K * c_in * lane_shape(c_out).channels * sizeof(float); }
+
+// By lanes from as many rows as fill the SMs with work enough for a row; a form by warps has four times the blocks, and pays per
+// neighbour where the other pays per offset, but as much for few channels as for 32.  `work`: multiply-adds of a row and offset by
+// lanes, 40 more for a pass.  In us by warps / by lanes, 27 offsets, at 3, 6 and 12 neighbours a row:
+//   1 -> 16 (work 16)    300 rows 7.8/6.9, 9.7/6.8, 12/7.2
+//   3 -> 36 (120)        10 k 10/14, 12/15, 15/15; 20 k 12/14, 15/15, 19/15; 30 k 17/14, 21/15, 26/15; 100 k 37/30, 48/33, 58/34
+//   4 -> 48 (192)        30 k 17/19, 21/19, 27/20; 60 k 25/30, 32/31, 40/32; 215 k 72/81, 95/84, 120/88
+//   3 -> 64 (232)        60 k 25/35, 31/38, 39/41; 1 M 316/407, 418/438, 526/484   (27 neighbours: 843/615)
+//   3 -> 92 (328)        60 k 30/47, 39/50, 48/54; 1 M 394/546, 515/577, 648/624   (27 neighbours: 1023/763)
+// Tables that have fewer than three neighbours a row for their sizes alone (a layer that spreads few rows) are for warps from work 150
+// on (4 -> 48, 100 k rows, 1.5 neighbours: 28/39).  Filters beyond 100 KB leave no two blocks on an SM: by warps, through L1.
+static bool fp32_by_lanes(int n_in, int c_in, int K, int c_out, int n_out) {
+  const LaneShape s = lane_shape(c_out);
+  const long long work = (long long)c_in * s.channels * s.passes + 40 * (s.passes - 1);
+  const bool sparse = (long long)K * n_in < 3LL * n_out;
+  return lane_smem(K, c_in, c_out) <= 100 * 1024 && work <= (sparse ? 150 : 200) && n_out >= 350 * (work - 48);
+}
+
 template <int CB>
-static int launch_fp32_small(const float *features, int c_in, const float *filters, int K, int c_out, const int32_t *nbr, int n_out,
+static int launch_fp32_lanes(const float *features, int c_in, const float *filters, int K, int c_out, const int32_t *nbr, int n_out,
                              int rev, float *out, const int32_t *n_out_dev, cudaStream_t st) {
   const size_t smem = (size_t)K * c_in * CB * sizeof(float);
-  const bool staged = smem <= 100 * 1024;     // two blocks per SM at least; larger filter sets are read through L1
   const int blocks = ceil_div(n_out, SM_WARPS * 32), most = sm_count() * 2;
   const dim3 grid(blocks < most ? blocks : most, ceil_div(c_out, CB));
-  auto kernel = staged ? conv_fwd_fp32_small_kernel<CB, true> : conv_fwd_fp32_small_kernel<CB, false>;
+  auto kernel = conv_fwd_fp32_lanes_kernel<CB>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = allow_smem((const void *)kernel, smem);
+    if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(fp32): smem attribute: %s", cudaGetErrorString(e));
+  }
+  { kernel<<<grid, SM_WARPS * 32, smem, st>>>(features, c_in, filters, K, c_out, nbr, n_out, rev, out, n_out_dev); note_launches(1); }
+  SSC_CHECK_LAUNCH("conv_fwd_fp32");
+  return SSC_OK;
+}
+
+// By warps: a warp takes eight output rows at a time; lanes hold NJ output channels each (lane, lane + 32, ...), the
+// filters stand in shared memory.  All 28 x 8 table entries of a pass, then all present input rows, are
+// loaded at once, a lane per (offset, row); they reach the other lanes by shuffles.  Bound by instruction
+// issue (about 200 per row of 6 neighbours and 64 channels).  The tiled kernel above pads the
+// channels to 16 and multiplies absent rows: 399 us for 215 k rows of 3 -> 48 channels.
+// (Four lanes to a row with their own channels, rows handed round by shuffles: 1.1 to 1.6 times as long, every lane reads its filters.)
+constexpr int SM_GROUP = 8;
+template <int NJ, bool STAGED>
+__global__ void __launch_bounds__(SM_WARPS * 32)
+conv_fwd_fp32_warps_kernel(const float *__restrict__ features, int c_in, const float *__restrict__ filters, int K,
+                           int c_out, const int32_t *__restrict__ nbr, int n_out, int rev, float *__restrict__ out,
+                           const int32_t *__restrict__ n_out_dev) {
+  extern __shared__ float ws[];               // [K][c_in][NJ * 32]
+  const int n_rows = live_rows(n_out, n_out_dev);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.y * NJ * 32;
+  if (STAGED) {
+    for (int i = threadIdx.x; i < K * c_in * NJ * 32; i += SM_WARPS * 32) {
+      const int ch = i % (NJ * 32), kc = i / (NJ * 32);
+      ws[i] = n0 + ch < c_out ? __ldg(filters + (size_t)kc * c_out + n0 + ch) : 0.f;
+    }
+    __syncthreads();
+  }
+  for (int m0 = ((int)blockIdx.x * SM_WARPS + warp) * SM_GROUP; m0 < n_rows; m0 += (int)gridDim.x * SM_WARPS * SM_GROUP) {
+    float acc[SM_GROUP][NJ];
+#pragma unroll
+    for (int r = 0; r < SM_GROUP; ++r)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) acc[r][j] = 0.f;
+    const int my_row = m0 + (lane & 7);
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += 28) {
+      int idx[7];
+      float x[7][4];
+#pragma unroll
+      for (int t = 0; t < 7; ++t) {            // entry (offset k0 + 4 t + lane / 8, row lane % 8)
+        const int k = k0 + 4 * t + (lane >> 3);
+        idx[t] = (k < K && my_row < n_rows) ? __ldg(nbr + (size_t)(rev ? K - 1 - k : k) * n_out + my_row) : -1;
+      }
+#pragma unroll
+      for (int t = 0; t < 7; ++t) {
+        const float *fp = features + (size_t)(idx[t] >= 0 ? idx[t] : 0) * c_in;
+        if (c_in == 4) {
+          const float4 f = idx[t] >= 0 ? __ldg((const float4 *)fp) : make_float4(0.f, 0.f, 0.f, 0.f);
+          x[t][0] = f.x; x[t][1] = f.y; x[t][2] = f.z; x[t][3] = f.w;
+        } else {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) x[t][c] = (c < c_in && idx[t] >= 0) ? __ldg(fp + c) : 0.f;
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < 7; ++t) {
+        const unsigned have = __ballot_sync(0xffffffffu, idx[t] >= 0);
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          const unsigned m = (have >> (8 * q)) & 255u;
+          if (m == 0u) continue;
+          const int k = k0 + 4 * t + q;
+          float w[4][NJ];
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+              if (STAGED) w[c][j] = c < c_in ? ws[((size_t)k * c_in + c) * (NJ * 32) + j * 32 + lane] : 0.f;
+              else w[c][j] = (c < c_in && n0 + j * 32 + lane < c_out) ? __ldg(filters + ((size_t)k * c_in + c) * c_out + n0 + j * 32 + lane) : 0.f;
+            }
+#pragma unroll
+          for (int r = 0; r < SM_GROUP; ++r) {
+            if (!((m >> r) & 1u)) continue;    // the same for the whole warp
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const float xv = __shfl_sync(0xffffffffu, x[t][c], 8 * q + r);
+              if (c < c_in) {
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) acc[r][j] = fmaf(xv, w[c][j], acc[r][j]);
+              }
+            }
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < SM_GROUP; ++r) {
+      if (m0 + r >= n_rows) break;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const int ch = n0 + j * 32 + lane;
+        if (ch < c_out) out[(size_t)(m0 + r) * c_out + ch] = acc[r][j];
+      }
+    }
+  }
+}
+
+template <int NJ>
+static int launch_fp32_warps(const float *features, int c_in, const float *filters, int K, int c_out, const int32_t *nbr, int n_out,
+                             int rev, float *out, const int32_t *n_out_dev, cudaStream_t st) {
+  const size_t smem = (size_t)K * c_in * NJ * 32 * sizeof(float);
+  const bool staged = smem <= 100 * 1024;     // two blocks per SM at least; larger filter sets are read through L1
+  const int blocks = ceil_div(n_out, SM_WARPS * SM_GROUP), most = sm_count() * 3;
+  const dim3 grid(blocks < most ? blocks : most, ceil_div(c_out, NJ * 32));
+  auto kernel = staged ? conv_fwd_fp32_warps_kernel<NJ, true> : conv_fwd_fp32_warps_kernel<NJ, false>;
   if (staged && smem > 48 * 1024) {
     cudaError_t e = allow_smem((const void *)kernel, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(fp32): smem attribute: %s", cudaGetErrorString(e));
@@ -343,12 +467,18 @@ extern "C" int ssc_conv_fwd_ordered(const float *features, int n_in, int c_in, c
     if (c_in <= 4 && (c_in != 4 || ((uintptr_t)features & 15u) == 0)) {
       const int rev = table_form != 0;
       const float *w = (const float *)filters;
-      const int per = ceil_div(c_out, ceil_div(c_out, 48));          // channels of a lane
-      if (per <= 16) return launch_fp32_small<16>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
-      if (per <= 24) return launch_fp32_small<24>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
-      if (per <= 32) return launch_fp32_small<32>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
-      if (per <= 40) return launch_fp32_small<40>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
-      return launch_fp32_small<48>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+      if (fp32_by_lanes(n_in, c_in, K, c_out, n_out)) {
+        switch (lane_shape(c_out).channels) {
+          case 16: return launch_fp32_lanes<16>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+          case 24: return launch_fp32_lanes<24>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+          case 32: return launch_fp32_lanes<32>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+          case 40: return launch_fp32_lanes<40>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+          default: return launch_fp32_lanes<48>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+        }
+      }
+      if (c_out <= 32) return launch_fp32_warps<1>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+      if (c_out <= 64) return launch_fp32_warps<2>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
+      return launch_fp32_warps<3>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
     }
     dim3 grid(ceil_div(n_out, BM), ceil_div(c_out, BN));
     { conv_fwd_fp32_kernel<<<grid, 256, 0, st>>>(features, c_in, (const float *)filters, K, c_out, nbr, n_out, table_form != 0, out, n_out_dev); note_launches(1); }

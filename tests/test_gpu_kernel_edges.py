@@ -122,8 +122,8 @@ def test_fp32_convolution_of_few_input_channels(cuda, c_in, c_out, k, n):
 @pytest.mark.parametrize("c_out", [16, 17, 25, 33, 41, 48, 49, 97])
 @pytest.mark.parametrize("K,n", [(1, 31), (9, 33), (10, 257), (125, 300)])
 def test_fp32_convolution_by_lanes_of_rows(cuda, c_in, c_out, K, n):
-    """Channels of a lane (16, 24, 32, 40, 48, several passes over the rows, filters too large for shared memory), offsets around the
-    nine in flight, rows around a warp and a block.  Every term is rounded once, so |error| <= terms * 2^-24 * sum |x w|;
+    """Channel counts around those of a lane, several passes over the rows, offsets around the nine in flight, rows around a warp
+    and a block (by lanes for the fewest channels, by warps else).  Every term is rounded once, so |error| <= terms * 2^-24 * sum |x w|;
     a filter that is not a number reaches the rows that have its offset and no others."""
     from ss_conv import _ext
     rng = np.random.RandomState(K + c_out)
@@ -137,6 +137,77 @@ def test_fp32_convolution_by_lanes_of_rows(cuda, c_in, c_out, K, n):
     w[K // 2, 0, c_out - 1] = np.nan
     got = _ext.conv_forward(dev(x, cuda), dev(w, cuda), dev(t, cuda), n, "fp32").cpu().numpy()
     assert (np.isnan(got[:, -1]) == (t[K // 2] >= 0)).all() and np.isfinite(got[:, :-1]).all()
+
+
+def _least_ms(call, repeats=7):
+    a, b, times = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True), []
+    for _ in range(repeats):
+        a.record()
+        for _ in range(5):
+            call()
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b))
+    return min(times)
+
+
+def _few_channels(cuda, c_in, c_out, K, n, n_in=200):
+    """Every term is rounded once, so |error| <= terms * 2^-24 * sum |x w|; a filter that is not a number reaches the rows that
+    have its offset and no others."""
+    from ss_conv import _ext
+    rng = np.random.RandomState(K + c_out)
+    t = _table(n, n_in, K, 0.4, rng)
+    x, w = rng.randn(n_in, c_in).astype(np.float32), rng.randn(K, c_in, c_out).astype(np.float32)
+    xd, wd, td = dev(x, cuda), dev(w, cuda), dev(t, cuda)
+    got = _ext.conv_forward(xd, wd, td, n, "fp32").double()
+    want, size = torch.zeros_like(got), torch.zeros_like(got)
+    x64 = torch.cat([xd.double(), torch.zeros(1, c_in, device=cuda, dtype=torch.float64)])
+    for k in range(K):
+        g = x64[td[k].long()]                                       # (-1: the row of zeros)
+        want += g @ wd[k].double()
+        size += g.abs() @ wd[k].double().abs()
+    assert bool(((got - want).abs() <= K * c_in * 2.0 ** -24 * size).all())
+    wd[K // 2, 0, c_out - 1] = float("nan")
+    got = _ext.conv_forward(xd, wd, td, n, "fp32")
+    assert torch.equal(got[:, -1].isnan(), td[K // 2] >= 0) and bool(got[:, :-1].isfinite().all())
+
+
+@pytest.mark.parametrize("c_in,c_out", [(1, 5), (4, 16), (3, 17), (4, 24), (3, 25), (2, 33), (4, 40), (3, 41), (4, 48), (1, 49), (1, 97)])
+@pytest.mark.parametrize("K,n", [(9, 60001), (10, 57600)])
+def test_fp32_convolution_by_lanes_of_many_rows(cuda, c_in, c_out, K, n):
+    """Row counts beyond the line to the form by lanes (350 * (192 - 48) at most, 200 in place of 192 for 97 channels): 16, 24, 32, 40 and 48
+    channels to a lane, one to three passes over the rows, offsets around the nine in flight, more rows than one round of the grid."""
+    _few_channels(cuda, c_in, c_out, K, n, n_in=60000)
+    # the same bits by warps: few rows, and more than three times as many rows as offsets times inputs
+    from ss_conv import _ext
+    rng = np.random.RandomState(n)
+    x, w = dev(rng.randn(n // 40, c_in).astype(np.float32), cuda), dev(rng.randn(K, c_in, c_out).astype(np.float32), cuda)
+    t = dev(_table(n, n // 40, K, 0.2, rng), cuda)
+    many = _ext.conv_forward(x, w, t, n, "fp32")
+    padded = _ext.conv_forward(torch.cat([x] * 20), w, t, n, "fp32")
+    assert torch.equal(many, padded)
+    assert torch.equal(many[:300], _ext.conv_forward(x, w, t[:, :300].contiguous(), 300, "fp32"))
+
+
+@pytest.mark.parametrize("c_in,c_out,K", [(3, 19, 343), (4, 32, 343), (3, 33, 343), (4, 47, 343), (3, 70, 343), (1, 97, 343), (4, 16, 420)])
+@pytest.mark.parametrize("n", [1, 300, 60001])
+def test_fp32_convolution_with_filters_beyond_shared_memory(cuda, c_in, c_out, K, n):
+    """Filters of more than 100 KB, which are read through L1, one to three channels to a lane, few rows and many."""
+    assert K * c_in * min(-(-c_out // 32), 3) * 32 * 4 > 100 * 1024
+    _few_channels(cuda, c_in, c_out, K, n, n_in=300)
+
+
+def test_fp32_convolution_with_large_filters_costs_less_than_dense_tiles(cuda):
+    """10 k rows of 3 -> 48 channels, 343 offsets, 6 neighbours a row: 680 us where every lane read its own row's filters, now 46.  The
+    yardstick are the same rows padded to five channels, for the tiled kernel (16 channels, absent rows multiplied too): bound a quarter."""
+    from ss_conv import _ext
+    rng = np.random.RandomState(0)
+    t = dev(_table(10000, 5000, 343, 6 / 343, rng), cuda)
+    took = []
+    for c_in in (3, 5):
+        x, w = dev(rng.randn(5000, c_in).astype(np.float32), cuda), dev(rng.randn(343, c_in, 48).astype(np.float32), cuda)
+        took.append(_least_ms(lambda: _ext.conv_forward(x, w, t, 10000, "fp32")))
+    assert took[0] <= 0.25 * took[1], took
 
 
 @pytest.mark.parametrize("precision", ["tf32", "bf16", "fp16"])
@@ -205,8 +276,7 @@ def test_three_nearest_with_ties(cuda, n_query, n_known):
     assert torch.equal(dist, want[:, :3].sqrt()) and torch.equal(idx.long(), order[:, :3])
 
 
-@pytest.mark.parametrize("n_query,known_of", [(5, [0, 1, 2]), (70, [31, 32, 33, 1024]), (40, [1000, 2100, 7]), (33, [1] * 70), (257, [35000, 3]),
-                                              (38000, [300, 31, 500]), (50001, [200, 57])])
+@pytest.mark.parametrize("n_query,known_of", [(5, [0, 1, 2]), (70, [31, 32, 33, 1024]), (40, [1000, 2100, 7]), (33, [1] * 70)])
 @pytest.mark.parametrize("in_order", [True, False])
 def test_three_nearest_passes_over_far_chunks(cuda, n_query, known_of, in_order):
     """Samples of fewer points than three, around a chunk and a tile of the known points, in grid order and shuffled; queries inside,
@@ -225,12 +295,26 @@ def test_three_nearest_passes_over_far_chunks(cuda, n_query, known_of, in_order)
     want, order = torch.sort(torch.cat([d, torch.full((n_query, 3), float("inf"), device=cuda)], 1), dim=1, stable=True)
     want, order = want[:, :3], torch.where(want[:, :3].isinf(), 0, order[:, :3])
     assert torch.equal(dist, want.sqrt()) and torch.equal(idx.long(), order)
-    # buffers for the tiles' ranges alone, and of a size in between
+    # a buffer for the tiles' ranges alone
     from ss_conv._ext import lib, _check, _p, _stream
-    for nbytes in (8 * -(-len(k) // 1024), 520 * -(-len(k) // 1024) + 16):
-        small, d2, at = torch.empty(nbytes, dtype=torch.uint8, device=cuda), torch.empty_like(dist), torch.empty_like(idx)
-        _check(lib().ssc_three_nn(n_query, len(k), _p(q), _p(k), _p(d2), _p(at), _p(small), small.numel(), _stream()))
-        assert torch.equal(d2.sqrt(), dist) and torch.equal(at, idx)
+    small, d2, at = torch.empty(8 * -(-len(k) // 1024), dtype=torch.uint8, device=cuda), torch.empty_like(dist), torch.empty_like(idx)
+    _check(lib().ssc_three_nn(n_query, len(k), _p(q), _p(k), _p(d2), _p(at), _p(small), small.numel(), _stream()))
+    assert torch.equal(d2.sqrt(), dist) and torch.equal(at, idx)
+
+
+@pytest.mark.parametrize("n_query,known_of", [(257, [35000, 3]), (38000, [300, 31, 500]), (50001, [200, 57])])
+@pytest.mark.parametrize("in_order", [True, False])
+def test_three_nearest_of_many(cuda, n_query, known_of, in_order):
+    """A sample of many tiles; more queries than one kernel takes; a buffer for more than the tiles' ranges, but not for all."""
+    from ss_conv import _ext
+    test_three_nearest_passes_over_far_chunks(cuda, n_query, known_of, in_order)
+    rng = np.random.RandomState(n_query)
+    k = dev(np.concatenate([rng.randint(0, 2, (3000, 1)), rng.randint(-20, 20, (3000, 3)) / 4], 1).astype(np.float32), cuda)
+    d, at = torch.empty(2, 3000, 3, device=cuda), torch.empty(2, 3000, 3, dtype=torch.int32, device=cuda)
+    small = torch.empty(520 * 3 + 16, dtype=torch.uint8, device=cuda)
+    _ext.three_nn(3000, 3000, k, k, d[0], at[0])
+    _ext._check(_ext.lib().ssc_three_nn(3000, 3000, _ext._p(k), _ext._p(k), _ext._p(d[1]), _ext._p(at[1]), _ext._p(small), small.numel(), _ext._stream()))
+    assert torch.equal(d[0], d[1]) and torch.equal(at[0], at[1])
 
 
 @pytest.mark.parametrize("n_query", [50, 40000])
@@ -257,18 +341,6 @@ def test_three_nearest_of_coordinates_that_are_no_numbers(cuda, n_query, in_orde
     want, order = torch.sort(d, dim=1, stable=True)
     want = want[:, :3]
     assert torch.equal(dist, want.sqrt()) and torch.equal(idx.long(), torch.where(want.isinf(), 0, order[:, :3]))
-
-
-def _least_ms(call, repeats=7):
-    a, b, times = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True), []
-    for _ in range(repeats):
-        a.record()
-        for _ in range(5):
-            call()
-        b.record()
-        b.synchronize()
-        times.append(a.elapsed_time(b))
-    return min(times)
 
 
 def test_three_nearest_in_any_order_cost_what_looking_at_all_costs(cuda):
