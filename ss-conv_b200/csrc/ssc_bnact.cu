@@ -259,8 +259,9 @@ static bool launch_bn_gate_rows(const float *x, int n, uint32_t groups, int c_in
 // eight chains of a row block are added in order, then the row blocks, then the channels of a field.
 // Batch statistics therefore repeat bit for bit, whatever grid or load width computes them.
 // A thread walks one chain of VEC channels with AHEAD loads in flight, the last of a chain too: chains are few (20 k threads
-// for 38 channels), so what bounds it is how many rows are on their way (72 k rows of 76 channels, sums, with sixteen and a
-// remainder one by one: 41 us, like this 14; 121 k rows of 76: 19.5 -> 7.2).
+// for 38 channels), so what bounds it is how many rows are on their way.  Whole batches of rows without a test between
+// the loads, then the rest.  (ssc_bn_train: 121 k rows of 38 / 76 / 150 channels 16.9 / 19.9 / 22.4 us; with sixteen ahead and a rest one by one
+// 25.1 / 39.6 / 27.5; with 32 or 64 ahead and a test before every load 25.4 / 27.3 / 46.4.  32 instead of 24: 16.8 / 19.3 / 23.2.)
 // MODE 0: sum of x; 1: sum of (x - mean_ch)^2.  part [chains][c].
 static int bn_row_blocks(int n) {
   const int rb = ceil_div(n, 8 * 64);
@@ -276,36 +277,43 @@ bn_colsum_kernel(const float *__restrict__ x, int n, int c, int chains, int lane
   for (int g = threadIdx.x % (blockDim.x / lanes); g < groups; g += blockDim.x / lanes) {
     const float *p = x + (size_t)chain * c + (size_t)g * VEC;
     const size_t step = (size_t)chains * c;
+    constexpr int AHEAD = 24;
     float s[VEC], mu[VEC];
 #pragma unroll
     for (int q = 0; q < VEC; ++q) {
       s[q] = 0.f;
       mu[q] = MODE != 0 ? chan_mean[g * VEC + q] : 0.f;
     }
-    constexpr int AHEAD = VEC == 4 ? 32 : 64;
+    float v[AHEAD][VEC];
+    auto load = [&](int i) {
+      if (VEC == 4) {
+        const float4 f = __ldg((const float4 *)(p + i * step));
+        v[i][0] = f.x; v[i][1 % VEC] = f.y; v[i][2 % VEC] = f.z; v[i][3 % VEC] = f.w;
+      } else {
+        v[i][0] = __ldg(p + i * step);
+      }
+    };
+    auto add = [&](int i) {
+#pragma unroll
+      for (int q = 0; q < VEC; ++q) {
+        const float d = v[i][q] - mu[q];
+        s[q] = MODE == 0 ? s[q] + d : fmaf(d, d, s[q]);
+      }
+    };
+    int left = (n - chain + chains - 1) / chains;          // rows of the chain (chain < n, or none)
 #pragma unroll 1
-    for (uint32_t r = chain; r < (uint32_t)n; r += AHEAD * chains, p += AHEAD * step) {
-      float v[AHEAD][VEC];
+    for (; left >= AHEAD; left -= AHEAD, p += AHEAD * step) {
 #pragma unroll
-      for (int i = 0; i < AHEAD; ++i) {
-        if (r + i * chains >= (uint32_t)n) break;
-        if (VEC == 4) {
-          const float4 f = __ldg((const float4 *)(p + i * step));
-          v[i][0] = f.x; v[i][1 % VEC] = f.y; v[i][2 % VEC] = f.z; v[i][3 % VEC] = f.w;
-        } else {
-          v[i][0] = __ldg(p + i * step);
-        }
-      }
+      for (int i = 0; i < AHEAD; ++i) load(i);
 #pragma unroll
-      for (int i = 0; i < AHEAD; ++i) {
-        if (r + i * chains >= (uint32_t)n) break;
-#pragma unroll
-        for (int q = 0; q < VEC; ++q) {
-          const float d = v[i][q] - mu[q];
-          s[q] = MODE == 0 ? s[q] + d : fmaf(d, d, s[q]);
-        }
-      }
+      for (int i = 0; i < AHEAD; ++i) add(i);
     }
+#pragma unroll
+    for (int i = 0; i < AHEAD - 1; ++i)
+      if (i < left) load(i);
+#pragma unroll
+    for (int i = 0; i < AHEAD - 1; ++i)
+      if (i < left) add(i);
 #pragma unroll
     for (int q = 0; q < VEC; ++q) part[(size_t)chain * c + g * VEC + q] = s[q];
   }
@@ -313,7 +321,7 @@ bn_colsum_kernel(const float *__restrict__ x, int n, int c, int chains, int lane
 
 // Sum of the chains of `count` consecutive channels from ch0, by one block, in the order stated above: the
 // row blocks' sums of eight chains in parallel, then one thread adds them up.  Result in every thread.
-constexpr int kFinishThreads = 512;        // (128: twice as many trips to memory, 7.1 us a launch for 6.3)
+constexpr int kFinishThreads = 512;        // (128: two rounds of loads for a field of four channels; ssc_bn_train of 72 k rows of 152: 18.0 us for 17.6)
 constexpr int kFinishTile = 16 * 64;       // (channel, row block) sums in shared memory at a time
 __device__ __forceinline__ float chain_total(const float *__restrict__ part, int row_blocks, int c, int ch0, int count) {
   __shared__ float sm[kFinishTile];
