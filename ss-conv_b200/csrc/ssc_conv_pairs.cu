@@ -200,7 +200,8 @@ __device__ __forceinline__ void deal_strips(const int32_t *__restrict__ starts, 
 
 // What the persistent kernel needs beforehand, in one launch: the strip table (block 0: 16 us of one block's
 // serial work), the operand image of the rows (n_stage pieces of 16 bytes, as ssc_conv_stage.cu writes it; 0 where it is there
-// already) and a cleared output.  The last two are bound by memory, and the strips come in their shadow.
+// already) and a cleared output.  The last two are bound by memory, and the strips come in their shadow (and bound the launch
+// where rows are few).  One piece at a time: four loads before the first store, as ssc_conv_stage.cu has them, were not tried here.
 // (42 k rows 192 -> 192 bf16: 9 + 7 + 16 us one after the other, 22 like this; the whole layer 246 -> 232.)
 template <bool F16>
 __global__ void __launch_bounds__(PL_MAX_CTAS)
@@ -213,14 +214,8 @@ pl_prepare_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_
   }
   const long long first = (long long)(blockIdx.x - 1) * PL_MAX_CTAS + threadIdx.x, step = (long long)(gridDim.x - 1) * PL_MAX_CTAS;
   for (long long i = first; i < n_stage; i += step) {
-    if (F16) {
-      const float4 a = __ldg(rows + 2 * i), b = __ldg(rows + 2 * i + 1);
-      staged[i] = bf16 ? make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w))
-                       : make_uint4(pack_f16x2(a.x, a.y), pack_f16x2(a.z, a.w), pack_f16x2(b.x, b.y), pack_f16x2(b.z, b.w));
-    } else {
-      const float4 v = __ldg(rows + i);
-      staged[i] = make_uint4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
-    }
+    if (F16) staged[i] = stage_piece_16(__ldg(rows + 2 * i), __ldg(rows + 2 * i + 1), bf16 != 0);
+    else staged[i] = stage_piece(__ldg(rows + i));
   }
   for (long long i = first; i < n_clear; i += step) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }

@@ -34,7 +34,7 @@ stage_features_kernel(const float4 *__restrict__ in, long long total_vec, uint4 
     if (first + q * 256 < total_vec) v[q] = __ldg(in + first + q * 256);
 #pragma unroll
   for (int q = 0; q < STAGE_VECS; ++q)
-    if (first + q * 256 < total_vec) out[first + q * 256] = make_uint4(to_tf32(v[q].x), to_tf32(v[q].y), to_tf32(v[q].z), to_tf32(v[q].w));
+    if (first + q * 256 < total_vec) out[first + q * 256] = stage_piece(v[q]);
 }
 
 // Channel counts that are not a multiple of four: rows padded with zeros to c_pad floats.
@@ -121,9 +121,7 @@ stage_features_16_vec_kernel(const float4 *__restrict__ in, long long total, uin
     }
 #pragma unroll
   for (int q = 0; q < STAGE_VECS; ++q)
-    if (first + q * 256 < total)
-      out[first + q * 256] = BF16 ? make_uint4(pack_bf16x2(a[q].x, a[q].y), pack_bf16x2(a[q].z, a[q].w), pack_bf16x2(b[q].x, b[q].y), pack_bf16x2(b[q].z, b[q].w))
-                                  : make_uint4(pack_f16x2(a[q].x, a[q].y), pack_f16x2(a[q].z, a[q].w), pack_f16x2(b[q].x, b[q].y), pack_f16x2(b[q].z, b[q].w));
+    if (first + q * 256 < total) out[first + q * 256] = stage_piece_16(a[q], b[q], BF16);
 }
 
 size_t conv_f16_scratch_bytes(int n_in, int c_in) { return (size_t)n_in * (size_t)f16_row_words(c_in) * 4 + 16; }

@@ -761,8 +761,9 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
       a_lo += slot_step;
       if (++s == (uint32_t)S) { s = 0; par ^= 1u; a_lo = a_lo0; }
       // A CTA alone on its SM has a deep ring, and this warp's chain of instructions is what bounds a step (440 cycles undisturbed,
-      // whatever the products): the next step's barrier is looked at before this one's products are issued.  (16 k rows
-      // 32 -> 38: 15.0 -> 14.1 us; 15 k rows 256 -> 304 bf16: 61.2 -> 60.2.  With two or four CTAs the look comes too early: +1 to 2 %.)
+      // whatever the products): the next step's barrier is looked at before this one's products are issued.  (Up to one tile per SM
+      // 1 to 12 % off: 16 k rows 32 -> 38 15.0 -> 14.1 us, 19 k rows 132 -> 136 51.8 -> 45.7.  With more tiles than SMs between -4 and +2 %:
+      // 60 k rows 128 -> 128 bf16 68.6 -> 66.8, 256 -> 304 TF32 405 -> 412.  With two or four CTAs the look comes too early: +1 to 2 %.)
       const bool passed = GROUPS == 2 && p.ctas == 1 && mbar_test_wait(full0 + s * 8u, par);
       for (int nt = 0; nt < (any ? p.nt_cta : 0); ++nt) {
         const uint32_t dn = tmem_base + (uint32_t)(nt * p.tile_n);
