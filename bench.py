@@ -516,7 +516,7 @@ def helper_cases(dev):
     # (the three gathered rows per point come from L2: the 102 MB of voxel features fit there)
     cases.append(("three_interpolate (three_interpolate_vec4_kernel)", lambda: _ext.three_interpolate_fp(ci, mk, nq, vfe, idx, w, iout),
                   4.0 * nq * ci + 4.0 * mk * ci + 24.0 * nq))
-    # 3-NN: compute-bound brute force within a sample; reported as queries/s
+    # 3-NN of voxels in no order: every one of the sample is looked at, bound by instruction issue
     nn_q, nn_m, nn_b = 262144, 65536, 64
     kb = np.repeat(np.arange(nn_b), nn_m // nn_b)
     known = torch.from_numpy(np.concatenate([kb[:, None], rng.uniform(-0.5, 0.5, (nn_m, 3))], 1).astype(np.float32)).to(dev)
@@ -524,7 +524,7 @@ def helper_cases(dev):
     unk = torch.from_numpy(np.concatenate([ub[:, None], rng.uniform(-0.5, 0.5, (nn_q, 3))], 1).astype(np.float32)).to(dev)
     d2 = torch.empty(nn_q, 3, device=dev)
     i3 = torch.empty(nn_q, 3, dtype=torch.int32, device=dev)
-    cases.append(("three_nn (three_nn_kernel), 4096 queries x 1024 voxels per sample", lambda: _ext.three_nn(nn_q, nn_m, unk, known, d2, i3),
+    cases.append(("three_nn (three_nn_tiles_kernel), 4096 queries x 1024 voxels per sample", lambda: _ext.three_nn(nn_q, nn_m, unk, known, d2, i3),
                   16.0 * (nn_q + nn_m) + 24.0 * nn_q))
     # filter materialisation of the cfg2 layer (tiny: launch-bound)
     layer = Layer(CFG2, dev)
