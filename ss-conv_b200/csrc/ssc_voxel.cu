@@ -470,16 +470,8 @@ __device__ __forceinline__ void nn_by_tiles(int first, int n, int m, const float
   }
 }
 
-// Where ranges of x are narrow: a warp per query.  Its lanes look at the ranges of 32 tiles at a time, then at the 32 chunks of a
-// tile that can hold points of the query's sample: first at the points of the chunks nearest in x, then of those whose distance in
-// x alone does not exceed the third best so far.  That distance, rounded like the points' own, is never more than theirs:
-// every rounding involved is monotonic.  Of several tiles the nearest in x comes first: in order, each of those before it
-// would hold the best so far and be looked at whole (4096 queries among 40 k points in order: 1170 us, 586 by tiles, 102 like this).
-// Each lane keeps its three best by (distance, index); the three best of the warp by that order are the result of the
-// exhaustive reference loop.
-
 // The tiles that can hold points of a sample: all within [first, end), multiples of 32.  share: how many of 1024 of their
-// chunks a point of the first of them lies in.
+// chunks a point lies in, on average of those among the first 32 that hold any.
 struct NnSpan {
   float sample;
   int first, end, share;
@@ -503,6 +495,13 @@ __device__ __forceinline__ NnSpan nn_span(float sample, int n_tiles, const float
   return s;
 }
 
+// Where ranges of x are narrow: a warp per query.  Its lanes look at the ranges of 32 tiles at a time, then at the 32 chunks of a
+// tile that can hold points of the query's sample: first at the points of the chunks nearest in x, then of those whose distance in
+// x alone does not exceed the third best so far.  That distance, rounded like the points' own, is never more than theirs:
+// every rounding involved is monotonic.  Of several tiles the nearest in x comes first: in order, each of those before it
+// would hold the best so far and be looked at whole (4096 queries among 40 k points in order: 1170 us, 586 by tiles, 102 like this).
+// Each lane keeps its three best by (distance, index); the three best of the warp by that order are the result of the
+// exhaustive reference loop.
 constexpr int NN_QUERIES = 4;                     // of a warp, one after the other
 __device__ __forceinline__ void nn_by_warps(int q0, float4 next, NnSpan span, int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known,
                                             const float4 *__restrict__ chunks, const float4 *__restrict__ tiles, const int32_t *__restrict__ shares,
