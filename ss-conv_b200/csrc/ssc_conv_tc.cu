@@ -181,7 +181,7 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
   if ((int)blockIdx.x * TC_M >= n_rows) return;
   extern __shared__ uint8_t smem_raw[];
   // operand stages need 1024-byte alignment for the 128-byte swizzle
-  uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t *smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
   const int stage_bytes = p.sps * (TC_A_BYTES + p.b_bytes);   // [sps x gathered slab][sps x filter slab]
   uint8_t *ctrl = smem + (size_t)p.stages * stage_bytes;
   uint64_t *empty_bars = (uint64_t *)ctrl;                 // [stages] slot free (its MMAs retired)
@@ -569,6 +569,71 @@ __device__ __forceinline__ void store_and_arrive(bool on, uint32_t at, uint32_t 
 // GATED: batch norm and gated activation on the way out.  As a pass of its own (ssc_bn_gate_fwd) they read and write
 // every row once more: 164 us of the 12 layers of a backbone, 320 us of 24 with bf16 rows.  A row's gate
 // scalars are evaluated first, a lane per row, into shared memory; the arithmetic is that pass's, so are the bits.
+// The issuing warp of the kernel below: its state and its loop.  Its own chain of instructions is what it takes a step for, so
+// the loop is straight: unrolled over N tiles, no way out of it from the middle, whole slabs with four products and
+// no test between them, and only tables with a row order are asked whether a step has any row (in others nearly all have).  In
+// isolation a step takes 225 cycles like this and took 450 with a loop of N tiles, a vote on the masks, a test before every
+// product and a way out after the wait.  Two steps to a turn take 167, but the kernel's first launch after others then waits
+// 3.5 us longer for instructions and later ones gain nothing.  (1.1 M rows 64 -> 76: 712 -> 690 us, 82 k rows 128 -> 152 bf16
+// 67.3 -> 64.5, 47 k rows 256 -> 304 bf16 119 -> 111, 16 k rows 59.8 -> 55.7.)
+struct RowsIssuer {
+  uint32_t idesc, a_lo0, a_lo, s, par, full0, empty0, d0;
+  const uint32_t *masks;
+  volatile int *abort_flag;
+};
+template <bool F16, int NT, bool SCAN, bool WHOLE>
+__device__ __forceinline__ bool rows_issue_step(RowsIssuer &w, const TcParams &p) {
+  const bool alive = mbar_wait_straight(w.full0 + w.s * 8u, w.par, w.abort_flag);
+  fence_async_smem();                             // the rows other threads' copies left, for the tensor core
+  tc_fence_after();
+  const uint4 off = *(const uint4 *)(w.masks + w.s * 4u);
+  bool any = true;
+  if (SCAN) any = __any_sync(0xffffffffu, (off.x & off.y & off.z & off.w) != 0xffffffffu);
+  if (any) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const uint32_t dn = w.d0 + (uint32_t)(nt * p.tile_n), bn = w.a_lo + (uint32_t)(TC_A_BYTES >> 4) + (uint32_t)nt * ((uint32_t)(p.tile_n * 128) >> 4);
+      if (WHOLE) {
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {
+            if (F16) mma_f16_ss_masked(dn, w.a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, w.idesc, off);
+            else mma_tf32_ss_masked(dn, w.a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, w.idesc, off);
+          }
+        }
+      } else {
+#pragma unroll 1
+        for (int kk = 0; kk < p.last_kk; ++kk)
+          if (elect_one()) {
+            if (F16) mma_f16_ss_masked(dn, w.a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, w.idesc, off);
+            else mma_tf32_ss_masked(dn, w.a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, w.idesc, off);
+          }
+      }
+    }
+  }
+  if (elect_one()) mma_commit(w.empty0 + w.s * 8u);
+  w.a_lo += (uint32_t)(TC_A_BYTES + p.b_bytes) >> 4;
+  if (++w.s == (uint32_t)p.stages) { w.s = 0; w.par ^= 1u; w.a_lo = w.a_lo0; }
+  return alive;
+}
+template <bool F16, int NT, bool SCAN>
+__device__ __forceinline__ void rows_issue_all(RowsIssuer &w, const TcParams &p, int n_act) {
+  const int whole = p.last_kk == 4 ? p.k_slabs : p.k_slabs - 1;   // slabs with four k-steps of real channels (the rest is zero on both sides)
+  bool alive = true;
+  if (whole == p.k_slabs) {
+    const int n = n_act * whole;
+#pragma unroll 1
+    for (int i = 0; i < n && alive; ++i) alive = rows_issue_step<F16, NT, SCAN, true>(w, p);
+  } else {
+#pragma unroll 1
+    for (int a = 0; a < n_act && alive; ++a) {
+#pragma unroll 1
+      for (int i = 0; i < whole; ++i) alive &= rows_issue_step<F16, NT, SCAN, true>(w, p);
+      alive &= rows_issue_step<F16, NT, SCAN, false>(w, p);
+    }
+  }
+}
+
 template <bool F16, bool GATED, int GROUPS>
 __global__ void __launch_bounds__(GROUPS * 128 + 32, GROUPS == 1 ? 4 : 2)
 conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
@@ -585,7 +650,7 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   __shared__ int abort_word, n_act_s;
   volatile int *abort_flag = &abort_word;
   // operand slots need 1024-byte alignment for the 128-byte swizzle
-  uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t *smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
   const int stage_bytes = TC_A_BYTES + p.b_bytes;
   const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
   constexpr int groups = GROUPS, mma_warp = groups * 4;              // producer groups of four warps
@@ -742,45 +807,15 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   } else {
     // ================================ MMA issuer: the whole warp, one elected lane issues ========
     // fp32 accumulator; operand formats: kind::tf32 2 = TF32; kind::f16 0 = fp16, 1 = bf16
+    RowsIssuer w;
     const uint32_t fmt = F16 ? (uint32_t)p.fmt16 : 2u;
-    const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.tile_n >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
-    const uint32_t a_lo0 = desc_lo(smem_base), slot_step = (uint32_t)stage_bytes >> 4, n_step = (uint32_t)(p.tile_n * 128) >> 4;
-    const uint32_t full0 = smem_u32(full_bars), empty0 = smem_u32(empty_bars);
-    uint32_t s = 0, par = 0, a_lo = a_lo0;
-    int slab = 0;
-    bool ready = false;
-    for (int it = 0; it < n_iter; ++it) {
-      if (!ready && !mbar_wait_uniform(full0 + s * 8u, par, abort_flag)) break;
-      fence_async_smem();                         // the rows other threads' copies left, for the tensor core
-      tc_fence_after();
-      const uint4 off = *(const uint4 *)(slot_masks + s * 4u);
-      // k-steps that hold real channels (the rest of the last slab is zero on both sides)
-      const int n_kk = slab == p.k_slabs - 1 ? p.last_kk : 4;
-      const bool any = __any_sync(0xffffffffu, (off.x & off.y & off.z & off.w) != 0xffffffffu);
-      const uint32_t an = a_lo, done = empty0 + s * 8u;
-      a_lo += slot_step;
-      if (++s == (uint32_t)S) { s = 0; par ^= 1u; a_lo = a_lo0; }
-      // A CTA alone on its SM has a deep ring, and this warp's chain of instructions is what bounds a step (440 cycles undisturbed,
-      // whatever the products): the next step's barrier is looked at before this one's products are issued.  (Up to one tile per SM
-      // 1 to 12 % off: 16 k rows 32 -> 38 15.0 -> 14.1 us, 19 k rows 132 -> 136 51.8 -> 45.7.  With more tiles than SMs between -4 and +2 %:
-      // 60 k rows 128 -> 128 bf16 68.6 -> 66.8, 256 -> 304 TF32 405 -> 412.  With two or four CTAs the look comes too early: +1 to 2 %.)
-      const bool passed = GROUPS == 2 && p.ctas == 1 && mbar_test_wait(full0 + s * 8u, par);
-      for (int nt = 0; nt < (any ? p.nt_cta : 0); ++nt) {
-        const uint32_t dn = tmem_base + (uint32_t)(nt * p.tile_n);
-        const uint32_t bn = an + (uint32_t)(TC_A_BYTES >> 4) + (uint32_t)nt * n_step;
-        if (elect_one()) {
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            if (kk >= n_kk) break;
-            if (F16) mma_f16_ss_masked(dn, an + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
-            else mma_tf32_ss_masked(dn, an + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, idesc, off);
-          }
-        }
-      }
-      if (++slab == p.k_slabs) slab = 0;
-      if (elect_one()) mma_commit(done);
-      ready = GROUPS == 2 && __all_sync(0xffffffffu, passed);
-    }
+    w.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.tile_n >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+    w.a_lo = w.a_lo0 = desc_lo(smem_base);
+    w.s = w.par = 0;
+    w.full0 = smem_u32(full_bars); w.empty0 = smem_u32(empty_bars);
+    w.masks = slot_masks; w.d0 = tmem_base; w.abort_flag = abort_flag;
+    if (p.nt_cta == 1) { if (scan) rows_issue_all<F16, 1, true>(w, p, n_act); else rows_issue_all<F16, 1, false>(w, p, n_act); }
+    else { if (scan) rows_issue_all<F16, 2, true>(w, p, n_act); else rows_issue_all<F16, 2, false>(w, p, n_act); }
     if (elect_one()) mma_commit(smem_u32(&done_bar));   // arrives once everything issued above has retired
   }
 

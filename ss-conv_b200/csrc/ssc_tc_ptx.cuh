@@ -102,6 +102,15 @@ __device__ __forceinline__ bool mbar_wait_uniform(uint32_t bar, uint32_t parity,
   *abort_flag = 1;
   return false;
 }
+// The same for a loop without a way out in the middle, which costs the issuing warp more than the wait itself: after a wait has
+// failed the next ones look once and fail too.
+__device__ __forceinline__ bool mbar_wait_straight(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+  uint32_t i = 0;
+  bool ok;
+  do { ok = __all_sync(0xffffffffu, mbar_try_wait(bar, parity)); } while (!ok && ++i < kSpinLimit && ((i & 255u) != 255u || !__any_sync(0xffffffffu, *abort_flag)));
+  if (!ok) *abort_flag = 1;
+  return ok;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
