@@ -39,8 +39,7 @@ __device__ __forceinline__ void gate_scalars(Load load, const GateEpilogue &gate
         if (gate.scale) v[i] = fmaf(v[i], k.x, k.y);
       }
       if (gate.gate_act == 2) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = apply_act(v[i], 2);
+        apply_sigmoids<8>(v);
       } else if (gate.gate_act == 1) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = apply_act(v[i], 1);
@@ -60,10 +59,12 @@ __device__ __forceinline__ void block_from_columns(float *blk, const uint32_t *r
 }
 
 // Finished rows, 32 columns at first, first + step, ...  gates: of this quarter, and a last line of ones.  row0: the quarter's
-// first row; whole: the tile is full, in its own order and its rows are stored as vectors.
+// first row; whole: the tile is full, in its own order and its rows are stored as vectors; else m: this lane's row of `out`, -1 for none.
+// The columns that hold scalars, nearly always the first 32, go the same way as the others with a relu on top: by the general way, one
+// pair of rows after the other, they took 4600 cycles of a tile's way out and now take 1000.
 template <class Load>
-__device__ __forceinline__ void store_gated(Load load, const GateEpilogue &gate, const float4 *chan, const float *gates, float *blk, float *out, int c_out, int row0,
-                                            int n_rows, const int32_t *order, bool whole, bool vec, int lane, int first, int step) {
+__device__ __forceinline__ void store_gated(Load load, const GateEpilogue &gate, const float4 *chan, const float *gates, float *blk, float *out, int c_out, int row0, int m,
+                                            bool whole, bool vec, int lane, int first, int step) {
   const int c_row = gate.c_keep, n_gates = c_out - c_row;
   const bool affine = gate.scale != nullptr;
   for (int c0 = first; c0 < c_row; c0 += step) {
@@ -87,54 +88,60 @@ __device__ __forceinline__ void store_gated(Load load, const GateEpilogue &gate,
       scalar[j] = g == -1;
       gp[j] = gates + (g >= 0 ? g : n_gates) * 33 + row4;
     }
-    const bool scalars = __any_sync(0xffffffffu, scalar[0] || scalar[1] || scalar[2] || scalar[3]) && gate.scalar_act != 0;
-    if (col >= c_row) continue;
+    const bool scalars = gate.scalar_act != 0 && __any_sync(0xffffffffu, scalar[0] || scalar[1] || scalar[2] || scalar[3]);
     // rows 4 i + row4 of the warp's 32: the swizzle of even and odd i, the rest are constants
     const float *even = blk + row4 * 32 + ((q ^ row4) << 2), *odd = blk + row4 * 32 + ((q ^ row4 ^ 4) << 2);
-    auto finished = [&](int i, bool act) {
+    auto finished = [&](int i, int act) {         // act: 0 no scalar among the columns, 1 relu, 2 whatever it is
       const float4 x = *(const float4 *)((i & 1 ? odd : even) + i * 128);
       float v[4] = {x.x, x.y, x.z, x.w};
       if (affine) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[j] = fmaf(v[j], sc[j], sh[j]);
       }
-      if (act) {
+      if (act == 1) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = scalar[j] && !(v[j] > 0.f) ? 0.f : v[j];
+      } else if (act == 2) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           if (scalar[j]) v[j] = apply_act(v[j], gate.scalar_act);
       }
       return make_float4(v[0] * gp[0][4 * i], v[1] * gp[1][4 * i], v[2] * gp[2][4 * i], v[3] * gp[3][4 * i]);
     };
-    const int my_row0 = row0 + row4;
-    if (!scalars && whole && gate.out16 == 0) {          // most columns of most tiles
-      float *to = out + (size_t)my_row0 * c_row + col;
+    auto packed = [&](float4 v) {
+      return gate.out16 == 2 ? make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w)) : make_uint2(pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w));
+    };
+    if (whole && (!scalars || gate.scalar_act == 1)) {   // most tiles
+      if (col >= c_row) continue;
+      const size_t at = (size_t)(row0 + row4) * c_row + col;
+      if (gate.out16 == 0) {
+        float *to = out + at;
+        if (!scalars) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i, to += 4 * c_row) *(float4 *)to = finished(i, false);
-    } else if (!scalars && whole) {
-      uint16_t *to = (uint16_t *)out + (size_t)my_row0 * c_row + col;
-      if (gate.out16 == 2) {
+          for (int i = 0; i < 8; ++i, to += 4 * c_row) *(float4 *)to = finished(i, 0);
+        } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i, to += 4 * c_row) {
-          const float4 v = finished(i, false);
-          *(uint2 *)to = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+          for (int i = 0; i < 8; ++i, to += 4 * c_row) *(float4 *)to = finished(i, 1);
         }
       } else {
+        uint16_t *to = (uint16_t *)out + at;
+        if (!scalars) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i, to += 4 * c_row) {
-          const float4 v = finished(i, false);
-          *(uint2 *)to = make_uint2(pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w));
+          for (int i = 0; i < 8; ++i, to += 4 * c_row) *(uint2 *)to = packed(finished(i, 0));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i, to += 4 * c_row) *(uint2 *)to = packed(finished(i, 1));
         }
       }
     } else {
 #pragma unroll 2
       for (int i = 0; i < 8; ++i) {
-        const int at_row = my_row0 + 4 * i;
-        const float4 v = finished(i, scalars);
-        if (at_row >= n_rows) continue;
-        const size_t at = (size_t)(order ? __ldg(order + at_row) : at_row) * c_row + col;
+        const int to = __shfl_sync(0xffffffffu, m, 4 * i + row4);
+        if (to < 0 || col >= c_row) continue;
+        const float4 v = finished(i, scalars ? 2 : 0);
+        const size_t at = (size_t)to * c_row + col;
         if (gate.out16 != 0) {                    // c_row is a multiple of eight
-          *(uint2 *)((uint16_t *)out + at) = gate.out16 == 2 ? make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w))
-                                                            : make_uint2(pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w));
+          *(uint2 *)((uint16_t *)out + at) = packed(v);
         } else if (vec) {
           *(float4 *)(out + at) = v;
         } else {

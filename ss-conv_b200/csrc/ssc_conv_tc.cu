@@ -849,6 +849,7 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
     float *blk = (float *)(smem + (size_t)warp * 4096u);
     const int c_row = GATED ? gate.c_keep : c_out;          // channels of a stored row
     const bool vec = (c_row & 3) == 0 && ((uintptr_t)out & 15u) == 0;
+    const int m = m_tile < n_rows ? (order ? __ldg(order + m_tile) : m_tile) : -1;   // this lane's row of `out`
     if (GATED) {                                  // one CTA has all channels
       float4 *chan = (float4 *)(smem + (size_t)groups * 4u * 4096u);   // [c_out]
       // act(gate g) of row r of the quarter at g * 33 + r, and a last line of ones
@@ -863,9 +864,8 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
       if (group == 0) gates[n_gates * 33 + lane] = 1.f;
       gate_scalars(load16, gate, chan, gates, c_out, lane, (c_row & ~15) + 16 * group, 16 * groups);
       asm volatile("bar.sync 1, %0;" ::"r"(groups * 128) : "memory");
-      store_gated(load16, gate, chan, gates, blk, out, c_out, m0 + quarter * 32, n_rows, order, whole, vec, lane, 32 * group, 32 * groups);
+      store_gated(load16, gate, chan, gates, blk, out, c_out, m0 + quarter * 32, m, whole, vec, lane, 32 * group, 32 * groups);
     } else {
-      const int m = m_tile < n_rows ? (order ? __ldg(order + m_tile) : m_tile) : -1;
       store_plain(load16, blk, out, m, col0, p.n_cta, c_row, vec, lane, 32 * group, 32 * groups);
     }
   }

@@ -435,6 +435,27 @@ def test_gated_convolution_has_the_bits_of_the_two_passes(cuda, c_in, c_out, c_k
         assert torch.equal(_ext.conv_forward(feats, W, nbr, n, precision, row_order=order, gate=(scale, shift, table, c_keep, 1, 2)), want)
 
 
+@pytest.mark.parametrize("scalar_act", [0, 1, 2])
+def test_gated_convolution_at_the_ends_of_the_activations(cuda, scalar_act):
+    """Gates far out on both sides, where the sigmoid's denominator is beyond every quick reciprocal, zeros of both
+    signs, infinities and NaN, in whole tiles and in a part of one: the bits of the gate pass."""
+    from ss_conv import _ext
+    n, c_out, keep = 300, 46, 32
+    x = torch.randn(n, 32, device=cuda)
+    W = torch.zeros(1, 32, c_out, device=cuda)
+    W[0, torch.arange(32), torch.arange(32)] = 1.0        # channel c is x[:, c] rounded to TF32; the gates come from the shift
+    ends = [-200.0, -126.5, -104.0, -88.8, -88.0, -87.4, -87.3, -86.7, -1e-30, 0.0, 17.0, 90.0, float("inf"), float("nan")]
+    scale, shift = torch.ones(c_out, device=cuda), torch.zeros(c_out, device=cuda)
+    shift[keep:] = torch.tensor(ends, device=cuda)
+    x[1::7, :3], x[2::7, :3], x[3::7, 1] = -0.0, float("-inf"), float("nan")
+    table = torch.where(torch.arange(keep, device=cuda) < 3, -1, torch.arange(keep, device=cuda) % len(ends)).to(torch.int32)
+    nbr = torch.arange(n, dtype=torch.int32, device=cuda).view(1, n)
+    got = _ext.conv_forward(x, W, nbr, n, "tf32", gate=(scale, shift, table, keep, scalar_act, 2))
+    want = _ext.bn_gate_forward(_ext.conv_forward(x, W, nbr, n, "tf32"), scale, shift, table, keep, keep, scalar_act, 2, None, None)
+    _ext.check_status(cuda)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+
+
 @pytest.mark.parametrize("n,batch", [(0, 1), (1, 3), (1025, 1024), (16384, 4096), (16385, 7), (300, 4097)])
 def test_batch_offsets_at_the_sizes_of_the_one_block_form(cuda, n, batch):
     """Rows in any order, samples without rows, ids outside the batch (counted nowhere): a plain histogram's prefix."""
