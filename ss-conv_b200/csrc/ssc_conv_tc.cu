@@ -20,6 +20,7 @@
 // through a shared flag, every other wait then gives up too, and the kernel frees its tensor
 // memory and returns.
 #include "ssc_conv_epilogue.cuh"
+#include <type_traits>
 
 namespace ssc {
 
@@ -50,12 +51,14 @@ struct TcParams {
   int opk;        // kernel offsets per 128-byte operand row: 1, or 32 / c_pad for TF32 layers with c_pad = 4, 8, 16
   int rev;        // 1: the table's row of kernel offset kappa is K - 1 - kappa (the transpose of a centred submanifold table)
   int32_t *alarm; // mapped host word that tells of an expired wait (may be NULL)
+  int pair;       // 1: two CTAs with 128 rows each share the filter slabs (half a slab in each) and the products
   int nbr_by_pos; // 1: the table's columns are already in the order of `order` (column j <-> output row order[j])
                   // channels (a first layer with 3 input channels packs 8 offsets into one step)
 };
 
 // Shared-memory plan: [stages x (A 16 KB + B)] [control 1 KB].
-static bool tc_params(int c_in, int c_out, TcParams &p, bool split_n = false, bool one_cta_per_sm = false, int opk = 1) {
+static bool tc_params(int c_in, int c_out, TcParams &p, bool split_n = false, int max_ctas = 4, int opk = 1, bool pair = false) {
+  p.pair = pair;
   p.k_slabs = (c_in + TC_SLAB - 1) / TC_SLAB;
   p.last_kk = (c_in - (p.k_slabs - 1) * TC_SLAB + 7) / 8;     // c_in counts 4-byte words of an operand row
   p.opk = opk;
@@ -83,16 +86,15 @@ static bool tc_params(int c_in, int c_out, TcParams &p, bool split_n = false, bo
   p.sps = 1;
   p.fmt16 = 0;
   p.k_groups = (p.k_slabs + p.sps - 1) / p.sps;
-  int stage = p.sps * (TC_A_BYTES + p.b_bytes);
+  int stage = p.sps * (TC_A_BYTES + (pair ? p.b_bytes / 2 : p.b_bytes));
   // behind the slots: control block, alignment slack
   int fixed = TC_CTRL_BYTES + 1024;
   // Resident CTAs hide each other's per-step latencies, so take as many per SM as tensor
-  // memory (512 columns) and shared memory (two ring slots each at least) allow, up to four.
-  // A launch with no more CTAs than SMs has nobody to share an SM with: all of the shared memory
-  // goes into ring slots (a deeper pipeline is what a lone CTA has against the latency of a step).
+  // memory (512 columns) and shared memory (two ring slots each at least) allow, up to four and to as many as the launch has for an
+  // SM: what is left of the shared memory goes into ring slots (a deeper pipeline is what few CTAs have against the latency of a step).
   int ctas = 512 / p.tmem_cols;
   if (ctas > 4) ctas = 4;
-  if (one_cta_per_sm) ctas = 1;
+  if (ctas > max_ctas) ctas = max_ctas;
   while (ctas > 1 && ((227 * 1024) / ctas - 1024 - fixed) / stage < 2) --ctas;
   p.stages = ((227 * 1024) / ctas - 1024 - fixed) / stage;
   if (p.stages > TC_MAX_STAGES) p.stages = TC_MAX_STAGES;
@@ -549,6 +551,78 @@ __device__ __forceinline__ void store_and_arrive(bool on, uint32_t at, uint32_t 
       : "memory");
 }
 
+// The issuing warp of the kernel below: its state and its loop.  Its own chain of instructions is what it takes a step for, so
+// the loop is straight: unrolled over N tiles, no way out of it from the middle, whole slabs with four products and
+// no test between them, and only tables with a row order are asked whether a step has any row (in others nearly all have).  In
+// isolation a step takes 225 cycles like this and took 450 with a loop of N tiles, a vote on the masks, a test before every
+// product and a way out after the wait.  Two steps to a turn take 167, but the kernel's first launch after others then waits
+// 3.5 us longer for instructions and later ones gain nothing.  (1.1 M rows 64 -> 76: 712 -> 690 us, 82 k rows 128 -> 152 bf16
+// 67.3 -> 64.5, 47 k rows 256 -> 304 bf16 119 -> 111, 16 k rows 59.8 -> 55.7.)
+struct RowsIssuer {
+  uint32_t idesc, a_lo0, a_lo, s, par, full0, empty0, d0, b_bytes;
+  const uint32_t *masks;      // [slots][4], with a pair of CTAs [slots][8]
+  volatile int *abort_flag;
+};
+template <bool PAIR>
+__device__ __forceinline__ void rows_commit(uint32_t bar) {
+  if (PAIR) mma_commit_pair(bar);
+  else mma_commit(bar);
+}
+template <bool F16, bool PAIR>
+__device__ __forceinline__ void rows_mma(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint4 off, uint4 off2) {
+  if (PAIR) mma_pair_masked<F16>(d, a_lo, b_lo, idesc, off, off2);
+  else if (F16) mma_f16_ss_masked(d, a_lo, b_lo, idesc, off);
+  else mma_tf32_ss_masked(d, a_lo, b_lo, idesc, off);
+}
+template <bool F16, int NT, bool SCAN, bool WHOLE, bool PAIR>
+__device__ __forceinline__ bool rows_issue_step(RowsIssuer &w, const TcParams &p) {
+  const bool alive = PAIR ? mbar_wait_straight_cluster(w.full0 + w.s * 8u, w.par, w.abort_flag) : mbar_wait_straight(w.full0 + w.s * 8u, w.par, w.abort_flag);
+  fence_async_smem();                             // the rows other threads' copies left, for the tensor core
+  tc_fence_after();
+  const uint4 off = *(const uint4 *)(w.masks + w.s * (PAIR ? 8u : 4u));
+  uint4 off2 = off;
+  if (PAIR) off2 = *(const uint4 *)(w.masks + w.s * 8u + 4u);
+  bool any = true;
+  if (SCAN) any = __any_sync(0xffffffffu, (off.x & off.y & off.z & off.w) != 0xffffffffu);
+  if (any) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const uint32_t dn = w.d0 + (uint32_t)(nt * p.tile_n), bn = w.a_lo + (uint32_t)(TC_A_BYTES >> 4) + (uint32_t)nt * ((uint32_t)(p.tile_n * (PAIR ? 64 : 128)) >> 4);
+      if (WHOLE) {
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) rows_mma<F16, PAIR>(dn, w.a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, w.idesc, off, off2);
+        }
+      } else {
+#pragma unroll 1
+        for (int kk = 0; kk < p.last_kk; ++kk)
+          if (elect_one()) rows_mma<F16, PAIR>(dn, w.a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, w.idesc, off, off2);
+      }
+    }
+  }
+  if (elect_one()) rows_commit<PAIR>(w.empty0 + w.s * 8u);
+  w.a_lo += (uint32_t)(TC_A_BYTES + w.b_bytes) >> 4;
+  if (++w.s == (uint32_t)p.stages) { w.s = 0; w.par ^= 1u; w.a_lo = w.a_lo0; }
+  return alive;
+}
+template <bool F16, int NT, bool SCAN, bool PAIR>
+__device__ __forceinline__ void rows_issue_all(RowsIssuer &w, const TcParams &p, int n_act) {
+  const int whole = p.last_kk == 4 ? p.k_slabs : p.k_slabs - 1;   // slabs with four k-steps of real channels (the rest is zero on both sides)
+  bool alive = true;
+  if (whole == p.k_slabs) {
+    const int n = n_act * whole;
+#pragma unroll 1
+    for (int i = 0; i < n && alive; ++i) alive = rows_issue_step<F16, NT, SCAN, true, PAIR>(w, p);
+  } else {
+#pragma unroll 1
+    for (int a = 0; a < n_act && alive; ++a) {
+#pragma unroll 1
+      for (int i = 0; i < whole; ++i) alive &= rows_issue_step<F16, NT, SCAN, true, PAIR>(w, p);
+      alive &= rows_issue_step<F16, NT, SCAN, false, PAIR>(w, p);
+    }
+  }
+}
+
 // The kernel for staged operands (TF32-rounded fp32 rows, or fp16 / bf16 rows: F16), one kernel offset and one
 // 128-byte slab per step.  GROUPS of four warps produce, a lane per output row of the tile (and run the epilogue); two
 // groups fill every other slot each.  The last warp issues the MMAs.
@@ -562,88 +636,29 @@ __device__ __forceinline__ void store_and_arrive(bool on, uint32_t at, uint32_t 
 //   * nobody waits for copies: the copies' completion arrives on the slot's barrier by itself
 //     (cp.async.mbarrier.arrive.noinc), the warps go on to the next free slot, and the issuing warp orders
 //     the landed rows for the tensor core (fence.proxy.async behind the barrier);
-//   * table entries are loaded two offsets ahead.
+//   * table entries are loaded two offsets ahead, and whole slabs of a row are copied at constants from one address.
 // Sums are accumulated in the order of the steps (ascending offset, ascending slab), whatever the tile's
 // other rows need.
 //
 // GATED: batch norm and gated activation on the way out.  As a pass of its own (ssc_bn_gate_fwd) they read and write
 // every row once more: 164 us of the 12 layers of a backbone, 320 us of 24 with bf16 rows.  A row's gate
 // scalars are evaluated first, a lane per row, into shared memory; the arithmetic is that pass's, so are the bits.
-// The issuing warp of the kernel below: its state and its loop.  Its own chain of instructions is what it takes a step for, so
-// the loop is straight: unrolled over N tiles, no way out of it from the middle, whole slabs with four products and
-// no test between them, and only tables with a row order are asked whether a step has any row (in others nearly all have).  In
-// isolation a step takes 225 cycles like this and took 450 with a loop of N tiles, a vote on the masks, a test before every
-// product and a way out after the wait.  Two steps to a turn take 167, but the kernel's first launch after others then waits
-// 3.5 us longer for instructions and later ones gain nothing.  (1.1 M rows 64 -> 76: 712 -> 690 us, 82 k rows 128 -> 152 bf16
-// 67.3 -> 64.5, 47 k rows 256 -> 304 bf16 119 -> 111, 16 k rows 59.8 -> 55.7.)
-struct RowsIssuer {
-  uint32_t idesc, a_lo0, a_lo, s, par, full0, empty0, d0;
-  const uint32_t *masks;
-  volatile int *abort_flag;
-};
-template <bool F16, int NT, bool SCAN, bool WHOLE>
-__device__ __forceinline__ bool rows_issue_step(RowsIssuer &w, const TcParams &p) {
-  const bool alive = mbar_wait_straight(w.full0 + w.s * 8u, w.par, w.abort_flag);
-  fence_async_smem();                             // the rows other threads' copies left, for the tensor core
-  tc_fence_after();
-  const uint4 off = *(const uint4 *)(w.masks + w.s * 4u);
-  bool any = true;
-  if (SCAN) any = __any_sync(0xffffffffu, (off.x & off.y & off.z & off.w) != 0xffffffffu);
-  if (any) {
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const uint32_t dn = w.d0 + (uint32_t)(nt * p.tile_n), bn = w.a_lo + (uint32_t)(TC_A_BYTES >> 4) + (uint32_t)nt * ((uint32_t)(p.tile_n * 128) >> 4);
-      if (WHOLE) {
-        if (elect_one()) {
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            if (F16) mma_f16_ss_masked(dn, w.a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, w.idesc, off);
-            else mma_tf32_ss_masked(dn, w.a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, w.idesc, off);
-          }
-        }
-      } else {
-#pragma unroll 1
-        for (int kk = 0; kk < p.last_kk; ++kk)
-          if (elect_one()) {
-            if (F16) mma_f16_ss_masked(dn, w.a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, w.idesc, off);
-            else mma_tf32_ss_masked(dn, w.a_lo + 2u * (uint32_t)kk, bn + 2u * (uint32_t)kk, w.idesc, off);
-          }
-      }
-    }
-  }
-  if (elect_one()) mma_commit(w.empty0 + w.s * 8u);
-  w.a_lo += (uint32_t)(TC_A_BYTES + p.b_bytes) >> 4;
-  if (++w.s == (uint32_t)p.stages) { w.s = 0; w.par ^= 1u; w.a_lo = w.a_lo0; }
-  return alive;
-}
-template <bool F16, int NT, bool SCAN>
-__device__ __forceinline__ void rows_issue_all(RowsIssuer &w, const TcParams &p, int n_act) {
-  const int whole = p.last_kk == 4 ? p.k_slabs : p.k_slabs - 1;   // slabs with four k-steps of real channels (the rest is zero on both sides)
-  bool alive = true;
-  if (whole == p.k_slabs) {
-    const int n = n_act * whole;
-#pragma unroll 1
-    for (int i = 0; i < n && alive; ++i) alive = rows_issue_step<F16, NT, SCAN, true>(w, p);
-  } else {
-#pragma unroll 1
-    for (int a = 0; a < n_act && alive; ++a) {
-#pragma unroll 1
-      for (int i = 0; i < whole; ++i) alive &= rows_issue_step<F16, NT, SCAN, true>(w, p);
-      alive &= rows_issue_step<F16, NT, SCAN, false>(w, p);
-    }
-  }
-}
-
-template <bool F16, bool GATED, int GROUPS>
-__global__ void __launch_bounds__(GROUPS * 128 + 32, GROUPS == 1 ? 4 : 2)
-conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
-                     const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out, int32_t *status, TcParams p,
-                     const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order, GateEpilogue gate) {
+//
+// PAIR: two CTAs of a cluster, 128 rows each, as one product of 256 rows (cta_group::2).  Every tile brings in the whole filter image, and
+// that is most of what its steps move (10 of 14 KB for 64 -> 76 channels, 20 of 26 for 152); of a pair each holds half of a slab.
+// CTA 0 issues for both.  A slot of CTA 1 is full on a barrier there; its last warp passes that on, with the row masks, by one
+// asynchronous store that counts on CTA 0's barrier (a store and a released arrival one after the other: 2100 cycles a step).
+template <bool F16, bool GATED, int GROUPS, bool PAIR>
+__device__ __forceinline__ void
+conv_fwd_rows(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
+              const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out, int32_t *status, const TcParams &p,
+              const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order, const GateEpilogue &gate) {
   const int n_rows = live_rows(n_out, n_out_dev);
-  if ((int)blockIdx.x * TC_M >= n_rows) return;
+  if ((int)(PAIR ? blockIdx.x & ~1u : blockIdx.x) * TC_M >= n_rows) return;
+  const int rank = PAIR ? (int)blockIdx.x & 1 : 0;                   // in the pair: 0 issues for both
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t empty_bars[TC_MAX_STAGES], full_bars[TC_MAX_STAGES], done_bar;
-  __shared__ __align__(16) uint32_t slot_masks[TC_MAX_STAGES * 4];   // rows of the slot's step WITHOUT a neighbour
+  __shared__ __align__(16) uint32_t slot_masks[TC_MAX_STAGES * (PAIR ? 8 : 4)];   // rows of the slot's step WITHOUT a neighbour
   __shared__ uint32_t act_bits[8];
   __shared__ uint8_t act_list[256];
   __shared__ uint32_t tmem_slot;
@@ -651,7 +666,8 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   volatile int *abort_flag = &abort_word;
   // operand slots need 1024-byte alignment for the 128-byte swizzle
   uint8_t *smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
-  const int stage_bytes = TC_A_BYTES + p.b_bytes;
+  const int b_bytes = PAIR ? p.b_bytes >> 1 : p.b_bytes;             // (a pair's filter slab lies half in each)
+  const int stage_bytes = TC_A_BYTES + b_bytes;
   const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
   constexpr int groups = GROUPS, mma_warp = groups * 4;              // producer groups of four warps
   const int quarter = warp & 3;                                      // the 32 rows of the tile a producer warp works on
@@ -662,18 +678,24 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   // table is scanned for them first.  In any other order nearly every offset has a row among 128, the
   // scan (8 us when all CTAs of the first wave do it at once) finds nothing, and a step without a
   // row costs its filter copy but no multiplication.
-  const bool scan = order != nullptr;
+  const bool scan = !PAIR && order != nullptr;
   const int m_tile = m0 + quarter * 32 + lane;    // (producers) this lane's row of the tile
   int my_row = -1;                                // its column of the table
   if (warp == mma_warp) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)p.tmem_cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)p.tmem_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)p.tmem_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   } else {
     if (tid < 8) act_bits[tid] = 0u;
     if (tid == 32) {
       for (int s = 0; s < S; ++s) {
         mbar_init(smem_u32(empty_bars + s), 1);
-        // 128 arrivals by copies, one per warp for the row mask, one for the filter copy's byte count
+        // 128 arrivals by copies, one per warp for the row mask, one for the filter copy's byte count; in the
+        // issuing CTA of a pair one that tells of all these in the other
         mbar_init(smem_u32(full_bars + s), 128 + 4 + 1);
       }
       mbar_init(smem_u32(&done_bar), 1);
@@ -726,6 +748,7 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();                       // the other CTA's barriers stand and its accumulators are clear
   tc_fence_after();
   const int n_act = scan ? n_act_s : K, n_iter = n_act * p.k_slabs;
   const uint32_t smem_base = smem_u32(smem);
@@ -740,83 +763,129 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
     // means step it - 2 S, which came no later as long as there are two slots.
     const int sub = lane & 3, row8 = lane >> 2, group = warp >> 2;
     const uint32_t warp_rows = smem_base + (uint32_t)quarter * 4096u + (uint32_t)row8 * 128u;   // row of the warp's first 8-row group
-    const uint32_t first0 = warp_rows + (((uint32_t)sub ^ (uint32_t)row8) << 4), first1 = warp_rows + (((uint32_t)(sub + 4) ^ (uint32_t)row8) << 4);
+    const uint32_t first0 = warp_rows + (((uint32_t)sub ^ (uint32_t)row8) << 4);                // (its second piece: bit 6 the other way)
     const uint32_t full0 = smem_u32(full_bars), empty0 = smem_u32(empty_bars), masks0 = smem_u32(slot_masks + quarter);
+    constexpr uint32_t mask_step = PAIR ? 32u : 16u;
     const uint32_t b_to = smem_base + (uint32_t)TC_A_BYTES, row_bytes = (uint32_t)row_words * 4u;
     const char *lane_rows = (const char *)features + sub * 16;
     const char *b_from = (const char *)packed + (size_t)nt0 * (size_t)(p.tile_n * 128);
     const bool in_rows = my_row >= 0, lead = lane == 0;
     const int32_t *my_entries = nbr + (p.rev ? (size_t)(K - 1) * n_out : 0) + max(my_row, 0);
     const int k_slabs = p.k_slabs, offset_step = p.rev ? -n_out : n_out, last = n_act - 1;
-    auto offset_of = [&](int a) { return scan ? (int)act_list[a] : a; };
-    auto entry = [&](int a) {                     // (past the last offset: anything, it is not used)
-      const int v = __ldg(my_entries + (long long)offset_of(min(a, last)) * offset_step);
-      return in_rows ? v : -1;
+    const int a_step = GROUPS == 2 && k_slabs == 1 ? 2 : 1;           // a group's offsets
+    const int whole = row_words / TC_SLAB;                            // slabs that a row fills
+    // A table entry is loaded into the register it is used from, two offsets ahead (handed on from one to another it would be
+    // waited for at once: with two groups 600 of a step's 1100 cycles).
+    int a = a_step == 2 ? group : 0, asked = a;
+    const long long entry_step = (long long)offset_step * a_step;
+    const int32_t *ent = my_entries + (long long)min(a, max(last, 0)) * offset_step;
+    auto next_entry = [&]() {                     // (past the last offset: that one again, not used)
+      if (scan) ent = my_entries + (long long)act_list[min(asked, last)] * offset_step;
+      const int v = __ldg(ent);
+      asked += a_step;
+      if (!scan && asked <= last) ent += entry_step;
+      return v;
     };
-    // a group's offsets and, of each, its slabs
-    const int a_step = groups == 2 && k_slabs == 1 ? 2 : 1;
-    int src = -1, nxt = -1, a = a_step == 2 ? group : 0;
-    if (n_act > 0) { src = entry(a); nxt = entry(a + a_step); }
-    int slot = group;                             // (two slots at least)
-    uint32_t par = 1;                             // parity the slot's "empty" barrier has to have passed (first uses: none)
+    uint32_t slot = (uint32_t)group, par = 1u;    // (two slots at least); parity the slot's "empty" barrier has to have passed (a fresh one: has)
     bool alive = true;
-#pragma unroll 1
-    for (; a < n_act && alive; a += a_step) {
-      const int after = entry(a + 2 * a_step);
-      const unsigned have = __ballot_sync(0xffffffffu, src >= 0);
-      int from[4];
+    uint32_t lost = 0u;                           // rows of the warp without a neighbour
+    int from[4];
+    const char *at[4];
+    auto turn = [&](auto piece, int kappa, int slab) {
+      alive = mbar_wait_straight(empty0 + slot * 8u, par, abort_flag);
+      const uint32_t full = full0 + slot * 8u, slot_off = slot * (uint32_t)stage_bytes, dst0 = first0 + slot_off, dst1 = dst0 ^ 64u;
+      if (quarter == 0 && elect_one()) {          // the pre-packed filter slab of this step
+        mbar_expect_tx(full, (uint32_t)b_bytes + (PAIR && rank == 0 ? 16u : 0u));   // (and the other CTA's masks)
+        const char *from_slab = b_from + (size_t)(uint32_t)(kappa * k_slabs + slab) * (uint32_t)(p.n_pad * 128);
+        if (PAIR) {                               // this CTA's half of every N tile
+          const uint32_t half = (uint32_t)p.tile_n * 64u;
+          for (int nt = 0; nt < p.nt_cta; ++nt) bulk_g2s(b_to + slot_off + (uint32_t)nt * half, from_slab + (uint32_t)(2 * nt + rank) * half, half, full);
+        } else {
+          bulk_g2s(b_to + slot_off, from_slab, (uint32_t)b_bytes, full);
+        }
+      }
+      if constexpr (decltype(piece)::value >= 0) {
+        copy_rows<decltype(piece)::value>(from, at, dst0, dst1);
+      } else {                                    // the last slab of a row that does not fill it
+        const char *base = lane_rows + slab * 128;
+        const int words = row_words - slab * TC_SLAB - sub * 4;       // from this lane's first piece to the row's end
+        const uint32_t bytes0 = words > 0 ? 16u : 0u, bytes1 = words > 16 ? 16u : 0u;
+        const char *base0 = bytes0 ? base : (const char *)features, *base1 = bytes1 ? base + 64 : (const char *)features;
+        const uint32_t stride0 = bytes0 ? row_bytes : 0u, stride1 = bytes1 ? row_bytes : 0u;
+        copy_row_ends<0>(from[0], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
+        copy_row_ends<1024>(from[1], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
+        copy_row_ends<2048>(from[2], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
+        copy_row_ends<3072>(from[3], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
+      store_and_arrive(lead, masks0 + slot * mask_step, lost, full);
+      slot += GROUPS;
+      if (slot >= (uint32_t)S) { slot -= (uint32_t)S; par ^= 1u; }
+    };
+    auto offset = [&](int &e) {                   // the group's slabs of the next of its offsets
+      const int src = in_rows ? e : -1;
+      lost = ~__ballot_sync(0xffffffffu, src >= 0);
 #pragma unroll
       for (int i = 0; i < 4; ++i) from[i] = __shfl_sync(0xffffffffu, src, i * 8 + row8);
-      const int kappa = offset_of(a);
+      e = next_entry();
+      const int kappa = scan ? (int)act_list[a] : a;
 #pragma unroll 1
-      for (int slab = groups == 1 || a_step == 2 ? 0 : (group ^ (a & k_slabs)) & 1; slab < k_slabs; slab += groups) {
-        const uint32_t full = full0 + (uint32_t)slot * 8u, slot_off = (uint32_t)slot * (uint32_t)stage_bytes;
-        const char *base = lane_rows + slab * 128, *at[4];      // (ready before the slot is: nothing but the copies behind the wait)
+      for (int slab = GROUPS == 1 || a_step == 2 ? 0 : (group ^ (a & k_slabs)) & 1; slab < whole; slab += 2) {
+        const char *base = lane_rows + slab * 128;
 #pragma unroll
         for (int i = 0; i < 4; ++i) at[i] = base + (unsigned long long)(uint32_t)from[i] * row_bytes;
-        if (a * k_slabs + slab >= S && !mbar_wait_uniform(empty0 + (uint32_t)slot * 8u, par, abort_flag)) { alive = false; break; }
-        if (quarter == 0 && elect_one()) {        // the pre-packed filter slab of this step: one bulk copy
-          mbar_expect_tx(full, (uint32_t)p.b_bytes);
-          bulk_g2s(b_to + slot_off, b_from + (size_t)(uint32_t)(kappa * k_slabs + slab) * (uint32_t)(p.n_pad * 128), (uint32_t)p.b_bytes, full);
-        }
-        const uint32_t dst0 = first0 + slot_off, dst1 = first1 + slot_off;
-        if ((slab + 1) * TC_SLAB <= row_words) {
-          copy_row_pieces<0>(from[0], dst0, dst1, at[0]);
-          copy_row_pieces<1024>(from[1], dst0, dst1, at[1]);
-          copy_row_pieces<2048>(from[2], dst0, dst1, at[2]);
-          copy_row_pieces<3072>(from[3], dst0, dst1, at[3]);
-        } else {                                  // the last slab of a row that does not fill it
-          const int words = row_words - slab * TC_SLAB - sub * 4;   // from this lane's first piece to the row's end
-          const uint32_t bytes0 = words > 0 ? 16u : 0u, bytes1 = words > 16 ? 16u : 0u;
-          const char *base0 = bytes0 ? base : (const char *)features, *base1 = bytes1 ? base + 64 : (const char *)features;
-          const uint32_t stride0 = bytes0 ? row_bytes : 0u, stride1 = bytes1 ? row_bytes : 0u;
-          copy_row_ends<0>(from[0], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
-          copy_row_ends<1024>(from[1], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
-          copy_row_ends<2048>(from[2], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
-          copy_row_ends<3072>(from[3], dst0, dst1, base0, stride0, bytes0, base1, stride1, bytes1);
-        }
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
-        store_and_arrive(lead, masks0 + (uint32_t)slot * 16u, ~have, full);
-        slot += groups;
-        if (slot >= S) { slot -= S; par ^= 1u; }
+        turn(std::integral_constant<int, 0>{}, kappa, slab);
+        if (GROUPS == 1 && slab + 1 < whole) turn(std::integral_constant<int, 128>{}, kappa, slab + 1);
       }
-      src = nxt;
-      nxt = after;
+      // (of two groups the one whose turn it is)
+      if (whole < k_slabs && (GROUPS == 1 || a_step == 2 || ((group ^ (a & k_slabs) ^ whole) & 1) == 0)) turn(std::integral_constant<int, -1>{}, kappa, whole);
+      a += a_step;
+    };
+    if (a < n_act) {
+      int e0 = next_entry(), e1 = next_entry();
+#pragma unroll 1
+      while (a < n_act && alive) {
+        offset(e0);
+        if (a < n_act && alive) offset(e1);
+      }
     }
     cp_async_wait_all();
+  } else if (PAIR && rank == 1) {
+    // ================================ the other CTA of a pair: tells the issuing one of its full slots =====
+    const uint32_t full0 = smem_u32(full_bars);
+    const uint32_t there = peer_address(full0, 0u), masks_there = peer_address(smem_u32(slot_masks), 0u) + 16u;
+    uint32_t s = 0, par = 0;
+    bool alive = true;
+#pragma unroll 1
+    for (int it = 0; it < n_iter && alive; ++it) {
+      alive = mbar_wait_straight(full0 + s * 8u, par, abort_flag);
+      fence_async_smem();
+      const uint4 off = *(const uint4 *)(slot_masks + s * 8u);
+      if (alive && elect_one()) st_async_v4(masks_there + s * 32u, off, there + s * 8u);
+      if (++s == (uint32_t)S) { s = 0; par ^= 1u; }
+    }
   } else {
     // ================================ MMA issuer: the whole warp, one elected lane issues ========
     // fp32 accumulator; operand formats: kind::tf32 2 = TF32; kind::f16 0 = fp16, 1 = bf16
     RowsIssuer w;
     const uint32_t fmt = F16 ? (uint32_t)p.fmt16 : 2u;
-    w.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.tile_n >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+    w.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.tile_n >> 3) << 17) | ((uint32_t)((PAIR ? 2 * TC_M : TC_M) >> 4) << 24);
+    w.b_bytes = (uint32_t)b_bytes;
     w.a_lo = w.a_lo0 = desc_lo(smem_base);
     w.s = w.par = 0;
     w.full0 = smem_u32(full_bars); w.empty0 = smem_u32(empty_bars);
     w.masks = slot_masks; w.d0 = tmem_base; w.abort_flag = abort_flag;
-    if (p.nt_cta == 1) { if (scan) rows_issue_all<F16, 1, true>(w, p, n_act); else rows_issue_all<F16, 1, false>(w, p, n_act); }
-    else { if (scan) rows_issue_all<F16, 2, true>(w, p, n_act); else rows_issue_all<F16, 2, false>(w, p, n_act); }
-    if (elect_one()) mma_commit(smem_u32(&done_bar));   // arrives once everything issued above has retired
+    if (PAIR) {
+      if (p.nt_cta == 1) rows_issue_all<F16, 1, false, true>(w, p, n_act);
+      else rows_issue_all<F16, 2, false, true>(w, p, n_act);
+    } else if (p.nt_cta == 1) {
+      if (scan) rows_issue_all<F16, 1, true, false>(w, p, n_act);
+      else rows_issue_all<F16, 1, false, false>(w, p, n_act);
+    } else {
+      if (scan) rows_issue_all<F16, 2, true, false>(w, p, n_act);
+      else rows_issue_all<F16, 2, false, false>(w, p, n_act);
+    }
+    if (elect_one()) rows_commit<PAIR>(smem_u32(&done_bar));   // arrives once everything issued above has retired
   }
 
   // ================================ epilogue: TMEM -> shared memory -> global ====================
@@ -878,13 +947,32 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && *abort_flag) report_expired(status, p.alarm);
-  if (warp == mma_warp) {
+  if (PAIR) {                                     // neither leaves while the other may still signal it
+    cluster_sync();
+    if (warp == mma_warp) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols) : "memory");
+    cluster_sync();
+  } else if (warp == mma_warp) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols) : "memory");
   }
 }
 
+template <bool F16, bool GATED, int GROUPS>
+__global__ void __launch_bounds__(GROUPS * 128 + 32, GROUPS == 1 ? 4 : 2)
+conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
+                     const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out, int32_t *status, const __grid_constant__ TcParams p,
+                     const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order, const __grid_constant__ GateEpilogue gate) {
+  conv_fwd_rows<F16, GATED, GROUPS, false>(features, row_words, packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
+}
+template <bool F16, bool GATED, int GROUPS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GROUPS * 128 + 32, GROUPS == 1 ? 4 : 2)
+conv_fwd_pair_rows_kernel(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
+                          const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out, int32_t *status, const __grid_constant__ TcParams p,
+                          const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order, const __grid_constant__ GateEpilogue gate) {
+  conv_fwd_rows<F16, GATED, GROUPS, true>(features, row_words, packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
+}
+
 static size_t tc_smem_bytes(const TcParams &p) {
-  return (size_t)p.stages * p.sps * (TC_A_BYTES + p.b_bytes) + 1024 /*alignment slack*/ + TC_CTRL_BYTES;
+  return (size_t)p.stages * p.sps * (TC_A_BYTES + (p.pair ? p.b_bytes / 2 : p.b_bytes)) + 1024 /*alignment slack*/ + TC_CTRL_BYTES;
 }
 
 // 16-bit operands: filters [K, c_in, c_out] fp32 -> [K][k_slabs][n_pad rows][64 fp16 or bf16], same
@@ -917,15 +1005,25 @@ __global__ void pack_filters_16_kernel(const float *__restrict__ filters, int K,
   packed[block + off] = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
-// The plan of a launch over n_out rows: few row tiles spread the N tiles over CTAs too, and CTAs that are alone on
-// their SM take all of its shared memory.  Row tiles that fit the SMs by themselves but not with their N tiles
+// The plan of a launch over n_out rows: few row tiles spread the N tiles over CTAs too, and no more CTAs are put on an SM than
+// the launch has for it, so that they share its memory for deeper rings (256 tiles of 64 -> 76 bf16 channels, two on an SM instead of
+// four: 20.2 -> 15.7 us).  Row tiles that fit the SMs by themselves but not with their N tiles
 // spread stay whole: a few SMs with two CTAs would make all wait for rings of half the depth (79 row tiles
 // of 256 -> 304 bf16 channels: 62 us spread).
-static bool rows_params(int words, int c_out, int n_out, TcParams &p, int opk = 1) {
-  const int grid = ceil_div(n_out, TC_M), sms = sm_count();
-  if (!tc_params(words, c_out, p, false, grid <= sms, opk)) return false;
-  if (p.n_tiles == 1 || grid >= 2 * sms || (grid <= sms && grid * p.n_tiles > sms)) return true;
-  return tc_params(words, c_out, p, true, grid * p.n_tiles <= sms, opk);
+// Pairs: from 128 columns a CTA and four slabs an offset on, up to two tiles an SM.  There the filter slab, which every
+// tile brings in whole, is most of what a step moves (TF32 128 -> 152, 238 tiles: 59.1 -> 52.3 us; 256 -> 304 bf16, 125 tiles: 54.4 -> 52.6).  The second CTA's
+// news reaches the issuing one some 300 cycles late, so short loops lose (256 tiles of 128 -> 152 bf16: 30.8 -> 31.9), rings of two slots
+// more so (64 -> 76, 1.1 M rows: 690 -> 770), and with many tiles on an SM another one fills the time (637 tiles of 128 -> 152 bf16: 63 -> 65).
+static bool rows_params(int words, int c_out, int n_out, TcParams &p, int opk = 1, bool pairs = false) {
+  const int grid = n_out > 0 ? ceil_div(n_out, TC_M) : 1, sms = sm_count();
+  auto plan = [&](bool pair) {
+    if (!tc_params(words, c_out, p, false, ceil_div(grid, sms), opk, pair)) return false;
+    if (p.n_tiles == 1 || grid >= 2 * sms || (grid <= sms && grid * p.n_tiles > sms)) return true;
+    return tc_params(words, c_out, p, true, ceil_div(grid * p.n_tiles, sms), opk, pair);
+  };
+  if (!plan(false)) return false;
+  if (pairs && grid > 1 && grid <= 2 * sms && p.n_cta >= 128 && p.k_slabs >= 4) return plan(true);
+  return true;
 }
 
 // Producer groups.  Three or four CTAs on an SM have producers enough between them, and a second group in each would leave
@@ -937,6 +1035,10 @@ using RowsKernel = void (*)(const float *, int, const uint4 *, int, int, const i
                             const int32_t *, GateEpilogue);
 template <bool F16>
 static RowsKernel rows_kernel(const TcParams &p, bool gated) {
+  if (p.pair) {
+    if (rows_groups(p) == 1) return gated ? conv_fwd_pair_rows_kernel<F16, true, 1> : conv_fwd_pair_rows_kernel<F16, false, 1>;
+    return gated ? conv_fwd_pair_rows_kernel<F16, true, 2> : conv_fwd_pair_rows_kernel<F16, false, 2>;
+  }
   if (rows_groups(p) == 1) return gated ? conv_fwd_rows_kernel<F16, true, 1> : conv_fwd_rows_kernel<F16, false, 1>;
   return gated ? conv_fwd_rows_kernel<F16, true, 2> : conv_fwd_rows_kernel<F16, false, 2>;
 }
@@ -947,7 +1049,7 @@ static int rows_threads(const TcParams &p) { return rows_groups(p) * 128 + 32; }
 static bool gate_fits(const TcParams &p, int c_out, int c_keep) {
   const size_t warps = (size_t)rows_groups(p) * 4;
   return p.nt_cta == p.n_tiles &&
-         warps * 4096 + (size_t)c_out * 16 + (size_t)4 * 33 * 4 * (c_out - c_keep + 1) <= (size_t)p.stages * (TC_A_BYTES + p.b_bytes);
+         warps * 4096 + (size_t)c_out * 16 + (size_t)4 * 33 * 4 * (c_out - c_keep + 1) <= (size_t)p.stages * (TC_A_BYTES + (p.pair ? p.b_bytes / 2 : p.b_bytes));
 }
 
 bool conv_gate_covered(int c_in, int c_out, int c_keep, int precision, int n_out) {
@@ -968,7 +1070,10 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
     return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): needs the staging buffer of ssc_conv_scratch_bytes (16-byte aligned)");
   int grid = ceil_div(n_out, TC_M);
   TcParams p;
-  if (!rows_params(words, c_out, n_out, p)) return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): c_out %d / kernel volume %d not supported", c_out, K);
+  const bool gated = gate.gate_of_channel != nullptr;
+  bool planned = rows_params(words, c_out, n_out, p, 1, order == nullptr);
+  if (planned && gated && p.pair && !gate_fits(p, c_out, gate.c_keep)) planned = rows_params(words, c_out, n_out, p);
+  if (!planned) return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): c_out %d / kernel volume %d not supported", c_out, K);
   p.fmt16 = bf16 ? 1 : 0;
   p.nbr_by_pos = ((table_form & SSC_CONV_TABLE_IN_ORDER) && order) ? 1 : 0;
   p.rev = (table_form & SSC_CONV_TABLE_REVERSED) ? 1 : 0;
@@ -978,12 +1083,11 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
     if (rc != SSC_OK) return rc;
   }
   const size_t smem = tc_smem_bytes(p);
-  const bool gated = gate.gate_of_channel != nullptr;
   if (gated && !gate_fits(p, c_out, gate.c_keep)) return fail(SSC_ERR_INVALID, "conv_fwd(16-bit): the gated epilogue does not cover %d -> %d channels", c_out, gate.c_keep);
   const RowsKernel kernel = rows_kernel<true>(p, gated);
   cudaError_t e = allow_smem((const void *)kernel, smem);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(16-bit): smem attribute: %s", cudaGetErrorString(e));
-  const dim3 grid2(grid, p.n_tiles / p.nt_cta);
+  const dim3 grid2(p.pair ? (grid + 1) & ~1 : grid, p.n_tiles / p.nt_cta);
   { kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_fwd_16");
   return SSC_OK;
@@ -996,7 +1100,12 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
   if (K > 256) return fail(SSC_ERR_INVALID, "conv_fwd(tf32): kernel volume %d > 256", K);
   int grid = ceil_div(n_out, TC_M);
   const int opk = tf32_offsets_per_row(c_in);
-  if (!rows_params(c_in, c_out, n_out, p, opk)) return fail(SSC_ERR_INVALID, "conv_fwd(tf32): c_out %d / kernel volume %d not supported", c_out, K);
+  const bool gated = gate.gate_of_channel != nullptr;
+  // (a pair runs on staged rows only, and those come with a scratch buffer)
+  const bool fits = scratch != nullptr && scratch_bytes + 16 >= conv_tf32_scratch_bytes(n_in, c_in) && ((uintptr_t)scratch & 15u) == 0;
+  bool planned = rows_params(c_in, c_out, n_out, p, opk, order == nullptr && fits && opk == 1);
+  if (planned && gated && p.pair && !gate_fits(p, c_out, gate.c_keep)) planned = rows_params(c_in, c_out, n_out, p, opk);
+  if (!planned) return fail(SSC_ERR_INVALID, "conv_fwd(tf32): c_out %d / kernel volume %d not supported", c_out, K);
   p.nbr_by_pos = ((table_form & SSC_CONV_TABLE_IN_ORDER) && order) ? 1 : 0;
   p.rev = (table_form & SSC_CONV_TABLE_REVERSED) ? 1 : 0;
   p.alarm = alarm_word();
@@ -1004,8 +1113,6 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
   // With a staging buffer the feature rows are rounded to TF32 once, up front, instead of after
   // every gather (a row is gathered about K/2 times).
   const int c_pad = (c_in + 3) & ~3;  // row stride of the staged image (zero-padded channels)
-  const size_t stage_need = conv_tf32_scratch_bytes(n_in, c_in);
-  const bool fits = scratch != nullptr && scratch_bytes + 16 >= stage_need && ((uintptr_t)scratch & 15u) == 0;
   if (prestaged && !fits) return fail(SSC_ERR_INVALID, "conv_fwd(tf32): SSC_CONV_PRESTAGED without the staged image in scratch");
   // layers with few input channels have their filters packed for several offsets per operand row,
   // which the kernel can only feed from the staged (padded) rows
@@ -1017,8 +1124,8 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
     int rc = stage_features(features, n_in, c_in, scratch, st);
     if (rc != SSC_OK) return rc;
   }
-  const dim3 grid2(grid, p.n_tiles / p.nt_cta);
-  const bool rows = staged && opk == 1, gated = gate.gate_of_channel != nullptr;
+  const dim3 grid2(p.pair ? (grid + 1) & ~1 : grid, p.n_tiles / p.nt_cta);
+  const bool rows = staged && opk == 1;
   if (gated && !(rows && gate_fits(p, c_out, gate.c_keep)))
     return fail(SSC_ERR_INVALID, "conv_fwd(tf32): the gated epilogue does not cover %d -> %d channels without a staging buffer", c_out, gate.c_keep);
   if (rows) {

@@ -111,6 +111,37 @@ __device__ __forceinline__ bool mbar_wait_straight(uint32_t bar, uint32_t parity
   if (!ok) *abort_flag = 1;
   return ok;
 }
+// Pairs of CTAs (a cluster of two): the address of the same place in CTA `rank`'s shared memory, stores and arrivals there, and
+// the wait that sees them (mbar_wait_straight at cluster scope).
+__device__ __forceinline__ uint32_t peer_address(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_async_v4(uint32_t addr, uint4 v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w),
+               "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ bool mbar_wait_straight_cluster(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+  uint32_t i = 0, got;
+  bool ok;
+  do {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(got)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    ok = __all_sync(0xffffffffu, got != 0);
+  } while (!ok && ++i < kSpinLimit && ((i & 255u) != 255u || !__any_sync(0xffffffffu, *abort_flag)));
+  if (!ok) *abort_flag = 1;
+  return ok;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -216,6 +247,27 @@ __device__ __forceinline__ void mma_tf32_ss_masked(uint32_t tmem_c, uint32_t a_l
       : "r"(tmem_c), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(1u), "r"(kDescHi), "r"(off.x), "r"(off.y), "r"(off.z), "r"(off.w)
       : "memory");
 }
+// The same for a pair of CTAs, 256 rows: rows 0-127 (off) and half of B's rows in this one, the others at the same addresses in
+// the second.
+template <bool F16>
+__device__ __forceinline__ void mma_pair_masked(uint32_t tmem_c, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint4 off, uint4 off2) {
+  if (F16)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, {%6, %7, %8, %9, %10, %11, %12, %13}, p;\n\t}" ::"r"(tmem_c), "r"(a_lo), "r"(b_lo), "r"(idesc),
+        "r"(1u), "r"(kDescHi), "r"(off.x), "r"(off.y), "r"(off.z), "r"(off.w), "r"(off2.x), "r"(off2.y), "r"(off2.z), "r"(off2.w)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::2.kind::tf32 [%0], da, db, %3, {%6, %7, %8, %9, %10, %11, %12, %13}, p;\n\t}" ::"r"(tmem_c), "r"(a_lo), "r"(b_lo), "r"(idesc),
+        "r"(1u), "r"(kDescHi), "r"(off.x), "r"(off.y), "r"(off.z), "r"(off.w), "r"(off2.x), "r"(off2.y), "r"(off2.z), "r"(off2.w)
+        : "memory");
+}
+// The pair's commit arrives on the barrier at this address in both CTAs.
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
 // The same for fp16 operands (kind::f16, 16 elements = 32 bytes along K per instruction).
 __device__ __forceinline__ void mma_f16_ss_masked(uint32_t tmem_c, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint4 off) {
   asm volatile(
@@ -266,15 +318,21 @@ __device__ __forceinline__ void cp_async_wait(int n) {
 // All of the thread's copies, committed to a group or not (copies that arrive on a barrier by themselves never are).
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// The two 16-byte pieces a lane copies of a row (none if `from` is negative), OFF bytes into its part of the slot;
-// predicated instead of branched around: the instructions around the copies are what the producers' time goes into.
-template <int OFF>
-__device__ __forceinline__ void copy_row_pieces(int from, uint32_t dst0, uint32_t dst1, const char *at) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %0, 0;\n\t"
-      "@p cp.async.cg.shared.global [%1+%4], [%3], 16;\n\t"
-      "@p cp.async.cg.shared.global [%2+%4], [%3+64], 16;\n\t}" ::"r"(from), "r"(dst0), "r"(dst1), "l"(at), "n"(OFF)
-      : "memory");
+// The two 16-byte pieces a lane copies of each of its four rows (none where `from` is negative), P bytes into the row; its part of the
+// slot is eight rows on for each.  Predicated instead of branched around: the instructions around the copies are what the producers' time goes into.
+template <int P>
+__device__ __forceinline__ void copy_rows(const int *from, const char *const *at, uint32_t dst0, uint32_t dst1) {
+#define SSC_ROW(I, OFF) \
+  asm volatile( \
+      "{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %0, 0;\n\t" \
+      "@p cp.async.cg.shared.global [%1+%4], [%3+%5], 16;\n\t" \
+      "@p cp.async.cg.shared.global [%2+%4], [%3+%6], 16;\n\t}" ::"r"(from[I]), "r"(dst0), "r"(dst1), "l"(at[I]), "n"(OFF), "n"(P), "n"(P + 64) \
+      : "memory")
+  SSC_ROW(0, 0);
+  SSC_ROW(1, 1024);
+  SSC_ROW(2, 2048);
+  SSC_ROW(3, 3072);
+#undef SSC_ROW
 }
 // The same where a piece may lie past the row's end: it is zero-filled then, and its (base, stride) lead somewhere valid.
 template <int OFF>

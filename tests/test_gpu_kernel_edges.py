@@ -435,6 +435,33 @@ def test_gated_convolution_has_the_bits_of_the_two_passes(cuda, c_in, c_out, c_k
         assert torch.equal(_ext.conv_forward(feats, W, nbr, n, precision, row_order=order, gate=(scale, shift, table, c_keep, 1, 2)), want)
 
 
+@pytest.mark.parametrize("c_in,c_out,n,precision", [(128, 152, 129, "tf32"), (100, 128, 300, "tf32"), (256, 304, 1000, "bf16"),
+                                                    (250, 130, 257, "fp16"), (128, 512, 385, "tf32"), (140, 256, 18944, "tf32"), (128, 128, 37888, "tf32"),
+                                                    (128, 128, 37889, "tf32"), (124, 128, 128, "tf32"), (256, 304, 18945, "bf16")])
+def test_convolution_by_pairs_of_tiles(cuda, c_in, c_out, n, precision):
+    """Odd and even numbers of tiles around the sizes at which pairs of CTAs take over, a second tile with one row, rows that do
+    not fill their last slab, N tiles in one CTA and spread, fewer rows on the device than the launch has: the bits of the same rows in
+    any row order (which no pair takes)."""
+    from ss_conv import _ext
+    rng = np.random.RandomState(n + c_in)
+    g = torch.Generator(cuda).manual_seed(n)
+    K, n_in = 5, 200
+    nbr = torch.where(torch.rand(K, n, generator=g, device=cuda) < .5, torch.randint(0, n_in, (K, n), generator=g, device=cuda), -1).to(torch.int32)
+    x, W = dev(rng.randn(n_in, c_in).astype(np.float32), cuda), dev(rng.randn(K, c_in, c_out).astype(np.float32) * .1, cuda)
+    order = torch.arange(n, dtype=torch.int32, device=cuda)
+    want = _ext.conv_forward(x, W, nbr, n, precision, row_order=order)
+    assert torch.equal(_ext.conv_forward(x, W, nbr, n, precision), want)
+    few = max(1, n - 130)
+    count = torch.tensor([few], dtype=torch.int32, device=cuda)
+    got = _ext.conv_forward(x, W, nbr, n, precision, n_out_dev=count)
+    _ext.check_status(cuda)
+    assert torch.equal(got[:few], want[:few])
+    rows = np.unique(np.r_[0, n - 1, rng.randint(0, n, 40)])
+    t, xd, wd = nbr.cpu().numpy(), x.double().cpu().numpy(), W.double().cpu().numpy()
+    ref = np.stack([sum((xd[t[k, r]] @ wd[k] for k in range(K) if t[k, r] >= 0), np.zeros(c_out)) for r in rows])
+    assert rel_err(want[rows].cpu().numpy(), ref) < (1e-2 if precision == "bf16" else 1e-3)     # the operands' rounding
+
+
 @pytest.mark.parametrize("scalar_act", [0, 1, 2])
 def test_gated_convolution_at_the_ends_of_the_activations(cuda, scalar_act):
     """Gates far out on both sides, where the sigmoid's denominator is beyond every quick reciprocal, zeros of both
