@@ -604,6 +604,222 @@ bn_gate_bwd_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__res
   }
 }
 
+// The two passes for rows of up to 256 kept channels in fours, which is what the layers have: a lane has four channels (QL: or
+// eight) of a row, L lanes a row, 32 / L rows a warp at a time, straight from and to global memory, the next rows on their way.
+// Through shared memory go only (go, y), for the gates' sums, and the gates' values; a gate scalar belongs to one lane (or two do to one
+// lane), which keeps its sums like those of its kept channels.  PASS 0 adds up rows in registers: the warps' rows in ascending order, then a warp's
+// rows, then a block's warps in order; a block is one chain of the totals.  The form above hands every element through shared memory
+// and adds up a channel per thread, 32 rows at a time, while the other threads wait: 162 k rows of 32 + 6 channels 47 + 33 us, here
+// 19 + 16; 93 k rows of 64 + 12 30 + 25, here 18 + 16 (the bytes of the two passes take 8 and 12).  A gate's sum takes fields of up
+// to seven channels at once: as a loop it was half of the kernel.  Wider rows, others than fours and unaligned gradients stay above.
+template <int VEC>
+__device__ __forceinline__ void row_quad(const float *at, float (&v)[4]) {
+  if (VEC == 4) {
+    const float4 q = __ldg((const float4 *)at);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  } else if (VEC == 2) {
+    const float2 a = __ldg((const float2 *)at), b = __ldg((const float2 *)at + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = __ldg(at + i);
+  }
+}
+template <int PASS, int VEC, int QL>
+__global__ void __launch_bounds__(256, QL == 1 ? 4 : 2)
+bn_gate_bwd_lanes_kernel(BnGateBwd p, int L, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
+                         float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int GL = QL;                       // gate scalars of a lane
+  const int c = p.c, c_out = p.c_out, n_gates = p.n_gates, n = p.n;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int at = lane & (L - 1), slot = lane / L, per = 32 / L;
+  const bool affine = p.scale != nullptr;
+  float2 *pairs = (float2 *)sm + (size_t)(warp * per + slot) * c_out;                    // (go, y) of the lane's row
+  float *acts = sm + (size_t)16 * per * c_out + (size_t)(warp * per + slot) * (n_gates + 1);   // its gates' values, and a one
+  // constants of the lane's channels
+  float sc[QL][4], sh[QL][4], mu[QL][4], cs[QL][4], ca[QL][4], cg[QL][4];
+  const float *act[QL][4];                     // what a channel's gradient is multiplied by
+  uint32_t scalars = 0u;                       // bit 4 q + i
+  bool mine[QL];
+#pragma unroll
+  for (int q = 0; q < QL; ++q) {
+    mine[q] = (at + q * L) * 4 < c_out;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int ch = mine[q] ? (at + q * L) * 4 + i : 0;
+      sc[q][i] = affine ? __ldg(p.scale + ch) : 1.f;
+      sh[q][i] = affine ? __ldg(p.shift + ch) : 0.f;
+      mu[q][i] = p.mu ? __ldg(p.mu + ch) : 0.f;
+      const int gate = p.gate_of_channel ? __ldg(p.gate_of_channel + ch) : -2;
+      act[q][i] = acts + (gate >= 0 ? gate : n_gates);
+      if (gate == -1 && p.s_act != 0) scalars |= 1u << (4 * q + i);
+      if (PASS == 1 && ks) { cs[q][i] = __ldg(ks + ch); ca[q][i] = __ldg(ka + ch); cg[q][i] = __ldg(kg + ch); }
+    }
+  }
+  float gsc[GL], gsh[GL], gmu[GL], gcs[GL], gca[GL], gcg[GL];
+  const float2 *field[GL];
+  int glen[GL];
+  bool has[GL];
+#pragma unroll
+  for (int k = 0; k < GL; ++k) {
+    const int j = at + k * L, ch = c_out + j;
+    has[k] = j < n_gates;
+    gsc[k] = has[k] && affine ? __ldg(p.scale + ch) : 1.f;
+    gsh[k] = has[k] && affine ? __ldg(p.shift + ch) : 0.f;
+    gmu[k] = has[k] && p.mu ? __ldg(p.mu + ch) : 0.f;
+    field[k] = pairs + (has[k] ? __ldg(p.field_start + j) : 0);
+    glen[k] = has[k] ? __ldg(p.field_len + j) : 0;
+    if (PASS == 1 && ks && has[k]) { gcs[k] = __ldg(ks + ch); gca[k] = __ldg(ka + ch); gcg[k] = __ldg(kg + ch); }
+  }
+  if (at == 0) acts[n_gates] = 1.f;
+  float sum_a[QL][4], sum_g[QL][4], gsum_a[GL], gsum_g[GL];
+#pragma unroll
+  for (int q = 0; q < QL; ++q)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum_a[q][i] = sum_g[q][i] = 0.f;
+#pragma unroll
+  for (int k = 0; k < GL; ++k) gsum_a[k] = gsum_g[k] = 0.f;
+  __syncwarp();
+
+  const int step = (int)gridDim.x * 8 * per;
+  int row = ((int)blockIdx.x * 8 + warp) * per + slot;
+  for (int left = n - (row - slot); left > 0; left -= step, row += step) {     // rows from the warp's first on
+    const bool in = slot < left;
+    float x[QL][4], go[QL][4], xg[GL], gate_g[GL];
+    const float *xr = p.x + (size_t)row * c, *gr = p.go + (size_t)row * c_out;
+#pragma unroll
+    for (int q = 0; q < QL; ++q) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[q][i] = go[q][i] = 0.f;
+      if (in && mine[q]) {
+        row_quad<VEC>(xr + (at + q * L) * 4, x[q]);
+        row_quad<4>(gr + (at + q * L) * 4, go[q]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < GL; ++k) xg[k] = in && has[k] ? __ldg(xr + c_out + at + k * L) : 0.f;
+    if (n_gates > 0) {
+#pragma unroll
+      for (int q = 0; q < QL; ++q)
+        if (mine[q]) {
+          float y[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) y[i] = affine ? fmaf(x[q][i], sc[q][i], sh[q][i]) : x[q][i];
+          float4 *to = (float4 *)(pairs + (at + q * L) * 4);
+          to[0] = make_float4(go[q][0], y[0], go[q][1], y[1]);
+          to[1] = make_float4(go[q][2], y[2], go[q][3], y[3]);
+        }
+      __syncwarp();
+      float v[GL], f[GL];
+#pragma unroll
+      for (int k = 0; k < GL; ++k) {
+        float2 t[7];                           // (fields of up to order three at once)
+#pragma unroll
+        for (int i = 0; i < 7; ++i) t[i] = i < glen[k] ? field[k][i] : make_float2(0.f, 0.f);
+        float acc = 0.f;
+#pragma unroll
+        for (int i = 0; i < 7; ++i)
+          if (i < glen[k]) acc = fmaf(t[i].x, t[i].y, acc);
+        for (int i = 7; i < glen[k]; ++i) {
+          const float2 u = field[k][i];
+          acc = fmaf(u.x, u.y, acc);
+        }
+        gate_g[k] = acc;
+        v[k] = affine ? fmaf(xg[k], gsc[k], gsh[k]) : xg[k];
+        f[k] = v[k];
+      }
+      if (p.g_act == 2) {
+        apply_sigmoids<GL>(f);
+      } else {
+#pragma unroll
+        for (int k = 0; k < GL; ++k) f[k] = apply_act(v[k], p.g_act);
+      }
+#pragma unroll
+      for (int k = 0; k < GL; ++k) {
+        gate_g[k] *= act_grad(v[k], f[k], p.g_act);
+        if (has[k]) acts[at + k * L] = f[k];
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int q = 0; q < QL; ++q) {
+      float g[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g[i] = n_gates > 0 ? go[q][i] * *act[q][i] : go[q][i];
+      if ((scalars >> (4 * q)) & 15u) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if ((scalars >> (4 * q + i)) & 1u) {
+            const float y = affine ? fmaf(x[q][i], sc[q][i], sh[q][i]) : x[q][i];
+            g[i] *= act_grad(y, p.s_act == 2 ? apply_act(y, 2) : 0.f, p.s_act);
+          }
+      }
+      if (!in || !mine[q]) continue;
+      if (PASS == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          sum_g[q][i] += g[i];
+          sum_a[q][i] = fmaf(g[i], x[q][i] - mu[q][i], sum_a[q][i]);
+        }
+      } else {
+        float o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = ks ? cs[q][i] * g[i] - ca[q][i] * (x[q][i] - mu[q][i]) - cg[q][i] : g[i];
+        float *to = gx + (size_t)row * c + (at + q * L) * 4;
+        if (VEC == 4) {
+          *(float4 *)to = make_float4(o[0], o[1], o[2], o[3]);
+        } else if (VEC == 2) {
+          *(float2 *)to = make_float2(o[0], o[1]);
+          *((float2 *)to + 1) = make_float2(o[2], o[3]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) to[i] = o[i];
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < GL; ++k)
+      if (in && has[k]) {
+        const float d = xg[k] - gmu[k];
+        if (PASS == 0) {
+          gsum_g[k] += gate_g[k];
+          gsum_a[k] = fmaf(gate_g[k], d, gsum_a[k]);
+        } else {
+          gx[(size_t)row * c + c_out + at + k * L] = ks ? gcs[k] * gate_g[k] - gca[k] * d - gcg[k] : gate_g[k];
+        }
+      }
+  }
+  if (PASS == 0) {
+    auto rows_of_warp = [&](float v) {
+      for (int o = L; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      return v;
+    };
+    __syncthreads();
+    float *ra = sm + (size_t)warp * 2 * c, *rg = ra + c;
+#pragma unroll
+    for (int q = 0; q < QL; ++q)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float a = rows_of_warp(sum_a[q][i]), g = rows_of_warp(sum_g[q][i]);
+        if (slot == 0 && mine[q]) { ra[(at + q * L) * 4 + i] = a; rg[(at + q * L) * 4 + i] = g; }
+      }
+#pragma unroll
+    for (int k = 0; k < GL; ++k) {
+      const float a = rows_of_warp(gsum_a[k]), g = rows_of_warp(gsum_g[k]);
+      if (slot == 0 && has[k]) { ra[c_out + at + k * L] = a; rg[c_out + at + k * L] = g; }
+    }
+    __syncthreads();
+    for (int ch = threadIdx.x; ch < c; ch += 256) {
+      float a = sm[ch], g = sm[c + ch];
+#pragma unroll
+      for (int w = 1; w < 8; ++w) { a += sm[(size_t)w * 2 * c + ch]; g += sm[(size_t)w * 2 * c + c + ch]; }
+      part_a[(size_t)blockIdx.x * c + ch] = a;
+      part_g[(size_t)blockIdx.x * c + ch] = g;
+    }
+  }
+}
+
 // The same for rows of which not even one fits shared memory twice with its constants (more than about 4800
 // channels): a thread per channel, everything read where it lies.  Same sums in the same order.
 template <int PASS>
@@ -852,11 +1068,37 @@ static int launch_bwd_vec(const BnGateBwd &p, size_t smem, const float *ks, cons
   return SSC_OK;
 }
 
+template <int PASS, int QL>
+static void launch_bwd_lanes(const BnGateBwd &p, int lanes, const float *ks, const float *ka, const float *kg, float *gx, float *part_a, float *part_g, cudaStream_t st) {
+  const int per = 32 / lanes;
+  size_t smem = ((size_t)16 * per * p.c_out + (size_t)8 * per * (p.n_gates + 1)) * sizeof(float);
+  if (PASS == 0 && smem < (size_t)16 * p.c * sizeof(float)) smem = (size_t)16 * p.c * sizeof(float);
+  int blocks = p.chains;
+  if (PASS == 1) {
+    blocks = ceil_div(p.n, 8 * per);
+    const int most = (QL == 1 ? 4 : 2) * sm_count();
+    if (blocks > most) blocks = most;
+  }
+  const uintptr_t at = (uintptr_t)p.x | (uintptr_t)gx;
+  if ((p.c & 3) == 0 && (at & 15u) == 0) bn_gate_bwd_lanes_kernel<PASS, 4, QL><<<blocks, 256, smem, st>>>(p, lanes, ks, ka, kg, gx, part_a, part_g);
+  else if ((p.c & 1) == 0 && (at & 7u) == 0) bn_gate_bwd_lanes_kernel<PASS, 2, QL><<<blocks, 256, smem, st>>>(p, lanes, ks, ka, kg, gx, part_a, part_g);
+  else bn_gate_bwd_lanes_kernel<PASS, 1, QL><<<blocks, 256, smem, st>>>(p, lanes, ks, ka, kg, gx, part_a, part_g);
+  note_launches(1);
+}
+
 template <int PASS>
 static int launch_bwd(BnGateBwd p, const float *ks, const float *ka, const float *kg, float *gx, float *part_a, float *part_g, cudaStream_t st) {
   size_t smem;
-  p.rows = bwd_tile_rows(p.c, p.c_out, p.n_gates, PASS == 0 ? 32 : 64, &smem);
   p.chains = 8 * bn_row_blocks(p.n);
+  int lanes = 1;
+  while (lanes < 32 && lanes * 4 < p.c_out) lanes <<= 1;
+  if ((p.c_out & 3) == 0 && p.c_out <= 256 && p.n_gates <= 2 * lanes && ((uintptr_t)p.go & 15u) == 0) {
+    if (p.c_out <= 128 && p.n_gates <= lanes) launch_bwd_lanes<PASS, 1>(p, lanes, ks, ka, kg, gx, part_a, part_g, st);
+    else launch_bwd_lanes<PASS, 2>(p, lanes, ks, ka, kg, gx, part_a, part_g, st);
+    SSC_CHECK_LAUNCH("bn_gate_bwd");
+    return SSC_OK;
+  }
+  p.rows = bwd_tile_rows(p.c, p.c_out, p.n_gates, PASS == 0 ? 32 : 64, &smem);
   if (smem > 227 * 1024) {
     const int blocks = PASS == 0 ? p.chains : (p.n < 4 * 148 ? p.n : 4 * 148);
     bn_gate_bwd_wide_kernel<PASS><<<dim3(blocks, ceil_div(p.c, 256)), 256, 0, st>>>(p, ks, ka, kg, gx, part_a, part_g);
