@@ -27,7 +27,7 @@
 // TF32 yet are rounded in place once they have landed.  Pairs past the end of a list are zero rows;
 // channels past c_out / c_in are whatever the buffer holds: they only reach rows and columns of D
 // that nobody reads.
-//   warps 0 .. stages-1: producers, warp w owns ring slot w, pair indices one round ahead
+//   warps 0 .. 2 stages - 1: producers, two to a ring slot (gradients, inputs), pair indices one round ahead
 //   the next warp: tensor-memory allocation and the MMA-issuing thread
 //   four more: write finished partials (two accumulator buffers where tensor memory allows, so that
 //   the next offset's sums run meanwhile)
@@ -41,7 +41,7 @@ namespace ssc {
 
 constexpr int WT_M = 128;          // output channels per CTA
 constexpr int WT_K = 32;           // pairs per chunk
-constexpr int WT_MAX_STAGES = 8;
+constexpr int WT_MAX_STAGES = 5;   // two CTAs of 15 warps with 64 registers a thread fit an SM
 constexpr int WT_BLOCK = WT_K * 128;   // 32 channels of a chunk's pairs
 
 // Which output rows have a neighbour: a warp makes four words (128 rows) of one kernel offset (blockIdx.y), four
@@ -151,7 +151,19 @@ __device__ __forceinline__ void mma_tf32_mn(uint32_t tmem_c, uint32_t a_lo, uint
       : "memory");
 }
 
-__global__ void __launch_bounds__((WT_MAX_STAGES + 5) * 32)
+// Eight pairs' pieces of one 32-channel block, OFF bytes into the rows and BLK into the operand (constants: with running addresses half
+// of the fetch was additions).
+template <int OFF, int BLK>
+__device__ __forceinline__ void copy_block(uint32_t dst, const float *const (&g)[WT_K / 4], const uint32_t (&bytes)[WT_K / 4], bool on) {
+#pragma unroll
+  for (int i = 0; i < WT_K / 4; ++i)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t"
+        "@p cp.async.cg.shared.global [%0+%4], [%1+%5], 16, %2;\n\t}" ::"r"(dst + (uint32_t)i * 512u), "l"(g[i]), "r"(bytes[i]), "r"((uint32_t)on), "n"(BLK), "n"(OFF)
+        : "memory");
+}
+
+__global__ void __launch_bounds__((2 * WT_MAX_STAGES + 5) * 32, 2)
 conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in,
                      const int32_t *__restrict__ starts, int K, float *__restrict__ partial, int32_t *status) {
   extern __shared__ uint8_t smem_raw[];
@@ -163,11 +175,11 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
 
   const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
-  const int S = p.stages, mma_warp = S;
+  const int S = p.stages, mma_warp = 2 * S;
   const int co0 = blockIdx.y * WT_M;
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(smem_u32(full_bars + s), 32);
+      mbar_init(smem_u32(full_bars + s), 64);      // the lanes of the slot's two warps
       mbar_init(smem_u32(empty_bars + s), 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -195,46 +207,54 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
   int kappa0 = 0;                               // the offset the share begins in
   while (kappa0 + 1 < K && first[kappa0 + 1] <= q_begin) ++kappa0;
 
-  if (warp < S) {
+  if (warp < mma_warp) {
     // ====================================== producers ========================================
+    // Two warps to a slot, one for the gradients' rows and one for the inputs'.  (A warp for both: 1500 of a slot's 3800 cycles went into its
+    // copies and 900 into rounding; 93 k rows of 64 -> 76 channels 101 -> 89 us, with rows rounded before 64: then the rows' way from L2
+    // is the bound, 8 TB/s.)
     uint32_t par = 0;
     int kappa = kappa0;
-    int row_y = -1, row_x = -1;                 // this lane's pair of the next chunk
-    auto load_pair = [&](int q) {
-      row_y = row_x = -1;
+    const int own = warp >> 1;                  // slot
+    const bool is_x = (warp & 1) != 0;
+    const int32_t *list = is_x ? pair_in : pair_out;
+    int next_row = -1;                          // this lane's row of the next chunk
+    auto load_row = [&](int q) {
+      next_row = -1;
       if (q >= q_end) return;
       while (first[kappa + 1] <= q) ++kappa;
       const int j = __ldg(starts + kappa) + (q - first[kappa]) * WT_K + lane;
-      if (j < __ldg(starts + kappa + 1)) {
-        row_y = __ldg(pair_out + j);
-        row_x = __ldg(pair_in + j);
-      }
+      if (j < __ldg(starts + kappa + 1)) next_row = __ldg(list + j);
     };
     const int sub = lane & 7, grp = lane >> 3;  // 16-byte piece of a line, pair of a group of four
     // lines 0 .. 31 of every 32-channel block; piece `sub` of line k lies at 32-byte atom (sub >> 1) ^ (k & 3)
     const uint32_t piece = (uint32_t)grp * 128u + ((((uint32_t)sub >> 1) ^ (uint32_t)grp) << 5) + ((uint32_t)sub & 1u) * 16u;
-    // (straight-line over the eight groups of four pairs: as a rolled loop with its address arithmetic this
-    //  was 4100 warp instructions per chunk and the kernel's bound, 172 us on the layer above)
-    auto fetch = [&](const float *rows, int words, int n_ch, int my_row, uint32_t tile) {
+    const float *rows = is_x ? p.x : p.dy + co0;
+    const int words = is_x ? p.x_words : p.y_words, n_ch = is_x ? p.c_in : m_cnt, rounds = is_x ? p.x_round : p.y_round;
+    const bool vec = (words & 3) == 0 && ((uintptr_t)rows & 15u) == 0;
+    auto fetch = [&](int my_row, uint32_t tile) {
       const float *g[WT_K / 4];
       uint32_t bytes[WT_K / 4];
 #pragma unroll
       for (int i = 0; i < WT_K / 4; ++i) {
         const int row = __shfl_sync(0xffffffffu, my_row, i * 4 + grp);
-        g[i] = rows + (size_t)(row >= 0 ? row : 0) * words + sub * 4;
+        g[i] = rows + (unsigned long long)(uint32_t)(row >= 0 ? row : 0) * (uint32_t)words + sub * 4;
         bytes[i] = row >= 0 ? 16u : 0u;
       }
       uint32_t dst = tile + piece;
-      if ((words & 3) == 0 && ((uintptr_t)rows & 15u) == 0) {
-        for (int left = n_ch - sub * 4; left > 0; left -= 32, dst += WT_BLOCK) {
+      int left = n_ch - sub * 4;                // channels from this lane's first piece on
+      if (vec) {
+        for (int c0 = 0; c0 < n_ch; c0 += 128, left -= 128, dst += 4 * WT_BLOCK) {
+          copy_block<0, 0>(dst, g, bytes, left > 0);
+          if (c0 + 32 < n_ch) copy_block<128, WT_BLOCK>(dst, g, bytes, left > 32);
+          if (c0 + 64 < n_ch) copy_block<256, 2 * WT_BLOCK>(dst, g, bytes, left > 64);
+          if (c0 + 96 < n_ch) copy_block<384, 3 * WT_BLOCK>(dst, g, bytes, left > 96);
+          if (c0 + 128 < n_ch) {
 #pragma unroll
-          for (int i = 0; i < WT_K / 4; ++i) {
-            cp_async16_cg(dst + (uint32_t)i * 512u, g[i], bytes[i]);
-            g[i] += 32;
+            for (int i = 0; i < WT_K / 4; ++i) g[i] += 128;
           }
         }
       } else {
-        for (int left = n_ch - sub * 4; left > 0; left -= 32, dst += WT_BLOCK) {
+        for (; left > 0; left -= 32, dst += WT_BLOCK) {
           for (int i = 0; i < WT_K / 4; ++i)
             for (int e = 0; e < 4; ++e)
               if (e < left) cp_async4(dst + (uint32_t)i * 512u + 4u * e, g[i] + e, bytes[i] >> 2);
@@ -259,24 +279,23 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
         }
       }
     };
-    uint8_t *slot = smem + (size_t)warp * p.stage_bytes;
-    const uint32_t slot_addr = smem_base + (uint32_t)warp * (uint32_t)p.stage_bytes;
-    load_pair(q_begin + warp);
-    for (int q = q_begin + warp; q < q_end; q += S) {
-      const int ry = row_y, rx = row_x;
-      load_pair(q + S);
+    const uint32_t operand = is_x ? (uint32_t)p.a_bytes : 0u;
+    uint8_t *slot = smem + (size_t)own * p.stage_bytes + operand;
+    const uint32_t slot_addr = smem_base + (uint32_t)own * (uint32_t)p.stage_bytes + operand;
+    load_row(q_begin + own);
+    for (int q = q_begin + own; q < q_end; q += S) {
+      const int row = next_row;
+      load_row(q + S);
       if (q >= q_begin + S) {
-        if (!mbar_wait_warp(smem_u32(empty_bars + warp), par ^ 1u, abort_flag)) break;
+        if (!mbar_wait_straight(smem_u32(empty_bars + own), par ^ 1u, abort_flag)) break;
         tc_fence_after();
       }
-      fetch(p.dy + co0, p.y_words, m_cnt, ry, slot_addr);
-      fetch(p.x, p.x_words, p.c_in, rx, slot_addr + (uint32_t)p.a_bytes);
+      fetch(row, slot_addr);
       cp_async_commit();
       cp_async_wait(0);
-      if (p.y_round) round_tile(m_cnt, slot);
-      if (p.x_round) round_tile(p.c_in, slot + p.a_bytes);
+      if (rounds) round_tile(n_ch, slot);
       fence_async_smem();
-      mbar_arrive(smem_u32(full_bars + warp));
+      mbar_arrive(smem_u32(full_bars + own));
       par ^= 1u;
     }
   } else if (warp == mma_warp) {
@@ -555,7 +574,7 @@ int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_wgrad(tf32): smem attribute: %s", cudaGetErrorString(e));
     const WtParams w = {features, out_grad, c_in, c_out, (staged & 1) ? (c_in + 3) & ~3 : c_in, (staged & 2) ? (c_out + 3) & ~3 : c_out,
                         (staged & 1) ? 0 : 1, (staged & 2) ? 0 : 1, p.n_pad, p.a_bytes, p.stage_bytes, p.stages, p.n_buf, p.buf_cols, alarm_word()};
-    { conv_wgrad_tc_kernel<<<dim3(p.shares, p.co_blocks), (p.stages + 5) * 32, p.smem, st>>>(w, pl.pair_out, pl.pair_in, pl.starts, K, partial, status); note_launches(1); }
+    { conv_wgrad_tc_kernel<<<dim3(p.shares, p.co_blocks), (2 * p.stages + 5) * 32, p.smem, st>>>(w, pl.pair_out, pl.pair_in, pl.starts, K, partial, status); note_launches(1); }
     SSC_CHECK_LAUNCH("conv_wgrad_tc");
   } else if (p.small) {
     const dim3 grid(p.shares / 4, p.co_blocks);
