@@ -30,7 +30,7 @@
 //   * warps 5 .. 12: epilogue, two per quarter of the tensor-memory lanes (they take the
 //     32-column blocks in turn).  tcgen05.ld (lane = pair), a transposition through shared memory,
 //     16 rows at a time, so that eight neighbouring lanes hold the 128 contiguous bytes of one
-//     output row, then red.global.add.v4.f32: the reductions reach L2 as whole 128-byte lines.
+//     output row, then red.global.add.v4.f32: the reductions reach L2 as whole 128-byte lines (a warp has every other block).
 //     The epilogue of tile t runs under the MMAs of tile t+1.
 //
 // The output must be zero before the launch (the host wrapper clears it).  The sums of an output
@@ -66,13 +66,14 @@ struct PlParams {
   int ctas_per_sm;
   uint32_t idesc;
   int32_t *alarm;   // mapped host word that tells of an expired wait (may be NULL)
+  int pair;         // 1: two CTAs to a strip, half of the filter matrix in each; n_cta is the whole width then, a tile 256 pairs
   int f16;          // kind::f16 (fp16 / bf16 operands) instead of kind::tf32
 };
 
 // Strip table of one (pair lists, grid) combination.
 //   strips[s] = {virtual offset kv = kappa * n_split + half, first tile, tile stride, number of tiles}
 //   owner[s]  = the CTA that runs strip s (a CTA runs its strips in ascending s)
-//   hdr       = {number of strips, K, n_split, n_ctas}: the table is kept with the pair lists and only
+//   hdr       = {number of strips, K, n_split, n_ctas, rows of a tile}: the table is kept with the pair lists and only
 //               built when the header does not match (another grid or channel split)
 // L = the grid's fair share of all tiles.  An offset with T <= L tiles is one strip; up to 1.5 L it
 // is a main strip of L tiles plus a tail; beyond that it is cut into round(T / L) interleaved strips
@@ -84,16 +85,16 @@ struct PlParams {
 // strip cost a scan of all of them, 140 us for the 330 strips of a 5^3 layer; with a load per thread of the
 // block and two barriers per strip 30 us.  One warp now holds ten loads per lane in registers (the lowest
 // CTA wins ties); the first strip of every CTA needs no decision (all loads are zero, so they go in order).
-__device__ __forceinline__ void deal_strips(const int32_t *__restrict__ starts, int K, int n_split, int n_ctas,
+__device__ __forceinline__ void deal_strips(const int32_t *__restrict__ starts, int K, int n_split, int tile, int n_ctas,
                                             int32_t *__restrict__ hdr, int4 *__restrict__ strips, int32_t *__restrict__ owner) {
   __shared__ int tiles[256], first[257], tiles_of[PL_MAX_CTAS];
   __shared__ int L_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (hdr[0] > 0 && hdr[1] == K && hdr[2] == n_split && hdr[3] == n_ctas) return;   // built before for this grid
+  if (hdr[0] > 0 && hdr[1] == K && hdr[2] == n_split && hdr[3] == n_ctas && hdr[4] == tile) return;   // built before for this grid
   int T = 0;
   if (tid < K) {
     const int n = starts[tid + 1] - starts[tid];
-    T = n > 0 ? (n + PL_M - 1) / PL_M : 0;
+    T = n > 0 ? (n + tile - 1) / tile : 0;
   }
   if (tid < 256) tiles[tid] = T;
   __syncthreads();
@@ -193,6 +194,7 @@ __device__ __forceinline__ void deal_strips(const int32_t *__restrict__ starts, 
     hdr[1] = K;
     hdr[2] = n_split;
     hdr[3] = n_ctas;
+    hdr[4] = tile;
     __threadfence();
     hdr[0] = n_strips;
   }
@@ -205,11 +207,11 @@ __device__ __forceinline__ void deal_strips(const int32_t *__restrict__ starts, 
 // (42 k rows 192 -> 192 bf16: 9 + 7 + 16 us one after the other, 22 like this; the whole layer 246 -> 232.)
 template <bool F16>
 __global__ void __launch_bounds__(PL_MAX_CTAS)
-pl_prepare_kernel(const int32_t *__restrict__ starts, int K, int n_split, int n_ctas, int32_t *__restrict__ hdr, int4 *__restrict__ strips,
+pl_prepare_kernel(const int32_t *__restrict__ starts, int K, int n_split, int tile, int n_ctas, int32_t *__restrict__ hdr, int4 *__restrict__ strips,
                   int32_t *__restrict__ owner, const float4 *__restrict__ rows, long long n_stage, int bf16, uint4 *__restrict__ staged,
                   float4 *__restrict__ out, long long n_clear) {
   if (blockIdx.x == 0) {
-    deal_strips(starts, K, n_split, n_ctas, hdr, strips, owner);
+    deal_strips(starts, K, n_split, tile, n_ctas, hdr, strips, owner);
     return;
   }
   const long long first = (long long)(blockIdx.x - 1) * PL_MAX_CTAS + threadIdx.x, step = (long long)(gridDim.x - 1) * PL_MAX_CTAS;
@@ -231,15 +233,28 @@ __device__ __forceinline__ void copy_rows(int a, int b, uint32_t dst0, uint32_t 
       : "memory");
 }
 
-template <bool F16>
-__global__ void __launch_bounds__((PL_PRODUCERS + 1 + PL_EPI_WARPS) * 32, 1)
-conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict__ packed, int c_out,
-                      const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in,
-                      const int32_t *__restrict__ starts, const int4 *__restrict__ strips,
-                      const int32_t *__restrict__ owner, const int32_t *__restrict__ n_strips_dev,
-                      float *__restrict__ out, int32_t *status, PlParams p) {
+template <bool PAIR>
+__device__ __forceinline__ void pl_commit(uint32_t bar) {
+  if (PAIR) mma_commit_pair(bar);
+  else mma_commit(bar);
+}
+
+// Two CTAs to a strip (a cluster): its tiles have 256 pairs, 128 each, multiplied as one (cta_group::2), and each CTA holds half of the
+// filter matrix, so that a matrix that does not fit one CTA needs no second gather of its rows.  CTA 0 issues for both; what it
+// has to know of the other (rows landed, filters landed, accumulators read out) comes as asynchronous stores of
+// 16 bytes that count on its barriers.
+template <bool F16, bool PAIR>
+__device__ __forceinline__ void
+conv_fwd_pairs_body(const float *__restrict__ staged, const uint4 *__restrict__ packed, int c_out,
+                    const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in,
+                    const int32_t *__restrict__ starts, const int4 *__restrict__ strips,
+                    const int32_t *__restrict__ owner, const int32_t *__restrict__ n_strips_dev,
+                    float *__restrict__ out, int32_t *status, const PlParams &p) {
+  const int unit = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, rank = PAIR ? (int)blockIdx.x & 1 : 0;
+  constexpr int TILE = PAIR ? 2 * PL_M : PL_M;
+  const int tile_row0 = rank * PL_M;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t *smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
   uint8_t *w_smem = smem;                                       // resident filters, [k_slabs][n_cta][128 B]
   uint8_t *a_smem = smem + p.w_bytes;                           // [stages][16 KB]
   uint8_t *stg = a_smem + (size_t)p.stages * PL_A_BYTES;        // epilogue transpose blocks
@@ -253,6 +268,7 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
   uint64_t *final_bar = wfree_bar + 1;
   uint32_t *tmem_slot = (uint32_t *)(final_bar + 1);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+  const uint32_t news = smem_u32(ctrl + 512);                   // where the other CTA's stores go
 
   const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
   const int S = p.stages;
@@ -261,7 +277,7 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(smem_u32(full_bars + s), PL_PRODUCERS * 32);    // arrivals by copies
+      mbar_init(smem_u32(full_bars + s), PL_PRODUCERS * 32 + (PAIR && rank == 0 ? 1 : 0));    // arrivals by copies, the other CTA's news
       mbar_init(smem_u32(empty_bars + s), 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -275,13 +291,17 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == mma_warp) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"((uint32_t)(2 * p.acc_cols))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)(2 * p.acc_cols)) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)(2 * p.acc_cols)) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();                               // the other CTA's barriers stand
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t a_base = smem_u32(a_smem), w_base = smem_u32(w_smem);
@@ -304,13 +324,13 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
     uint32_t par = 1;                                     // (a fresh barrier counts as passed with parity 1)
     bool alive = true;
     for (int si = 0; si < n_strips && alive; ++si) {
-      if (__ldg(owner + si) != (int)blockIdx.x) continue;
+      if (__ldg(owner + si) != unit) continue;
       const int4 sd = __ldg(strips + si);
       const int kappa = sd.x / p.n_split;
       const int list0 = __ldg(starts + kappa), n_pairs = __ldg(starts + kappa + 1) - list0;
       const int n_tiles = sd.w;
       auto row_of = [&](int ti) {                         // input row of this lane's pair
-        const int j = (sd.y + ti * sd.z) * PL_M + warp * 32 + lane;
+        const int j = (sd.y + ti * sd.z) * TILE + tile_row0 + warp * 32 + lane;
         return ti < n_tiles && j < n_pairs ? __ldg(pair_in + list0 + j) : -1;
       };
       int src = row_of(0);
@@ -320,12 +340,13 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
 #pragma unroll
         for (int i = 0; i < 8; ++i) from[i] = __shfl_sync(0xffffffffu, src, i * 4 + row4);
 #pragma unroll 1
-        for (int slab = 0; slab < k_slabs; ++slab) {
+        for (int slab = 0; slab < k_slabs && alive; ++slab) {
           // pieces past the last channel are zero-filled (and read nothing)
           const uint32_t bytes = slab * 32 + piece * 4 < slab_words ? 16u : 0u, stride = bytes ? row_bytes : 0u;
           const char *base = bytes ? lane_rows + slab * 128 : (const char *)staged;
           const uint32_t full = full0 + (uint32_t)slot * 8u, slot_off = (uint32_t)slot * (uint32_t)PL_A_BYTES;
-          if (!mbar_wait_uniform(empty0 + (uint32_t)slot * 8u, par, abort_flag)) { alive = false; break; }
+          alive = mbar_wait_straight(empty0 + (uint32_t)slot * 8u, par, abort_flag);
+          if (PAIR && rank == 0 && warp == 0 && elect_one()) mbar_expect_tx(full, 16u);
           const uint32_t dst0 = first0 + slot_off, dst1 = first1 + slot_off;
           copy_rows<0>(from[0], from[1], dst0, dst1, base, stride, bytes);
           copy_rows<1024>(from[2], from[3], dst0, dst1, base, stride, bytes);
@@ -343,70 +364,87 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
     int tcount = 0, scount = 0, w_issued = 0;
     uint32_t slot = 0, slot_par = 0;
     bool alive = true;
+    const uint32_t news0 = PAIR ? peer_address(news, 0u) : 0u, full0_there = PAIR ? peer_address(smem_u32(full_bars), 0u) : 0u;
     for (int si = 0; si < n_strips && alive; ++si) {
-      if (__ldg(owner + si) != (int)blockIdx.x) continue;
+      if (__ldg(owner + si) != unit) continue;
       const int4 sd = __ldg(strips + si);
       const int n_tiles = sd.w, kappa = sd.x / p.n_split, half = sd.x - kappa * p.n_split;
       // the strip's filter matrix: one bulk copy per slab, after the MMAs of the last strip retired
       if (scount > 0 && !mbar_wait_uniform(smem_u32(wfree_bar), (uint32_t)(scount - 1) & 1u, abort_flag)) break;
+      const uint32_t own_rows = (uint32_t)(PAIR ? p.n_cta >> 1 : p.n_cta), slab_bytes = own_rows * 128u;    // filter rows in this CTA
       if (elect_one()) {
-        const uint32_t bar = smem_u32(wfull_bar), slab_bytes = (uint32_t)p.n_cta * 128u;
-        mbar_expect_tx(bar, (uint32_t)p.w_bytes);
+        const uint32_t bar = smem_u32(wfull_bar);
+        mbar_expect_tx(bar, (uint32_t)p.w_bytes + (PAIR && rank == 0 ? 16u : 0u));
         for (int s = 0; s < p.k_slabs; ++s)
           bulk_g2s(w_base + (uint32_t)s * slab_bytes,
-                   packed + ((size_t)kappa * p.k_slabs + s) * (size_t)(p.n_pad * 8) + (size_t)half * (size_t)(p.n_cta * 8), slab_bytes, bar);
+                   packed + ((size_t)kappa * p.k_slabs + s) * (size_t)(p.n_pad * 8) + (size_t)(PAIR ? rank : half) * (size_t)(own_rows * 8), slab_bytes, bar);
       }
       ++w_issued;
-      if (!mbar_wait_uniform(smem_u32(wfull_bar), (uint32_t)scount & 1u, abort_flag)) break;
+      if (!(PAIR ? mbar_wait_straight_cluster(smem_u32(wfull_bar), (uint32_t)scount & 1u, abort_flag) : mbar_wait_straight(smem_u32(wfull_bar), (uint32_t)scount & 1u, abort_flag))) break;
       tc_fence_after();
+      if (PAIR && rank == 1) {                            // only tells the other CTA
+        if (elect_one()) st_async_v4(news0, make_uint4(0u, 0u, 0u, 0u), peer_address(smem_u32(wfull_bar), 0u));
+        for (int n = n_tiles * p.k_slabs; n > 0 && alive; --n) {
+          alive = mbar_wait_straight(smem_u32(full_bars + slot), slot_par, abort_flag);
+          fence_async_smem();
+          if (alive && elect_one()) st_async_v4(news0, make_uint4(0u, 0u, 0u, 0u), full0_there + slot * 8u);
+          if (++slot == (uint32_t)S) { slot = 0; slot_par ^= 1u; }
+        }
+        ++scount;
+        continue;
+      }
       for (int ti = 0; ti < n_tiles && alive; ++ti, ++tcount) {
         const int buf = tcount & 1;
         if (tcount >= 2) {
-          if (!mbar_wait_uniform(smem_u32(acce_bars + buf), (uint32_t)((tcount >> 1) - 1) & 1u, abort_flag)) { alive = false; break; }
+          const uint32_t bar = smem_u32(acce_bars + buf), passed = (uint32_t)((tcount >> 1) - 1) & 1u;
+          if (!(PAIR ? mbar_wait_straight_cluster(bar, passed, abort_flag) : mbar_wait_straight(bar, passed, abort_flag))) { alive = false; break; }
           tc_fence_after();
         }
         const uint32_t d = tmem_base + (uint32_t)(buf * p.acc_cols);
         for (int s = 0; s < p.k_slabs; ++s) {
-          if (!mbar_wait_uniform(smem_u32(full_bars + slot), slot_par, abort_flag)) { alive = false; break; }
+          if (!(PAIR ? mbar_wait_straight_cluster(smem_u32(full_bars + slot), slot_par, abort_flag) : mbar_wait_straight(smem_u32(full_bars + slot), slot_par, abort_flag))) { alive = false; break; }
           fence_async_smem();                             // the rows other threads' copies left, for the tensor core
           tc_fence_after();
           const uint32_t a_lo = desc_lo(a_base + slot * PL_A_BYTES);
-          const uint32_t b_lo = desc_lo(w_base + (uint32_t)s * (uint32_t)p.n_cta * 128u);
+          const uint32_t b_lo = desc_lo(w_base + (uint32_t)s * slab_bytes);
           if (elect_one()) {
 #pragma unroll
             for (uint32_t kk = 0; kk < 4; ++kk) {
-              if (F16) mma_f16_ss(d, a_lo + 2u * kk, b_lo + 2u * kk, p.idesc, (s | (int)kk) != 0 ? 1u : 0u);
+              if (PAIR) mma_pair<F16>(d, a_lo + 2u * kk, b_lo + 2u * kk, p.idesc, (s | (int)kk) != 0 ? 1u : 0u);
+              else if (F16) mma_f16_ss(d, a_lo + 2u * kk, b_lo + 2u * kk, p.idesc, (s | (int)kk) != 0 ? 1u : 0u);
               else mma_tf32_ss(d, a_lo + 2u * kk, b_lo + 2u * kk, p.idesc, (s | (int)kk) != 0 ? 1u : 0u);
             }
-            mma_commit(smem_u32(empty_bars + slot));
+            pl_commit<PAIR>(smem_u32(empty_bars + slot));
           }
           if (++slot == (uint32_t)S) { slot = 0; slot_par ^= 1u; }
         }
-        if (alive && elect_one()) mma_commit(smem_u32(accf_bars + buf));
+        if (alive && elect_one()) pl_commit<PAIR>(smem_u32(accf_bars + buf));
       }
-      if (alive && elect_one()) mma_commit(smem_u32(wfree_bar));
+      if (alive && elect_one()) pl_commit<PAIR>(smem_u32(wfree_bar));
       ++scount;
     }
     // everything issued above (on any path) retires before the CTA hands its tensor memory back
-    if (elect_one()) mma_commit(smem_u32(final_bar));
+    if (rank == 0 && elect_one()) pl_commit<PAIR>(smem_u32(final_bar));
     mbar_wait_drain(smem_u32(final_bar), 0u);
     // a wait gave up while a filter copy may still be in flight: let it land before the CTA exits
     if (*abort_flag && w_issued > 0) mbar_wait_drain(smem_u32(wfull_bar), (uint32_t)(w_issued - 1) & 1u);
   } else {
     // ==================================== epilogue ==============================================
     // Two warps per quarter of the tensor-memory lanes; they take the 32-column blocks of the
-    // accumulator in turn.  The load of a warp's next block is in flight while it transposes and
-    // reduces the current one.
+    // accumulator in turn.  Their chain of instructions bounds the kernel (8300 of a tile's 9100 cycles for 256 channels, whether the
+    // reductions are issued or not), so a tile's addresses are worked out once and four loads from shared memory are in flight: 679 -> 644 us,
+    // bf16 192 -> 192 136 -> 128.  (Twelve warps gain nothing more, sixteen leave less room for the ring: 736 us.)
+    const uint32_t news0 = PAIR ? peer_address(news, 0u) : 0u;
     const int ew = warp - mma_warp - 1;                    // 0 .. 7
     const int quarter = warp & 3;                          // the 32 tensor-memory lanes this warp may read
-    const int part = ew >> 2;                              // blocks part, part + 2, ...
+    const int part = ew >> 2;                              // blocks part, part + 2, ... (eight warps)
     uint8_t *blk = stg + (size_t)ew * 16 * PL_STG_ROW;
     const bool vec_ok = (c_out & 3) == 0 && ((uintptr_t)out & 15u) == 0;
     const int sub = lane & 7, grp = lane >> 3;             // 16-byte piece of a row, row of a pass
     int tcount = 0;
     bool alive = true;
     for (int si = 0; si < n_strips && alive; ++si) {
-      if (__ldg(owner + si) != (int)blockIdx.x) continue;
+      if (__ldg(owner + si) != unit) continue;
       const int4 sd = __ldg(strips + si);
       const int kappa = sd.x / p.n_split, half = sd.x - kappa * p.n_split;
       const int list0 = __ldg(starts + kappa), n_pairs = __ldg(starts + kappa + 1) - list0;
@@ -416,7 +454,7 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
       const int n_blocks = cols > 0 ? (cols + 31) >> 5 : 0;       // 32-column blocks with real columns
       // output row of this lane's pair, fetched one tile ahead
       auto out_row_of = [&](int ti) {
-        const int j = (sd.y + ti * sd.z) * PL_M + quarter * 32 + lane;
+        const int j = (sd.y + ti * sd.z) * TILE + tile_row0 + quarter * 32 + lane;
         return (ti < n_tiles && j < n_pairs) ? __ldg(pair_out + list0 + j) : -1;
       };
       int next_out = out_row_of(0);
@@ -427,29 +465,25 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
         if (!mbar_wait_warp(smem_u32(accf_bars + buf), (uint32_t)(tcount >> 1) & 1u, abort_flag)) { alive = false; break; }
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * p.acc_cols);
-        // one load = this lane's row of a 32 x 32 block (two x16 loads in flight together)
-        auto tld = [&](uint32_t(&v)[32], int blk_i) {
-          const uint32_t ta = taddr + (uint32_t)(blk_i * 32);
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-              : "r"(ta)
-              : "memory");
-          if (blk_i * 32 + 16 < p.n_cta) {
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                : "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-                  "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                : "r"(ta + 16u)
-                : "memory");
-          }
-        };
-        // The 32 columns of 16 lanes' rows go to shared memory, then four rows per pass come back with
+        // this lane's places: row 16 h + 4 i + grp, 16-byte piece `sub` of the strip's columns
+        float *place[8];
+        uint32_t there = 0u;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const int orow = __shfl_sync(0xffffffffu, my_out, 4 * r + grp);
+          place[r] = out + (size_t)(orow >= 0 ? orow : 0) * c_out + col0 + sub * 4;
+          if (orow >= 0) there |= 1u << r;
+        }
+        // A 32 x 32 block at a time.  The 32 columns of 16 lanes' rows go to shared memory, then four rows per pass come back with
         // eight neighbouring lanes holding the 128 contiguous bytes of one output row: the
         // reductions reach L2 as whole 128-byte lines (the L2 slices take ~20 % more bytes per
         // second in that shape than in 64-byte pieces).
-        auto reduce_block = [&](const uint32_t(&v)[32], int blk_i) {
+        for (int b = part; b < n_blocks; b += PL_EPI_WARPS / 4) {
+          uint32_t v[32];
+          tmem_ld16(v, taddr + (uint32_t)(b * 32));
+          if (b * 32 + 16 < p.n_cta) tmem_ld16(v + 16, taddr + (uint32_t)(b * 32 + 16));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          const bool in = b * 32 + sub * 4 < cols;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             if ((lane >> 4) == h) {
@@ -458,44 +492,34 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
                 *(uint4 *)(blk + (lane & 15) * PL_STG_ROW + ((q ^ (lane & 7)) << 4)) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             }
             __syncwarp();
-            const int c_local = blk_i * 32 + sub * 4;       // column within the strip's range
-            const int cc = col0 + c_local;
+            float4 x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = *(const float4 *)(blk + (4 * i + grp) * PL_STG_ROW + ((sub ^ ((4 * i + grp) & 7)) << 4));
+            __syncwarp();
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              const int row = 4 * i + grp;
-              const int orow = __shfl_sync(0xffffffffu, my_out, 16 * h + row);
-              const float4 x = *(const float4 *)(blk + row * PL_STG_ROW + ((sub ^ (row & 7)) << 4));
-              if (orow >= 0 && c_local < cols) {
-                float *dst = out + (size_t)orow * c_out + cc;
-                if (vec_ok) {
-                  red_add_v4(dst, x);
-                } else {
-                  atomicAdd(dst, x.x);
-                  if (cc + 1 < c_out) atomicAdd(dst + 1, x.y);
-                  if (cc + 2 < c_out) atomicAdd(dst + 2, x.z);
-                  if (cc + 3 < c_out) atomicAdd(dst + 3, x.w);
-                }
+              if (!in || !((there >> (4 * h + i)) & 1u)) continue;
+              float *dst = place[4 * h + i] + b * 32;
+              if (vec_ok) {
+                red_add_v4(dst, x[i]);
+              } else {
+                const int cc = col0 + b * 32 + sub * 4;
+                atomicAdd(dst, x[i].x);
+                if (cc + 1 < c_out) atomicAdd(dst + 1, x[i].y);
+                if (cc + 2 < c_out) atomicAdd(dst + 2, x[i].z);
+                if (cc + 3 < c_out) atomicAdd(dst + 3, x[i].w);
               }
             }
-            __syncwarp();
-          }
-        };
-        uint32_t va[32], vb[32];
-        if (part < n_blocks) tld(va, part);
-        for (int b = part; b < n_blocks; b += 4) {
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (b + 2 < n_blocks) tld(vb, b + 2);
-          reduce_block(va, b);
-          if (b + 2 < n_blocks) {
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (b + 4 < n_blocks) tld(va, b + 4);
-            reduce_block(vb, b + 2);
           }
         }
         // this warp has read its share of the buffer: the MMA thread may overwrite it
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(acce_bars + buf));
+        if (lane == 0) {
+          if (PAIR && rank == 1) st_async_v4(news0, make_uint4(0u, 0u, 0u, 0u), peer_address(smem_u32(acce_bars + buf), 0u));
+          else if (PAIR && ew == 0) mbar_expect_tx(smem_u32(acce_bars + buf), PL_EPI_WARPS * 16u);     // (an arrival too)
+          else mbar_arrive(smem_u32(acce_bars + buf));
+        }
       }
     }
   }
@@ -503,11 +527,27 @@ conv_fwd_pairs_kernel(const float *__restrict__ staged, const uint4 *__restrict_
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && *abort_flag) report_expired(status, p.alarm);
-  if (warp == mma_warp) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(2 * p.acc_cols))
-                 : "memory");
+  if (PAIR) {                                              // neither leaves while the other may still signal it
+    cluster_sync();
+    if (warp == mma_warp) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(2 * p.acc_cols)) : "memory");
+    cluster_sync();
+  } else if (warp == mma_warp) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(2 * p.acc_cols)) : "memory");
   }
 }
+
+#define PL_ARGS const float *__restrict__ staged, const uint4 *__restrict__ packed, int c_out, const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in, \
+      const int32_t *__restrict__ starts, const int4 *__restrict__ strips, const int32_t *__restrict__ owner, const int32_t *__restrict__ n_strips, \
+      float *__restrict__ out, int32_t *status, const __grid_constant__ PlParams p
+template <bool F16>
+__global__ void __launch_bounds__((PL_PRODUCERS + 1 + PL_EPI_WARPS) * 32, 1) conv_fwd_pairs_kernel(PL_ARGS) {
+  conv_fwd_pairs_body<F16, false>(staged, packed, c_out, pair_out, pair_in, starts, strips, owner, n_strips, out, status, p);
+}
+template <bool F16>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((PL_PRODUCERS + 1 + PL_EPI_WARPS) * 32, 1) conv_fwd_pairs_by_two_kernel(PL_ARGS) {
+  conv_fwd_pairs_body<F16, true>(staged, packed, c_out, pair_out, pair_in, starts, strips, owner, n_strips, out, status, p);
+}
+#undef PL_ARGS
 
 static size_t pl_smem_bytes(const PlParams &p) {
   return (size_t)p.w_bytes + (size_t)p.stages * PL_A_BYTES + PL_STG_BYTES + PL_CTRL_BYTES + 1024 /*alignment slack*/;
@@ -516,6 +556,7 @@ static size_t pl_smem_bytes(const PlParams &p) {
 // Shapes the kernel covers: the filter matrix of one offset (or one range of its output channels)
 // resident in shared memory next to at least three ring slots.
 static bool pl_params(int c_in, int c_out, int precision, PlParams &p) {
+  p.pair = 0;
   const bool is16 = precision == SSC_PREC_F16 || precision == SSC_PREC_BF16;
   if (!is16 && tf32_offsets_per_row(c_in) > 1) return false;   // those filters are packed several offsets per row
   const int words = is16 ? f16_row_words(c_in) : c_in;
@@ -538,6 +579,14 @@ static bool pl_params(int c_in, int c_out, int precision, PlParams &p) {
     break;
   }
   if (p.n_split == 0 || p.n_cta < 16) return false;
+  // A matrix that one CTA cannot hold whole goes to two (with ranges of its channels every row is gathered once per range): 177 k rows
+  // of 256 -> 256 TF32 866 -> 679 us, 50 k rows of 208 -> 224 330 -> 239.  One that fits stays: 41 k rows of 192 -> 192 bf16 178 and 182.
+  if (p.n_split > 1 && p.n_pad <= 256 && (size_t)p.k_slabs * (p.n_pad / 2) * 128 + 3 * (size_t)PL_A_BYTES <= budget) {
+    p.pair = 1;
+    p.n_split = 1;
+    p.n_cta = p.n_pad;
+    p.w_bytes = p.k_slabs * (p.n_pad / 2) * 128;
+  }
   p.acc_cols = 32;
   while (p.acc_cols < p.n_cta) p.acc_cols <<= 1;
   p.ctas_per_sm = 1;      // 13 warps with ~120 registers each: one persistent CTA per SM
@@ -547,7 +596,7 @@ static bool pl_params(int c_in, int c_out, int precision, PlParams &p) {
   if (p.stages < 3) return false;
   p.threads = (PL_PRODUCERS + 1 + PL_EPI_WARPS) * 32;
   const uint32_t fmt = is16 ? (precision == SSC_PREC_BF16 ? 1u : 0u) : 2u;
-  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.n_cta >> 3) << 17) | ((uint32_t)(PL_M >> 4) << 24);
+  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.n_cta >> 3) << 17) | ((uint32_t)((p.pair ? 2 * PL_M : PL_M) >> 4) << 24);
   return true;
 }
 
@@ -570,6 +619,7 @@ int conv_fwd_pairs(const float *rows, int n_in, void *staged, int c_in, const vo
   p.alarm = alarm_word();
   int n_ctas = sm_count() * p.ctas_per_sm;
   if (n_ctas > PL_MAX_CTAS) n_ctas = PL_MAX_CTAS;
+  if (p.pair) n_ctas &= ~1;
   int32_t *hdr = (int32_t *)strip_mem;
   int4 *strips = (int4 *)((uint8_t *)strip_mem + 256);
   int32_t *owner = (int32_t *)(strips + max_strips(K));
@@ -595,10 +645,11 @@ int conv_fwd_pairs(const float *rows, int n_in, void *staged, int c_in, const vo
   const int want = ceil_div(n_stage > n_clear ? n_stage : n_clear, PL_MAX_CTAS * 2), most = sm_count() * 6;
   const int blocks = 1 + (want < most ? want : most);
   auto prepare = p.f16 ? pl_prepare_kernel<true> : pl_prepare_kernel<false>;
-  { prepare<<<blocks, PL_MAX_CTAS, 0, st>>>(pl.starts, K, p.n_split, n_ctas, hdr, strips, owner, (const float4 *)rows, n_stage, bf16 ? 1 : 0, (uint4 *)staged, (float4 *)out, n_clear); note_launches(1); }
+  { prepare<<<blocks, PL_MAX_CTAS, 0, st>>>(pl.starts, K, p.n_split, p.pair ? 2 * PL_M : PL_M, p.pair ? n_ctas / 2 : n_ctas, hdr, strips, owner, (const float4 *)rows, n_stage, bf16 ? 1 : 0, (uint4 *)staged, (float4 *)out, n_clear); note_launches(1); }
   SSC_CHECK_LAUNCH("pl_prepare");
   const size_t smem = pl_smem_bytes(p);
-  auto kernel = p.f16 ? conv_fwd_pairs_kernel<true> : conv_fwd_pairs_kernel<false>;
+  auto kernel = p.pair ? (p.f16 ? conv_fwd_pairs_by_two_kernel<true> : conv_fwd_pairs_by_two_kernel<false>)
+                       : (p.f16 ? conv_fwd_pairs_kernel<true> : conv_fwd_pairs_kernel<false>);
   e = allow_smem((const void *)kernel, smem);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd_pairs: smem attribute: %s", cudaGetErrorString(e));
   { kernel<<<n_ctas, p.threads, smem, st>>>((const float *)staged, (const uint4 *)packed, c_out, pl.pair_out, pl.pair_in, pl.starts,

@@ -264,6 +264,22 @@ __device__ __forceinline__ void mma_pair_masked(uint32_t tmem_c, uint32_t a_lo, 
         "r"(1u), "r"(kDescHi), "r"(off.x), "r"(off.y), "r"(off.z), "r"(off.w), "r"(off2.x), "r"(off2.y), "r"(off2.z), "r"(off2.w)
         : "memory");
 }
+// D (+)= A * B of a pair, all rows.
+template <bool F16>
+__device__ __forceinline__ void mma_pair(uint32_t tmem_c, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  if (F16)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, {%6, %6, %6, %6, %6, %6, %6, %6}, p;\n\t}" ::"r"(tmem_c), "r"(a_lo), "r"(b_lo), "r"(idesc),
+        "r"(accumulate), "r"(kDescHi), "r"(0u)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::2.kind::tf32 [%0], da, db, %3, {%6, %6, %6, %6, %6, %6, %6, %6}, p;\n\t}" ::"r"(tmem_c), "r"(a_lo), "r"(b_lo), "r"(idesc),
+        "r"(accumulate), "r"(kDescHi), "r"(0u)
+        : "memory");
+}
 // The pair's commit arrives on the barrier at this address in both CTAs.
 __device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");

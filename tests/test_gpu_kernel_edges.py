@@ -256,10 +256,11 @@ def test_fp32_convolution_with_large_filters_costs_less_than_dense_tiles(cuda):
 
 
 @pytest.mark.parametrize("precision", ["tf32", "bf16", "fp16"])
-@pytest.mark.parametrize("c_in,c_out,n", [(128, 128, 1), (132, 136, 129), (134, 130, 300), (192, 130, 77)])
+@pytest.mark.parametrize("c_in,c_out,n", [(128, 128, 1), (132, 136, 129), (134, 130, 300), (192, 130, 77),
+                                          (256, 256, 1), (250, 256, 129), (256, 250, 700), (208, 224, 1500), (700, 256, 300)])
 def test_pair_lists_prepared_in_one_launch(cuda, precision, c_in, c_out, n):
     """Rows staged and outputs cleared next to the strip table, and by the general kernels where rows or outputs are no whole
-    16-byte pieces.  Same operands and fp32 sums as the output-stationary kernel, in another order."""
+    16-byte pieces; filter matrices that fit a CTA, two, and neither.  Same operands and fp32 sums as the output-stationary kernel, in another order."""
     from ss_conv import _ext
     if not _ext.lib().ssc_conv_pairs_supported(c_in, c_out, _ext._PREC_OF[precision]):
         pytest.skip("shape not covered by the pair-list kernel")
