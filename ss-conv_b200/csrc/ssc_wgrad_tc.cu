@@ -16,7 +16,7 @@
 // bitwise repeatable.  (One CTA range per offset: 237 us on 61 k surface voxels, 64 -> 76 channels, of
 // which the centre offset alone kept ten CTAs busy.)
 //
-// conv_wgrad_tc_kernel (TF32 operands, tcgen05): a CTA accumulates D[co][ci] (M = 128 rows = output channels
+// conv_wgrad_tc_kernel (TF32 operands, tcgen05): a CTA accumulates D[co][ci] (or D[ci][co], see wgrad_plan; M = 128 rows = output channels
 // of one block of 128, N = input channels) in tensor memory; K = pairs, 32 per chunk.  The rows go to
 // shared memory as they lie in global memory (channels contiguous) and the tensor core takes both
 // operands MN-major: 32 channels of a pair are one 128-byte line, pairs follow one another, the 32-byte
@@ -131,6 +131,7 @@ struct WtParams {
   int x_words, y_words;        // row strides
   int x_round, y_round;        // 1: rows still to be rounded to TF32
   int n_pad, a_bytes, stage_bytes, stages, n_buf;
+  int in_rows;                 // 1: D[ci][co], input channels are the rows of a product; 0: D[co][ci]
   uint32_t buf_cols;
   int32_t *alarm;              // mapped host word that tells of an expired wait (may be NULL)
 };
@@ -176,7 +177,8 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
 
   const int tid = threadIdx.x, warp = warp_id(), lane = tid & 31;
   const int S = p.stages, mma_warp = 2 * S;
-  const int co0 = blockIdx.y * WT_M;
+  const bool in_rows = p.in_rows != 0;
+  const int co0 = (int)blockIdx.y * (in_rows ? p.n_pad : WT_M);
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(smem_u32(full_bars + s), 64);      // the lanes of the slot's two warps
@@ -201,7 +203,7 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
   const uint32_t smem_base = smem_u32(smem);
-  const int m_cnt = min(WT_M, p.c_out - co0);   // output channels of this CTA
+  const int co_cnt = min(in_rows ? p.n_pad : WT_M, p.c_out - co0);   // output channels of this CTA
   const int total = first[K];
   const int q_begin = share_begin((int)blockIdx.x, total, (int)gridDim.x), q_end = share_begin((int)blockIdx.x + 1, total, (int)gridDim.x);
   int kappa0 = 0;                               // the offset the share begins in
@@ -215,7 +217,7 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
     uint32_t par = 0;
     int kappa = kappa0;
     const int own = warp >> 1;                  // slot
-    const bool is_x = (warp & 1) != 0;
+    const bool second = (warp & 1) != 0, is_x = second != in_rows;    // which operand, whose rows
     const int32_t *list = is_x ? pair_in : pair_out;
     int next_row = -1;                          // this lane's row of the next chunk
     auto load_row = [&](int q) {
@@ -229,7 +231,7 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
     // lines 0 .. 31 of every 32-channel block; piece `sub` of line k lies at 32-byte atom (sub >> 1) ^ (k & 3)
     const uint32_t piece = (uint32_t)grp * 128u + ((((uint32_t)sub >> 1) ^ (uint32_t)grp) << 5) + ((uint32_t)sub & 1u) * 16u;
     const float *rows = is_x ? p.x : p.dy + co0;
-    const int words = is_x ? p.x_words : p.y_words, n_ch = is_x ? p.c_in : m_cnt, rounds = is_x ? p.x_round : p.y_round;
+    const int words = is_x ? p.x_words : p.y_words, n_ch = is_x ? p.c_in : co_cnt, rounds = is_x ? p.x_round : p.y_round;
     const bool vec = (words & 3) == 0 && ((uintptr_t)rows & 15u) == 0;
     auto fetch = [&](int my_row, uint32_t tile) {
       const float *g[WT_K / 4];
@@ -279,7 +281,7 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
         }
       }
     };
-    const uint32_t operand = is_x ? (uint32_t)p.a_bytes : 0u;
+    const uint32_t operand = second ? (uint32_t)p.a_bytes : 0u;
     uint8_t *slot = smem + (size_t)own * p.stage_bytes + operand;
     const uint32_t slot_addr = smem_base + (uint32_t)own * (uint32_t)p.stage_bytes + operand;
     load_row(q_begin + own);
@@ -335,7 +337,8 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
   } else {
     // ====================================== epilogue ===========================================
     const int quarter = warp & 3;
-    const int co = co0 + quarter * 32 + lane;
+    const int co = co0 + quarter * 32 + lane, ci = quarter * 32 + lane;
+    const bool vec = (p.c_out & 3) == 0 && ((uintptr_t)partial & 15u) == 0;
     int kappa = kappa0, seg = 0;
     for (int q = q_begin; q < q_end; ++seg) {
       while (first[kappa + 1] <= q) ++kappa;
@@ -354,7 +357,17 @@ conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int
             : "r"(taddr)
             : "memory");
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (co < p.c_out) {
+        if (in_rows) {
+          if (ci < p.c_in) {
+            float *to = dst + (size_t)ci * p.c_out + co0 + c0;
+#pragma unroll
+            for (int k = 0; k < 16; k += 4) {
+              if (vec && c0 + k < co_cnt) *(uint4 *)(to + k) = make_uint4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+              for (int i = k; !vec && i < k + 4; ++i)
+                if (c0 + i < co_cnt) to[i] = __uint_as_float(v[i]);
+            }
+          }
+        } else if (co < p.c_out) {
 #pragma unroll
           for (int k = 0; k < 16; ++k)
             if (c0 + k < p.c_in) dst[(size_t)(c0 + k) * p.c_out + co] = __uint_as_float(v[k]);  // lanes = consecutive co: coalesced
@@ -515,7 +528,7 @@ int pair_lists_build(const int32_t *nbr, int K, int n_out, void *lists, PairList
 
 // Shapes and shares of the two list kernels.
 struct WgradPlan {
-  bool tc, small;
+  bool tc, small, in_rows;
   int n_pad, n_buf, co_blocks, shares, stages, a_bytes, stage_bytes;
   uint32_t buf_cols;
   size_t smem;
@@ -527,15 +540,24 @@ static WgradPlan wgrad_plan(int K, int c_in, int c_out, int n_out, bool tf32) {
   // never more shares than the table could hold chunks
   const long long most = (long long)K * ceil_div(n_out > 0 ? n_out : 1, WT_K);
   if (tf32) {
-    p.n_pad = (c_in + 15) & ~15;
+    // Blocks of 128 output channels bring the input rows in once each.  Where there are several and the input channels fit the rows of a
+    // product, they are those, and up to 256 output channels its columns (93 k rows of 64 -> 152 169 -> 101 us, 30 k of 128 -> 152 64 -> 40, of 128 -> 304 90 -> 68).
+    p.in_rows = c_out > WT_M && c_in <= WT_M;
+    if (p.in_rows) {
+      p.co_blocks = ceil_div(c_out, 256);
+      p.n_pad = (ceil_div(c_out, p.co_blocks) + 15) & ~15;
+    } else {
+      p.co_blocks = ceil_div(c_out, WT_M);
+      p.n_pad = (c_in + 15) & ~15;
+    }
     if (p.n_pad > 256) return p;
     p.tc = true;
     p.buf_cols = 32;
     while ((int)p.buf_cols < p.n_pad) p.buf_cols <<= 1;
-    p.co_blocks = ceil_div(c_out, WT_M);
     // The 128 rows of an MMA are always read: channels that do not exist come from whatever lies behind the
     // operand's real blocks (the slack behind the last slot keeps that inside the buffer).
-    p.a_bytes = ceil_div(c_out < WT_M ? c_out : WT_M, 32) * WT_BLOCK;
+    const int m_side = p.in_rows ? c_in : c_out;
+    p.a_bytes = ceil_div(m_side < WT_M ? m_side : WT_M, 32) * WT_BLOCK;
     p.stage_bytes = p.a_bytes + ceil_div(p.n_pad, 32) * WT_BLOCK;
     // two CTAs per SM (tensor memory: 512 columns) where four slots fit each; two accumulator buffers where the columns allow
     const size_t slack = 1024 + (size_t)4 * WT_BLOCK, fixed = 2048;
@@ -573,7 +595,7 @@ int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int
     cudaError_t e = allow_smem((const void *)conv_wgrad_tc_kernel, p.smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_wgrad(tf32): smem attribute: %s", cudaGetErrorString(e));
     const WtParams w = {features, out_grad, c_in, c_out, (staged & 1) ? (c_in + 3) & ~3 : c_in, (staged & 2) ? (c_out + 3) & ~3 : c_out,
-                        (staged & 1) ? 0 : 1, (staged & 2) ? 0 : 1, p.n_pad, p.a_bytes, p.stage_bytes, p.stages, p.n_buf, p.buf_cols, alarm_word()};
+                        (staged & 1) ? 0 : 1, (staged & 2) ? 0 : 1, p.n_pad, p.a_bytes, p.stage_bytes, p.stages, p.n_buf, p.in_rows ? 1 : 0, p.buf_cols, alarm_word()};
     { conv_wgrad_tc_kernel<<<dim3(p.shares, p.co_blocks), (2 * p.stages + 5) * 32, p.smem, st>>>(w, pl.pair_out, pl.pair_in, pl.starts, K, partial, status); note_launches(1); }
     SSC_CHECK_LAUNCH("conv_wgrad_tc");
   } else if (p.small) {

@@ -665,6 +665,20 @@ def test_norm_entry_points_for_c_callers(cuda, n, training):
     assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
+@pytest.mark.parametrize("c_in,c_out,n", [(64, 152, 300), (128, 304, 130), (17, 129, 77), (128, 257, 64), (96, 512, 33), (130, 304, 65), (128, 128, 40)])
+def test_filter_gradient_on_either_side_of_a_product(cuda, c_in, c_out, n):
+    """Around 128 input and 128 and 256 output channels, where they change places: against float64.  TF32 rounds the
+    operands to 11 bits, so a sum of products is within 2^-11 of the sum of magnitudes, typically a tenth of it."""
+    from ss_conv import _ext
+    rng = np.random.RandomState(n)
+    t = _table(n, n, 9, 0.6, rng)
+    x, g = rng.randn(n, c_in).astype(np.float32), rng.randn(n, c_out).astype(np.float32)
+    got = _ext.conv_wgrad(dev(x, cuda), dev(g, cuda), dev(t, cuda), precision="tf32")
+    _ext.check_status(cuda)
+    want = np.stack([x.astype(np.float64)[t[k][t[k] >= 0]].T @ g.astype(np.float64)[t[k] >= 0] for k in range(9)])
+    assert rel_err(got.cpu().numpy(), want) < 1e-3
+
+
 @pytest.mark.parametrize("c_in,c_out,n", [(16, 8, 1), (18, 22, 130), (64, 76, 400)])
 def test_filter_gradient_of_staged_operands(cuda, c_in, c_out, n):
     """Operands that are rounded and padded already (the flags of ssc_conv_wgrad_lists, alone and together) give the bits of
