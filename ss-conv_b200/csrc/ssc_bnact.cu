@@ -163,6 +163,8 @@ bn_gate_rows_kernel(const float *__restrict__ x, uint32_t n_rows, uint32_t group
                     const int32_t *__restrict__ gate_of_channel, int c_gate_base, int n_gates, int scalar_act,
                     int gate_act, const float *__restrict__ scalar_bias, const float *__restrict__ gate_bias,
                     void *__restrict__ out) {
+  after_previous();
+  next_may_start();
   extern __shared__ float gate_s[];                    // [R][n_gates]
   // block = (groups, R): threadIdx.x is the group of VEC channels, threadIdx.y the row of the block
   // (no integer division anywhere in the kernel).  VEC = 4 / 2 / 1 for channel counts that are
@@ -247,7 +249,7 @@ static bool launch_bn_gate_rows(const float *x, int n, uint32_t groups, int c_in
   const uint32_t R = 256u / groups;
   const size_t smem = (size_t)R * n_gates * sizeof(float);
   if (smem > 48 * 1024) return false;
-  { bn_gate_rows_kernel<OUT, VEC><<<ceil_div(n, (int)R), dim3(groups, R), smem, st>>>(x, (uint32_t)n, groups, c_in_total, scale, shift,
+  { launch_ready(bn_gate_rows_kernel<OUT, VEC>, dim3(ceil_div(n, (int)R)), dim3(dim3(groups, R)), smem, st, x, (uint32_t)n, groups, c_in_total, scale, shift,
                                                                           gate_of_channel, c_gate_base, n_gates, scalar_act, gate_act,
                                                                           scalar_bias, gate_bias, out); note_launches(1); }
   return true;
@@ -271,6 +273,8 @@ template <int MODE, int VEC>
 __global__ void __launch_bounds__(256)
 bn_colsum_kernel(const float *__restrict__ x, int n, int c, int chains, int lanes, const float *__restrict__ chan_mean,
                  float *__restrict__ part) {
+  after_previous();
+  next_may_start();
   const int groups = c / VEC;
   const int lane = threadIdx.x / (blockDim.x / lanes), chain = blockIdx.x * lanes + lane;
   if (lane >= lanes || chain >= chains) return;
@@ -358,6 +362,8 @@ __device__ __forceinline__ float chain_total(const float *__restrict__ part, int
 __global__ void __launch_bounds__(kFinishThreads)
 bn_finish_mean_kernel(const float *__restrict__ part, int row_blocks, int n, int c, const int32_t *__restrict__ scalar_of_channel,
                       float momentum, float keep, float *running_mean, float *mean, float *chan_mean) {
+  after_previous();
+  next_may_start();
   const int ch = blockIdx.x, s = scalar_of_channel[ch];
   if (s < 0) {
     if (threadIdx.x == 0) chan_mean[ch] = 0.f;
@@ -388,6 +394,8 @@ bn_finish_var_kernel(const float *__restrict__ part, int row_blocks, int n, int 
                      const int32_t *__restrict__ scalar_of_channel, const float *__restrict__ chan_mean,
                      const float *__restrict__ weight, const float *__restrict__ bias, float eps, float momentum, float keep,
                      float *running_var, float *var, float *scale, float *shift) {
+  after_previous();
+  next_may_start();
   const int f = blockIdx.x;
   const int2 fc = field_channels(field_of_channel, c, f);
   const float v = chain_total(part, row_blocks, c, fc.x, fc.y) / (float)n;
@@ -629,6 +637,8 @@ template <int PASS, int VEC, int QL>
 __global__ void __launch_bounds__(256, QL == 1 ? 4 : 2)
 bn_gate_bwd_lanes_kernel(BnGateBwd p, int L, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
                          float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
+  after_previous();
+  next_may_start();
   extern __shared__ __align__(16) float sm[];
   constexpr int GL = QL;                       // gate scalars of a lane
   const int c = p.c, c_out = p.c_out, n_gates = p.n_gates, n = p.n;
@@ -872,6 +882,8 @@ bn_bwd_finish_kernel(const float *__restrict__ part_a, const float *__restrict__
                      const float *__restrict__ var, const float *__restrict__ weight, float eps, int training,
                      float *__restrict__ ks, float *__restrict__ ka, float *__restrict__ kg, float *__restrict__ d_weight,
                      float *__restrict__ d_bias) {
+  after_previous();
+  next_may_start();
   const int f = blockIdx.x;
   const int2 fc = field_channels(field_of_channel, c, f);
   const float A = chain_total(part_a, row_blocks, c, fc.x, fc.y);
@@ -1001,11 +1013,11 @@ static int launch_colsum(int mode, const float *x, int n, int c, const float *ch
   if (lanes < 1) lanes = 1;
   const int threads = lanes * (groups < 256 ? groups : 256), blocks = ceil_div(chains, lanes);
   if (vec) {
-    if (mode == 0) bn_colsum_kernel<0, 4><<<blocks, threads, 0, st>>>(x, n, c, chains, lanes, chan_mean, part);
-    else bn_colsum_kernel<1, 4><<<blocks, threads, 0, st>>>(x, n, c, chains, lanes, chan_mean, part);
+    if (mode == 0) launch_ready(bn_colsum_kernel<0, 4>, dim3(blocks), dim3(threads), 0, st, x, n, c, chains, lanes, chan_mean, part);
+    else launch_ready(bn_colsum_kernel<1, 4>, dim3(blocks), dim3(threads), 0, st, x, n, c, chains, lanes, chan_mean, part);
   } else {
-    if (mode == 0) bn_colsum_kernel<0, 1><<<blocks, threads, 0, st>>>(x, n, c, chains, lanes, chan_mean, part);
-    else bn_colsum_kernel<1, 1><<<blocks, threads, 0, st>>>(x, n, c, chains, lanes, chan_mean, part);
+    if (mode == 0) launch_ready(bn_colsum_kernel<0, 1>, dim3(blocks), dim3(threads), 0, st, x, n, c, chains, lanes, chan_mean, part);
+    else launch_ready(bn_colsum_kernel<1, 1>, dim3(blocks), dim3(threads), 0, st, x, n, c, chains, lanes, chan_mean, part);
   }
   note_launches(1);
   SSC_CHECK_LAUNCH("bn_colsum");
@@ -1025,9 +1037,9 @@ extern "C" int ssc_bn_train(const float *x, int n, int c, const int32_t *field_o
   const int rb = bn_row_blocks(n);
   const float m = (float)momentum, keep = (float)(1.0 - momentum);
   if (int e = launch_colsum(0, x, n, c, nullptr, part, st)) return e;
-  { bn_finish_mean_kernel<<<c, kFinishThreads, 0, st>>>(part, rb, n, c, scalar_of_channel, m, keep, running_mean, mean, chan_mean); note_launches(1); }
+  { launch_ready(bn_finish_mean_kernel, dim3(c), dim3(kFinishThreads), 0, st, part, rb, n, c, scalar_of_channel, m, keep, running_mean, mean, chan_mean); note_launches(1); }
   if (int e = launch_colsum(1, x, n, c, chan_mean, part, st)) return e;
-  { bn_finish_var_kernel<<<n_field, kFinishThreads, 0, st>>>(part, rb, n, c, field_of_channel, scalar_of_channel, chan_mean, weight, bias,
+  { launch_ready(bn_finish_var_kernel, dim3(n_field), dim3(kFinishThreads), 0, st, part, rb, n, c, field_of_channel, scalar_of_channel, chan_mean, weight, bias,
                                                            eps, m, keep, running_var, var, scale, shift); note_launches(1); }
   SSC_CHECK_LAUNCH("bn_train");
   return SSC_OK;
@@ -1080,9 +1092,9 @@ static void launch_bwd_lanes(const BnGateBwd &p, int lanes, const float *ks, con
     if (blocks > most) blocks = most;
   }
   const uintptr_t at = (uintptr_t)p.x | (uintptr_t)gx;
-  if ((p.c & 3) == 0 && (at & 15u) == 0) bn_gate_bwd_lanes_kernel<PASS, 4, QL><<<blocks, 256, smem, st>>>(p, lanes, ks, ka, kg, gx, part_a, part_g);
-  else if ((p.c & 1) == 0 && (at & 7u) == 0) bn_gate_bwd_lanes_kernel<PASS, 2, QL><<<blocks, 256, smem, st>>>(p, lanes, ks, ka, kg, gx, part_a, part_g);
-  else bn_gate_bwd_lanes_kernel<PASS, 1, QL><<<blocks, 256, smem, st>>>(p, lanes, ks, ka, kg, gx, part_a, part_g);
+  if ((p.c & 3) == 0 && (at & 15u) == 0) launch_ready(bn_gate_bwd_lanes_kernel<PASS, 4, QL>, dim3(blocks), dim3(256), smem, st, p, lanes, ks, ka, kg, gx, part_a, part_g);
+  else if ((p.c & 1) == 0 && (at & 7u) == 0) launch_ready(bn_gate_bwd_lanes_kernel<PASS, 2, QL>, dim3(blocks), dim3(256), smem, st, p, lanes, ks, ka, kg, gx, part_a, part_g);
+  else launch_ready(bn_gate_bwd_lanes_kernel<PASS, 1, QL>, dim3(blocks), dim3(256), smem, st, p, lanes, ks, ka, kg, gx, part_a, part_g);
   note_launches(1);
 }
 
@@ -1130,7 +1142,7 @@ extern "C" int ssc_bn_gate_bwd(const float *x, const float *gout, int n, int c, 
   BnGateBwd p = {x, gout, n, c, c_out, gate_of_channel ? c - c_out : 0, 0, 0, scale, shift, chan_mean, gate_of_channel, field_start, field_len,
                  scalar_act, gate_act};
   if (int e = launch_bwd<0>(p, nullptr, nullptr, nullptr, nullptr, part_a, part_g, st)) return e;
-  { bn_bwd_finish_kernel<<<n_field, kFinishThreads, 0, st>>>(part_a, part_g, rb, n, c, field_of_channel, scalar_of_channel, var, weight, eps,
+  { launch_ready(bn_bwd_finish_kernel, dim3(n_field), dim3(kFinishThreads), 0, st, part_a, part_g, rb, n, c, field_of_channel, scalar_of_channel, var, weight, eps,
                                                            training, ks, ka, kg, d_weight, d_bias); note_launches(1); }
   SSC_CHECK_LAUNCH("bn_bwd_finish");
   return launch_bwd<1>(p, ks, ka, kg, gx, nullptr, nullptr, st);

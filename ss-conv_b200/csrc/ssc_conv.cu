@@ -11,6 +11,8 @@ __global__ void materialize_kernel(const float *__restrict__ weight, const float
                                    const int32_t *__restrict__ block_table, int n_blocks_in,
                                    const int32_t *__restrict__ out_field, const int32_t *__restrict__ in_field,
                                    int c_out, int c_in, int K, float *__restrict__ filters) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long total = (long long)K * c_in * c_out;
   if (t >= total) return;
@@ -177,6 +179,8 @@ __global__ void __launch_bounds__(SM_WARPS * 32)
 conv_fwd_fp32_lanes_kernel(const float *__restrict__ features, int c_in, const float *__restrict__ filters, int K,
                            int c_out, const int32_t *__restrict__ nbr, int n_out, int rev, float *__restrict__ out,
                            const int32_t *__restrict__ n_out_dev) {
+  after_previous();
+  next_may_start();
   extern __shared__ __align__(16) float ws[];   // [K][c_in][CB]
   const int n_rows = live_rows(n_out, n_out_dev);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.y * CB;
@@ -283,7 +287,7 @@ static int launch_fp32_lanes(const float *features, int c_in, const float *filte
     cudaError_t e = allow_smem((const void *)kernel, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(fp32): smem attribute: %s", cudaGetErrorString(e));
   }
-  { kernel<<<grid, SM_WARPS * 32, smem, st>>>(features, c_in, filters, K, c_out, nbr, n_out, rev, out, n_out_dev); note_launches(1); }
+  { launch_ready(kernel, grid, dim3(SM_WARPS * 32), smem, st, features, c_in, filters, K, c_out, nbr, n_out, rev, out, n_out_dev); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_fwd_fp32");
   return SSC_OK;
 }
@@ -407,7 +411,7 @@ extern "C" int ssc_materialize(const float *weight, const float *basis, const in
   SSC_REQUIRE(c_out > 0 && c_in > 0 && K > 0 && n_blocks_in > 0, "materialize: bad sizes");
   SSC_REQUIRE(weight && basis && block_table && out_field && in_field && filters, "materialize: null pointer");
   long long total = (long long)K * c_in * c_out;
-  { materialize_kernel<<<ceil_div(total, 256), 256, 0, as_stream(stream)>>>(weight, basis, block_table, n_blocks_in,
+  { launch_ready(materialize_kernel, dim3(ceil_div(total, 256)), dim3(256), 0, as_stream(stream), weight, basis, block_table, n_blocks_in,
                                                                          out_field, in_field, c_out, c_in, K, filters); note_launches(1); }
   SSC_CHECK_LAUNCH("materialize");
   return SSC_OK;

@@ -210,6 +210,8 @@ __global__ void __launch_bounds__(PL_MAX_CTAS)
 pl_prepare_kernel(const int32_t *__restrict__ starts, int K, int n_split, int tile, int n_ctas, int32_t *__restrict__ hdr, int4 *__restrict__ strips,
                   int32_t *__restrict__ owner, const float4 *__restrict__ rows, long long n_stage, int bf16, uint4 *__restrict__ staged,
                   float4 *__restrict__ out, long long n_clear) {
+  after_previous();
+  next_may_start();
   if (blockIdx.x == 0) {
     deal_strips(starts, K, n_split, tile, n_ctas, hdr, strips, owner);
     return;
@@ -541,10 +543,14 @@ conv_fwd_pairs_body(const float *__restrict__ staged, const uint4 *__restrict__ 
       float *__restrict__ out, int32_t *status, const __grid_constant__ PlParams p
 template <bool F16>
 __global__ void __launch_bounds__((PL_PRODUCERS + 1 + PL_EPI_WARPS) * 32, 1) conv_fwd_pairs_kernel(PL_ARGS) {
+  after_previous();
+  next_may_start();
   conv_fwd_pairs_body<F16, false>(staged, packed, c_out, pair_out, pair_in, starts, strips, owner, n_strips, out, status, p);
 }
 template <bool F16>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((PL_PRODUCERS + 1 + PL_EPI_WARPS) * 32, 1) conv_fwd_pairs_by_two_kernel(PL_ARGS) {
+  after_previous();
+  next_may_start();
   conv_fwd_pairs_body<F16, true>(staged, packed, c_out, pair_out, pair_in, starts, strips, owner, n_strips, out, status, p);
 }
 #undef PL_ARGS
@@ -645,14 +651,14 @@ int conv_fwd_pairs(const float *rows, int n_in, void *staged, int c_in, const vo
   const int want = ceil_div(n_stage > n_clear ? n_stage : n_clear, PL_MAX_CTAS * 2), most = sm_count() * 6;
   const int blocks = 1 + (want < most ? want : most);
   auto prepare = p.f16 ? pl_prepare_kernel<true> : pl_prepare_kernel<false>;
-  { prepare<<<blocks, PL_MAX_CTAS, 0, st>>>(pl.starts, K, p.n_split, p.pair ? 2 * PL_M : PL_M, p.pair ? n_ctas / 2 : n_ctas, hdr, strips, owner, (const float4 *)rows, n_stage, bf16 ? 1 : 0, (uint4 *)staged, (float4 *)out, n_clear); note_launches(1); }
+  { launch_ready(prepare, dim3(blocks), dim3(PL_MAX_CTAS), 0, st, pl.starts, K, p.n_split, p.pair ? 2 * PL_M : PL_M, p.pair ? n_ctas / 2 : n_ctas, hdr, strips, owner, (const float4 *)rows, n_stage, bf16 ? 1 : 0, (uint4 *)staged, (float4 *)out, n_clear); note_launches(1); }
   SSC_CHECK_LAUNCH("pl_prepare");
   const size_t smem = pl_smem_bytes(p);
   auto kernel = p.pair ? (p.f16 ? conv_fwd_pairs_by_two_kernel<true> : conv_fwd_pairs_by_two_kernel<false>)
                        : (p.f16 ? conv_fwd_pairs_kernel<true> : conv_fwd_pairs_kernel<false>);
   e = allow_smem((const void *)kernel, smem);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd_pairs: smem attribute: %s", cudaGetErrorString(e));
-  { kernel<<<n_ctas, p.threads, smem, st>>>((const float *)staged, (const uint4 *)packed, c_out, pl.pair_out, pl.pair_in, pl.starts,
+  { launch_ready(kernel, dim3(n_ctas), dim3(p.threads), smem, st, (const float *)staged, (const uint4 *)packed, c_out, pl.pair_out, pl.pair_in, pl.starts,
                                           strips, owner, hdr, out, status, p); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_fwd_pairs");
   return SSC_OK;

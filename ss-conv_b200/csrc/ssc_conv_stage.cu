@@ -27,6 +27,7 @@ int sm_count() {
 constexpr int STAGE_VECS = 4;
 __global__ void __launch_bounds__(256)
 stage_features_kernel(const float4 *__restrict__ in, long long total_vec, uint4 *__restrict__ out) {
+  after_previous();
   const long long first = (long long)blockIdx.x * (256 * STAGE_VECS) + threadIdx.x;
   float4 v[STAGE_VECS];
 #pragma unroll
@@ -35,6 +36,7 @@ stage_features_kernel(const float4 *__restrict__ in, long long total_vec, uint4 
 #pragma unroll
   for (int q = 0; q < STAGE_VECS; ++q)
     if (first + q * 256 < total_vec) out[first + q * 256] = stage_piece(v[q]);
+  next_may_start();
 }
 
 // Channel counts that are not a multiple of four: rows padded with zeros to c_pad floats.
@@ -72,7 +74,7 @@ int stage_features(const float *features, int n_in, int c_in, void *staged, cuda
   if (n_in == 0) return SSC_OK;
   if (c_pad == c_in && ((uintptr_t)features & 15u) == 0) {
     const long long total_vec = (long long)n_in * c_in / 4;
-    { stage_features_kernel<<<ceil_div(total_vec, 256 * STAGE_VECS), 256, 0, st>>>((const float4 *)features, total_vec, (uint4 *)staged); note_launches(1); }
+    { launch_ready(stage_features_kernel, dim3(ceil_div(total_vec, 256 * STAGE_VECS)), dim3(256), 0, st, (const float4 *)features, total_vec, (uint4 *)staged); note_launches(1); }
   } else if (c_pad <= 1024) {
     const int groups = c_pad >> 2, rows = 256 / groups;
     { stage_features_padded_rows_kernel<<<ceil_div(n_in, rows), dim3(groups, rows), 0, st>>>(features, n_in, c_in, (uint4 *)staged); note_launches(1); }
@@ -111,6 +113,7 @@ __global__ void stage_features_16_kernel(const float *__restrict__ in, long long
 template <bool BF16>
 __global__ void __launch_bounds__(256)
 stage_features_16_vec_kernel(const float4 *__restrict__ in, long long total, uint4 *__restrict__ out) {
+  after_previous();
   const long long first = (long long)blockIdx.x * (256 * STAGE_VECS) + threadIdx.x;
   float4 a[STAGE_VECS], b[STAGE_VECS];
 #pragma unroll
@@ -122,6 +125,7 @@ stage_features_16_vec_kernel(const float4 *__restrict__ in, long long total, uin
 #pragma unroll
   for (int q = 0; q < STAGE_VECS; ++q)
     if (first + q * 256 < total) out[first + q * 256] = stage_piece_16(a[q], b[q], BF16);
+  next_may_start();
 }
 
 size_t conv_f16_scratch_bytes(int n_in, int c_in) { return (size_t)n_in * (size_t)f16_row_words(c_in) * 4 + 16; }
@@ -132,8 +136,7 @@ int stage_features_16(const float *features, int n_in, int c_in, bool bf16, void
   if ((c_in & 7) == 0 && (((uintptr_t)features | (uintptr_t)staged) & 15u) == 0) {
     const long long total = (long long)n_in * c_in / 8;
     const int vb = ceil_div(total, 256 * STAGE_VECS);
-    if (bf16) stage_features_16_vec_kernel<true><<<vb, 256, 0, st>>>((const float4 *)features, total, (uint4 *)staged);
-    else stage_features_16_vec_kernel<false><<<vb, 256, 0, st>>>((const float4 *)features, total, (uint4 *)staged);
+    launch_ready(bf16 ? stage_features_16_vec_kernel<true> : stage_features_16_vec_kernel<false>, dim3(vb), dim3(256), 0, st, (const float4 *)features, total, (uint4 *)staged);
     note_launches(1);
     SSC_CHECK_LAUNCH("stage_features_16");
     return SSC_OK;

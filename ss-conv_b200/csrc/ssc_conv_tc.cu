@@ -653,6 +653,7 @@ __device__ __forceinline__ void
 conv_fwd_rows(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
               const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out, int32_t *status, const TcParams &p,
               const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order, const GateEpilogue &gate) {
+  after_previous();
   const int n_rows = live_rows(n_out, n_out_dev);
   if ((int)(PAIR ? blockIdx.x & ~1u : blockIdx.x) * TC_M >= n_rows) return;
   const int rank = PAIR ? (int)blockIdx.x & 1 : 0;                   // in the pair: 0 issues for both
@@ -938,6 +939,7 @@ conv_fwd_rows(const float *__restrict__ features, int row_words, const uint4 *__
       store_plain(load16, blk, out, m, col0, p.n_cta, c_row, vec, lane, 32 * group, 32 * groups);
     }
   }
+  next_may_start();
   // a wait gave up: what was issued still arrives on done_bar (committed on every path) and filter copies land
   // within microseconds; both before the accumulators and the shared memory are handed back
   if (*abort_flag) {
@@ -1088,7 +1090,8 @@ int conv_fwd_16(const float *features, int n_in, int c_in, bool bf16, const void
   cudaError_t e = allow_smem((const void *)kernel, smem);
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(16-bit): smem attribute: %s", cudaGetErrorString(e));
   const dim3 grid2(p.pair ? (grid + 1) & ~1 : grid, p.n_tiles / p.nt_cta);
-  { kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate); note_launches(1); }
+  e = launch_ready(kernel, grid2, dim3(rows_threads(p)), smem, st, (const float *)scratch, words, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
+  note_launches(1);
   SSC_CHECK_LAUNCH("conv_fwd_16");
   return SSC_OK;
 }
@@ -1132,7 +1135,7 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
     const RowsKernel kernel = rows_kernel<false>(p, gated);
     cudaError_t e = allow_smem((const void *)kernel, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
-    kernel<<<grid2, rows_threads(p), smem, st>>>((const float *)scratch, c_pad, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
+    e = launch_ready(kernel, grid2, dim3(rows_threads(p)), smem, st, (const float *)scratch, c_pad, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
   } else {
     auto kernel = opk > 1 ? conv_fwd_tf32_kernel<true> : conv_fwd_tf32_kernel<false>;
     cudaError_t e = allow_smem((const void *)kernel, smem);

@@ -52,6 +52,8 @@ __global__ void __launch_bounds__(256)
 pool_fwd_kernel(const void *__restrict__ features, int c, const int32_t *__restrict__ nbr, int K,
                 int n_out, const int32_t *__restrict__ summaryrf, float *__restrict__ out,
                 const int32_t *__restrict__ n_out_dev, int R) {
+  after_previous();
+  next_may_start();
   extern __shared__ int32_t pool_smem[];
   const PoolTile tile = pool_tile(nbr, K, n_out, live_rows(n_out, n_out_dev), R, pool_smem);   // n_out: row stride of nbr
   const uint32_t cg = (uint32_t)(c + 3) / 4, items = (uint32_t)tile.rows * cg;
@@ -75,6 +77,8 @@ template <int MODE, int IN, int PIECE, int G>
 __global__ void __launch_bounds__(256)
 pool_fwd_few_kernel(const void *__restrict__ features, int c, const int32_t *__restrict__ nbr, int K, int n_out,
                     const int32_t *__restrict__ summaryrf, float *__restrict__ out, const int32_t *__restrict__ n_out_dev) {
+  after_previous();
+  next_may_start();
   const uint32_t cg = (uint32_t)(c + 3) / 4;
   const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
   if (t >= (long long)live_rows(n_out, n_out_dev) * cg) return;
@@ -150,6 +154,8 @@ __global__ void summary_rf_kernel(const int32_t *__restrict__ nbr, int K, int n_
 template <bool MAX>
 __global__ void global_pool_kernel(const float *__restrict__ feats, const int32_t *__restrict__ offsets, int c,
                                    float *__restrict__ out, int32_t *__restrict__ maxidx) {
+  after_previous();
+  next_may_start();
   __shared__ float sv[8][33];
   __shared__ int si[8][33];
   int s = blockIdx.x;
@@ -256,8 +262,8 @@ static int launch_pool_as(const void *features, int c, const int32_t *nbr, int K
   cudaStream_t st = as_stream(stream);
   if (K <= 8) {
     const int blocks = ceil_div((long long)n_out * ((c + 3) / 4), 256);
-    if (K >= 4) pool_fwd_few_kernel<MODE, IN, PIECE, 4><<<blocks, 256, 0, st>>>(features, c, nbr, K, n_out, rf, out, n_out_dev);
-    else pool_fwd_few_kernel<MODE, IN, PIECE, 1><<<blocks, 256, 0, st>>>(features, c, nbr, K, n_out, rf, out, n_out_dev);
+    if (K >= 4) launch_ready(pool_fwd_few_kernel<MODE, IN, PIECE, 4>, dim3(blocks), dim3(256), 0, st, features, c, nbr, K, n_out, rf, out, n_out_dev);
+    else launch_ready(pool_fwd_few_kernel<MODE, IN, PIECE, 1>, dim3(blocks), dim3(256), 0, st, features, c, nbr, K, n_out, rf, out, n_out_dev);
   } else {
     const PoolShape p = pool_shape(n_out, K);
     SSC_REQUIRE(p.rows > 0, "%s: kernel of %d offsets is too large", name, K);
@@ -265,7 +271,7 @@ static int launch_pool_as(const void *features, int c, const int32_t *nbr, int K
       cudaError_t e = allow_smem((const void *)pool_fwd_kernel<MODE, IN, PIECE>, p.smem);
       if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "%s: smem attribute: %s", name, cudaGetErrorString(e));
     }
-    pool_fwd_kernel<MODE, IN, PIECE><<<p.grid, 256, p.smem, st>>>(features, c, nbr, K, n_out, rf, out, n_out_dev, p.rows);
+    launch_ready(pool_fwd_kernel<MODE, IN, PIECE>, dim3(p.grid), dim3(256), p.smem, st, features, c, nbr, K, n_out, rf, out, n_out_dev, p.rows);
   }
   note_launches(1);
   if (MODE == 1 && rf != nullptr) {
@@ -322,7 +328,7 @@ extern "C" int ssc_global_avgpool_fwd(const float *feats, const int32_t *offsets
   if (n_samples == 0) return SSC_OK;
   SSC_REQUIRE(offsets && out, "global_avgpool: null pointer");
   dim3 grid(n_samples, ceil_div(c, 32)), block(32, 8);
-  { global_pool_kernel<false><<<grid, block, 0, as_stream(stream)>>>(feats, offsets, c, out, nullptr); note_launches(1); }
+  { launch_ready(global_pool_kernel<false>, dim3(grid), dim3(block), 0, as_stream(stream), feats, offsets, c, out, nullptr); note_launches(1); }
   SSC_CHECK_LAUNCH("global_avgpool");
   return SSC_OK;
 }
@@ -333,7 +339,7 @@ extern "C" int ssc_global_maxpool_fwd(const float *feats, const int32_t *offsets
   if (n_samples == 0) return SSC_OK;
   SSC_REQUIRE(offsets && out, "global_maxpool: null pointer");
   dim3 grid(n_samples, ceil_div(c, 32)), block(32, 8);
-  { global_pool_kernel<true><<<grid, block, 0, as_stream(stream)>>>(feats, offsets, c, out, maxidx); note_launches(1); }
+  { launch_ready(global_pool_kernel<true>, dim3(grid), dim3(block), 0, as_stream(stream), feats, offsets, c, out, maxidx); note_launches(1); }
   SSC_CHECK_LAUNCH("global_maxpool");
   return SSC_OK;
 }

@@ -125,6 +125,8 @@ __global__ void hash_insert_kernel(const int4 *__restrict__ indices, int n, int 
 // Dense alternative to hash_insert_kernel: row_map[flat input cell] = row + 1 (largest row wins on duplicates).
 __global__ void map_insert_kernel(const int4 *__restrict__ indices, int n, int batch, Geometry g,
                                   int32_t *__restrict__ row_map, int32_t *status, const int32_t *__restrict__ n_dev) {
+  after_previous();
+  next_may_start();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= live_rows(n, n_dev)) return;
   int4 c = indices[j];
@@ -188,6 +190,8 @@ constexpr int kMarkImageWords = 1024;
 __global__ void __launch_bounds__(128)
 mark_outputs_kernel(const int4 *__restrict__ indices, int n, int batch, Geometry g, uint32_t *bitmap,
                     const int32_t *__restrict__ n_dev, int32_t *__restrict__ row_map, int32_t *status) {
+  after_previous();
+  next_may_start();
   __shared__ uint32_t image[kMarkImageWords];
   __shared__ unsigned cell_min, cell_max;
   __shared__ int any_row;
@@ -289,6 +293,8 @@ __global__ void mark_outputs_generic_kernel(const int4 *__restrict__ indices, in
 __global__ void decode_outputs_bits_kernel(const uint32_t *__restrict__ bitmap,
                                            const uint32_t *__restrict__ word_prefix, long long n_words,
                                            Geometry g, int n_out, int4 *out_indices) {
+  after_previous();
+  next_may_start();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long w = t >> 5;
   if (w >= n_words) return;
@@ -312,6 +318,8 @@ __global__ void decode_outputs_bits_kernel(const uint32_t *__restrict__ bitmap,
 __global__ void decode_outputs_kernel(const uint32_t *__restrict__ bitmap,
                                       const uint32_t *__restrict__ word_prefix, long long n_words,
                                       Geometry g, int n_out, int4 *out_indices) {
+  after_previous();
+  next_may_start();
   // one thread per bitmap word (32 cells): most words of a sparse grid are empty and leave at once;
   // the set bits of a word get consecutive ranks from the word's prefix.  The coordinates of the
   // word's first cell are decoded once (three integer divisions); a set bit is that cell plus its
@@ -346,9 +354,9 @@ constexpr long long kDecodePerBitMaxWords = 32768;
 static void launch_decode(const uint32_t *bitmap, const uint32_t *word_prefix, long long n_words, const Geometry &g, int n_out,
                           int4 *out_indices, cudaStream_t st) {
   if (n_words <= kDecodePerBitMaxWords) {
-    { decode_outputs_bits_kernel<<<ceil_div(n_words * 32, 256), 256, 0, st>>>(bitmap, word_prefix, n_words, g, n_out, out_indices); note_launches(1); }
+    { launch_ready(decode_outputs_bits_kernel, dim3(ceil_div(n_words * 32, 256)), dim3(256), 0, st, bitmap, word_prefix, n_words, g, n_out, out_indices); note_launches(1); }
   } else {
-    { decode_outputs_kernel<<<ceil_div(n_words, 256), 256, 0, st>>>(bitmap, word_prefix, n_words, g, n_out, out_indices); note_launches(1); }
+    { launch_ready(decode_outputs_kernel, dim3(ceil_div(n_words, 256)), dim3(256), 0, st, bitmap, word_prefix, n_words, g, n_out, out_indices); note_launches(1); }
   }
 }
 
@@ -365,6 +373,8 @@ template <int WORDS>
 __global__ void __launch_bounds__(kRankThreads)
 rank_decode_kernel(const uint32_t *__restrict__ bitmap, int n_words, Geometry g, int n_out, int4 *__restrict__ out_indices,
                    int32_t *__restrict__ total_dev, const int32_t *__restrict__ status, CountPost post) {
+  after_previous();
+  next_may_start();
   __shared__ uint32_t smem[33], word_s[WORDS], prefix_s[WORDS];
   const int w0 = (int)blockIdx.x * WORDS;
   uint32_t before = 0;
@@ -415,6 +425,8 @@ __global__ void __launch_bounds__(256)
 lookup_dense_kernel(const int4 *__restrict__ out_indices, int n_out, int batch, Geometry g,
                     const int32_t *__restrict__ row_map, int32_t *__restrict__ nbr,
                     int32_t *__restrict__ chunk_counts, int n_chunks, const int32_t *__restrict__ n_out_dev) {
+  after_previous();
+  next_may_start();
   extern __shared__ int32_t cnt[];  // [K] when counting
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
   const int n_rows = live_rows(n_out, n_out_dev);
@@ -659,7 +671,7 @@ static int build_hash(const int32_t *indices, int n_in, int batch, const Geometr
   if (s.row_map != nullptr) {
     cudaMemsetAsync(s.row_map, 0, (size_t)s.in_cells * 4, st);
     if (n_in > 0) {
-      { map_insert_kernel<<<ceil_div(n_in, 256), 256, 0, st>>>((const int4 *)indices, n_in, batch, g, s.row_map,
+      { launch_ready(map_insert_kernel, dim3(ceil_div(n_in, 256)), dim3(256), 0, st, (const int4 *)indices, n_in, batch, g, s.row_map,
                                                             status ? status : s.misc + 1, n_in_dev); note_launches(1); }
     }
     SSC_CHECK_LAUNCH("map_insert");
@@ -686,7 +698,7 @@ static int lookup_and_compact(const int32_t *out_indices, int n_out, int n_in, i
     const dim3 lgrid(ceil_div(n_out > 0 ? n_out : 1, 256), g.ksize[0]);
     const int side = g.ksize[1] == g.ksize[2] ? g.ksize[1] : 0;
     auto lookup = side == 3 ? lookup_dense_kernel<3> : side == 5 ? lookup_dense_kernel<5> : side == 2 ? lookup_dense_kernel<2> : lookup_dense_kernel<0>;
-    { lookup<<<lgrid, 256, K * sizeof(int32_t), st>>>(
+    { launch_ready(lookup, lgrid, dim3(256), K * sizeof(int32_t), st,
           (const int4 *)out_indices, n_out, batch, g, s.row_map, nbr, counts, n_chunks, n_out_dev); note_launches(1); }
   } else {
     dim3 grid(n_chunks, K);
@@ -869,7 +881,7 @@ static int mark_outputs(const char *who, const int32_t *indices, int n_in, int b
   }
   if (n_in > 0) {
     if (simple) {
-      { mark_outputs_kernel<<<ceil_div(n_in, 128), 128, 0, st>>>((const int4 *)indices, n_in, batch, g, s.bitmap, n_in_dev,
+      { launch_ready(mark_outputs_kernel, dim3(ceil_div(n_in, 128)), dim3(128), 0, st, (const int4 *)indices, n_in, batch, g, s.bitmap, n_in_dev,
                                                                 together ? s.row_map : nullptr, status ? status : s.misc + 1); note_launches(1); }
     } else {
       { mark_outputs_generic_kernel<<<ceil_div((long long)n_in * g.K, 256), 256, 0, st>>>((const int4 *)indices, n_in, batch, g, s.bitmap, n_in_dev); note_launches(1); }
@@ -891,8 +903,8 @@ static int rulebook_conv_ahead(const int32_t *indices, int n_in, int batch, cons
   const CountPost post = next_post(place);
   if (s.n_words <= kRankedWords) {
     const int n = (int)s.n_words;
-    if (n <= 8192) rank_decode_kernel<32><<<ceil_div(n, 32), kRankThreads, 0, st>>>(s.bitmap, n, g, n_out, (int4 *)out_indices, n_out_dev, status, post);
-    else rank_decode_kernel<128><<<ceil_div(n, 128), kRankThreads, 0, st>>>(s.bitmap, n, g, n_out, (int4 *)out_indices, n_out_dev, status, post);
+    if (n <= 8192) launch_ready(rank_decode_kernel<32>, dim3(ceil_div(n, 32)), dim3(kRankThreads), 0, st, s.bitmap, n, g, n_out, (int4 *)out_indices, n_out_dev, status, post);
+    else launch_ready(rank_decode_kernel<128>, dim3(ceil_div(n, 128)), dim3(kRankThreads), 0, st, s.bitmap, n, g, n_out, (int4 *)out_indices, n_out_dev, status, post);
     note_launches(1);
     SSC_CHECK_LAUNCH("rank_decode");
   } else {

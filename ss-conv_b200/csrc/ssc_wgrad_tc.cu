@@ -48,6 +48,8 @@ constexpr int WT_BLOCK = WT_K * 128;   // 32 channels of a chunk's pairs
 // loads in flight per lane.  HBM-bound: the table is read once.
 __global__ void __launch_bounds__(256)
 pair_bitmap_kernel(const int32_t *__restrict__ nbr, int n_out, int words_per_row, uint32_t *__restrict__ bitmap) {
+  after_previous();
+  next_may_start();
   const int w0 = ((int)blockIdx.x * 8 + (int)(threadIdx.x >> 5)) * 4, lane = threadIdx.x & 31;
   if (w0 >= words_per_row) return;
   const int32_t *row = nbr + (size_t)blockIdx.y * n_out;
@@ -74,6 +76,8 @@ __global__ void __launch_bounds__(256)
 pair_scatter_kernel(const int32_t *__restrict__ nbr, int n_out, int words_per_row,
                     const uint32_t *__restrict__ bitmap, const uint32_t *__restrict__ prefix,
                     int32_t *__restrict__ pair_out, int32_t *__restrict__ pair_in, int32_t *__restrict__ starts) {
+  after_previous();
+  next_may_start();
   __shared__ uint16_t list_s[8][1024];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kappa = blockIdx.y;
   const int w0 = ((int)blockIdx.x * 8 + warp) * 32, w = w0 + lane;
@@ -167,6 +171,8 @@ __device__ __forceinline__ void copy_block(uint32_t dst, const float *const (&g)
 __global__ void __launch_bounds__((2 * WT_MAX_STAGES + 5) * 32, 2)
 conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in,
                      const int32_t *__restrict__ starts, int K, float *__restrict__ partial, int32_t *status) {
+  after_previous();
+  next_may_start();
   extern __shared__ uint8_t smem_raw[];
   __shared__ int first[257];
   __shared__ uint64_t full_bars[WT_MAX_STAGES], empty_bars[WT_MAX_STAGES], accf_bars[2], acce_bars[2], done_bar;
@@ -436,6 +442,8 @@ template <int VEC>
 __global__ void __launch_bounds__(256)
 wgrad_reduce_shares_kernel(const float *__restrict__ partial, const int32_t *__restrict__ starts, int K, int shares, int elems,
                            float *__restrict__ out) {
+  after_previous();
+  next_may_start();
   __shared__ int first[257];
   __shared__ float sm[8][32 * VEC + 1];
   chunk_prefix(starts, K, first);
@@ -516,11 +524,11 @@ PairLists pair_lists_view(void *lists, int K, int n_out) {
 // bitmap of the table, popcount scan, scatter: three small launches
 int pair_lists_build(const int32_t *nbr, int K, int n_out, void *lists, PairLists *out, cudaStream_t st) {
   const ListPlan p = plan_lists(lists, K, n_out);
-  { pair_bitmap_kernel<<<dim3(ceil_div(p.wpr, 32), K), 256, 0, st>>>(nbr, n_out, p.wpr, p.bitmap); note_launches(1); }
+  { launch_ready(pair_bitmap_kernel, dim3(dim3(ceil_div(p.wpr, 32), K)), dim3(256), 0, st, nbr, n_out, p.wpr, p.bitmap); note_launches(1); }
   SSC_CHECK_LAUNCH("pair_bitmap");
   int rc = exclusive_scan_u32<true>(p.bitmap, p.words, p.prefix, p.block_sums, p.starts + K, nullptr, st);
   if (rc != 0) return rc;
-  { pair_scatter_kernel<<<dim3(ceil_div(p.wpr, 256), K), 256, 0, st>>>(nbr, n_out, p.wpr, p.bitmap, p.prefix, p.pair_out, p.pair_in, p.starts); note_launches(1); }
+  { launch_ready(pair_scatter_kernel, dim3(dim3(ceil_div(p.wpr, 256), K)), dim3(256), 0, st, nbr, n_out, p.wpr, p.bitmap, p.prefix, p.pair_out, p.pair_in, p.starts); note_launches(1); }
   SSC_CHECK_LAUNCH("pair_scatter");
   if (out) *out = PairLists{p.pair_out, p.pair_in, p.starts};
   return SSC_OK;
@@ -596,7 +604,7 @@ int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_wgrad(tf32): smem attribute: %s", cudaGetErrorString(e));
     const WtParams w = {features, out_grad, c_in, c_out, (staged & 1) ? (c_in + 3) & ~3 : c_in, (staged & 2) ? (c_out + 3) & ~3 : c_out,
                         (staged & 1) ? 0 : 1, (staged & 2) ? 0 : 1, p.n_pad, p.a_bytes, p.stage_bytes, p.stages, p.n_buf, p.in_rows ? 1 : 0, p.buf_cols, alarm_word()};
-    { conv_wgrad_tc_kernel<<<dim3(p.shares, p.co_blocks), (2 * p.stages + 5) * 32, p.smem, st>>>(w, pl.pair_out, pl.pair_in, pl.starts, K, partial, status); note_launches(1); }
+    { launch_ready(conv_wgrad_tc_kernel, dim3(dim3(p.shares, p.co_blocks)), dim3((2 * p.stages + 5) * 32), p.smem, st, w, pl.pair_out, pl.pair_in, pl.starts, K, partial, status); note_launches(1); }
     SSC_CHECK_LAUNCH("conv_wgrad_tc");
   } else if (p.small) {
     const dim3 grid(p.shares / 4, p.co_blocks);
@@ -611,8 +619,8 @@ int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int
   const bool vec = (elems & 3) == 0 && ((uintptr_t)partial & 15u) == 0;
   const int tiles = ceil_div(elems, vec ? 128 : 32), most = ceil_div(8 * sm_count(), K);      // one wave of blocks
   const dim3 grid(tiles < most ? tiles : most, K);
-  if (vec) wgrad_reduce_shares_kernel<4><<<grid, 256, 0, st>>>(partial, pl.starts, K, p.shares, elems, d_filters);
-  else wgrad_reduce_shares_kernel<1><<<grid, 256, 0, st>>>(partial, pl.starts, K, p.shares, elems, d_filters);
+  if (vec) launch_ready(wgrad_reduce_shares_kernel<4>, dim3(grid), dim3(256), 0, st, partial, pl.starts, K, p.shares, elems, d_filters);
+  else launch_ready(wgrad_reduce_shares_kernel<1>, dim3(grid), dim3(256), 0, st, partial, pl.starts, K, p.shares, elems, d_filters);
   note_launches(1);
   SSC_CHECK_LAUNCH("conv_wgrad_reduce");
   return SSC_OK;

@@ -697,3 +697,51 @@ def test_filter_gradient_of_staged_operands(cuda, c_in, c_out, n):
                                           _p(got), _p(_ext.status_word(cuda)), _p(scratch), scratch.numel(), _stream()))
         assert torch.equal(got, want)
     _ext.check_status(cuda)
+
+
+@pytest.mark.parametrize("n,channels", [(90, 12), (900, 24)])
+def test_kernels_queued_behind_one_another(cuda, monkeypatch, n, channels):
+    """A training step over one set of rows after another, all queued while the device is busy, gives the gradients of the
+    same calls with the device idle between any two.  Every call writes buffers that the step before has just read, so a
+    kernel that started on unfinished rows would be off by the size of the values.  Sums that are added up in another
+    order can move an operand by one step of TF32, 2^-11 of it, in each of the four convolutions of the two directions."""
+    from ss_conv import _ext
+    from ss_conv.activation import Activation
+    from ss_conv.batchnorm import BatchNorm
+    from ss_conv.convolution import Convolution
+    from ss_conv.pool import MaxPool
+    from ss_conv.sp_ops.tensor import SparseTensor
+    torch.manual_seed(n)
+    rng = np.random.RandomState(n)
+    fields = [(channels // 4, 0), (channels // 4, 1)]
+    gated = fields + [(channels // 4, 0)]
+    net = [Convolution([(4, 0)], gated, 3, padding=1, subm=True), BatchNorm(gated), Activation(fields, (torch.relu, torch.sigmoid)),
+           Convolution(fields, gated, 3, stride=2, padding=1), BatchNorm(gated), Activation(fields, (torch.relu, torch.sigmoid)),
+           MaxPool(2, stride=2)]
+    net = [m.to(cuda).train() for m in net]
+    sets = [dev(random_voxels(rng, 2, 12, n), cuda) for _ in range(4)]
+    rows = [torch.randn(len(i), 4, device=cuda) for i in sets]
+
+    def steps():
+        out = []
+        torch.cuda._sleep(20_000_000)
+        for i, f in zip(sets, rows):
+            x = SparseTensor(f, i, [12] * 3, 2)
+            for m in net:
+                x = m(x)
+            grads = torch.autograd.grad((x.features * torch.arange(1, x.features.shape[1] + 1, device=cuda)).sum(),
+                                        [p for m in net for p in m.parameters() if p.requires_grad], allow_unused=True)
+            out.append([x.features.detach()] + [g for g in grads if g is not None])
+        torch.cuda.synchronize()
+        return [[t.cpu().numpy() for t in o] for o in out]
+
+    steps()
+    queued = steps()
+    check = _ext._check
+    monkeypatch.setattr(_ext, "_check", lambda rc: (check(rc), torch.cuda.synchronize()))
+    alone = steps()
+    _ext.check_status(cuda)
+    for got, want in zip(queued, alone):
+        assert len(got) == len(want) > 6
+        for a, b in zip(got, want):
+            assert rel_err(a, b) < 4 * 2.0 ** -11
