@@ -19,6 +19,8 @@
 namespace ssc {
 
 __global__ void nbr_transpose_kernel(const int32_t *__restrict__ nbr, int n_out, int n_in, int32_t *__restrict__ nbr_in) {
+  after_previous();
+  next_may_start();
   int o = blockIdx.x * blockDim.x + threadIdx.x;
   int kappa = blockIdx.y;
   if (o >= n_out) return;
@@ -34,6 +36,8 @@ __global__ void __launch_bounds__(256)
 conv_wgrad_partial_kernel(const float *__restrict__ features, int c_in, const float *__restrict__ out_grad, int c_out,
                           const int32_t *__restrict__ nbr, int n_out, int rows_per_split, int tiles_co,
                           float *__restrict__ partial) {
+  after_previous();
+  next_may_start();
   __shared__ float As[WG_ROWS][WG_T + 4];
   __shared__ float Bs[WG_ROWS][WG_T + 4];
   __shared__ int rows[WG_ROWS];
@@ -89,6 +93,8 @@ conv_wgrad_partial_kernel(const float *__restrict__ features, int c_in, const fl
 }
 
 __global__ void wgrad_reduce_kernel(const float *__restrict__ partial, int splits, long long elems, float *__restrict__ out) {
+  after_previous();
+  next_may_start();
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= elems) return;
   float s = 0.f;
@@ -105,6 +111,8 @@ __global__ void __launch_bounds__(256)
 pool_bwd_kernel(const float *__restrict__ features, const float *__restrict__ out_features,
                 const float *__restrict__ out_grad, int c, const int32_t *__restrict__ nbr_in, int K,
                 int n_in, const int32_t *__restrict__ summaryrf, float *__restrict__ d_in, int R) {
+  after_previous();
+  next_may_start();
   extern __shared__ int32_t pool_smem[];
   struct Item {
     Channels g, y;
@@ -145,6 +153,8 @@ pool_bwd_kernel(const float *__restrict__ features, const float *__restrict__ ou
 // grid (samples, channel groups of 32), block (32, 8)
 __global__ void global_avgpool_bwd_kernel(const float *__restrict__ d_out, const int32_t *__restrict__ offsets, int c,
                                           float *__restrict__ d_feats) {
+  after_previous();
+  next_may_start();
   const int s = blockIdx.x, ch = blockIdx.y * 32 + threadIdx.x;
   const int start = offsets[s], end = offsets[s + 1];
   if (ch >= c || end <= start) return;
@@ -154,6 +164,8 @@ __global__ void global_avgpool_bwd_kernel(const float *__restrict__ d_out, const
 
 __global__ void global_maxpool_bwd_kernel(const float *__restrict__ d_out, const int32_t *__restrict__ maxidx, long long total,
                                           int c, long long n_rows, float *__restrict__ d_feats) {
+  after_previous();
+  next_may_start();
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= total) return;
   const int row = maxidx[e];
@@ -164,6 +176,8 @@ __global__ void global_maxpool_bwd_kernel(const float *__restrict__ d_out, const
 // row [count, point ids...].  A point is listed by one voxel only, so plain stores suffice.
 __global__ void voxelize_bwd_kernel(const float *__restrict__ d_out, const int32_t *__restrict__ rules, int n_voxel,
                                     int max_active, int c, int average, float *__restrict__ d_feats) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n_voxel * c) return;
   const int v = (int)(t / c), ch = (int)(t - (long long)v * c);
@@ -178,6 +192,8 @@ __global__ void voxelize_bwd_kernel(const float *__restrict__ d_out, const int32
 __global__ void three_interpolate_bwd_kernel(int c, int n, const float *__restrict__ grad_out,
                                              const int32_t *__restrict__ idx, const float *__restrict__ weight,
                                              float *__restrict__ grad_points) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n * c) return;
   const int p = (int)(t / c), ch = (int)(t - (long long)p * c);
@@ -204,7 +220,7 @@ extern "C" int ssc_voxelize_bwd(const float *d_out, const int32_t *rules, int mo
   if (n_voxel == 0 || n_point == 0) return SSC_OK;
   SSC_REQUIRE(d_out && rules, "voxelize_bwd: null pointer");
   long long total = (long long)n_voxel * c;
-  { voxelize_bwd_kernel<<<ceil_div(total, 256), 256, 0, st>>>(d_out, rules, n_voxel, max_active, c, mode == 4, d_feats); note_launches(1); }
+  { launch_ready(voxelize_bwd_kernel, dim3(ceil_div(total, 256)), dim3(256), 0, st, d_out, rules, n_voxel, max_active, c, mode == 4, d_feats); note_launches(1); }
   SSC_CHECK_LAUNCH("voxelize_bwd");
   return SSC_OK;
 }
@@ -220,7 +236,7 @@ extern "C" int ssc_three_interpolate_bwd(int c, int n, int m, const float *grad_
   if (n == 0 || m == 0) return SSC_OK;
   SSC_REQUIRE(grad_out && idx && weight, "three_interpolate_bwd: null pointer");
   long long total = (long long)n * c;
-  { three_interpolate_bwd_kernel<<<ceil_div(total, 256), 256, 0, st>>>(c, n, grad_out, idx, weight, grad_points); note_launches(1); }
+  { launch_ready(three_interpolate_bwd_kernel, dim3(ceil_div(total, 256)), dim3(256), 0, st, c, n, grad_out, idx, weight, grad_points); note_launches(1); }
   SSC_CHECK_LAUNCH("three_interpolate_bwd");
   return SSC_OK;
 }
@@ -233,7 +249,7 @@ extern "C" int ssc_nbr_transpose(const int32_t *nbr, int K, int n_out, int n_in,
   cudaMemsetAsync(nbr_in, 0xFF, (size_t)K * n_in * 4, st);
   if (n_out > 0) {
     dim3 grid(ceil_div(n_out, 256), K);
-    { nbr_transpose_kernel<<<grid, 256, 0, st>>>(nbr, n_out, n_in, nbr_in); note_launches(1); }
+    { launch_ready(nbr_transpose_kernel, dim3(grid), dim3(256), 0, st, nbr, n_out, n_in, nbr_in); note_launches(1); }
   }
   SSC_CHECK_LAUNCH("nbr_transpose");
   return SSC_OK;
@@ -298,10 +314,10 @@ extern "C" int ssc_conv_wgrad_lists(const float *features, int c_in, const float
   rows_per_split = ceil_div(rows_per_split, WG_ROWS) * WG_ROWS;
   const int tiles_co = ceil_div(c_out, WG_T);
   dim3 grid(splits, K, ceil_div(c_in, WG_T) * tiles_co);
-  { conv_wgrad_partial_kernel<<<grid, 256, 0, st>>>(features, c_in, out_grad, c_out, nbr, n_out, rows_per_split, tiles_co,
+  { launch_ready(conv_wgrad_partial_kernel, dim3(grid), dim3(256), 0, st, features, c_in, out_grad, c_out, nbr, n_out, rows_per_split, tiles_co,
                                                    (float *)scratch); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_wgrad_partial");
-  { wgrad_reduce_kernel<<<ceil_div(elems, 256), 256, 0, st>>>((const float *)scratch, splits, elems, d_filters); note_launches(1); }
+  { launch_ready(wgrad_reduce_kernel, dim3(ceil_div(elems, 256)), dim3(256), 0, st, (const float *)scratch, splits, elems, d_filters); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_wgrad_reduce");
   return SSC_OK;
 }
@@ -328,7 +344,7 @@ static int launch_pool_bwd(const float *features, const float *out_features, con
     cudaError_t e = allow_smem((const void *)kernel, p.smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "%s: smem attribute: %s", name, cudaGetErrorString(e));
   }
-  kernel<<<p.grid, 256, p.smem, as_stream(stream)>>>(features, out_features, out_grad, c, nbr_in, K, n_in, rf, d_in, p.rows);
+  launch_ready(kernel, dim3(p.grid), dim3(256), p.smem, as_stream(stream), features, out_features, out_grad, c, nbr_in, K, n_in, rf, d_in, p.rows);
   note_launches(1);
   SSC_CHECK_LAUNCH(name);
   return SSC_OK;
@@ -353,7 +369,7 @@ extern "C" int ssc_global_avgpool_bwd(const float *d_out, const int32_t *offsets
   if (n_samples == 0 || n_rows == 0) return SSC_OK;
   SSC_REQUIRE(d_out && offsets && d_feats, "global_avgpool_bwd: null pointer");
   dim3 grid(n_samples, ceil_div(c, 32)), block(32, 8);
-  { global_avgpool_bwd_kernel<<<grid, block, 0, st>>>(d_out, offsets, c, d_feats); note_launches(1); }
+  { launch_ready(global_avgpool_bwd_kernel, dim3(grid), dim3(block), 0, st, d_out, offsets, c, d_feats); note_launches(1); }
   SSC_CHECK_LAUNCH("global_avgpool_bwd");
   return SSC_OK;
 }
@@ -366,7 +382,7 @@ extern "C" int ssc_global_maxpool_bwd(const float *d_out, const int32_t *maxidx,
   if (n_samples == 0 || n_rows == 0) return SSC_OK;
   SSC_REQUIRE(d_out && maxidx && d_feats, "global_maxpool_bwd: null pointer");
   long long total = (long long)n_samples * c;
-  { global_maxpool_bwd_kernel<<<ceil_div(total, 256), 256, 0, st>>>(d_out, maxidx, total, c, n_rows, d_feats); note_launches(1); }
+  { launch_ready(global_maxpool_bwd_kernel, dim3(ceil_div(total, 256)), dim3(256), 0, st, d_out, maxidx, total, c, n_rows, d_feats); note_launches(1); }
   SSC_CHECK_LAUNCH("global_maxpool_bwd");
   return SSC_OK;
 }

@@ -9,6 +9,8 @@ namespace ssc {
 __global__ void bn_fold_kernel(const float *running_mean, const float *running_var, const float *weight,
                                const float *bias, const int32_t *field_of_channel, const int32_t *scalar_of_channel,
                                int c, float eps, float *scale, float *shift) {
+  after_previous();
+  next_may_start();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
   int f = field_of_channel[ch], s = scalar_of_channel[ch];
@@ -29,6 +31,8 @@ __global__ void bn_gate_kernel(const float *__restrict__ x, long long total, int
                                const int32_t *__restrict__ gate_of_channel, int c_out, int c_gate_base,
                                int scalar_act, int gate_act, const float *__restrict__ scalar_bias,
                                const float *__restrict__ gate_bias, float *__restrict__ out) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= total) return;
   long long row = t / c_out;
@@ -59,6 +63,8 @@ bn_gate_vec4_kernel(const float *__restrict__ x, uint32_t total, uint32_t groups
                     const float *__restrict__ scale, const float *__restrict__ shift,
                     const int32_t *__restrict__ gate_of_channel, int c_gate_base, int scalar_act, int gate_act,
                     const float *__restrict__ scalar_bias, const float *__restrict__ gate_bias, float *__restrict__ out) {
+  after_previous();
+  next_may_start();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= total) return;
   const uint32_t row = t / groups, g4 = t - row * groups;
@@ -109,6 +115,8 @@ bn_gate_vec4_out16_kernel(const float *__restrict__ x, uint32_t total, uint32_t 
                     const float *__restrict__ scale, const float *__restrict__ shift,
                     const int32_t *__restrict__ gate_of_channel, int c_gate_base, int scalar_act, int gate_act,
                     const float *__restrict__ scalar_bias, const float *__restrict__ gate_bias, uint2 *__restrict__ out) {
+  after_previous();
+  next_may_start();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= total) return;
   const uint32_t row = t / groups, g4 = t - row * groups;
@@ -249,7 +257,7 @@ static bool launch_bn_gate_rows(const float *x, int n, uint32_t groups, int c_in
   const uint32_t R = 256u / groups;
   const size_t smem = (size_t)R * n_gates * sizeof(float);
   if (smem > 48 * 1024) return false;
-  { launch_ready(bn_gate_rows_kernel<OUT, VEC>, dim3(ceil_div(n, (int)R)), dim3(dim3(groups, R)), smem, st, x, (uint32_t)n, groups, c_in_total, scale, shift,
+  { launch_ready(bn_gate_rows_kernel<OUT, VEC>, dim3(ceil_div(n, (int)R)), dim3(groups, R), smem, st, x, (uint32_t)n, groups, c_in_total, scale, shift,
                                                                           gate_of_channel, c_gate_base, n_gates, scalar_act, gate_act,
                                                                           scalar_bias, gate_bias, out); note_launches(1); }
   return true;
@@ -467,6 +475,8 @@ template <int PASS, int VEC>
 __global__ void __launch_bounds__(256)
 bn_gate_bwd_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
                    float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
+  after_previous();
+  next_may_start();
   extern __shared__ __align__(16) float sm[];
   const int R = p.rows, c = p.c, c_out = p.c_out, n_gates = p.n_gates;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -836,6 +846,8 @@ template <int PASS>
 __global__ void __launch_bounds__(256)
 bn_gate_bwd_wide_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
                         float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
+  after_previous();
+  next_may_start();
   const int ch = (int)(blockIdx.y * 256 + threadIdx.x);
   if (ch >= p.c) return;
   auto normed = [&](const float *xr, int k) { return p.scale ? fmaf(__ldg(xr + k), __ldg(p.scale + k), __ldg(p.shift + k)) : __ldg(xr + k); };
@@ -904,6 +916,8 @@ bn_bwd_finish_kernel(const float *__restrict__ part_a, const float *__restrict__
 
 // chan_mean[ch] = mean of a scalar channel (0 for l>0 channels).
 __global__ void bn_chan_mean_kernel(const float *mean, const int32_t *scalar_of_channel, int c, float *chan_mean) {
+  after_previous();
+  next_may_start();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c) return;
   const int s = scalar_of_channel[i];
@@ -918,7 +932,7 @@ extern "C" int ssc_bn_fold(const float *running_mean, const float *running_var, 
                            const float *bias, const int32_t *field_of_channel, const int32_t *scalar_of_channel,
                            int c, float eps, float *scale, float *shift, void *stream) {
   SSC_REQUIRE(c >= 1 && running_var && field_of_channel && scalar_of_channel && scale && shift, "bn_fold: bad arguments");
-  { bn_fold_kernel<<<ceil_div(c, 128), 128, 0, as_stream(stream)>>>(running_mean, running_var, weight, bias,
+  { launch_ready(bn_fold_kernel, dim3(ceil_div(c, 128)), dim3(128), 0, as_stream(stream), running_mean, running_var, weight, bias,
                                                                  field_of_channel, scalar_of_channel, c, eps, scale, shift); note_launches(1); }
   SSC_CHECK_LAUNCH("bn_fold");
   return SSC_OK;
@@ -942,7 +956,7 @@ extern "C" int ssc_bn_gate_fwd(const float *x, int n, int c_in_total, const floa
       SSC_CHECK_LAUNCH("bn_gate_fwd");
       return SSC_OK;
     }
-    { bn_gate_vec4_kernel<<<ceil_div(total4, 256), 256, 0, as_stream(stream)>>>(x, total4, groups, c_in_total, scale, shift,
+    { launch_ready(bn_gate_vec4_kernel, dim3(ceil_div(total4, 256)), dim3(256), 0, as_stream(stream), x, total4, groups, c_in_total, scale, shift,
                                                                             gate_of_channel, c_gate_base, scalar_act, gate_act,
                                                                             scalar_bias, gate_bias, out); note_launches(1); }
     SSC_CHECK_LAUNCH("bn_gate_fwd");
@@ -958,7 +972,7 @@ extern "C" int ssc_bn_gate_fwd(const float *x, int n, int c_in_total, const floa
     SSC_CHECK_LAUNCH("bn_gate_fwd");
     return SSC_OK;
   }
-  { bn_gate_kernel<<<ceil_div(total, 256), 256, 0, as_stream(stream)>>>(x, total, c_in_total, scale, shift, gate_of_channel,
+  { launch_ready(bn_gate_kernel, dim3(ceil_div(total, 256)), dim3(256), 0, as_stream(stream), x, total, c_in_total, scale, shift, gate_of_channel,
                                                                      c_out, c_gate_base, scalar_act, gate_act,
                                                                      scalar_bias, gate_bias, out); note_launches(1); }
   SSC_CHECK_LAUNCH("bn_gate_fwd");
@@ -990,9 +1004,9 @@ extern "C" int ssc_bn_gate_fwd16(const float *x, int n, int c_in_total, const fl
     return SSC_OK;
   }
   if (precision == SSC_PREC_BF16) {
-    { bn_gate_vec4_out16_kernel<2><<<ceil_div(total4, 256), 256, 0, as_stream(stream)>>>(x, total4, groups, c_in_total, scale, shift, gate_of_channel, c_gate_base, scalar_act, gate_act, scalar_bias, gate_bias, (uint2 *)out16); note_launches(1); }
+    { launch_ready(bn_gate_vec4_out16_kernel<2>, dim3(ceil_div(total4, 256)), dim3(256), 0, as_stream(stream), x, total4, groups, c_in_total, scale, shift, gate_of_channel, c_gate_base, scalar_act, gate_act, scalar_bias, gate_bias, (uint2 *)out16); note_launches(1); }
   } else {
-    { bn_gate_vec4_out16_kernel<1><<<ceil_div(total4, 256), 256, 0, as_stream(stream)>>>(x, total4, groups, c_in_total, scale, shift, gate_of_channel, c_gate_base, scalar_act, gate_act, scalar_bias, gate_bias, (uint2 *)out16); note_launches(1); }
+    { launch_ready(bn_gate_vec4_out16_kernel<1>, dim3(ceil_div(total4, 256)), dim3(256), 0, as_stream(stream), x, total4, groups, c_in_total, scale, shift, gate_of_channel, c_gate_base, scalar_act, gate_act, scalar_bias, gate_bias, (uint2 *)out16); note_launches(1); }
   }
   SSC_CHECK_LAUNCH("bn_gate_fwd16");
   return SSC_OK;
@@ -1074,7 +1088,7 @@ static int launch_bwd_vec(const BnGateBwd &p, size_t smem, const float *ks, cons
   }
   int blocks = PASS == 0 ? p.chains : ceil_div(p.n, p.rows);
   if (PASS == 1 && blocks > 5 * 148) blocks = 5 * 148;
-  bn_gate_bwd_kernel<PASS, VEC><<<dim3(blocks, PASS == 0 ? ceil_div(p.c, 256 * kBwdMaxAcc) : 1), 256, smem, st>>>(p, ks, ka, kg, gx, part_a, part_g);
+  launch_ready(bn_gate_bwd_kernel<PASS, VEC>, dim3(blocks, PASS == 0 ? ceil_div(p.c, 256 * kBwdMaxAcc) : 1), dim3(256), smem, st, p, ks, ka, kg, gx, part_a, part_g);
   note_launches(1);
   SSC_CHECK_LAUNCH("bn_gate_bwd");
   return SSC_OK;
@@ -1113,7 +1127,7 @@ static int launch_bwd(BnGateBwd p, const float *ks, const float *ka, const float
   p.rows = bwd_tile_rows(p.c, p.c_out, p.n_gates, PASS == 0 ? 32 : 64, &smem);
   if (smem > 227 * 1024) {
     const int blocks = PASS == 0 ? p.chains : (p.n < 4 * 148 ? p.n : 4 * 148);
-    bn_gate_bwd_wide_kernel<PASS><<<dim3(blocks, ceil_div(p.c, 256)), 256, 0, st>>>(p, ks, ka, kg, gx, part_a, part_g);
+    launch_ready(bn_gate_bwd_wide_kernel<PASS>, dim3(blocks, ceil_div(p.c, 256)), dim3(256), 0, st, p, ks, ka, kg, gx, part_a, part_g);
     note_launches(1);
     SSC_CHECK_LAUNCH("bn_gate_bwd");
     return SSC_OK;
@@ -1156,7 +1170,7 @@ extern "C" int ssc_bn_bwd(const float *x, const float *gy, int n, int c, const i
   SSC_REQUIRE(n_scalar == 0 || mean, "bn_bwd: null pointer");
   SSC_REQUIRE(scalar_of_channel && scratch && scratch_bytes >= ssc_bn_scratch_bytes(n, c), "bn_bwd: scratch too small (ssc_bn_scratch_bytes)");
   float *chan_mean = (float *)scratch + (size_t)2 * 8 * bn_row_blocks(n) * c + (size_t)3 * c;
-  { bn_chan_mean_kernel<<<ceil_div(c, 128), 128, 0, as_stream(stream)>>>(mean, scalar_of_channel, c, chan_mean); note_launches(1); }
+  { launch_ready(bn_chan_mean_kernel, dim3(ceil_div(c, 128)), dim3(128), 0, as_stream(stream), mean, scalar_of_channel, c, chan_mean); note_launches(1); }
   SSC_CHECK_LAUNCH("bn_chan_mean");
   return ssc_bn_gate_bwd(x, gy, n, c, c, field_of_channel, scalar_of_channel, n_field, nullptr, nullptr, chan_mean, var, weight, eps, training,
                          nullptr, nullptr, nullptr, 0, 0, gx, d_weight, d_bias, scratch, scratch_bytes, stream);

@@ -46,6 +46,8 @@ materialize_bwd_kernel(const float *__restrict__ g, const float *__restrict__ ba
                        int n_blocks_in, const int32_t *__restrict__ out_field, const int32_t *__restrict__ in_field,
                        const int32_t *__restrict__ out_start, const int32_t *__restrict__ in_start, int c_out, int c_in, int K,
                        int staged, float *__restrict__ d_weight) {
+  after_previous();
+  next_may_start();
   extern __shared__ float gs[];
   const int co0 = out_start[blockIdx.y], ci0 = in_start[blockIdx.x];
   const int i = out_field[co0 * 3], u = out_field[co0 * 3 + 1], j = in_field[ci0 * 3], v = in_field[ci0 * 3 + 1];
@@ -90,6 +92,8 @@ __global__ void __launch_bounds__(256)
 conv_fwd_fp32_kernel(const float *__restrict__ features, int c_in, const float *__restrict__ filters, int K,
                      int c_out, const int32_t *__restrict__ nbr, int n_out, int rev, float *__restrict__ out,
                      const int32_t *__restrict__ n_out_dev) {
+  after_previous();
+  next_may_start();
   __shared__ float As[BK][BM + 4];
   __shared__ float Bs[BK][BN + 4];
   __shared__ int rows[BM];
@@ -304,6 +308,8 @@ __global__ void __launch_bounds__(SM_WARPS * 32)
 conv_fwd_fp32_warps_kernel(const float *__restrict__ features, int c_in, const float *__restrict__ filters, int K,
                            int c_out, const int32_t *__restrict__ nbr, int n_out, int rev, float *__restrict__ out,
                            const int32_t *__restrict__ n_out_dev) {
+  after_previous();
+  next_may_start();
   extern __shared__ float ws[];               // [K][c_in][NJ * 32]
   const int n_rows = live_rows(n_out, n_out_dev);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.y * NJ * 32;
@@ -396,7 +402,7 @@ static int launch_fp32_warps(const float *features, int c_in, const float *filte
     cudaError_t e = allow_smem((const void *)kernel, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(fp32): smem attribute: %s", cudaGetErrorString(e));
   }
-  { kernel<<<grid, SM_WARPS * 32, staged ? smem : 0, st>>>(features, c_in, filters, K, c_out, nbr, n_out, rev, out, n_out_dev); note_launches(1); }
+  { launch_ready(kernel, grid, dim3(SM_WARPS * 32), staged ? smem : 0, st, features, c_in, filters, K, c_out, nbr, n_out, rev, out, n_out_dev); note_launches(1); }
   SSC_CHECK_LAUNCH("conv_fwd_fp32");
   return SSC_OK;
 }
@@ -430,7 +436,7 @@ extern "C" int ssc_materialize_bwd(const float *d_filters, const float *basis, c
     cudaError_t e = allow_smem((const void *)materialize_bwd_kernel, need);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "materialize_bwd: smem attribute: %s", cudaGetErrorString(e));
   }
-  { materialize_bwd_kernel<<<dim3(n_in, n_out), kMatBwdThreads, staged ? need : 0, as_stream(stream)>>>(
+  { launch_ready(materialize_bwd_kernel, dim3(n_in, n_out), dim3(kMatBwdThreads), staged ? need : 0, as_stream(stream), 
         d_filters, basis, block_table, n_blocks_in, out_field, in_field, out_start, in_start, c_out, c_in, K, staged, d_weight); note_launches(1); }
   SSC_CHECK_LAUNCH("materialize_bwd");
   return SSC_OK;
@@ -485,7 +491,7 @@ extern "C" int ssc_conv_fwd_ordered(const float *features, int n_in, int c_in, c
       return launch_fp32_warps<3>(features, c_in, w, K, c_out, nbr, n_out, rev, out, n_out_dev, st);
     }
     dim3 grid(ceil_div(n_out, BM), ceil_div(c_out, BN));
-    { conv_fwd_fp32_kernel<<<grid, 256, 0, st>>>(features, c_in, (const float *)filters, K, c_out, nbr, n_out, table_form != 0, out, n_out_dev); note_launches(1); }
+    { launch_ready(conv_fwd_fp32_kernel, dim3(grid), dim3(256), 0, st, features, c_in, (const float *)filters, K, c_out, nbr, n_out, table_form != 0, out, n_out_dev); note_launches(1); }
     SSC_CHECK_LAUNCH("conv_fwd_fp32");
     return SSC_OK;
   }

@@ -42,6 +42,8 @@ stage_features_kernel(const float4 *__restrict__ in, long long total_vec, uint4 
 // Channel counts that are not a multiple of four: rows padded with zeros to c_pad floats.
 __global__ void stage_features_padded_kernel(const float *__restrict__ in, long long n_rows, int c_in, int c_pad,
                                              long long total, uint32_t *__restrict__ out) {
+  after_previous();
+  next_may_start();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long step = (long long)gridDim.x * blockDim.x;
   for (; i < total; i += step) {
@@ -56,6 +58,8 @@ __global__ void stage_features_padded_kernel(const float *__restrict__ in, long 
 // division per element).
 __global__ void __launch_bounds__(256)
 stage_features_padded_rows_kernel(const float *__restrict__ in, int n_rows, int c_in, uint4 *__restrict__ out) {
+  after_previous();
+  next_may_start();
   const int row = blockIdx.x * blockDim.y + threadIdx.y, c0 = threadIdx.x * 4;
   if (row >= n_rows) return;
   const float *src = in + (size_t)row * c_in + c0;
@@ -77,12 +81,12 @@ int stage_features(const float *features, int n_in, int c_in, void *staged, cuda
     { launch_ready(stage_features_kernel, dim3(ceil_div(total_vec, 256 * STAGE_VECS)), dim3(256), 0, st, (const float4 *)features, total_vec, (uint4 *)staged); note_launches(1); }
   } else if (c_pad <= 1024) {
     const int groups = c_pad >> 2, rows = 256 / groups;
-    { stage_features_padded_rows_kernel<<<ceil_div(n_in, rows), dim3(groups, rows), 0, st>>>(features, n_in, c_in, (uint4 *)staged); note_launches(1); }
+    { launch_ready(stage_features_padded_rows_kernel, dim3(ceil_div(n_in, rows)), dim3(groups, rows), 0, st, features, n_in, c_in, (uint4 *)staged); note_launches(1); }
   } else {
     const long long total = (long long)n_in * c_pad;
     int blocks = ceil_div(total, 256 * 4);
     if (blocks > sm_count() * 16) blocks = sm_count() * 16;
-    { stage_features_padded_kernel<<<blocks, 256, 0, st>>>(features, n_in, c_in, c_pad, total, (uint32_t *)staged); note_launches(1); }
+    { launch_ready(stage_features_padded_kernel, dim3(blocks), dim3(256), 0, st, features, n_in, c_in, c_pad, total, (uint32_t *)staged); note_launches(1); }
   }
   SSC_CHECK_LAUNCH("stage_features");
   return SSC_OK;
@@ -93,6 +97,8 @@ int stage_features(const float *features, int n_in, int c_in, void *staged, cuda
 template <bool BF16>
 __global__ void stage_features_16_kernel(const float *__restrict__ in, long long n_rows, int c_in, int c_pad,
                                          long long total_pairs, uint32_t *__restrict__ out) {
+  after_previous();
+  next_may_start();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long step = (long long)gridDim.x * blockDim.x;
   const int pairs = c_pad >> 1;
@@ -145,8 +151,8 @@ int stage_features_16(const float *features, int n_in, int c_in, bool bf16, void
   int blocks = ceil_div(total_pairs, 256 * 4);
   const int max_blocks = sm_count() * 16;
   if (blocks > max_blocks) blocks = max_blocks;
-  if (bf16) { stage_features_16_kernel<true><<<blocks, 256, 0, st>>>(features, n_in, c_in, words * 2, total_pairs, (uint32_t *)staged); note_launches(1); }
-  else { stage_features_16_kernel<false><<<blocks, 256, 0, st>>>(features, n_in, c_in, words * 2, total_pairs, (uint32_t *)staged); note_launches(1); }
+  if (bf16) { launch_ready(stage_features_16_kernel<true>, dim3(blocks), dim3(256), 0, st, features, n_in, c_in, words * 2, total_pairs, (uint32_t *)staged); note_launches(1); }
+  else { launch_ready(stage_features_16_kernel<false>, dim3(blocks), dim3(256), 0, st, features, n_in, c_in, words * 2, total_pairs, (uint32_t *)staged); note_launches(1); }
   SSC_CHECK_LAUNCH("stage_features_16");
   return SSC_OK;
 }

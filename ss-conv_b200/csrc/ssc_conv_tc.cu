@@ -121,6 +121,8 @@ bool tc_operand_layout(int c_in, int c_out, int *k_slabs, int *n_pad, int *tile_
 // swizzled operand layout (row = output channel, 16-byte chunk index XOR (row & 7)).
 __global__ void pack_filters_tf32_kernel(const float *__restrict__ filters, int K, int c_in, int c_out, TcParams p,
                                          uint4 *__restrict__ packed) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long total = (long long)K * p.k_slabs * p.n_pad * 8;
   if (t >= total) return;
@@ -146,6 +148,8 @@ __global__ void pack_filters_tf32_kernel(const float *__restrict__ filters, int 
 // [ceil(K / opk)][n_pad rows][32 tf32], word (o' * c_pad + c) of a row = W[g * opk + o', c, n].
 __global__ void pack_filters_tf32_grouped_kernel(const float *__restrict__ filters, int K, int c_in, int c_out, int c_pad,
                                                  int opk, int n_groups, int n_pad, uint4 *__restrict__ packed) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long total = (long long)n_groups * n_pad * 8;
   if (t >= total) return;
@@ -174,6 +178,8 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
                      int c_out, const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out,
                      int32_t *status, TcParams p, const int32_t *__restrict__ n_out_dev,
                      const int32_t *__restrict__ order) {
+  after_previous();
+  next_may_start();
   // `order` (may be NULL): the rows of tile t are order[128 t .. 128 t + 127] instead of the same
   // consecutive numbers; rows that use the same kernel offsets, put next to each other, make a
   // tile skip the offsets none of them uses.
@@ -982,6 +988,8 @@ static size_t tc_smem_bytes(const TcParams &p) {
 template <bool BF16>
 __global__ void pack_filters_16_kernel(const float *__restrict__ filters, int K, int c_in, int c_out, TcParams p,
                                         uint4 *__restrict__ packed) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long total = (long long)K * p.k_slabs * p.n_pad * 8;
   if (t >= total) return;
@@ -1140,7 +1148,7 @@ int conv_fwd_tf32(const float *features, int n_in, int c_in, const void *packed,
     auto kernel = opk > 1 ? conv_fwd_tf32_kernel<true> : conv_fwd_tf32_kernel<false>;
     cudaError_t e = allow_smem((const void *)kernel, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_fwd(tf32): smem attribute: %s", cudaGetErrorString(e));
-    kernel<<<grid2, p.threads, smem, st>>>(staged ? (const float *)scratch : features, staged ? c_pad : c_in, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order);
+    launch_ready(kernel, grid2, dim3(p.threads), smem, st, staged ? (const float *)scratch : features, staged ? c_pad : c_in, (const uint4 *)packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order);
   }
   note_launches(1);
   SSC_CHECK_LAUNCH("conv_fwd_tf32");
@@ -1171,16 +1179,16 @@ extern "C" int ssc_conv_pack_filters(const float *filters, int K, int c_in, int 
   if (precision == SSC_PREC_TF32 && tf32_offsets_per_row(c_in) > 1) {
     const int opk = tf32_offsets_per_row(c_in), n_groups = ceil_div(K, opk);
     const long long total_g = (long long)n_groups * p.n_pad * 8;
-    { pack_filters_tf32_grouped_kernel<<<ceil_div(total_g, 256), 256, 0, as_stream(stream)>>>(filters, K, c_in, c_out, (c_in + 3) & ~3, opk,
+    { launch_ready(pack_filters_tf32_grouped_kernel, dim3(ceil_div(total_g, 256)), dim3(256), 0, as_stream(stream), filters, K, c_in, c_out, (c_in + 3) & ~3, opk,
                                                                                          n_groups, p.n_pad, (uint4 *)packed); note_launches(1); }
     SSC_CHECK_LAUNCH("pack_filters");
     return SSC_OK;
   }
   long long total = (long long)K * p.k_slabs * p.n_pad * 8;
   const int blocks = ceil_div(total, 256);
-  if (precision == SSC_PREC_F16) { pack_filters_16_kernel<false><<<blocks, 256, 0, as_stream(stream)>>>(filters, K, c_in, c_out, p, (uint4 *)packed); note_launches(1); }
-  else if (precision == SSC_PREC_BF16) { pack_filters_16_kernel<true><<<blocks, 256, 0, as_stream(stream)>>>(filters, K, c_in, c_out, p, (uint4 *)packed); note_launches(1); }
-  else { pack_filters_tf32_kernel<<<blocks, 256, 0, as_stream(stream)>>>(filters, K, c_in, c_out, p, (uint4 *)packed); note_launches(1); }
+  if (precision == SSC_PREC_F16) { launch_ready(pack_filters_16_kernel<false>, dim3(blocks), dim3(256), 0, as_stream(stream), filters, K, c_in, c_out, p, (uint4 *)packed); note_launches(1); }
+  else if (precision == SSC_PREC_BF16) { launch_ready(pack_filters_16_kernel<true>, dim3(blocks), dim3(256), 0, as_stream(stream), filters, K, c_in, c_out, p, (uint4 *)packed); note_launches(1); }
+  else { launch_ready(pack_filters_tf32_kernel, dim3(blocks), dim3(256), 0, as_stream(stream), filters, K, c_in, c_out, p, (uint4 *)packed); note_launches(1); }
   SSC_CHECK_LAUNCH("pack_filters");
   return SSC_OK;
 }

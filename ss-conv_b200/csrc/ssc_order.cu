@@ -24,6 +24,8 @@ constexpr int ORD_MAX_K = 343;   // 7^3: the scatter kernel keeps 32 x (K + 1) c
 __global__ void __launch_bounds__(ORD_BLOCK)
 row_key_hist_kernel(const int32_t *__restrict__ nbr, int K, int n_rows, uint16_t *__restrict__ keys,
                     uint32_t *__restrict__ hist, int n_blocks) {
+  after_previous();
+  next_may_start();
   extern __shared__ uint32_t hist_s[];  // [K + 1]
   const int B = K + 1;
   for (int b = threadIdx.x; b < B; b += ORD_BLOCK) hist_s[b] = 0u;
@@ -47,6 +49,8 @@ __global__ void __launch_bounds__(ORD_BLOCK)
 row_scatter_kernel(const uint16_t *__restrict__ keys, int B, int n_rows, const uint32_t *__restrict__ base, int n_blocks,
                    int32_t *__restrict__ order, const int32_t *__restrict__ nbr = nullptr, int K = 0,
                    int32_t *__restrict__ nbr_in_order = nullptr) {
+  after_previous();
+  next_may_start();
   extern __shared__ uint32_t cnt[];  // [warps of the block][B] rows of each group in each warp
   for (int i = threadIdx.x; i < (int)(blockDim.x >> 5) * B; i += blockDim.x) cnt[i] = 0u;
   __syncthreads();
@@ -82,6 +86,8 @@ constexpr int PLANE_MAX_BITS = 9;
 // bucket_of[key] = rank of the key by (offsets it allows, descending; key, ascending): one block, once per call
 __global__ void __launch_bounds__(PLANE_BLOCK)
 plane_bucket_table_kernel(int kx, int ky, int kz, uint16_t *__restrict__ bucket_of) {
+  after_previous();
+  next_may_start();
   __shared__ uint8_t weight_s[1 << PLANE_MAX_BITS];
   const int n_keys = 1 << (kx + ky + kz);
   for (int key = threadIdx.x; key < n_keys; key += PLANE_BLOCK)
@@ -102,6 +108,8 @@ __global__ void __launch_bounds__(PLANE_BLOCK)
 row_plane_key_hist_kernel(const int32_t *__restrict__ nbr, int kx, int ky, int kz, int n_rows,
                           const int32_t *__restrict__ n_rows_dev, const uint16_t *__restrict__ bucket_table,
                           uint16_t *__restrict__ keys, uint32_t *__restrict__ hist, int n_blocks) {
+  after_previous();
+  next_may_start();
   extern __shared__ uint32_t hist_s[];  // [B] counters, then [B - 1] bucket of every key
   const int bits = kx + ky + kz, B = (1 << bits) + 1;
   uint32_t *bucket_of = hist_s + B;
@@ -157,11 +165,11 @@ extern "C" int ssc_nbr_row_order(const int32_t *nbr, int K, int n_rows, int32_t 
   uint32_t *base = (uint32_t *)sp;
   sp += order_align(cells * 4);
   uint32_t *block_sums = (uint32_t *)sp;
-  { row_key_hist_kernel<<<n_blocks, ORD_BLOCK, (K + 1) * 4, st>>>(nbr, K, n_rows, keys, hist, n_blocks); note_launches(1); }
+  { launch_ready(row_key_hist_kernel, dim3(n_blocks), dim3(ORD_BLOCK), (K + 1) * 4, st, nbr, K, n_rows, keys, hist, n_blocks); note_launches(1); }
   SSC_CHECK_LAUNCH("row_key_hist");
   int rc = exclusive_scan_u32<false>(hist, (long long)cells, base, block_sums, nullptr, nullptr, st);
   if (rc != 0) return rc;
-  { row_scatter_kernel<<<n_blocks, ORD_BLOCK, 32 * (K + 1) * 4, st>>>(keys, K + 1, n_rows, base, n_blocks, order); note_launches(1); }
+  { launch_ready(row_scatter_kernel, dim3(n_blocks), dim3(ORD_BLOCK), 32 * (K + 1) * 4, st, keys, K + 1, n_rows, base, n_blocks, order, nullptr, 0, nullptr); note_launches(1); }
   SSC_CHECK_LAUNCH("row_scatter");
   return SSC_OK;
 }
@@ -197,12 +205,12 @@ extern "C" int ssc_nbr_row_order_planes(const int32_t *nbr, const int ksize[3], 
   uint32_t *block_sums = (uint32_t *)sp;
   sp += order_align((cells / 1024 + 2) * 4);
   uint16_t *bucket_table = (uint16_t *)sp;
-  { plane_bucket_table_kernel<<<1, PLANE_BLOCK, 0, st>>>(ksize[0], ksize[1], ksize[2], bucket_table); note_launches(1); }
-  { row_plane_key_hist_kernel<<<n_blocks, PLANE_BLOCK, (2 * B - 1) * 4, st>>>(nbr, ksize[0], ksize[1], ksize[2], n_rows, n_rows_dev, bucket_table, keys, hist, n_blocks); note_launches(1); }
+  { launch_ready(plane_bucket_table_kernel, dim3(1), dim3(PLANE_BLOCK), 0, st, ksize[0], ksize[1], ksize[2], bucket_table); note_launches(1); }
+  { launch_ready(row_plane_key_hist_kernel, dim3(n_blocks), dim3(PLANE_BLOCK), (2 * B - 1) * 4, st, nbr, ksize[0], ksize[1], ksize[2], n_rows, n_rows_dev, bucket_table, keys, hist, n_blocks); note_launches(1); }
   SSC_CHECK_LAUNCH("row_plane_key_hist");
   int rc = exclusive_scan_u32<false>(hist, (long long)cells, base, block_sums, nullptr, nullptr, st);
   if (rc != 0) return rc;
-  { row_scatter_kernel<<<n_blocks, PLANE_BLOCK, (PLANE_BLOCK / 32) * B * 4, st>>>(keys, B, n_rows, base, n_blocks, order, nbr,
+  { launch_ready(row_scatter_kernel, dim3(n_blocks), dim3(PLANE_BLOCK), (PLANE_BLOCK / 32) * B * 4, st, keys, B, n_rows, base, n_blocks, order, nbr,
                                                                                     ksize[0] * ksize[1] * ksize[2], nbr_in_order); note_launches(1); }
   SSC_CHECK_LAUNCH("row_scatter");
   return SSC_OK;

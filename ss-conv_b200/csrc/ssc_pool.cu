@@ -121,6 +121,8 @@ template <int IN>
 __global__ void __launch_bounds__(256)
 pool_divided_rows_kernel(const void *__restrict__ features, int c, const int32_t *__restrict__ nbr, int K, int n_out,
                          const int32_t *__restrict__ summaryrf, float *__restrict__ out, const int32_t *__restrict__ n_out_dev) {
+  after_previous();
+  next_may_start();
   const int lane = threadIdx.x & 31, row0 = (int)(blockIdx.x * 256 + (threadIdx.x & ~31u)), n_rows = live_rows(n_out, n_out_dev);
   const int count = lane < n_rows - row0 ? __ldg(summaryrf + row0 + lane) : 1;
   for (unsigned left = __ballot_sync(0xffffffffu, !whole_count(count)); left != 0u; left &= left - 1u) {
@@ -142,6 +144,8 @@ pool_divided_rows_kernel(const void *__restrict__ features, int c, const int32_t
 }
 
 __global__ void summary_rf_kernel(const int32_t *__restrict__ nbr, int K, int n_out, int32_t *__restrict__ rf) {
+  after_previous();
+  next_may_start();
   int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= n_out) return;
   int cnt = 0;
@@ -200,6 +204,8 @@ __global__ void global_pool_kernel(const float *__restrict__ feats, const int32_
 // row queued up at a single address: 38 us for 138 k rows).
 __global__ void batch_count_kernel(const int4 *__restrict__ indices, int n, int batch, int32_t *offsets,
                                    const int32_t *__restrict__ n_dev) {
+  after_previous();
+  next_may_start();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int b = -1;
   if (i < live_rows(n, n_dev)) b = __ldg((const int32_t *)(indices + i));
@@ -208,6 +214,8 @@ __global__ void batch_count_kernel(const int4 *__restrict__ indices, int n, int 
 }
 
 __global__ void batch_scan_kernel(int32_t *offsets, int batch) {
+  after_previous();
+  next_may_start();
   int lane = threadIdx.x;
   int running = 0;
   for (int base = 1; base <= batch; base += 32) {
@@ -228,6 +236,8 @@ constexpr int kOffsetsRows = 16384, kOffsetsBatch = 4096;
 __global__ void __launch_bounds__(1024)
 batch_offsets_small_kernel(const int4 *__restrict__ indices, int n, int batch, int32_t *__restrict__ offsets,
                            const int32_t *__restrict__ n_dev) {
+  after_previous();
+  next_may_start();
   __shared__ int hist[kOffsetsBatch];
   __shared__ uint32_t sums[33];
   for (int i = threadIdx.x; i < batch; i += 1024) hist[i] = 0;
@@ -275,7 +285,7 @@ static int launch_pool_as(const void *features, int c, const int32_t *nbr, int K
   }
   note_launches(1);
   if (MODE == 1 && rf != nullptr) {
-    pool_divided_rows_kernel<IN><<<ceil_div(n_out, 256), 256, 0, st>>>(features, c, nbr, K, n_out, rf, out, n_out_dev);
+    launch_ready(pool_divided_rows_kernel<IN>, dim3(ceil_div(n_out, 256)), dim3(256), 0, st, features, c, nbr, K, n_out, rf, out, n_out_dev);
     note_launches(1);
   }
   SSC_CHECK_LAUNCH(name);
@@ -317,7 +327,7 @@ extern "C" int ssc_summary_rf(const int32_t *nbr, int K, int n_out, int32_t *rf,
   SSC_REQUIRE(K > 0 && n_out >= 0, "summary_rf: bad sizes");
   if (n_out == 0) return SSC_OK;
   SSC_REQUIRE(nbr && rf, "summary_rf: null pointer");
-  { summary_rf_kernel<<<ceil_div(n_out, 256), 256, 0, as_stream(stream)>>>(nbr, K, n_out, rf); note_launches(1); }
+  { launch_ready(summary_rf_kernel, dim3(ceil_div(n_out, 256)), dim3(256), 0, as_stream(stream), nbr, K, n_out, rf); note_launches(1); }
   SSC_CHECK_LAUNCH("summary_rf");
   return SSC_OK;
 }
@@ -349,14 +359,14 @@ extern "C" int ssc_batch_offsets(const int32_t *indices, int n, int batch, int32
   SSC_REQUIRE(n >= 0 && batch >= 1 && offsets, "batch_offsets: bad arguments");
   cudaStream_t st = as_stream(stream);
   if (n <= kOffsetsRows && batch <= kOffsetsBatch) {
-    batch_offsets_small_kernel<<<1, 1024, 0, st>>>((const int4 *)indices, n, batch, offsets, n_dev);
+    launch_ready(batch_offsets_small_kernel, dim3(1), dim3(1024), 0, st, (const int4 *)indices, n, batch, offsets, n_dev);
     note_launches(1);
     SSC_CHECK_LAUNCH("batch_offsets");
     return SSC_OK;
   }
   cudaMemsetAsync(offsets, 0, (size_t)(batch + 1) * 4, st);
-  if (n > 0) { batch_count_kernel<<<ceil_div(n, 256), 256, 0, st>>>((const int4 *)indices, n, batch, offsets, n_dev); note_launches(1); }
-  { batch_scan_kernel<<<1, 32, 0, st>>>(offsets, batch); note_launches(1); }
+  if (n > 0) { launch_ready(batch_count_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, st, (const int4 *)indices, n, batch, offsets, n_dev); note_launches(1); }
+  { launch_ready(batch_scan_kernel, dim3(1), dim3(32), 0, st, offsets, batch); note_launches(1); }
   SSC_CHECK_LAUNCH("batch_offsets");
   return SSC_OK;
 }

@@ -97,6 +97,8 @@ __device__ __forceinline__ bool in_range3(int x, int y, int z, const int *shape)
 __global__ void hash_insert_kernel(const int4 *__restrict__ indices, int n, int batch,
                                    Geometry g, unsigned long long *table, uint32_t mask,
                                    int32_t *status, const int32_t *__restrict__ n_dev) {
+  after_previous();
+  next_may_start();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= live_rows(n, n_dev)) return;
   int4 c = indices[j];
@@ -264,6 +266,8 @@ mark_outputs_kernel(const int4 *__restrict__ indices, int n, int batch, Geometry
 // General fallback (stride and dilation both above one in some dimension): one thread per (input row, kernel offset).
 __global__ void mark_outputs_generic_kernel(const int4 *__restrict__ indices, int n, int batch, Geometry g,
                                             uint32_t *bitmap, const int32_t *__restrict__ n_dev) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)live_rows(n, n_dev) * g.K) return;
   int j = (int)(t / g.K);
@@ -509,6 +513,8 @@ lookup_neighbours_kernel(const int4 *__restrict__ out_indices, int n_out, int ba
                          const unsigned long long *__restrict__ table, uint32_t mask,
                          int32_t *__restrict__ nbr, int32_t *__restrict__ chunk_counts, int n_chunks,
                          const int32_t *__restrict__ n_out_dev) {
+  after_previous();
+  next_may_start();
   const unsigned full = 0xffffffffu;
   int kappa = blockIdx.y;
   int o = blockIdx.x * kChunk + threadIdx.x;
@@ -579,6 +585,8 @@ lookup_neighbours_kernel(const int4 *__restrict__ out_indices, int n_out, int ba
 
 // One block per kernel offset: exclusive scan of its chunk counts, total -> indice_num.
 __global__ void scan_chunks_kernel(int32_t *chunk_counts, int n_chunks, int32_t *indice_num) {
+  after_previous();
+  next_may_start();
   __shared__ uint32_t smem[33];
   int32_t *row = chunk_counts + (size_t)blockIdx.x * n_chunks;
   uint32_t running = 0;
@@ -598,6 +606,8 @@ __global__ void __launch_bounds__(kChunk)
 fill_pairs_kernel(const int32_t *__restrict__ nbr, int n_out, int n_in,
                   const int32_t *__restrict__ chunk_offsets, int n_chunks,
                   const int32_t *__restrict__ indice_num, int32_t *__restrict__ pairs) {
+  after_previous();
+  next_may_start();
   __shared__ uint32_t smem[33];
   int kappa = blockIdx.y;
   int o = blockIdx.x * kChunk + threadIdx.x;
@@ -622,6 +632,8 @@ fill_pairs_kernel(const int32_t *__restrict__ nbr, int n_out, int n_in,
 __global__ void pairs_to_nbr_kernel(const int32_t *__restrict__ pairs,
                                     const int32_t *__restrict__ indice_num, int n_cols, int n_out,
                                     int swap, int32_t *__restrict__ nbr) {
+  after_previous();
+  next_may_start();
   int kappa = blockIdx.y;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_cols || i >= indice_num[kappa]) return;
@@ -635,6 +647,8 @@ __global__ void pairs_to_nbr_kernel(const int32_t *__restrict__ pairs,
 // that already exist).
 __global__ void __launch_bounds__(kChunk)
 count_chunks_kernel(const int32_t *__restrict__ nbr, int n_out, int32_t *__restrict__ chunk_counts, int n_chunks) {
+  after_previous();
+  next_may_start();
   int kappa = blockIdx.y;
   int o = blockIdx.x * kChunk + threadIdx.x;
   int cnt = __syncthreads_count(o < n_out && nbr[(size_t)kappa * n_out + o] >= 0);
@@ -679,7 +693,7 @@ static int build_hash(const int32_t *indices, int n_in, int batch, const Geometr
   }
   cudaMemsetAsync(s.table, 0xFF, (size_t)s.n_buckets * kBucketSlots * 8, st);
   if (n_in > 0) {
-    { hash_insert_kernel<<<ceil_div(n_in, 256), 256, 0, st>>>((const int4 *)indices, n_in, batch, g, s.table,
+    { launch_ready(hash_insert_kernel, dim3(ceil_div(n_in, 256)), dim3(256), 0, st, (const int4 *)indices, n_in, batch, g, s.table,
                                                            s.n_buckets - 1, status ? status : s.misc + 1, n_in_dev); note_launches(1); }
   }
   SSC_CHECK_LAUNCH("hash_insert");
@@ -702,17 +716,17 @@ static int lookup_and_compact(const int32_t *out_indices, int n_out, int n_in, i
           (const int4 *)out_indices, n_out, batch, g, s.row_map, nbr, counts, n_chunks, n_out_dev); note_launches(1); }
   } else {
     dim3 grid(n_chunks, K);
-    { lookup_neighbours_kernel<<<grid, kChunk, 0, st>>>((const int4 *)out_indices, n_out, batch, g, s.table,
+    { launch_ready(lookup_neighbours_kernel, dim3(grid), dim3(kChunk), 0, st, (const int4 *)out_indices, n_out, batch, g, s.table,
                                                      s.n_buckets - 1, nbr, s.chunk_counts, n_chunks, n_out_dev); note_launches(1); }
   }
   SSC_CHECK_LAUNCH("lookup_neighbours");
   if (indice_num == nullptr) return 0;
-  { scan_chunks_kernel<<<K, 256, 0, st>>>(s.chunk_counts, n_chunks, indice_num); note_launches(1); }
+  { launch_ready(scan_chunks_kernel, dim3(K), dim3(256), 0, st, s.chunk_counts, n_chunks, indice_num); note_launches(1); }
   SSC_CHECK_LAUNCH("scan_chunks");
   if (pairs != nullptr && n_in > 0) {
     int n_chunks_in = ceil_div(n_in, kChunk);
     dim3 grid2(n_chunks > n_chunks_in ? n_chunks : n_chunks_in, K);
-    { fill_pairs_kernel<<<grid2, kChunk, 0, st>>>(nbr, n_out, n_in, s.chunk_counts, n_chunks, indice_num, pairs); note_launches(1); }
+    { launch_ready(fill_pairs_kernel, dim3(grid2), dim3(kChunk), 0, st, nbr, n_out, n_in, s.chunk_counts, n_chunks, indice_num, pairs); note_launches(1); }
     SSC_CHECK_LAUNCH("fill_pairs");
   }
   return 0;
@@ -884,7 +898,7 @@ static int mark_outputs(const char *who, const int32_t *indices, int n_in, int b
       { launch_ready(mark_outputs_kernel, dim3(ceil_div(n_in, 128)), dim3(128), 0, st, (const int4 *)indices, n_in, batch, g, s.bitmap, n_in_dev,
                                                                 together ? s.row_map : nullptr, status ? status : s.misc + 1); note_launches(1); }
     } else {
-      { mark_outputs_generic_kernel<<<ceil_div((long long)n_in * g.K, 256), 256, 0, st>>>((const int4 *)indices, n_in, batch, g, s.bitmap, n_in_dev); note_launches(1); }
+      { launch_ready(mark_outputs_generic_kernel, dim3(ceil_div((long long)n_in * g.K, 256)), dim3(256), 0, st, (const int4 *)indices, n_in, batch, g, s.bitmap, n_in_dev); note_launches(1); }
     }
     SSC_CHECK_LAUNCH("mark_outputs");
   }
@@ -983,7 +997,7 @@ extern "C" int ssc_pairs_to_nbr(const int32_t *pairs, const int32_t *indice_num,
   cudaMemsetAsync(nbr, 0xFF, (size_t)K * n_out * 4, st);
   if (n_cols > 0) {
     dim3 grid(ceil_div(n_cols, 256), K);
-    { pairs_to_nbr_kernel<<<grid, 256, 0, st>>>(pairs, indice_num, n_cols, n_out, swap, nbr); note_launches(1); }
+    { launch_ready(pairs_to_nbr_kernel, dim3(grid), dim3(256), 0, st, pairs, indice_num, n_cols, n_out, swap, nbr); note_launches(1); }
   }
   SSC_CHECK_LAUNCH("pairs_to_nbr");
   return SSC_OK;
@@ -1004,12 +1018,12 @@ extern "C" int ssc_pairs_from_nbr(const int32_t *nbr, int K, int n_out, int n_in
   int n_chunks = ceil_div(n_out > 0 ? n_out : 1, kChunk);
   int32_t *chunk_counts = (int32_t *)scratch;
   dim3 grid(n_chunks, K);
-  { count_chunks_kernel<<<grid, kChunk, 0, st>>>(nbr, n_out, chunk_counts, n_chunks); note_launches(1); }
-  { scan_chunks_kernel<<<K, 256, 0, st>>>(chunk_counts, n_chunks, indice_num); note_launches(1); }
+  { launch_ready(count_chunks_kernel, dim3(grid), dim3(kChunk), 0, st, nbr, n_out, chunk_counts, n_chunks); note_launches(1); }
+  { launch_ready(scan_chunks_kernel, dim3(K), dim3(256), 0, st, chunk_counts, n_chunks, indice_num); note_launches(1); }
   if (n_in > 0) {
     int n_chunks_in = ceil_div(n_in, kChunk);
     dim3 grid2(n_chunks > n_chunks_in ? n_chunks : n_chunks_in, K);
-    { fill_pairs_kernel<<<grid2, kChunk, 0, st>>>(nbr, n_out, n_in, chunk_counts, n_chunks, indice_num, pairs); note_launches(1); }
+    { launch_ready(fill_pairs_kernel, dim3(grid2), dim3(kChunk), 0, st, nbr, n_out, n_in, chunk_counts, n_chunks, indice_num, pairs); note_launches(1); }
   }
   SSC_CHECK_LAUNCH("pairs_from_nbr");
   return SSC_OK;

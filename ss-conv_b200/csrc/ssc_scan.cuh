@@ -49,6 +49,8 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s
 template <bool POPC>
 __global__ void popc_block_sums_kernel(const uint32_t *__restrict__ bitmap, long long n_words,
                                        uint32_t *block_sums) {
+  after_previous();
+  next_may_start();
   __shared__ uint32_t smem[33];
   long long base = (long long)blockIdx.x * 1024 + threadIdx.x * 4;
   uint32_t s = 0;
@@ -62,6 +64,8 @@ __global__ void popc_block_sums_kernel(const uint32_t *__restrict__ bitmap, long
 // Single block: in-place exclusive scan of block_sums[0..n); writes the total to
 // block_sums[n] and to the two int32 outputs.
 static __global__ void scan_block_sums_kernel(uint32_t *block_sums, int n, int32_t *total_a, int32_t *total_b) {
+  after_previous();
+  next_may_start();
   __shared__ uint32_t smem[33];
   uint32_t running = 0;
   for (int base = 0; base < n; base += blockDim.x) {
@@ -82,6 +86,8 @@ static __global__ void scan_block_sums_kernel(uint32_t *block_sums, int n, int32
 template <bool POPC>
 __global__ void word_prefix_kernel(const uint32_t *__restrict__ bitmap, long long n_words,
                                    const uint32_t *__restrict__ block_sums, uint32_t *word_prefix) {
+  after_previous();
+  next_may_start();
   __shared__ uint32_t smem[33];
   long long base = (long long)blockIdx.x * 1024 + threadIdx.x * 4;
   uint32_t c[4];
@@ -107,6 +113,8 @@ constexpr long long kSingleScanMax = 1 << 13;
 template <bool POPC>
 __global__ void __launch_bounds__(1024)
 single_block_scan_kernel(const uint32_t *values, int n, uint32_t *prefix, int32_t *total_a, int32_t *total_b) {
+  after_previous();
+  next_may_start();
   // values and prefix may be the same array (in-place scan): every value is read before its slot is written
   __shared__ uint32_t smem[33];
   const int per = (n + 1023) / 1024;          // values per thread (<= 8)
@@ -133,16 +141,16 @@ template <bool POPC>
 static inline int exclusive_scan_u32(const uint32_t *values, long long n, uint32_t *prefix, uint32_t *block_sums,
                                      int32_t *total_a, int32_t *total_b, cudaStream_t st) {
   if (n >= 1 && n <= kSingleScanMax) {
-    { single_block_scan_kernel<POPC><<<1, 1024, 0, st>>>(values, (int)n, prefix, total_a, total_b); note_launches(1); }
+    { launch_ready(single_block_scan_kernel<POPC>, dim3(1), dim3(1024), 0, st, values, (int)n, prefix, total_a, total_b); note_launches(1); }
     cudaError_t e1 = cudaGetLastError();
     if (e1 != cudaSuccess) return fail(SSC_ERR_CUDA, "exclusive_scan: %s", cudaGetErrorString(e1));
     return 0;
   }
   int blocks = (int)((n + 1023) / 1024);
   if (blocks < 1) blocks = 1;
-  { popc_block_sums_kernel<POPC><<<blocks, 256, 0, st>>>(values, n, block_sums); note_launches(1); }
-  { scan_block_sums_kernel<<<1, 1024, 0, st>>>(block_sums, blocks, total_a, total_b); note_launches(1); }
-  { word_prefix_kernel<POPC><<<blocks, 256, 0, st>>>(values, n, block_sums, prefix); note_launches(1); }
+  { launch_ready(popc_block_sums_kernel<POPC>, dim3(blocks), dim3(256), 0, st, values, n, block_sums); note_launches(1); }
+  { launch_ready(scan_block_sums_kernel, dim3(1), dim3(1024), 0, st, block_sums, blocks, total_a, total_b); note_launches(1); }
+  { launch_ready(word_prefix_kernel<POPC>, dim3(blocks), dim3(256), 0, st, values, n, block_sums, prefix); note_launches(1); }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "exclusive_scan: %s", cudaGetErrorString(e));
   return 0;

@@ -7,6 +7,8 @@ namespace ssc {
 // ------------------------------------------------------------ voxel2point_map / voxelize
 __global__ void v2p_map_kernel(const int32_t *__restrict__ inverse, const int32_t *__restrict__ ids, int32_t *maps,
                                int n_point, int n_voxel, int max_active, int mode) {
+  after_previous();
+  next_may_start();
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n_point) return;
   int v = inverse[p];
@@ -27,6 +29,8 @@ __global__ void v2p_map_kernel(const int32_t *__restrict__ inverse, const int32_
 
 // Modes 3/4: order every row's ids ascending so that later sums are reproducible.
 __global__ void v2p_sort_rows_kernel(int32_t *maps, int n_voxel, int max_active) {
+  after_previous();
+  next_may_start();
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n_voxel) return;
   int32_t *row = maps + (size_t)v * (max_active + 1);
@@ -44,6 +48,8 @@ __global__ void v2p_sort_rows_kernel(int32_t *maps, int n_voxel, int max_active)
 
 __global__ void voxelize_fwd_kernel(const float *__restrict__ feats, float *__restrict__ out,
                                     const int32_t *__restrict__ maps, int average, int n_voxel, int max_active, int c) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n_voxel * c) return;
   int v = (int)(t / c), ch = (int)(t - (long long)v * c);
@@ -112,6 +118,8 @@ __device__ __forceinline__ bool point_cell(const float *p, int b, int batch, con
 
 __global__ void p2v_mark_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, int n,
                                 int batch, VoxelGrid g, uint32_t *bitmap, int32_t *status) {
+  after_previous();
+  next_may_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float p[3] = {points[i * 3 + 0], points[i * 3 + 1], points[i * 3 + 2]};
@@ -139,6 +147,8 @@ __device__ __forceinline__ bool point_inside(const float *__restrict__ p, const 
 // stats[3] the last batch id.
 __global__ void p2v_stats_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, int n,
                                  VoxelGrid g, int32_t *stats) {
+  after_previous();
+  next_may_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool out = false, down = false, change = false;
   if (i < n) {
@@ -163,6 +173,8 @@ __global__ void p2v_stats_kernel(const float *__restrict__ points, const int32_t
 __global__ void __launch_bounds__(256)
 p2v_kept_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, int n, VoxelGrid g, int n_sample,
                 int32_t *__restrict__ kept) {
+  after_previous();
+  next_may_start();
   const int i = blockIdx.x * 256 + threadIdx.x;
   int b = -1;
   if (i < n && point_inside(points + (size_t)i * 3, g)) b = __ldg(batch_ids + i);
@@ -173,6 +185,8 @@ p2v_kept_kernel(const float *__restrict__ points, const int32_t *__restrict__ ba
 __global__ void __launch_bounds__(256)
 p2v_stays_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, int n, VoxelGrid g, int n_sample,
                  const int32_t *__restrict__ kept, uint32_t *__restrict__ bitmap, float *__restrict__ flag, int32_t *__restrict__ n_empty) {
+  after_previous();
+  next_may_start();
   const int i = blockIdx.x * 256 + threadIdx.x;
   bool stays = false, empty = false;
   if (i < n) {
@@ -191,6 +205,8 @@ __global__ void __launch_bounds__(256)
 p2v_gather_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, const float *__restrict__ feats, int n, int c,
                   VoxelGrid g, const uint32_t *__restrict__ bitmap, const uint32_t *__restrict__ prefix,
                   float *__restrict__ new_points, int32_t *__restrict__ new_ids, float *__restrict__ new_feats) {
+  after_previous();
+  next_may_start();
   const uint32_t groups = (uint32_t)(c / VEC);
   const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
   if (t >= (long long)n * groups) return;
@@ -219,6 +235,8 @@ __global__ void p2v_inverse_kernel(const float *__restrict__ points, const int32
                                    int batch, VoxelGrid g, const uint32_t *__restrict__ bitmap,
                                    const uint32_t *__restrict__ word_prefix, int mode, int32_t *inverse,
                                    uint32_t *count, uint32_t *select) {
+  after_previous();
+  next_may_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float p[3] = {points[i * 3 + 0], points[i * 3 + 1], points[i * 3 + 2]};
@@ -239,6 +257,8 @@ __global__ void p2v_inverse_kernel(const float *__restrict__ points, const int32
 // counted, so this pass needs no atomics (the lists are put into point order by the pass after it).
 __global__ void p2v_scatter_kernel(const int32_t *__restrict__ inverse, int n, const uint32_t *__restrict__ start,
                                    const uint32_t *__restrict__ rank, int32_t *order) {
+  after_previous();
+  next_may_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int v = inverse[i];
@@ -247,6 +267,8 @@ __global__ void p2v_scatter_kernel(const int32_t *__restrict__ inverse, int n, c
 }
 
 __global__ void p2v_sort_segments_kernel(const uint32_t *__restrict__ start, int n_voxel, int32_t *order) {
+  after_previous();
+  next_may_start();
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n_voxel) return;
   int a = (int)start[v], b = (int)start[v + 1];
@@ -262,6 +284,8 @@ __global__ void p2v_sort_segments_kernel(const uint32_t *__restrict__ start, int
 
 __global__ void p2v_reduce_kernel(const float *__restrict__ feats, int c, const uint32_t *__restrict__ start,
                                   const int32_t *__restrict__ order, int n_voxel, int average, float *__restrict__ out) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n_voxel * c) return;
   int v = (int)(t / c), ch = (int)(t - (long long)v * c);
@@ -280,6 +304,8 @@ template <int CMAX>
 __global__ void __launch_bounds__(256)
 p2v_reduce_small_kernel(const float *__restrict__ feats, int c, const uint32_t *__restrict__ start,
                         const int32_t *__restrict__ order, int n_voxel, int average, float *__restrict__ out) {
+  after_previous();
+  next_may_start();
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n_voxel) return;
   const int a = (int)start[v], b = (int)start[v + 1];
@@ -302,6 +328,8 @@ p2v_reduce_small_kernel(const float *__restrict__ feats, int c, const uint32_t *
 
 __global__ void p2v_select_kernel(const float *__restrict__ feats, int c, const uint32_t *__restrict__ select,
                                   int n_voxel, int n_point, float *__restrict__ out) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n_voxel * c) return;
   int v = (int)(t / c), ch = (int)(t - (long long)v * c);
@@ -330,6 +358,8 @@ constexpr int NN_SHARES = 1024;
 __global__ void __launch_bounds__(NN_TILE)
 nn_ranges_kernel(const float4 *__restrict__ known, int m, float2 *__restrict__ ranges, float4 *__restrict__ chunks, float4 *__restrict__ tiles,
                  int32_t *__restrict__ shares) {
+  after_previous();
+  next_may_start();
   __shared__ float4 chunk_s[32];
   __shared__ int in_s[32];
   const int lane = threadIdx.x & 31, c = threadIdx.x >> 5, k = blockIdx.x * NN_TILE + (int)threadIdx.x;
@@ -629,6 +659,8 @@ __global__ void __launch_bounds__(256)
 three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known, const float2 *__restrict__ ranges,
                 const float4 *__restrict__ chunks, const float4 *__restrict__ tiles, const int32_t *__restrict__ shares, float *__restrict__ dist2,
                 int32_t *__restrict__ idx) {
+  after_previous();
+  next_may_start();
   const int first = (int)blockIdx.x * 32, q0 = first + ((int)threadIdx.x >> 5) * NN_QUERIES;
   const float4 own = __ldg(unknown + min(q0, n - 1));
   NnSpan span = {0.f, 0, 0, NN_SHARES};
@@ -641,6 +673,8 @@ three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *
 __global__ void __launch_bounds__(256)
 three_nn_warps_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known, const float4 *__restrict__ chunks,
                       const float4 *__restrict__ tiles, const int32_t *__restrict__ shares, float *__restrict__ dist2, int32_t *__restrict__ idx) {
+  after_previous();
+  next_may_start();
   const int first = (int)blockIdx.x * 32, q0 = first + ((int)threadIdx.x >> 5) * NN_QUERIES;
   const float4 own = __ldg(unknown + min(q0, n - 1));
   const NnSpan span = nn_group<64>(first, m, unknown, tiles, shares);
@@ -649,6 +683,8 @@ three_nn_warps_kernel(int n, int m, const float4 *__restrict__ unknown, const fl
 __global__ void __launch_bounds__(256)
 three_nn_tiles_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known, const float2 *__restrict__ ranges,
                       const float4 *__restrict__ tiles, const int32_t *__restrict__ shares, float *__restrict__ dist2, int32_t *__restrict__ idx) {
+  after_previous();
+  next_may_start();
   const int first = (int)blockIdx.x * 64;
   if (tiles != nullptr && nn_group<64>(first, m, unknown, tiles, shares).share <= NN_MOST) return;
   nn_by_tiles<4>(first, n, m, unknown, known, ranges, dist2, idx);
@@ -658,6 +694,8 @@ three_nn_tiles_kernel(int n, int m, const float4 *__restrict__ unknown, const fl
 // element for element the torch expressions of Voxel2Point, a dozen launches of a few microseconds otherwise.
 __global__ void __launch_bounds__(256)
 voxel_centres_kernel(const int4 *__restrict__ indices, int n, float3 unit, float3 half_extent, float3 half_unit, float4 *__restrict__ out) {
+  after_previous();
+  next_may_start();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   const int4 v = __ldg(indices + i);
@@ -667,11 +705,15 @@ voxel_centres_kernel(const int4 *__restrict__ indices, int n, float3 unit, float
 }
 __global__ void __launch_bounds__(256)
 point_rows_kernel(const float *__restrict__ points, const int32_t *__restrict__ ids, int n, float4 *__restrict__ out) {
+  after_previous();
+  next_may_start();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i < n) out[i] = make_float4((float)__ldg(ids + i), __ldg(points + (size_t)i * 3), __ldg(points + (size_t)i * 3 + 1), __ldg(points + (size_t)i * 3 + 2));
 }
 __global__ void __launch_bounds__(256)
 nn_weights_kernel(const float *__restrict__ dist2, int n, float *__restrict__ weight) {
+  after_previous();
+  next_may_start();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   float r[3];
@@ -685,6 +727,8 @@ nn_weights_kernel(const float *__restrict__ dist2, int n, float *__restrict__ we
 __global__ void three_interpolate_kernel(int c, int n, const float *__restrict__ points,
                                          const int32_t *__restrict__ idx, const float *__restrict__ weight,
                                          float *__restrict__ out) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n * c) return;
   int p = (int)(t / c), ch = (int)(t - (long long)p * c);
@@ -702,6 +746,8 @@ __global__ void three_interpolate_kernel(int c, int n, const float *__restrict__
 __global__ void __launch_bounds__(256)
 three_interpolate_vec4_kernel(uint32_t groups, uint32_t total, const float4 *__restrict__ points,
                               const int32_t *__restrict__ idx, const float *__restrict__ weight, float4 *__restrict__ out) {
+  after_previous();
+  next_may_start();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= total) return;
   const uint32_t p = t / groups, g = t - p * groups;
@@ -729,8 +775,8 @@ extern "C" int ssc_voxel2point_map(const int32_t *inverse, const int32_t *ids, i
   if (n_point == 0 || n_voxel == 0) return SSC_OK;
   SSC_REQUIRE(inverse && ids && maps, "voxel2point_map: null pointer");
   cudaStream_t st = as_stream(stream);
-  { v2p_map_kernel<<<ceil_div(n_point, 256), 256, 0, st>>>(inverse, ids, maps, n_point, n_voxel, max_active, mode); note_launches(1); }
-  if (mode >= 3) { v2p_sort_rows_kernel<<<ceil_div(n_voxel, 128), 128, 0, st>>>(maps, n_voxel, max_active); note_launches(1); }
+  { launch_ready(v2p_map_kernel, dim3(ceil_div(n_point, 256)), dim3(256), 0, st, inverse, ids, maps, n_point, n_voxel, max_active, mode); note_launches(1); }
+  if (mode >= 3) { launch_ready(v2p_sort_rows_kernel, dim3(ceil_div(n_voxel, 128)), dim3(128), 0, st, maps, n_voxel, max_active); note_launches(1); }
   SSC_CHECK_LAUNCH("voxel2point_map");
   return SSC_OK;
 }
@@ -741,7 +787,7 @@ extern "C" int ssc_voxelize_fwd(const float *feats, float *out, const int32_t *m
   if (n_voxel == 0) return SSC_OK;
   SSC_REQUIRE(feats && out && maps, "voxelize_fwd: null pointer");
   long long threads = (long long)n_voxel * c;
-  { voxelize_fwd_kernel<<<ceil_div(threads, 256), 256, 0, as_stream(stream)>>>(feats, out, maps, mode == 4, n_voxel,
+  { launch_ready(voxelize_fwd_kernel, dim3(ceil_div(threads, 256)), dim3(256), 0, as_stream(stream), feats, out, maps, mode == 4, n_voxel,
                                                                             max_active, c); note_launches(1); }
   SSC_CHECK_LAUNCH("voxelize_fwd");
   return SSC_OK;
@@ -767,6 +813,8 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 steer_matrices_kernel(const T *__restrict__ rot, int orders, const double *__restrict__ dirs,
                       const double *__restrict__ pinv, int axes, int stride, float *__restrict__ dmats) {
+  after_previous();
+  next_may_start();
   extern __shared__ double ys[];                 // per order [S][2 l + 1], as pinv
   const int b = blockIdx.x;
   double R[3][3], Q[3][3];
@@ -839,6 +887,8 @@ __global__ void steer_kernel(const float *__restrict__ points, const float *__re
                              const float *__restrict__ scale, const float *__restrict__ dmats, int d_stride,
                              const int32_t *__restrict__ chan, int n, int c, int n_sample, float *__restrict__ new_points,
                              float *__restrict__ new_feats) {
+  after_previous();
+  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int width = c + 3;
   if (t >= (long long)n * width) return;
@@ -881,7 +931,7 @@ static int steer_matrices(const T *rot, int batch, int orders, const double *dir
     cudaError_t e = allow_smem((const void *)steer_matrices_kernel<T>, smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "steer_matrices: smem attribute: %s", cudaGetErrorString(e));
   }
-  { steer_matrices_kernel<T><<<batch, 128, smem, as_stream(stream)>>>(rot, orders, dirs, pinv, axes, stride, dmats); note_launches(1); }
+  { launch_ready(steer_matrices_kernel<T>, dim3(batch), dim3(128), smem, as_stream(stream), rot, orders, dirs, pinv, axes, stride, dmats); note_launches(1); }
   SSC_CHECK_LAUNCH("steer_matrices");
   return SSC_OK;
 }
@@ -904,7 +954,7 @@ extern "C" int ssc_steer_fwd(const float *points, const float *feats, const int3
   if (n == 0) return SSC_OK;
   SSC_REQUIRE(points && feats && ids && rot && trans && dmats && chan && new_points && new_feats, "steer_fwd: null pointer");
   long long total = (long long)n * (c + 3);
-  { steer_kernel<<<ceil_div(total, 256), 256, 0, as_stream(stream)>>>(points, feats, ids, rot, trans, scale, dmats, d_stride,
+  { launch_ready(steer_kernel, dim3(ceil_div(total, 256)), dim3(256), 0, as_stream(stream), points, feats, ids, rot, trans, scale, dmats, d_stride,
                                                                     chan, n, c, n_sample, new_points, new_feats); note_launches(1); }
   SSC_CHECK_LAUNCH("steer_fwd");
   return SSC_OK;
@@ -919,7 +969,7 @@ extern "C" int ssc_p2v_stats(const float *points, const int32_t *batch_ids, int 
   SSC_REQUIRE(points && batch_ids, "p2v_stats: null pointer");
   VoxelGrid g;
   fill_grid(g, grid, unit);
-  { p2v_stats_kernel<<<ceil_div(n_point, 256), 256, 0, st>>>(points, batch_ids, n_point, g, stats_dev); note_launches(1); }
+  { launch_ready(p2v_stats_kernel, dim3(ceil_div(n_point, 256)), dim3(256), 0, st, points, batch_ids, n_point, g, stats_dev); note_launches(1); }
   SSC_CHECK_LAUNCH("p2v_stats");
   return SSC_OK;
 }
@@ -945,14 +995,14 @@ extern "C" int ssc_p2v_keep(const float *points, const int32_t *batch_ids, const
   cudaMemsetAsync(kept, 0, (size_t)n_sample * 4, st);
   cudaMemsetAsync(counts_dev, 0, 8, st);
   const int blocks = ceil_div(n_point, 256);
-  p2v_kept_kernel<<<blocks, 256, 0, st>>>(points, batch_ids, n_point, g, n_sample, kept);
-  p2v_stays_kernel<<<blocks, 256, 0, st>>>(points, batch_ids, n_point, g, n_sample, kept, bitmap, flag, counts_dev + 1);
+  launch_ready(p2v_kept_kernel, dim3(blocks), dim3(256), 0, st, points, batch_ids, n_point, g, n_sample, kept);
+  launch_ready(p2v_stays_kernel, dim3(blocks), dim3(256), 0, st, points, batch_ids, n_point, g, n_sample, kept, bitmap, flag, counts_dev + 1);
   note_launches(2);
   if (int e = exclusive_scan_u32<true>(bitmap, (long long)words, prefix, sums, counts_dev, nullptr, st)) return e;
   if (c % 4 == 0 && (((uintptr_t)feats | (uintptr_t)new_feats) & 15u) == 0)
-    p2v_gather_kernel<4><<<ceil_div((long long)n_point * (c / 4), 256), 256, 0, st>>>(points, batch_ids, feats, n_point, c, g, bitmap, prefix, new_points, new_ids, new_feats);
+    launch_ready(p2v_gather_kernel<4>, dim3(ceil_div((long long)n_point * (c / 4), 256)), dim3(256), 0, st, points, batch_ids, feats, n_point, c, g, bitmap, prefix, new_points, new_ids, new_feats);
   else
-    p2v_gather_kernel<1><<<ceil_div((long long)n_point * c, 256), 256, 0, st>>>(points, batch_ids, feats, n_point, c, g, bitmap, prefix, new_points, new_ids, new_feats);
+    launch_ready(p2v_gather_kernel<1>, dim3(ceil_div((long long)n_point * c, 256)), dim3(256), 0, st, points, batch_ids, feats, n_point, c, g, bitmap, prefix, new_points, new_ids, new_feats);
   note_launches(1);
   SSC_CHECK_LAUNCH("p2v_keep");
   return SSC_OK;
@@ -962,7 +1012,7 @@ extern "C" int ssc_voxel_centres(const int32_t *indices, int n, const float unit
   SSC_REQUIRE(n >= 0 && unit && extent, "voxel_centres: bad arguments");
   if (n == 0) return SSC_OK;
   SSC_REQUIRE(indices && rows, "voxel_centres: null pointer");
-  voxel_centres_kernel<<<ceil_div(n, 256), 256, 0, as_stream(stream)>>>((const int4 *)indices, n, make_float3(unit[0], unit[1], unit[2]),
+  launch_ready(voxel_centres_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, as_stream(stream), (const int4 *)indices, n, make_float3(unit[0], unit[1], unit[2]),
                                                                         make_float3(0.5f * extent[0], 0.5f * extent[1], 0.5f * extent[2]),
                                                                         make_float3(0.5f * unit[0], 0.5f * unit[1], 0.5f * unit[2]), (float4 *)rows);
   note_launches(1);
@@ -974,7 +1024,7 @@ extern "C" int ssc_point_rows(const float *points, const int32_t *ids, int n, fl
   SSC_REQUIRE(n >= 0, "point_rows: bad size");
   if (n == 0) return SSC_OK;
   SSC_REQUIRE(points && ids && rows, "point_rows: null pointer");
-  point_rows_kernel<<<ceil_div(n, 256), 256, 0, as_stream(stream)>>>(points, ids, n, (float4 *)rows);
+  launch_ready(point_rows_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, as_stream(stream), points, ids, n, (float4 *)rows);
   note_launches(1);
   SSC_CHECK_LAUNCH("point_rows");
   return SSC_OK;
@@ -984,7 +1034,7 @@ extern "C" int ssc_nn_weights(const float *dist2, int n, float *weight, void *st
   SSC_REQUIRE(n >= 0, "nn_weights: bad size");
   if (n == 0) return SSC_OK;
   SSC_REQUIRE(dist2 && weight, "nn_weights: null pointer");
-  nn_weights_kernel<<<ceil_div(n, 256), 256, 0, as_stream(stream)>>>(dist2, n, weight);
+  launch_ready(nn_weights_kernel, dim3(ceil_div(n, 256)), dim3(256), 0, as_stream(stream), dist2, n, weight);
   note_launches(1);
   SSC_CHECK_LAUNCH("nn_weights");
   return SSC_OK;
@@ -1003,7 +1053,7 @@ extern "C" int ssc_p2v_count(const float *points, const int32_t *batch_ids, int 
   fill_grid(g, grid, unit);
   cudaMemsetAsync(s.bitmap, 0, (size_t)s.n_words * 4, st);
   cudaMemsetAsync(s.misc, 0, 256, st);
-  if (n_point > 0) { p2v_mark_kernel<<<ceil_div(n_point, 256), 256, 0, st>>>(points, batch_ids, n_point, batch, g, s.bitmap, status ? status : s.misc + 1); note_launches(1); }
+  if (n_point > 0) { launch_ready(p2v_mark_kernel, dim3(ceil_div(n_point, 256)), dim3(256), 0, st, points, batch_ids, n_point, batch, g, s.bitmap, status ? status : s.misc + 1); note_launches(1); }
   SSC_CHECK_LAUNCH("p2v_mark");
   if (int e = exclusive_scan_u32<true>(s.bitmap, s.n_words, s.word_prefix, s.block_sums, s.misc, n_voxel_dev, st)) return e;
   SSC_CHECK_LAUNCH("p2v_count");
@@ -1026,24 +1076,24 @@ extern "C" int ssc_p2v_fill(const float *points, const int32_t *batch_ids, const
   if (int e = bitmap_decode(s.bitmap, s.word_prefix, s.n_words, grid, n_voxel, voxel_indices, st)) return e;
   if (mode >= 3) cudaMemsetAsync(s.count, 0, ((size_t)n_voxel + 1) * 4, st);
   else cudaMemsetAsync(s.cursor, mode == 1 ? 0xFF : 0x00, (size_t)n_voxel * 4, st);
-  { p2v_inverse_kernel<<<ceil_div(n_point, 256), 256, 0, st>>>(points, batch_ids, n_point, batch, g, s.bitmap, s.word_prefix,
+  { launch_ready(p2v_inverse_kernel, dim3(ceil_div(n_point, 256)), dim3(256), 0, st, points, batch_ids, n_point, batch, g, s.bitmap, s.word_prefix,
                                                             mode, inverse, s.count, s.cursor); note_launches(1); }
   SSC_CHECK_LAUNCH("p2v_inverse");
   long long threads = (long long)n_voxel * c;
   if (mode >= 3) {
     // counts -> exclusive start offsets (in place), cursor = copy
     if (int e = exclusive_scan_u32<false>(s.count, (long long)n_voxel + 1, s.count, s.block_sums2, nullptr, nullptr, st)) return e;
-    { p2v_scatter_kernel<<<ceil_div(n_point, 256), 256, 0, st>>>(inverse, n_point, s.count, s.cursor, s.order); note_launches(1); }
-    { p2v_sort_segments_kernel<<<ceil_div(n_voxel, 128), 128, 0, st>>>(s.count, n_voxel, s.order); note_launches(1); }
+    { launch_ready(p2v_scatter_kernel, dim3(ceil_div(n_point, 256)), dim3(256), 0, st, inverse, n_point, s.count, s.cursor, s.order); note_launches(1); }
+    { launch_ready(p2v_sort_segments_kernel, dim3(ceil_div(n_voxel, 128)), dim3(128), 0, st, s.count, n_voxel, s.order); note_launches(1); }
     if (c <= 4) {
-      { p2v_reduce_small_kernel<4><<<ceil_div(n_voxel, 256), 256, 0, st>>>(feats, c, s.count, s.order, n_voxel, mode == 4, voxel_feats); note_launches(1); }
+      { launch_ready(p2v_reduce_small_kernel<4>, dim3(ceil_div(n_voxel, 256)), dim3(256), 0, st, feats, c, s.count, s.order, n_voxel, mode == 4, voxel_feats); note_launches(1); }
     } else if (c <= 8) {
-      { p2v_reduce_small_kernel<8><<<ceil_div(n_voxel, 256), 256, 0, st>>>(feats, c, s.count, s.order, n_voxel, mode == 4, voxel_feats); note_launches(1); }
+      { launch_ready(p2v_reduce_small_kernel<8>, dim3(ceil_div(n_voxel, 256)), dim3(256), 0, st, feats, c, s.count, s.order, n_voxel, mode == 4, voxel_feats); note_launches(1); }
     } else {
-      { p2v_reduce_kernel<<<ceil_div(threads, 256), 256, 0, st>>>(feats, c, s.count, s.order, n_voxel, mode == 4, voxel_feats); note_launches(1); }
+      { launch_ready(p2v_reduce_kernel, dim3(ceil_div(threads, 256)), dim3(256), 0, st, feats, c, s.count, s.order, n_voxel, mode == 4, voxel_feats); note_launches(1); }
     }
   } else {
-    { p2v_select_kernel<<<ceil_div(threads, 256), 256, 0, st>>>(feats, c, s.cursor, n_voxel, n_point, voxel_feats); note_launches(1); }
+    { launch_ready(p2v_select_kernel, dim3(ceil_div(threads, 256)), dim3(256), 0, st, feats, c, s.cursor, n_voxel, n_point, voxel_feats); note_launches(1); }
   }
   SSC_CHECK_LAUNCH("p2v_fill");
   return SSC_OK;
@@ -1074,15 +1124,15 @@ extern "C" int ssc_three_nn(int n, int m, const float *unknown, const float *kno
     ranges = (float2 *)(tiles + nn_tiles(m));
     shares = (int32_t *)(ranges + nn_tiles(m));
   }
-  { nn_ranges_kernel<<<(int)nn_tiles(m), NN_TILE, 0, st>>>((const float4 *)known, m, ranges, chunks, tiles, shares); note_launches(1); }
+  { launch_ready(nn_ranges_kernel, dim3((int)nn_tiles(m)), dim3(NN_TILE), 0, st, (const float4 *)known, m, ranges, chunks, tiles, shares); note_launches(1); }
   // 32 queries to a block fill the SMs up to 256 queries per SM; beyond, by tiles, a tile's way to shared memory and the merging pay
   // for 64 only (64 k queries in any order 131 us in one kernel, 123 in two; in grid order 77 and 79.  20 k: 309 and 357).
   if (n < sm_count() * 256) {
-    { three_nn_kernel<<<ceil_div(n, 32), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, ranges, chunks, tiles, shares, dist2, idx); note_launches(1); }
+    { launch_ready(three_nn_kernel, dim3(ceil_div(n, 32)), dim3(256), 0, st, n, m, (const float4 *)unknown, (const float4 *)known, ranges, chunks, tiles, shares, dist2, idx); note_launches(1); }
   } else {
-    { three_nn_tiles_kernel<<<ceil_div(n, 64), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, ranges, tiles, shares, dist2, idx); note_launches(1); }
+    { launch_ready(three_nn_tiles_kernel, dim3(ceil_div(n, 64)), dim3(256), 0, st, n, m, (const float4 *)unknown, (const float4 *)known, ranges, tiles, shares, dist2, idx); note_launches(1); }
     if (chunks != nullptr)
-      { three_nn_warps_kernel<<<ceil_div(n, 32), 256, 0, st>>>(n, m, (const float4 *)unknown, (const float4 *)known, chunks, tiles, shares, dist2, idx); note_launches(1); }
+      { launch_ready(three_nn_warps_kernel, dim3(ceil_div(n, 32)), dim3(256), 0, st, n, m, (const float4 *)unknown, (const float4 *)known, chunks, tiles, shares, dist2, idx); note_launches(1); }
   }
   SSC_CHECK_LAUNCH("three_nn");
   return SSC_OK;
@@ -1096,11 +1146,11 @@ extern "C" int ssc_three_interpolate_fwd(int c, int m, int n, const float *point
   long long threads = (long long)n * c;
   if ((c & 3) == 0 && threads / 4 < (1ll << 31) && (((uintptr_t)points | (uintptr_t)out) & 15u) == 0) {
     const uint32_t groups = (uint32_t)(c >> 2), total = (uint32_t)(threads >> 2);
-    { three_interpolate_vec4_kernel<<<ceil_div(total, 256), 256, 0, as_stream(stream)>>>(groups, total, (const float4 *)points, idx, weight, (float4 *)out); note_launches(1); }
+    { launch_ready(three_interpolate_vec4_kernel, dim3(ceil_div(total, 256)), dim3(256), 0, as_stream(stream), groups, total, (const float4 *)points, idx, weight, (float4 *)out); note_launches(1); }
     SSC_CHECK_LAUNCH("three_interpolate");
     return SSC_OK;
   }
-  { three_interpolate_kernel<<<ceil_div(threads, 256), 256, 0, as_stream(stream)>>>(c, n, points, idx, weight, out); note_launches(1); }
+  { launch_ready(three_interpolate_kernel, dim3(ceil_div(threads, 256)), dim3(256), 0, as_stream(stream), c, n, points, idx, weight, out); note_launches(1); }
   SSC_CHECK_LAUNCH("three_interpolate");
   return SSC_OK;
 }

@@ -400,6 +400,8 @@ __global__ void __launch_bounds__(128)
 conv_wgrad_small_kernel(const float *__restrict__ features, int c_in, const float *__restrict__ out_grad, int c_out,
                         const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in,
                         const int32_t *__restrict__ starts, int K, float *__restrict__ partial) {
+  after_previous();
+  next_may_start();
   __shared__ int first[257];
   chunk_prefix(starts, K, first);
   const int lane = threadIdx.x & 31, co = blockIdx.y * 32 + lane;
@@ -524,11 +526,11 @@ PairLists pair_lists_view(void *lists, int K, int n_out) {
 // bitmap of the table, popcount scan, scatter: three small launches
 int pair_lists_build(const int32_t *nbr, int K, int n_out, void *lists, PairLists *out, cudaStream_t st) {
   const ListPlan p = plan_lists(lists, K, n_out);
-  { launch_ready(pair_bitmap_kernel, dim3(dim3(ceil_div(p.wpr, 32), K)), dim3(256), 0, st, nbr, n_out, p.wpr, p.bitmap); note_launches(1); }
+  { launch_ready(pair_bitmap_kernel, dim3(ceil_div(p.wpr, 32), K), dim3(256), 0, st, nbr, n_out, p.wpr, p.bitmap); note_launches(1); }
   SSC_CHECK_LAUNCH("pair_bitmap");
   int rc = exclusive_scan_u32<true>(p.bitmap, p.words, p.prefix, p.block_sums, p.starts + K, nullptr, st);
   if (rc != 0) return rc;
-  { launch_ready(pair_scatter_kernel, dim3(dim3(ceil_div(p.wpr, 256), K)), dim3(256), 0, st, nbr, n_out, p.wpr, p.bitmap, p.prefix, p.pair_out, p.pair_in, p.starts); note_launches(1); }
+  { launch_ready(pair_scatter_kernel, dim3(ceil_div(p.wpr, 256), K), dim3(256), 0, st, nbr, n_out, p.wpr, p.bitmap, p.prefix, p.pair_out, p.pair_in, p.starts); note_launches(1); }
   SSC_CHECK_LAUNCH("pair_scatter");
   if (out) *out = PairLists{p.pair_out, p.pair_in, p.starts};
   return SSC_OK;
@@ -604,13 +606,13 @@ int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_wgrad(tf32): smem attribute: %s", cudaGetErrorString(e));
     const WtParams w = {features, out_grad, c_in, c_out, (staged & 1) ? (c_in + 3) & ~3 : c_in, (staged & 2) ? (c_out + 3) & ~3 : c_out,
                         (staged & 1) ? 0 : 1, (staged & 2) ? 0 : 1, p.n_pad, p.a_bytes, p.stage_bytes, p.stages, p.n_buf, p.in_rows ? 1 : 0, p.buf_cols, alarm_word()};
-    { launch_ready(conv_wgrad_tc_kernel, dim3(dim3(p.shares, p.co_blocks)), dim3((2 * p.stages + 5) * 32), p.smem, st, w, pl.pair_out, pl.pair_in, pl.starts, K, partial, status); note_launches(1); }
+    { launch_ready(conv_wgrad_tc_kernel, dim3(p.shares, p.co_blocks), dim3((2 * p.stages + 5) * 32), p.smem, st, w, pl.pair_out, pl.pair_in, pl.starts, K, partial, status); note_launches(1); }
     SSC_CHECK_LAUNCH("conv_wgrad_tc");
   } else if (p.small) {
     const dim3 grid(p.shares / 4, p.co_blocks);
-    if (c_in <= 4) { conv_wgrad_small_kernel<4><<<grid, 128, 0, st>>>(features, c_in, out_grad, c_out, pl.pair_out, pl.pair_in, pl.starts, K, partial); note_launches(1); }
-    else if (c_in <= 8) { conv_wgrad_small_kernel<8><<<grid, 128, 0, st>>>(features, c_in, out_grad, c_out, pl.pair_out, pl.pair_in, pl.starts, K, partial); note_launches(1); }
-    else { conv_wgrad_small_kernel<16><<<grid, 128, 0, st>>>(features, c_in, out_grad, c_out, pl.pair_out, pl.pair_in, pl.starts, K, partial); note_launches(1); }
+    if (c_in <= 4) { launch_ready(conv_wgrad_small_kernel<4>, dim3(grid), dim3(128), 0, st, features, c_in, out_grad, c_out, pl.pair_out, pl.pair_in, pl.starts, K, partial); note_launches(1); }
+    else if (c_in <= 8) { launch_ready(conv_wgrad_small_kernel<8>, dim3(grid), dim3(128), 0, st, features, c_in, out_grad, c_out, pl.pair_out, pl.pair_in, pl.starts, K, partial); note_launches(1); }
+    else { launch_ready(conv_wgrad_small_kernel<16>, dim3(grid), dim3(128), 0, st, features, c_in, out_grad, c_out, pl.pair_out, pl.pair_in, pl.starts, K, partial); note_launches(1); }
     SSC_CHECK_LAUNCH("conv_wgrad_small");
   } else {
     return -1;
