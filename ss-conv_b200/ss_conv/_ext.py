@@ -897,7 +897,9 @@ TABLE_REVERSED = 0x1000
 WGRAD_X_STAGED = 0x400
 WGRAD_DY_STAGED = 0x800
 # Input rows are read once per neighbour by the filter gradient: from here on they are rounded once, up front, instead of after every read (93 k
-# rows of 64 -> 76: 89 us, 64 + 5 rounded before; 162 k of 32 -> 38: 74, 64 + 4; 65 k of 16 -> 38: 12, 11 + 3).
+# rows of 64 -> 76: 89 us, 64 + 5 rounded before; 162 k of 32 -> 38: 74, 64 + 4; 65 k of 16 -> 38: 12, 11 + 3.  Not where there are
+# more input rows than output rows: a stride of two reads a row three or four times instead of ten (both gradients of 240 k ->
+# 129 k rows, 64 -> 76, in a graph: 177 us rounded before, 172 after every read).
 WGRAD_STAGE_ELEMENTS = 1 << 21
 # (features.data_ptr(), filters.data_ptr()) -> (prec, packed, scratch, nbytes) left by conv_prepare for the
 # conv_forward call that follows on the same tensors
@@ -1234,7 +1236,7 @@ def conv_wgrad(features, out_grad, nbr, precision=None, dy_image=None):
     x, dy = _p(features, torch.float32), _p(out_grad, torch.float32)
     if mode == PREC_TF32 and c_in <= 256 and K <= 256 and dy_image is not None:
         dy, mode = _p(dy_image), mode | WGRAD_DY_STAGED
-        if features.numel() >= WGRAD_STAGE_ELEMENTS:
+        if features.numel() >= WGRAD_STAGE_ELEMENTS and features.shape[0] <= n_out:
             x_image = stage_tf32(features)
             x, mode = _p(x_image), mode | WGRAD_X_STAGED
     _check(lib().ssc_conv_wgrad_lists(x, c_in, dy, c_out, _p(nbr, torch.int32), K, n_out, _p(lists),
