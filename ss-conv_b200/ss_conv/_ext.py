@@ -897,7 +897,7 @@ TABLE_REVERSED = 0x1000
 WGRAD_X_STAGED = 0x400
 WGRAD_DY_STAGED = 0x800
 # Input rows are read once per neighbour by the filter gradient: from here on they are rounded once, up front, instead of after every read (93 k
-# rows of 64 -> 76: 89 us, 64 + 5 rounded before; 162 k of 32 -> 38: 74, 64 + 4; 65 k of 16 -> 38: 12, 11 + 3.  Not where there are
+# rows of 64 -> 76: 89 us, 64 + 5 rounded before; 162 k of 32 -> 38: 74, 64 + 4; 65 k of 16 -> 38: 12, 11 + 3).  Not where there are
 # more input rows than output rows: a stride of two reads a row three or four times instead of ten (both gradients of 240 k ->
 # 129 k rows, 64 -> 76, in a graph: 177 us rounded before, 172 after every read).
 WGRAD_STAGE_ELEMENTS = 1 << 21
