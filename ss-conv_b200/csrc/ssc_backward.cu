@@ -20,7 +20,6 @@ namespace ssc {
 
 __global__ void nbr_transpose_kernel(const int32_t *__restrict__ nbr, int n_out, int n_in, int32_t *__restrict__ nbr_in) {
   after_previous();
-  next_may_start();
   int o = blockIdx.x * blockDim.x + threadIdx.x;
   int kappa = blockIdx.y;
   if (o >= n_out) return;
@@ -37,7 +36,6 @@ conv_wgrad_partial_kernel(const float *__restrict__ features, int c_in, const fl
                           const int32_t *__restrict__ nbr, int n_out, int rows_per_split, int tiles_co,
                           float *__restrict__ partial) {
   after_previous();
-  next_may_start();
   __shared__ float As[WG_ROWS][WG_T + 4];
   __shared__ float Bs[WG_ROWS][WG_T + 4];
   __shared__ int rows[WG_ROWS];
@@ -94,7 +92,6 @@ conv_wgrad_partial_kernel(const float *__restrict__ features, int c_in, const fl
 
 __global__ void wgrad_reduce_kernel(const float *__restrict__ partial, int splits, long long elems, float *__restrict__ out) {
   after_previous();
-  next_may_start();
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= elems) return;
   float s = 0.f;
@@ -112,7 +109,6 @@ pool_bwd_kernel(const float *__restrict__ features, const float *__restrict__ ou
                 const float *__restrict__ out_grad, int c, const int32_t *__restrict__ nbr_in, int K,
                 int n_in, const int32_t *__restrict__ summaryrf, float *__restrict__ d_in, int R) {
   after_previous();
-  next_may_start();
   extern __shared__ int32_t pool_smem[];
   struct Item {
     Channels g, y;
@@ -154,7 +150,6 @@ pool_bwd_kernel(const float *__restrict__ features, const float *__restrict__ ou
 __global__ void global_avgpool_bwd_kernel(const float *__restrict__ d_out, const int32_t *__restrict__ offsets, int c,
                                           float *__restrict__ d_feats) {
   after_previous();
-  next_may_start();
   const int s = blockIdx.x, ch = blockIdx.y * 32 + threadIdx.x;
   const int start = offsets[s], end = offsets[s + 1];
   if (ch >= c || end <= start) return;
@@ -165,7 +160,6 @@ __global__ void global_avgpool_bwd_kernel(const float *__restrict__ d_out, const
 __global__ void global_maxpool_bwd_kernel(const float *__restrict__ d_out, const int32_t *__restrict__ maxidx, long long total,
                                           int c, long long n_rows, float *__restrict__ d_feats) {
   after_previous();
-  next_may_start();
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= total) return;
   const int row = maxidx[e];
@@ -177,7 +171,6 @@ __global__ void global_maxpool_bwd_kernel(const float *__restrict__ d_out, const
 __global__ void voxelize_bwd_kernel(const float *__restrict__ d_out, const int32_t *__restrict__ rules, int n_voxel,
                                     int max_active, int c, int average, float *__restrict__ d_feats) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n_voxel * c) return;
   const int v = (int)(t / c), ch = (int)(t - (long long)v * c);
@@ -193,7 +186,6 @@ __global__ void three_interpolate_bwd_kernel(int c, int n, const float *__restri
                                              const int32_t *__restrict__ idx, const float *__restrict__ weight,
                                              float *__restrict__ grad_points) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n * c) return;
   const int p = (int)(t / c), ch = (int)(t - (long long)p * c);

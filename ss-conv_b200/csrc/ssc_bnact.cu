@@ -10,7 +10,6 @@ __global__ void bn_fold_kernel(const float *running_mean, const float *running_v
                                const float *bias, const int32_t *field_of_channel, const int32_t *scalar_of_channel,
                                int c, float eps, float *scale, float *shift) {
   after_previous();
-  next_may_start();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
   int f = field_of_channel[ch], s = scalar_of_channel[ch];
@@ -32,7 +31,6 @@ __global__ void bn_gate_kernel(const float *__restrict__ x, long long total, int
                                int scalar_act, int gate_act, const float *__restrict__ scalar_bias,
                                const float *__restrict__ gate_bias, float *__restrict__ out) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= total) return;
   long long row = t / c_out;
@@ -64,7 +62,6 @@ bn_gate_vec4_kernel(const float *__restrict__ x, uint32_t total, uint32_t groups
                     const int32_t *__restrict__ gate_of_channel, int c_gate_base, int scalar_act, int gate_act,
                     const float *__restrict__ scalar_bias, const float *__restrict__ gate_bias, float *__restrict__ out) {
   after_previous();
-  next_may_start();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= total) return;
   const uint32_t row = t / groups, g4 = t - row * groups;
@@ -116,7 +113,6 @@ bn_gate_vec4_out16_kernel(const float *__restrict__ x, uint32_t total, uint32_t 
                     const int32_t *__restrict__ gate_of_channel, int c_gate_base, int scalar_act, int gate_act,
                     const float *__restrict__ scalar_bias, const float *__restrict__ gate_bias, uint2 *__restrict__ out) {
   after_previous();
-  next_may_start();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= total) return;
   const uint32_t row = t / groups, g4 = t - row * groups;
@@ -172,7 +168,6 @@ bn_gate_rows_kernel(const float *__restrict__ x, uint32_t n_rows, uint32_t group
                     int gate_act, const float *__restrict__ scalar_bias, const float *__restrict__ gate_bias,
                     void *__restrict__ out) {
   after_previous();
-  next_may_start();
   extern __shared__ float gate_s[];                    // [R][n_gates]
   // block = (groups, R): threadIdx.x is the group of VEC channels, threadIdx.y the row of the block
   // (no integer division anywhere in the kernel).  VEC = 4 / 2 / 1 for channel counts that are
@@ -282,7 +277,6 @@ __global__ void __launch_bounds__(256)
 bn_colsum_kernel(const float *__restrict__ x, int n, int c, int chains, int lanes, const float *__restrict__ chan_mean,
                  float *__restrict__ part) {
   after_previous();
-  next_may_start();
   const int groups = c / VEC;
   const int lane = threadIdx.x / (blockDim.x / lanes), chain = blockIdx.x * lanes + lane;
   if (lane >= lanes || chain >= chains) return;
@@ -371,7 +365,6 @@ __global__ void __launch_bounds__(kFinishThreads)
 bn_finish_mean_kernel(const float *__restrict__ part, int row_blocks, int n, int c, const int32_t *__restrict__ scalar_of_channel,
                       float momentum, float keep, float *running_mean, float *mean, float *chan_mean) {
   after_previous();
-  next_may_start();
   const int ch = blockIdx.x, s = scalar_of_channel[ch];
   if (s < 0) {
     if (threadIdx.x == 0) chan_mean[ch] = 0.f;
@@ -403,7 +396,6 @@ bn_finish_var_kernel(const float *__restrict__ part, int row_blocks, int n, int 
                      const float *__restrict__ weight, const float *__restrict__ bias, float eps, float momentum, float keep,
                      float *running_var, float *var, float *scale, float *shift) {
   after_previous();
-  next_may_start();
   const int f = blockIdx.x;
   const int2 fc = field_channels(field_of_channel, c, f);
   const float v = chain_total(part, row_blocks, c, fc.x, fc.y) / (float)n;
@@ -476,7 +468,6 @@ __global__ void __launch_bounds__(256)
 bn_gate_bwd_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
                    float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
   after_previous();
-  next_may_start();
   extern __shared__ __align__(16) float sm[];
   const int R = p.rows, c = p.c, c_out = p.c_out, n_gates = p.n_gates;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -648,7 +639,6 @@ __global__ void __launch_bounds__(256, QL == 1 ? 4 : 2)
 bn_gate_bwd_lanes_kernel(BnGateBwd p, int L, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
                          float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
   after_previous();
-  next_may_start();
   extern __shared__ __align__(16) float sm[];
   constexpr int GL = QL;                       // gate scalars of a lane
   const int c = p.c, c_out = p.c_out, n_gates = p.n_gates, n = p.n;
@@ -847,7 +837,6 @@ __global__ void __launch_bounds__(256)
 bn_gate_bwd_wide_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
                         float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
   after_previous();
-  next_may_start();
   const int ch = (int)(blockIdx.y * 256 + threadIdx.x);
   if (ch >= p.c) return;
   auto normed = [&](const float *xr, int k) { return p.scale ? fmaf(__ldg(xr + k), __ldg(p.scale + k), __ldg(p.shift + k)) : __ldg(xr + k); };
@@ -895,7 +884,6 @@ bn_bwd_finish_kernel(const float *__restrict__ part_a, const float *__restrict__
                      float *__restrict__ ks, float *__restrict__ ka, float *__restrict__ kg, float *__restrict__ d_weight,
                      float *__restrict__ d_bias) {
   after_previous();
-  next_may_start();
   const int f = blockIdx.x;
   const int2 fc = field_channels(field_of_channel, c, f);
   const float A = chain_total(part_a, row_blocks, c, fc.x, fc.y);
@@ -917,7 +905,6 @@ bn_bwd_finish_kernel(const float *__restrict__ part_a, const float *__restrict__
 // chan_mean[ch] = mean of a scalar channel (0 for l>0 channels).
 __global__ void bn_chan_mean_kernel(const float *mean, const int32_t *scalar_of_channel, int c, float *chan_mean) {
   after_previous();
-  next_may_start();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c) return;
   const int s = scalar_of_channel[i];

@@ -12,7 +12,6 @@ __global__ void materialize_kernel(const float *__restrict__ weight, const float
                                    const int32_t *__restrict__ out_field, const int32_t *__restrict__ in_field,
                                    int c_out, int c_in, int K, float *__restrict__ filters) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long total = (long long)K * c_in * c_out;
   if (t >= total) return;
@@ -47,7 +46,6 @@ materialize_bwd_kernel(const float *__restrict__ g, const float *__restrict__ ba
                        const int32_t *__restrict__ out_start, const int32_t *__restrict__ in_start, int c_out, int c_in, int K,
                        int staged, float *__restrict__ d_weight) {
   after_previous();
-  next_may_start();
   extern __shared__ float gs[];
   const int co0 = out_start[blockIdx.y], ci0 = in_start[blockIdx.x];
   const int i = out_field[co0 * 3], u = out_field[co0 * 3 + 1], j = in_field[ci0 * 3], v = in_field[ci0 * 3 + 1];
@@ -93,7 +91,6 @@ conv_fwd_fp32_kernel(const float *__restrict__ features, int c_in, const float *
                      int c_out, const int32_t *__restrict__ nbr, int n_out, int rev, float *__restrict__ out,
                      const int32_t *__restrict__ n_out_dev) {
   after_previous();
-  next_may_start();
   __shared__ float As[BK][BM + 4];
   __shared__ float Bs[BK][BN + 4];
   __shared__ int rows[BM];
@@ -184,7 +181,6 @@ conv_fwd_fp32_lanes_kernel(const float *__restrict__ features, int c_in, const f
                            int c_out, const int32_t *__restrict__ nbr, int n_out, int rev, float *__restrict__ out,
                            const int32_t *__restrict__ n_out_dev) {
   after_previous();
-  next_may_start();
   extern __shared__ __align__(16) float ws[];   // [K][c_in][CB]
   const int n_rows = live_rows(n_out, n_out_dev);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.y * CB;
@@ -309,7 +305,6 @@ conv_fwd_fp32_warps_kernel(const float *__restrict__ features, int c_in, const f
                            int c_out, const int32_t *__restrict__ nbr, int n_out, int rev, float *__restrict__ out,
                            const int32_t *__restrict__ n_out_dev) {
   after_previous();
-  next_may_start();
   extern __shared__ float ws[];               // [K][c_in][NJ * 32]
   const int n_rows = live_rows(n_out, n_out_dev);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.y * NJ * 32;

@@ -211,7 +211,6 @@ pl_prepare_kernel(const int32_t *__restrict__ starts, int K, int n_split, int ti
                   int32_t *__restrict__ owner, const float4 *__restrict__ rows, long long n_stage, int bf16, uint4 *__restrict__ staged,
                   float4 *__restrict__ out, long long n_clear) {
   after_previous();
-  next_may_start();
   if (blockIdx.x == 0) {
     deal_strips(starts, K, n_split, tile, n_ctas, hdr, strips, owner);
     return;
@@ -544,13 +543,11 @@ conv_fwd_pairs_body(const float *__restrict__ staged, const uint4 *__restrict__ 
 template <bool F16>
 __global__ void __launch_bounds__((PL_PRODUCERS + 1 + PL_EPI_WARPS) * 32, 1) conv_fwd_pairs_kernel(PL_ARGS) {
   after_previous();
-  next_may_start();
   conv_fwd_pairs_body<F16, false>(staged, packed, c_out, pair_out, pair_in, starts, strips, owner, n_strips, out, status, p);
 }
 template <bool F16>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((PL_PRODUCERS + 1 + PL_EPI_WARPS) * 32, 1) conv_fwd_pairs_by_two_kernel(PL_ARGS) {
   after_previous();
-  next_may_start();
   conv_fwd_pairs_body<F16, true>(staged, packed, c_out, pair_out, pair_in, starts, strips, owner, n_strips, out, status, p);
 }
 #undef PL_ARGS

@@ -36,14 +36,12 @@ stage_features_kernel(const float4 *__restrict__ in, long long total_vec, uint4 
 #pragma unroll
   for (int q = 0; q < STAGE_VECS; ++q)
     if (first + q * 256 < total_vec) out[first + q * 256] = stage_piece(v[q]);
-  next_may_start();
 }
 
 // Channel counts that are not a multiple of four: rows padded with zeros to c_pad floats.
 __global__ void stage_features_padded_kernel(const float *__restrict__ in, long long n_rows, int c_in, int c_pad,
                                              long long total, uint32_t *__restrict__ out) {
   after_previous();
-  next_may_start();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long step = (long long)gridDim.x * blockDim.x;
   for (; i < total; i += step) {
@@ -59,7 +57,6 @@ __global__ void stage_features_padded_kernel(const float *__restrict__ in, long 
 __global__ void __launch_bounds__(256)
 stage_features_padded_rows_kernel(const float *__restrict__ in, int n_rows, int c_in, uint4 *__restrict__ out) {
   after_previous();
-  next_may_start();
   const int row = blockIdx.x * blockDim.y + threadIdx.y, c0 = threadIdx.x * 4;
   if (row >= n_rows) return;
   const float *src = in + (size_t)row * c_in + c0;
@@ -98,7 +95,6 @@ template <bool BF16>
 __global__ void stage_features_16_kernel(const float *__restrict__ in, long long n_rows, int c_in, int c_pad,
                                          long long total_pairs, uint32_t *__restrict__ out) {
   after_previous();
-  next_may_start();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long step = (long long)gridDim.x * blockDim.x;
   const int pairs = c_pad >> 1;
@@ -131,7 +127,6 @@ stage_features_16_vec_kernel(const float4 *__restrict__ in, long long total, uin
 #pragma unroll
   for (int q = 0; q < STAGE_VECS; ++q)
     if (first + q * 256 < total) out[first + q * 256] = stage_piece_16(a[q], b[q], BF16);
-  next_may_start();
 }
 
 size_t conv_f16_scratch_bytes(int n_in, int c_in) { return (size_t)n_in * (size_t)f16_row_words(c_in) * 4 + 16; }

@@ -122,7 +122,6 @@ bool tc_operand_layout(int c_in, int c_out, int *k_slabs, int *n_pad, int *tile_
 __global__ void pack_filters_tf32_kernel(const float *__restrict__ filters, int K, int c_in, int c_out, TcParams p,
                                          uint4 *__restrict__ packed) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long total = (long long)K * p.k_slabs * p.n_pad * 8;
   if (t >= total) return;
@@ -149,7 +148,6 @@ __global__ void pack_filters_tf32_kernel(const float *__restrict__ filters, int 
 __global__ void pack_filters_tf32_grouped_kernel(const float *__restrict__ filters, int K, int c_in, int c_out, int c_pad,
                                                  int opk, int n_groups, int n_pad, uint4 *__restrict__ packed) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long total = (long long)n_groups * n_pad * 8;
   if (t >= total) return;
@@ -179,7 +177,6 @@ conv_fwd_tf32_kernel(const float *__restrict__ features, int c_in, const uint4 *
                      int32_t *status, TcParams p, const int32_t *__restrict__ n_out_dev,
                      const int32_t *__restrict__ order) {
   after_previous();
-  next_may_start();
   // `order` (may be NULL): the rows of tile t are order[128 t .. 128 t + 127] instead of the same
   // consecutive numbers; rows that use the same kernel offsets, put next to each other, make a
   // tile skip the offsets none of them uses.
@@ -951,7 +948,6 @@ conv_fwd_rows(const float *__restrict__ features, int row_words, const uint4 *__
       store_plain(load16, blk, out, m, col0, p.n_cta, c_row, vec, lane, 32 * group, 32 * groups);
     }
   }
-  next_may_start();
   // a wait gave up: what was issued still arrives on done_bar (committed on every path) and filter copies land
   // within microseconds; both before the accumulators and the shared memory are handed back
   if (*abort_flag) {
@@ -995,7 +991,6 @@ template <bool BF16>
 __global__ void pack_filters_16_kernel(const float *__restrict__ filters, int K, int c_in, int c_out, TcParams p,
                                         uint4 *__restrict__ packed) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long total = (long long)K * p.k_slabs * p.n_pad * 8;
   if (t >= total) return;

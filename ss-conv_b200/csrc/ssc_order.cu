@@ -25,7 +25,6 @@ __global__ void __launch_bounds__(ORD_BLOCK)
 row_key_hist_kernel(const int32_t *__restrict__ nbr, int K, int n_rows, uint16_t *__restrict__ keys,
                     uint32_t *__restrict__ hist, int n_blocks) {
   after_previous();
-  next_may_start();
   extern __shared__ uint32_t hist_s[];  // [K + 1]
   const int B = K + 1;
   for (int b = threadIdx.x; b < B; b += ORD_BLOCK) hist_s[b] = 0u;
@@ -50,7 +49,6 @@ row_scatter_kernel(const uint16_t *__restrict__ keys, int B, int n_rows, const u
                    int32_t *__restrict__ order, const int32_t *__restrict__ nbr = nullptr, int K = 0,
                    int32_t *__restrict__ nbr_in_order = nullptr) {
   after_previous();
-  next_may_start();
   extern __shared__ uint32_t cnt[];  // [warps of the block][B] rows of each group in each warp
   for (int i = threadIdx.x; i < (int)(blockDim.x >> 5) * B; i += blockDim.x) cnt[i] = 0u;
   __syncthreads();
@@ -87,7 +85,6 @@ constexpr int PLANE_MAX_BITS = 9;
 __global__ void __launch_bounds__(PLANE_BLOCK)
 plane_bucket_table_kernel(int kx, int ky, int kz, uint16_t *__restrict__ bucket_of) {
   after_previous();
-  next_may_start();
   __shared__ uint8_t weight_s[1 << PLANE_MAX_BITS];
   const int n_keys = 1 << (kx + ky + kz);
   for (int key = threadIdx.x; key < n_keys; key += PLANE_BLOCK)
@@ -109,7 +106,6 @@ row_plane_key_hist_kernel(const int32_t *__restrict__ nbr, int kx, int ky, int k
                           const int32_t *__restrict__ n_rows_dev, const uint16_t *__restrict__ bucket_table,
                           uint16_t *__restrict__ keys, uint32_t *__restrict__ hist, int n_blocks) {
   after_previous();
-  next_may_start();
   extern __shared__ uint32_t hist_s[];  // [B] counters, then [B - 1] bucket of every key
   const int bits = kx + ky + kz, B = (1 << bits) + 1;
   uint32_t *bucket_of = hist_s + B;

@@ -53,7 +53,6 @@ pool_fwd_kernel(const void *__restrict__ features, int c, const int32_t *__restr
                 int n_out, const int32_t *__restrict__ summaryrf, float *__restrict__ out,
                 const int32_t *__restrict__ n_out_dev, int R) {
   after_previous();
-  next_may_start();
   extern __shared__ int32_t pool_smem[];
   const PoolTile tile = pool_tile(nbr, K, n_out, live_rows(n_out, n_out_dev), R, pool_smem);   // n_out: row stride of nbr
   const uint32_t cg = (uint32_t)(c + 3) / 4, items = (uint32_t)tile.rows * cg;
@@ -78,7 +77,6 @@ __global__ void __launch_bounds__(256)
 pool_fwd_few_kernel(const void *__restrict__ features, int c, const int32_t *__restrict__ nbr, int K, int n_out,
                     const int32_t *__restrict__ summaryrf, float *__restrict__ out, const int32_t *__restrict__ n_out_dev) {
   after_previous();
-  next_may_start();
   const uint32_t cg = (uint32_t)(c + 3) / 4;
   const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
   if (t >= (long long)live_rows(n_out, n_out_dev) * cg) return;
@@ -122,7 +120,6 @@ __global__ void __launch_bounds__(256)
 pool_divided_rows_kernel(const void *__restrict__ features, int c, const int32_t *__restrict__ nbr, int K, int n_out,
                          const int32_t *__restrict__ summaryrf, float *__restrict__ out, const int32_t *__restrict__ n_out_dev) {
   after_previous();
-  next_may_start();
   const int lane = threadIdx.x & 31, row0 = (int)(blockIdx.x * 256 + (threadIdx.x & ~31u)), n_rows = live_rows(n_out, n_out_dev);
   const int count = lane < n_rows - row0 ? __ldg(summaryrf + row0 + lane) : 1;
   for (unsigned left = __ballot_sync(0xffffffffu, !whole_count(count)); left != 0u; left &= left - 1u) {
@@ -145,7 +142,6 @@ pool_divided_rows_kernel(const void *__restrict__ features, int c, const int32_t
 
 __global__ void summary_rf_kernel(const int32_t *__restrict__ nbr, int K, int n_out, int32_t *__restrict__ rf) {
   after_previous();
-  next_may_start();
   int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= n_out) return;
   int cnt = 0;
@@ -159,7 +155,6 @@ template <bool MAX>
 __global__ void global_pool_kernel(const float *__restrict__ feats, const int32_t *__restrict__ offsets, int c,
                                    float *__restrict__ out, int32_t *__restrict__ maxidx) {
   after_previous();
-  next_may_start();
   __shared__ float sv[8][33];
   __shared__ int si[8][33];
   int s = blockIdx.x;
@@ -205,7 +200,6 @@ __global__ void global_pool_kernel(const float *__restrict__ feats, const int32_
 __global__ void batch_count_kernel(const int4 *__restrict__ indices, int n, int batch, int32_t *offsets,
                                    const int32_t *__restrict__ n_dev) {
   after_previous();
-  next_may_start();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int b = -1;
   if (i < live_rows(n, n_dev)) b = __ldg((const int32_t *)(indices + i));
@@ -215,7 +209,6 @@ __global__ void batch_count_kernel(const int4 *__restrict__ indices, int n, int 
 
 __global__ void batch_scan_kernel(int32_t *offsets, int batch) {
   after_previous();
-  next_may_start();
   int lane = threadIdx.x;
   int running = 0;
   for (int base = 1; base <= batch; base += 32) {
@@ -237,7 +230,6 @@ __global__ void __launch_bounds__(1024)
 batch_offsets_small_kernel(const int4 *__restrict__ indices, int n, int batch, int32_t *__restrict__ offsets,
                            const int32_t *__restrict__ n_dev) {
   after_previous();
-  next_may_start();
   __shared__ int hist[kOffsetsBatch];
   __shared__ uint32_t sums[33];
   for (int i = threadIdx.x; i < batch; i += 1024) hist[i] = 0;

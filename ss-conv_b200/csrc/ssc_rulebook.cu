@@ -98,7 +98,6 @@ __global__ void hash_insert_kernel(const int4 *__restrict__ indices, int n, int 
                                    Geometry g, unsigned long long *table, uint32_t mask,
                                    int32_t *status, const int32_t *__restrict__ n_dev) {
   after_previous();
-  next_may_start();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= live_rows(n, n_dev)) return;
   int4 c = indices[j];
@@ -128,7 +127,6 @@ __global__ void hash_insert_kernel(const int4 *__restrict__ indices, int n, int 
 __global__ void map_insert_kernel(const int4 *__restrict__ indices, int n, int batch, Geometry g,
                                   int32_t *__restrict__ row_map, int32_t *status, const int32_t *__restrict__ n_dev) {
   after_previous();
-  next_may_start();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= live_rows(n, n_dev)) return;
   int4 c = indices[j];
@@ -193,7 +191,6 @@ __global__ void __launch_bounds__(128)
 mark_outputs_kernel(const int4 *__restrict__ indices, int n, int batch, Geometry g, uint32_t *bitmap,
                     const int32_t *__restrict__ n_dev, int32_t *__restrict__ row_map, int32_t *status) {
   after_previous();
-  next_may_start();
   __shared__ uint32_t image[kMarkImageWords];
   __shared__ unsigned cell_min, cell_max;
   __shared__ int any_row;
@@ -267,7 +264,6 @@ mark_outputs_kernel(const int4 *__restrict__ indices, int n, int batch, Geometry
 __global__ void mark_outputs_generic_kernel(const int4 *__restrict__ indices, int n, int batch, Geometry g,
                                             uint32_t *bitmap, const int32_t *__restrict__ n_dev) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)live_rows(n, n_dev) * g.K) return;
   int j = (int)(t / g.K);
@@ -298,7 +294,6 @@ __global__ void decode_outputs_bits_kernel(const uint32_t *__restrict__ bitmap,
                                            const uint32_t *__restrict__ word_prefix, long long n_words,
                                            Geometry g, int n_out, int4 *out_indices) {
   after_previous();
-  next_may_start();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long w = t >> 5;
   if (w >= n_words) return;
@@ -323,7 +318,6 @@ __global__ void decode_outputs_kernel(const uint32_t *__restrict__ bitmap,
                                       const uint32_t *__restrict__ word_prefix, long long n_words,
                                       Geometry g, int n_out, int4 *out_indices) {
   after_previous();
-  next_may_start();
   // one thread per bitmap word (32 cells): most words of a sparse grid are empty and leave at once;
   // the set bits of a word get consecutive ranks from the word's prefix.  The coordinates of the
   // word's first cell are decoded once (three integer divisions); a set bit is that cell plus its
@@ -378,7 +372,6 @@ __global__ void __launch_bounds__(kRankThreads)
 rank_decode_kernel(const uint32_t *__restrict__ bitmap, int n_words, Geometry g, int n_out, int4 *__restrict__ out_indices,
                    int32_t *__restrict__ total_dev, const int32_t *__restrict__ status, CountPost post) {
   after_previous();
-  next_may_start();
   __shared__ uint32_t smem[33], word_s[WORDS], prefix_s[WORDS];
   const int w0 = (int)blockIdx.x * WORDS;
   uint32_t before = 0;
@@ -430,7 +423,6 @@ lookup_dense_kernel(const int4 *__restrict__ out_indices, int n_out, int batch, 
                     const int32_t *__restrict__ row_map, int32_t *__restrict__ nbr,
                     int32_t *__restrict__ chunk_counts, int n_chunks, const int32_t *__restrict__ n_out_dev) {
   after_previous();
-  next_may_start();
   extern __shared__ int32_t cnt[];  // [K] when counting
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
   const int n_rows = live_rows(n_out, n_out_dev);
@@ -514,7 +506,6 @@ lookup_neighbours_kernel(const int4 *__restrict__ out_indices, int n_out, int ba
                          int32_t *__restrict__ nbr, int32_t *__restrict__ chunk_counts, int n_chunks,
                          const int32_t *__restrict__ n_out_dev) {
   after_previous();
-  next_may_start();
   const unsigned full = 0xffffffffu;
   int kappa = blockIdx.y;
   int o = blockIdx.x * kChunk + threadIdx.x;
@@ -586,7 +577,6 @@ lookup_neighbours_kernel(const int4 *__restrict__ out_indices, int n_out, int ba
 // One block per kernel offset: exclusive scan of its chunk counts, total -> indice_num.
 __global__ void scan_chunks_kernel(int32_t *chunk_counts, int n_chunks, int32_t *indice_num) {
   after_previous();
-  next_may_start();
   __shared__ uint32_t smem[33];
   int32_t *row = chunk_counts + (size_t)blockIdx.x * n_chunks;
   uint32_t running = 0;
@@ -607,7 +597,6 @@ fill_pairs_kernel(const int32_t *__restrict__ nbr, int n_out, int n_in,
                   const int32_t *__restrict__ chunk_offsets, int n_chunks,
                   const int32_t *__restrict__ indice_num, int32_t *__restrict__ pairs) {
   after_previous();
-  next_may_start();
   __shared__ uint32_t smem[33];
   int kappa = blockIdx.y;
   int o = blockIdx.x * kChunk + threadIdx.x;
@@ -633,7 +622,6 @@ __global__ void pairs_to_nbr_kernel(const int32_t *__restrict__ pairs,
                                     const int32_t *__restrict__ indice_num, int n_cols, int n_out,
                                     int swap, int32_t *__restrict__ nbr) {
   after_previous();
-  next_may_start();
   int kappa = blockIdx.y;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_cols || i >= indice_num[kappa]) return;
@@ -648,7 +636,6 @@ __global__ void pairs_to_nbr_kernel(const int32_t *__restrict__ pairs,
 __global__ void __launch_bounds__(kChunk)
 count_chunks_kernel(const int32_t *__restrict__ nbr, int n_out, int32_t *__restrict__ chunk_counts, int n_chunks) {
   after_previous();
-  next_may_start();
   int kappa = blockIdx.y;
   int o = blockIdx.x * kChunk + threadIdx.x;
   int cnt = __syncthreads_count(o < n_out && nbr[(size_t)kappa * n_out + o] >= 0);

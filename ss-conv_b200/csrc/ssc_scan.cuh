@@ -50,7 +50,6 @@ template <bool POPC>
 __global__ void popc_block_sums_kernel(const uint32_t *__restrict__ bitmap, long long n_words,
                                        uint32_t *block_sums) {
   after_previous();
-  next_may_start();
   __shared__ uint32_t smem[33];
   long long base = (long long)blockIdx.x * 1024 + threadIdx.x * 4;
   uint32_t s = 0;
@@ -65,7 +64,6 @@ __global__ void popc_block_sums_kernel(const uint32_t *__restrict__ bitmap, long
 // block_sums[n] and to the two int32 outputs.
 static __global__ void scan_block_sums_kernel(uint32_t *block_sums, int n, int32_t *total_a, int32_t *total_b) {
   after_previous();
-  next_may_start();
   __shared__ uint32_t smem[33];
   uint32_t running = 0;
   for (int base = 0; base < n; base += blockDim.x) {
@@ -87,7 +85,6 @@ template <bool POPC>
 __global__ void word_prefix_kernel(const uint32_t *__restrict__ bitmap, long long n_words,
                                    const uint32_t *__restrict__ block_sums, uint32_t *word_prefix) {
   after_previous();
-  next_may_start();
   __shared__ uint32_t smem[33];
   long long base = (long long)blockIdx.x * 1024 + threadIdx.x * 4;
   uint32_t c[4];
@@ -114,7 +111,6 @@ template <bool POPC>
 __global__ void __launch_bounds__(1024)
 single_block_scan_kernel(const uint32_t *values, int n, uint32_t *prefix, int32_t *total_a, int32_t *total_b) {
   after_previous();
-  next_may_start();
   // values and prefix may be the same array (in-place scan): every value is read before its slot is written
   __shared__ uint32_t smem[33];
   const int per = (n + 1023) / 1024;          // values per thread (<= 8)

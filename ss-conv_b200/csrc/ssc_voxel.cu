@@ -8,7 +8,6 @@ namespace ssc {
 __global__ void v2p_map_kernel(const int32_t *__restrict__ inverse, const int32_t *__restrict__ ids, int32_t *maps,
                                int n_point, int n_voxel, int max_active, int mode) {
   after_previous();
-  next_may_start();
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n_point) return;
   int v = inverse[p];
@@ -30,7 +29,6 @@ __global__ void v2p_map_kernel(const int32_t *__restrict__ inverse, const int32_
 // Modes 3/4: order every row's ids ascending so that later sums are reproducible.
 __global__ void v2p_sort_rows_kernel(int32_t *maps, int n_voxel, int max_active) {
   after_previous();
-  next_may_start();
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n_voxel) return;
   int32_t *row = maps + (size_t)v * (max_active + 1);
@@ -49,7 +47,6 @@ __global__ void v2p_sort_rows_kernel(int32_t *maps, int n_voxel, int max_active)
 __global__ void voxelize_fwd_kernel(const float *__restrict__ feats, float *__restrict__ out,
                                     const int32_t *__restrict__ maps, int average, int n_voxel, int max_active, int c) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n_voxel * c) return;
   int v = (int)(t / c), ch = (int)(t - (long long)v * c);
@@ -119,7 +116,6 @@ __device__ __forceinline__ bool point_cell(const float *p, int b, int batch, con
 __global__ void p2v_mark_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, int n,
                                 int batch, VoxelGrid g, uint32_t *bitmap, int32_t *status) {
   after_previous();
-  next_may_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float p[3] = {points[i * 3 + 0], points[i * 3 + 1], points[i * 3 + 2]};
@@ -148,7 +144,6 @@ __device__ __forceinline__ bool point_inside(const float *__restrict__ p, const 
 __global__ void p2v_stats_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, int n,
                                  VoxelGrid g, int32_t *stats) {
   after_previous();
-  next_may_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool out = false, down = false, change = false;
   if (i < n) {
@@ -174,7 +169,6 @@ __global__ void __launch_bounds__(256)
 p2v_kept_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, int n, VoxelGrid g, int n_sample,
                 int32_t *__restrict__ kept) {
   after_previous();
-  next_may_start();
   const int i = blockIdx.x * 256 + threadIdx.x;
   int b = -1;
   if (i < n && point_inside(points + (size_t)i * 3, g)) b = __ldg(batch_ids + i);
@@ -186,7 +180,6 @@ __global__ void __launch_bounds__(256)
 p2v_stays_kernel(const float *__restrict__ points, const int32_t *__restrict__ batch_ids, int n, VoxelGrid g, int n_sample,
                  const int32_t *__restrict__ kept, uint32_t *__restrict__ bitmap, float *__restrict__ flag, int32_t *__restrict__ n_empty) {
   after_previous();
-  next_may_start();
   const int i = blockIdx.x * 256 + threadIdx.x;
   bool stays = false, empty = false;
   if (i < n) {
@@ -206,7 +199,6 @@ p2v_gather_kernel(const float *__restrict__ points, const int32_t *__restrict__ 
                   VoxelGrid g, const uint32_t *__restrict__ bitmap, const uint32_t *__restrict__ prefix,
                   float *__restrict__ new_points, int32_t *__restrict__ new_ids, float *__restrict__ new_feats) {
   after_previous();
-  next_may_start();
   const uint32_t groups = (uint32_t)(c / VEC);
   const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
   if (t >= (long long)n * groups) return;
@@ -236,7 +228,6 @@ __global__ void p2v_inverse_kernel(const float *__restrict__ points, const int32
                                    const uint32_t *__restrict__ word_prefix, int mode, int32_t *inverse,
                                    uint32_t *count, uint32_t *select) {
   after_previous();
-  next_may_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float p[3] = {points[i * 3 + 0], points[i * 3 + 1], points[i * 3 + 2]};
@@ -258,7 +249,6 @@ __global__ void p2v_inverse_kernel(const float *__restrict__ points, const int32
 __global__ void p2v_scatter_kernel(const int32_t *__restrict__ inverse, int n, const uint32_t *__restrict__ start,
                                    const uint32_t *__restrict__ rank, int32_t *order) {
   after_previous();
-  next_may_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int v = inverse[i];
@@ -268,7 +258,6 @@ __global__ void p2v_scatter_kernel(const int32_t *__restrict__ inverse, int n, c
 
 __global__ void p2v_sort_segments_kernel(const uint32_t *__restrict__ start, int n_voxel, int32_t *order) {
   after_previous();
-  next_may_start();
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n_voxel) return;
   int a = (int)start[v], b = (int)start[v + 1];
@@ -285,7 +274,6 @@ __global__ void p2v_sort_segments_kernel(const uint32_t *__restrict__ start, int
 __global__ void p2v_reduce_kernel(const float *__restrict__ feats, int c, const uint32_t *__restrict__ start,
                                   const int32_t *__restrict__ order, int n_voxel, int average, float *__restrict__ out) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n_voxel * c) return;
   int v = (int)(t / c), ch = (int)(t - (long long)v * c);
@@ -305,7 +293,6 @@ __global__ void __launch_bounds__(256)
 p2v_reduce_small_kernel(const float *__restrict__ feats, int c, const uint32_t *__restrict__ start,
                         const int32_t *__restrict__ order, int n_voxel, int average, float *__restrict__ out) {
   after_previous();
-  next_may_start();
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n_voxel) return;
   const int a = (int)start[v], b = (int)start[v + 1];
@@ -329,7 +316,6 @@ p2v_reduce_small_kernel(const float *__restrict__ feats, int c, const uint32_t *
 __global__ void p2v_select_kernel(const float *__restrict__ feats, int c, const uint32_t *__restrict__ select,
                                   int n_voxel, int n_point, float *__restrict__ out) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n_voxel * c) return;
   int v = (int)(t / c), ch = (int)(t - (long long)v * c);
@@ -359,7 +345,6 @@ __global__ void __launch_bounds__(NN_TILE)
 nn_ranges_kernel(const float4 *__restrict__ known, int m, float2 *__restrict__ ranges, float4 *__restrict__ chunks, float4 *__restrict__ tiles,
                  int32_t *__restrict__ shares) {
   after_previous();
-  next_may_start();
   __shared__ float4 chunk_s[32];
   __shared__ int in_s[32];
   const int lane = threadIdx.x & 31, c = threadIdx.x >> 5, k = blockIdx.x * NN_TILE + (int)threadIdx.x;
@@ -660,7 +645,6 @@ three_nn_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *
                 const float4 *__restrict__ chunks, const float4 *__restrict__ tiles, const int32_t *__restrict__ shares, float *__restrict__ dist2,
                 int32_t *__restrict__ idx) {
   after_previous();
-  next_may_start();
   const int first = (int)blockIdx.x * 32, q0 = first + ((int)threadIdx.x >> 5) * NN_QUERIES;
   const float4 own = __ldg(unknown + min(q0, n - 1));
   NnSpan span = {0.f, 0, 0, NN_SHARES};
@@ -674,7 +658,6 @@ __global__ void __launch_bounds__(256)
 three_nn_warps_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known, const float4 *__restrict__ chunks,
                       const float4 *__restrict__ tiles, const int32_t *__restrict__ shares, float *__restrict__ dist2, int32_t *__restrict__ idx) {
   after_previous();
-  next_may_start();
   const int first = (int)blockIdx.x * 32, q0 = first + ((int)threadIdx.x >> 5) * NN_QUERIES;
   const float4 own = __ldg(unknown + min(q0, n - 1));
   const NnSpan span = nn_group<64>(first, m, unknown, tiles, shares);
@@ -684,7 +667,6 @@ __global__ void __launch_bounds__(256)
 three_nn_tiles_kernel(int n, int m, const float4 *__restrict__ unknown, const float4 *__restrict__ known, const float2 *__restrict__ ranges,
                       const float4 *__restrict__ tiles, const int32_t *__restrict__ shares, float *__restrict__ dist2, int32_t *__restrict__ idx) {
   after_previous();
-  next_may_start();
   const int first = (int)blockIdx.x * 64;
   if (tiles != nullptr && nn_group<64>(first, m, unknown, tiles, shares).share <= NN_MOST) return;
   nn_by_tiles<4>(first, n, m, unknown, known, ranges, dist2, idx);
@@ -695,7 +677,6 @@ three_nn_tiles_kernel(int n, int m, const float4 *__restrict__ unknown, const fl
 __global__ void __launch_bounds__(256)
 voxel_centres_kernel(const int4 *__restrict__ indices, int n, float3 unit, float3 half_extent, float3 half_unit, float4 *__restrict__ out) {
   after_previous();
-  next_may_start();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   const int4 v = __ldg(indices + i);
@@ -706,14 +687,12 @@ voxel_centres_kernel(const int4 *__restrict__ indices, int n, float3 unit, float
 __global__ void __launch_bounds__(256)
 point_rows_kernel(const float *__restrict__ points, const int32_t *__restrict__ ids, int n, float4 *__restrict__ out) {
   after_previous();
-  next_may_start();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i < n) out[i] = make_float4((float)__ldg(ids + i), __ldg(points + (size_t)i * 3), __ldg(points + (size_t)i * 3 + 1), __ldg(points + (size_t)i * 3 + 2));
 }
 __global__ void __launch_bounds__(256)
 nn_weights_kernel(const float *__restrict__ dist2, int n, float *__restrict__ weight) {
   after_previous();
-  next_may_start();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   float r[3];
@@ -728,7 +707,6 @@ __global__ void three_interpolate_kernel(int c, int n, const float *__restrict__
                                          const int32_t *__restrict__ idx, const float *__restrict__ weight,
                                          float *__restrict__ out) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)n * c) return;
   int p = (int)(t / c), ch = (int)(t - (long long)p * c);
@@ -747,7 +725,6 @@ __global__ void __launch_bounds__(256)
 three_interpolate_vec4_kernel(uint32_t groups, uint32_t total, const float4 *__restrict__ points,
                               const int32_t *__restrict__ idx, const float *__restrict__ weight, float4 *__restrict__ out) {
   after_previous();
-  next_may_start();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= total) return;
   const uint32_t p = t / groups, g = t - p * groups;
@@ -814,7 +791,6 @@ __global__ void __launch_bounds__(128)
 steer_matrices_kernel(const T *__restrict__ rot, int orders, const double *__restrict__ dirs,
                       const double *__restrict__ pinv, int axes, int stride, float *__restrict__ dmats) {
   after_previous();
-  next_may_start();
   extern __shared__ double ys[];                 // per order [S][2 l + 1], as pinv
   const int b = blockIdx.x;
   double R[3][3], Q[3][3];
@@ -888,7 +864,6 @@ __global__ void steer_kernel(const float *__restrict__ points, const float *__re
                              const int32_t *__restrict__ chan, int n, int c, int n_sample, float *__restrict__ new_points,
                              float *__restrict__ new_feats) {
   after_previous();
-  next_may_start();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int width = c + 3;
   if (t >= (long long)n * width) return;

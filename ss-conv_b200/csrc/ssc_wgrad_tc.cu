@@ -49,7 +49,6 @@ constexpr int WT_BLOCK = WT_K * 128;   // 32 channels of a chunk's pairs
 __global__ void __launch_bounds__(256)
 pair_bitmap_kernel(const int32_t *__restrict__ nbr, int n_out, int words_per_row, uint32_t *__restrict__ bitmap) {
   after_previous();
-  next_may_start();
   const int w0 = ((int)blockIdx.x * 8 + (int)(threadIdx.x >> 5)) * 4, lane = threadIdx.x & 31;
   if (w0 >= words_per_row) return;
   const int32_t *row = nbr + (size_t)blockIdx.y * n_out;
@@ -77,7 +76,6 @@ pair_scatter_kernel(const int32_t *__restrict__ nbr, int n_out, int words_per_ro
                     const uint32_t *__restrict__ bitmap, const uint32_t *__restrict__ prefix,
                     int32_t *__restrict__ pair_out, int32_t *__restrict__ pair_in, int32_t *__restrict__ starts) {
   after_previous();
-  next_may_start();
   __shared__ uint16_t list_s[8][1024];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kappa = blockIdx.y;
   const int w0 = ((int)blockIdx.x * 8 + warp) * 32, w = w0 + lane;
@@ -172,7 +170,6 @@ __global__ void __launch_bounds__((2 * WT_MAX_STAGES + 5) * 32, 2)
 conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in,
                      const int32_t *__restrict__ starts, int K, float *__restrict__ partial, int32_t *status) {
   after_previous();
-  next_may_start();
   extern __shared__ uint8_t smem_raw[];
   __shared__ int first[257];
   __shared__ uint64_t full_bars[WT_MAX_STAGES], empty_bars[WT_MAX_STAGES], accf_bars[2], acce_bars[2], done_bar;
@@ -401,7 +398,6 @@ conv_wgrad_small_kernel(const float *__restrict__ features, int c_in, const floa
                         const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in,
                         const int32_t *__restrict__ starts, int K, float *__restrict__ partial) {
   after_previous();
-  next_may_start();
   __shared__ int first[257];
   chunk_prefix(starts, K, first);
   const int lane = threadIdx.x & 31, co = blockIdx.y * 32 + lane;
@@ -445,7 +441,6 @@ __global__ void __launch_bounds__(256)
 wgrad_reduce_shares_kernel(const float *__restrict__ partial, const int32_t *__restrict__ starts, int K, int shares, int elems,
                            float *__restrict__ out) {
   after_previous();
-  next_may_start();
   __shared__ int first[257];
   __shared__ float sm[8][32 * VEC + 1];
   chunk_prefix(starts, K, first);

@@ -363,3 +363,27 @@ def test_packed_filter_sizes_follow_the_operand_layout():
     assert L.ssc_conv_packed_bytes(27, 3, 38, _ext.PREC_BF16) == full(27, 1)
     assert L.ssc_conv_packed_bytes(27, 100, 38, _ext.PREC_F16) == full(27, 2)
     assert L.ssc_conv_pairs_supported(16, 256, _ext.PREC_TF32) == 0                  # grouped filters: not for the pair-list kernel
+
+
+def _device_code():
+    """The kernels' sources without comments."""
+    folder = os.path.join(ROOT, "ss-conv_b200", "csrc")
+    for name in sorted(os.listdir(folder)):
+        if name.endswith((".cu", ".cuh")):
+            yield name, re.sub(r"//[^\n]*|/\*.*?\*/", "", open(os.path.join(folder, name)).read(), flags=re.S)
+
+
+def test_kernels_wait_for_the_ones_before_them_and_do_not_let_the_next_in():
+    """A kernel that is launched while the one before it may still run waits in its first statement (the row convolution
+    behind a prefetch, which reads nothing); only kernels launched the ordinary way do without.  None lets the next one's
+    blocks in before its own have ended."""
+    waits, plain, without = set(), set(), set()
+    for name, text in _device_code():
+        assert "launch_dependents" not in text, name
+        plain |= set(re.findall(r"\b(\w+)(?:<[^<>;]*>)?<<<", text))
+        for header, first in re.findall(r"__global__([^{};]*)\{\s*([^;]*;)", text):
+            kernel = re.findall(r"(\w+)\s*\((?:[^()]|\([^()]*\))*\)\s*$", header)[0]
+            (waits if first == "after_previous();" or first.startswith("conv_fwd_rows<") else without).add(kernel)
+    assert len(waits) > 60 and without == plain, (without, plain)
+    body = dict(_device_code())["ssc_conv_tc.cu"].split("conv_fwd_rows(const float *", 1)[1].split("{", 1)[1]
+    assert not re.search(r"features|nbr|out\b|live_rows", body.split("after_previous();", 1)[0])
