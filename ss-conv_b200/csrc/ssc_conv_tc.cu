@@ -1020,7 +1020,9 @@ __global__ void pack_filters_16_kernel(const float *__restrict__ filters, int K,
 // the launch has for it, so that they share its memory for deeper rings (256 tiles of 64 -> 76 bf16 channels, two on an SM instead of
 // four: 20.2 -> 15.7 us).  Row tiles that fit the SMs by themselves but not with their N tiles
 // spread stay whole: a few SMs with two CTAs would make all wait for rings of half the depth (79 row tiles
-// of 256 -> 304 bf16 channels: 62 us spread).
+// of 256 -> 304 bf16 channels: 62 us spread).  Rows of one slab take four CTAs on an SM where the launch has three: their rings turn
+// over quickly, and a fourth place takes the tiles of a row order that are left (45 k rows, 3 and 4 CTAs: 16 -> 22 in order 32.2 and 30.8 us,
+// 32 -> 38 in order 32.3 and 30.9, 8 -> 22 21.1 and 19.4, 20 -> 38 28.2 and 28.5; of three slabs, 76 -> 64 in order, 39.1 and 44.7).
 // Pairs: from 128 columns a CTA and four slabs an offset on, up to two tiles an SM.  There the filter slab, which every
 // tile brings in whole, is most of what a step moves (TF32 128 -> 152, 238 tiles: 59.1 -> 52.3 us; 256 -> 304 bf16, 125 tiles: 54.4 -> 52.6).  The second CTA's
 // news reaches the issuing one some 300 cycles late, so short loops lose (256 tiles of 128 -> 152 bf16: 30.8 -> 31.9), rings of two slots
@@ -1028,7 +1030,8 @@ __global__ void pack_filters_16_kernel(const float *__restrict__ filters, int K,
 static bool rows_params(int words, int c_out, int n_out, TcParams &p, int opk = 1, bool pairs = false) {
   const int grid = n_out > 0 ? ceil_div(n_out, TC_M) : 1, sms = sm_count();
   auto plan = [&](bool pair) {
-    if (!tc_params(words, c_out, p, false, ceil_div(grid, sms), opk, pair)) return false;
+    const int ctas = ceil_div(grid, sms);
+    if (!tc_params(words, c_out, p, false, ctas == 3 && words <= TC_SLAB ? 4 : ctas, opk, pair)) return false;
     if (p.n_tiles == 1 || grid >= 2 * sms || (grid <= sms && grid * p.n_tiles > sms)) return true;
     return tc_params(words, c_out, p, true, ceil_div(grid * p.n_tiles, sms), opk, pair);
   };
