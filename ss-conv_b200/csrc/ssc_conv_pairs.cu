@@ -558,7 +558,7 @@ static size_t pl_smem_bytes(const PlParams &p) {
 
 // Shapes the kernel covers: the filter matrix of one offset (or one range of its output channels)
 // resident in shared memory next to at least three ring slots.
-static bool pl_params(int c_in, int c_out, int precision, PlParams &p) {
+static bool pl_params(int c_in, int c_out, int precision, PlParams &p, bool by_two = true) {
   p.pair = 0;
   const bool is16 = precision == SSC_PREC_F16 || precision == SSC_PREC_BF16;
   if (!is16 && tf32_offsets_per_row(c_in) > 1) return false;   // those filters are packed several offsets per row
@@ -584,7 +584,7 @@ static bool pl_params(int c_in, int c_out, int precision, PlParams &p) {
   if (p.n_split == 0 || p.n_cta < 16) return false;
   // A matrix that one CTA cannot hold whole goes to two (with ranges of its channels every row is gathered once per range): 177 k rows
   // of 256 -> 256 TF32 866 -> 679 us, 50 k rows of 208 -> 224 330 -> 239.  One that fits stays: 41 k rows of 192 -> 192 bf16 178 and 182.
-  if (p.n_split > 1 && p.n_pad <= 256 && (size_t)p.k_slabs * (p.n_pad / 2) * 128 + 3 * (size_t)PL_A_BYTES <= budget) {
+  if (by_two && p.n_split > 1 && p.n_pad <= 256 && (size_t)p.k_slabs * (p.n_pad / 2) * 128 + 3 * (size_t)PL_A_BYTES <= budget) {
     p.pair = 1;
     p.n_split = 1;
     p.n_cta = p.n_pad;
@@ -617,7 +617,12 @@ size_t conv_pairs_strip_bytes(int K) { return 256 + max_strips(K) * (sizeof(int4
 int conv_fwd_pairs(const float *rows, int n_in, void *staged, int c_in, const void *packed, int K, int c_out, int precision,
                    const PairLists &pl, int n_out, float *out, int32_t *status, void *strip_mem, cudaStream_t st) {
   PlParams p;
-  if (K > 256 || !pl_params(c_in, c_out, precision, p))
+  // Lists of few pairs, most of them shorter than a CTA's 128, leave the second CTA of a tile idle, and with channels that are added one by one
+  // the adding, which it does not share.  27 offsets, 2 and 9 neighbours a row, ranges of channels and two CTAs, us: 200 rows of
+  // 256 -> 256 15.0, 15.0 and 15.5, 15.8; 600 15.1, 20.1 and 16.1, 17.0; 2000 20.2, 26.6 and 17.4, 23.8; of 200 -> 250 200 rows 17.4, 20.7 and 17.7, 23.6;
+  // 2000 28.4, 48.0 and 31.6, 50.6; 5000 40.0, 109.9 and 36.7, 90.7.  (125 offsets: 35.5 and 29.0 for 200 rows.)
+  const bool by_two = K >= 64 || n_out >= ((c_out & 3) == 0 ? 1024 : 4096);
+  if (K > 256 || !pl_params(c_in, c_out, precision, p, by_two))
     return fail(SSC_ERR_INVALID, "conv_fwd_pairs: shape (c_in %d, c_out %d, kernel volume %d) not covered by the pair-list kernel", c_in, c_out, K);
   p.alarm = alarm_word();
   int n_ctas = sm_count() * p.ctas_per_sm;

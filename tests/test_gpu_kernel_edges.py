@@ -273,6 +273,25 @@ def test_pair_lists_prepared_in_one_launch(cuda, precision, c_in, c_out, n):
     assert rel_err(pairs.cpu(), rows.cpu()) <= 5e-5
 
 
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("K,c_in,c_out,n", [(63, 256, 256, 200), (64, 256, 256, 1), (64, 250, 256, 129), (64, 256, 250, 700), (27, 256, 256, 1023), (27, 256, 256, 1024),
+                                            (27, 256, 250, 4095), (27, 256, 250, 4096), (27, 512, 256, 1024)])
+def test_pair_lists_by_one_cta_and_by_two(cuda, precision, K, c_in, c_out, n):
+    """Both sides of the lines from which two CTAs share a filter matrix (64 offsets; 1024 rows, 4096 where channels are added one
+    by one): same operands and fp32 sums as the output-stationary kernel, in another order."""
+    from ss_conv import _ext
+    if not _ext.lib().ssc_conv_pairs_supported(c_in, c_out, _ext._PREC_OF[precision]):
+        pytest.skip("shape not covered by the pair-list kernel")
+    rng = np.random.RandomState(n)
+    t = dev(_table(n, 150, K, 0.3, rng), cuda)
+    x = dev(rng.randn(150, c_in).astype(np.float32), cuda)
+    w = dev((rng.randn(K, c_in, c_out) * 0.1).astype(np.float32), cuda)
+    rows = _ext.conv_forward(x, w, t, n, precision, algo="rows")
+    pairs = _ext.conv_forward(x, w, t, n, precision, algo="pairs")
+    _ext.check_status(cuda)
+    assert rel_err(pairs.cpu(), rows.cpu()) <= 5e-5
+
+
 @pytest.mark.parametrize("orders,batch", [(1, 1), (4, 65), (8, 3)])
 @pytest.mark.parametrize("frame", ["kernel", "reference"])
 def test_steering_matrices_match_the_host_form(cuda, orders, batch, frame):
