@@ -403,7 +403,7 @@ conv_fwd_pairs_body(const float *__restrict__ staged, const uint4 *__restrict__ 
         }
         const uint32_t d = tmem_base + (uint32_t)(buf * p.acc_cols);
         for (int s = 0; s < p.k_slabs; ++s) {
-          if (!(PAIR ? mbar_wait_straight_cluster(smem_u32(full_bars + slot), slot_par, abort_flag) : mbar_wait_straight(smem_u32(full_bars + slot), slot_par, abort_flag))) { alive = false; break; }
+          if (!(PAIR ? mbar_wait_straight_cluster(smem_u32(full_bars + slot), slot_par, abort_flag) : mbar_wait_uniform(smem_u32(full_bars + slot), slot_par, abort_flag))) { alive = false; break; }
           fence_async_smem();                             // the rows other threads' copies left, for the tensor core
           tc_fence_after();
           const uint32_t a_lo = desc_lo(a_base + slot * PL_A_BYTES);
