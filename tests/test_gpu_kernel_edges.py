@@ -684,9 +684,11 @@ def test_norm_entry_points_for_c_callers(cuda, n, training):
     assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
-@pytest.mark.parametrize("c_in,c_out,n", [(64, 152, 300), (128, 304, 130), (17, 129, 77), (128, 257, 64), (96, 512, 33), (130, 304, 65), (128, 128, 40)])
+@pytest.mark.parametrize("c_in,c_out,n", [(64, 152, 300), (128, 304, 130), (17, 129, 77), (128, 257, 64), (96, 512, 33), (130, 304, 65), (128, 128, 40),
+                                          (64, 152, 4095), (64, 152, 4096), (128, 304, 4100), (17, 129, 4097), (128, 257, 4096), (130, 304, 4096), (40, 177, 16383),
+                                          (40, 177, 16384), (24, 512, 16385), (128, 190, 16400)])
 def test_filter_gradient_on_either_side_of_a_product(cuda, c_in, c_out, n):
-    """Around 128 input and 128 and 256 output channels, where they change places: against float64.  TF32 rounds the
+    """Around 128 input and 128 and 256 output channels and 4096 and 16384 rows, where they change places: against float64.  TF32 rounds the
     operands to 11 bits, so a sum of products is within 2^-11 of the sum of magnitudes, typically a tenth of it."""
     from ss_conv import _ext
     rng = np.random.RandomState(n)

@@ -387,3 +387,11 @@ def test_kernels_wait_for_the_ones_before_them_and_do_not_let_the_next_in():
     assert len(waits) > 60 and without == plain, (without, plain)
     body = dict(_device_code())["ssc_conv_tc.cu"].split("conv_fwd_rows(const float *", 1)[1].split("{", 1)[1]
     assert not re.search(r"features|nbr|out\b|live_rows", body.split("after_previous();", 1)[0])
+
+
+@pytest.mark.parametrize("c_in,c_out,line", [(128, 152, 4096), (128, 256, 16384)])
+def test_few_pairs_keep_few_partial_filter_gradients(c_in, c_out, line):
+    """Input channels as rows of one product double the partial sums of a launch, which few rows do not pay for."""
+    from ss_conv._ext import lib
+    few, many = (lib().ssc_conv_wgrad_scratch_bytes(27, c_in, c_out, n) - lib().ssc_conv_pairs_list_bytes(27, n) for n in (line - 1, line))
+    assert few < 0.75 * many
