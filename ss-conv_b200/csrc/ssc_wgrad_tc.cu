@@ -41,7 +41,8 @@ namespace ssc {
 
 constexpr int WT_M = 128;          // output channels per CTA
 constexpr int WT_K = 32;           // pairs per chunk
-constexpr int WT_MAX_STAGES = 5;   // two CTAs of 15 warps with 64 registers a thread fit an SM
+constexpr int WT_MAX_STAGES = 8;   // of a CTA by itself on its SM; two of 15 warps with 64 registers a thread fit one: 5 each
+constexpr int wt_stages(int ctas) { return ctas == 2 ? 5 : WT_MAX_STAGES; }
 constexpr int WT_BLOCK = WT_K * 128;   // 32 channels of a chunk's pairs
 
 // Which output rows have a neighbour: a warp makes four words (128 rows) of one kernel offset (blockIdx.y), four
@@ -166,7 +167,8 @@ __device__ __forceinline__ void copy_block(uint32_t dst, const float *const (&g)
         : "memory");
 }
 
-__global__ void __launch_bounds__((2 * WT_MAX_STAGES + 5) * 32, 2)
+template <int CTAS>
+__global__ void __launch_bounds__((2 * wt_stages(CTAS) + 5) * 32, CTAS)
 conv_wgrad_tc_kernel(WtParams p, const int32_t *__restrict__ pair_out, const int32_t *__restrict__ pair_in,
                      const int32_t *__restrict__ starts, int K, float *__restrict__ partial, int32_t *status) {
   after_previous();
@@ -534,7 +536,7 @@ int pair_lists_build(const int32_t *nbr, int K, int n_out, void *lists, PairList
 // Shapes and shares of the two list kernels.
 struct WgradPlan {
   bool tc, small, in_rows;
-  int n_pad, n_buf, co_blocks, shares, stages, a_bytes, stage_bytes;
+  int n_pad, n_buf, co_blocks, shares, ctas, stages, a_bytes, stage_bytes;
   uint32_t buf_cols;
   size_t smem;
 };
@@ -572,7 +574,8 @@ static WgradPlan wgrad_plan(int K, int c_in, int c_out, int n_out, bool tf32) {
     const size_t slack = 1024 + (size_t)4 * WT_BLOCK, fixed = 2048;
     const int ctas = 4 * (size_t)p.stage_bytes + slack + fixed <= 113 * 1024 ? 2 : 1;
     p.stages = (int)(((ctas == 2 ? 113 : 226) * 1024 - slack - fixed) / p.stage_bytes);
-    if (p.stages > WT_MAX_STAGES) p.stages = WT_MAX_STAGES;
+    if (p.stages > wt_stages(ctas)) p.stages = wt_stages(ctas);
+    p.ctas = ctas;
     if (p.stages < 2) { p.tc = false; return p; }
     p.smem = (size_t)p.stages * p.stage_bytes + slack;
     p.n_buf = (int)p.buf_cols * 2 * ctas <= 512 ? 2 : 1;
@@ -601,11 +604,12 @@ int conv_wgrad_lists(const float *features, int c_in, const float *out_grad, int
                      bool tf32, int staged, float *partial, float *d_filters, int32_t *status, cudaStream_t st) {
   const WgradPlan p = wgrad_plan(K, c_in, c_out, n_out, tf32);
   if (p.tc) {
-    cudaError_t e = allow_smem((const void *)conv_wgrad_tc_kernel, p.smem);
+    auto kernel = p.ctas == 2 ? conv_wgrad_tc_kernel<2> : conv_wgrad_tc_kernel<1>;
+    cudaError_t e = allow_smem((const void *)kernel, p.smem);
     if (e != cudaSuccess) return fail(SSC_ERR_CUDA, "conv_wgrad(tf32): smem attribute: %s", cudaGetErrorString(e));
     const WtParams w = {features, out_grad, c_in, c_out, (staged & 1) ? (c_in + 3) & ~3 : c_in, (staged & 2) ? (c_out + 3) & ~3 : c_out,
                         (staged & 1) ? 0 : 1, (staged & 2) ? 0 : 1, p.n_pad, p.a_bytes, p.stage_bytes, p.stages, p.n_buf, p.in_rows ? 1 : 0, p.buf_cols, alarm_word()};
-    { launch_ready(conv_wgrad_tc_kernel, dim3(p.shares, p.co_blocks), dim3((2 * p.stages + 5) * 32), p.smem, st, w, pl.pair_out, pl.pair_in, pl.starts, K, partial, status); note_launches(1); }
+    { launch_ready(kernel, dim3(p.shares, p.co_blocks), dim3((2 * p.stages + 5) * 32), p.smem, st, w, pl.pair_out, pl.pair_in, pl.starts, K, partial, status); note_launches(1); }
     SSC_CHECK_LAUNCH("conv_wgrad_tc");
   } else if (p.small) {
     const dim3 grid(p.shares / 4, p.co_blocks);
