@@ -620,7 +620,7 @@ bn_gate_bwd_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__res
 // rows, then a block's warps in order; a block is one chain of the totals.  The form above hands every element through shared memory
 // and adds up a channel per thread, 32 rows at a time, while the other threads wait: 162 k rows of 32 + 6 channels 47 + 33 us, here
 // 19 + 16; 93 k rows of 64 + 12 30 + 25, here 18 + 16 (the bytes of the two passes take 8 and 12).  A gate's sum takes fields of up
-// to seven channels at once: as a loop it was half of the kernel.  Wider rows, others than fours and unaligned gradients stay above.
+// to seven channels at once: as a loop it was half of the kernel.  Wider rows and others than fours stay above.
 template <int VEC>
 __device__ __forceinline__ void row_quad(const float *at, float (&v)[4]) {
   if (VEC == 4) {
@@ -634,7 +634,7 @@ __device__ __forceinline__ void row_quad(const float *at, float (&v)[4]) {
     for (int i = 0; i < 4; ++i) v[i] = __ldg(at + i);
   }
 }
-template <int PASS, int VEC, int QL>
+template <int PASS, int VEC, int GVEC, int QL>
 __global__ void __launch_bounds__(256, QL == 1 ? 4 : 2)
 bn_gate_bwd_lanes_kernel(BnGateBwd p, int L, const float *__restrict__ ks, const float *__restrict__ ka, const float *__restrict__ kg,
                          float *__restrict__ gx, float *__restrict__ part_a, float *__restrict__ part_g) {
@@ -704,7 +704,7 @@ bn_gate_bwd_lanes_kernel(BnGateBwd p, int L, const float *__restrict__ ks, const
       for (int i = 0; i < 4; ++i) x[q][i] = go[q][i] = 0.f;
       if (in && mine[q]) {
         row_quad<VEC>(xr + (at + q * L) * 4, x[q]);
-        row_quad<4>(gr + (at + q * L) * 4, go[q]);
+        row_quad<GVEC>(gr + (at + q * L) * 4, go[q]);
       }
     }
 #pragma unroll
@@ -1092,10 +1092,14 @@ static void launch_bwd_lanes(const BnGateBwd &p, int lanes, const float *ks, con
     const int most = (QL == 1 ? 4 : 2) * sm_count();
     if (blocks > most) blocks = most;
   }
+  // (the order of the sums does not depend on where rows and gradients lie: only how they are loaded does)
   const uintptr_t at = (uintptr_t)p.x | (uintptr_t)gx;
-  if ((p.c & 3) == 0 && (at & 15u) == 0) launch_ready(bn_gate_bwd_lanes_kernel<PASS, 4, QL>, dim3(blocks), dim3(256), smem, st, p, lanes, ks, ka, kg, gx, part_a, part_g);
-  else if ((p.c & 1) == 0 && (at & 7u) == 0) launch_ready(bn_gate_bwd_lanes_kernel<PASS, 2, QL>, dim3(blocks), dim3(256), smem, st, p, lanes, ks, ka, kg, gx, part_a, part_g);
-  else launch_ready(bn_gate_bwd_lanes_kernel<PASS, 1, QL>, dim3(blocks), dim3(256), smem, st, p, lanes, ks, ka, kg, gx, part_a, part_g);
+  auto kernel = bn_gate_bwd_lanes_kernel<PASS, 1, 1, QL>;
+  if (((uintptr_t)p.go & 15u) == 0)
+    kernel = (p.c & 3) == 0 && (at & 15u) == 0  ? bn_gate_bwd_lanes_kernel<PASS, 4, 4, QL>
+             : (p.c & 1) == 0 && (at & 7u) == 0 ? bn_gate_bwd_lanes_kernel<PASS, 2, 4, QL>
+                                                : bn_gate_bwd_lanes_kernel<PASS, 1, 4, QL>;
+  launch_ready(kernel, dim3(blocks), dim3(256), smem, st, p, lanes, ks, ka, kg, gx, part_a, part_g);
   note_launches(1);
 }
 
@@ -1105,7 +1109,7 @@ static int launch_bwd(BnGateBwd p, const float *ks, const float *ka, const float
   p.chains = 8 * bn_row_blocks(p.n);
   int lanes = 1;
   while (lanes < 32 && lanes * 4 < p.c_out) lanes <<= 1;
-  if ((p.c_out & 3) == 0 && p.c_out <= 256 && p.n_gates <= 2 * lanes && ((uintptr_t)p.go & 15u) == 0) {
+  if ((p.c_out & 3) == 0 && p.c_out <= 256 && p.n_gates <= 2 * lanes) {
     if (p.c_out <= 128 && p.n_gates <= lanes) launch_bwd_lanes<PASS, 1>(p, lanes, ks, ka, kg, gx, part_a, part_g, st);
     else launch_bwd_lanes<PASS, 2>(p, lanes, ks, ka, kg, gx, part_a, part_g, st);
     SSC_CHECK_LAUNCH("bn_gate_bwd");

@@ -571,6 +571,33 @@ def test_norm_and_gate_gradients_at_tile_edges(cuda, Rs, n, training):
         assert float((got.cpu().double() - want).abs().max()) <= 1e-4 * max(float(want.abs().max()), 1.0)
 
 
+@pytest.mark.parametrize("Rs,n", [([(1, 0), (1, 1)], 9), ([(2, 0), (2, 1), (2, 2), (2, 3)], 4999), ([(8, 0), (8, 1), (8, 2)], 700), ([(16, 0), (16, 1), (16, 2)], 513),
+                                  ([(3, 0), (3, 1), (1, 2)], 300)])
+@pytest.mark.parametrize("alone", [False, True])
+def test_norm_gradients_do_not_depend_on_where_rows_lie(cuda, Rs, n, alone):
+    """Rows and gradients at offsets of one, two and three floats: the same bits as on 16-byte boundaries."""
+    from ss_conv import _ext
+    from ss_conv.activation import Activation
+    from ss_conv.batchnorm import BatchNorm
+    torch.manual_seed(n)
+    n_gates = 0 if alone else sum(m for m, l in Rs if l > 0)
+    bn = BatchNorm(Rs + ([(n_gates, 0)] if n_gates else [])).to(cuda)
+    gate = None if alone else Activation(Rs, (torch.relu, torch.sigmoid), bias=False, checkpoint=False).gate_tables(cuda)
+    field, scalar = bn._device_tables(cuda)
+    sizes, w = (bn.running_var.numel(), bn.running_mean.numel()), bn.weight.detach()
+    c_out = sum(m * (2 * l + 1) for m, l in Rs)
+    x, g = torch.randn(n, c_out + n_gates, device=cuda) + 0.2, torch.randn(n, c_out, device=cuda)
+    _, var, mean, scale, shift = _ext.bn_train(x, field, scalar, *sizes, w, None, 1e-5, 0.1)
+
+    def shifted(t, by):
+        return torch.empty(t.numel() + by, device=cuda)[by:].view_as(t).copy_(t)
+
+    want = _ext.bn_gate_backward(x, g, field, scalar, *sizes, scale, shift, mean, var, w, 1e-5, True, gate)
+    for dx, dg in ((0, 1), (0, 2), (1, 0), (2, 3), (1, 1)):
+        got = _ext.bn_gate_backward(shifted(x, dx), shifted(g, dg), field, scalar, *sizes, scale, shift, mean, var, w, 1e-5, True, gate)
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), (dx, dg)
+
+
 @pytest.mark.parametrize("batch,grid,per", [(1, 3, 5), (1, 16, 300), (3, 17, 900), (8, 32, 700), (2, 64, 3000), (40, 32, 400)])
 def test_rulebook_in_one_go_equals_the_two_phases(cuda, batch, grid, per):
     """Bitmaps of one word, around the 128 words of a block, at the most words of the one-launch form and above, with
