@@ -620,7 +620,7 @@ bn_gate_bwd_kernel(BnGateBwd p, const float *__restrict__ ks, const float *__res
 // rows, then a block's warps in order; a block is one chain of the totals.  The form above hands every element through shared memory
 // and adds up a channel per thread, 32 rows at a time, while the other threads wait: 162 k rows of 32 + 6 channels 47 + 33 us, here
 // 19 + 16; 93 k rows of 64 + 12 30 + 25, here 18 + 16 (the bytes of the two passes take 8 and 12).  A gate's sum takes fields of up
-// to seven channels at once: as a loop it was half of the kernel.  Wider rows and others than fours stay above.
+// to seven channels at once: as a loop it was half of the kernel.  Wider rows, others than fours and some of many rows (launch_bwd) stay above.
 template <int VEC>
 __device__ __forceinline__ void row_quad(const float *at, float (&v)[4]) {
   if (VEC == 4) {
@@ -1109,7 +1109,12 @@ static int launch_bwd(BnGateBwd p, const float *ks, const float *ka, const float
   p.chains = 8 * bn_row_blocks(p.n);
   int lanes = 1;
   while (lanes < 32 && lanes * 4 < p.c_out) lanes <<= 1;
-  if ((p.c_out & 3) == 0 && p.c_out <= 256 && p.n_gates <= 2 * lanes) {
+  // Of many rows of which two fifths of the lanes have no channels the other form is the faster one where its copies are of 16 bytes and
+  // little else is to do: 132 to 152 normed channels without gates (144: 60 k rows 63.6 and 61.4 us here, 100 k
+  // 97.9 and 105.6, 600 k 518 and 565), the gate's gradient alone of 68 and 72 (72 + 16: 100 k rows 36.3 and 38.4, 600 k 205 and 222).
+  const bool idle = p.n > 65536 && p.c_out * 5 < lanes * (p.c_out <= 128 ? 12 : 24) && (p.c & 3) == 0;
+  const bool wide = p.c_out > 128 ? p.n_gates == 0 : PASS == 1 && ks == nullptr && p.c_out > 64;
+  if ((p.c_out & 3) == 0 && p.c_out <= 256 && p.n_gates <= 2 * lanes && !(idle && wide)) {
     if (p.c_out <= 128 && p.n_gates <= lanes) launch_bwd_lanes<PASS, 1>(p, lanes, ks, ka, kg, gx, part_a, part_g, st);
     else launch_bwd_lanes<PASS, 2>(p, lanes, ks, ka, kg, gx, part_a, part_g, st);
     SSC_CHECK_LAUNCH("bn_gate_bwd");

@@ -539,7 +539,7 @@ def test_points_outside_the_grid_are_dropped_as_the_torch_steps_do(cuda, n, batc
 @pytest.mark.parametrize("Rs,n", [([(1, 0)], 1), ([(2, 0), (3, 1)], 9), ([(4, 0), (4, 1), (4, 2), (4, 3)], 520), ([(2, 0), (2, 1), (2, 2), (2, 3)], 4999),
                                   ([(40, 0), (40, 1)], 70), ([(300, 0), (200, 1)], 33),
                                   ([(1, 0), (1, 1)], 700), ([(1, 0), (1, 1), (1, 2), (1, 3)], 8193), ([(8, 0), (40, 1)], 4097), ([(4, 0), (4, 4)], 1000),
-                                  ([(16, 0), (16, 1), (16, 2), (16, 3)], 513), ([(3, 0), (3, 1)], 65)])
+                                  ([(16, 0), (16, 1), (16, 2), (16, 3)], 513), ([(3, 0), (3, 1)], 65), ([(132, 0)], 65536), ([(152, 0)], 65537)])
 @pytest.mark.parametrize("training", [True, False])
 def test_norm_and_gate_gradients_at_tile_edges(cuda, Rs, n, training):
     """One row and a few more than a tile, channels that are odd, even and multiples of four, no gates, more gates than
