@@ -155,8 +155,10 @@ static __device__ __forceinline__ void post_count(const CountPost &post, int32_t
 // in it, and the instruction itself is dear where a block does little (us without it, with it, and of an ordinary launch:
 // gradients of 10 k rows of 250 normed channels 35.4, 46.5, 36.2; max pool over 27 offsets, 20 k rows of 76 15.7, 20.8, 16.0;
 // filter gradient of 300 rows 32 -> 38 12.6, 16.3, 14.2; transpose of a table of 27 offsets, 700 k rows 29.6, 54.8, 29.6).
-template <class... P, class... A>
-inline cudaError_t launch_ready(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+template <class T>
+struct AsIs { using type = T; };      // (keeps a parameter out of the deduction: arguments convert to the kernel's types as in a call)
+template <class... P>
+inline cudaError_t launch_ready(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, typename AsIs<P>::type... args) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -167,7 +169,7 @@ inline cudaError_t launch_ready(void (*kernel)(P...), dim3 grid, dim3 block, siz
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -395,3 +395,19 @@ def test_few_pairs_keep_few_partial_filter_gradients(c_in, c_out, line):
     from ss_conv._ext import lib
     few, many = (lib().ssc_conv_wgrad_scratch_bytes(27, c_in, c_out, n) - lib().ssc_conv_pairs_list_bytes(27, n) for n in (line - 1, line))
     assert few < 0.75 * many
+
+
+@pytest.mark.parametrize("argument,accepted", [("const float *", True), ("float *", True), ("const double *", False), ("const int32_t *", False)])
+def test_launches_check_the_types_of_their_arguments(tmp_path, argument, accepted):
+    """launch_ready takes what a call of the kernel would: a pointer may gain a const, not become one of another type."""
+    import subprocess
+    source = tmp_path / "launch.cu"
+    source.write_text("""#include "ssc_common.cuh"
+__global__ void kernel(const float *x, int n, float *y) { ssc::after_previous(); }
+cudaError_t run(%s x, float *y) { return ssc::launch_ready(kernel, dim3(1), dim3(32), 0, nullptr, x, 3, y); }
+""" % argument)
+    nvcc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "bin", "nvcc")
+    made = subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", os.path.join(ROOT, "ss-conv_b200", "csrc"), "-I", os.path.join(ROOT, "include"),
+                           "-c", str(source), "-o", str(tmp_path / "launch.o")], capture_output=True, text=True, timeout=300)
+    assert (made.returncode == 0) == accepted, made.stderr
+    assert accepted or "launch_ready" in made.stderr, made.stderr
