@@ -103,11 +103,12 @@ __device__ __forceinline__ bool mbar_wait_uniform(uint32_t bar, uint32_t parity,
   return false;
 }
 // The same for a loop without a way out in the middle, which costs the issuing warp more than the wait itself: after a wait has
-// failed the next ones look once and fail too.
+// failed the next ones look once, and fail too unless the barrier is ready.  What a loop still copies until its end goes to slots that nobody
+// reads any more and is waited for, like all copies, before the CTA leaves.
 __device__ __forceinline__ bool mbar_wait_straight(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
   uint32_t i = 0;
   bool ok;
-  do { ok = __all_sync(0xffffffffu, mbar_try_wait(bar, parity)); } while (!ok && ++i < kSpinLimit && ((i & 255u) != 255u || !__any_sync(0xffffffffu, *abort_flag)));
+  do { ok = __all_sync(0xffffffffu, mbar_try_wait(bar, parity)); } while (!ok && ++i < kSpinLimit && !__any_sync(0xffffffffu, *abort_flag));
   if (!ok) *abort_flag = 1;
   return ok;
 }
@@ -135,7 +136,7 @@ __device__ __forceinline__ bool mbar_wait_straight_cluster(uint32_t bar, uint32_
         : "r"(bar), "r"(parity)
         : "memory");
     ok = __all_sync(0xffffffffu, got != 0);
-  } while (!ok && ++i < kSpinLimit && ((i & 255u) != 255u || !__any_sync(0xffffffffu, *abort_flag)));
+  } while (!ok && ++i < kSpinLimit && !__any_sync(0xffffffffu, *abort_flag));
   if (!ok) *abort_flag = 1;
   return ok;
 }
