@@ -225,7 +225,7 @@ pl_prepare_kernel(const int32_t *__restrict__ starts, int K, int n_split, int ti
 
 // A lane's piece of two rows (none of a negative one), OFF bytes into its part of the slot.
 template <int OFF>
-__device__ __forceinline__ void copy_rows(int a, int b, uint32_t dst0, uint32_t dst1, const char *base, uint32_t stride, uint32_t bytes) {
+__device__ __forceinline__ void copy_two_rows(int a, int b, uint32_t dst0, uint32_t dst1, const char *base, uint32_t stride, uint32_t bytes) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t.reg .b64 s, t;\n\tsetp.ge.s32 p, %0, 0;\n\tsetp.ge.s32 q, %1, 0;\n\t"
       "mad.wide.u32 s, %0, %5, %4;\n\tmad.wide.u32 t, %1, %5, %4;\n\t"
@@ -349,10 +349,10 @@ conv_fwd_pairs_body(const float *__restrict__ staged, const uint4 *__restrict__ 
           alive = mbar_wait_straight(empty0 + (uint32_t)slot * 8u, par, abort_flag);
           if (PAIR && rank == 0 && warp == 0 && elect_one()) mbar_expect_tx(full, 16u);
           const uint32_t dst0 = first0 + slot_off, dst1 = first1 + slot_off;
-          copy_rows<0>(from[0], from[1], dst0, dst1, base, stride, bytes);
-          copy_rows<1024>(from[2], from[3], dst0, dst1, base, stride, bytes);
-          copy_rows<2048>(from[4], from[5], dst0, dst1, base, stride, bytes);
-          copy_rows<3072>(from[6], from[7], dst0, dst1, base, stride, bytes);
+          copy_two_rows<0>(from[0], from[1], dst0, dst1, base, stride, bytes);
+          copy_two_rows<1024>(from[2], from[3], dst0, dst1, base, stride, bytes);
+          copy_two_rows<2048>(from[4], from[5], dst0, dst1, base, stride, bytes);
+          copy_two_rows<3072>(from[6], from[7], dst0, dst1, base, stride, bytes);
           asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
           if (++slot == S) { slot = 0; par ^= 1u; }
         }

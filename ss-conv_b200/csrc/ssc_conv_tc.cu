@@ -49,11 +49,11 @@ struct TcParams {
   int fmt16;      // 16-bit operands: 0 = fp16, 1 = bf16 (operand format field of the instruction descriptor)
   int last_kk;    // MMA k-steps (32 bytes of K each) that hold real channels in the LAST slab: 1..4
   int opk;        // kernel offsets per 128-byte operand row: 1, or 32 / c_pad for TF32 layers with c_pad = 4, 8, 16
+                  // channels (a first layer with 3 input channels packs 8 offsets into one step)
   int rev;        // 1: the table's row of kernel offset kappa is K - 1 - kappa (the transpose of a centred submanifold table)
   int32_t *alarm; // mapped host word that tells of an expired wait (may be NULL)
   int pair;       // 1: two CTAs with 128 rows each share the filter slabs (half a slab in each) and the products
   int nbr_by_pos; // 1: the table's columns are already in the order of `order` (column j <-> output row order[j])
-                  // channels (a first layer with 3 input channels packs 8 offsets into one step)
 };
 
 // Shared-memory plan: [stages x (A 16 KB + B)] [control 1 KB].
@@ -704,8 +704,8 @@ conv_fwd_rows(const float *__restrict__ features, int row_words, const uint4 *__
     if (tid == 32) {
       for (int s = 0; s < S; ++s) {
         mbar_init(smem_u32(empty_bars + s), 1);
-        // 128 arrivals by copies, one per warp for the row mask, one for the filter copy's byte count; in the
-        // issuing CTA of a pair one that tells of all these in the other
+        // 128 arrivals by copies, one per warp for the row mask, one for the filter copy's byte count, which in the
+        // issuing CTA of a pair has 16 bytes more, of the store that tells of all these in the other
         mbar_init(smem_u32(full_bars + s), 128 + 4 + 1);
       }
       mbar_init(smem_u32(&done_bar), 1);
@@ -973,12 +973,12 @@ conv_fwd_rows_kernel(const float *__restrict__ features, int row_words, const ui
                      const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order, const __grid_constant__ GateEpilogue gate) {
   conv_fwd_rows<F16, GATED, GROUPS, false>(features, row_words, packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
 }
-template <bool F16, bool GATED, int GROUPS>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GROUPS * 128 + 32, GROUPS == 1 ? 4 : 2)
+template <bool F16, bool GATED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(2 * 128 + 32, 2)
 conv_fwd_pair_rows_kernel(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
                           const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out, int32_t *status, const __grid_constant__ TcParams p,
                           const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order, const __grid_constant__ GateEpilogue gate) {
-  conv_fwd_rows<F16, GATED, GROUPS, true>(features, row_words, packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
+  conv_fwd_rows<F16, GATED, 2, true>(features, row_words, packed, K, c_out, nbr, n_out, out, status, p, n_out_dev, order, gate);
 }
 
 static size_t tc_smem_bytes(const TcParams &p) {
@@ -1043,16 +1043,13 @@ static bool rows_params(int words, int c_out, int n_out, TcParams &p, int opk = 
 // Producer groups.  Three or four CTAs on an SM have producers enough between them, and a second group in each would leave
 // its threads 56 registers, which costs more instructions than it brings; one or two CTAs need both (64 -> 76
 // channels, four CTAs: 95 us with two groups, 88 with one; 128 -> 152 bf16 channels, two CTAs: 77 and 83).
-static int rows_groups(const TcParams &p) { return p.ctas > 2 ? 1 : 2; }
+static int rows_groups(const TcParams &p) { return p.ctas > 2 && !p.pair ? 1 : 2; }     // (pairs have two CTAs on an SM at most)
 
 using RowsKernel = void (*)(const float *, int, const uint4 *, int, int, const int32_t *, int, float *, int32_t *, TcParams, const int32_t *,
                             const int32_t *, GateEpilogue);
 template <bool F16>
 static RowsKernel rows_kernel(const TcParams &p, bool gated) {
-  if (p.pair) {
-    if (rows_groups(p) == 1) return gated ? conv_fwd_pair_rows_kernel<F16, true, 1> : conv_fwd_pair_rows_kernel<F16, false, 1>;
-    return gated ? conv_fwd_pair_rows_kernel<F16, true, 2> : conv_fwd_pair_rows_kernel<F16, false, 2>;
-  }
+  if (p.pair) return gated ? conv_fwd_pair_rows_kernel<F16, true> : conv_fwd_pair_rows_kernel<F16, false>;
   if (rows_groups(p) == 1) return gated ? conv_fwd_rows_kernel<F16, true, 1> : conv_fwd_rows_kernel<F16, false, 1>;
   return gated ? conv_fwd_rows_kernel<F16, true, 2> : conv_fwd_rows_kernel<F16, false, 2>;
 }
