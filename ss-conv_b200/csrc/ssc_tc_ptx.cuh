@@ -100,8 +100,18 @@ __device__ __forceinline__ bool mbar_wait_straight(uint32_t bar, uint32_t parity
   if (!ok) *abort_flag = 1;
   return ok;
 }
-// Pairs of CTAs (a cluster of two): the address of the same place in CTA `rank`'s shared memory, stores and arrivals there, and
-// the wait that sees them (mbar_wait_straight at cluster scope).
+// Pairs of CTAs (a cluster of two): the address of the same place in CTA `rank`'s shared memory, the store that tells the other CTA
+// something, and the wait that sees it (mbar_wait_straight at cluster scope).
+//
+// Why what the second CTA tells of is visible to the tensor core that the first one's issuing warp starts.  The rows of a slot
+// are other warps' copies (cp.async) and a bulk copy of filters; all of them count on the slot's barrier in the second CTA
+// when they have landed.  One warp there waits for that barrier, which orders them before what it does next, and then orders them
+// for the async proxy (fence_async_smem).  Behind both, in program order, it issues st_async_v4: its 16 bytes count on the
+// first CTA's barrier, and that completion is a release at cluster scope (PTX ISA, st.async).  The issuing warp's wait on that barrier acquires at cluster
+// scope, and causality passes through a release and an acquire to everything the releasing side had seen, by whatever
+// thread it was done.  tcgen05.fence::after_thread_sync then stands between that wait and the products, which read both CTAs' slots.  Accumulators
+// go the same way: tcgen05.ld, tcgen05.wait::ld, tcgen05.fence::before_thread_sync, the warp's lanes together, the store.
+// (A store and a released remote arrival say the same in two operations, at 2100 cycles a step.)
 __device__ __forceinline__ uint32_t peer_address(uint32_t addr, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
