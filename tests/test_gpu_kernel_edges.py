@@ -727,7 +727,7 @@ def test_filter_gradient_on_either_side_of_a_product(cuda, c_in, c_out, n):
     assert rel_err(got.cpu().numpy(), want) < 1e-3
 
 
-@pytest.mark.parametrize("c_in,c_out,n", [(16, 8, 1), (18, 22, 130), (64, 76, 400)])
+@pytest.mark.parametrize("c_in,c_out,n", [(16, 8, 1), (18, 22, 130), (64, 76, 400), (66, 154, 4097), (18, 257, 4200), (128, 130, 300), (30, 178, 16400)])
 def test_filter_gradient_of_staged_operands(cuda, c_in, c_out, n):
     """Operands that are rounded and padded already (the flags of ssc_conv_wgrad_lists, alone and together) give the bits of
     those that the kernel rounds itself."""
@@ -747,11 +747,30 @@ def test_filter_gradient_of_staged_operands(cuda, c_in, c_out, n):
     _ext.check_status(cuda)
 
 
+@pytest.mark.parametrize("n_in,n_out", [(300, 300), (300, 4500), (700, 300)])
+@pytest.mark.parametrize("c_in,c_out", [(38, 22), (66, 154)])
+def test_filter_gradient_with_input_rows_rounded_up_front(cuda, monkeypatch, n_in, n_out, c_in, c_out):
+    """Input rows from WGRAD_STAGE_ELEMENTS on are rounded before the kernel, not where there are more of them than output rows: on both
+    sides of that line the bits of the kernel that rounds them itself."""
+    from ss_conv import _ext
+    rng = np.random.RandomState(n_out)
+    t = dev(_table(n_out, n_in, 27, 0.3, rng), cuda)
+    x, g = torch.randn(n_in, c_in, device=cuda), torch.randn(n_out, c_out, device=cuda)
+    image, staged, stage = _ext.stage_tf32(g), [], _ext.stage_tf32
+    monkeypatch.setattr(_ext, "stage_tf32", lambda rows: (staged.append(rows), stage(rows))[1])
+    want = _ext.conv_wgrad(x, g, t, "tf32")
+    for line, expected in ((x.numel() + 1, 0), (x.numel(), 1 if n_in <= n_out else 0)):
+        monkeypatch.setattr(_ext, "WGRAD_STAGE_ELEMENTS", line)
+        staged.clear()
+        assert torch.equal(_ext.conv_wgrad(x, g, t, "tf32", dy_image=image), want) and len(staged) == expected
+    _ext.check_status(cuda)
+
+
 @pytest.mark.parametrize("n,channels", [(90, 12), (900, 24)])
 def test_kernels_queued_behind_one_another(cuda, monkeypatch, n, channels):
-    """A training step over one set of rows after another, all queued while the device is busy, gives the gradients of the
-    same calls with the device idle between any two.  Every call writes buffers that the step before has just read, so a
-    kernel that started on unfinished rows would be off by the size of the values.  Sums that are added up in another
+    """Training steps over one set of rows after another, without a wait of the caller's between the calls, give the gradients of the
+    same calls with the device idle between any two.  (The strided layer and the pool wait for their row counts themselves; chains of
+    which no call waits are the next test's.)  Sums that are added up in another
     order can move an operand by one step of TF32, 2^-11 of it, in each of the four convolutions of the two directions."""
     from ss_conv import _ext
     from ss_conv.activation import Activation
@@ -793,6 +812,87 @@ def test_kernels_queued_behind_one_another(cuda, monkeypatch, n, channels):
         assert len(got) == len(want) > 6
         for a, b in zip(got, want):
             assert rel_err(a, b) < 4 * 2.0 ** -11
+
+
+@pytest.mark.parametrize("n,recorded", [(3000, False), (20000, False), (20000, True)])
+def test_chains_without_a_wait_have_the_bits_of_single_calls(cuda, monkeypatch, n, recorded):
+    """Convolution, batch statistics, norm and gate, pool and all their gradients, each call on what the one before has just written,
+    over other rows every time in the same buffers: queued behind a busy device, or replayed from a graph, without any wait of the host.  The same
+    bits as with the device idle between any two calls: a kernel that read before its turn would find the rows of the time before.  The
+    pair-list kernel adds in any order: its rows within 5e-5 of the largest, as where it is compared with the other form."""
+    from ss_conv import _ext
+    from ss_conv.activation import Activation
+    from ss_conv.batchnorm import BatchNorm
+    torch.manual_seed(n)
+    g = torch.Generator(cuda).manual_seed(n)
+    n_down, fields, gated = n // 3, [(16, 0), (16, 1), (8, 2)], [(16, 0), (16, 1), (8, 2), (24, 0)]
+    c, c_all = 104, 128
+
+    def table(rows, of, K, present):
+        t = torch.randint(0, of, (K, rows), generator=g, device=cuda)
+        return torch.where(torch.rand(K, rows, generator=g, device=cuda) < present, t, -1).to(torch.int32)
+
+    same, down, pool = table(n, n, 27, .3), table(n_down, n, 27, .25), table(n_down, n_down, 8, .5)
+    w1, w2, w3 = (torch.randn(27, a, b, generator=g, device=cuda) * .05 for a, b in ((c, c_all), (c, c_all), (c_all, c_all)))
+    bn, act = BatchNorm(gated).to(cuda), Activation(fields, (torch.relu, torch.sigmoid), bias=False, checkpoint=False).to(cuda)
+    (field, scalar), gate, w = bn._device_tables(cuda), act.gate_tables(cuda), bn.weight.detach()
+    sizes = (bn.running_var.numel(), bn.running_mean.numel())
+    inputs = [torch.randn(n, c, generator=g, device=cuda) for _ in range(5)]
+    x = torch.empty(n, c, device=cuda)
+    order = torch.argsort((same >= 0).int().argmax(0)).to(torch.int32)
+
+    def layer(rows, filters, nbr):
+        y = _ext.conv_forward(rows, filters, nbr, nbr.shape[1], "tf32", algo="rows")
+        _, var, mean, scale, shift = _ext.bn_train(y, field, scalar, *sizes, w, None, 1e-5, 0.1)
+        return y, (scale, shift, mean, var), _ext.bn_gate_forward(y, scale, shift, gate[0], c, c, gate[3], gate[4], None, None)
+
+    def back(rows, filters, nbr, y, stats, grad):
+        gy, d_w, d_b = _ext.bn_gate_backward(y, grad, field, scalar, *sizes, *stats, w, 1e-5, True, gate)
+        return (d_w, d_b) + tuple(_ext.conv_backward(rows, filters, gy, nbr, precision="tf32"))
+
+    def chain():
+        y1, s1, z1 = layer(x, w1, same)
+        y2, s2, z2 = layer(z1, w2, down)
+        top = torch.empty(n_down, c, device=cuda)
+        _ext._check(_ext.lib().ssc_maxpool_fwd(_ext._p(z2), c, _ext._p(pool), 8, n_down, _ext._p(top), None, _ext._stream()))
+        d2 = back(z1, w2, down, y2, s2, top)
+        d1 = back(x, w1, same, y1, s1, d2[2])
+        ordered = _ext.conv_forward(d1[2], w1, same, n, "bf16", algo="rows", row_order=order)
+        return [_ext.conv_forward(ordered, w3, same, n, "tf32", algo="pairs"), y1, z1, z2, top, ordered, *d2, *d1]
+
+    def warm():
+        with torch.cuda.stream(side):
+            x.copy_(inputs[0])
+            chain()
+        torch.cuda.synchronize()
+
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    warm()
+    if recorded:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            kept = chain()
+    out = []
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)
+        for rows in inputs:
+            x.copy_(rows)
+            if recorded:
+                graph.replay()
+                out.append([t.clone() for t in kept])
+            else:
+                out.append(chain())
+        assert not side.query()                  # everything was queued before the device was through
+    torch.cuda.synchronize()
+    check = _ext._check
+    monkeypatch.setattr(_ext, "_check", lambda rc: (check(rc), torch.cuda.synchronize()))
+    for rows, got in zip(inputs, out):
+        x.copy_(rows)
+        want = chain()
+        assert rel_err(got[0].cpu(), want[0].cpu()) <= 5e-5
+        assert all(torch.equal(a, b) for a, b in zip(got[1:], want[1:]))
+    _ext.check_status(cuda)
 
 
 def test_transposing_a_table_costs_little_more_than_a_copy(cuda):
