@@ -503,6 +503,46 @@ def test_gated_convolution_at_the_ends_of_the_activations(cuda, scalar_act):
     assert torch.equal(got.view(torch.int32), want.view(torch.int32))
 
 
+def test_quick_sigmoids_have_the_bits_of_the_functions(cuda, tmp_path):
+    """Every denominator from 1 to 2^125 through the quick reciprocal and every fp32 argument through the sigmoids side by side."""
+    import ctypes
+    import os
+    import subprocess
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    source = tmp_path / "sweep.cu"
+    source.write_text("""#include "ssc_act.cuh"
+__device__ __forceinline__ bool same(float a, float b) { return __float_as_uint(a) == __float_as_uint(b) || (a != a && b != b); }
+__global__ void sweep(unsigned long long *differ) {
+  const unsigned long long first = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x, step = (unsigned long long)gridDim.x * blockDim.x;
+  const unsigned one = 0x3f800000u, top = 0x7e000000u;     // 1 and 2^125
+  unsigned long long a = 0, b = 0;
+  for (unsigned long long i = first; i <= top - one; i += step) {
+    const float d = __uint_as_float(one + (unsigned)i);
+    a += same(ssc::quick_reciprocal(d), __frcp_rn(d)) ? 0 : 1;
+  }
+  for (unsigned long long i = first; i < 1ull << 31; i += step) {
+    float v[2] = {__uint_as_float((unsigned)i), __uint_as_float((unsigned)i | 0x80000000u)};
+    const float w[2] = {ssc::apply_act(v[0], 2), ssc::apply_act(v[1], 2)};
+    ssc::apply_sigmoids<2>(v);
+    b += (same(v[0], w[0]) ? 0 : 1) + (same(v[1], w[1]) ? 0 : 1);
+  }
+  if (a) atomicAdd(differ, a);
+  if (b) atomicAdd(differ + 1, b);
+}
+extern "C" int run(unsigned long long *differ) {
+  sweep<<<148 * 8, 256>>>(differ);
+  return (int)cudaDeviceSynchronize();
+}
+""")
+    nvcc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "bin", "nvcc")
+    subprocess.run([nvcc, "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC", "-shared", "-I", os.path.join(root, "ss-conv_b200", "csrc"),
+                    str(source), "-o", str(tmp_path / "sweep.so")], check=True, timeout=300)
+    differ = torch.zeros(2, dtype=torch.int64, device=cuda)
+    torch.cuda.synchronize()
+    assert ctypes.CDLL(str(tmp_path / "sweep.so")).run(ctypes.c_void_p(differ.data_ptr())) == 0
+    assert differ.tolist() == [0, 0]
+
+
 @pytest.mark.parametrize("n,batch", [(0, 1), (1, 3), (1025, 1024), (16384, 4096), (16385, 7), (300, 4097)])
 def test_batch_offsets_at_the_sizes_of_the_one_block_form(cuda, n, batch):
     """Rows in any order, samples without rows, ids outside the batch (counted nowhere): a plain histogram's prefix."""
