@@ -896,11 +896,15 @@ TABLE_IN_ORDER = 0x200
 TABLE_REVERSED = 0x1000
 WGRAD_X_STAGED = 0x400
 WGRAD_DY_STAGED = 0x800
-# Input rows are read once per neighbour by the filter gradient: from here on they are rounded once, up front, instead of after every read (93 k
-# rows of 64 -> 76: 89 us, 64 + 5 rounded before; 162 k of 32 -> 38: 74, 64 + 4; 65 k of 16 -> 38: 12, 11 + 3).  Not where there are
-# more input rows than output rows: a stride of two reads a row three or four times instead of ten (both gradients of 240 k ->
-# 129 k rows, 64 -> 76, in a graph: 177 us rounded before, 172 after every read).
+# The filter gradient reads an input row once for each output row that uses it: images of between so many elements are rounded once, up
+# front, instead of after every read.  That pays from about four reads a row on, which the pairs would tell and the host does not
+# know; rows do: a stride of two reads a row three or four times, hence not where there are more input rows than output rows.
+# With 9 neighbours a row, rounded after every read and before: 93 k rows of 64 -> 76 66.1 and 58.5 us, 162 k of 32 -> 38
+# 72.1 and 69.6, 162 k of 16 -> 38 70.3 and 65.4.  Tables of two neighbours a row lose by it (36.7 and 44.4, 24.4 and 28.1, 23.6 and 25.0),
+# the more where the image (four bytes an element, held until the gradient is there) does not fit L2: 162 k of 256 -> 128 93 and 130, hence the upper end.  Rows of
+# no whole fours are read a float at a time and always gain: 93 k of 38 -> 32, 1.5 and 9 neighbours, 24.8 and 21.9, 87.1 and 47.0.
 WGRAD_STAGE_ELEMENTS = 1 << 21
+WGRAD_STAGE_ELEMENTS_MOST = 1 << 25
 # (features.data_ptr(), filters.data_ptr()) -> (prec, packed, scratch, nbytes) left by conv_prepare for the
 # conv_forward call that follows on the same tensors
 _prepared = {}
@@ -1236,7 +1240,8 @@ def conv_wgrad(features, out_grad, nbr, precision=None, dy_image=None):
     x, dy = _p(features, torch.float32), _p(out_grad, torch.float32)
     if mode == PREC_TF32 and c_in <= 256 and K <= 256 and dy_image is not None:
         dy, mode = _p(dy_image), mode | WGRAD_DY_STAGED
-        if features.numel() >= WGRAD_STAGE_ELEMENTS and features.shape[0] <= n_out:
+        if features.shape[0] <= n_out and features.numel() >= WGRAD_STAGE_ELEMENTS and (
+                c_in % 4 != 0 or features.numel() <= WGRAD_STAGE_ELEMENTS_MOST):
             x_image = stage_tf32(features)
             x, mode = _p(x_image), mode | WGRAD_X_STAGED
     _check(lib().ssc_conv_wgrad_lists(x, c_in, dy, c_out, _p(nbr, torch.int32), K, n_out, _p(lists),

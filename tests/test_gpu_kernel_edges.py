@@ -788,10 +788,11 @@ def test_filter_gradient_of_staged_operands(cuda, c_in, c_out, n):
 
 
 @pytest.mark.parametrize("n_in,n_out", [(300, 300), (300, 4500), (700, 300)])
-@pytest.mark.parametrize("c_in,c_out", [(38, 22), (66, 154)])
+@pytest.mark.parametrize("c_in,c_out", [(38, 22), (66, 154), (40, 22)])
 def test_filter_gradient_with_input_rows_rounded_up_front(cuda, monkeypatch, n_in, n_out, c_in, c_out):
-    """Input rows from WGRAD_STAGE_ELEMENTS on are rounded before the kernel, not where there are more of them than output rows: on both
-    sides of that line the bits of the kernel that rounds them itself."""
+    """Input rows from WGRAD_STAGE_ELEMENTS to WGRAD_STAGE_ELEMENTS_MOST, without an end where their channels are no multiple of four, are
+    rounded before the kernel, not where there are more of them than output rows: on both sides of those lines the bits of the kernel that
+    rounds them itself."""
     from ss_conv import _ext
     rng = np.random.RandomState(n_out)
     t = dev(_table(n_out, n_in, 27, 0.3, rng), cuda)
@@ -799,10 +800,12 @@ def test_filter_gradient_with_input_rows_rounded_up_front(cuda, monkeypatch, n_i
     image, staged, stage = _ext.stage_tf32(g), [], _ext.stage_tf32
     monkeypatch.setattr(_ext, "stage_tf32", lambda rows: (staged.append(rows), stage(rows))[1])
     want = _ext.conv_wgrad(x, g, t, "tf32")
-    for line, expected in ((x.numel() + 1, 0), (x.numel(), 1 if n_in <= n_out else 0)):
-        monkeypatch.setattr(_ext, "WGRAD_STAGE_ELEMENTS", line)
+    for least, most, expected in ((1, 0, 0), (0, 0, 1), (0, -1, c_in % 4)):
+        monkeypatch.setattr(_ext, "WGRAD_STAGE_ELEMENTS", x.numel() + least)
+        monkeypatch.setattr(_ext, "WGRAD_STAGE_ELEMENTS_MOST", x.numel() + most)
         staged.clear()
-        assert torch.equal(_ext.conv_wgrad(x, g, t, "tf32", dy_image=image), want) and len(staged) == expected
+        assert torch.equal(_ext.conv_wgrad(x, g, t, "tf32", dy_image=image), want)
+        assert len(staged) == (1 if expected and n_in <= n_out else 0)
     _ext.check_status(cuda)
 
 
