@@ -943,6 +943,11 @@ def rulebook_next_to_features(rows, build):
         out = build()
         after.record(rb)
     cur.wait_stream(rb)
+    if out is not None:
+        # Kernels on the current stream read these, and the next rulebook on the side stream waits for none of them: what is freed
+        # here must not be handed out there while the graph is being recorded.
+        for t in (out[0], out[1]._nbr_cap, out[1]._n_out_dev):
+            t.record_stream(cur)
     return out, after
 
 

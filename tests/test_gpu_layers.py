@@ -364,6 +364,61 @@ def test_graphed_chain_replays_match_eager_results(cuda):
         _ext.set_precision("auto")
 
 
+@pytest.mark.parametrize("batch,grid,per", [(19, 33, 926), (3, 38, 851), (5, 40, 900), (2, 17, 300)])
+@pytest.mark.parametrize("pool", [False, True])
+def test_recorded_rulebooks_keep_their_memory_from_one_another(cuda, monkeypatch, batch, grid, per, pool):
+    """Rulebooks of a recorded chain are built on a stream of their own, ahead of the kernels that read the ones before: none may get
+    memory of one that is still to be read, whatever the sizes (the table of a layer fits the next one's place or not).  Every replay
+    of every input gives what the layers give one by one."""
+    from ss_conv import _ext
+    from ss_conv.activation import Activation
+    from ss_conv.batchnorm import BatchNorm
+    from ss_conv.convolution import Convolution
+    from ss_conv.graph import GraphedPoints
+    from ss_conv.pool import GlobalAvgPool, MaxPool
+    from ss_conv.sp_ops.voxelize import Point2Voxel
+    torch.manual_seed(batch)
+    widths, layers = (3, 8, 16, 24, 32), []
+    for a, b in zip(widths[:-1], widths[1:]):
+        gated = [(b // 4, 0), (b // 4, 1), (b // 4, 0)]
+        rs_in = [(3, 0)] if a == 3 else [(a // 4, 0), (a // 4, 1)]
+        layers += [Convolution(rs_in, gated, 3, stride=2, padding=1), BatchNorm(gated), Activation(gated[:2], (torch.relu, torch.sigmoid), bias=False, checkpoint=False)]
+        if pool:
+            layers += [MaxPool(3, stride=1, padding=1)]
+    net = torch.nn.Sequential(*layers, GlobalAvgPool()).to(cuda).eval()
+    p2v = Point2Voxel([grid] * 3, [1.0 / grid] * 3, 4, trusted_batch_size=batch)
+    ids = torch.arange(batch, device=cuda, dtype=torch.int32).repeat_interleave(per)
+
+    def cloud(seed):
+        g = torch.Generator(cuda).manual_seed(seed)
+        pts = torch.randn(batch * per, 3, generator=g, device=cuda)
+        return pts / pts.norm(dim=1, keepdim=True) * torch.tensor([.45, .35, .25], device=cuda), torch.randn(batch * per, 3, generator=g, device=cuda), ids
+
+    given, build = [], _ext.get_indice_pairs_ahead
+
+    def watched(*args, **kw):
+        out = build(*args, **kw)
+        if out is not None and torch.cuda.is_current_stream_capturing():
+            given.append([(t.data_ptr(), t.data_ptr() + t.numel() * t.element_size()) for t in (out[0], out[1]._nbr_cap, out[1]._n_out_dev)])
+        return out
+
+    monkeypatch.setattr(_ext, "get_indice_pairs_ahead", watched)
+    with torch.no_grad():
+        graphed = GraphedPoints(p2v, net, batch * per, 3, cuda)
+        graphed._ready(*cloud(0))
+        side = given[1:]                         # (the first is built on the stream of the layers)
+        assert len(side) == (7 if pool else 3)
+        for k, one in enumerate(side):
+            for other in side[k + 1:]:
+                assert all(b <= c or d <= a for a, b in one for c, d in other)
+        for seed in range(3):
+            want = net(p2v(*cloud(seed))[1])
+            for _ in range(4):
+                assert torch.equal(graphed(*cloud(seed)), want)
+    assert graphed.fallbacks <= 1
+    _ext.check_status(cuda)
+
+
 def test_voxelizer_count_stays_on_the_device_into_a_graphed_chain(cuda):
     """Point2Voxel hands out a tensor whose voxel count is still on the device; a GraphedChain
     takes it as it is (the count is checked after the replay).  Results equal the exact path."""
