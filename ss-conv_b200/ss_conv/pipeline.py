@@ -35,6 +35,11 @@ class HostStream:
         if self.stage_in[slot] is None:
             self.stage_in[slot] = [torch.empty((self.cap,) + tuple(t.shape[1:]), dtype=t.dtype, device=self.dev)
                                    for t in batch]
+            # memory of the computing stream: work queued there may still read what was in it, and an upload under way
+            # must not find it handed on when the buffers go
+            self.up.wait_stream(torch.cuda.current_stream(self.dev))
+            for buf in self.stage_in[slot]:
+                buf.record_stream(self.up)
         views = []
         with torch.cuda.stream(self.up):
             if self.in_free[slot] is not None:

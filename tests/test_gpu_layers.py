@@ -152,6 +152,23 @@ def test_host_stream_gives_the_same_results_as_direct_calls(cuda):
     _ext.check_status(cuda)
 
 
+def test_host_stream_waits_for_the_readers_of_its_buffers_memory(cuda):
+    """The input buffers may be given memory that was freed with work still queued on it: the first uploads come behind that work."""
+    from ss_conv.pipeline import HostStream
+    rows = 1 << 20
+    old = [torch.full((rows, 8), float(k + 1), device=cuda) for k in range(2)]
+    at = {t.data_ptr() for t in old}
+    torch.cuda.synchronize()
+    torch.cuda._sleep(100_000_000)
+    kept = [t.sum() for t in old]
+    del old
+    stream = HostStream(lambda x: (x.sum().reshape(1),), cuda, rows)
+    host = [torch.full((rows, 8), 9.0).pin_memory() for _ in range(3)]
+    got = [float(out[0]) for out in stream.run((h,) for h in host)]
+    assert {b.data_ptr() for slot in stream.stage_in for b in slot} == at        # (else nothing was put to the test)
+    assert got == [9.0 * 8 * rows] * 3 and [float(t) for t in kept] == [8.0 * rows, 16.0 * rows]
+
+
 def test_layers_that_run_ahead_of_the_output_count(cuda, monkeypatch):
     """A strided convolution + max pool whose rulebooks are sized by a guessed capacity (output
     count read back after the kernels were queued) give bit-identical results to the exact
