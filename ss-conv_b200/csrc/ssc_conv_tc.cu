@@ -656,10 +656,10 @@ __device__ __forceinline__ void
 conv_fwd_rows(const float *__restrict__ features, int row_words, const uint4 *__restrict__ packed, int K, int c_out,
               const int32_t *__restrict__ nbr, int n_out, float *__restrict__ out, int32_t *status, const TcParams &p,
               const int32_t *__restrict__ n_out_dev, const int32_t *__restrict__ order, const GateEpilogue &gate) {
-  // Every CTA walks the filters in the same order at the same time, so each slab that is not in L2 stalls all of them.  While
-  // the kernel before this one still runs each thread asks for one line of 128 bytes; of a grid too small to cover the
+  // Every CTA walks the filters in the same order at the same time, so each slab that is not in L2 stalls all of them.  Before
+  // it waits for the kernel before this one, each thread asks for one line of 128 bytes; of a grid too small to cover the
   // image only the first slabs are asked for.  Nothing is read yet: L2 is where a filter that is still being packed is
-  // written.  Plain-12 network 1132 -> 1114 us, its training step 6140 -> 5958, strided layer with a pool 206 -> 202.
+  // written.  Strided layer with a pool 207 -> 202 us, voxel codec 206 -> 203, plain-12 network 1064 -> 1055.
   const int line = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (line < K * p.k_slabs * p.n_pad) asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)packed + (size_t)line * 128));
   after_previous();
