@@ -61,6 +61,14 @@ def _no_gc():
             gc.enable()
 
 
+def _finished(out):
+    """What the chain returns, with the norm that a last BatchNorm has only noted on it applied in the recording: applied when
+    the result is first looked at, it would be that batch's for good."""
+    if isinstance(out, SparseTensor):
+        out.raw()
+    return out
+
+
 class _Recording(object):
     """One capture of the chain: the graph, its input buffers, its outputs and its row counts."""
 
@@ -84,7 +92,7 @@ class _Recording(object):
         try:
             pinned = torch.empty(256, dtype=torch.int32).pin_memory()
             with _no_gc(), torch.cuda.graph(graph):
-                out = chain.fn(x)
+                out = _finished(chain.fn(x))
                 # input count first, the kernel status word last: it is read back with the counts
                 counts = torch.cat([self.n] + [r.n_dev.reshape(1) for r in log] + [_ext.status_word(chain.dev)])
                 if counts.shape[0] > pinned.shape[0]:
@@ -306,7 +314,7 @@ class _PointRecording(object):
         try:
             pinned = torch.empty(256, dtype=torch.int32).pin_memory()
             with _no_gc(), torch.cuda.graph(graph):
-                out = owner.fn(owner.p2v(self.pts, self.fts, self.ids)[1])
+                out = _finished(owner.fn(owner.p2v(self.pts, self.fts, self.ids)[1]))
                 counts = torch.cat([r.n_dev.reshape(1) for r in log] + [_ext.status_word(owner.dev)])
                 if counts.shape[0] > pinned.shape[0]:
                     raise RuntimeError("chain with more than %d pending row counts" % (pinned.shape[0] - 1))

@@ -436,6 +436,39 @@ def test_recorded_rulebooks_keep_their_memory_from_one_another(cuda, monkeypatch
     _ext.check_status(cuda)
 
 
+@pytest.mark.parametrize("points", [False, True])
+def test_recorded_chains_that_end_in_a_norm(cuda, points):
+    """An eval-mode BatchNorm notes its scale and shift on the tensor and whoever comes next applies them: as the last layer of a
+    recorded chain it is part of every replay."""
+    from ss_conv.batchnorm import BatchNorm
+    from ss_conv.convolution import Convolution
+    from ss_conv.graph import GraphedChain, GraphedPoints
+    from ss_conv.sp_ops.tensor import SparseTensor
+    from ss_conv.sp_ops.voxelize import Point2Voxel
+    torch.manual_seed(0)
+    rs = [(4, 0), (2, 1)]
+    net = torch.nn.Sequential(Convolution([(3, 0)], rs, 3, stride=2, padding=1), BatchNorm(rs)).to(cuda).eval()
+    with torch.no_grad():
+        net[1].weight.uniform_(0.5, 1.5)
+        net[1].bias.normal_()
+        if points:
+            p2v = Point2Voxel([16] * 3, [1 / 16.] * 3, 4, trusted_batch_size=2)
+            graphed = GraphedPoints(p2v, net, 400, 3, cuda)
+            ids = torch.arange(2, device=cuda, dtype=torch.int32).repeat_interleave(200)
+            inputs = [(torch.rand(400, 3, device=cuda) - 0.5, torch.randn(400, 3, device=cuda), ids) for _ in range(3)]
+            want = [net(p2v(*v)[1]) for v in inputs]
+        else:
+            graphed = GraphedChain(net, [16] * 3, 2, 3, 600, cuda)
+            rng = np.random.RandomState(0)
+            inputs = [(torch.randn(500, 3, device=cuda), dev(random_voxels(rng, 2, 16, 250), cuda)) for _ in range(3)]
+            want = [net(SparseTensor(f, i, [16] * 3, 2)) for f, i in inputs]
+        want = [(y.features.clone(), y.indices.clone()) for y in want]
+        for _ in range(2):
+            for v, (f, i) in zip(inputs, want):
+                y = graphed(*v)
+                assert torch.equal(y.indices, i) and torch.equal(y.features, f)
+
+
 def test_voxelizer_count_stays_on_the_device_into_a_graphed_chain(cuda):
     """Point2Voxel hands out a tensor whose voxel count is still on the device; a GraphedChain
     takes it as it is (the count is checked after the replay).  Results equal the exact path."""
