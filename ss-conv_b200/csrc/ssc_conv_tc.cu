@@ -1027,6 +1027,8 @@ __global__ void pack_filters_16_kernel(const float *__restrict__ filters, int K,
 // tile brings in whole, is most of what a step moves (TF32 128 -> 152, 238 tiles: 59.1 -> 52.3 us; 256 -> 304 bf16, 125 tiles: 54.4 -> 52.6).  The second CTA's
 // news reaches the issuing one some 300 cycles late, so short loops lose (256 tiles of 128 -> 152 bf16: 30.8 -> 31.9), rings of two slots
 // more so (64 -> 76, 1.1 M rows: 690 -> 770), and with many tiles on an SM another one fills the time (637 tiles of 128 -> 152 bf16: 63 -> 65).
+// Of eight TF32 and four 16-bit widths at 19 sizes one lost, where its second wave begins a few tiles earlier than single CTAs' (187 tiles of
+// 256 -> 304: 163 -> 174; 174 tiles 160 -> 151, 200 tiles 176 and 176).
 static bool rows_params(int words, int c_out, int n_out, TcParams &p, int opk = 1, bool pairs = false) {
   const int grid = n_out > 0 ? ceil_div(n_out, TC_M) : 1, sms = sm_count();
   auto plan = [&](bool pair) {

@@ -939,11 +939,11 @@ def test_chains_without_a_wait_have_the_bits_of_single_calls(cuda, monkeypatch, 
 
 
 def test_transposing_a_table_costs_little_more_than_a_copy(cuda):
-    """700 k rows of 27 offsets, 7 % of them present: 28 us, 55 where every block also told the next kernel to come, against some
-    25 us of a copy of the table."""
+    """700 k rows of 27 offsets, 7 % of them present, 1.4 times as long as a copy of the table, 2.5 times where every block also told the
+    next kernel to come: bound between the two."""
     from ss_conv import _ext
     n, n_in = 700000, 48000
     g = torch.Generator(cuda).manual_seed(0)
     t = torch.where(torch.rand(27, n, generator=g, device=cuda) < .07, torch.randint(0, n_in, (27, n), generator=g, device=cuda), -1).to(torch.int32)
     took = [_least_ms(f) for f in (lambda: _ext.input_major_table(t, n_in), lambda: t.clone())]
-    assert took[0] <= 1.7 * took[1], took
+    assert took[0] <= 1.9 * took[1], took
